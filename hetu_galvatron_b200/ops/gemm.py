@@ -38,6 +38,16 @@ _PAIR_MODE = os.environ.get("HG_GEMM_PAIR", "auto")
 _pair_ok = True
 
 
+def _use_skinny(M: int, N: int, a_mn: bool, out_mode: int, max_ctas: int, pair) -> bool:
+    """Whether the weight-streaming kernel (csrc/sm100/gemm_skinny.cu) takes the product.  Up to 64 rows it was at least
+    as fast everywhere (4 rows, cold: 4096 x 4096 16 us against 35 for the one-CTA kernel, 4096 x 11008 29 against 78,
+    152064 x 3584 176 against 208).  From 65 to 128 rows it pays for outputs of up to 64 of its tiles (128 rows: 4096
+    columns 25 against 35 us, 11008 columns 45 against 43, 152064 columns 221 against 207)."""
+    if a_mn or out_mode not in (OUT_BF16, OUT_F32) or pair is not None or max_ctas != 0 or _PAIR_MODE == "1":
+        return False
+    return M <= 64 or (M <= 128 and N <= 8192)
+
+
 def _use_pair(M: int, N: int, pair) -> bool:
     if pair is not None:
         return bool(pair)
@@ -89,6 +99,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         if out.shape[0] != M or out.shape[1] != N or out.stride(1) != 1:
             raise ValueError("bad output tensor")
     lib = _lib.load()
+    if _use_skinny(M, N, a_mn, out_mode, max_ctas, pair):
+        rc = lib.hg_gemm_skinny_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(bias), M, N, K, a.stride(0),
+                                     b.stride(0), out.stride(0), int(b_mn), out_mode, 0, _lib.stream())
+        if rc != 0:
+            raise _lib.KernelError("hg_gemm_skinny_bf16 failed with code %d (M=%d N=%d K=%d b_mn=%d)" % (rc, M, N, K, b_mn))
+        _lib.count_launch()
+        return out
     if _use_pair(M, N, pair):
         rc = lib.hg_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(bias), M, N, K, a.stride(0),
                                b.stride(0), out.stride(0), int(a_mn), int(b_mn), out_mode, max_ctas, _lib.stream())
