@@ -197,10 +197,8 @@ __global__ void glu_bwd_kernel(const hg_lp_t* __restrict__ g, const hg_lp_t* __r
 __global__ void embedding_fwd_kernel(const int64_t* __restrict__ ids, const hg_lp_t* __restrict__ W,
                                      const hg_lp_t* __restrict__ pos_emb, hg_lp_t* __restrict__ out,
                                      int tokens, int H, int v0, int v1, int batch, int pos_offset) {
-  const int vpr = H >> 3;
-  const int64_t total = int64_t(tokens) * vpr;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
-    const int t = int(i / vpr), c = int(i % vpr);
+  for (RowColWalk w(H >> 3); w.row < tokens; w.next()) {
+    const int t = int(w.row), c = w.col;
     const int64_t id = ids[t];
     uint4 v = make_uint4(0, 0, 0, 0);
     if (id >= v0 && id < v1) v = reinterpret_cast<const uint4*>(W + size_t(id - v0) * H)[c];
@@ -216,26 +214,32 @@ __global__ void embedding_fwd_kernel(const int64_t* __restrict__ ids, const hg_l
   }
 }
 
+// Adds eight gradients to eight consecutive fp32 words.  What bounds the scatter is the number of reductions the L2
+// executes, not the bytes: two 16-byte reductions do the work of eight 4-byte ones (8192 tokens x 4096, token
+// frequencies as in text: 191 us with 4-byte reductions, 59 us).
+template <bool VEC>
+__device__ __forceinline__ void add8(float* dst, const float (&g)[8]) {
+  if (VEC) {
+    atomicAdd(reinterpret_cast<float4*>(dst), make_float4(g[0], g[1], g[2], g[3]));
+    atomicAdd(reinterpret_cast<float4*>(dst) + 1, make_float4(g[4], g[5], g[6], g[7]));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) atomicAdd(dst + j, g[j]);
+  }
+}
+
+// VEC: dW and dpos are 16-byte aligned (their rows then are, too: H is a multiple of 8)
+template <bool VEC>
 __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids, const hg_lp_t* __restrict__ dout,
                                      float* __restrict__ dW, float* __restrict__ dpos, int tokens, int H, int v0,
                                      int v1, int batch, int pos_offset) {
-  const int vpr = H >> 3;
-  const int64_t total = int64_t(tokens) * vpr;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < total; i += int64_t(gridDim.x) * blockDim.x) {
-    const int t = int(i / vpr), c = int(i % vpr);
+  for (RowColWalk w(H >> 3); w.row < tokens; w.next()) {
+    const int t = int(w.row), c = w.col;
     const int64_t id = ids[t];
     float g[8];
     unpack8(reinterpret_cast<const uint4*>(dout + size_t(t) * H)[c], g);
-    if (id >= v0 && id < v1) {
-      float* dst = dW + size_t(id - v0) * H + c * 8;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) atomicAdd(dst + j, g[j]);
-    }
-    if (dpos) {
-      float* dst = dpos + size_t(t / batch + pos_offset) * H + c * 8;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) atomicAdd(dst + j, g[j]);
-    }
+    if (id >= v0 && id < v1) add8<VEC>(dW + size_t(id - v0) * H + c * 8, g);
+    if (dpos) add8<VEC>(dpos + size_t(t / batch + pos_offset) * H + c * 8, g);
   }
 }
 
@@ -379,8 +383,13 @@ int hg_embedding_bwd(const void* ids, const void* dout, void* dW, void* dpos, in
                      int batch, int pos_offset, void* stream) {
   if (tokens <= 0) return 0;
   if (H & 7) return -1;
-  embedding_bwd_kernel<<<grid_for(int64_t(tokens) * (H >> 3), 256), 256, 0, (cudaStream_t)stream>>>(
-      (const int64_t*)ids, (const hg_lp_t*)dout, (float*)dW, (float*)dpos, tokens, H, v0, v1, batch, pos_offset);
+  const int g = grid_for(int64_t(tokens) * (H >> 3), 256);
+  if (((uintptr_t(dW) | uintptr_t(dpos)) & 15) == 0)
+    embedding_bwd_kernel<true><<<g, 256, 0, (cudaStream_t)stream>>>(
+        (const int64_t*)ids, (const hg_lp_t*)dout, (float*)dW, (float*)dpos, tokens, H, v0, v1, batch, pos_offset);
+  else
+    embedding_bwd_kernel<false><<<g, 256, 0, (cudaStream_t)stream>>>(
+        (const int64_t*)ids, (const hg_lp_t*)dout, (float*)dW, (float*)dpos, tokens, H, v0, v1, batch, pos_offset);
   return int(cudaGetLastError());
 }
 
