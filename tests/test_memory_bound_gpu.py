@@ -30,3 +30,34 @@ def test_embedding_gradient_into_any_buffer(shift):
     assert rel_err(W.main_grad, ref) < 1e-6                         # fp32 sums of a few terms
     assert rel_err(P.main_grad, 1.0 + g.double().view(S, B, H).sum(1)) < 1e-6
     _lib.assert_healthy()
+
+
+# every group size of the norm backward (32 to 512 threads per row, one to four chunks per thread), rows fewer than,
+# equal to and more than the row groups of the grid
+@pytest.mark.parametrize("rms", [True, False])
+@pytest.mark.parametrize("rows,H", [(1, 8), (5000, 256), (37, 264), (1500, 768), (3, 1024), (700, 1600), (300, 4104),
+                                    (20, 8200), (310, 16384)])
+def test_norm_backward(rms, rows, H):
+    g = torch.Generator(device=DEV).manual_seed(rows + H)
+    r = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    x = r(rows, H).to(torch.bfloat16).requires_grad_()
+    w = (1 + 0.1 * r(H)).to(torch.bfloat16).requires_grad_()
+    b = None if rms else (0.1 * r(H)).to(torch.bfloat16).requires_grad_()
+    res = r(rows, H).to(torch.bfloat16)
+    y, h = ops.norm(x, w, b, 1e-5, rms, residual=res)
+    gy, gh = r(rows, H).to(torch.bfloat16), r(rows, H).to(torch.bfloat16)
+    w.main_grad = torch.full((H + 1,), 2.0, device=DEV)[1:]        # accumulated into, at any alignment
+    torch.autograd.backward([y, h], [gy, gh])
+    hd = h.detach().double().requires_grad_()
+    wd = w.detach().double().requires_grad_()
+    bd = None if rms else b.detach().double().requires_grad_()
+    if rms:
+        yd = hd * torch.rsqrt(hd.pow(2).mean(-1, keepdim=True) + 1e-5) * wd
+    else:
+        yd = torch.nn.functional.layer_norm(hd, (H,), wd, bd, 1e-5)
+    torch.autograd.backward([yd, hd], [gy.double(), gh.double()])
+    assert rel_err(x.grad, hd.grad) < 2.0 ** -8                     # fp32 arithmetic, one rounding
+    assert rel_err(w.main_grad, wd.grad + 2.0) < 1e-5               # fp32 sums
+    if not rms:
+        assert rel_err(b.grad, bd.grad) < 2.0 ** -8
+    _lib.assert_healthy()
