@@ -244,6 +244,69 @@ __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids, const hg_l
 }
 
 // ---------------------------------------------------------------------------------------------
+// Column sums of a 16-bit matrix (bias gradients): out[c] = sum_r x[r, c] in fp32, rounded once.
+// A CTA takes 256 columns (32 lanes of eight) and one of `parts` row ranges, its eight warps share the rows.
+// x is read once with 16-byte loads and nothing is widened in memory; rows are added in a fixed order.  2997 x 6400 with
+// the final sum: 11 us (38 MB; 50 us as a widening copy, a reduction and a cast).
+// ---------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+colsum_kernel(const hg_lp_t* __restrict__ x, int64_t pitch, int rows, int cols, float* __restrict__ partial,
+              hg_lp_t* __restrict__ out) {
+  __shared__ float red[8][256];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c0 = blockIdx.x * 256 + lane * 8;
+  const int r0 = int(int64_t(rows) * blockIdx.y / gridDim.y), r1 = int(int64_t(rows) * (blockIdx.y + 1) / gridDim.y);
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (c0 + 8 <= cols) {
+    const hg_lp_t* p = x + c0;
+    int r = r0 + warp;
+    for (; r + 24 < r1; r += 32) {                     // four rows in flight per warp
+      uint4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = __ldcs(reinterpret_cast<const uint4*>(p + int64_t(r + 8 * k) * pitch));
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float f[8];
+        unpack8(v[k], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] += f[j];
+      }
+    }
+    for (; r < r1; r += 8) {
+      float f[8];
+      unpack8(*reinterpret_cast<const uint4*>(p + int64_t(r) * pitch), f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s[j] += f[j];
+    }
+  } else {
+    for (int r = r0 + warp; r < r1; r += 8)
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (c0 + j < cols) s[j] += hg_lp2f(x[int64_t(r) * pitch + c0 + j]);
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) red[warp][lane * 8 + j] = s[j];
+  __syncthreads();
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  if (c < cols) {
+    float t = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t += red[k][threadIdx.x];
+    if (gridDim.y > 1) partial[int64_t(blockIdx.y) * cols + c] = t;
+    else out[c] = hg_f2lp(t);
+  }
+}
+
+__global__ void colsum_final_kernel(const float* __restrict__ partial, int parts, int cols, hg_lp_t* __restrict__ out) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  float t = 0.f;
+#pragma unroll 8
+  for (int p = 0; p < parts; ++p) t += partial[int64_t(p) * cols + c];
+  out[c] = hg_f2lp(t);
+}
+
+// ---------------------------------------------------------------------------------------------
 // Casts and the bf16 residual add
 // ---------------------------------------------------------------------------------------------
 __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ in, hg_lp_t* __restrict__ out, int64_t n) {
@@ -390,6 +453,27 @@ int hg_embedding_bwd(const void* ids, const void* dout, void* dW, void* dpos, in
   else
     embedding_bwd_kernel<false><<<g, 256, 0, (cudaStream_t)stream>>>(
         (const int64_t*)ids, (const hg_lp_t*)dout, (float*)dW, (float*)dpos, tokens, H, v0, v1, batch, pos_offset);
+  return int(cudaGetLastError());
+}
+
+// Row ranges the column sums of a [rows, cols] matrix are cut into: about four CTAs per SM, each warp with at least
+// four rows.  `partial` of hg_colsum_bf16 holds that many rows of `cols` floats.
+int hg_colsum_parts(int rows, int cols) {
+  const int blocks = (cols + 255) / 256;
+  int parts = (148 * 4 + blocks - 1) / (blocks > 0 ? blocks : 1);
+  if (parts > rows / 32) parts = rows / 32;
+  return parts < 1 ? 1 : (parts > 64 ? 64 : parts);
+}
+
+// out[c] = sum over rows of x[r, c]; x 16-byte aligned, pitch a multiple of 8 elements.
+int hg_colsum_bf16(const void* x, long long pitch, int rows, int cols, void* partial, int parts, void* out, void* stream) {
+  if (cols <= 0) return 0;
+  if ((pitch & 7) || (uintptr_t(x) & 15) || parts < 1 || parts > 65535) return -1;
+  cudaStream_t st = (cudaStream_t)stream;
+  colsum_kernel<<<dim3((cols + 255) / 256, parts), 256, 0, st>>>((const hg_lp_t*)x, pitch, rows, cols, (float*)partial,
+                                                                 (hg_lp_t*)out);
+  if (parts > 1)
+    colsum_final_kernel<<<(cols + 127) / 128, 128, 0, st>>>((const float*)partial, parts, cols, (hg_lp_t*)out);
   return int(cudaGetLastError());
 }
 

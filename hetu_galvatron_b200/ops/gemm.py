@@ -151,8 +151,25 @@ class _Linear(torch.autograd.Function):
             else:
                 dw = gemm(dy, x, a_mn=True, b_mn=True)
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy.float().sum(0).to(dy.dtype)
+            db = column_sums(dy)
         return dx, dw, db
+
+
+def column_sums(x: torch.Tensor) -> torch.Tensor:
+    """``x.float().sum(0)`` of a matrix, rounded back to its dtype: the gradient of a bias."""
+    rows, cols = x.shape
+    if x.is_cuda and x.dtype == _lib.lp_dtype():
+        x = _rowmajor(x)
+    if rows == 0 or cols == 0 or not x.is_cuda or x.dtype != _lib.lp_dtype() or x.stride(0) % 8 or x.data_ptr() % 16:
+        return x.float().sum(0).to(x.dtype)
+    lib = _lib.load()
+    out = torch.empty(cols, dtype=x.dtype, device=x.device)
+    parts = lib.hg_colsum_parts(rows, cols)
+    partial = torch.empty((parts, cols), dtype=torch.float32, device=x.device) if parts > 1 else None
+    _lib.check(lib.hg_colsum_bf16(x.data_ptr(), x.stride(0), rows, cols, _lib.ptr(partial), parts, out.data_ptr(),
+                                  _lib.stream()), "hg_colsum_bf16")
+    _lib.count_launch(2 if parts > 1 else 1)
+    return out
 
 
 def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:

@@ -4,6 +4,7 @@ import torch
 
 from hetu_galvatron_b200 import ops
 from hetu_galvatron_b200.ops import _lib
+from hetu_galvatron_b200.ops.gemm import column_sums
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -61,3 +62,14 @@ def test_norm_backward(rms, rows, H):
     if not rms:
         assert rel_err(b.grad, bd.grad) < 2.0 ** -8
     _lib.assert_healthy()
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (31, 264), (64, 1000), (2997, 6400), (100000, 16), (5, 70000)])
+def test_column_sums(rows, cols):
+    x = torch.randn(rows, cols, device=DEV).to(torch.bfloat16)
+    ref = x.double().sum(0)
+    # fp32 sums of `rows` unit-variance terms, one rounding of the result
+    assert torch.allclose(column_sums(x).double(), ref, rtol=2.0 ** -8, atol=1e-6 * rows)
+    wide = torch.randn(rows, cols + 8, device=DEV).to(torch.bfloat16)
+    assert torch.allclose(column_sums(wide[:, :cols]).double(), wide[:, :cols].double().sum(0), rtol=2.0 ** -8,
+                          atol=1e-6 * rows)
