@@ -27,7 +27,7 @@ import torch.distributed as dist
 import torch.nn as nn
 
 from .. import ops
-from ..ops.gemm import OUT_F32, OUT_F32_ACC
+from ..ops.gemm import OUT_F32, OUT_F32_ACC, _rowmajor
 from ..parallel import mappings as mp
 from ..parallel.zero import ShardedUnit, UnitWrapper
 from .modules import GalvatronAttention, Norm, _param, init_normal_sharded_, ops_add
@@ -429,6 +429,97 @@ def _aligned_starts(counts: torch.Tensor) -> Tuple[torch.Tensor, int]:
     return starts, int(starts[-1].item())
 
 
+def local_dispatch_usable(x: torch.Tensor, idx: torch.Tensor, E: int, k: int) -> bool:
+    """Whether the kernels of csrc/sm100/moe_local.cu take this call: 16-bit rows of whole 16-byte groups on a GPU."""
+    from ..ops import _lib
+
+    return x.is_cuda and x.dtype == _lib.lp_dtype() and x.shape[1] % 8 == 0 and E <= 256 and idx.shape[0] == x.shape[0]
+
+
+class _LocalPlan:
+    """Placement of every (token, slot) pair in this GPU's expert buffer (built on the device, nothing is read back):
+    ``row_start [E + 1]`` aligned segment starts, ``dest [T * k]`` row of each pair (-1: dropped), ``src [rows]`` pair of
+    each row (-1: padding).  ``rows`` is the least static size that holds any routing."""
+
+    def __init__(self, idx: torch.Tensor, E: int):
+        from ..ops import _lib
+
+        self.T, self.k = idx.shape
+        n = idx.numel()
+        flat = idx.reshape(-1).to(torch.int64)
+        self.rows = max((n + E * (SEG_ALIGN - 1)) // SEG_ALIGN * SEG_ALIGN, SEG_ALIGN)
+        i32 = dict(dtype=torch.int32, device=idx.device)
+        counts = torch.empty((max(1, (n + 1023) // 1024), E), **i32)
+        self.row_start = torch.empty(E + 1, **i32)
+        self.dest, self.src = torch.empty(n, **i32), torch.empty(self.rows, **i32)
+        _lib.check(_lib.load().hg_moe_plan(flat.data_ptr(), n, E, SEG_ALIGN, self.rows, counts.data_ptr(),
+                                           self.row_start.data_ptr(), self.dest.data_ptr(), self.src.data_ptr(),
+                                           _lib.stream()), "hg_moe_plan")
+        _lib.count_launch(2)
+
+
+def _moe_scatter(x, plan, w=None):
+    """``buf[r] = w[src[r]] * x[src[r] // k]``, zeros where no pair fills the row."""
+    from ..ops import _lib
+
+    buf = torch.empty((plan.rows, x.shape[1]), dtype=x.dtype, device=x.device)
+    _lib.check(_lib.load().hg_moe_scatter(x.data_ptr(), x.stride(0), plan.src.data_ptr(), _lib.ptr(w), plan.rows, plan.k,
+                                          x.shape[1], buf.data_ptr(), _lib.stream()), "hg_moe_scatter")
+    _lib.count_launch()
+    return buf
+
+
+def _moe_gather(y, plan, w=None):
+    """``out[t] = sum_j w[t, j] * y[dest[t, j]]`` (fp32 sums in slot order)."""
+    from ..ops import _lib
+
+    out = torch.empty((plan.T, y.shape[1]), dtype=y.dtype, device=y.device)
+    _lib.check(_lib.load().hg_moe_gather(y.data_ptr(), plan.dest.data_ptr(), _lib.ptr(w), plan.T, plan.k, y.shape[1],
+                                         out.data_ptr(), _lib.stream()), "hg_moe_gather")
+    _lib.count_launch()
+    return out
+
+
+class _LocalDispatch(torch.autograd.Function):
+    """Tokens -> aligned, zero-padded expert segments; the gradient of a token is the sum over its copies."""
+
+    @staticmethod
+    def forward(ctx, x, plan):
+        ctx.plan = plan
+        return _moe_scatter(_rowmajor(x), plan)
+
+    @staticmethod
+    def backward(ctx, g):
+        return _moe_gather(g.contiguous(), ctx.plan), None
+
+
+class _LocalCombine(torch.autograd.Function):
+    """``out[t] = sum_j w[t, j] * y[dest[t, j]]`` and its gradients."""
+
+    @staticmethod
+    def forward(ctx, y, w, plan):
+        y, w = y.contiguous(), w.contiguous()
+        ctx.plan = plan
+        ctx.save_for_backward(y, w)
+        return _moe_gather(y, plan, w)
+
+    @staticmethod
+    def backward(ctx, g):
+        from ..ops import _lib
+
+        y, w = ctx.saved_tensors
+        plan = ctx.plan
+        g = _rowmajor(g)
+        dy = _moe_scatter(g, plan, w) if ctx.needs_input_grad[0] else None
+        dw = None
+        if ctx.needs_input_grad[1]:
+            dw = torch.empty_like(w)
+            _lib.check(_lib.load().hg_moe_dot(y.data_ptr(), g.data_ptr(), g.stride(0), plan.dest.data_ptr(), w.numel(),
+                                              plan.k, y.shape[1], dw.data_ptr(), _lib.stream()), "hg_moe_dot")
+            _lib.count_launch()
+        return dy, dw, None
+
+
 class GalvatronMoEMLP(nn.Module):
     """Token dispatch + experts + combine."""
 
@@ -495,6 +586,11 @@ class GalvatronMoEMLP(nn.Module):
                 w = torch.where(idx >= 0, probs, torch.zeros_like(probs)).to(torch.float32)
                 # the routing weights are applied inside the pull kernel: no [T, k, H] intermediate
                 return fa.moe_combine_weighted(out_buf, w, plan)
+        if ep == 1 and local_dispatch_usable(x2d, idx, E, k):
+            plan = _LocalPlan(idx, E)
+            buf = _LocalDispatch.apply(x2d, plan)
+            out_buf = self.experts(buf, plan.row_start)
+            return _LocalCombine.apply(out_buf, probs.to(torch.float32), plan)
         flat_e = idx.reshape(-1)
         valid = flat_e >= 0
         sort_key = torch.where(valid, flat_e, torch.full_like(flat_e, E))

@@ -66,6 +66,11 @@ _SIGNATURES = {
     "hg_gemm_skinny_bf16": [c_void_p] * 4 + [c_int] * 9 + [c_void_p],
     "hg_colsum_parts": [c_int, c_int],
     "hg_colsum_bf16": [c_void_p, c_ll, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p],
+    "hg_moe_plan": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+    "hg_moe_scatter": [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+    "hg_moe_gather": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+    "hg_moe_dot": [c_void_p, c_void_p, c_ll, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
+    "hg_zero_outside": [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "hg_grouped_gemm_bf16": [c_void_p] * 4 + [c_int] * 9 + [c_void_p],
     "hg_grouped_wgrad_bf16": [c_void_p] * 4 + [c_int] * 8 + [c_void_p],
     "hg_norm_fwd": [c_void_p] * 8 + [c_int, c_int, c_float, c_int, c_void_p],

@@ -193,8 +193,10 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, row_start: torch.Tensor, *, b
         K, N = b.shape[1], b.shape[2]
     else:
         N, K = b.shape[1], b.shape[2]
-    if out is None:
-        out = torch.zeros((a.shape[0], N), dtype=a.dtype, device=a.device)
+    fresh = out is None
+    if fresh:
+        # on the GPU the product covers every row of a segment: only the rows outside them are cleared (below)
+        out = (torch.empty if a.is_cuda and N % 8 == 0 else torch.zeros)((a.shape[0], N), dtype=a.dtype, device=a.device)
     if not a.is_cuda:
         rs = row_start.tolist()
         for g in range(G):
@@ -210,6 +212,10 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, row_start: torch.Tensor, *, b
                                   K, a.stride(0), b2.stride(0), out.stride(0), int(b_mn), OUT_BF16, _lib.stream())
     _lib.check(rc, "hg_grouped_gemm_bf16")
     _lib.count_launch()
+    if fresh and N % 8 == 0:
+        _lib.check(lib.hg_zero_outside(out.data_ptr(), row_start.data_ptr(), G, out.shape[0], N, _lib.stream()),
+                   "hg_zero_outside")
+        _lib.count_launch()
     return out
 
 

@@ -1,0 +1,81 @@
+"""Single-GPU expert dispatch (csrc/sm100/moe_local.cu): the placement against a list-based restatement, and the row
+passes against index operations in 64 bits."""
+import pytest
+import torch
+
+from hetu_galvatron_b200.models.moe import SEG_ALIGN, _LocalCombine, _LocalDispatch, _LocalPlan
+from hetu_galvatron_b200.ops import _lib
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def placement(idx, E):
+    """(row_start, dest) of every pair, expert-major and in pair order."""
+    by = [[] for _ in range(E)]
+    for p, e in enumerate(idx.reshape(-1).tolist()):
+        if e >= 0:
+            by[e].append(p)
+    starts, dest = [0], [-1] * idx.numel()
+    for e in range(E):
+        for i, p in enumerate(by[e]):
+            dest[p] = starts[-1] + i
+        starts.append(starts[-1] + (len(by[e]) + SEG_ALIGN - 1) // SEG_ALIGN * SEG_ALIGN)
+    return starts, dest
+
+
+# one token; all pairs on one expert; chunk edges of the placement kernel (1024 pairs); dropped pairs; 256 experts
+@pytest.mark.parametrize("T,k,E,H,drop", [(1, 1, 1, 8, 0.0), (128, 2, 8, 264, 0.0), (512, 2, 8, 4096, 0.1),
+                                          (513, 2, 4, 72, 1.0), (1000, 8, 160, 256, 0.3), (341, 3, 256, 2048, 0.0)])
+def test_local_dispatch_and_combine(T, k, E, H, drop):
+    g = torch.Generator().manual_seed(T + k + E)
+    idx = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(T)])
+    idx[torch.rand(T, k, generator=g) < drop] = -1
+    plan = _LocalPlan(idx.to(DEV), E)
+    starts, dest = placement(idx, E)
+    assert plan.row_start.tolist() == starts and plan.dest.tolist() == dest
+    src = [-1] * plan.rows
+    for p, r in enumerate(dest):
+        if r >= 0:
+            src[r] = p
+    assert plan.src.tolist() == src
+
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV).requires_grad_()
+    w = torch.rand(T, k, generator=g).to(DEV).requires_grad_()
+    buf = _LocalDispatch.apply(x, plan)
+    tok = torch.tensor([p // k if p >= 0 else 0 for p in src], device=DEV)
+    live = torch.tensor([p >= 0 for p in src], device=DEV)[:, None]
+    assert torch.equal(buf, torch.where(live, x.detach()[tok], torch.zeros_like(x.detach()[tok])))
+    dbuf = torch.randn(plan.rows, H, generator=g).to(torch.bfloat16).to(DEV)
+    buf.backward(dbuf)
+    d = torch.tensor(dest, device=DEV).view(T, k)
+    rows = dbuf.double()[d.clamp(min=0)] * (d >= 0)[..., None]
+    assert torch.allclose(x.grad.double(), rows.sum(1), rtol=2.0 ** -8, atol=1e-5)   # one rounding to bf16
+
+    y = torch.randn(plan.rows, H, generator=g).to(torch.bfloat16).to(DEV).requires_grad_()
+    out = _LocalCombine.apply(y, w, plan)
+    rows = y.detach().double()[d.clamp(min=0)] * (d >= 0)[..., None]
+    ref = (rows * w.detach().double()[..., None]).sum(1)
+    assert torch.allclose(out.double(), ref, rtol=2.0 ** -8, atol=1e-5)
+    dout = torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV)
+    out.backward(dout)
+    ref_dw = (rows * dout.double()[:, None]).sum(-1)
+    assert torch.allclose(w.grad.double(), ref_dw, rtol=1e-4, atol=1e-5 * H ** 0.5)  # fp32 sums of H products
+    ref_dy = torch.zeros(plan.rows, H, dtype=torch.float64, device=DEV)
+    ref_dy[d[d >= 0]] = (w.detach().double()[..., None] * dout.double()[:, None])[d >= 0]
+    assert torch.allclose(y.grad.double(), ref_dy, rtol=2.0 ** -8, atol=1e-7)
+    _lib.assert_healthy()
+
+
+def test_grouped_gemm_clears_the_rows_outside_its_segments():
+    from hetu_galvatron_b200 import ops
+
+    a = torch.randn(640, 64, device=DEV).to(torch.bfloat16)
+    b = torch.randn(2, 72, 64, device=DEV).to(torch.bfloat16)
+    junk = torch.full((640, 72), float("nan"), device=DEV, dtype=torch.bfloat16)
+    del junk                                                            # the allocator hands these bytes out again
+    out = ops.grouped_gemm(a, b, torch.tensor([128, 256, 512], device=DEV, dtype=torch.int32))
+    assert (out[:128] == 0).all() and (out[512:] == 0).all()
+    ref = torch.cat([a[128:256].double() @ b[0].double().t(), a[256:512].double() @ b[1].double().t()])
+    assert ((out[128:512].double() - ref).norm() / ref.norm()).item() < 2.0 ** -8
+    _lib.assert_healthy()
