@@ -92,7 +92,7 @@ grouped_gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       // tiles of this group owned by this CTA: global index = counter + t
       int t = (int(blockIdx.x) - counter % int(gridDim.x) + int(gridDim.x)) % int(gridDim.x);
       for (; t < cnt; t += gridDim.x) {
-        const int tm = t / tiles_n, tn = t % tiles_n;
+        const int tm = t % tm_cnt, tn = t / tm_cnt;   // an expert's weight tile is read once for all its row tiles
         if (!fn(g, r0 + tm * BM, r1, tn * BN)) return;
       }
       counter += cnt;

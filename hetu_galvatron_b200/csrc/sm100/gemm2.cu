@@ -23,19 +23,11 @@
 namespace hg {
 namespace gemm2 {
 
-template <bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(192, 1)
-gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Params p) {
-  extern __shared__ uint8_t smem_raw[];
-  Smem2 s = carve2(smem_raw);
-  const int warp = threadIdx.x >> 5;
-  const uint32_t rank = cluster_ctarank();
-  const int num_tiles = p.tiles_m * p.tiles_n;
-  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-
+// Barriers, tensor memory and the first meeting of the pair; returns the tensor-memory base address.
+__device__ __forceinline__ uint32_t pair_setup(const Smem2& s, const CUtensorMap* tmA, const CUtensorMap* tmB, int warp) {
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
+    tma_prefetch_desc(tmA);
+    tma_prefetch_desc(tmB);
 #pragma unroll
     for (int i = 0; i < STAGES2; ++i) {
       mbar_init(&s.full[i], 1);
@@ -57,7 +49,30 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   cluster_sync_all();  // the partner's barriers exist before anything arrives on them remotely
   tc_fence_after();
-  const uint32_t tmem_base = *s.tmem_base;
+  return *s.tmem_base;
+}
+
+__device__ __forceinline__ void pair_teardown(uint32_t tmem_base, int warp) {
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // neither CTA frees tensor memory or leaves while its partner may still touch it
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, TMEM_COLS);
+  }
+}
+
+template <bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(192, 1)
+gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  Smem2 s = carve2(smem_raw);
+  const int warp = threadIdx.x >> 5;
+  const uint32_t rank = cluster_ctarank();
+  const int num_tiles = p.tiles_m * p.tiles_n;
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+
+  const uint32_t tmem_base = pair_setup(s, &tmA, &tmB, warp);
 
   if (warp == 0) {
     producer2<A_MN, B_MN>(&tmA, &tmB, p, s, rank, pair, pairs, num_tiles);
@@ -67,13 +82,190 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     epilogue2(p, s, tmem_base, rank, pair, pairs, num_tiles);
   }
 
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync_all();  // neither CTA frees tensor memory or leaves while its partner may still touch it
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc_pair(tmem_base, TMEM_COLS);
+  pair_teardown(tmem_base, warp);
+}
+
+// ---- grouped products on the pair's tile (mixture-of-experts layers) ------------------------------------------------
+// One launch for the G products of a layer whose sizes only the device knows.  Every role of every pair walks the same
+// tile list; `fn(tile)` returns false to stop.
+struct GroupedTile {
+  int m, m_end, n;        // first row and column of the output tile; rows from m_end on are another group's
+  int a_k, b_off;         // offsets into the stacked operands (see the loads below)
+  int num_kb;
+  long long c_off;
+};
+
+// C[r0:r1] = A[r0:r1] op(B_g) for the row segments [r0, r1) = row_start[g..g+1].  Inside a segment up to eight row tiles
+// of one column tile come first: the weight is then read from HBM once by the pairs that need it at the same time, and
+// A, whose eight tiles fit the L2, is what is re-read.  (Walking the columns first streamed an expert's whole weight
+// once per row tile.)
+struct RowSegments {
+  const int* row_start;
+  int G, tiles_n, num_kb, b_group_rows, max_rows;
+  int* status;
+  static constexpr int kGroupM = 8;
+  template <typename F>
+  __device__ __forceinline__ void walk(int pair, int pairs, F&& fn) const {
+    int counter = 0;
+    for (int g = 0; g < G; ++g) {
+      const int r0 = row_start[g], r1 = row_start[g + 1];
+      // an expert's row range must lie inside the operand and not run backwards (checked in the debug build)
+      if (!HG_BOUNDS_OK(r0 >= 0 && r1 >= r0 && r1 <= max_rows, status)) return;
+      const int tm_cnt = (r1 - r0 + CM - 1) / CM, cnt = tm_cnt * tiles_n;
+      for (int t = (pair - counter % pairs + pairs) % pairs; t < cnt; t += pairs) {
+        const int first = t / (kGroupM * tiles_n) * kGroupM, gsize = min(kGroupM, tm_cnt - first);
+        const int r = t - first * tiles_n;
+        GroupedTile w{r0 + (first + r % gsize) * CM, r1, r / gsize * BN, 0, g * b_group_rows, num_kb, 0};
+        if (!fn(w)) return;
+      }
+      counter += cnt;
+    }
   }
+};
+
+// C_g (+)= A[k0:k1]^T B[k0:k1] for the contraction ranges [k0, k1) = k_start[g..g+1] (multiples of 64).
+struct ContractionRanges {
+  const int* k_start;
+  int G, tiles_m, tiles_n, M;
+  long long c_group_stride;
+  static constexpr int kGroupM = 4;
+  template <typename F>
+  __device__ __forceinline__ void walk(int pair, int pairs, F&& fn) const {
+    const int per = tiles_m * tiles_n;
+    for (int t = pair; t < per * G; t += pairs) {
+      const int g = t / per, u = t - g * per;
+      const int first = u / (kGroupM * tiles_n) * kGroupM, gsize = min(kGroupM, tiles_m - first);
+      const int r = u - first * tiles_n;
+      const int k0 = k_start[g];
+      GroupedTile w{(first + r % gsize) * CM, M, r / gsize * BN, k0, k0, (k_start[g + 1] - k0 + BK - 1) / BK,
+                    g * c_group_stride};
+      if (!fn(w)) return;
+    }
+  }
+};
+
+template <bool A_MN, bool B_MN, typename Tiles>
+__global__ void __launch_bounds__(192, 1)
+grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Params p,
+                     const Tiles tiles) {
+  extern __shared__ uint8_t smem_raw[];
+  Smem2 s = carve2(smem_raw);
+  const int warp = threadIdx.x >> 5;
+  const uint32_t rank = cluster_ctarank();
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+  const uint32_t tmem_base = pair_setup(s, &tmA, &tmB, warp);
+
+  if (warp == 0) {
+    uint32_t stage = 0, phase = 0;
+    bool ok = true;
+    const bool issuer = elect_one() != 0;
+    tiles.walk(pair, pairs, [&](const GroupedTile& w) {
+      const int m = w.m + int(rank) * BM, n = w.n + int(rank) * HALF_N;
+      for (int kb = 0; kb < w.num_kb; ++kb) {
+        if (!mbar_wait_warp(&s.empty[stage], phase ^ 1, p.status, kTimeoutSmemEmpty, s.abort)) { ok = false; return false; }
+        const uint32_t bar = map_to_cta(smem_u32(&s.full[stage]), 0);
+        uint8_t* sa = s.a + stage * A2_BYTES;
+        uint8_t* sb = s.b + stage * B2_BYTES;
+        const int k0 = kb * BK;
+        if (issuer) {
+          if (rank == 0) mbar_expect_tx(&s.full[stage], 2 * (A2_BYTES + B2_BYTES));
+          if (A_MN) {
+#pragma unroll
+            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * SLAB_BYTES, &tmA, bar, m + j * 64, w.a_k + k0);
+          } else {
+            tma_load_2d_pair(sa, &tmA, bar, k0, m);
+          }
+          if (B_MN) {
+#pragma unroll
+            for (int j = 0; j < HALF_N / 64; ++j) tma_load_2d_pair(sb + j * SLAB_BYTES, &tmB, bar, n + j * 64, w.b_off + k0);
+          } else {
+            tma_load_2d_pair(sb, &tmB, bar, k0, w.b_off + n);
+          }
+        }
+        __syncwarp();
+        if (++stage == STAGES2) { stage = 0; phase ^= 1; }
+      }
+      return true;
+    });
+    if (!ok) {
+      *s.abort = 1;
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);  // 2 ms: far longer than a tile load
+    }
+  } else if (warp == 1) {
+    if (rank == 0) {
+      constexpr uint32_t idesc = make_idesc_lp(CM, BN, A_MN, B_MN);
+      constexpr uint32_t a_lbo = A_MN ? SLAB_BYTES : 16, a_kadv = A_MN ? 2048 : 32;
+      constexpr uint32_t b_lbo = B_MN ? SLAB_BYTES : 16, b_kadv = B_MN ? 2048 : 32;
+      uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+      bool ok = true;
+      const bool issuer = elect_one() != 0;
+      tiles.walk(pair, pairs, [&](const GroupedTile& w) {
+        if (w.num_kb <= 0) return true;   // nothing to contract: the epilogue writes the result
+        if (!mbar_wait_warp(&s.tmem_empty[acc], acc_phase ^ 1, p.status, kTimeoutTmemEmpty, s.abort)) { ok = false; return false; }
+        tc_fence_after();
+        const uint32_t d = tmem_base + acc * BN;
+        for (int kb = 0; kb < w.num_kb; ++kb) {
+          if (!mbar_wait_warp(&s.full[stage], phase, p.status, kTimeoutSmemFull, s.abort)) { ok = false; return false; }
+          tc_fence_after();
+          const uint32_t sa = smem_u32(s.a + stage * A2_BYTES);
+          const uint32_t sb = smem_u32(s.b + stage * B2_BYTES);
+          if (issuer) {
+#pragma unroll
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_f16_ss_pair(d, make_smem_desc(sa + k * a_kadv, a_lbo, 1024), make_smem_desc(sb + k * b_kadv, b_lbo, 1024),
+                               idesc, (kb | k) != 0);
+            umma_commit_pair(&s.empty[stage], kPairMask);
+          }
+          __syncwarp();
+          if (++stage == STAGES2) { stage = 0; phase ^= 1; }
+        }
+        if (issuer) umma_commit_pair(&s.tmem_full[acc], kPairMask);
+        __syncwarp();
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        return true;
+      });
+      if (!ok) *s.abort = 1;
+    }
+  } else {
+    const int wq = warp & 3, lane = int(lane_id());
+    const uint32_t lane_off = uint32_t(wq * 32) << 16;
+    float* stg = s.epi_stage + wq * EPI_STAGE_FLOATS;
+    uint32_t acc = 0, acc_phase = 0;
+    tiles.walk(pair, pairs, [&](const GroupedTile& w) {
+      const int row0 = w.m + int(rank) * BM + wq * 32;
+      Params q = p;
+      q.M = w.m_end;
+      q.C = p.out_mode == kOutF32 || p.out_mode == kOutF32Acc ? static_cast<void*>(reinterpret_cast<float*>(p.C) + w.c_off)
+                                                              : static_cast<void*>(reinterpret_cast<hg_lp_t*>(p.C) + w.c_off);
+      const bool empty = w.num_kb <= 0;
+      if (!empty) {
+        if (!mbar_wait_warp(&s.tmem_full[acc], acc_phase, p.status, kTimeoutTmemFull, s.abort)) { *s.abort = 1; return false; }
+        tc_fence_after();
+      }
+#pragma unroll 1
+      for (int c = 0; c < BN / 32; ++c) {
+        if (row0 >= w.m_end || w.n + c * 32 >= p.N) break;   // warp-uniform
+        uint32_t r0[32];
+        if (!empty) {
+          tmem_ld32(tmem_base + lane_off + acc * BN + c * 32, r0);
+          tmem_ld_wait();
+        }
+#pragma unroll
+        for (int i = 0; i < 32; ++i) stg[lane * 33 + i] = empty ? 0.f : __uint_as_float(r0[i]);
+        __syncwarp();
+        store_block_rows(q, stg, row0, w.n + c * 32);
+        __syncwarp();
+      }
+      if (empty) return true;
+      tc_fence_before();
+      if (rank == 0) mbar_arrive(&s.tmem_empty[acc]);
+      else mbar_arrive_cluster(map_to_cta(smem_u32(&s.tmem_empty[acc]), 0));
+      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      return true;
+    });
+  }
+  pair_teardown(tmem_base, warp);
 }
 
 }  // namespace gemm2
@@ -132,35 +324,55 @@ bool split_enabled() {
 
 }  // namespace
 
+// Launch attributes of a kernel of CTA pairs, and how many pairs of it the device holds at once (-2: none).
+template <typename K>
+static int pair_config(K kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int* max_pairs, cudaStream_t st) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = 2;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg->blockDim = dim3(192, 1, 1);
+  cfg->dynamicSmemBytes = SMEM2_BYTES;
+  cfg->stream = st;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+  if (*max_pairs < 0) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES);
+    if (e != cudaSuccess) return int(e);
+    int sms = 0, dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cfg->gridDim = dim3(unsigned(sms / 2 * 2), 1, 1);
+    int n = 0;
+    e = cudaOccupancyMaxActiveClusters(&n, kernel, cfg);
+    if (e != cudaSuccess) return int(e);
+    if (n <= 0) return -2;
+    *max_pairs = n;
+  }
+  return 0;
+}
+
+template <bool A_MN, bool B_MN, typename Tiles>
+static int launch_grouped2(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, const Tiles& tiles, int want_pairs,
+                           cudaStream_t st) {
+  static int max_pairs = -1;
+  auto k = grouped_gemm2_kernel<A_MN, B_MN, Tiles>;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr;
+  if (int rc = pair_config(k, &cfg, &attr, &max_pairs, st)) return rc;
+  const int pairs = want_pairs < max_pairs ? want_pairs : max_pairs;
+  cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
+  return int(cudaLaunchKernelEx(&cfg, k, ta, tb, p, tiles));
+}
+
 template <bool A_MN, bool B_MN>
 static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p_in, int want_pairs, cudaStream_t st) {
   Params p = p_in;
   static int max_pairs = -1;
   auto k = gemm2_bf16_kernel<A_MN, B_MN>;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(192, 1, 1);
-  cfg.dynamicSmemBytes = SMEM2_BYTES;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  if (max_pairs < 0) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM2_BYTES);
-    if (e != cudaSuccess) return int(e);
-    int sms = 0, dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cfg.gridDim = dim3(unsigned(sms / 2 * 2), 1, 1);
-    int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, k, &cfg);
-    if (e != cudaSuccess) return int(e);
-    if (n <= 0) return -2;
-    max_pairs = n;
-  }
+  cudaLaunchAttribute attr;
+  if (int rc = pair_config(k, &cfg, &attr, &max_pairs, st)) return rc;
   const int pairs = want_pairs < max_pairs ? want_pairs : max_pairs;
   cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
   // Last wave partly filled: let several pairs share each of its tiles (see Params::split_s).
@@ -216,6 +428,42 @@ int hg_gemm2_bf16(const void* A, const void* B, void* C, const void* bias, int M
   if (a_mn) return launch2<true, false>(ta, tb, p, pairs, st);
   if (b_mn) return launch2<false, true>(ta, tb, p, pairs, st);
   return launch2<false, false>(ta, tb, p, pairs, st);
+}
+
+// Same contracts as hg_grouped_gemm_bf16 and hg_grouped_wgrad_bf16 (gemm.cu), computed by CTA pairs; -2 as above.
+int hg_grouped_gemm2_bf16(const void* A, const void* B, void* C, const void* row_start, int G, int max_rows, int N,
+                          int K, int lda, int ldb, int ldc, int b_mn, int out_mode, void* stream) {
+  if (G <= 0 || max_rows <= 0) return 0;
+  if ((lda & 7) || (ldb & 7)) return -1;
+  CUtensorMap ta, tb;
+  int rc = hg_host::make_tmap_2d_bf16(&ta, A, max_rows, K, lda, BM, 64);
+  if (rc) return rc;
+  if (b_mn) rc = hg_host::make_tmap_2d_bf16(&tb, B, uint64_t(G) * K, N, ldb, 64, 64);
+  else      rc = hg_host::make_tmap_2d_bf16(&tb, B, uint64_t(G) * N, K, ldb, HALF_N, 64);
+  if (rc) return rc;
+  Params p{};
+  p.M = max_rows; p.N = N; p.K = K; p.ldc = ldc; p.C = C; p.out_mode = out_mode; p.status = hg_host::status_ptr();
+  RowSegments t{reinterpret_cast<const int*>(row_start), G, (N + BN - 1) / BN, (K + BK - 1) / BK, b_mn ? K : N, max_rows,
+                p.status};
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  return b_mn ? launch_grouped2<false, true>(ta, tb, p, t, 1 << 20, st) : launch_grouped2<false, false>(ta, tb, p, t, 1 << 20, st);
+}
+
+int hg_grouped_wgrad2_bf16(const void* dy, const void* x, void* out, const void* row_start, int G, int rows, int N,
+                           int K, int lddy, int ldx, int out_mode, int max_ctas, void* stream) {
+  if (G <= 0 || rows <= 0) return 0;
+  if ((lddy & 7) || (ldx & 7)) return -1;
+  CUtensorMap ta, tb;
+  int rc = hg_host::make_tmap_2d_bf16(&ta, dy, rows, N, lddy, 64, 64);
+  if (rc) return rc;
+  rc = hg_host::make_tmap_2d_bf16(&tb, x, rows, K, ldx, 64, 64);
+  if (rc) return rc;
+  Params p{};
+  p.M = N; p.N = K; p.K = rows; p.ldc = K; p.C = out; p.out_mode = out_mode; p.status = hg_host::status_ptr();
+  ContractionRanges t{reinterpret_cast<const int*>(row_start), G, (N + CM - 1) / CM, (K + BN - 1) / BN, N, (long long)N * K};
+  int pairs = t.tiles_m * t.tiles_n * G;
+  if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
+  return launch_grouped2<true, true>(ta, tb, p, t, pairs, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -208,8 +208,11 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, row_start: torch.Tensor, *, b
     a = _rowmajor(a)
     b2 = b.reshape(G * b.shape[1], b.shape[2])
     lib = _lib.load()
-    rc = lib.hg_grouped_gemm_bf16(a.data_ptr(), b2.data_ptr(), out.data_ptr(), row_start.data_ptr(), G, a.shape[0], N,
-                                  K, a.stride(0), b2.stride(0), out.stride(0), int(b_mn), OUT_BF16, _lib.stream())
+    args = (a.data_ptr(), b2.data_ptr(), out.data_ptr(), row_start.data_ptr(), G, a.shape[0], N, K, a.stride(0),
+            b2.stride(0), out.stride(0), int(b_mn), OUT_BF16, _lib.stream())
+    rc = lib.hg_grouped_gemm2_bf16(*args) if _use_pair(a.shape[0], N, None) else -2
+    if rc == -2:
+        rc = lib.hg_grouped_gemm_bf16(*args)
     _lib.check(rc, "hg_grouped_gemm_bf16")
     _lib.count_launch()
     if fresh and N % 8 == 0:
@@ -235,9 +238,11 @@ def grouped_wgrad(dy: torch.Tensor, x: torch.Tensor, row_start: torch.Tensor, ou
         return out
     dy, x = _rowmajor(dy), _rowmajor(x)
     lib = _lib.load()
-    rc = lib.hg_grouped_wgrad_bf16(dy.data_ptr(), x.data_ptr(), out.data_ptr(), row_start.data_ptr(), G, dy.shape[0],
-                                   out.shape[1], out.shape[2], dy.stride(0), x.stride(0),
-                                   OUT_F32_ACC if accumulate else OUT_F32, 0, _lib.stream())
+    args = (dy.data_ptr(), x.data_ptr(), out.data_ptr(), row_start.data_ptr(), G, dy.shape[0], out.shape[1],
+            out.shape[2], dy.stride(0), x.stride(0), OUT_F32_ACC if accumulate else OUT_F32, 0, _lib.stream())
+    rc = lib.hg_grouped_wgrad2_bf16(*args) if _use_pair(out.shape[1], out.shape[2], None) else -2
+    if rc == -2:
+        rc = lib.hg_grouped_wgrad_bf16(*args)
     _lib.check(rc, "hg_grouped_wgrad_bf16")
     _lib.count_launch()
     return out
