@@ -219,6 +219,136 @@ __global__ void scale_kernel(T* __restrict__ x, int64_t n, const float* __restri
   }
 }
 
+// ---------------------------------------------------------------------------------------------
+// The same two passes over a list of buffers in one launch.  A model has a unit per layer plus a few small ones, and a
+// step over a small model is bound by its launches (each unit: two for the norm, one for its gradient scale, one for the
+// update); the list travels in the kernel's parameters and a block finds its buffer by a binary search over them.
+// ---------------------------------------------------------------------------------------------
+constexpr int kMaxList = 48;
+
+struct ListHeader {
+  int count;
+  int first_block[kMaxList + 1];
+};
+struct SumsqList {
+  ListHeader h;
+  const float* x[kMaxList];
+  long long n[kMaxList];
+  float scale[kMaxList];
+};
+struct AdamList {
+  ListHeader h;
+  float *p[kMaxList], *m[kMaxList], *v[kMaxList];
+  const float* g[kMaxList];
+  hg_lp_t* p_lp[kMaxList];
+  long long n[kMaxList];
+};
+static_assert(sizeof(AdamList) <= 3 * 1024, "kernel parameters");
+
+__device__ __forceinline__ int list_entry(const ListHeader& h) {
+  int lo = 0, hi = h.count - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (h.first_block[mid] <= int(blockIdx.x)) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+// partial[block] = scale * sum of squares of the block's share of its buffer
+__global__ void __launch_bounds__(256)
+sumsq_list_kernel(const __grid_constant__ SumsqList L, float* __restrict__ partial) {
+  const int e = list_entry(L.h);
+  const int block = blockIdx.x - L.h.first_block[e], blocks = L.h.first_block[e + 1] - L.h.first_block[e];
+  const float* x = L.x[e];
+  const int64_t n = L.n[e], stride = int64_t(blocks) * 256, first = int64_t(block) * 256 + threadIdx.x;
+  float s = 0.f;
+  int64_t done = 0;
+  if ((uintptr_t(x) & 15) == 0) {
+    const int64_t groups = n / 4;
+    int64_t i = first;
+    for (; i + stride < groups; i += 2 * stride) {
+      const float a = sumsq_group<float>(x, i), b = sumsq_group<float>(x, i + stride);
+      s += a + b;
+    }
+    if (i < groups) s += sumsq_group<float>(x, i);
+    done = groups * 4;
+  }
+  for (int64_t i = done + first; i < n; i += stride) s += x[i] * x[i];
+  __shared__ float red[8];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float t = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t += red[i];
+    partial[blockIdx.x] = t * L.scale[e];
+  }
+}
+
+__global__ void __launch_bounds__(256)
+adamw_list_kernel(const __grid_constant__ AdamList L, AdamArgs a, const float* __restrict__ gscale, float host_scale) {
+  const int e = list_entry(L.h);
+  const int block = blockIdx.x - L.h.first_block[e], blocks = L.h.first_block[e + 1] - L.h.first_block[e];
+  const float gs = (gscale ? *gscale : 1.f) * host_scale;
+  const float step = a.lr / a.bias1;
+  const float inv_b2 = rsqrtf(a.bias2);
+  float4 *p4 = reinterpret_cast<float4*>(L.p[e]), *m4 = reinterpret_cast<float4*>(L.m[e]), *v4 = reinterpret_cast<float4*>(L.v[e]);
+  const float4* g4 = reinterpret_cast<const float4*>(L.g[e]);
+  uint2* lp = reinterpret_cast<uint2*>(L.p_lp[e]);
+  const int64_t n4 = L.n[e] / 4, stride = int64_t(blocks) * 256;
+  for (int64_t i = int64_t(block) * 256 + threadIdx.x; i < n4; i += 2 * stride) {
+    const int64_t idx[2] = {i, i + stride};
+    const bool on[2] = {true, i + stride < n4};
+    float4 pv[2], gv[2], mv[2], vv[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (on[h]) {
+        pv[h] = p4[idx[h]];
+        gv[h] = __ldcs(g4 + idx[h]);
+        mv[h] = m4[idx[h]];
+        vv[h] = v4[idx[h]];
+      }
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (on[h]) {
+        const float x0 = adam_one(pv[h].x, gv[h].x * gs, mv[h].x, vv[h].x, a, step, inv_b2);
+        const float x1 = adam_one(pv[h].y, gv[h].y * gs, mv[h].y, vv[h].y, a, step, inv_b2);
+        const float x2 = adam_one(pv[h].z, gv[h].z * gs, mv[h].z, vv[h].z, a, step, inv_b2);
+        const float x3 = adam_one(pv[h].w, gv[h].w * gs, mv[h].w, vv[h].w, a, step, inv_b2);
+        p4[idx[h]] = pv[h];
+        m4[idx[h]] = mv[h];
+        v4[idx[h]] = vv[h];
+        if (lp) lp[idx[h]] = make_uint2(hg::pack_bf16(x0, x1), hg::pack_bf16(x2, x3));
+      }
+  }
+  if (block == 0 && threadIdx.x < (L.n[e] & 3)) {
+    const int64_t i = n4 * 4 + threadIdx.x;
+    float p = L.p[e][i], m = L.m[e][i], v = L.v[e][i];
+    const float x = adam_one(p, L.g[e][i] * gs, m, v, a, step, inv_b2);
+    L.p[e][i] = p;
+    L.m[e][i] = m;
+    L.v[e][i] = v;
+    if (L.p_lp[e]) L.p_lp[e][i] = hg_f2lp(x);
+  }
+}
+
+// Blocks of each entry: one per 1024 elements, at most its share of 148 * 8 (never none).
+void assign_blocks(ListHeader& h, const long long* n, int count) {
+  long long total = 0;
+  for (int i = 0; i < count; ++i) total += n[i];
+  h.count = count;
+  h.first_block[0] = 0;
+  for (int i = 0; i < count; ++i) {
+    long long want = (n[i] + 1023) / 1024;
+    const long long share = total > 0 ? (long long)(148.0 * 8 * double(n[i]) / double(total)) : 0;
+    if (want > share) want = share;
+    h.first_block[i + 1] = h.first_block[i] + int(want < 1 ? 1 : want);
+  }
+}
+
 inline int grid_for(int64_t n) {
   int64_t g = (n + 1023) / 1024;
   return int(g < 1 ? 1 : (g > 148 * 8 ? 148 * 8 : g));
@@ -278,6 +408,53 @@ int hg_sumsq(const void* x, long long n, int is_bf16, void* partial, void* out, 
     else sumsq_partial_kernel<float><<<g, 256, 0, st>>>((const float*)x, n, (float*)partial, vec);
   }
   sumsq_final_kernel<<<1, 256, 0, st>>>((const float*)partial, g, (float*)out, accumulate, scale);
+  return int(cudaGetLastError());
+}
+
+// Most buffers of one hg_sumsq_list / hg_adamw_list call, and floats of scratch of hg_sumsq_list.
+int hg_list_capacity() { return kMaxList; }
+int hg_list_scratch() { return 148 * 8 + kMaxList; }
+
+// out[0] (+)= sum_i scale[i] * sum(x_i^2) over `count` fp32 buffers.
+int hg_sumsq_list(const void* const* x, const long long* n, const float* scale, int count, void* partial, void* out,
+                  int accumulate, void* stream) {
+  if (count < 1 || count > kMaxList) return -1;
+  SumsqList L{};
+  for (int i = 0; i < count; ++i) {
+    L.x[i] = (const float*)x[i];
+    L.n[i] = n[i];
+    L.scale[i] = scale[i];
+  }
+  assign_blocks(L.h, n, count);
+  const int blocks = L.h.first_block[count];
+  cudaStream_t st = (cudaStream_t)stream;
+  sumsq_list_kernel<<<blocks, 256, 0, st>>>(L, (float*)partial);
+  sumsq_final_kernel<<<1, 256, 0, st>>>((const float*)partial, blocks, (float*)out, accumulate, 1.f);
+  return int(cudaGetLastError());
+}
+
+// One AdamW step on `count` buffers that share the hyper-parameters and the step: fp32 p, g, m, v (16-byte aligned) and
+// the 16-bit copy p_lp (8-byte aligned); the gradient is multiplied by host_scale and by *gscale (optional).
+int hg_adamw_list(void* const* p, const void* const* g, void* const* m, void* const* v, void* const* p_lp,
+                  const long long* n, int count, float lr, float beta1, float beta2, float eps, float weight_decay, int step,
+                  const void* gscale, float host_scale, void* stream) {
+  if (count < 1 || count > kMaxList) return -1;
+  AdamList L{};
+  for (int i = 0; i < count; ++i) {
+    if (((uintptr_t(p[i]) | uintptr_t(g[i]) | uintptr_t(m[i]) | uintptr_t(v[i])) & 15) || (uintptr_t(p_lp[i]) & 7)) return -1;
+    L.p[i] = (float*)p[i];
+    L.g[i] = (const float*)g[i];
+    L.m[i] = (float*)m[i];
+    L.v[i] = (float*)v[i];
+    L.p_lp[i] = (hg_lp_t*)p_lp[i];
+    L.n[i] = n[i];
+  }
+  AdamArgs a;
+  a.lr = lr; a.beta1 = beta1; a.beta2 = beta2; a.eps = eps; a.weight_decay = weight_decay;
+  a.bias1 = 1.f - powf(beta1, float(step));
+  a.bias2 = 1.f - powf(beta2, float(step));
+  assign_blocks(L.h, n, count);
+  adamw_list_kernel<<<L.h.first_block[count], 256, 0, (cudaStream_t)stream>>>(L, a, (const float*)gscale, host_scale);
   return int(cudaGetLastError());
 }
 

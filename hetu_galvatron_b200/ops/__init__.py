@@ -5,4 +5,5 @@ from .attention import (attention_merge, attention_reference, flash_attention, f
 from .fused import (activation, apply_mrope, cross_entropy, embedding, mrope_angles, norm, rope_packed,  # noqa: F401
                     rope_tables, router_topk)
 from .gemm import gemm, grouped_gemm, grouped_wgrad, linear  # noqa: F401
-from .optim import adamw_step, cast_bf16, clip_coefficient, scale_, sumsq  # noqa: F401
+from .optim import (adamw_step, adamw_step_list, cast_bf16, clip_coefficient, scale_, sumsq,  # noqa: F401
+                    sumsq_list)

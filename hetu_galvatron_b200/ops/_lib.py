@@ -73,6 +73,10 @@ _SIGNATURES = {
     "hg_zero_outside": [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "hg_grouped_gemm2_bf16": [c_void_p] * 4 + [c_int] * 9 + [c_void_p],
     "hg_grouped_wgrad2_bf16": [c_void_p] * 4 + [c_int] * 8 + [c_void_p],
+    "hg_list_capacity": [],
+    "hg_list_scratch": [],
+    "hg_sumsq_list": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p],
+    "hg_adamw_list": [c_void_p] * 6 + [c_int] + [c_float] * 5 + [c_int, c_void_p, c_float, c_void_p],
     "hg_grouped_gemm_bf16": [c_void_p] * 4 + [c_int] * 9 + [c_void_p],
     "hg_grouped_wgrad_bf16": [c_void_p] * 4 + [c_int] * 8 + [c_void_p],
     "hg_norm_fwd": [c_void_p] * 8 + [c_int, c_int, c_float, c_int, c_void_p],

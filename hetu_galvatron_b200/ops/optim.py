@@ -5,6 +5,8 @@ Oracle for AdamW: ``torch.optim.AdamW`` (decoupled weight decay, bias-corrected 
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _lib
@@ -68,6 +70,49 @@ def sumsq(x: torch.Tensor, out: torch.Tensor, accumulate: bool = True, scale: fl
     _lib.check(rc, "hg_sumsq")
     _lib.count_launch(2)
     return out
+
+
+def _pointers(tensors):
+    return (ctypes.c_void_p * len(tensors))(*[_lib.ptr(t) for t in tensors])
+
+
+def _counts(tensors):
+    return (ctypes.c_longlong * len(tensors))(*[t.numel() for t in tensors])
+
+
+def sumsq_list(terms, out: torch.Tensor, accumulate: bool = True):
+    """``out[0] (+)= sum(scale * sum(x^2))`` over ``terms`` of ``(x, scale)`` with a fixed reduction order: two launches
+    for up to ``hg_list_capacity()`` fp32 CUDA buffers."""
+    if not terms or not out.is_cuda or any(x.dtype != torch.float32 or not x.is_contiguous() for x, _ in terms):
+        if not accumulate:
+            out.zero_()
+        for x, scale in terms:
+            sumsq(x, out, accumulate=True, scale=scale)
+        return out
+    lib = _lib.load()
+    cap = lib.hg_list_capacity()
+    partial = torch.empty(lib.hg_list_scratch(), dtype=torch.float32, device=out.device)
+    for i in range(0, len(terms), cap):
+        xs, scales = [x for x, _ in terms[i:i + cap]], [float(c) for _, c in terms[i:i + cap]]
+        rc = lib.hg_sumsq_list(_pointers(xs), _counts(xs), (ctypes.c_float * len(xs))(*scales), len(xs), partial.data_ptr(),
+                               out.data_ptr(), int(accumulate or i > 0), _lib.stream())
+        _lib.check(rc, "hg_sumsq_list")
+        _lib.count_launch(2)
+    return out
+
+
+def adamw_step_list(entries, *, lr: float, beta1: float, beta2: float, eps: float, weight_decay: float, step: int,
+                    gscale: torch.Tensor | None = None, scale: float = 1.0):
+    """:func:`adamw_step` on a list of ``(p32, grad32, m, v, p_lp)`` flat CUDA buffers that share the hyper-parameters
+    and the step, in one launch per ``hg_list_capacity()`` of them; gradients are multiplied by ``scale`` and ``gscale``."""
+    lib = _lib.load()
+    cap = lib.hg_list_capacity()
+    for i in range(0, len(entries), cap):
+        cols = list(zip(*entries[i:i + cap]))
+        rc = lib.hg_adamw_list(*[_pointers(c) for c in cols], _counts(cols[0]), len(cols[0]), lr, beta1, beta2, eps,
+                               weight_decay, step, _lib.ptr(gscale), float(scale), _lib.stream())
+        _lib.check(rc, "hg_adamw_list")
+        _lib.count_launch()
 
 
 def clip_coefficient(total_sumsq: torch.Tensor, max_norm: float, coef: torch.Tensor, norm_out: torch.Tensor):

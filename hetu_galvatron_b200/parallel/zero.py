@@ -502,22 +502,36 @@ class ShardedUnit:
         self.grad_shard = self._target()
         self._reduced = True
 
-    def grad_sumsq(self, out: torch.Tensor):
-        """Add this rank's share of the squared gradient norm to ``out[0]`` so that a SUM over all ranks
+    def norm_terms(self):
+        """``(buffer, scale)`` terms of the squared gradient norm: summed over all ranks, ``scale * sum(buffer^2)``
         counts every parameter element exactly once."""
         if not self.count_in_norm:
-            return
+            return []
         g = self.grad_shard
         inv = 1.0 / (self.dp_size * self.dp_size)  # gradients are still dp-sums here
         rep = self.n if self.dp_type == "ddp" else 1  # identical copies held by the sdp group
-        ops.sumsq(g, out, accumulate=True, scale=inv / rep)
+        terms = [(g, inv / rep)]
         if self.tp_n > 1 and self.replicated_numel > 0:
             lo, hi = self.shard_range()
             a, b = max(lo, 0), min(hi, self.replicated_numel)
             if b > a:
-                ops.sumsq(g[a - lo:b - lo], out, accumulate=True, scale=inv / rep * (1.0 / self.tp_n - 1.0))
+                terms.append((g[a - lo:b - lo], inv / rep * (1.0 / self.tp_n - 1.0)))
+        return terms
+
+    def grad_sumsq(self, out: torch.Tensor):
+        """Add this rank's share of the squared gradient norm (:meth:`norm_terms`) to ``out[0]``."""
+        for x, scale in self.norm_terms():
+            ops.sumsq(x, out, accumulate=True, scale=scale)
 
     # ---- optimizer --------------------------------------------------------------------------------------
+    def takes_list_step(self) -> bool:
+        """Whether this unit's update is AdamW on its own buffers and nothing else (no parameter exchange, fp32 gradient
+        and 16-bit parameters on a GPU), so that it can share a launch with other units."""
+        return (bool(self.params) and not self.fused and self.dp_type == "ddp" and self.device.type == "cuda"
+                and self.dtype in (torch.bfloat16, torch.float16) and self.grad_shard.dtype == torch.float32
+                and all(t.data_ptr() % 16 == 0 for t in (self.master, self.grad_shard, self.exp_avg, self.exp_avg_sq,
+                                                         self.shard_lp)))
+
     def optimizer_step(self, lr, beta1, beta2, eps, weight_decay, clip_coef: Optional[torch.Tensor] = None):
         if not self.params:
             return

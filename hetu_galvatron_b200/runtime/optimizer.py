@@ -68,9 +68,7 @@ class ShardedAdamW:
             REDUCE.join(self.units[0].device)
 
     def compute_grad_norm(self):
-        self._sumsq.zero_()
-        for u in self.units:
-            u.grad_sumsq(self._sumsq)
+        ops.sumsq_list([t for u in self.units for t in u.norm_terms()], self._sumsq, accumulate=False)
         if dist.is_initialized() and dist.get_world_size() > 1:
             dist.all_reduce(self._sumsq)
         ops.clip_coefficient(self._sumsq, self.clip_grad, self._coef, self._norm)
@@ -84,8 +82,17 @@ class ShardedAdamW:
         self.reduce_gradients()
         self.compute_grad_norm()
         coef = self._coef if self.clip_grad > 0 else None
+        together: Dict = {}                # units whose whole update is one AdamW pass share launches
         for u in self.units:
-            u.optimizer_step(g["lr"], g["betas"][0], g["betas"][1], g["eps"], g["weight_decay"], coef)
+            if u.takes_list_step():
+                u.step_count += 1
+                together.setdefault((u.step_count, u.dp_size), []).append(u)
+            else:
+                u.optimizer_step(g["lr"], g["betas"][0], g["betas"][1], g["eps"], g["weight_decay"], coef)
+        for (step, dp_size), units in together.items():
+            ops.adamw_step_list([(u.master, u.grad_shard, u.exp_avg, u.exp_avg_sq, u.shard_lp) for u in units], lr=g["lr"],
+                                beta1=g["betas"][0], beta2=g["betas"][1], eps=g["eps"], weight_decay=g["weight_decay"],
+                                step=step, gscale=coef, scale=1.0 / dp_size)
         self._sync_fused_groups()          # peers' parameter stores have landed before the next forward
 
     def state_dict(self) -> Dict:
