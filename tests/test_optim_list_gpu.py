@@ -1,0 +1,38 @@
+"""AdamW and the squared norm over a list of buffers against the one-buffer kernels and 64-bit sums."""
+import pytest
+import torch
+
+from hetu_galvatron_b200 import ops
+from hetu_galvatron_b200.ops import _lib
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# one buffer, a tiny one beside a large one, lengths that are no multiple of four, more buffers than one launch takes
+@pytest.mark.parametrize("sizes", [[1], [3, 1_000_003], [64, 4096, 5, 70_000], [4 * i + i % 4 + 1 for i in range(100)]])
+def test_list_step_equals_single_steps(sizes):
+    g = torch.Generator(device=DEV).manual_seed(len(sizes))
+    hp = dict(lr=1e-3, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=3)
+    coef = torch.full((1,), 0.7, device=DEV)
+    rows = []
+    for n in sizes:
+        p, gr, m = (torch.randn(n, device=DEV, generator=g) for _ in range(3))
+        rows.append((p, gr, m, torch.rand(n, device=DEV, generator=g), p.to(torch.bfloat16)))
+    want = [tuple(t.clone() for t in r) for r in rows]
+    for r in want:
+        ops.adamw_step(*r, gscale=coef * 0.5, **hp)
+    ops.adamw_step_list(rows, gscale=coef, scale=0.5, **hp)
+    assert all(torch.equal(a, b) for r, w in zip(rows, want) for a, b in zip(r, w))
+
+    out = torch.full((1,), 5.0, device=DEV)
+    terms = [(r[1], 1.0 + i) for i, r in enumerate(rows)]
+    ref = sum(c * x.double().pow(2).sum().item() for x, c in terms)
+    ops.sumsq_list(terms, out)
+    assert abs(out.item() - 5.0 - ref) < 1e-5 * (ref + 5.0)        # fp32 sums in a fixed order
+    ops.sumsq_list(terms, out, accumulate=False)
+    assert abs(out.item() - ref) < 1e-5 * ref
+    shifted = torch.randn(1001, device=DEV, generator=g)[1:]      # not 16-byte aligned
+    ops.sumsq_list([(shifted, 1.0)], out, accumulate=False)
+    assert abs(out.item() - shifted.double().pow(2).sum().item()) < 1e-2
+    _lib.assert_healthy()
