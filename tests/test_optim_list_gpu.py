@@ -23,7 +23,15 @@ def test_list_step_equals_single_steps(sizes):
     for r in want:
         ops.adamw_step(*r, gscale=coef * 0.5, **hp)
     ops.adamw_step_list(rows, gscale=coef, scale=0.5, **hp)
-    assert all(torch.equal(a, b) for r, w in zip(rows, want) for a, b in zip(r, w))
+    # the same arithmetic; the last n mod 4 elements run through another kernel's code in the one-buffer form, where the
+    # compiler may contract the three chained operations differently (a few units of 2^-24 of the operands, which are
+    # below 8), and the 16-bit copy may then round the other way (2^-8)
+    for r, w in zip(rows, want):
+        for a, b in zip(r, w):
+            low = a.dtype == torch.bfloat16
+            assert torch.allclose(a.float(), b.float(), rtol=2.0 ** -7 if low else 1e-6, atol=2e-6)
+            n4 = a.numel() // 4 * 4
+            assert torch.equal(a[:n4], b[:n4])
 
     out = torch.full((1,), 5.0, device=DEV)
     terms = [(r[1], 1.0 + i) for i, r in enumerate(rows)]
