@@ -726,28 +726,57 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 // =================================================================================================
 // Backward, part 0:  D[b,h,s] = sum_d dO * O
 // =================================================================================================
-__global__ void attn_bwd_dot_kernel(const hg_lp_t* __restrict__ O, const hg_lp_t* __restrict__ dO,
-                                    int64_t ss, int64_t sb, int64_t dss, int64_t dsb, int S, int B, int nheads, int hd,
-                                    float* __restrict__ D) {
-  // one warp per (s, b, h)
-  const int64_t total = int64_t(S) * B * nheads;
-  const int64_t gw = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (gw >= total) return;
-  const int h = int(gw % nheads);
-  const int b = int((gw / nheads) % B);
-  const int s = int(gw / (int64_t(nheads) * B));
-  const hg_lp_t* o = O + s * ss + b * sb + h * hd;
-  const hg_lp_t* d = dO + s * dss + b * dsb + h * hd;
-  float acc = 0.f;
-  for (int i = lane * 2; i < hd; i += 64) {
-    const float2 a = hg_lp22ff(*reinterpret_cast<const hg_lp2_t*>(o + i));
-    const float2 c = hg_lp22ff(*reinterpret_cast<const hg_lp2_t*>(d + i));
-    acc += a.x * c.x + a.y * c.y;
-  }
+// O and dO are read once, 16 bytes per lane: HD / 8 lanes share a (token, head) row and meet in log2(HD / 8) shuffles.
+// (A warp per row with 4-byte loads had half a kilobyte in flight per warp and reached a third of the memory rate:
+// 64 us for the 134 MB of 8192 tokens x 32 heads x 128.)
+// VEC = false: for an O or dO whose rows are not 16-byte aligned.
+template <bool VEC>
+__device__ __forceinline__ uint4 dot_load8(const hg_lp_t* p) {
+  if (VEC) return __ldcs(reinterpret_cast<const uint4*>(p));
+  uint4 u;
+  hg_lp_t* e = reinterpret_cast<hg_lp_t*>(&u);
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-  if (lane == 0) D[(size_t(b) * nheads + h) * S + s] = acc;
+  for (int i = 0; i < 8; ++i) e[i] = p[i];
+  return u;
+}
+template <int HD, bool VEC>
+__global__ void __launch_bounds__(256)
+attn_bwd_dot_kernel(const hg_lp_t* __restrict__ O, const hg_lp_t* __restrict__ dO, int64_t ss, int64_t sb, int64_t dss,
+                    int64_t dsb, int S, int B, int nheads, float* __restrict__ D) {
+  constexpr int LPR = HD / 8, U = 4;              // lanes per row, rows in flight per thread
+  const int64_t total = int64_t(S) * B * nheads;
+  const int sub = threadIdx.x % LPR;
+  const int64_t stride = int64_t(gridDim.x) * (256 / LPR);
+  for (int64_t r0 = int64_t(blockIdx.x) * (256 / LPR) + threadIdx.x / LPR; r0 - threadIdx.x / LPR < total; r0 += U * stride) {
+    uint4 a[U], c[U];
+    float* dst[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int64_t row = r0 + u * stride;
+      dst[u] = nullptr;
+      a[u] = c[u] = make_uint4(0, 0, 0, 0);
+      if (row < total) {
+        const int tok = int(row / nheads), h = int(row - int64_t(tok) * nheads), s = tok / B, b = tok - s * B;
+        a[u] = dot_load8<VEC>(O + s * ss + b * sb + h * HD + sub * 8);
+        c[u] = dot_load8<VEC>(dO + s * dss + b * dsb + h * HD + sub * 8);
+        dst[u] = D + (size_t(b) * nheads + h) * S + s;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t* x = reinterpret_cast<const uint32_t*>(&a[u]);
+      const uint32_t* y = reinterpret_cast<const uint32_t*>(&c[u]);
+      float acc = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 p = hg_unpack2(x[i]), q = hg_unpack2(y[i]);
+        acc += p.x * q.x + p.y * q.y;
+      }
+#pragma unroll
+      for (int o = LPR / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (sub == 0 && dst[u] != nullptr) *dst[u] = acc;
+    }
+  }
 }
 
 // =================================================================================================
@@ -2162,10 +2191,14 @@ int hg_flash_bwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTenso
   cudaStream_t st = (cudaStream_t)stream;
   int rc;
   {
-    const int64_t warps = int64_t(Sq) * B * nheads;
-    const int blocks = int((warps * 32 + 255) / 256);
-    attn_bwd_dot_kernel<<<blocks, 256, 0, st>>>((const hg_lp_t*)o->ptr, (const hg_lp_t*)d_o->ptr, o->ss,
-                                                o->sb, d_o->ss, d_o->sb, Sq, B, nheads, hd, (float*)dsum);
+    const bool vec = (((uintptr_t(o->ptr) | uintptr_t(d_o->ptr)) & 15) | ((o->ss | o->sb | d_o->ss | d_o->sb) & 7)) == 0;
+    const int64_t rows = int64_t(Sq) * B * nheads;
+    const int64_t want = (rows * (hd / 8) + 256 * 4 - 1) / (256 * 4);
+    const int blocks = int(want < 148 * 8 ? want : 148 * 8);
+    auto k = hd == 128 ? (vec ? attn_bwd_dot_kernel<128, true> : attn_bwd_dot_kernel<128, false>)
+                       : (vec ? attn_bwd_dot_kernel<64, true> : attn_bwd_dot_kernel<64, false>);
+    k<<<blocks, 256, 0, st>>>((const hg_lp_t*)o->ptr, (const hg_lp_t*)d_o->ptr, o->ss, o->sb, d_o->ss, d_o->sb, Sq, B,
+                              nheads, (float*)dsum);
   }
   BwdParams p{};
   p.Sq = Sq; p.Skv = Skv; p.B = B; p.nheads = nheads; p.qpg = nheads / nkv; p.causal = causal;
