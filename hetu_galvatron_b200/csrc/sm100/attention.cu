@@ -413,7 +413,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 }
 
 // =================================================================================================
-// Forward with two query tiles per CTA and P in tensor memory (head dim 128).
+// Forward with two query tiles per CTA and P in tensor memory (both head dims).
 // In the one-tile kernel a scheduler hosts a single softmax warp, so every latency of its step (the loads from tensor
 // memory, the maximum, the exp2 / convert chains) is exposed, and the tensor core idles while the softmax of its only
 // tile runs.  Here a CTA owns 256 queries as two tiles of 128, one softmax warpgroup per tile: while one tile's
@@ -437,7 +437,7 @@ template <int HD>
 __global__ void __launch_bounds__(320, 1)
 flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const FwdParams p) {
-  static_assert(HD == 128, "the two-tile forward is written for head dim 128");
+  static_assert(HD == 64 || HD == 128, "tensor memory holds two S tiles and two O tiles of up to 128 columns");
   extern __shared__ uint8_t smem_raw[];
   using L = Fwd2Smem<HD>;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1131,7 +1131,8 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 }
 
 // =================================================================================================
-// Backward, part 1 with 128-query steps and the probabilities kept in tensor memory (head dim 128).
+// Backward, part 1 with 128-query steps and the probabilities kept in tensor memory (both head dims; gpt2-xl sized,
+// 8 x 1024 x 25 heads of 64: 170 -> 144 us against the 64-query kernel).
 // The 64-query version issues its score products with N = 64, which occupy the tensor core as long as N = 128 would,
 // and stages P^T / dS^T through 64 KB of shared memory.  Here a step covers 128 queries:
 //   S^T = K Q^T and dP^T = V dO^T are 128 x 128 products (8 MMAs each);
@@ -1160,7 +1161,8 @@ struct Dkv128Smem {
   static constexpr int kStats = 2 * 2 * 128 * 4;  // -lse*log2e and D of a step, double buffered
   static constexpr int kBars = 256;
   static constexpr int kUsed = 2 * kKV + (kQStages + kDOStages) * kQD + kStats + kBars;
-  static constexpr int kTotal = 232448;          // everything a CTA can have; the 1024-byte alignment of the tiles comes out of the rest
+  // head dim 128: everything a CTA can have; the 1024-byte alignment of the tiles comes out of the rest
+  static constexpr int kTotal = HD == 128 ? 232448 : kUsed + 1024;
 };
 
 // NWG softmax warpgroups (2 or 4): thread == key row, warpgroup g owns query columns [g * 128 / NWG, (g + 1) * 128 / NWG)
@@ -1171,9 +1173,11 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1)
 flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                         const BwdParams p) {
-  static_assert(HD == 128, "the 128-query dK/dV kernel is written for head dim 128");
+  static_assert(HD == 64 || HD == 128, "tensor memory holds S^T, dP^T and two accumulators of up to 128 columns");
   static_assert(NWG == 2 || NWG == 4, "two or four softmax warpgroups");
   constexpr int kSoftmaxWarps = 4 * NWG;
+  // head dim 64: dS^T is formed from fp32 probabilities, as in the 64-query kernel
+  constexpr bool kExactP = HD == 64;
   constexpr int CPT = 128 / NWG;               // query columns per thread and step
   extern __shared__ uint8_t smem_raw[];
   using L = Dkv128Smem<HD>;
@@ -1409,6 +1413,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       if (++cur_qs == n_qs) cur_qs = qs0;
       const float* st = sStats + sb * 256;
       uint32_t pp[CPT / 2];               // this thread's probabilities, packed, kept for the second phase
+      float pf[kExactP ? CPT : 1];        // and in fp32, where dS^T is formed from those
       // ---------------- S^T -> probabilities (kept in registers; the S^T columns are released at once)
       if (!mbar_wait_warp(&stats_full[sb], (it >> 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
       if (!mbar_wait_warp(st_full, ph, p.status, kTimeoutTmemFull, abort_flag)) { ok = false; break; }
@@ -1443,6 +1448,10 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
                 e[u] = (u < HG_DKV_POLY_OF_4) ? ex2_poly(x) : ex2(x);
                 if (decltype(masked)::value && (!k_valid || (p.causal && k_pos > q_base + i + u))) e[u] = 0.f;
               }
+              if constexpr (kExactP) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) pf[hh * 32 + i + u] = e[u];
+              }
               pp[hh * 16 + (i >> 1)] = pack_bf16(e[0], e[1]);
               pp[hh * 16 + (i >> 1) + 1] = pack_bf16(e[2], e[3]);
             }
@@ -1474,7 +1483,14 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
             const float4 dd = dd4[i >> 2];
-            const float2 p01 = hg_unpack2(pp[hh * 16 + (i >> 1)]), p23 = hg_unpack2(pp[hh * 16 + (i >> 1) + 1]);
+            float2 p01, p23;
+            if constexpr (kExactP) {
+              p01 = make_float2(pf[hh * 32 + i], pf[hh * 32 + i + 1]);
+              p23 = make_float2(pf[hh * 32 + i + 2], pf[hh * 32 + i + 3]);
+            } else {
+              p01 = hg_unpack2(pp[hh * 16 + (i >> 1)]);
+              p23 = hg_unpack2(pp[hh * 16 + (i >> 1) + 1]);
+            }
             dsp[hh * 16 + (i >> 1)] = pack_bf16(p01.x * (__uint_as_float(r[i]) - dd.x),
                                                  p01.y * (__uint_as_float(r[i + 1]) - dd.y));
             dsp[hh * 16 + (i >> 1) + 1] = pack_bf16(p23.x * (__uint_as_float(r[i + 2]) - dd.z),
@@ -1548,248 +1564,8 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
 }
 
 // =================================================================================================
-// Backward, part 2: one CTA per (query block of 128, head, batch); loops over 64-row key steps.
-// Thread == query row.   S = Q K^T, dP = dO V^T (N = 64);  dS = P * (dP - D);  dQ += dS K
-// =================================================================================================
-template <int HD>
-struct DqSmem {
-  static constexpr int kQ = 128 * HD * 2;     // resident Q or dO
-  static constexpr int kKV = 64 * HD * 2;     // one stage of K or V
-  static constexpr int kDS = 128 * 64 * 2;    // one dS buffer (two are kept so that step i+1 is written while step i is multiplied)
-  static constexpr int kTotal = 2 * kQ + 4 * kKV + 2 * kDS + 1024 + 256;
-};
-
-template <int HD>
-__global__ void __launch_bounds__(kBwdThreads, 1)
-flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                    const BwdParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = base;
-  uint8_t* sDO = sQ + DqSmem<HD>::kQ;
-  uint8_t* sK = sDO + DqSmem<HD>::kQ;            // 2 stages
-  uint8_t* sV = sK + 2 * DqSmem<HD>::kKV;        // 2 stages
-  uint8_t* sDS = sV + 2 * DqSmem<HD>::kKV;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sDS + 2 * DqSmem<HD>::kDS);
-  uint64_t* qdo_full = bars;       // 1
-  uint64_t* kv_full = bars + 1;    // 2
-  uint64_t* kv_empty = bars + 3;   // 2
-  uint64_t* s_full = bars + 5;     // 2
-  uint64_t* s_empty = bars + 7;    // 2
-  uint64_t* ds_full = bars + 9;    // 2
-  uint64_t* ds_empty = bars + 11;  // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-  const int warp = threadIdx.x >> 5;
-  const int qb = gridDim.x - 1 - blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int q0 = qb * 128;
-  int kv_len = p.Skv;
-  if (p.causal) kv_len = min(p.Skv, p.q_pos0 + q0 + 127 - p.k_pos0 + 1);
-  const int n_it = kv_len > 0 ? (kv_len + 63) / 64 : 0;
-
-  if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmDO);
-    mbar_init(qdo_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
-      mbar_init(&s_full[i], 1);
-      mbar_init(&s_empty[i], kBwdSoftmaxThreads);
-      mbar_init(&ds_full[i], kBwdSoftmaxThreads);
-      mbar_init(&ds_empty[i], 1);
-    }
-    *abort_flag = 0;
-    mbar_fence_init();
-  }
-  if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-  const uint32_t tS[2] = {tmem, tmem + 128};
-  const uint32_t tDP[2] = {tmem + 64, tmem + 192};
-  const uint32_t tDQ = tmem + 256;
-
-  const int qslot = p.qmap.slot(h, p.qpg), kslot = p.kmap.slot(h, p.qpg), vslot = p.vmap.slot(h, p.qpg),
-            doslot = p.domap.slot(h, p.qpg);
-
-  if (warp == 0) {
-    if (n_it > 0) {
-      // the whole warp walks the loop, one elected lane issues the copies (see producer_loop in gemm_core.cuh)
-      const bool issuer = elect_one() != 0;
-      if (issuer) mbar_expect_tx(qdo_full, 2 * DqSmem<HD>::kQ);
-#pragma unroll
-      for (int c = 0; c < HD / 64; ++c) {
-        if (issuer) tma_load_4d(sQ + c * 128 * 128, &tmQ, qdo_full, c * 64, qslot, q0, b);
-        if (issuer) tma_load_4d(sDO + c * 128 * 128, &tmDO, qdo_full, c * 64, doslot, q0, b);
-      }
-      for (int it = 0; it < n_it; ++it) {
-        const int st = it & 1;
-        if (!mbar_wait_warp(&kv_empty[st], ((it >> 1) & 1) ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { *abort_flag = 1; break; }
-        if (issuer) mbar_expect_tx(&kv_full[st], 2 * DqSmem<HD>::kKV);
-#pragma unroll
-        for (int c = 0; c < HD / 64; ++c) {
-          if (issuer) tma_load_4d(sK + st * DqSmem<HD>::kKV + c * 64 * 128, &tmK, &kv_full[st], c * 64, kslot, it * 64, b);
-          if (issuer) tma_load_4d(sV + st * DqSmem<HD>::kKV + c * 64 * 128, &tmV, &kv_full[st], c * 64, vslot, it * 64, b);
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (n_it > 0) {
-      // the whole warp walks the loop, one elected lane issues (see mma_loop in gemm_core.cuh)
-      const bool issuer = elect_one() != 0;
-      constexpr uint32_t idesc_s = make_idesc_lp(128, 64, false, false);
-      constexpr uint32_t idesc_dq = make_idesc_lp(128, HD, false, true);
-      const uint32_t aQ = smem_u32(sQ), aDO = smem_u32(sDO), aDS = smem_u32(sDS);
-      bool ok = mbar_wait_warp(qdo_full, 0, p.status, kTimeoutSmemFull, abort_flag);
-      auto issue_s = [&](int it) -> bool {
-        const int st = it & 1;
-        const uint32_t ph = (it >> 1) & 1;
-        if (!mbar_wait_warp(&kv_full[st], ph, p.status, kTimeoutSmemFull, abort_flag)) return false;
-        if (!mbar_wait_warp(&s_empty[st], ph ^ 1, p.status, kTimeoutTmemEmpty, abort_flag)) return false;
-        tc_fence_after();
-        const uint32_t aK = smem_u32(sK + st * DqSmem<HD>::kKV), aV = smem_u32(sV + st * DqSmem<HD>::kKV);
-        if (issuer) {
-#pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk)
-            umma_f16_ss(tS[st], kmajor_desc(aQ, 128, kk), kmajor_desc(aK, 64, kk), idesc_s, kk != 0);
-#pragma unroll
-          for (int kk = 0; kk < HD / 16; ++kk)
-            umma_f16_ss(tDP[st], kmajor_desc(aDO, 128, kk), kmajor_desc(aV, 64, kk), idesc_s, kk != 0);
-          umma_commit(&s_full[st]);
-        }
-        __syncwarp();
-        return true;
-      };
-      if (ok) ok = issue_s(0);
-      for (int it = 0; ok && it < n_it; ++it) {
-        if (it + 1 < n_it) { ok = issue_s(it + 1); if (!ok) break; }
-        const int st = it & 1;
-        if (!mbar_wait_warp(&ds_full[st], (it >> 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t aK = smem_u32(sK + st * DqSmem<HD>::kKV);
-        const uint32_t aDSs = aDS + st * DqSmem<HD>::kDS;
-        if (issuer) {
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_f16_ss(tDQ, kmajor_desc(aDSs, 128, kk), mnmajor_desc(aK, 64, kk), idesc_dq, (it | kk) != 0);
-          umma_commit(&kv_empty[st]);
-          umma_commit(&ds_empty[st]);
-        }
-        __syncwarp();
-      }
-      if (!ok) *abort_flag = 1;
-    }
-  } else {
-    const int wq = warp & 3;
-    const int half = (warp - 2) >> 2;     // which 32 of the step's 64 key columns this warpgroup owns
-    const int c0 = half * 32;
-    const int row = wq * 32 + lane_id();
-    const uint32_t lane_off = uint32_t(wq * 32) << 16;
-    const float sl2 = p.scale * kLog2e;
-    const int srow = q0 + row;
-    const int q_pos = p.q_pos0 + srow;
-    float lse2 = INFINITY, dsum = 0.f;
-    if (srow < p.Sq) {
-      const size_t idx = (size_t(b) * p.nheads + h) * p.Sq + srow;
-      lse2 = p.LSE[idx] * kLog2e;
-      dsum = p.D[idx];
-    }
-    const float nlse2 = -lse2;
-    bool ok = true;
-    for (int it = 0; it < n_it; ++it) {
-      const int st = it & 1;
-      if (!mbar_wait_warp(&s_full[st], (it >> 1) & 1, p.status, kTimeoutTmemFull, abort_flag)) { ok = false; break; }
-      tc_fence_after();
-      float ds[32];
-      {
-        float sv[32];
-        {
-          uint32_t r0[32], r1[32];
-          tmem_ld32(tS[st] + lane_off + c0, r0);
-          tmem_ld32(tDP[st] + lane_off + c0, r1);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) { sv[i] = __uint_as_float(r0[i]); ds[i] = __uint_as_float(r1[i]); }
-        }
-        tc_fence_before();
-        mbar_arrive(&s_empty[st]);
-        const int kbase = it * 64 + c0;
-        const bool need_mask = (p.causal && (p.k_pos0 + kbase + 31 > p.q_pos0 + q0)) || (kbase + 32 > p.Skv);
-        if (!need_mask) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) ds[i] = ex2(fmaf(sv[i], sl2, nlse2)) * (ds[i] - dsum);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const bool dead = (kbase + i >= p.Skv) || (p.causal && (p.k_pos0 + kbase + i > q_pos));
-            ds[i] = dead ? 0.f : ex2(fmaf(sv[i], sl2, nlse2)) * (ds[i] - dsum);
-          }
-        }
-      }
-      if (it >= 2) {   // this buffer was last read by the dQ product of step it-2
-        if (!mbar_wait_warp(&ds_empty[st], ((it >> 1) & 1) ^ 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
-      }
-      uint8_t* sDSs = sDS + st * DqSmem<HD>::kDS;
-#pragma unroll
-      for (int cc = 0; cc < 4; ++cc) {
-        uint4 w;
-        w.x = pack_bf16(ds[cc * 8 + 0], ds[cc * 8 + 1]); w.y = pack_bf16(ds[cc * 8 + 2], ds[cc * 8 + 3]);
-        w.z = pack_bf16(ds[cc * 8 + 4], ds[cc * 8 + 5]); w.w = pack_bf16(ds[cc * 8 + 6], ds[cc * 8 + 7]);
-        *reinterpret_cast<uint4*>(sDSs + sw128_offset(row, half * 4 + cc)) = w;
-      }
-      fence_proxy_async_smem();
-      tc_fence_before();
-      mbar_arrive(&ds_full[st]);
-    }
-    const int dqslot = p.dqmap.slot(h, p.qpg);
-    hg_lp_t* dq = p.dQ + int64_t(srow) * p.dq_ss + int64_t(b) * p.dq_sb + int64_t(dqslot) * HD;
-    if (n_it == 0) {
-      if (srow < p.Sq) {
-#pragma unroll
-        for (int i = half; i < HD / 8; i += 2) reinterpret_cast<uint4*>(dq)[i] = make_uint4(0, 0, 0, 0);
-      }
-    } else if (ok && !*abort_flag &&
-               mbar_wait_warp(&ds_empty[(n_it - 1) & 1], ((n_it - 1) >> 1) & 1, p.status, kTimeoutOther, abort_flag)) {
-      tc_fence_after();
-#pragma unroll
-      for (int c = half; c < HD / 32; c += 2) {   // the two warpgroups take alternate 32-column chunks
-        uint32_t r[32];
-        tmem_ld32(tDQ + lane_off + c * 32, r);
-        tmem_ld_wait();
-        if (srow < p.Sq) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            uint4 u;
-            u.x = pack_bf16(__uint_as_float(r[q * 8 + 0]) * p.scale, __uint_as_float(r[q * 8 + 1]) * p.scale);
-            u.y = pack_bf16(__uint_as_float(r[q * 8 + 2]) * p.scale, __uint_as_float(r[q * 8 + 3]) * p.scale);
-            u.z = pack_bf16(__uint_as_float(r[q * 8 + 4]) * p.scale, __uint_as_float(r[q * 8 + 5]) * p.scale);
-            u.w = pack_bf16(__uint_as_float(r[q * 8 + 6]) * p.scale, __uint_as_float(r[q * 8 + 7]) * p.scale);
-            reinterpret_cast<uint4*>(dq + c * 32)[q] = u;
-          }
-        }
-      }
-    } else {
-      *abort_flag = 1;
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem, 512);
-  }
-}
-
-
-// =================================================================================================
-// Backward, part 2 with 128-key steps (head dim 128).  A tcgen05.mma of shape 128 x N x 16 occupies the tensor core
+// Backward, part 2 with 128-key steps (both head dims; head dim 64, 8 x 1024 x 25 heads: 182 us with 64-key steps
+// staged through shared memory, 107 us).  A tcgen05.mma of shape 128 x N x 16 occupies the tensor core
 // for the same time whatever N <= 256 is, so the score products are issued with N = 128 instead of 64: per 128 keys
 // the kernel issues 24 MMAs (8 S, 8 dP, 8 dQ) where the 64-key version issues 40.  Shared memory holds three K
 // stages and one V stage of 128 rows (128 KB) and Q and dO (64 KB); tensor memory holds one S / dP pair (256 columns),
@@ -2106,16 +1882,64 @@ int make_map(CUtensorMap* out, const void* base, int hd, int slots, int S, int B
   return r == CUDA_SUCCESS ? 0 : -(1000 + int(r));
 }
 
-// dK/dV kernel for head dim 128: 0 = 128-query steps with P^T / dS^T in tensor memory, 1 = 64-query steps staged
-// through shared memory (kept for head dim 64 and for side-by-side timing).
+// dK/dV kernel: 0 = 128-query steps with P^T / dS^T in tensor memory, 1 = 64-query steps staged
+// through shared memory (kept for side-by-side tests and timing).
 int g_dkv_variant = 0;
-// Forward kernel for head dim 128: 0 = two query tiles per CTA with P in tensor memory (sequences longer than one
-// tile), 1 = one tile per CTA with P staged in shared memory (also what head dim 64 and single-tile calls use).
+// Forward kernel: 0 = two query tiles per CTA with P in tensor memory (sequences longer than one
+// tile; head dim 64, 8 x 1024 x 25 heads: 123 -> 93 us), 1 = one tile per CTA with P staged in shared memory (also
+// what single-tile calls use).
 int g_fwd_variant = 0;
 
 template <typename K>
 int set_smem(K kernel, int bytes) {
   return int(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+}
+
+// Sequences longer than one tile: two query tiles per CTA with P in tensor memory, both head dims.
+template <int HD>
+int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t st) {
+  int rc;
+  if (p.Sq > 128 && g_fwd_variant == 0) {
+    static bool cfg = false;
+    if (!cfg) { if ((rc = set_smem(flash_fwd2_kernel<HD>, Fwd2Smem<HD>::kTotal))) return rc; cfg = true; }
+    const dim3 grid((p.Sq + 255) / 256, p.nheads, p.B);
+    flash_fwd2_kernel<HD><<<grid, 320, Fwd2Smem<HD>::kTotal, st>>>(tq, tk, tv, p);
+  } else {
+    static bool cfg = false;
+    if (!cfg) { if ((rc = set_smem(flash_fwd_kernel<HD>, FwdSmem<HD>::kTotal))) return rc; cfg = true; }
+    const dim3 grid((p.Sq + 127) / 128, p.nheads, p.B);
+    flash_fwd_kernel<HD><<<grid, kThreads, FwdSmem<HD>::kTotal, st>>>(tq, tk, tv, p);
+  }
+  return int(cudaGetLastError());
+}
+
+template <int HD>
+int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+               const BwdParams& p, int Skv, int nkv, bool wide, cudaStream_t st) {
+  int rc;
+  const dim3 grid((Skv + 127) / 128, nkv, p.B);
+  if (wide) {
+    static bool cfg = false;
+    auto k = flash_bwd_dkv128_kernel<HD, kDkvWarpgroups>;
+    if (!cfg) { if ((rc = set_smem(k, Dkv128Smem<HD>::kTotal))) return rc; cfg = true; }
+    k<<<grid, 64 + 128 * kDkvWarpgroups, Dkv128Smem<HD>::kTotal, st>>>(tq, tk, tv, tdo, p);
+  } else {
+    static bool cfg = false;
+    if (!cfg) { if ((rc = set_smem(flash_bwd_dkv_kernel<HD>, DkvSmem<HD>::kTotal))) return rc; cfg = true; }
+    flash_bwd_dkv_kernel<HD><<<grid, kBwdThreads, DkvSmem<HD>::kTotal, st>>>(tq, tk, tv, tdo, p);
+  }
+  return int(cudaGetLastError());
+}
+
+template <int HD>
+int launch_dq(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+              const BwdParams& p, cudaStream_t st) {
+  int rc;
+  static bool cfg = false;
+  auto k = flash_bwd_dq128_kernel<HD, kDqWarpgroups>;
+  if (!cfg) { if ((rc = set_smem(k, Dq128Smem<HD>::kTotal))) return rc; cfg = true; }
+  k<<<dim3((p.Sq + 127) / 128, p.nheads, p.B), 64 + 128 * kDqWarpgroups, Dq128Smem<HD>::kTotal, st>>>(tq, tk, tv, tdo, p);
+  return int(cudaGetLastError());
 }
 
 }  // namespace
@@ -2148,33 +1972,18 @@ int hg_flash_fwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTenso
   p.O = reinterpret_cast<hg_lp_t*>(o->ptr); p.o_ss = o->ss; p.o_sb = o->sb;
   p.LSE = reinterpret_cast<float*>(lse);
   p.status = hg_host::status_ptr();
-  dim3 grid((Sq + 127) / 128, nheads, B);
   cudaStream_t st = (cudaStream_t)stream;
-  if (hd == 128 && Sq > 128 && g_fwd_variant == 0) {   // two query tiles per CTA, P in tensor memory
-    static bool cfg = false;
-    if (!cfg) { if ((rc = set_smem(flash_fwd2_kernel<128>, Fwd2Smem<128>::kTotal))) return rc; cfg = true; }
-    dim3 grid2((Sq + 255) / 256, nheads, B);
-    flash_fwd2_kernel<128><<<grid2, 320, Fwd2Smem<128>::kTotal, st>>>(tq, tk, tv, p);
-  } else if (hd == 128) {
-    static bool cfg = false;
-    if (!cfg) { if ((rc = set_smem(flash_fwd_kernel<128>, FwdSmem<128>::kTotal))) return rc; cfg = true; }
-    flash_fwd_kernel<128><<<grid, kThreads, FwdSmem<128>::kTotal, st>>>(tq, tk, tv, p);
-  } else {
-    static bool cfg = false;
-    if (!cfg) { if ((rc = set_smem(flash_fwd_kernel<64>, FwdSmem<64>::kTotal))) return rc; cfg = true; }
-    flash_fwd_kernel<64><<<grid, kThreads, FwdSmem<64>::kTotal, st>>>(tq, tk, tv, p);
-  }
-  return int(cudaGetLastError());
+  return hd == 128 ? launch_fwd<128>(tq, tk, tv, p, st) : launch_fwd<64>(tq, tk, tv, p, st);
 }
 
-// Selects the forward kernel used for head dim 128 (see g_fwd_variant); returns the previous value.
+// Selects the forward kernel (see g_fwd_variant); returns the previous value.
 int hg_attn_set_fwd_variant(int v) {
   const int old = g_fwd_variant;
   g_fwd_variant = v ? 1 : 0;
   return old;
 }
 
-// Selects the dK/dV kernel used for head dim 128 (see g_dkv_variant); returns the previous value.
+// Selects the dK/dV kernel (see g_dkv_variant); returns the previous value.
 int hg_attn_set_dkv_variant(int v) {
   const int old = g_dkv_variant;
   g_dkv_variant = v ? 1 : 0;
@@ -2212,46 +2021,21 @@ int hg_flash_bwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTenso
   p.status = hg_host::status_ptr();
   {
     CUtensorMap tq, tk, tv, tdo;
-    const bool wide = (hd == 128) && g_dkv_variant == 0;   // 128-query steps, P^T / dS^T in tensor memory
+    const bool wide = g_dkv_variant == 0;   // 128-query steps, P^T / dS^T in tensor memory
     const int q_rows = wide ? 128 : 64;
     if ((rc = make_map(&tq, q->ptr, hd, q->slots, Sq, B, q->ss, q->sb, q_rows))) return rc;
     if ((rc = make_map(&tk, k->ptr, hd, k->slots, Skv, B, k->ss, k->sb, 128))) return rc;
     if ((rc = make_map(&tv, v->ptr, hd, v->slots, Skv, B, v->ss, v->sb, 128))) return rc;
     if ((rc = make_map(&tdo, d_o->ptr, hd, d_o->slots, Sq, B, d_o->ss, d_o->sb, q_rows))) return rc;
-    dim3 grid((Skv + 127) / 128, nkv, B);
-    if (wide) {
-      static bool cfg = false;
-      if (!cfg) { if ((rc = set_smem(flash_bwd_dkv128_kernel<128, kDkvWarpgroups>, Dkv128Smem<128>::kTotal))) return rc; cfg = true; }
-      flash_bwd_dkv128_kernel<128, kDkvWarpgroups><<<grid, 64 + 128 * kDkvWarpgroups, Dkv128Smem<128>::kTotal, st>>>(tq, tk, tv, tdo, p);
-    } else if (hd == 128) {
-      static bool cfg = false;
-      if (!cfg) { if ((rc = set_smem(flash_bwd_dkv_kernel<128>, DkvSmem<128>::kTotal))) return rc; cfg = true; }
-      flash_bwd_dkv_kernel<128><<<grid, kBwdThreads, DkvSmem<128>::kTotal, st>>>(tq, tk, tv, tdo, p);
-    } else {
-      static bool cfg = false;
-      if (!cfg) { if ((rc = set_smem(flash_bwd_dkv_kernel<64>, DkvSmem<64>::kTotal))) return rc; cfg = true; }
-      flash_bwd_dkv_kernel<64><<<grid, kBwdThreads, DkvSmem<64>::kTotal, st>>>(tq, tk, tv, tdo, p);
-    }
+    if ((rc = hd == 128 ? launch_dkv<128>(tq, tk, tv, tdo, p, Skv, nkv, wide, st)
+                        : launch_dkv<64>(tq, tk, tv, tdo, p, Skv, nkv, wide, st))) return rc;
   }
-  {
-    CUtensorMap tq, tk, tv, tdo;
-    const int kv_rows = (hd == 128) ? 128 : 64;   // keys per step of the dQ kernel
-    if ((rc = make_map(&tq, q->ptr, hd, q->slots, Sq, B, q->ss, q->sb, 128))) return rc;
-    if ((rc = make_map(&tk, k->ptr, hd, k->slots, Skv, B, k->ss, k->sb, kv_rows))) return rc;
-    if ((rc = make_map(&tv, v->ptr, hd, v->slots, Skv, B, v->ss, v->sb, kv_rows))) return rc;
-    if ((rc = make_map(&tdo, d_o->ptr, hd, d_o->slots, Sq, B, d_o->ss, d_o->sb, 128))) return rc;
-    dim3 grid((Sq + 127) / 128, nheads, B);
-    if (hd == 128) {
-      static bool cfg = false;
-      if (!cfg) { if ((rc = set_smem(flash_bwd_dq128_kernel<128, kDqWarpgroups>, Dq128Smem<128>::kTotal))) return rc; cfg = true; }
-      flash_bwd_dq128_kernel<128, kDqWarpgroups><<<grid, 64 + 128 * kDqWarpgroups, Dq128Smem<128>::kTotal, st>>>(tq, tk, tv, tdo, p);
-    } else {
-      static bool cfg = false;
-      if (!cfg) { if ((rc = set_smem(flash_bwd_dq_kernel<64>, DqSmem<64>::kTotal))) return rc; cfg = true; }
-      flash_bwd_dq_kernel<64><<<grid, kBwdThreads, DqSmem<64>::kTotal, st>>>(tq, tk, tv, tdo, p);
-    }
-  }
-  return int(cudaGetLastError());
+  CUtensorMap tq, tk, tv, tdo;
+  if ((rc = make_map(&tq, q->ptr, hd, q->slots, Sq, B, q->ss, q->sb, 128))) return rc;
+  if ((rc = make_map(&tk, k->ptr, hd, k->slots, Skv, B, k->ss, k->sb, 128))) return rc;
+  if ((rc = make_map(&tv, v->ptr, hd, v->slots, Skv, B, v->ss, v->sb, 128))) return rc;
+  if ((rc = make_map(&tdo, d_o->ptr, hd, d_o->slots, Sq, B, d_o->ss, d_o->sb, 128))) return rc;
+  return hd == 128 ? launch_dq<128>(tq, tk, tv, tdo, p, st) : launch_dq<64>(tq, tk, tv, tdo, p, st);
 }
 
 }  // extern "C"
