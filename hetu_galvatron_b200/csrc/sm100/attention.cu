@@ -90,7 +90,7 @@ constexpr int kDqWarpgroups = HG_DQ_WARPGROUPS;
   } while (0)
 #define HG_DKV_REPORT(off, n, a, b, c, d)                                                                   \
   do {                                                                                                      \
-    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && lane_id() == 0 && (warp == 1 || warp == 2)) { \
+    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && lane_id() == 0 && (warp == 1 || warp == 2 || warp == 4)) { \
       p.status[16 + off] = n;                                                                               \
       p.status[17 + off] = int(a);                                                                          \
       p.status[18 + off] = int(b);                                                                          \
@@ -433,8 +433,19 @@ struct Fwd2Smem {
   static constexpr int kTotal = 2 * kQ + 4 * kKV + 1024 + 256;
 };
 
+// Registers.  A softmax thread holds its 128 scores and a half row of packed probabilities, more than the 168 registers
+// an even share of twelve warps leaves; the warpgroup of the TMA and MMA warps (warps 0-3, two of them idle) gives most
+// of its share away.  setmaxnreg moves registers inside what the block was launched with: 384 threads x 168 = 64512
+// (as ptxas reports for this kernel) >= 128 x 56 + 256 x 216 = 62464.
+constexpr int kFwd2Threads = 384;
+constexpr int kFwd2AuxRegs = 56, kFwd2SoftmaxRegs = 216;
+template <int N>
+__device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N>
+__device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+
 template <int HD>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(kFwd2Threads, 1)
 flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                   const __grid_constant__ CUtensorMap tmV, const FwdParams p) {
   static_assert(HD == 64 || HD == 128, "tensor memory holds two S tiles and two O tiles of up to 128 columns");
@@ -451,9 +462,9 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   uint64_t* v_full = bars + 5;      // 2
   uint64_t* v_empty = bars + 7;     // 2
   uint64_t* s_full = bars + 9;      // 2 (per tile)
-  uint64_t* p_full = bars + 11;     // 2 (per tile)
-  uint64_t* o_done = bars + 13;     // 2 (per tile)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* p_full = bars + 11;     // 4 (per tile and half of the key block)
+  uint64_t* o_done = bars + 15;     // 2 (per tile)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -482,7 +493,8 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       mbar_init(&v_full[i], 1);
       mbar_init(&v_empty[i], 1);
       mbar_init(&s_full[i], 1);
-      mbar_init(&p_full[i], 4);      // one arrival per softmax warp of the tile (mbar_arrive_warp)
+      mbar_init(&p_full[2 * i], 4);  // one arrival per softmax warp of the tile (mbar_arrive_warp)
+      mbar_init(&p_full[2 * i + 1], 4);
       mbar_init(&o_done[i], 1);
     }
     *abort_flag = 0;
@@ -501,6 +513,8 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 
   const int qslot = p.qmap.slot(h, p.qpg), kslot = p.kmap.slot(h, p.qpg), vslot = p.vmap.slot(h, p.qpg);
 
+  if (warp < 4) {
+  regs_dec<kFwd2AuxRegs>();
   if (warp == 0) {
     if (n_kv > 0) {
       // the whole warp walks the loop, one elected lane issues the copies (see producer_loop in gemm_core.cuh)
@@ -560,15 +574,23 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (!ok || j >= n_kv_t[t]) continue;
-          if (!mbar_wait_warp(&p_full[t], j & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&p_full[2 * t], j & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
           if (t == 0) { HG_DKV_TOCK(tm_wait_p0, t0); } else { HG_DKV_TOCK(tm_wait_p1, t0); }
           if (!mbar_wait_warp(&v_full[st], (j >> 1) & 1, p.status, kTimeoutSmemFull, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t aV = smem_u32(sV + st * L::kKV);
           if (issuer) {
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk)   // k-step kk = keys 16kk..16kk+15 = 8 packed columns of P
+            for (int kk = 0; kk < 4; ++kk)   // k-step kk = keys 16kk..16kk+15 = 8 packed columns of P
               umma_f16_ts(tO[t], tS[t] + kk * 8, mnmajor_desc(aV, 128, kk), idesc_o, (j | kk) != 0);
+          }
+          __syncwarp();
+          if (!mbar_wait_warp(&p_full[2 * t + 1], j & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          if (issuer) {
+#pragma unroll
+            for (int kk = 4; kk < 8; ++kk)
+              umma_f16_ts(tO[t], tS[t] + kk * 8, mnmajor_desc(aV, 128, kk), idesc_o, true);
             if (t == last_user(j)) umma_commit(&v_empty[st]);
             if (j + 1 >= n_kv_t[t]) umma_commit(&o_done[t]);
           }
@@ -580,9 +602,11 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       HG_DKV_REPORT(8, n_kv, tm_wait_p0, tm_wait_p1, tm_issue, tm_unused);
       if (!ok) *abort_flag = 1;
     }
+  }
   } else {
+    regs_inc<kFwd2SoftmaxRegs>();
     // ---- softmax: one warpgroup per tile, thread == query row ----
-    const int t = (warp - 2) >> 2;
+    const int t = (warp - 4) >> 2;
     const int wq = warp & 3;
     const int row = wq * 32 + lane_id();
     const uint32_t lane_off = uint32_t(wq * 32) << 16;
@@ -637,22 +661,6 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         rescale = (j > 0);
       }
       const float nmref = (m_used == -INFINITY) ? 0.f : -m_used;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
-      uint32_t pk[64];
-#pragma unroll
-      for (int i = 0; i < 128; i += 4) {
-        float e[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float x = fmaf(s[i + u], sl2, nmref);
-          e[u] = (u < HG_FWD_POLY_OF_4) ? ex2_poly(x) : ex2(x);
-          sum4[u] += e[u];
-        }
-        pk[i >> 1] = pack_bf16(e[0], e[1]);
-        pk[(i >> 1) + 1] = pack_bf16(e[2], e[3]);
-      }
-      l = l * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-      HG_DKV_TOCK(tm_math, t0);
       // S(t, j) was issued after PV(t, j-1), and the tensor core executes in order: O holds steps 0..j-1 by now
       if (__any_sync(0xffffffffu, rescale)) {
 #pragma unroll
@@ -665,16 +673,31 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           tmem_st32(tO[t] + lane_off + c * 32, r);
         }
       }
-      // P, packed, over the first 64 of this row's S columns
-      {
-        const uint32_t(&lo)[32] = *reinterpret_cast<const uint32_t(*)[32]>(&pk[0]);
-        const uint32_t(&hi)[32] = *reinterpret_cast<const uint32_t(*)[32]>(&pk[32]);
-        tmem_st32(tS[t] + lane_off, lo);
-        tmem_st32(tS[t] + lane_off + 32, hi);
+      // P, packed, over the first 64 of this row's S columns, in two halves: the PV product of keys 0..63 runs while
+      // the exponentials of keys 64..127 are taken
+      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int hh = 0; hh < 2; ++hh) {
+        uint32_t pk[32];
+#pragma unroll
+        for (int i = 0; i < 64; i += 4) {
+          float e[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float x = fmaf(s[hh * 64 + i + u], sl2, nmref);
+            e[u] = (u < HG_FWD_POLY_OF_4) ? ex2_poly(x) : ex2(x);
+            sum4[u] += e[u];
+          }
+          pk[i >> 1] = pack_bf16(e[0], e[1]);
+          pk[(i >> 1) + 1] = pack_bf16(e[2], e[3]);
+        }
+        tmem_st32(tS[t] + lane_off + hh * 32, pk);
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive_warp(&p_full[2 * t + hh]);
+        if (hh == 0) { HG_DKV_TOCK(tm_math, t0); }
       }
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive_warp(&p_full[t]);
+      l = l * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
       HG_DKV_TOCK(tm_st, t0);
     }
     if (t == 0) { HG_DKV_REPORT(0, my_kv, tm_wait_s, tm_ld, tm_math, tm_st); }
@@ -1903,7 +1926,7 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(flash_fwd2_kernel<HD>, Fwd2Smem<HD>::kTotal))) return rc; cfg = true; }
     const dim3 grid((p.Sq + 255) / 256, p.nheads, p.B);
-    flash_fwd2_kernel<HD><<<grid, 320, Fwd2Smem<HD>::kTotal, st>>>(tq, tk, tv, p);
+    flash_fwd2_kernel<HD><<<grid, kFwd2Threads, Fwd2Smem<HD>::kTotal, st>>>(tq, tk, tv, p);
   } else {
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(flash_fwd_kernel<HD>, FwdSmem<HD>::kTotal))) return rc; cfg = true; }
