@@ -54,13 +54,13 @@ struct RowColWalk {
 
 // ---------------------------------------------------------------------------------------------
 // RoPE, rotate-half (non-interleaved) form, applied in place to `nheads` heads that sit at
-// column offsets head_off[h] (elements) of every token row of a [tokens, row_pitch] buffer.
+// column offsets slot[h] * slot_width (elements) of every token row of a [tokens, row_pitch] buffer.
 //   out[i]        = x[i]*cos[i] - x[i+half]*sin[i]
 //   out[i+half]   = x[i+half]*cos[i] + x[i]*sin[i]       (sign of sin flipped for the backward)
 // Token t has position pos[t] when `pos` is given, else (t / batch) + pos_offset ([S,B] order).
 // cos/sin tables are fp32 [max_pos, half].
 // ---------------------------------------------------------------------------------------------
-__global__ void rope_kernel(hg_lp_t* __restrict__ buf, const int* __restrict__ head_off, int nheads,
+__global__ void rope_kernel(hg_lp_t* __restrict__ buf, const int* __restrict__ slot, int slot_width, int nheads,
                             int row_pitch, int tokens, int batch, const int* __restrict__ pos, int pos_offset,
                             const float* __restrict__ cos_t, const float* __restrict__ sin_t, int half, float sign) {
   const int vec_per_head = half >> 3;  // uint4 chunks in one half
@@ -69,7 +69,7 @@ __global__ void rope_kernel(hg_lp_t* __restrict__ buf, const int* __restrict__ h
     const int t = int(w.row);
     const int h = w.col / vec_per_head, c = w.col - h * vec_per_head;
     const int p = pos ? pos[t] : (t / batch + pos_offset);
-    hg_lp_t* base = buf + size_t(t) * row_pitch + head_off[h] + c * 8;
+    hg_lp_t* base = buf + size_t(t) * row_pitch + slot[h] * slot_width + c * 8;
     float a[8], b[8], cs[8], sn[8];
     unpack8(*reinterpret_cast<const uint4*>(base), a);
     unpack8(*reinterpret_cast<const uint4*>(base + half), b);
@@ -95,7 +95,7 @@ __global__ void rope_kernel(hg_lp_t* __restrict__ buf, const int* __restrict__ h
 //   out[2i]   = x[2i]*cos[i] - x[2i+1]*sin[i]
 //   out[2i+1] = x[2i+1]*cos[i] + x[2i]*sin[i]
 // One thread takes 8 consecutive channels (4 pairs) of one head of one token.
-__global__ void rope_interleaved_kernel(hg_lp_t* __restrict__ buf, const int* __restrict__ head_off, int nheads,
+__global__ void rope_interleaved_kernel(hg_lp_t* __restrict__ buf, const int* __restrict__ slot, int slot_width, int nheads,
                                         int row_pitch, int tokens, int batch, const int* __restrict__ pos,
                                         int pos_offset, const float* __restrict__ cos_t,
                                         const float* __restrict__ sin_t, int half, float sign) {
@@ -105,7 +105,7 @@ __global__ void rope_interleaved_kernel(hg_lp_t* __restrict__ buf, const int* __
     const int t = int(w.row);
     const int h = w.col / vec_per_head, c = w.col - h * vec_per_head;
     const int p = pos ? pos[t] : (t / batch + pos_offset);
-    hg_lp_t* base = buf + size_t(t) * row_pitch + head_off[h] + c * 8;
+    hg_lp_t* base = buf + size_t(t) * row_pitch + slot[h] * slot_width + c * 8;
     float x[8], o[8];
     unpack8(*reinterpret_cast<const uint4*>(base), x);
     const float4 cs = *reinterpret_cast<const float4*>(cos_t + size_t(p) * half + c * 4);
@@ -388,7 +388,7 @@ inline int grid_for(int64_t work, int threads) {
 
 extern "C" {
 
-int hg_rope(void* buf, const void* head_off, int nheads, int row_pitch, int tokens, int batch, const void* pos,
+int hg_rope(void* buf, const void* slots, int slot_width, int nheads, int row_pitch, int tokens, int batch, const void* pos,
             int pos_offset, const void* cos_t, const void* sin_t, int rot_dim, int flags, void* stream) {
   // flags: bit 0 = backward (rotate by the negative angle), bit 1 = interleaved channel pairs
   if (tokens <= 0 || nheads <= 0) return 0;
@@ -398,12 +398,12 @@ int hg_rope(void* buf, const void* head_off, int nheads, int row_pitch, int toke
   if (flags & 2) {
     const int64_t work = int64_t(tokens) * nheads * (half >> 2);
     rope_interleaved_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
-        (hg_lp_t*)buf, (const int*)head_off, nheads, row_pitch, tokens, batch, (const int*)pos, pos_offset,
+        (hg_lp_t*)buf, (const int*)slots, slot_width, nheads, row_pitch, tokens, batch, (const int*)pos, pos_offset,
         (const float*)cos_t, (const float*)sin_t, half, sign);
   } else {
     const int64_t work = int64_t(tokens) * nheads * (half >> 3);
     rope_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
-        (hg_lp_t*)buf, (const int*)head_off, nheads, row_pitch, tokens, batch, (const int*)pos, pos_offset,
+        (hg_lp_t*)buf, (const int*)slots, slot_width, nheads, row_pitch, tokens, batch, (const int*)pos, pos_offset,
         (const float*)cos_t, (const float*)sin_t, half, sign);
   }
   return int(cudaGetLastError());

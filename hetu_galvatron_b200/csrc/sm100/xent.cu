@@ -23,7 +23,7 @@ __device__ __forceinline__ void unpack8(const uint4& u, float* f) {
 __global__ void __launch_bounds__(kThreads)
 xent_stats_kernel(const hg_lp_t* __restrict__ logits, int64_t pitch, const int64_t* __restrict__ targets,
                   int v0, int V, float* __restrict__ out_max, float* __restrict__ out_sum,
-                  float* __restrict__ out_pred, int rows) {
+                  float* __restrict__ out_pred, float* __restrict__ out_loss, int rows) {
   __shared__ float sm[kThreads / 32], ss[kThreads / 32];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const hg_lp_t* x = logits + size_t(row) * pitch;
@@ -66,7 +66,9 @@ xent_stats_kernel(const hg_lp_t* __restrict__ logits, int64_t pitch, const int64
       out_max[row] = M;
       out_sum[row] = S;
       const int64_t t = targets[row] - v0;
-      out_pred[row] = (t >= 0 && t < V) ? hg_lp2f(x[t]) : 0.f;
+      const float pred = (t >= 0 && t < V) ? hg_lp2f(x[t]) : 0.f;
+      out_pred[row] = pred;
+      if (out_loss) out_loss[row] = logf(S) + M - pred;   // the whole vocabulary is here: three launches less
     }
   }
 }
@@ -109,14 +111,15 @@ xent_bwd_kernel(hg_lp_t* __restrict__ logits, int64_t pitch, const int64_t* __re
 
 extern "C" {
 
+// out_loss (optional): the per-row loss, for a vocabulary that is not split over ranks.
 int hg_xent_stats(const void* logits, long long pitch, const void* targets, int v0, int V, void* out_max,
-                  void* out_sum, void* out_pred, int rows, void* stream) {
+                  void* out_sum, void* out_pred, void* out_loss, int rows, void* stream) {
   if (rows <= 0) return 0;
   if (pitch & 7) return -1;
   const int grid = rows < 148 * 8 ? rows : 148 * 8;
   xent_stats_kernel<<<grid, kThreads, 0, (cudaStream_t)stream>>>((const hg_lp_t*)logits, pitch,
                                                                  (const int64_t*)targets, v0, V, (float*)out_max,
-                                                                 (float*)out_sum, (float*)out_pred, rows);
+                                                                 (float*)out_sum, (float*)out_pred, (float*)out_loss, rows);
   return int(cudaGetLastError());
 }
 

@@ -195,10 +195,15 @@ class SelfAttention(nn.Module):
         s, c = self.spec, self.ctx
         from ..parallel.tp_layers import column_parallel_linear, row_parallel_linear
 
-        qkv = column_parallel_linear(x, self.linear_qkv.weight, self.linear_qkv.bias, c)  # [S_att, B, P]
-        S_att, B = qkv.shape[0], qkv.shape[1]
+        if c.tp_size == 1:
+            # the projection of a matrix is not a view, so the in-place rotation below needs no copies in the backward
+            S_att, B = x.shape[0], x.shape[1]
+            qkv = qkv2 = column_parallel_linear(x.reshape(S_att * B, -1), self.linear_qkv.weight, self.linear_qkv.bias, c)
+        else:
+            qkv = column_parallel_linear(x, self.linear_qkv.weight, self.linear_qkv.bias, c)  # [S_att, B, P]
+            S_att, B = qkv.shape[0], qkv.shape[1]
+            qkv2 = qkv.reshape(S_att * B, -1)
         S_full = c.seq_len or S_att * c.cp_size * c.sp_size
-        qkv2 = qkv.reshape(S_att * B, -1)
         if self.q_layernorm is not None:
             if s.test_mode:
                 self.run_realtime_tests()

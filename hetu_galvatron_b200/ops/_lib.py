@@ -94,7 +94,7 @@ _SIGNATURES = {
                                         c_void_p],
     "hg_add_inplace_f32": [c_void_p, c_void_p, c_ll, c_void_p],
     "hg_zero_adamw_allgather": [c_void_p] * 5 + [c_int, c_ll, c_ll] + [ctypes.c_float] * 5 + [c_int, c_void_p, c_void_p, c_void_p],
-    "hg_rope": [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,
+    "hg_rope": [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int,
                 c_void_p],
     "hg_glu_fwd": [c_void_p, c_void_p, c_ll, c_int, c_int, c_void_p],
     "hg_glu_bwd": [c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_void_p],
@@ -105,7 +105,7 @@ _SIGNATURES = {
     "hg_attn_set_dkv_variant": [c_int],
     "hg_attn_set_fwd_variant": [c_int],
     "hg_attn_merge": [c_void_p, c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
-    "hg_xent_stats": [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
+    "hg_xent_stats": [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
     "hg_xent_bwd": [c_void_p, c_ll, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p],
     "hg_adamw": [c_void_p] * 5 + [c_ll, c_int, c_float, c_float, c_float, c_float, c_float, c_int, c_void_p,
                                   c_void_p, c_void_p],

@@ -160,27 +160,27 @@ class _RopeInplace(torch.autograd.Function):
     """Rotates the listed head slots of a ``[tokens, slots*hd]`` buffer in place."""
 
     @staticmethod
-    def forward(ctx, buf, head_off, cos, sin, batch, pos, pos_offset, rot_dim, interleaved=False):
-        ctx.args = (head_off, cos, sin, batch, pos, pos_offset, rot_dim, interleaved)
-        _rope_launch(buf, head_off, cos, sin, batch, pos, pos_offset, rot_dim, False, interleaved)
+    def forward(ctx, buf, slots, width, cos, sin, batch, pos, pos_offset, rot_dim, interleaved=False):
+        ctx.args = (slots, width, cos, sin, batch, pos, pos_offset, rot_dim, interleaved)
+        _rope_launch(buf, slots, width, cos, sin, batch, pos, pos_offset, rot_dim, False, interleaved)
         ctx.mark_dirty(buf)
         return buf
 
     @staticmethod
     def backward(ctx, g):
-        head_off, cos, sin, batch, pos, pos_offset, rot_dim, interleaved = ctx.args
+        slots, width, cos, sin, batch, pos, pos_offset, rot_dim, interleaved = ctx.args
         # the incoming gradient buffer is produced by the attention backward for this op alone, so it is
         # rotated back in place
         if not g.is_contiguous():
             g = g.contiguous()
-        _rope_launch(g, head_off, cos, sin, batch, pos, pos_offset, rot_dim, True, interleaved)
-        return g, None, None, None, None, None, None, None, None
+        _rope_launch(g, slots, width, cos, sin, batch, pos, pos_offset, rot_dim, True, interleaved)
+        return g, None, None, None, None, None, None, None, None, None
 
 
-def _rope_launch(buf, head_off, cos, sin, batch, pos, pos_offset, rot_dim, backward, interleaved=False):
+def _rope_launch(buf, slots, width, cos, sin, batch, pos, pos_offset, rot_dim, backward, interleaved=False):
     lib = _lib.load()
     tokens, pitch = buf.shape
-    rc = lib.hg_rope(buf.data_ptr(), head_off.data_ptr(), head_off.numel(), pitch, tokens, batch, _lib.ptr(pos),
+    rc = lib.hg_rope(buf.data_ptr(), slots.data_ptr(), width, slots.numel(), pitch, tokens, batch, _lib.ptr(pos),
                      pos_offset, cos.data_ptr(), sin.data_ptr(), rot_dim, int(backward) | (2 if interleaved else 0), _lib.stream())
     _lib.check(rc, "hg_rope")
     _lib.count_launch()
@@ -204,10 +204,10 @@ def rope_packed(qkv: torch.Tensor, head_slots: torch.Tensor, hd: int, cos: torch
         idx = head_slots.long()
         out[:, idx] = _rope_ref(t3[:, idx], cos, sin, p, interleaved=interleaved)
         return out.view_as(qkv)
-    head_off = (head_slots.to(torch.int32) * hd).contiguous()
+    head_slots = head_slots.to(torch.int32).contiguous()
     if pos is not None:
         pos = pos.to(torch.int32).contiguous()
-    return _RopeInplace.apply(qkv, head_off, cos, sin, batch, pos, pos_offset, rot_dim, interleaved)
+    return _RopeInplace.apply(qkv, head_slots, hd, cos, sin, batch, pos, pos_offset, rot_dim, interleaved)
 
 
 def mrope_angles(position_ids: torch.Tensor, mrope_section, rot_dim: int, base: float = 10000.0,
@@ -366,9 +366,11 @@ class _CrossEntropy(torch.autograd.Function):
         rows, V = logits.shape
         dev = logits.device
         stats = torch.empty((3, rows), dtype=torch.float32, device=dev)
+        # the kernel writes the loss itself when the vocabulary is not split
+        loss = torch.empty(rows, dtype=torch.float32, device=dev) if group is None else None
         _lib.check(lib.hg_xent_stats(logits.data_ptr(), logits.stride(0), targets.data_ptr(), v0, V,
-                                     stats[0].data_ptr(), stats[1].data_ptr(), stats[2].data_ptr(), rows,
-                                     _lib.stream()), "hg_xent_stats")
+                                     stats[0].data_ptr(), stats[1].data_ptr(), stats[2].data_ptr(),
+                                     _lib.ptr(loss), rows, _lib.stream()), "hg_xent_stats")
         _lib.count_launch()
         lmax, lsum, pred = stats[0], stats[1], stats[2]
         if group is not None:
@@ -377,9 +379,9 @@ class _CrossEntropy(torch.autograd.Function):
             packed = torch.stack([lsum * torch.exp(lmax - gmax), pred])
             dist.all_reduce(packed, group=group)
             gsum, pred = packed[0], packed[1]
+            loss = torch.log(gsum) + gmax - pred
         else:
             gmax, gsum = lmax, lsum
-        loss = torch.log(gsum) + gmax - pred
         ctx.save_for_backward(logits, targets, gmax, gsum)
         ctx.v0 = v0
         return loss

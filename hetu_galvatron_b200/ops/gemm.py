@@ -178,7 +178,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -
         return torch.nn.functional.linear(x, w, bias)
     shp = x.shape
     y = _Linear.apply(x.reshape(-1, shp[-1]), w, bias)
-    return y.view(*shp[:-1], w.shape[0])
+    return y if len(shp) == 2 else y.view(*shp[:-1], w.shape[0])
 
 
 def grouped_gemm(a: torch.Tensor, b: torch.Tensor, row_start: torch.Tensor, *, b_mn: bool = False,
