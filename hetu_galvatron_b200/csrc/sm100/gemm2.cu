@@ -64,7 +64,8 @@ __device__ __forceinline__ void pair_teardown(uint32_t tmem_base, int warp) {
 
 template <bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(192, 1)
-gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Params p) {
+gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                  const __grid_constant__ CUtensorMap tmC, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   Smem2 s = carve2(smem_raw);
   const int warp = threadIdx.x >> 5;
@@ -79,7 +80,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   } else if (warp == 1) {
     if (rank == 0) mma2<A_MN, B_MN>(p, s, tmem_base, pair, pairs, num_tiles);
   } else {
-    epilogue2(p, s, tmem_base, rank, pair, pairs, num_tiles);
+    epilogue2(p, &tmC, s, tmem_base, rank, pair, pairs, num_tiles);
   }
 
   pair_teardown(tmem_base, warp);
@@ -92,7 +93,8 @@ struct GroupedTile {
   int m, m_end, n;        // first row and column of the output tile; rows from m_end on are another group's
   int a_k, b_off;         // offsets into the stacked operands (see the loads below)
   int num_kb;
-  long long c_off;
+  int c_row;              // row of the tensor map of C at which this group's rows start
+  long long c_off;        // elements of C before this group
 };
 
 // C[r0:r1] = A[r0:r1] op(B_g) for the row segments [r0, r1) = row_start[g..g+1].  Inside a segment up to eight row tiles
@@ -115,7 +117,7 @@ struct RowSegments {
       for (int t = (pair - counter % pairs + pairs) % pairs; t < cnt; t += pairs) {
         const int first = t / (kGroupM * tiles_n) * kGroupM, gsize = min(kGroupM, tm_cnt - first);
         const int r = t - first * tiles_n;
-        GroupedTile w{r0 + (first + r % gsize) * CM, r1, r / gsize * BN, 0, g * b_group_rows, num_kb, 0};
+        GroupedTile w{r0 + (first + r % gsize) * CM, r1, r / gsize * BN, 0, g * b_group_rows, num_kb, 0, 0};
         if (!fn(w)) return;
       }
       counter += cnt;
@@ -138,7 +140,7 @@ struct ContractionRanges {
       const int r = u - first * tiles_n;
       const int k0 = k_start[g];
       GroupedTile w{(first + r % gsize) * CM, M, r / gsize * BN, k0, k0, (k_start[g + 1] - k0 + BK - 1) / BK,
-                    g * c_group_stride};
+                    g * M, g * c_group_stride};
       if (!fn(w)) return;
     }
   }
@@ -146,8 +148,8 @@ struct ContractionRanges {
 
 template <bool A_MN, bool B_MN, typename Tiles>
 __global__ void __launch_bounds__(192, 1)
-grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const Params p,
-                     const Tiles tiles) {
+grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                     const __grid_constant__ CUtensorMap tmC, const Params p, const Tiles tiles) {
   extern __shared__ uint8_t smem_raw[];
   Smem2 s = carve2(smem_raw);
   const int warp = threadIdx.x >> 5;
@@ -230,7 +232,7 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   } else {
     const int wq = warp & 3, lane = int(lane_id());
     const uint32_t lane_off = uint32_t(wq * 32) << 16;
-    float* stg = s.epi_stage + wq * EPI_STAGE_FLOATS;
+    StoreStage st{smem_u32(s.epi_stage + wq * EPI_STAGE_FLOATS), 0};
     uint32_t acc = 0, acc_phase = 0;
     tiles.walk(pair, pairs, [&](const GroupedTile& w) {
       const int row0 = w.m + int(rank) * BM + wq * 32;
@@ -238,32 +240,30 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       q.M = w.m_end;
       q.C = p.out_mode == kOutF32 || p.out_mode == kOutF32Acc ? static_cast<void*>(reinterpret_cast<float*>(p.C) + w.c_off)
                                                               : static_cast<void*>(reinterpret_cast<hg_lp_t*>(p.C) + w.c_off);
-      const bool empty = w.num_kb <= 0;
-      if (!empty) {
-        if (!mbar_wait_warp(&s.tmem_full[acc], acc_phase, p.status, kTimeoutTmemFull, s.abort)) { *s.abort = 1; return false; }
-        tc_fence_after();
-      }
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        if (row0 >= w.m_end || w.n + c * 32 >= p.N) break;   // warp-uniform
-        uint32_t r0[32];
-        if (!empty) {
-          tmem_ld32(tmem_base + lane_off + acc * BN + c * 32, r0);
-          tmem_ld_wait();
+      if (w.num_kb <= 0) {                          // nothing contracted: zeros (or C unchanged)
+        if (p.c_tma) {
+          if (lane == 0) tma_store_wait_read<0>();
+          __syncwarp();
         }
-#pragma unroll
-        for (int i = 0; i < 32; ++i) stg[lane * 33 + i] = empty ? 0.f : __uint_as_float(r0[i]);
-        __syncwarp();
-        store_block_rows(q, stg, row0, w.n + c * 32);
-        __syncwarp();
+        const uint32_t zero[32] = {};
+        for (int c = 0; c < BN && row0 < w.m_end && w.n + c < p.N; c += 32) {
+          float4 old[8];
+          load_old(q, row0, w.n + c, old);
+          store_block_rows(q, st.base, row0, w.n + c, zero, old);
+        }
+        return true;
       }
-      if (empty) return true;
+      if (!mbar_wait_warp(&s.tmem_full[acc], acc_phase, p.status, kTimeoutTmemFull, s.abort)) { *s.abort = 1; return false; }
+      tc_fence_after();
+      if (row0 < w.m_end)   // warp-uniform; a block that reaches into the next group's rows is stored row by row
+        store_tile_part(q, &tmC, st, tmem_base + lane_off + acc * BN, row0, w.c_row + row0, w.n, row0 + 32 <= w.m_end);
       tc_fence_before();
       if (rank == 0) mbar_arrive(&s.tmem_empty[acc]);
       else mbar_arrive_cluster(map_to_cta(smem_u32(&s.tmem_empty[acc]), 0));
       if (++acc == 2) { acc = 0; acc_phase ^= 1; }
       return true;
     });
+    if (p.c_tma && lane == 0) tma_store_wait<0>();   // shared memory is released after this
   }
   pair_teardown(tmem_base, warp);
 }
@@ -353,8 +353,8 @@ static int pair_config(K kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* a
 }
 
 template <bool A_MN, bool B_MN, typename Tiles>
-static int launch_grouped2(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, const Tiles& tiles, int want_pairs,
-                           cudaStream_t st) {
+static int launch_grouped2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p,
+                           const Tiles& tiles, int want_pairs, cudaStream_t st) {
   static int max_pairs = -1;
   auto k = grouped_gemm2_kernel<A_MN, B_MN, Tiles>;
   cudaLaunchConfig_t cfg = {};
@@ -362,11 +362,12 @@ static int launch_grouped2(const CUtensorMap& ta, const CUtensorMap& tb, const P
   if (int rc = pair_config(k, &cfg, &attr, &max_pairs, st)) return rc;
   const int pairs = want_pairs < max_pairs ? want_pairs : max_pairs;
   cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
-  return int(cudaLaunchKernelEx(&cfg, k, ta, tb, p, tiles));
+  return int(cudaLaunchKernelEx(&cfg, k, ta, tb, tc, p, tiles));
 }
 
 template <bool A_MN, bool B_MN>
-static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p_in, int want_pairs, cudaStream_t st) {
+static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p_in, int want_pairs,
+                   cudaStream_t st) {
   Params p = p_in;
   static int max_pairs = -1;
   auto k = gemm2_bf16_kernel<A_MN, B_MN>;
@@ -390,8 +391,19 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p
       if (me != cudaSuccess) return int(me);
     }
   }
-  cudaError_t e = cudaLaunchKernelEx(&cfg, k, ta, tb, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, k, ta, tb, tc, p);
   return int(e);
+}
+
+// The tensor map of C for the plain 16-bit store (p.c_tma says whether it is used; `any` fills the kernel's parameter else).
+static int store_map(CUtensorMap* tc, const CUtensorMap& any, Params& p, uint64_t rows) {
+  p.c_tma = 0;
+  *tc = any;
+  if (p.out_mode != kOutBf16) return 0;
+  const int rc = hg_host::make_tmap_2d_store(tc, p.C, rows, uint64_t(p.N), uint64_t(p.ldc));
+  if (rc == 0) p.c_tma = 1;
+  else *tc = any;
+  return rc < 0 ? rc : 0;
 }
 
 extern "C" {
@@ -423,11 +435,13 @@ int hg_gemm2_bf16(const void* A, const void* B, void* C, const void* bias, int M
   p.k_ranges = nullptr; p.groups = 1; p.c_group_stride = 0;
   int pairs = p.tiles_m * p.tiles_n;
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
+  CUtensorMap tc;
+  if ((rc = store_map(&tc, ta, p, M))) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (a_mn && b_mn) return launch2<true, true>(ta, tb, p, pairs, st);
-  if (a_mn) return launch2<true, false>(ta, tb, p, pairs, st);
-  if (b_mn) return launch2<false, true>(ta, tb, p, pairs, st);
-  return launch2<false, false>(ta, tb, p, pairs, st);
+  if (a_mn && b_mn) return launch2<true, true>(ta, tb, tc, p, pairs, st);
+  if (a_mn) return launch2<true, false>(ta, tb, tc, p, pairs, st);
+  if (b_mn) return launch2<false, true>(ta, tb, tc, p, pairs, st);
+  return launch2<false, false>(ta, tb, tc, p, pairs, st);
 }
 
 // Same contracts as hg_grouped_gemm_bf16 and hg_grouped_wgrad_bf16 (gemm.cu), computed by CTA pairs; -2 as above.
@@ -446,7 +460,10 @@ int hg_grouped_gemm2_bf16(const void* A, const void* B, void* C, const void* row
   RowSegments t{reinterpret_cast<const int*>(row_start), G, (N + BN - 1) / BN, (K + BK - 1) / BK, b_mn ? K : N, max_rows,
                 p.status};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  return b_mn ? launch_grouped2<false, true>(ta, tb, p, t, 1 << 20, st) : launch_grouped2<false, false>(ta, tb, p, t, 1 << 20, st);
+  CUtensorMap tc;
+  if ((rc = store_map(&tc, ta, p, max_rows))) return rc;
+  return b_mn ? launch_grouped2<false, true>(ta, tb, tc, p, t, 1 << 20, st)
+              : launch_grouped2<false, false>(ta, tb, tc, p, t, 1 << 20, st);
 }
 
 int hg_grouped_wgrad2_bf16(const void* dy, const void* x, void* out, const void* row_start, int G, int rows, int N,
@@ -463,7 +480,9 @@ int hg_grouped_wgrad2_bf16(const void* dy, const void* x, void* out, const void*
   ContractionRanges t{reinterpret_cast<const int*>(row_start), G, (N + CM - 1) / CM, (K + BN - 1) / BN, N, (long long)N * K};
   int pairs = t.tiles_m * t.tiles_n * G;
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
-  return launch_grouped2<true, true>(ta, tb, p, t, pairs, reinterpret_cast<cudaStream_t>(stream));
+  CUtensorMap tc;
+  if ((rc = store_map(&tc, ta, p, uint64_t(G) * N))) return rc;
+  return launch_grouped2<true, true>(ta, tb, tc, p, t, pairs, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

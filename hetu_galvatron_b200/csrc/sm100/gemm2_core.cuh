@@ -14,8 +14,10 @@ constexpr int HALF_N = BN / 2;                // B rows staged by one CTA
 constexpr int STAGES2 = 6;
 constexpr int A2_BYTES = BM * BK * 2;         // 16 KB
 constexpr int B2_BYTES = HALF_N * BK * 2;     // 16 KB
-constexpr int EPI_STAGE_FLOATS = 32 * 33;     // one 32 x 32 fp32 block per epilogue warp, rows padded to 33 words
-constexpr int SMEM2_BYTES = STAGES2 * (A2_BYTES + B2_BYTES) + 1024 + 256 + EPI_WARPS * EPI_STAGE_FLOATS * 4;
+// Per epilogue warp: two 32-row x 128-byte blocks on their way to C, or one 32 x 32 fp32 block in rows of 36 words.
+constexpr int EPI_STAGE_FLOATS = 2 * 32 * 32;   // >= 32 rows of 36 words
+constexpr int SMEM2_BYTES = STAGES2 * (A2_BYTES + B2_BYTES) + EPI_WARPS * EPI_STAGE_FLOATS * 4 + 1024 + 256;
+static_assert(SMEM2_BYTES <= 232448, "one CTA per SM");
 constexpr uint16_t kPairMask = 0x3;
 
 struct Smem2 {
@@ -35,14 +37,14 @@ __device__ __forceinline__ Smem2 carve2(uint8_t* raw) {
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
   s.a = base;
   s.b = base + STAGES2 * A2_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(base + STAGES2 * (A2_BYTES + B2_BYTES));
+  s.epi_stage = reinterpret_cast<float*>(base + STAGES2 * (A2_BYTES + B2_BYTES));   // 1024-byte aligned
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s.epi_stage + EPI_WARPS * EPI_STAGE_FLOATS);
   s.full = bars;
   s.empty = bars + STAGES2;
   s.tmem_full = bars + 2 * STAGES2;
   s.tmem_empty = bars + 2 * STAGES2 + 2;
   s.tmem_base = reinterpret_cast<uint32_t*>(bars + 2 * STAGES2 + 4);
   s.abort = reinterpret_cast<volatile int*>(s.tmem_base + 1);
-  s.epi_stage = reinterpret_cast<float*>(base + STAGES2 * (A2_BYTES + B2_BYTES) + 256);
   return s;
 }
 
@@ -259,65 +261,222 @@ __device__ __forceinline__ void mma2(const Params& p, const Smem2& s, uint32_t t
   if (!ok) *s.abort = 1;
 }
 
-// Epilogue: tcgen05.ld hands every thread one accumulator ROW (32 consecutive columns), but a row per thread is the
-// wrong shape for global memory: a warp's 16-byte accesses land in 32 different rows and fill only half of every
-// 32-byte sector (138 MB of L2 writes for a 67 MB result, and twice that again for the read-modify-write of the
-// fp32 accumulate mode).  Each warp therefore turns its 32 x 32 block through shared memory and touches global
-// memory one row at a time, 32 lanes on 32 consecutive columns: whole sectors only.
-// `part` (optional): the other slices' partial sums of this 32 x 32 block, slice k at part + k * kSplitTileFloats,
-// rows 256 floats apart, already offset to this lane's column; they are added in slice order before anything else.
-__device__ __forceinline__ void store_block_rows(const Params& p, float* stg, int row0, int col0,
-                                                 const float* part = nullptr, int nparts = 0) {
-  const int lane = int(lane_id());
-  if (part != nullptr) {
-    for (int k = 0; k < nparts; ++k) {
-      float add[32];
+// Epilogue.  tcgen05.ld hands every thread one accumulator ROW (32 consecutive columns), but a row per thread is the
+// wrong shape for global memory, so each warp turns its blocks through shared memory.
+//
+// Plain 16-bit stores: 32 rows x 128 bytes are written to the warp's stage in the layout of the 128-byte
+// swizzle, eight conflict-free 16-byte stores per thread, and leave as one TMA store that clips at the matrix' edges;
+// two blocks alternate, so that one is filled while the other is read.
+// Anything else (fp32 results, accumulating modes, an unaligned C, the ragged end of an expert's rows, a tile shared along
+// K): a 32 x 32 fp32 block at a time through 36-word rows (conflict-free 16-byte accesses both ways), eight lanes on 32
+// consecutive columns of a row, four elements each, all loads of a block before its first store.  (fp32 results by TMA
+// store were slower: expert weight gradients 4.14 against 3.13 ms.)
+//
+// Before, every mode took the second path row by row through generic pointers, where the compiler has to order each
+// shared-memory read behind the previous row's global store: 9.9 us for the 16-bit and 8.7 us for the fp32 store of a
+// 256 x 256 tile, hidden only under more than thirty k-blocks.
+__device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ float4 lds128(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// This warp's two store blocks; `next` alternates.  Bulk groups belong to a thread: lane 0 issues and waits.
+struct StoreStage {
+  uint32_t base;
+  int next;
+};
+
+// w: the 128 bytes of this thread's row, to columns col0.. of rows y0 .. y0 + 31 of the map.
+__device__ __forceinline__ void tma_store_rows(const CUtensorMap* tm, StoreStage& st, const uint32_t (&w)[32], int col0, int y0) {
+  const uint32_t lane = lane_id(), buf = st.base + st.next * 4096;
+  if (lane == 0) tma_store_wait_read<1>();          // the store before the last one has left this block
+  __syncwarp();
 #pragma unroll
-      for (int r = 0; r < 32; ++r) add[r] = __ldcg(part + size_t(k) * kSplitTileFloats + r * BN);
-#pragma unroll
-      for (int r = 0; r < 32; ++r) stg[r * 33 + lane] += add[r];
-    }
+  for (int j = 0; j < 8; ++j)
+    sts128(buf + sw128_offset(lane, j), w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (lane == 0) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+                 :
+                 : "l"(reinterpret_cast<uint64_t>(tm)), "r"(buf), "r"(col0), "r"(y0)
+                 : "memory");
+    tma_store_commit();
   }
-  const int col = col0 + lane;
-  if (!HG_BOUNDS_OK(row0 >= 0 && row0 < p.M && col0 >= 0 && col0 < p.N, p.status)) return;
-  if (col >= p.N) return;
-  const float bias = p.bias != nullptr ? hg_lp2f(p.bias[col]) : 0.f;
-  const int rows = min(32, p.M - row0);
-  if (p.out_mode == kOutBf16 || p.out_mode == kOutBf16Acc) {
-    hg_lp_t* c = reinterpret_cast<hg_lp_t*>(p.C) + size_t(row0) * p.ldc + col;
-    float old[32];
-    if (p.out_mode == kOutBf16Acc) {   // all 32 loads in flight before the first use
+  st.next ^= 1;
+}
+
+// A 32 x 64 block from registers (thread = row) through the tensor map.
+__device__ __forceinline__ void store_block64_tma(const Params& p, const CUtensorMap* tm, StoreStage& st, int y0, int col0,
+                                                  const uint32_t (&r0)[32], const uint32_t (&r1)[32]) {
+  auto add_bias = [&](const uint32_t (&r)[32], int c, uint32_t (&v)[32]) {
 #pragma unroll
-      for (int r = 0; r < 32; ++r) old[r] = r < rows ? hg_lp2f(c[size_t(r) * p.ldc]) : 0.f;
-    } else {
-#pragma unroll
-      for (int r = 0; r < 32; ++r) old[r] = 0.f;
+    for (int i = 0; i < 32; ++i) {
+      const float b = p.bias != nullptr && c + i < p.N ? hg_lp2f(p.bias[c + i]) : 0.f;
+      v[i] = p.bias != nullptr ? __float_as_uint(__uint_as_float(r[i]) + b) : r[i];
     }
+  };
+  uint32_t v0[32], v1[32];
+  add_bias(r0, col0, v0);
+  add_bias(r1, col0 + 32, v1);
+  uint32_t w[32];
 #pragma unroll
-    for (int r = 0; r < 32; ++r)
-      if (r < rows) c[size_t(r) * p.ldc] = hg_f2lp(stg[r * 33 + lane] + bias + old[r]);
-  } else {
-    float* c = reinterpret_cast<float*>(p.C) + size_t(row0) * p.ldc + col;
-    float old[32];
+  for (int i = 0; i < 16; ++i) {
+    w[i] = pack_bf16(__uint_as_float(v0[2 * i]), __uint_as_float(v0[2 * i + 1]));
+    w[16 + i] = pack_bf16(__uint_as_float(v1[2 * i]), __uint_as_float(v1[2 * i + 1]));
+  }
+  tma_store_rows(tm, st, w, col0, y0);
+}
+
+// Row by row: lane l works on columns 4 (l % 8) .. + 3 of rows l / 8, l / 8 + 4, ... of a 32 x 32 block.
+// Whether those four elements can move as one access (C and its pitch multiples of four elements).
+__device__ __forceinline__ bool four_aligned(const Params& p) {
+  const uint32_t es = p.out_mode == kOutBf16 || p.out_mode == kOutBf16Acc ? 2 : 4;
+  return (reinterpret_cast<uintptr_t>(p.C) & (4 * es - 1)) == 0 && (p.ldc & 3) == 0;
+}
+
+// What the accumulating modes add to a block (zeros otherwise): all loads in flight together.
+__device__ __forceinline__ void load_old(const Params& p, int row0, int col0, float4 (&old)[8]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) old[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (p.out_mode != kOutF32Acc && p.out_mode != kOutBf16Acc) return;
+  const int lane = int(lane_id()), col = col0 + (lane & 7) * 4, rows = p.M - row0;
+  const bool vec = four_aligned(p) && col + 3 < p.N;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = i * 4 + (lane >> 3);
+    if (r >= rows) continue;
+    const size_t at = size_t(row0 + r) * p.ldc + col;
     if (p.out_mode == kOutF32Acc) {
+      const float* c = reinterpret_cast<const float*>(p.C) + at;
+      if (vec) {
+        old[i] = *reinterpret_cast<const float4*>(c);
+      } else {
+        float* o = reinterpret_cast<float*>(&old[i]);
 #pragma unroll
-      for (int r = 0; r < 32; ++r) old[r] = r < rows ? c[size_t(r) * p.ldc] : 0.f;
+        for (int j = 0; j < 4; ++j)
+          if (col + j < p.N) o[j] = c[j];
+      }
     } else {
+      const hg_lp_t* c = reinterpret_cast<const hg_lp_t*>(p.C) + at;
+      if (vec) {
+        const uint2 u = *reinterpret_cast<const uint2*>(c);
+        const float2 lo = hg_unpack2(u.x), hi = hg_unpack2(u.y);
+        old[i] = make_float4(lo.x, lo.y, hi.x, hi.y);
+      } else {
+        float* o = reinterpret_cast<float*>(&old[i]);
 #pragma unroll
-      for (int r = 0; r < 32; ++r) old[r] = 0.f;
+        for (int j = 0; j < 4; ++j)
+          if (col + j < p.N) o[j] = hg_lp2f(c[j]);
+      }
     }
-#pragma unroll
-    for (int r = 0; r < 32; ++r)
-      if (r < rows) c[size_t(r) * p.ldc] = stg[r * 33 + lane] + bias + old[r];
   }
 }
 
-__device__ __forceinline__ void epilogue2(const Params& p, const Smem2& s, uint32_t tmem_base, uint32_t rank, int first,
-                                          int step, int num_tiles) {
+// One 32 x 32 block from registers (thread = row), any output mode.  `part` (optional): the other slices' partial sums of
+// this block, slice k at part + k * kSplitTileFloats, rows 256 floats apart; they are added in slice order before anything
+// else.
+__device__ __forceinline__ void store_block_rows(const Params& p, uint32_t stg, int row0, int col0, const uint32_t (&src)[32],
+                                                 const float4 (&old)[8], const float* part = nullptr, int nparts = 0) {
+  const int lane = int(lane_id());
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    sts128(stg + lane * 144 + j * 16, src[4 * j], src[4 * j + 1], src[4 * j + 2], src[4 * j + 3]);
+  __syncwarp();
+  const int q = (lane & 7) * 4, col = col0 + q;
+  float4 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = lds128(stg + (i * 4 + (lane >> 3)) * 144 + q * 4);
+  __syncwarp();
+  if (!HG_BOUNDS_OK(row0 >= 0 && row0 < p.M && col0 >= 0 && col0 < p.N, p.status)) return;
+  if (part != nullptr) {
+    for (int k = 0; k < nparts; ++k) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float4 a = __ldcg(reinterpret_cast<const float4*>(part + size_t(k) * kSplitTileFloats + (i * 4 + (lane >> 3)) * BN + q));
+        v[i].x += a.x; v[i].y += a.y; v[i].z += a.z; v[i].w += a.w;
+      }
+    }
+  }
+  if (col >= p.N) return;
+  float b[4] = {0.f, 0.f, 0.f, 0.f};
+  if (p.bias != nullptr) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (col + j < p.N) b[j] = hg_lp2f(p.bias[col + j]);
+  }
+  const bool vec = four_aligned(p) && col + 3 < p.N;
+  const int rows = p.M - row0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = i * 4 + (lane >> 3);
+    if (r >= rows) continue;
+    const float o[4] = {v[i].x + b[0] + old[i].x, v[i].y + b[1] + old[i].y, v[i].z + b[2] + old[i].z, v[i].w + b[3] + old[i].w};
+    const size_t at = size_t(row0 + r) * p.ldc + col;
+    if (p.out_mode == kOutBf16 || p.out_mode == kOutBf16Acc) {
+      hg_lp_t* c = reinterpret_cast<hg_lp_t*>(p.C) + at;
+      if (vec) {
+        *reinterpret_cast<uint2*>(c) = make_uint2(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (col + j < p.N) c[j] = hg_f2lp(o[j]);
+      }
+    } else {
+      float* c = reinterpret_cast<float*>(p.C) + at;
+      if (vec) {
+        *reinterpret_cast<float4*>(c) = make_float4(o[0], o[1], o[2], o[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (col + j < p.N) c[j] = o[j];
+      }
+    }
+  }
+}
+
+// The 32 x 256 part of a tile that this warp's lanes hold in tensor memory at `src`: rows row0.. of C (p.M: the first row
+// that is not this tile's), rows y0.. of the tensor map.
+__device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorMap* tmC, StoreStage& st, uint32_t src, int row0,
+                                                int y0, int n0, bool whole_rows, const float* part = nullptr,
+                                                int nparts = 0) {
+  if (p.c_tma && whole_rows && part == nullptr) {
+#pragma unroll 1
+    for (int c = 0; c < BN && n0 + c < p.N; c += 64) {
+      uint32_t r0[32], r1[32];
+      tmem_ld32(src + c, r0);
+      tmem_ld32(src + c + 32, r1);
+      tmem_ld_wait();
+      if (!HG_BOUNDS_OK(row0 >= 0 && row0 < p.M, p.status)) continue;
+      store_block64_tma(p, tmC, st, y0, n0 + c, r0, r1);
+    }
+    return;
+  }
+  if (p.c_tma) {                                    // the stage is about to be written past the stores that read it
+    if (lane_id() == 0) tma_store_wait_read<0>();
+    __syncwarp();
+  }
+#pragma unroll 1
+  for (int c = 0; c < BN && n0 + c < p.N; c += 32) {
+    float4 old[8];
+    load_old(p, row0, n0 + c, old);
+    uint32_t r0[32];
+    tmem_ld32(src + c, r0);
+    tmem_ld_wait();
+    store_block_rows(p, st.base, row0, n0 + c, r0, old, part ? part + c : nullptr, nparts);
+  }
+}
+
+__device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tmC, const Smem2& s, uint32_t tmem_base,
+                                          uint32_t rank, int first, int step, int num_tiles) {
   const int wq = (threadIdx.x >> 5) & 3;
   const int lane = int(lane_id());
   const uint32_t lane_off = uint32_t(wq * 32) << 16;
-  float* stg = s.epi_stage + wq * EPI_STAGE_FLOATS;
+  StoreStage st{smem_u32(s.epi_stage + wq * EPI_STAGE_FLOATS), 0};
   uint32_t acc = 0, acc_phase = 0;
   const int num_kb = (p.K + BK - 1) / BK;
   const int n_units = unit_count(p, first, step, num_tiles);
@@ -367,26 +526,23 @@ __device__ __forceinline__ void epilogue2(const Params& p, const Smem2& s, uint3
         break;
       }
     }
+    const uint32_t src = tmem_base + lane_off + acc * BN;
+    if (ws_mine != nullptr) {
 #pragma unroll 1
-    for (int c = 0; c < BN / 32; ++c) {
-      uint32_t r0[32];
-      tmem_ld32(tmem_base + lane_off + acc * BN + c * 32, r0);
-      tmem_ld_wait();
-      if (ws_mine != nullptr) {
+      for (int c = 0; c < BN / 32; ++c) {
+        uint32_t r0[32];
+        tmem_ld32(src + c * 32, r0);
+        tmem_ld_wait();
         // partial tile: row r of this thread's lane = tile row in_row + lane, 32 consecutive floats
         float* dst = ws_mine + size_t(in_row + lane) * BN + c * 32;
 #pragma unroll
         for (int i = 0; i < 32; i += 4)
           __stcg(reinterpret_cast<float4*>(dst + i), make_float4(__uint_as_float(r0[i]), __uint_as_float(r0[i + 1]),
                                                                  __uint_as_float(r0[i + 2]), __uint_as_float(r0[i + 3])));
-      } else if (row0 < p.M && n0 + c * 32 < p.N) {   // warp-uniform
-#pragma unroll
-        for (int i = 0; i < 32; ++i) stg[lane * 33 + i] = __uint_as_float(r0[i]);   // bank (lane + i) % 32: no conflicts
-        __syncwarp();
-        store_block_rows(p, stg, row0, n0 + c * 32,
-                         ws_others ? ws_others + size_t(in_row) * BN + c * 32 + lane : nullptr, p.split_s - 1);
-        __syncwarp();
       }
+    } else if (row0 < p.M) {   // warp-uniform
+      store_tile_part(p, tmC, st, src, row0, row0, n0, true, ws_others ? ws_others + size_t(in_row) * BN : nullptr,
+                      p.split_s - 1);
     }
     if (ws_mine != nullptr) {
       __threadfence();
@@ -399,6 +555,7 @@ __device__ __forceinline__ void epilogue2(const Params& p, const Smem2& s, uint3
     else mbar_arrive_cluster(map_to_cta(smem_u32(&s.tmem_empty[acc]), 0));
     if (++acc == 2) { acc = 0; acc_phase ^= 1; }
   }
+  if (p.c_tma && lane == 0) tma_store_wait<0>();     // shared memory is released after this
 }
 
 

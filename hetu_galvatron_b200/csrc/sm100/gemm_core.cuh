@@ -74,6 +74,7 @@ struct Params {
   int split_tail_begin;
   float* split_ws;
   int* split_flags;
+  int c_tma;                  // CTA-pair kernels: full blocks of C leave through the tensor map of C (plain 16-bit store)
 };
 
 struct TileInfo {

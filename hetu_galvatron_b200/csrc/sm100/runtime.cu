@@ -133,6 +133,12 @@ int encode_tmap_2d(CUtensorMap* out, const void* base, uint64_t rows, uint64_t c
   return r == CUDA_SUCCESS ? 0 : -(1000 + int(r));
 }
 
+int make_tmap_2d_store(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld) {
+  // a store clips columns in whole 16-byte groups only: with another width it would write past the last column
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld & 7) || (cols & 7)) return 1;
+  return make_tmap_2d_bf16(out, base, rows, cols, ld, 32, 64);
+}
+
 int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1,
                       uint64_t stride2, uint32_t box0, uint32_t box1, uint32_t box2) {
   EncodeTiledFn enc = get_encode_fn();

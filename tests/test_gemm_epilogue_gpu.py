@@ -1,0 +1,33 @@
+"""Stores of the CTA-pair GEMM: blocks that leave by TMA and blocks that are stored row by row, in every output mode."""
+import pytest
+import torch
+
+from hetu_galvatron_b200 import ops
+from hetu_galvatron_b200.ops import _lib
+from hetu_galvatron_b200.ops.gemm import OUT_BF16, OUT_BF16_ACC, OUT_F32, OUT_F32_ACC
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# whole tiles, ragged rows and columns (clipped boxes), a pitch that is no multiple of 16 bytes, more tiles than pairs
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (300, 328, 72), (257, 1000, 136), (1000, 333, 64), (2600, 2568, 64)])
+@pytest.mark.parametrize("mode", [OUT_BF16, OUT_F32, OUT_F32_ACC, OUT_BF16_ACC])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_every_store_of_the_pair_kernel(M, N, K, mode, shift):
+    g = torch.Generator(device=DEV).manual_seed(M + N + mode)
+    a, b = (torch.randn(n, K, device=DEV, generator=g).to(torch.bfloat16) for n in (M, N))
+    bias = torch.randn(N, device=DEV, generator=g).to(torch.bfloat16)
+    dt = torch.float32 if mode in (OUT_F32, OUT_F32_ACC) else torch.bfloat16
+    whole = torch.full((M + 2, N + 3 + shift), 2.0, device=DEV, dtype=dt)       # C is a window of a wider matrix
+    out = whole[1:M + 1, shift:N + shift]
+    ops.gemm(a, b, out=out, out_mode=mode, bias=bias, pair=True)
+    ref = a.double() @ b.double().t() + bias.double() + (2.0 if mode in (OUT_F32_ACC, OUT_BF16_ACC) else 0.0)
+    err = ((out.double() - ref).norm() / ref.norm()).item()
+    assert err < (1e-5 if dt == torch.float32 else 2.0 ** -8)                   # fp32 sums; one rounding
+    out.fill_(2.0)
+    assert (whole == 2.0).all()                                                 # nothing outside the window
+    packed = ops.gemm(a, b, out_mode=mode, bias=bias, pair=True) if mode in (OUT_BF16, OUT_F32) else None
+    if packed is not None:
+        assert ((packed.double() - ref).norm() / ref.norm()).item() < (1e-5 if dt == torch.float32 else 2.0 ** -8)
+    _lib.assert_healthy()
