@@ -12,6 +12,7 @@
 // galvatron/core/runtime/transformer/attention_impl.py:55-111,587-616,696-727.
 #include <type_traits>
 
+#include "attn_tensor.h"
 #include "sm100_common.cuh"
 
 namespace hg {
@@ -1968,15 +1969,6 @@ int launch_dq(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& t
 }  // namespace
 
 extern "C" {
-
-// Tensor descriptor passed from Python: base pointer, strides (elements) over s and b, number of head
-// slots in a token row, and the head->slot map (gs, hs, off).
-struct HgAttnTensor {
-  void* ptr;
-  long long ss, sb;
-  int slots;
-  int gs, hs, off;
-};
 
 int hg_flash_fwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o,
                  void* lse, int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0,

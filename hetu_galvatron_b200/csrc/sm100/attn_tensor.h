@@ -1,0 +1,10 @@
+// Tensor descriptor of the attention entry points (mirrored by ``AttnTensor`` in ops/_lib.py): base pointer, strides
+// (elements) over s and b, number of head slots in a token row, and the head -> slot map (gs, hs, off).
+#pragma once
+
+struct HgAttnTensor {
+  void* ptr;
+  long long ss, sb;
+  int slots;
+  int gs, hs, off;
+};

@@ -121,6 +121,60 @@ __global__ void rope_interleaved_kernel(hg_lp_t* __restrict__ buf, const int* __
 }
 
 // ---------------------------------------------------------------------------------------------
+// Cached attention: RoPE on the new tokens of a packed projection [tokens, ng * (qpg + 2) * hd] (per kv head: qpg query
+// heads, the key head, the value head).  Queries are rotated in place; rotated keys and the values go straight into
+// their rows of the cache, so that a decode step makes one launch where rotating, splitting and copying made seven.
+// An item is 8 channels of one slot of one token (with the 8 they rotate with in the rotate-half form); half = 0: no
+// rotation.  Cache element (s, b, g, d) at base + s * c_ss + b * c_sb + g * hd + d, s and b counted from the new tokens.
+// ---------------------------------------------------------------------------------------------
+__global__ void rope_append_kernel(hg_lp_t* __restrict__ qkv, int tokens, int batch, int ng, int qpg, int hd,
+                                   int pos_offset, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                                   int half, int interleaved, hg_lp_t* __restrict__ kc, hg_lp_t* __restrict__ vc,
+                                   int64_t k_ss, int64_t k_sb, int64_t v_ss, int64_t v_sb) {
+  const int vph = hd >> 3, slots = ng * (qpg + 2);
+  for (RowColWalk w(slots * vph); w.row < tokens; w.next()) {
+    const int t = int(w.row), slot = w.col / vph, c = w.col - slot * vph;
+    const int g = slot / (qpg + 2), j = slot - g * (qpg + 2);
+    const int s = t / batch, b = t - s * batch;
+    hg_lp_t* in = qkv + int64_t(t) * slots * hd + int64_t(slot) * hd + c * 8;
+    hg_lp_t* out = j < qpg ? in : j == qpg ? kc + s * k_ss + b * k_sb + g * hd + c * 8
+                                           : vc + s * v_ss + b * v_sb + g * hd + c * 8;
+    const float* ct = cos_t + int64_t(s + pos_offset) * half;
+    const float* st = sin_t + int64_t(s + pos_offset) * half;
+    const bool rotates = j <= qpg && c * 8 < 2 * half;
+    if (!rotates) {
+      if (j >= qpg) *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(in);
+    } else if (interleaved) {
+      float x[8], o[8];
+      unpack8(*reinterpret_cast<const uint4*>(in), x);
+      const float4 cs = *reinterpret_cast<const float4*>(ct + c * 4), sn = *reinterpret_cast<const float4*>(st + c * 4);
+      const float cv[4] = {cs.x, cs.y, cs.z, cs.w}, sv[4] = {sn.x, sn.y, sn.z, sn.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        o[2 * i] = x[2 * i] * cv[i] - x[2 * i + 1] * sv[i];
+        o[2 * i + 1] = x[2 * i + 1] * cv[i] + x[2 * i] * sv[i];
+      }
+      *reinterpret_cast<uint4*>(out) = pack8(o);
+    } else if (c * 8 < half) {                       // the item of channels half + 8c.. is covered here
+      float a[8], bb[8], cs[8], sn[8], oa[8], ob[8];
+      unpack8(*reinterpret_cast<const uint4*>(in), a);
+      unpack8(*reinterpret_cast<const uint4*>(in + half), bb);
+      *reinterpret_cast<float4*>(cs) = reinterpret_cast<const float4*>(ct + c * 8)[0];
+      *reinterpret_cast<float4*>(cs + 4) = reinterpret_cast<const float4*>(ct + c * 8)[1];
+      *reinterpret_cast<float4*>(sn) = reinterpret_cast<const float4*>(st + c * 8)[0];
+      *reinterpret_cast<float4*>(sn + 4) = reinterpret_cast<const float4*>(st + c * 8)[1];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        oa[i] = a[i] * cs[i] - bb[i] * sn[i];
+        ob[i] = bb[i] * cs[i] + a[i] * sn[i];
+      }
+      *reinterpret_cast<uint4*>(out) = pack8(oa);
+      *reinterpret_cast<uint4*>(out + half) = pack8(ob);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
 // Gated activations on y = [y1 | y2] (each F wide, row pitch 2F):  out = act(y1) * y2
 //   kind 0: SwiGLU (silu), kind 1: GeGLU (tanh GELU).  Non-gated kind 2: out = gelu_tanh(y) (pitch F).
 // ---------------------------------------------------------------------------------------------
@@ -406,6 +460,22 @@ int hg_rope(void* buf, const void* slots, int slot_width, int nheads, int row_pi
         (hg_lp_t*)buf, (const int*)slots, slot_width, nheads, row_pitch, tokens, batch, (const int*)pos, pos_offset,
         (const float*)cos_t, (const float*)sin_t, half, sign);
   }
+  return int(cudaGetLastError());
+}
+
+// See rope_append_kernel.  rot_dim = 0: no rotation (cos_t / sin_t unused).  Strides in elements, multiples of 8; all
+// pointers 16-byte aligned.
+int hg_rope_append(void* qkv, int tokens, int batch, int ng, int qpg, int hd, int pos_offset, const void* cos_t,
+                   const void* sin_t, int rot_dim, int interleaved, void* kc, void* vc, long long k_ss, long long k_sb,
+                   long long v_ss, long long v_sb, void* stream) {
+  if (tokens <= 0) return 0;
+  const int half = rot_dim / 2;
+  if ((hd & 7) || (half & 7) || batch < 1 || ng < 1 || qpg < 1 || ((k_ss | k_sb | v_ss | v_sb) & 7)) return -1;
+  if ((uintptr_t(qkv) | uintptr_t(kc) | uintptr_t(vc)) & 15) return -1;
+  const int64_t work = int64_t(tokens) * ng * (qpg + 2) * (hd >> 3);
+  rope_append_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
+      (hg_lp_t*)qkv, tokens, batch, ng, qpg, hd, pos_offset, (const float*)cos_t, (const float*)sin_t, half, interleaved,
+      (hg_lp_t*)kc, (hg_lp_t*)vc, k_ss, k_sb, v_ss, v_sb);
   return int(cudaGetLastError());
 }
 

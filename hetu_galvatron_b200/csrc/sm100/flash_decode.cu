@@ -1,0 +1,290 @@
+// Attention of a few queries over a long key / value cache (decode steps), forward only.
+//
+// The tile kernels of attention.cu give a CTA 128 query rows of one head: with one new token a CTA does 1 / 128 of the
+// work it is built for, walks all keys of its head alone, and the query heads that share a kv head read its keys once
+// each.  What bounds a decode step is reading K and V once, so here a CTA takes one kv head, CH keys and the (at most
+// eight) query rows that attend to them; the key ranges of a sequence are spread over the chip and their partial
+// results merged by a second small kernel (skipped when one range covers all keys).  Scores and probabilities stay in
+// fp32 throughout.
+//
+// Rows: r = s * qpg + j is query token s of query head g * qpg + j.  A lane holds eight channels, so HD / 8 lanes share a
+// key and a warp reads 32 / (HD / 8) keys per 16-byte access.
+#include "attn_tensor.h"
+#include "sm100_common.cuh"
+
+namespace {
+
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kLn2 = 0.6931471805599453f;
+constexpr int kMaxRows = 8;
+
+struct DecodeParams {
+  const hg_lp_t *Q, *K, *V;
+  int64_t q_ss, q_sb, k_ss, k_sb, v_ss, v_sb, o_ss, o_sb;
+  int q_gs, q_hs, q_off, k_gs, k_off, v_gs, v_off;    // slot of a head, see SlotMap in attention.cu
+  hg_lp_t* O;
+  float* LSE;               // [B, nheads, Sq]
+  float* ws;                // partial results, (HD + 2) floats per (row, key range)
+  int Sq, kv_len, B, nheads, nkv, qpg, causal, q_pos0, k_pos0;
+  float scale;
+};
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ void unpack8(const uint4& u, float* f) {
+  const hg_lp2_t* p = reinterpret_cast<const hg_lp2_t*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = hg_lp22ff(p[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+
+template <int HD, int R, int CH>
+__global__ void __launch_bounds__(128)
+flash_decode_kernel(const DecodeParams p) {
+  constexpr int LPK = HD / 8, KPW = 32 / LPK, STEPS = CH / (4 * KPW);
+  __shared__ float sS[R][CH];
+  __shared__ float sML[R][2];
+  __shared__ float sAcc[4][R][HD];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sub = lane / LPK, ch = (lane % LPK) * 8;
+  const int g = blockIdx.x, b = blockIdx.y, key0 = blockIdx.z * CH, ranges = gridDim.z;
+  const int rows = p.Sq * p.qpg;
+  const hg_lp_t* kb = p.K + int64_t(b) * p.k_sb + int64_t(g * p.k_gs + p.k_off) * HD + ch;
+  const hg_lp_t* vb = p.V + int64_t(b) * p.v_sb + int64_t(g * p.v_gs + p.v_off) * HD + ch;
+
+  // With one or two rows there are registers for all of a thread's keys and values: both are requested before anything
+  // is computed.
+  constexpr bool kPreload = R <= 2;
+  uint4 ku[kPreload ? STEPS : 1], vu[kPreload ? STEPS : 1];
+  if constexpr (kPreload) {
+#pragma unroll
+    for (int it = 0; it < STEPS; ++it) {
+      const int key = key0 + (it * 4 + warp) * KPW + sub;
+      ku[it] = key < p.kv_len ? *reinterpret_cast<const uint4*>(kb + int64_t(key) * p.k_ss) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int it = 0; it < STEPS; ++it) {
+      const int key = key0 + (it * 4 + warp) * KPW + sub;
+      vu[it] = key < p.kv_len ? *reinterpret_cast<const uint4*>(vb + int64_t(key) * p.v_ss) : make_uint4(0, 0, 0, 0);
+    }
+  }
+  {
+    float q[R][8];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      uint4 u = make_uint4(0, 0, 0, 0);
+      if (r < rows)
+        u = *reinterpret_cast<const uint4*>(p.Q + int64_t(r / p.qpg) * p.q_ss + int64_t(b) * p.q_sb +
+                                            int64_t(g * p.q_gs + (r % p.qpg) * p.q_hs + p.q_off) * HD + ch);
+      unpack8(u, q[r]);
+    }
+#pragma unroll (kPreload ? STEPS : 4)
+    for (int it = 0; it < STEPS; ++it) {
+      const int kl = (it * 4 + warp) * KPW + sub, key = key0 + kl;
+      uint4 u = make_uint4(0, 0, 0, 0);
+      if constexpr (kPreload) u = ku[it];
+      else if (key < p.kv_len) u = *reinterpret_cast<const uint4*>(kb + int64_t(key) * p.k_ss);
+      float f[8];
+      unpack8(u, f);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float d = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) d = fmaf(q[r][i], f[i], d);
+#pragma unroll
+        for (int o = LPK / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if (lane % LPK == 0) sS[r][kl] = d;
+      }
+    }
+  }
+  __syncthreads();
+  for (int r = warp; r < R; r += 4) {
+    const float sl2 = p.scale * kLog2e;
+    const int q_pos = p.q_pos0 + r / p.qpg;
+    float s[CH / 32], m = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < CH / 32; ++i) {
+      const int kl = i * 32 + lane, key = key0 + kl;
+      const bool seen = r < rows && key < p.kv_len && (!p.causal || p.k_pos0 + key <= q_pos);
+      s[i] = seen ? sS[r][kl] * sl2 : -INFINITY;
+      m = fmaxf(m, s[i]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float ref = m == -INFINITY ? 0.f : m;
+    float l = 0.f;
+#pragma unroll
+    for (int i = 0; i < CH / 32; ++i) {
+      const float e = ex2(s[i] - ref);
+      l += e;
+      sS[r][i * 32 + lane] = e;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    if (lane == 0) {
+      sML[r][0] = m;
+      sML[r][1] = l;
+    }
+  }
+  __syncthreads();
+  float acc[R][8];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[r][i] = 0.f;
+#pragma unroll (kPreload ? STEPS : 4)
+  for (int it = 0; it < STEPS; ++it) {
+    const int kl = (it * 4 + warp) * KPW + sub, key = key0 + kl;
+    uint4 u = make_uint4(0, 0, 0, 0);
+    if constexpr (kPreload) u = vu[it];
+    else if (key < p.kv_len) u = *reinterpret_cast<const uint4*>(vb + int64_t(key) * p.v_ss);
+    float f[8];
+    unpack8(u, f);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float e = sS[r][kl];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[r][i] = fmaf(e, f[i], acc[r][i]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+#pragma unroll
+      for (int o = LPK; o < 32; o <<= 1) acc[r][i] += __shfl_xor_sync(0xffffffffu, acc[r][i], o);
+      if (sub == 0) sAcc[warp][r][ch + i] = acc[r][i];
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < rows * HD; i += 128) {
+    const int r = i / HD, c = i % HD;
+    const float v = (sAcc[0][r][c] + sAcc[1][r][c]) + (sAcc[2][r][c] + sAcc[3][r][c]);
+    const float m = sML[r][0], l = sML[r][1];
+    if (ranges == 1) {
+      const int h = g * p.qpg + r % p.qpg, s = r / p.qpg;
+      p.O[int64_t(s) * p.o_ss + int64_t(b) * p.o_sb + int64_t(h) * HD + c] = hg_f2lp(l > 0.f ? v / l : 0.f);
+      if (c == 0) p.LSE[(size_t(b) * p.nheads + h) * p.Sq + s] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
+    } else {
+      float* w = p.ws + ((int64_t(b) * p.nkv + g) * rows + r) * int64_t(ranges) * (HD + 2) + int64_t(blockIdx.z) * (HD + 2);
+      w[c] = v;
+      if (c == 0) {
+        w[HD] = m;
+        w[HD + 1] = l;
+      }
+    }
+  }
+}
+
+// One CTA of HD threads per (sequence, kv head, row): the key ranges' partial results, merged in range order.
+template <int HD>
+__global__ void __launch_bounds__(HD)
+flash_decode_merge_kernel(const DecodeParams p, int ranges) {
+  const int rows = p.Sq * p.qpg;
+  const int r = blockIdx.x % rows, g = (blockIdx.x / rows) % p.nkv, b = blockIdx.x / rows / p.nkv, c = threadIdx.x;
+  const float* w = p.ws + int64_t(blockIdx.x) * ranges * (HD + 2);
+  float m = -INFINITY;
+#pragma unroll 8
+  for (int i = 0; i < ranges; ++i) m = fmaxf(m, w[int64_t(i) * (HD + 2) + HD]);
+  const float ref = m == -INFINITY ? 0.f : m;
+  float v = 0.f, l = 0.f;
+#pragma unroll 8
+  for (int i = 0; i < ranges; ++i) {
+    const float* wi = w + int64_t(i) * (HD + 2);
+    const float f = ex2(wi[HD] - ref);
+    v = fmaf(f, wi[c], v);
+    l = fmaf(f, wi[HD + 1], l);
+  }
+  const int h = g * p.qpg + r % p.qpg, s = r / p.qpg;
+  p.O[int64_t(s) * p.o_ss + int64_t(b) * p.o_sb + int64_t(h) * HD + c] = hg_f2lp(l > 0.f ? v / l : 0.f);
+  if (c == 0) p.LSE[(size_t(b) * p.nheads + h) * p.Sq + s] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
+}
+
+inline int keys_seen(int Sq, int Skv, int causal, int q_pos0, int k_pos0) {
+  long long n = Skv;
+  if (causal) {
+    const long long last = (long long)q_pos0 + Sq - k_pos0;   // keys that the last query may see
+    if (last < n) n = last;
+  }
+  return n < 0 ? 0 : int(n);
+}
+// Up to two rows: 64 keys per CTA, all loaded at once.  More rows: 128 where that still gives every SM several CTAs.
+inline int keys_per_cta(int rows, int kv_len, int nkv, int B) {
+  return rows > 2 && (long long)((kv_len + 127) / 128) * nkv * B >= 148 * 8 ? 128 : 64;
+}
+inline int range_count(int kv_len, int chunk) { return kv_len > chunk ? (kv_len + chunk - 1) / chunk : 1; }
+
+template <int HD, int R>
+int launch(const DecodeParams& p, int chunk, int ranges, cudaStream_t st) {
+  const dim3 grid(p.nkv, p.B, ranges);   // neighbours read neighbouring heads of the same cache rows
+  if constexpr (R > 2) {
+    if (chunk == 128) flash_decode_kernel<HD, R, 128><<<grid, 128, 0, st>>>(p);
+    else flash_decode_kernel<HD, R, 64><<<grid, 128, 0, st>>>(p);
+  } else {
+    flash_decode_kernel<HD, R, 64><<<grid, 128, 0, st>>>(p);
+  }
+  if (ranges > 1) flash_decode_merge_kernel<HD><<<p.B * p.nkv * p.Sq * p.qpg, HD, 0, st>>>(p, ranges);
+  return int(cudaGetLastError());
+}
+
+template <int HD>
+int launch_rows(const DecodeParams& p, int chunk, int ranges, cudaStream_t st) {
+  const int rows = p.Sq * p.qpg;
+  if (rows == 1) return launch<HD, 1>(p, chunk, ranges, st);
+  if (rows == 2) return launch<HD, 2>(p, chunk, ranges, st);
+  if (rows <= 4) return launch<HD, 4>(p, chunk, ranges, st);
+  return launch<HD, 8>(p, chunk, ranges, st);
+}
+
+}  // namespace
+
+extern "C" {
+
+// Floats of scratch hg_flash_decode needs (0: none), or -1 when it does not take the call: more than eight query rows
+// per kv head, another head dim, or rows that are not whole 16-byte groups.
+long long hg_flash_decode_scratch(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, int Sq, int Skv, int B,
+                                  int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
+  if ((hd != 64 && hd != 128) || Sq < 1 || Skv < 1 || B < 1 || nkv < 1 || nheads % nkv) return -1;
+  if ((long long)Sq * (nheads / nkv) > kMaxRows || nkv > 65535 || B > 65535) return -1;
+  for (const HgAttnTensor* t : {q, k, v})
+    if ((uintptr_t(t->ptr) & 15) || (t->ss & 7) || (t->sb & 7)) return -1;
+  const int kv_len = keys_seen(Sq, Skv, causal, q_pos0, k_pos0);
+  const int ranges = range_count(kv_len, keys_per_cta(Sq * (nheads / nkv), kv_len, nkv, B));
+  if (ranges > 65535) return -1;
+  return ranges > 1 ? (long long)B * nheads * Sq * ranges * (hd + 2) : 0;
+}
+
+// Whether spreading the keys beats the one-tile kernel.  That kernel takes a query head per CTA and walks its keys alone, so
+// it loses once its heads fill the chip or a head has many keys; below that its single launch wins over a launch and a
+// merge.  Measured, one query, head dim 128, cold (us, here against there): 4 sequences x 32 heads x 1000 keys 28 / 25, 1 x
+// 28 (4 kv heads) x 1000 23 / 21, 1 x 32 x 2000 24 / 33, 16 x 32 x 1000 65 / 79, 32 x 28 (4) x 2000 87 / 181.
+int hg_flash_decode_pays(int Sq, int Skv, int B, int nheads, int causal, int q_pos0, int k_pos0) {
+  return (long long)B * nheads > 148 || keys_seen(Sq, Skv, causal, q_pos0, k_pos0) >= 1536;
+}
+
+// Same contract as hg_flash_fwd for the calls that hg_flash_decode_scratch accepts; `ws` is its scratch.
+int hg_flash_decode(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o, void* lse,
+                    void* ws, int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0,
+                    float scale, void* stream) {
+  const long long need = hg_flash_decode_scratch(q, k, v, Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0);
+  if (need < 0 || (need > 0 && ws == nullptr)) return -1;
+  DecodeParams p{};
+  p.Q = (const hg_lp_t*)q->ptr; p.K = (const hg_lp_t*)k->ptr; p.V = (const hg_lp_t*)v->ptr; p.O = (hg_lp_t*)o->ptr;
+  p.q_ss = q->ss; p.q_sb = q->sb; p.k_ss = k->ss; p.k_sb = k->sb; p.v_ss = v->ss; p.v_sb = v->sb; p.o_ss = o->ss; p.o_sb = o->sb;
+  p.q_gs = q->gs; p.q_hs = q->hs; p.q_off = q->off;
+  p.k_gs = k->gs; p.k_off = k->off; p.v_gs = v->gs; p.v_off = v->off;
+  p.LSE = (float*)lse; p.ws = (float*)ws;
+  p.Sq = Sq; p.B = B; p.nheads = nheads; p.nkv = nkv; p.qpg = nheads / nkv; p.causal = causal;
+  p.q_pos0 = q_pos0; p.k_pos0 = k_pos0; p.scale = scale;
+  p.kv_len = keys_seen(Sq, Skv, causal, q_pos0, k_pos0);
+  const int chunk = keys_per_cta(Sq * p.qpg, p.kv_len, nkv, B), ranges = range_count(p.kv_len, chunk);
+  cudaStream_t st = (cudaStream_t)stream;
+  return hd == 128 ? launch_rows<128>(p, chunk, ranges, st) : launch_rows<64>(p, chunk, ranges, st);
+}
+
+}  // extern "C"

@@ -272,6 +272,24 @@ class SelfAttention(nn.Module):
                     return run().reshape(S_att, B, self.nh * self.hd)
         return run().reshape(S_att, B, self.nh * self.hd)
 
+    def cache_for(self, ic, like, S_new: int, B: int):
+        """``(key cache, value cache, cached tokens, first sequence, cos, sin)`` of this layer in the inference context
+        (allocated on first use); raises when the new tokens do not fit."""
+        past, b0, s = ic.sequence_len_offset, ic.batch_size_offset, self.spec
+        if past + S_new > ic.max_sequence_length or b0 + B > ic.max_batch_size:
+            raise ValueError("inference context too small: %d + %d tokens of %d, batch %d + %d of %d" %
+                             (past, S_new, ic.max_sequence_length, b0, B, ic.max_batch_size))
+        key = self.layer_number
+        if key not in ic.key_value_memory_dict:
+            shape = (ic.max_sequence_length, ic.max_batch_size, self.ng, self.hd)
+            ic.key_value_memory_dict[key] = tuple(torch.zeros(shape, dtype=like.dtype, device=like.device) for _ in "kv")
+        kc, vc = ic.key_value_memory_dict[key]
+        cos = sin = None
+        if s.pos == "rope":
+            cos, sin = ops.rope_tables(ic.max_sequence_length, self.rot_dim, s.rope_base, str(like.device), s.rope_interp,
+                                        s.rope_scaling_factor)
+        return kc, vc, past, b0, cos, sin
+
     def _cached_attention(self, qkv2, S_new: int, B: int):
         """Incremental forward with a key / value cache (static batching): the new keys and values are written
         behind the ``sequence_len_offset`` tokens already cached for this layer and the new queries attend to
@@ -281,25 +299,16 @@ class SelfAttention(nn.Module):
         s, c, ic = self.spec, self.ctx, self.inference_context
         if c.sp_size > 1 or c.cp_size > 1:
             raise NotImplementedError("cached attention needs sp = cp = 1")
-        past = ic.sequence_len_offset
-        b0 = ic.batch_size_offset
-        if past + S_new > ic.max_sequence_length or b0 + B > ic.max_batch_size:
-            raise ValueError("inference context too small: %d + %d tokens of %d, batch %d + %d of %d" %
-                             (past, S_new, ic.max_sequence_length, b0, B, ic.max_batch_size))
+        kc, vc, past, b0, cos, sin = self.cache_for(ic, qkv2, S_new, B)
+        if ops.attention.cached_attention_usable(qkv2, kc, vc, self.hd):
+            return ops.attention.cached_attention(qkv2, kc, vc, past, b0, S_new, B, self.nh, self.ng, self.hd, cos, sin,
+                                                  s.rope_interleaved)
         if s.pos == "rope":
-            cos, sin = ops.rope_tables(ic.max_sequence_length, self.rot_dim, s.rope_base, str(qkv2.device),
-                                        s.rope_interp, s.rope_scaling_factor)
             qkv2 = ops.rope_packed(qkv2, self.rope_slots, self.hd, cos, sin, B, None, past, s.rope_interleaved)
         q, k, v = ops.attention.split_packed(qkv2, self.nh, self.ng, self.hd)
         q = q.reshape(S_new, B, self.nh, self.hd)
         k = k.reshape(S_new, B, self.ng, self.hd)
         v = v.reshape(S_new, B, self.ng, self.hd)
-        key = self.layer_number
-        if key not in ic.key_value_memory_dict:
-            shape = (ic.max_sequence_length, ic.max_batch_size, self.ng, self.hd)
-            ic.key_value_memory_dict[key] = (torch.zeros(shape, dtype=k.dtype, device=k.device),
-                                             torch.zeros(shape, dtype=v.dtype, device=v.device))
-        kc, vc = ic.key_value_memory_dict[key]
         kc[past:past + S_new, b0:b0 + B] = k
         vc[past:past + S_new, b0:b0 + B] = v
         o = ops.flash_attention(q, kc[:past + S_new, b0:b0 + B], vc[:past + S_new, b0:b0 + B], causal=True,

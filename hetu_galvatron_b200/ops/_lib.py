@@ -113,6 +113,10 @@ _SIGNATURES = {
     "hg_clip_coef": [c_void_p, c_float, c_void_p, c_void_p, c_void_p],
     "hg_scale": [c_void_p, c_ll, c_int, c_void_p, c_float, c_void_p],
     "hg_flash_fwd": [ctypes.POINTER(AttnTensor)] * 4 + [c_void_p] + [c_int] * 9 + [c_float, c_void_p],
+    "hg_rope_append": [c_void_p] + [c_int] * 6 + [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p] + [c_ll] * 4 + [c_void_p],
+    "hg_flash_decode_pays": [c_int] * 7,
+    "hg_flash_decode_scratch": [ctypes.POINTER(AttnTensor)] * 3 + [c_int] * 9,
+    "hg_flash_decode": [ctypes.POINTER(AttnTensor)] * 4 + [c_void_p, c_void_p] + [c_int] * 9 + [c_float, c_void_p],
     "hg_flash_bwd": [ctypes.POINTER(AttnTensor)] * 5 + [c_void_p, c_void_p] + [ctypes.POINTER(AttnTensor)] * 3 +
                     [c_int] * 9 + [c_float, c_void_p],
     "hg_ag_gemm_bf16": [c_void_p] * 7 + [c_int] * 10 + [c_void_p],
@@ -154,6 +158,7 @@ def load():
             continue
         fn.argtypes = argtypes
         fn.restype = c_int
+    lib.hg_flash_decode_scratch.restype = c_ll
     if hasattr(lib, "hg_status_address"):
         lib.hg_status_address.restype = c_void_p
         lib.hg_status_address.argtypes = []

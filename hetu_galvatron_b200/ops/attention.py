@@ -121,10 +121,69 @@ def flash_attention_packed(qkv: torch.Tensor, S: int, B: int, nh: int, ng: int, 
     return _FlashPacked.apply(qkv.contiguous(), S, B, nh, ng, hd, causal, scale)
 
 
+def _forward_launch(q, k, v, o, lse, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, scale, spread=None):
+    """Forward on tensor descriptors: the kernels that split the keys over the chip when a kv head has at most eight
+    query rows and that pays (csrc/sm100/flash_decode.cu; ``spread`` forces or forbids it), the tile kernels otherwise."""
+    lib = _lib.load()
+    args = (S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0)
+    refs = [ctypes.byref(t) for t in (q, k, v)]
+    if spread is None:
+        spread = S * (nh // ng) <= 8 and lib.hg_flash_decode_pays(S, Skv, B, nh, int(causal), q_pos0, k_pos0)
+    need = lib.hg_flash_decode_scratch(*refs, *args) if spread else -1
+    if need >= 0:
+        ws = torch.empty(need, dtype=torch.float32, device=lse.device) if need else None
+        rc = lib.hg_flash_decode(*refs, ctypes.byref(o), lse.data_ptr(), _lib.ptr(ws), *args, float(scale), _lib.stream())
+        _lib.check(rc, "hg_flash_decode")
+        _lib.count_launch(2 if need else 1)
+        return
+    rc = lib.hg_flash_fwd(*refs, ctypes.byref(o), lse.data_ptr(), *args, float(scale), _lib.stream())
+    _lib.check(rc, "hg_flash_fwd")
+    _lib.count_launch()
+
+
+def caches_usable(like: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, hd: int) -> bool:
+    """Whether the kernels can write to and read from these caches ``[max_seq, max_batch, ng, hd]``: ``like``'s dtype and
+    device, contiguous heads, whole 16-byte groups, and no gradient recorded through them."""
+    return (kc.dtype == vc.dtype == like.dtype and kc.device == vc.device == like.device
+            and not (kc.requires_grad or vc.requires_grad)
+            and all(c.stride(3) == 1 and c.stride(2) == hd and c.stride(0) % 8 == c.stride(1) % 8 == 0
+                    and c.data_ptr() % 16 == 0 for c in (kc, vc)))
+
+
+def cached_attention_usable(qkv, kc, vc, hd: int) -> bool:
+    """Whether :func:`cached_attention` takes these tensors: no gradient wanted, a 16-bit packed projection on a GPU and
+    usable caches."""
+    return (qkv.is_cuda and not (torch.is_grad_enabled() and qkv.requires_grad) and hd in (64, 128)
+            and qkv.dtype == _lib.lp_dtype() and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0
+            and caches_usable(qkv, kc, vc, hd))
+
+
+def cached_attention(qkv: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, past: int, b0: int, S: int, B: int, nh: int,
+                     ng: int, hd: int, cos: torch.Tensor | None = None, sin: torch.Tensor | None = None,
+                     interleaved: bool = False) -> torch.Tensor:
+    """One cached forward of ``S`` new tokens (no gradient): rotates the queries of the packed ``qkv [S*B, P]`` in place,
+    writes the rotated keys and the values behind the ``past`` cached ones (``kc`` / ``vc`` ``[max_seq, max_batch, ng,
+    hd]``, sequences ``b0 ..``) and attends causally to everything cached.  Returns ``[S, B, nh*hd]``."""
+    lib = _lib.load()
+    qpg, P = nh // ng, qkv.shape[1]
+    kn, vn = kc[past:, b0:], vc[past:, b0:]
+    rc = lib.hg_rope_append(qkv.data_ptr(), S * B, B, ng, qpg, hd, past, _lib.ptr(cos), _lib.ptr(sin),
+                            2 * cos.shape[1] if cos is not None else 0, int(interleaved), kn.data_ptr(), vn.data_ptr(),
+                            kc.stride(0), kc.stride(1), vc.stride(0), vc.stride(1), _lib.stream())
+    _lib.check(rc, "hg_rope_append")
+    _lib.count_launch()
+    out = torch.empty((S, B, nh * hd), dtype=qkv.dtype, device=qkv.device)
+    lse = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
+    k, v = kc[:, b0:], vc[:, b0:]
+    _forward_launch(_desc(qkv, B * P, P, nh + 2 * ng, qpg + 2, 1, 0), _desc(k, k.stride(0), k.stride(1), ng, 1, 0, 0),
+                    _desc(v, v.stride(0), v.stride(1), ng, 1, 0, 0), _desc(out, B * nh * hd, nh * hd, nh, qpg, 1, 0), lse,
+                    S, past + S, B, nh, ng, hd, True, past, 0, 1.0 / math.sqrt(hd))
+    return out
+
+
 class _Flash(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, causal, scale, q_pos0, k_pos0):
-        lib = _lib.load()
         S, B, nh, hd = q.shape
         Skv, ng = k.shape[0], k.shape[2]
         qpg = nh // ng
@@ -134,10 +193,7 @@ class _Flash(torch.autograd.Function):
         kd = _desc(k, k.stride(0), k.stride(1), ng, 1, 0, 0)
         vd = _desc(v, v.stride(0), v.stride(1), ng, 1, 0, 0)
         od = _desc(out, out.stride(0), out.stride(1), nh, qpg, 1, 0)
-        rc = lib.hg_flash_fwd(ctypes.byref(qd), ctypes.byref(kd), ctypes.byref(vd), ctypes.byref(od), lse.data_ptr(),
-                              S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0, float(scale), _lib.stream())
-        _lib.check(rc, "hg_flash_fwd")
-        _lib.count_launch()
+        _forward_launch(qd, kd, vd, od, lse, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, scale)
         ctx.save_for_backward(q, k, v, out, lse)
         ctx.cfg = (causal, scale, q_pos0, k_pos0)
         ctx.mark_non_differentiable(lse)
