@@ -300,7 +300,7 @@ class SelfAttention(nn.Module):
         if c.sp_size > 1 or c.cp_size > 1:
             raise NotImplementedError("cached attention needs sp = cp = 1")
         kc, vc, past, b0, cos, sin = self.cache_for(ic, qkv2, S_new, B)
-        if ops.attention.cached_attention_usable(qkv2, kc, vc, self.hd):
+        if ops.attention.cached_attention_usable(qkv2, kc, vc, past, S_new, b0, B, self.ng, self.hd):
             return ops.attention.cached_attention(qkv2, kc, vc, past, b0, S_new, B, self.nh, self.ng, self.hd, cos, sin,
                                                   s.rope_interleaved)
         if s.pos == "rope":

@@ -141,21 +141,24 @@ def _forward_launch(q, k, v, o, lse, S, Skv, B, nh, ng, hd, causal, q_pos0, k_po
     _lib.count_launch()
 
 
-def caches_usable(like: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, hd: int) -> bool:
-    """Whether the kernels can write to and read from these caches ``[max_seq, max_batch, ng, hd]``: ``like``'s dtype and
-    device, contiguous heads, whole 16-byte groups, and no gradient recorded through them."""
-    return (kc.dtype == vc.dtype == like.dtype and kc.device == vc.device == like.device
+def caches_usable(like: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, past: int, S: int, b0: int, B: int, ng: int,
+                  hd: int) -> bool:
+    """Whether the kernels can write ``S`` tokens of ``B`` sequences behind ``past`` cached ones to these caches
+    ``[max_seq, max_batch, ng, hd]`` and read them: ``like``'s dtype and device, room for the tokens, contiguous heads,
+    whole 16-byte groups, elements that do not share memory, and no gradient recorded through them."""
+    return (past >= 0 and b0 >= 0 and kc.dtype == vc.dtype == like.dtype and kc.device == vc.device == like.device
             and not (kc.requires_grad or vc.requires_grad)
-            and all(c.stride(3) == 1 and c.stride(2) == hd and c.stride(0) % 8 == c.stride(1) % 8 == 0
-                    and c.data_ptr() % 16 == 0 for c in (kc, vc)))
+            and all(c.dim() == 4 and c.shape[0] >= past + S and c.shape[1] >= b0 + B and c.shape[2:] == (ng, hd)
+                    and c.stride(3) == 1 and c.stride(2) == hd and min(c.stride(0), c.stride(1)) >= ng * hd
+                    and c.stride(0) % 8 == c.stride(1) % 8 == 0 and c.data_ptr() % 16 == 0 for c in (kc, vc)))
 
 
-def cached_attention_usable(qkv, kc, vc, hd: int) -> bool:
+def cached_attention_usable(qkv, kc, vc, past: int, S: int, b0: int, B: int, ng: int, hd: int) -> bool:
     """Whether :func:`cached_attention` takes these tensors: no gradient wanted, a 16-bit packed projection on a GPU and
     usable caches."""
     return (qkv.is_cuda and not (torch.is_grad_enabled() and qkv.requires_grad) and hd in (64, 128)
             and qkv.dtype == _lib.lp_dtype() and qkv.is_contiguous() and qkv.data_ptr() % 16 == 0
-            and caches_usable(qkv, kc, vc, hd))
+            and caches_usable(qkv, kc, vc, past, S, b0, B, ng, hd))
 
 
 def cached_attention(qkv: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, past: int, b0: int, S: int, B: int, nh: int,
