@@ -1,0 +1,144 @@
+// One dense decoder layer of a cached forward (a decode step, or a short prompt), launched by a single native call:
+//
+//   n = norm(x);  qkv = n Wqkv^T;  rotate, append to the cache, attend;  a = ctx Wproj^T
+//   h = x + a;  out = h + act(norm(h) W1^T) W2^T
+//
+// The kernels are the ones the layer's modules launch one by one.  A decode step of a 7B-sized layer keeps the GPU busy
+// for about 100 us; eleven launches through the tensor library and the autograd wrappers took the host several times
+// that: a decode step of four 4096-wide layers, 4 sequences at 1000 cached positions, 1965 us launched one by one, 583
+// us from here with the attention kernels of flash_decode.cu (embedding, head and sampling included).  Host code
+// only.
+#include "attn_tensor.h"
+#include "sm100_common.cuh"
+
+extern "C" {
+
+int hg_norm_fwd(const void* x, const void* residual, const void* w, const void* b, void* y, void* h_out, void* rstd,
+                void* mean, int rows, int H, float eps, int rms, void* stream);
+int hg_gemm_skinny_bf16(const void* x, const void* W, void* C, const void* bias, int M, int N, int K, int ldx, int ldw,
+                        int ldc, int w_mn, int out_mode, int splits, void* stream);
+int hg_rope_append(void* qkv, int tokens, int batch, int ng, int qpg, int hd, int pos_offset, const void* cos_t,
+                   const void* sin_t, int rot_dim, int interleaved, void* kc, void* vc, long long k_ss, long long k_sb,
+                   long long v_ss, long long v_sb, void* stream);
+long long hg_flash_decode_scratch(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, int Sq, int Skv, int B,
+                                  int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0);
+int hg_flash_decode_pays(int Sq, int Skv, int B, int nheads, int causal, int q_pos0, int k_pos0);
+int hg_flash_decode(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o, void* lse,
+                    void* ws, int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0,
+                    float scale, void* stream);
+int hg_flash_fwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o, void* lse,
+                 int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0, float scale,
+                 void* stream);
+int hg_glu_fwd(const void* y, void* out, long long rows, int F, int kind, void* stream);
+int hg_add_bf16(const void* a, const void* b, void* out, long long n, void* stream);
+
+// Mirrored by ``DecoderStep`` in ops/_lib.py.  x and out are [S * B, H] contiguous (S tokens of B sequences, S * B <= 128);
+// the caches point at the first of the B sequences, position 0, and `past` positions of them are filled.
+struct HgDecoderStep {
+  int S, B, H, nh, ng, hd, F, past;
+  int rms, act, rot_dim, interleaved;      // act: kind of hg_glu_fwd; rot_dim 0: no rotation
+  float eps, scale;
+  const void *w_norm1, *b_norm1, *w_qkv, *b_qkv, *w_proj, *b_proj;
+  const void *w_norm2, *b_norm2, *w_fc1, *b_fc1, *w_fc2, *b_fc2;
+  const void *cos_t, *sin_t;
+  void *k_cache, *v_cache;
+  long long k_ss, k_sb, v_ss, v_sb;
+  const void* x;
+  void* out;
+  void* ws;
+  long long ws_bytes;
+};
+
+}  // extern "C"
+
+namespace {
+
+struct Buffers {
+  char *norm, *qkv, *ctx, *attn, *h, *fc1, *act, *mlp, *rstd, *mean, *lse, *part;
+  long long bytes, part_floats;
+};
+
+HgAttnTensor packed(const HgDecoderStep& d, void* base, int qpg, bool query) {
+  const long long P = (long long)(d.nh + 2 * d.ng) * d.hd;
+  return {base, d.B * P, P, d.nh + 2 * d.ng, qpg + 2, query ? 1 : 0, query ? 0 : qpg};
+}
+
+// Carves the scratch; every buffer starts on a 256-byte boundary.
+Buffers carve(const HgDecoderStep& d, char* base) {
+  Buffers b{};
+  long long at = 0;
+  auto take = [&](long long bytes) {
+    char* p = base + at;
+    at += (bytes + 255) / 256 * 256;
+    return p;
+  };
+  const long long T = (long long)d.S * d.B, lp = sizeof(hg_lp_t);
+  const int qpg = d.nh / d.ng;
+  b.norm = take(T * d.H * lp);
+  b.qkv = take(T * (d.nh + 2 * d.ng) * d.hd * lp);
+  b.ctx = take(T * d.nh * d.hd * lp);
+  b.attn = take(T * d.H * lp);
+  b.h = take(T * d.H * lp);
+  b.fc1 = take(T * d.F * (d.act == 2 ? 1 : 2) * lp);
+  b.act = take(T * d.F * lp);
+  b.mlp = take(T * d.H * lp);
+  b.rstd = take(T * 4);
+  b.mean = take(T * 4);
+  b.lse = take(T * d.nh * 4);
+  const HgAttnTensor q = packed(d, b.qkv, qpg, true), k{d.k_cache, d.k_ss, d.k_sb, d.ng, 1, 0, 0},
+                     v{d.v_cache, d.v_ss, d.v_sb, d.ng, 1, 0, 0};
+  b.part_floats = hg_flash_decode_pays(d.S, d.past + d.S, d.B, d.nh, 1, d.past, 0)
+                      ? hg_flash_decode_scratch(&q, &k, &v, d.S, d.past + d.S, d.B, d.nh, d.ng, d.hd, 1, d.past, 0) : -1;
+  b.part = take(b.part_floats > 0 ? b.part_floats * 4 : 0);
+  b.bytes = at;
+  return b;
+}
+
+bool valid(const HgDecoderStep& d) {
+  return d.S > 0 && d.B > 0 && (long long)d.S * d.B <= 128 && d.H > 0 && d.ng > 0 && d.nh > 0 && d.nh % d.ng == 0 &&
+         d.F > 0 && d.past >= 0 && d.act >= 0 && d.act <= 2 && (d.hd == 64 || d.hd == 128);
+}
+
+}  // namespace
+
+extern "C" {
+
+// Bytes of scratch (256-byte aligned) that hg_decoder_step needs, or -1 for a layer it does not take.
+long long hg_decoder_step_scratch(const HgDecoderStep* d) {
+  if (!valid(*d)) return -1;
+  char dummy alignas(256)[1];
+  return carve(*d, dummy).bytes;
+}
+
+int hg_decoder_step(const HgDecoderStep* dp, void* stream) {
+  const HgDecoderStep& d = *dp;
+  if (!valid(d)) return -1;
+  const Buffers b = carve(d, static_cast<char*>(d.ws));
+  if (b.bytes > d.ws_bytes) return -1;
+  const int T = d.S * d.B, qpg = d.nh / d.ng, P = (d.nh + 2 * d.ng) * d.hd, C = d.nh * d.hd;
+  const int F1 = d.F * (d.act == 2 ? 1 : 2);
+  void* mean = d.rms ? nullptr : b.mean;
+  int rc;
+  if ((rc = hg_norm_fwd(d.x, nullptr, d.w_norm1, d.b_norm1, b.norm, nullptr, b.rstd, mean, T, d.H, d.eps, d.rms, stream))) return rc;
+  if ((rc = hg_gemm_skinny_bf16(b.norm, d.w_qkv, b.qkv, d.b_qkv, T, P, d.H, d.H, d.H, P, 0, 0, 0, stream))) return rc;
+  const size_t lp = sizeof(hg_lp_t);
+  if ((rc = hg_rope_append(b.qkv, T, d.B, d.ng, qpg, d.hd, d.past, d.cos_t, d.sin_t, d.rot_dim, d.interleaved,
+                           static_cast<char*>(d.k_cache) + size_t(d.past) * d.k_ss * lp,
+                           static_cast<char*>(d.v_cache) + size_t(d.past) * d.v_ss * lp, d.k_ss, d.k_sb, d.v_ss, d.v_sb,
+                           stream))) return rc;
+  const HgAttnTensor q = packed(d, b.qkv, qpg, true), k{d.k_cache, d.k_ss, d.k_sb, d.ng, 1, 0, 0},
+                     v{d.v_cache, d.v_ss, d.v_sb, d.ng, 1, 0, 0}, o{b.ctx, (long long)d.B * C, C, d.nh, qpg, 1, 0};
+  if (b.part_floats >= 0)
+    rc = hg_flash_decode(&q, &k, &v, &o, b.lse, b.part, d.S, d.past + d.S, d.B, d.nh, d.ng, d.hd, 1, d.past, 0, d.scale, stream);
+  else
+    rc = hg_flash_fwd(&q, &k, &v, &o, b.lse, d.S, d.past + d.S, d.B, d.nh, d.ng, d.hd, 1, d.past, 0, d.scale, stream);
+  if (rc) return rc;
+  if ((rc = hg_gemm_skinny_bf16(b.ctx, d.w_proj, b.attn, d.b_proj, T, d.H, C, C, C, d.H, 0, 0, 0, stream))) return rc;
+  if ((rc = hg_norm_fwd(b.attn, d.x, d.w_norm2, d.b_norm2, b.norm, b.h, b.rstd, mean, T, d.H, d.eps, d.rms, stream))) return rc;
+  if ((rc = hg_gemm_skinny_bf16(b.norm, d.w_fc1, b.fc1, d.b_fc1, T, F1, d.H, d.H, d.H, F1, 0, 0, 0, stream))) return rc;
+  if ((rc = hg_glu_fwd(b.fc1, b.act, T, d.F, d.act, stream))) return rc;
+  if ((rc = hg_gemm_skinny_bf16(b.act, d.w_fc2, b.mlp, d.b_fc2, T, d.H, d.F, d.F, d.F, d.H, 0, 0, 0, stream))) return rc;
+  return hg_add_bf16(b.h, b.mlp, d.out, (long long)T * d.H, stream);
+}
+
+}  // extern "C"

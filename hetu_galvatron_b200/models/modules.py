@@ -500,7 +500,64 @@ class GalvatronDecoderLayer(nn.Module):
         self.ffn.reset_parameters(seed, full_init)
 
     def forward(self, x):
+        if self.attn.attention.inference_context is not None and self._takes_native_step(x):
+            return self._native_step(x)
         return self.ffn(self.attn(x), x)
+
+    def _takes_native_step(self, x) -> bool:
+        """A cached forward of few tokens whose kernels one native call can launch (csrc/sm100/decoder_step.cu): no
+        gradient, no parallelism inside the layer, nothing hooked into it, 16-bit contiguous tensors on one GPU."""
+        import torch.nn.modules.module as tm
+
+        from ..ops import _lib
+        from ..ops.gemm import NATIVE_STEP_ROWS, _PAIR_MODE
+
+        att, mlp, c = self.attn.attention, self.ffn.mlp, self.ctx
+        s = att.spec
+        F1 = mlp.Fl * (2 if s.gated else 1)
+        mods = (self, self.attn, self.attn.input_layernorm, att, self.ffn, self.ffn.post_attention_layernorm, mlp)
+        return (x.is_cuda and not torch.is_grad_enabled() and x.dtype == _lib.lp_dtype() and x.is_contiguous()
+                and _PAIR_MODE != "1" and x.dim() == 3 and x.shape[2] == s.hidden
+                and att.linear_qkv.weight.shape == ((att.nh + 2 * att.ng) * att.hd, s.hidden)
+                and att.linear_proj.weight.shape == (s.hidden, att.nh * att.hd)
+                and mlp.linear_fc1.weight.shape == (F1, s.hidden) and mlp.linear_fc2.weight.shape == (s.hidden, mlp.Fl)
+                and x.data_ptr() % 16 == 0 and 0 < x.shape[0] * x.shape[1] <= NATIVE_STEP_ROWS
+                and c.tp_size == c.sp_size == c.cp_size == 1
+                and att.q_layernorm is None and att.hd in (64, 128) and att.hd * att.nh % 8 == 0
+                and not (s.hidden_dropout > 0.0 and self.training)
+                and all(p.dtype == x.dtype and p.device == x.device and p.is_contiguous() and p.data_ptr() % 16 == 0
+                        for p in self.parameters())
+                and not any(m._forward_hooks or m._forward_pre_hooks for m in mods[1:])
+                and not (tm._global_forward_hooks or tm._global_forward_pre_hooks))
+
+    def _native_step(self, x):
+        import ctypes
+
+        from ..ops import _lib
+        from ..ops.fused import _KIND
+
+        att, mlp = self.attn.attention, self.ffn.mlp
+        s, ic = att.spec, att.inference_context
+        S, B, H = x.shape
+        kc, vc, past, b0, cos, sin = att.cache_for(ic, x, S, B)
+        if not ops.attention.caches_usable(x, kc, vc, past, S, b0, B, att.ng, att.hd):
+            return self.ffn(self.attn(x), x)
+        n1, n2 = self.attn.input_layernorm, self.ffn.post_attention_layernorm
+        out = torch.empty_like(x)
+        d = _lib.DecoderStep(
+            S, B, H, att.nh, att.ng, att.hd, mlp.Fl, past, int(n1.rms), _KIND[s.activation],
+            2 * cos.shape[1] if cos is not None else 0, int(s.rope_interleaved), n1.eps, 1.0 / math.sqrt(att.hd),
+            *[_lib.ptr(t) for t in (n1.weight, n1.bias, att.linear_qkv.weight, att.linear_qkv.bias, att.linear_proj.weight,
+                                    att.linear_proj.bias, n2.weight, n2.bias, mlp.linear_fc1.weight, mlp.linear_fc1.bias,
+                                    mlp.linear_fc2.weight, mlp.linear_fc2.bias, cos, sin, kc[:, b0:], vc[:, b0:])],
+            kc.stride(0), kc.stride(1), vc.stride(0), vc.stride(1), x.data_ptr(), out.data_ptr())
+        lib = _lib.load()
+        d.ws_bytes = lib.hg_decoder_step_scratch(ctypes.byref(d))
+        ws = torch.empty(max(d.ws_bytes, 1), dtype=torch.uint8, device=x.device)
+        d.ws = ws.data_ptr()
+        _lib.check(lib.hg_decoder_step(ctypes.byref(d), _lib.stream()), "hg_decoder_step")
+        _lib.count_launch(11)
+        return out
 
 
 class GalvatronEmbedding(nn.Module):

@@ -60,7 +60,20 @@ class AttnTensor(ctypes.Structure):
                 ("off", c_int)]
 
 
+class DecoderStep(ctypes.Structure):
+    """Mirror of ``HgDecoderStep`` in csrc/sm100/decoder_step.cu."""
+
+    _fields_ = ([(n, c_int) for n in ("S", "B", "H", "nh", "ng", "hd", "F", "past", "rms", "act", "rot_dim",
+                                      "interleaved")] + [("eps", c_float), ("scale", c_float)] +
+                [(n, c_void_p) for n in ("w_norm1", "b_norm1", "w_qkv", "b_qkv", "w_proj", "b_proj", "w_norm2", "b_norm2",
+                                         "w_fc1", "b_fc1", "w_fc2", "b_fc2", "cos_t", "sin_t", "k_cache", "v_cache")] +
+                [(n, c_ll) for n in ("k_ss", "k_sb", "v_ss", "v_sb")] +
+                [("x", c_void_p), ("out", c_void_p), ("ws", c_void_p), ("ws_bytes", c_ll)])
+
+
 _SIGNATURES = {
+    "hg_decoder_step_scratch": [ctypes.POINTER(DecoderStep)],
+    "hg_decoder_step": [ctypes.POINTER(DecoderStep), c_void_p],
     "hg_gemm_bf16": [c_void_p] * 4 + [c_int] * 10 + [c_void_p],
     "hg_gemm2_bf16": [c_void_p] * 4 + [c_int] * 10 + [c_void_p],
     "hg_gemm_skinny_bf16": [c_void_p] * 4 + [c_int] * 9 + [c_void_p],
@@ -158,7 +171,8 @@ def load():
             continue
         fn.argtypes = argtypes
         fn.restype = c_int
-    lib.hg_flash_decode_scratch.restype = c_ll
+    for name in ("hg_flash_decode_scratch", "hg_decoder_step_scratch"):
+        getattr(lib, name).restype = c_ll
     if hasattr(lib, "hg_status_address"):
         lib.hg_status_address.restype = c_void_p
         lib.hg_status_address.argtypes = []
@@ -180,7 +194,9 @@ def ptr(t):
 
 
 def stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream's handle (the raw getter: building a ``torch.cuda.Stream`` per launch costs more host time than
+    the rest of a short launch)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 _STATUS_NAMES = {0: "ok", 1: "timeout: smem stage never filled", 2: "timeout: smem stage never freed",

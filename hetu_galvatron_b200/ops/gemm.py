@@ -38,6 +38,11 @@ _PAIR_MODE = os.environ.get("HG_GEMM_PAIR", "auto")
 _pair_ok = True
 
 
+# Rows up to which every product of a decoder layer runs on the weight-streaming kernel, whatever its width
+# (csrc/sm100/decoder_step.cu launches such a layer in one call).
+NATIVE_STEP_ROWS = 64
+
+
 def _use_skinny(M: int, N: int, a_mn: bool, out_mode: int, max_ctas: int, pair) -> bool:
     """Whether the weight-streaming kernel (csrc/sm100/gemm_skinny.cu) takes the product.  Up to 64 rows it was at least
     as fast everywhere (4 rows, cold: 4096 x 4096 16 us against 35 for the one-CTA kernel, 4096 x 11008 29 against 78,
@@ -45,7 +50,7 @@ def _use_skinny(M: int, N: int, a_mn: bool, out_mode: int, max_ctas: int, pair) 
     columns 25 against 35 us, 11008 columns 45 against 43, 152064 columns 221 against 207)."""
     if a_mn or out_mode not in (OUT_BF16, OUT_F32) or pair is not None or max_ctas != 0 or _PAIR_MODE == "1":
         return False
-    return M <= 64 or (M <= 128 and N <= 8192)
+    return M <= NATIVE_STEP_ROWS or (M <= 128 and N <= 8192)
 
 
 def _use_pair(M: int, N: int, pair) -> bool:

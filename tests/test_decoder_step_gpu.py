@@ -1,0 +1,60 @@
+"""A decoder layer launched by one native call against the same layer run module by module."""
+import pytest
+import torch
+
+from hetu_galvatron_b200.models.inference import StaticInferenceContext
+from hetu_galvatron_b200.models.modules import GalvatronDecoderLayer
+from hetu_galvatron_b200.models.spec import LayerCtx, ModelSpec
+from hetu_galvatron_b200.ops import _lib
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def layer(norm, act, pos, bias, nh, ng, hd):
+    spec = ModelSpec(family="llama", hidden=nh * hd, layers=1, heads=nh, kv_heads=ng, head_dim=hd, ffn=264, vocab=512,
+                     padded_vocab=512, seq_len=0, norm=norm, activation=act, pos=pos, bias=bias, qkv_bias=bias)
+    m = GalvatronDecoderLayer(spec, LayerCtx(), DEV, "layer")
+    m.reset_parameters()
+    with torch.no_grad():
+        for p in m.parameters():
+            if p.dim() == 1:
+                p.add_(0.1 * torch.randn_like(p))
+    return m
+
+
+# one row and the most that the native call takes; grouped heads on both head dims; biases; no rotation; a cache whose
+# first sequences belong to others
+@pytest.mark.parametrize("norm,act,pos,bias,nh,ng,hd", [("RMSNorm", "swiglu", "rope", False, 4, 2, 128),
+                                                        ("LayerNorm", "gelu", "none", True, 6, 6, 64),
+                                                        ("RMSNorm", "geglu", "rope", True, 8, 1, 64)])
+@pytest.mark.parametrize("S,B,past,b0", [(1, 1, 0, 0), (1, 4, 70, 2), (16, 4, 5, 0)])
+def test_native_step_equals_the_modules(norm, act, pos, bias, nh, ng, hd, S, B, past, b0):
+    torch.manual_seed(S + B)
+    m = layer(norm, act, pos, bias, nh, ng, hd)
+    x = torch.randn(S, B, nh * hd, device=DEV).to(torch.bfloat16)
+    caches = torch.randn(2, past + S + 3, b0 + B + 1, ng, hd, device=DEV).to(torch.bfloat16)
+    got = []
+    for hooked in (False, True):                      # a hook inside the layer sends it module by module
+        ic = StaticInferenceContext(b0 + B + 1, past + S + 3)
+        ic.sequence_len_offset, ic.batch_size_offset = past, b0
+        mine = caches.clone()
+        ic.key_value_memory_dict[0] = (mine[0], mine[1])
+        m.attn.attention.inference_context = ic
+        h = m.ffn.mlp.register_forward_hook(lambda *_: None) if hooked else None
+        with torch.no_grad():
+            assert m._takes_native_step(x) is not hooked
+            got.append((m(x), mine))
+        if h is not None:
+            h.remove()
+        m.attn.attention.inference_context = None
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    _lib.assert_healthy()
+
+
+def test_native_step_is_left_to_inference_without_gradient():
+    m = layer("RMSNorm", "swiglu", "rope", False, 4, 4, 64)
+    x = torch.randn(65, 1, 256, device=DEV).to(torch.bfloat16)
+    with torch.no_grad():
+        assert not m._takes_native_step(x) and m._takes_native_step(x[:64].contiguous())
+    assert not m._takes_native_step(x[:1])
