@@ -1156,7 +1156,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
 // =================================================================================================
 // Backward, part 1 with 128-query steps and the probabilities kept in tensor memory (both head dims; gpt2-xl sized,
-// 8 x 1024 x 25 heads of 64: 170 -> 144 us against the 64-query kernel).
+// 8 x 1024 x 25 heads of 64: 170 -> 152 us against the 64-query kernel).
 // The 64-query version issues its score products with N = 64, which occupy the tensor core as long as N = 128 would,
 // and stages P^T / dS^T through 64 KB of shared memory.  Here a step covers 128 queries:
 //   S^T = K Q^T and dP^T = V dO^T are 128 x 128 products (8 MMAs each);
