@@ -5,7 +5,8 @@
 // each.  What bounds a decode step is reading K and V once, so here a CTA takes one kv head, CH keys and the (at most
 // eight) query rows that attend to them; the key ranges of a sequence are spread over the chip and their partial
 // results merged by a second small kernel (skipped when one range covers all keys).  Scores and probabilities stay in
-// fp32 throughout.
+// fp32 throughout.  A row that sees no key (its sum l is 0) is written as zeros; a NaN score or one of +inf makes l, and with
+// it the row of O, NaN (LSE -inf), as on the tile kernels.
 //
 // Rows: r = s * qpg + j is query token s of query head g * qpg + j.  A lane holds eight channels, so HD / 8 lanes share a
 // key and a warp reads 32 / (HD / 8) keys per 16-byte access.
@@ -168,7 +169,7 @@ flash_decode_kernel(const DecodeParams p) {
     const float m = sML[r][0], l = sML[r][1];
     if (ranges == 1) {
       const int h = g * p.qpg + r % p.qpg, s = r / p.qpg;
-      p.O[int64_t(s) * p.o_ss + int64_t(b) * p.o_sb + int64_t(h) * HD + c] = hg_f2lp(l > 0.f ? v / l : 0.f);
+      p.O[int64_t(s) * p.o_ss + int64_t(b) * p.o_sb + int64_t(h) * HD + c] = hg_f2lp(l == 0.f ? 0.f : v / l);
       if (c == 0) p.LSE[(size_t(b) * p.nheads + h) * p.Sq + s] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
     } else {
       float* w = p.ws + ((int64_t(b) * p.nkv + g) * rows + r) * int64_t(ranges) * (HD + 2) + int64_t(blockIdx.z) * (HD + 2);
@@ -201,7 +202,7 @@ flash_decode_merge_kernel(const DecodeParams p, int ranges) {
     l = fmaf(f, wi[HD + 1], l);
   }
   const int h = g * p.qpg + r % p.qpg, s = r / p.qpg;
-  p.O[int64_t(s) * p.o_ss + int64_t(b) * p.o_sb + int64_t(h) * HD + c] = hg_f2lp(l > 0.f ? v / l : 0.f);
+  p.O[int64_t(s) * p.o_ss + int64_t(b) * p.o_sb + int64_t(h) * HD + c] = hg_f2lp(l == 0.f ? 0.f : v / l);
   if (c == 0) p.LSE[(size_t(b) * p.nheads + h) * p.Sq + s] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
 }
 

@@ -53,6 +53,42 @@ def test_flash_decode(hd, Sq, B, nh, ng, Skv, causal, q0, k0):
     _lib.assert_healthy()
 
 
+# a NaN in a query, in one key that the row sees, in a key that it does not see; a score of +inf; -inf scores only.  One key
+# range (40 keys) and several, whose first holds the bad key
+@pytest.mark.parametrize("Skv", [40, 300])
+@pytest.mark.parametrize("qpg", [1, 4])
+@pytest.mark.parametrize("what", ["query", "key", "unseen", "inf", "-inf"])
+def test_flash_decode_passes_nan_and_inf_on(Skv, qpg, what):
+    """Bad scores reach the output as on the tile kernel."""
+    B, ng, hd = 2, 2, 64
+    g = torch.Generator(device=DEV).manual_seed(Skv + qpg)
+    q = torch.randn(1, B, ng * qpg, hd, device=DEV, generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(Skv, B, ng, hd, device=DEV, generator=g).to(torch.bfloat16) for _ in "kv")
+    q0 = Skv - 1
+    if what == "query":
+        q[0, 1, 0, 3] = float("nan")
+    elif what == "unseen":
+        q0, k[-1, 1, 0, 3] = Skv - 2, float("nan")
+    else:
+        q[0, 1, :, 3] = 1.0
+        k[slice(None) if what == "-inf" else 7, 1, 0, 3] = float("nan") if what == "key" else float(what)
+    got = []
+    for spread in (True, False):
+        out, lse = torch.empty_like(q), torch.empty(B, ng * qpg, 1, device=DEV)
+        d = [_desc(t, t.stride(0), t.stride(1), t.shape[2], n, 1, 0) for t, n in ((q, qpg), (k, 1), (v, 1), (out, qpg))]
+        d[1].hs = d[2].hs = 0
+        _forward_launch(*d, lse, 1, Skv, B, ng * qpg, ng, hd, True, q0, 0, 1.0 / math.sqrt(hd), spread=spread)
+        got.append((out, lse))
+    bad = {"query": 1, "key": qpg, "inf": qpg}.get(what, 0)          # query heads whose output has to be NaN
+    for out, _ in got:
+        assert out[0, 1, :bad].isnan().all() and out[0, 1, bad:].isfinite().all() and out[0, 0].isfinite().all()
+    live = got[0][0].isfinite()
+    assert torch.equal(live, got[1][0].isfinite())
+    assert torch.allclose(got[0][0][live].double(), got[1][0][live].double(), rtol=2e-2, atol=2e-2)   # 16-bit probabilities there
+    assert torch.equal(got[0][1].isfinite(), got[1][1].isfinite())
+    _lib.assert_healthy()
+
+
 @pytest.mark.parametrize("interleaved,rot", [(False, 1.0), (True, 1.0), (False, 0.5), (True, 0.25), (False, 0.0)])
 @pytest.mark.parametrize("S,B,nh,ng,hd,past", [(1, 4, 4, 4, 128, 70), (5, 2, 8, 2, 64, 3), (130, 1, 4, 1, 128, 0)])
 def test_cached_attention_against_rope_and_copies(S, B, nh, ng, hd, past, interleaved, rot):
