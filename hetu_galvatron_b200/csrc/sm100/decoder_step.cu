@@ -22,7 +22,7 @@ int hg_rope_append(void* qkv, int tokens, int batch, int ng, int qpg, int hd, in
                    long long v_ss, long long v_sb, void* stream);
 long long hg_flash_decode_scratch(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, int Sq, int Skv, int B,
                                   int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0);
-int hg_flash_decode_pays(int Sq, int Skv, int B, int nheads, int causal, int q_pos0, int k_pos0);
+int hg_flash_decode_pays(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0);
 int hg_flash_decode(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o, void* lse,
                     void* ws, int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0,
                     float scale, void* stream);
@@ -87,7 +87,7 @@ Buffers carve(const HgDecoderStep& d, char* base) {
   b.lse = take(T * d.nh * 4);
   const HgAttnTensor q = packed(d, b.qkv, qpg, true), k{d.k_cache, d.k_ss, d.k_sb, d.ng, 1, 0, 0},
                      v{d.v_cache, d.v_ss, d.v_sb, d.ng, 1, 0, 0};
-  b.part_floats = hg_flash_decode_pays(d.S, d.past + d.S, d.B, d.nh, 1, d.past, 0)
+  b.part_floats = hg_flash_decode_pays(d.S, d.past + d.S, d.B, d.nh, d.ng, d.hd, 1, d.past, 0)
                       ? hg_flash_decode_scratch(&q, &k, &v, d.S, d.past + d.S, d.B, d.nh, d.ng, d.hd, 1, d.past, 0) : -1;
   b.part = take(b.part_floats > 0 ? b.part_floats * 4 : 0);
   b.bytes = at;

@@ -260,12 +260,28 @@ long long hg_flash_decode_scratch(const HgAttnTensor* q, const HgAttnTensor* k, 
   return ranges > 1 ? (long long)B * nheads * Sq * ranges * (hd + 2) : 0;
 }
 
-// Whether spreading the keys beats the one-tile kernel.  That kernel takes a query head per CTA and walks its keys alone, so
-// it loses once its heads fill the chip or a head has many keys; below that its single launch wins over a launch and a
-// merge.  Measured, one query, head dim 128, cold (us, here against there): 4 sequences x 32 heads x 1000 keys 28 / 25, 1 x
-// 28 (4 kv heads) x 1000 23 / 21, 1 x 32 x 2000 24 / 33, 16 x 32 x 1000 65 / 79, 32 x 28 (4) x 2000 87 / 181.
-int hg_flash_decode_pays(int Sq, int Skv, int B, int nheads, int causal, int q_pos0, int k_pos0) {
-  return (long long)B * nheads > 148 || keys_seen(Sq, Skv, causal, q_pos0, k_pos0) >= 1536;
+// Whether spreading the keys beats the one-tile kernel.  That kernel gives a CTA all queries of one query head and walks
+// the head's keys alone: it loses when its heads leave part of the last wave of 148 idle, when a head has many keys, or
+// when query heads share a kv head and it reads those keys once for each.  It wins when a few queries of a head share its
+// one walk (here each is a row of its own), and below about 500 keys, where its single launch beats a launch and a merge.
+// Measured, us cold, here / there:
+//   one wave, 1 query   head dim 128: 32 heads (8 kv) x 2000 keys 24 / 32, 1000 24 / 20; 64 x 4000 48 / 54, 96 x 4000 62 / 57,
+//                       128 x 1536 36 / 31, 128 (32 kv) x 1536 28 / 27, x 2000 32 / 33; head dim 64: 128 x 1536 24 / 27
+//   two waves           head dim 128: 256 (64 kv) x 128 24 / 16, 512 24 / 26, 2000 46 / 60; 192 x 256 20 / 20, 384 25 / 22,
+//                       2000 54 / 66; 288 x 2000 75 / 72; head dim 64: 288 x 384 22 / 23, 2000 44 / 59
+//   three waves         head dim 128: 384 (96 kv) x 128 24 / 22, 192 26 / 29, 2000 64 / 86; 320 x 256 24 / 27, 2000 79 / 96
+//   more                head dim 128: 512 x 64 12 / 31, 1000 65 / 80; 1024 (256 kv) x 1000 62 / 119
+//   several queries     head dim 128: 4 x 192 heads x 2000 91 / 66, 8 x 512 x 2000 294 / 127; 2 x 320 (80 kv) x 2000 62 / 84
+int hg_flash_decode_pays(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
+  if (nkv < 1) return 0;
+  const long long heads = (long long)B * nheads;
+  const int keys = keys_seen(Sq, Skv, causal, q_pos0, k_pos0), qpg = nheads / nkv, rows = Sq * qpg;
+  if (Sq > 1 && qpg < 2 * Sq) return 0;
+  if (heads > 3 * 148) return 1;
+  if (heads > 2 * 148) return rows <= 2 || keys >= 192;
+  if (heads > 148) return rows > 2 ? keys >= 512 : rows == 2 || hd == 64 || keys <= 256 || (keys >= 512 && heads <= 224);
+  if (hd == 128 && rows == 1 && heads > 64) return 0;
+  return keys >= (hd == 128 && rows > 2 ? 2000 : 1536);
 }
 
 // Same contract as hg_flash_fwd for the calls that hg_flash_decode_scratch accepts; `ws` is its scratch.

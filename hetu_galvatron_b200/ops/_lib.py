@@ -127,7 +127,7 @@ _SIGNATURES = {
     "hg_scale": [c_void_p, c_ll, c_int, c_void_p, c_float, c_void_p],
     "hg_flash_fwd": [ctypes.POINTER(AttnTensor)] * 4 + [c_void_p] + [c_int] * 9 + [c_float, c_void_p],
     "hg_rope_append": [c_void_p] + [c_int] * 6 + [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p] + [c_ll] * 4 + [c_void_p],
-    "hg_flash_decode_pays": [c_int] * 7,
+    "hg_flash_decode_pays": [c_int] * 9,
     "hg_flash_decode_scratch": [ctypes.POINTER(AttnTensor)] * 3 + [c_int] * 9,
     "hg_flash_decode": [ctypes.POINTER(AttnTensor)] * 4 + [c_void_p, c_void_p] + [c_int] * 9 + [c_float, c_void_p],
     "hg_flash_bwd": [ctypes.POINTER(AttnTensor)] * 5 + [c_void_p, c_void_p] + [ctypes.POINTER(AttnTensor)] * 3 +

@@ -128,7 +128,7 @@ def _forward_launch(q, k, v, o, lse, S, Skv, B, nh, ng, hd, causal, q_pos0, k_po
     args = (S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0)
     refs = [ctypes.byref(t) for t in (q, k, v)]
     if spread is None:
-        spread = S * (nh // ng) <= 8 and lib.hg_flash_decode_pays(S, Skv, B, nh, int(causal), q_pos0, k_pos0)
+        spread = S * (nh // ng) <= 8 and lib.hg_flash_decode_pays(*args)
     need = lib.hg_flash_decode_scratch(*refs, *args) if spread else -1
     if need >= 0:
         ws = torch.empty(need, dtype=torch.float32, device=lse.device) if need else None
