@@ -5,7 +5,7 @@
 // What bounds it is reading W once from HBM, so the kernel is a weight streamer.  The roles of the operands are
 // swapped against the large-M kernels: 128 rows of W are the M side of the tcgen05 tile and the tokens, padded to
 // NT = 16, 32, 64 or 128, its N side, so that the tensor core does no more padded work than the token count needs
-// and a CTA's accumulator is only NT columns.  The contraction is cut over the S <= 8 CTAs of a cluster: a 4096 x 4096
+// and a CTA's accumulator is only NT columns.  A long contraction is cut over the S <= 8 CTAs of a cluster: a 4096 x 4096
 // weight has 32 row tiles, which keep 32 SMs busy, and 256 CTAs when each tile is shared by eight.  Two CTAs fit
 // an SM (at most 113 KB of shared memory each), which keeps about 200 KB of loads in flight per SM.  The partial
 // sums meet through distributed shared memory, added in rank order: no workspace, no atomics, the same bits every time.
@@ -276,13 +276,21 @@ template <bool W_MN, int NT>
 int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, int want_splits, cudaStream_t st) {
   const int tiles = (p.N + TM - 1) / TM, num_kb = (p.K + BK - 1) / BK;
   // The largest split whose clusters are all resident at once (they then share the memory bandwidth evenly and end
-  // together), as long as every CTA keeps at least four k-blocks to stream.
+  // together), or none where the contraction is too short for what the split costs, the partial tile's way through
+  // shared memory and M / splits rows added one after the other by each CTA: a split by two of a short contraction is the
+  // worst of both (64 rows, 512 columns, K = 512: 1, 2, 4, 8 CTAs a tile 8.8, 13.3, 10.8, 8.8 us; K = 1024: 10.8, 14.9, 10.8,
+  // 8.8; 8192 columns, four at most, K = 1024 14.1 alone, 14.9 by four, K = 2048 19.9, 17.8; 12288 columns, two at most,
+  // 4 rows, K = 2048 18.1 alone, 18.8 by two, K = 4096 29.0, 27.7).
   int splits = 1;
-  for (int s = kMaxSplits; s >= 1; --s) {
-    if (s > 1 && num_kb / s < 4) continue;
+  for (int s = kMaxSplits; s > 1; --s) {
+    if (num_kb * s < (s == 2 ? 128 : 96)) continue;
     int resident = 0;
     if (int rc = resident_clusters<W_MN, NT>(s, &resident)) return rc;
-    if (s == 1 || tiles <= resident) { splits = s; break; }
+    if (tiles <= resident) { splits = s; break; }
+  }
+  if (splits == 1) {                           // the first launch of a variant sets its shared memory limit here
+    int resident = 0;
+    if (int rc = resident_clusters<W_MN, NT>(1, &resident)) return rc;
   }
   if (want_splits > 0) splits = want_splits;
   cudaLaunchConfig_t cfg = {};

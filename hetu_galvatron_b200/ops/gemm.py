@@ -43,14 +43,16 @@ _pair_ok = True
 NATIVE_STEP_ROWS = 64
 
 
-def _use_skinny(M: int, N: int, a_mn: bool, out_mode: int, max_ctas: int, pair) -> bool:
-    """Whether the weight-streaming kernel (csrc/sm100/gemm_skinny.cu) takes the product.  Up to 64 rows it was at least
-    as fast everywhere (4 rows, cold: 4096 x 4096 16 us against 35 for the one-CTA kernel, 4096 x 11008 29 against 78,
-    152064 x 3584 176 against 208).  From 65 to 128 rows it pays for outputs of up to 64 of its tiles (128 rows: 4096
-    columns 25 against 35 us, 11008 columns 45 against 43, 152064 columns 221 against 207)."""
+def _use_skinny(M: int, N: int, K: int, a_mn: bool, out_mode: int, max_ctas: int, pair) -> bool:
+    """Whether the weight-streaming kernel (csrc/sm100/gemm_skinny.cu) takes the product.  Up to 64 rows it is as fast as
+    the one-CTA kernel or faster, by the microsecond that the timing resolves (4 rows, cold: 4096 x 4096 16 us against 35
+    for the one-CTA kernel, 4096 x 11008 29 against 78, 152064 x 3584 176 against 208; 64 rows: 512 x 512 8.8 against 9.2,
+    16384 columns x 1024 15.8 against 15.8).  From 65 to 128 rows it pays for long contractions of up to 64 of its tiles
+    (128 rows: 4096 columns, K = 1024 14.9 against 14.1, 1536 14.9 against 17.0, 4096 19.5 against 32.6; 8192 columns,
+    K = 2048 23.6 against 21.9, 3072 24.8 against 28.5; 16384 columns x 4096 41.5 against 39.5)."""
     if a_mn or out_mode not in (OUT_BF16, OUT_F32) or pair is not None or max_ctas != 0 or _PAIR_MODE == "1":
         return False
-    return M <= NATIVE_STEP_ROWS or (M <= 128 and N <= 8192)
+    return M <= NATIVE_STEP_ROWS or (M <= 128 and N <= 8192 and K >= (1536 if N <= 4096 else 3072))
 
 
 def _use_pair(M: int, N: int, pair) -> bool:
@@ -104,7 +106,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         if out.shape[0] != M or out.shape[1] != N or out.stride(1) != 1:
             raise ValueError("bad output tensor")
     lib = _lib.load()
-    if _use_skinny(M, N, a_mn, out_mode, max_ctas, pair):
+    if _use_skinny(M, N, K, a_mn, out_mode, max_ctas, pair):
         rc = lib.hg_gemm_skinny_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(bias), M, N, K, a.stride(0),
                                      b.stride(0), out.stride(0), int(b_mn), out_mode, 0, _lib.stream())
         if rc != 0:

@@ -34,6 +34,31 @@ def test_skinny_gemm(M, N, K, b_mn):
     _lib.assert_healthy()
 
 
+# contractions on both sides of the lengths from which eight CTAs (12 blocks of 64), four (24) and two (64) share a tile
+@pytest.mark.parametrize("N,K", [(512, 704), (512, 768), (520, 776), (8192, 1472), (8192, 1536), (12288, 4032), (12288, 4096)])
+@pytest.mark.parametrize("M", [4, 64, 128])
+def test_skinny_gemm_around_its_split_lengths(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    x = torch.randn(M, K, device=DEV, generator=g).to(torch.bfloat16)
+    w = torch.randn(N, K, device=DEV, generator=g).to(torch.bfloat16)
+    ref = x.double() @ w.double().t()
+    for s in (0, 1):                                                  # the rule's split, and none
+        out = torch.empty(M, N, device=DEV)
+        _lib.check(_lib.load().hg_gemm_skinny_bf16(x.data_ptr(), w.data_ptr(), out.data_ptr(), 0, M, N, K, K, K, N, 0, OUT_F32, s,
+                                                   _lib.stream()), "hg_gemm_skinny_bf16")
+        assert rel_err(out, ref) < 1e-5
+    _lib.assert_healthy()
+
+
+@pytest.mark.parametrize("M,N,K,few_rows", [(64, 512, 512, True), (65, 512, 512, False), (128, 4096, 1535, False),
+                                            (128, 4096, 1536, True), (128, 8192, 3064, False), (128, 8192, 3072, True),
+                                            (128, 8200, 4096, False), (129, 512, 4096, False)])
+def test_rule_of_the_few_row_kernel(M, N, K, few_rows):
+    from hetu_galvatron_b200.ops.gemm import OUT_BF16, _use_skinny
+
+    assert _use_skinny(M, N, K, False, OUT_BF16, 0, None) is few_rows
+
+
 def test_skinny_gemm_writes_only_its_rows_of_a_wider_output():
     M, N, K = 5, 200, 512
     x = torch.randn(M, K, device=DEV).to(torch.bfloat16)
