@@ -63,6 +63,16 @@ def _use_pair(M: int, N: int, pair) -> bool:
     return _PAIR_MODE == "1" or (M >= 256 and N >= 256)
 
 
+def _use_grouped_pair(rows: int, N: int, K: int, G: int) -> bool:
+    """Whether grouped products take the CTA-pair tile.  Its 256 rows are mostly padding for groups of one 128-row segment,
+    and the store of a 256 x 256 tile is hidden only under a long contraction, so it pays for groups of about 512 rows
+    and K from 2560 on.  Ragged groups, us, pair against one CTA: 8 x (128 rows, 28672 columns, K = 4096) 347 / 312, 512 rows
+    822 / 796, 1024 rows 1351 / 1554; 64 x (512, 2048, 1408) 220 / 177, 1024 rows 384 / 312; 64 x (1024, 2816, 2048) 615 / 605;
+    8 x (512, 4096, 2560) 87 / 89, 32 x (512, 4096, 3072) 323 / 333, 1024 rows 577 / 613.  (Weight gradients contract
+    over the rows and gain at every size: 64 x (128, 2816, 2048) 1206 / 1634.)"""
+    return _use_pair(rows, N, None) and (_PAIR_MODE == "1" or (rows >= 512 * G and K >= 2560))
+
+
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: torch.Tensor | None = None,
          out_mode: int = OUT_BF16, bias: torch.Tensor | None = None, max_ctas: int = 0, pair=None) -> torch.Tensor:
     """``C[M,N] = op(A) op(B)`` with fp32 accumulation.
@@ -217,7 +227,7 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, row_start: torch.Tensor, *, b
     lib = _lib.load()
     args = (a.data_ptr(), b2.data_ptr(), out.data_ptr(), row_start.data_ptr(), G, a.shape[0], N, K, a.stride(0),
             b2.stride(0), out.stride(0), int(b_mn), OUT_BF16, _lib.stream())
-    rc = lib.hg_grouped_gemm2_bf16(*args) if _use_pair(a.shape[0], N, None) else -2
+    rc = lib.hg_grouped_gemm2_bf16(*args) if _use_grouped_pair(a.shape[0], N, K, G) else -2
     if rc == -2:
         rc = lib.hg_grouped_gemm_bf16(*args)
     _lib.check(rc, "hg_grouped_gemm_bf16")

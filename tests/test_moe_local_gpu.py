@@ -79,3 +79,42 @@ def test_grouped_gemm_clears_the_rows_outside_its_segments():
     ref = torch.cat([a[128:256].double() @ b[0].double().t(), a[256:512].double() @ b[1].double().t()])
     assert ((out[128:512].double() - ref).norm() / ref.norm()).item() < 2.0 ** -8
     _lib.assert_healthy()
+
+
+# segments that end inside a block of 32 rows, an empty one, one row, more than a pair tile; ragged columns (a block of C
+# clipped at N) and a width that is no multiple of 16 bytes (no tensor map of C)
+@pytest.mark.parametrize("seg", [[77, 0, 301, 150], [1, 255, 257, 31], [300]])
+@pytest.mark.parametrize("N,K", [(264, 64), (512, 192), (260, 128)])
+@pytest.mark.parametrize("b_mn", [False, True])
+@pytest.mark.parametrize("pair", ["0", "1"])
+def test_grouped_gemm_of_ragged_segments(monkeypatch, seg, N, K, b_mn, pair):
+    import importlib
+
+    from hetu_galvatron_b200 import ops
+
+    if b_mn and N % 8:
+        pytest.skip("rows of an N-major operand are whole 16-byte groups")
+    monkeypatch.setattr(importlib.import_module("hetu_galvatron_b200.ops.gemm"), "_PAIR_MODE", pair)
+    g = torch.Generator(device=DEV).manual_seed(N + K + len(seg))
+    first, rows = 5, 5 + sum(seg) + 40                          # rows before and after the segments belong to nobody
+    starts = [first + sum(seg[:i]) for i in range(len(seg) + 1)]
+    a = torch.randn(rows, K, device=DEV, generator=g).to(torch.bfloat16)
+    b = torch.randn(len(seg), *((K, N) if b_mn else (N, K)), device=DEV, generator=g).to(torch.bfloat16)
+    whole = torch.full((rows + 2, N), 3.0, device=DEV, dtype=torch.bfloat16)
+    out = whole[1:rows + 1]
+    ops.grouped_gemm(a, b, torch.tensor(starts, device=DEV, dtype=torch.int32), b_mn=b_mn, out=out)
+    for i, n in enumerate(seg):
+        ref = a[starts[i]:starts[i + 1]].double() @ (b[i].double() if b_mn else b[i].double().t())
+        got = out[starts[i]:starts[i + 1]].double()
+        assert torch.allclose(got, ref, rtol=2.0 ** -8, atol=1e-4 * K ** 0.5)   # one rounding; fp32 sums of K products
+    out[first:starts[-1]] = 3.0
+    assert (whole == 3.0).all()
+    _lib.assert_healthy()
+
+
+@pytest.mark.parametrize("rows,N,K,G,pair", [(4096, 4096, 2560, 8, True), (4095, 4096, 2560, 8, False), (4096, 4096, 2552, 8, False),
+                                             (4096, 255, 4096, 8, False), (512, 256, 4096, 1, True)])
+def test_rule_of_the_grouped_pair_kernel(rows, N, K, G, pair):
+    from hetu_galvatron_b200.ops.gemm import _use_grouped_pair
+
+    assert _use_grouped_pair(rows, N, K, G) is pair
