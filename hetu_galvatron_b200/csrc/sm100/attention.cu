@@ -1909,9 +1909,8 @@ int make_map(CUtensorMap* out, const void* base, int hd, int slots, int S, int B
 // dK/dV kernel: 0 = 128-query steps with P^T / dS^T in tensor memory, 1 = 64-query steps staged
 // through shared memory (kept for side-by-side tests and timing).
 int g_dkv_variant = 0;
-// Forward kernel: 0 = two query tiles per CTA with P in tensor memory (sequences longer than one
-// tile; head dim 64, 8 x 1024 x 25 heads: 123 -> 93 us), 1 = one tile per CTA with P staged in shared memory (also
-// what single-tile calls use).
+// Forward kernel: 0 = the rule of two_tile_forward, 1 = one tile per CTA with P staged in shared memory, 2 = two query
+// tiles per CTA with P in tensor memory wherever a sequence is longer than one tile (1, 2: side-by-side tests and timing).
 int g_fwd_variant = 0;
 
 template <typename K>
@@ -1919,11 +1918,20 @@ int set_smem(K kernel, int bytes) {
   return int(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 
-// Sequences longer than one tile: two query tiles per CTA with P in tensor memory, both head dims.
+// Which calls take two query tiles per CTA: sequences longer than one tile.  With head dim 64 the one-tile kernel is the
+// faster one as long as all its CTAs run at once (heads x queries, us, two tiles / one: 1 x 4096 64 / 51, 12 x 512 18 / 14,
+// 12 x 1536 33 / 27, 48 x 384 16 / 16; beyond a wave 12 x 2048 39 / 41, 25 x 1024 27 / 31, 48 x 512 20 / 22, 74 x 257 16 / 22,
+// 200 x 1024 98 / 127).
+template <int HD>
+bool two_tile_forward(const FwdParams& p) {
+  if (p.Sq <= 128 || g_fwd_variant == 1) return false;
+  return HD == 128 || g_fwd_variant == 2 || (long long)((p.Sq + 127) / 128) * p.nheads * p.B > 148;
+}
+
 template <int HD>
 int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const FwdParams& p, cudaStream_t st) {
   int rc;
-  if (p.Sq > 128 && g_fwd_variant == 0) {
+  if (two_tile_forward<HD>(p)) {
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(flash_fwd2_kernel<HD>, Fwd2Smem<HD>::kTotal))) return rc; cfg = true; }
     const dim3 grid((p.Sq + 255) / 256, p.nheads, p.B);
@@ -1994,7 +2002,7 @@ int hg_flash_fwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTenso
 // Selects the forward kernel (see g_fwd_variant); returns the previous value.
 int hg_attn_set_fwd_variant(int v) {
   const int old = g_fwd_variant;
-  g_fwd_variant = v ? 1 : 0;
+  g_fwd_variant = v == 1 || v == 2 ? v : 0;
   return old;
 }
 

@@ -43,3 +43,27 @@ def test_head_dim_64(S, B, nh, ng, causal):
     assert rel_err(out, o1) < 4e-3 and torch.allclose(lse, l1, rtol=1e-5, atol=1e-5)
     assert rel_err(dk, dk1) < 5e-3 and rel_err(dv, dv1) < 5e-3
     _lib.assert_healthy()
+
+
+# one partly filled second tile, whole pairs of tiles, a last pair with one tile, and the edge of the rule (148 one-tile CTAs)
+@pytest.mark.parametrize("S,B,nh,ng", [(129, 1, 2, 2), (256, 2, 3, 1), (384, 1, 4, 2), (700, 1, 2, 2), (256, 1, 74, 74), (256, 1, 75, 75)])
+@pytest.mark.parametrize("causal", [True, False])
+def test_forward_kernels_of_head_dim_64(S, B, nh, ng, causal):
+    """Two query tiles per CTA, one, and what the rule takes."""
+    g = torch.Generator(device=DEV).manual_seed(S + nh)
+    q, k, v = (torch.randn(S, B, n, 64, device=DEV, generator=g).to(torch.bfloat16) for n in (nh, ng, ng))
+    s = torch.einsum("sbhd,tbhd->bhst", q.double(), k.double().repeat_interleave(nh // ng, 2)) * 0.125
+    if causal:
+        s = s.masked_fill(torch.ones(S, S, dtype=torch.bool, device=DEV).triu(1), float("-inf"))
+    ref = torch.einsum("bhst,tbhd->sbhd", torch.softmax(s, -1), v.double().repeat_interleave(nh // ng, 2))
+    lib, out = _lib.load(), {}
+    try:
+        for variant in (0, 1, 2):
+            lib.hg_attn_set_fwd_variant(variant)
+            out[variant], lse = ops.flash_attention(q, k, v, causal=causal, return_lse=True)
+            assert rel_err(out[variant], ref) < 4e-3                # as above
+            assert torch.allclose(lse.double(), torch.logsumexp(s, -1), rtol=1e-5, atol=1e-5)
+    finally:
+        lib.hg_attn_set_fwd_variant(0)
+    assert torch.equal(out[0], out[2 if -(-S // 128) * B * nh > 148 else 1])
+    _lib.assert_healthy()
