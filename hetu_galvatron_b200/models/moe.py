@@ -429,11 +429,14 @@ def _aligned_starts(counts: torch.Tensor) -> Tuple[torch.Tensor, int]:
     return starts, int(starts[-1].item())
 
 
-def local_dispatch_usable(x: torch.Tensor, idx: torch.Tensor, E: int, k: int) -> bool:
-    """Whether the kernels of csrc/sm100/moe_local.cu take this call: 16-bit rows of whole 16-byte groups on a GPU."""
+def local_dispatch_usable(x: torch.Tensor, probs: torch.Tensor, idx: torch.Tensor, E: int, k: int) -> bool:
+    """Whether the kernels of csrc/sm100/moe_local.cu take this call: 16-bit rows of whole 16-byte groups on a GPU, a whole
+    expert number and one weight for each of the ``k`` slots of every row, all on that GPU."""
     from ..ops import _lib
 
-    return x.is_cuda and x.dtype == _lib.lp_dtype() and x.shape[1] % 8 == 0 and E <= 256 and idx.shape[0] == x.shape[0]
+    return (x.is_cuda and x.dtype == _lib.lp_dtype() and x.shape[1] % 8 == 0 and 1 <= E <= 256
+            and idx.shape == (x.shape[0], k) and not idx.is_floating_point() and probs.numel() == idx.numel()
+            and idx.device == probs.device == x.device)
 
 
 class _LocalPlan:
@@ -571,6 +574,8 @@ class GalvatronMoEMLP(nn.Module):
         k, E, ep, E_loc = s.topk, s.experts, c.ep_size, self.experts.E_loc
         if local_only:
             E, ep = E_loc, 1
+        if probs.numel() < idx.numel():
+            raise IndexError("%d routing weights for %d (token, expert) pairs" % (probs.numel(), idx.numel()))
         # "flex" is the reference's fused dispatcher (DeepEP, moe/token_dispatcher.py:743-1037); here it selects the
         # peer-memory pull kernels, which the fused-communication switch also turns on for "alltoall"
         if ep > 1 and (getattr(c, "fused_comm", False) or s.dispatcher == "flex"):
@@ -586,7 +591,7 @@ class GalvatronMoEMLP(nn.Module):
                 w = torch.where(idx >= 0, probs, torch.zeros_like(probs)).to(torch.float32)
                 # the routing weights are applied inside the pull kernel: no [T, k, H] intermediate
                 return fa.moe_combine_weighted(out_buf, w, plan)
-        if ep == 1 and local_dispatch_usable(x2d, idx, E, k):
+        if ep == 1 and local_dispatch_usable(x2d, probs, idx, E, k):
             plan = _LocalPlan(idx, E)
             buf = _LocalDispatch.apply(x2d, plan)
             out_buf = self.experts(buf, plan.row_start)

@@ -1,0 +1,32 @@
+"""Host side of the single-GPU expert dispatch: which calls its kernels are handed."""
+import pytest
+import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
+
+from hetu_galvatron_b200.models.moe import GalvatronMoEMLP, local_dispatch_usable
+from hetu_galvatron_b200.models.spec import LayerCtx, ModelSpec
+
+
+@pytest.mark.parametrize("what,E,ok", [
+    ({}, 8, True), ({}, 256, True), ({}, 257, False), ({}, 0, False), ({"probs": (4, 1)}, 8, False), ({"probs": (3, 2)}, 8, False),
+    ({"probs": (8,)}, 8, True), ({"probs": (4, 3)}, 8, False), ({"idx": (3, 2)}, 8, False), ({"idx": (4, 3)}, 8, False),
+    ({"idx": (8,)}, 8, False), ({"x": (4, 12)}, 8, False), ({"idx_device": "cpu"}, 8, False), ({"probs_device": "cpu"}, 8, False),
+    ({"x_device": "cpu"}, 8, False), ({"dtype": torch.float32}, 8, False), ({"idx_dtype": torch.float32}, 8, False),
+    ({"idx_dtype": torch.int32}, 8, True)])
+def test_local_dispatch_usable(what, E, ok):
+    with FakeTensorMode():                       # tensors of a GPU that need not be there
+        x = torch.empty(what.get("x", (4, 16)), dtype=what.get("dtype", torch.bfloat16), device=what.get("x_device", "cuda"))
+        probs = torch.empty(what.get("probs", (4, 2)), device=what.get("probs_device", "cuda"))
+        idx = torch.empty(what.get("idx", (4, 2)), dtype=what.get("idx_dtype", torch.int64), device=what.get("idx_device", "cuda"))
+        assert local_dispatch_usable(x, probs, idx, E, 2) is ok
+
+
+def test_fewer_weights_than_pairs_are_refused():
+    spec = ModelSpec(family="llama", hidden=16, layers=1, heads=2, kv_heads=2, head_dim=8, ffn=16, vocab=64, padded_vocab=64,
+                     seq_len=0, experts=4, moe_ffn=16, topk=2, dtype=torch.float32)
+    m = GalvatronMoEMLP(spec, LayerCtx(), "cpu", "mlp")
+    m.reset_parameters()
+    idx = torch.tensor([[0, 1], [2, 3], [1, 0]])
+    with pytest.raises(IndexError):
+        m(torch.randn(3, 16), torch.rand(3, 1), idx)
+    assert m(torch.randn(3, 16), torch.rand(3, 2), idx).shape == (3, 16)
