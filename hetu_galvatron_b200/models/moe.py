@@ -449,7 +449,7 @@ class _LocalPlan:
 
         self.T, self.k = idx.shape
         n = idx.numel()
-        flat = idx.reshape(-1).to(torch.int64)
+        flat = idx.reshape(-1).to(torch.int64).contiguous()   # reshaping a column of a wider matrix gives a strided view
         self.rows = max((n + E * (SEG_ALIGN - 1)) // SEG_ALIGN * SEG_ALIGN, SEG_ALIGN)
         i32 = dict(dtype=torch.int32, device=idx.device)
         counts = torch.empty((max(1, (n + 1023) // 1024), E), **i32)

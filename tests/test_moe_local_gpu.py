@@ -67,6 +67,18 @@ def test_local_dispatch_and_combine(T, k, E, H, drop):
     _lib.assert_healthy()
 
 
+# one column, every other column and a transposed matrix of expert numbers; 32-bit ones
+@pytest.mark.parametrize("view", [lambda i: i[:, :1], lambda i: i[:, ::2], lambda i: i[:, :2].t().contiguous().t(),
+                                  lambda i: i.to(torch.int32)[:, 1:2]])
+def test_placement_of_strided_indices(view):
+    E = 8
+    idx = torch.randint(0, E, (300, 4), generator=torch.Generator().manual_seed(3))
+    plan = _LocalPlan(view(idx.to(DEV)), E)
+    starts, dest = placement(view(idx), E)
+    assert plan.row_start.tolist() == starts and plan.dest.tolist() == dest
+    _lib.assert_healthy()
+
+
 def test_grouped_gemm_clears_the_rows_outside_its_segments():
     from hetu_galvatron_b200 import ops
 
