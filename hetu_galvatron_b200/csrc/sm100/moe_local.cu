@@ -192,6 +192,7 @@ zero_outside_kernel(hg_lp_t* __restrict__ buf, const int* __restrict__ row_start
     reinterpret_cast<uint4*>(buf)[i < head ? i : i - head + int64_t(last) * vec] = make_uint4(0, 0, 0, 0);
 }
 
+inline bool aligned16(const void* p) { return (uintptr_t(p) & 15) == 0; }
 inline int row_grid(int rows) { return rows < 148 * 16 ? rows : 148 * 16; }
 
 }  // namespace
@@ -215,7 +216,7 @@ int hg_moe_plan(const void* idx, int n, int E, int align, int bound, void* count
 int hg_moe_scatter(const void* x, long long x_pitch, const void* src, const void* w, int rows, int k, int H, void* buf,
                    void* stream) {
   if (rows <= 0) return 0;
-  if (k < 1 || (H & 7) || (x_pitch & 7)) return -1;
+  if (k < 1 || (H & 7) || (x_pitch & 7) || !aligned16(x) || !aligned16(buf)) return -1;
   moe_scatter_kernel<<<row_grid(rows), 256, 0, (cudaStream_t)stream>>>((const hg_lp_t*)x, x_pitch, (const int*)src,
                                                                        (const float*)w, rows, k, H / 8, (hg_lp_t*)buf);
   return int(cudaGetLastError());
@@ -223,7 +224,7 @@ int hg_moe_scatter(const void* x, long long x_pitch, const void* src, const void
 
 int hg_moe_gather(const void* y, const void* dest, const void* w, int T, int k, int H, void* out, void* stream) {
   if (T <= 0) return 0;
-  if (k < 1 || (H & 7)) return -1;
+  if (k < 1 || (H & 7) || !aligned16(y) || !aligned16(out)) return -1;
   moe_gather_kernel<<<row_grid(T), 256, 0, (cudaStream_t)stream>>>((const hg_lp_t*)y, (const int*)dest, (const float*)w, T,
                                                                    k, H / 8, (hg_lp_t*)out);
   return int(cudaGetLastError());
@@ -232,7 +233,7 @@ int hg_moe_gather(const void* y, const void* dest, const void* w, int T, int k, 
 int hg_moe_dot(const void* y, const void* dout, long long dout_pitch, const void* dest, int n, int k, int H, void* dw,
                void* stream) {
   if (n <= 0) return 0;
-  if (k < 1 || (H & 7) || (dout_pitch & 7)) return -1;
+  if (k < 1 || (H & 7) || (dout_pitch & 7) || !aligned16(y) || !aligned16(dout)) return -1;
   moe_dot_kernel<<<(n + 7) / 8, 256, 0, (cudaStream_t)stream>>>((const hg_lp_t*)y, (const hg_lp_t*)dout, dout_pitch,
                                                                 (const int*)dest, n, k, H / 8, (float*)dw);
   return int(cudaGetLastError());
@@ -242,7 +243,7 @@ int hg_moe_dot(const void* y, const void* dout, long long dout_pitch, const void
 // ascending) covers become zero.
 int hg_zero_outside(void* buf, const void* row_start, int G, int rows, int width, void* stream) {
   if (rows <= 0 || width <= 0) return 0;
-  if ((width & 7) || (uintptr_t(buf) & 15) || G < 0) return -1;
+  if ((width & 7) || !aligned16(buf) || G < 0) return -1;
   zero_outside_kernel<<<148 * 4, 256, 0, (cudaStream_t)stream>>>((hg_lp_t*)buf, (const int*)row_start, G, rows, width / 8);
   return int(cudaGetLastError());
 }

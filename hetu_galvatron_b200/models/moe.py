@@ -461,6 +461,13 @@ class _LocalPlan:
         _lib.count_launch(2)
 
 
+def _rows16(t: torch.Tensor) -> torch.Tensor:
+    """``t`` in rows of 16-byte groups as the kernels read them: a copy where its storage starts between two of them (a
+    packed tensor may: a slice of a flat buffer)."""
+    t = _rowmajor(t)
+    return t if t.data_ptr() % 16 == 0 else t.clone(memory_format=torch.contiguous_format)
+
+
 def _moe_scatter(x, plan, w=None):
     """``buf[r] = w[src[r]] * x[src[r] // k]``, zeros where no pair fills the row."""
     from ..ops import _lib
@@ -489,11 +496,11 @@ class _LocalDispatch(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, plan):
         ctx.plan = plan
-        return _moe_scatter(_rowmajor(x), plan)
+        return _moe_scatter(_rows16(x), plan)
 
     @staticmethod
     def backward(ctx, g):
-        return _moe_gather(g.contiguous(), ctx.plan), None
+        return _moe_gather(_rows16(g.contiguous()), ctx.plan), None
 
 
 class _LocalCombine(torch.autograd.Function):
@@ -501,7 +508,7 @@ class _LocalCombine(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, y, w, plan):
-        y, w = y.contiguous(), w.contiguous()
+        y, w = _rows16(y.contiguous()), w.contiguous()
         ctx.plan = plan
         ctx.save_for_backward(y, w)
         return _moe_gather(y, plan, w)
@@ -512,7 +519,7 @@ class _LocalCombine(torch.autograd.Function):
 
         y, w = ctx.saved_tensors
         plan = ctx.plan
-        g = _rowmajor(g)
+        g = _rows16(g)
         dy = _moe_scatter(g, plan, w) if ctx.needs_input_grad[0] else None
         dw = None
         if ctx.needs_input_grad[1]:

@@ -3,7 +3,7 @@ import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
-from hetu_galvatron_b200.models.moe import GalvatronMoEMLP, local_dispatch_usable
+from hetu_galvatron_b200.models.moe import GalvatronMoEMLP, _rows16, local_dispatch_usable
 from hetu_galvatron_b200.models.spec import LayerCtx, ModelSpec
 
 
@@ -30,3 +30,12 @@ def test_fewer_weights_than_pairs_are_refused():
     with pytest.raises(IndexError):
         m(torch.randn(3, 16), torch.rand(3, 1), idx)
     assert m(torch.randn(3, 16), torch.rand(3, 2), idx).shape == (3, 16)
+
+
+@pytest.mark.parametrize("offset,copied", [(0, False), (8, False), (1, True), (4, True)])
+def test_rows_start_on_16_byte_boundaries(offset, copied):
+    flat = torch.arange(64 + 24, dtype=torch.int16)
+    flat = flat[(-flat.data_ptr() % 16) // 2:]
+    for t in (flat[offset:offset + 64].view(4, 16), flat[offset:offset + 64].view(2, 32)[:, :16]):
+        r = _rows16(t)
+        assert r.data_ptr() % 16 == 0 and torch.equal(r, t) and (r.data_ptr() != t.data_ptr()) is copied

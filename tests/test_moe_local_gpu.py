@@ -79,6 +79,33 @@ def test_placement_of_strided_indices(view):
     _lib.assert_healthy()
 
 
+def test_rows_between_16_byte_boundaries():
+    """Tokens, expert rows and their gradients as slices of a flat buffer that start anywhere."""
+    T, k, E, H = 5, 2, 4, 64
+    idx = torch.randint(0, E, (T, k), device=DEV)
+    plan = _LocalPlan(idx, E)
+
+    def both(shape):
+        n = shape[0] * shape[1]
+        t = torch.randn(n + 3, device=DEV).to(torch.bfloat16)[3:].view(shape)
+        return [v.requires_grad_() for v in (t.detach(), t.detach().clone())]
+
+    w = torch.rand(T, k, device=DEV)
+    for f, shape, out_shape in ((lambda t: _LocalDispatch.apply(t, plan), (T, H), (plan.rows, H)),
+                                (lambda t: _LocalCombine.apply(t, w, plan), (plan.rows, H), (T, H))):
+        xs, gs = both(shape), both(out_shape)
+        outs = [f(x) for x in xs]
+        for o, g in zip(outs, gs):
+            o.backward(g.detach())
+        assert torch.equal(outs[0], outs[1]) and torch.equal(xs[0].grad, xs[1].grad)
+    lib = _lib.load()
+    odd = torch.zeros(E * 256 * H + 1, device=DEV, dtype=torch.bfloat16)[1:]
+    assert lib.hg_moe_scatter(odd.data_ptr(), H, plan.src.data_ptr(), 0, plan.rows, k, H, xs[1].data_ptr(), 0) == -1
+    assert lib.hg_moe_gather(odd.data_ptr(), plan.dest.data_ptr(), 0, T, k, H, xs[1].data_ptr(), 0) == -1
+    assert lib.hg_moe_dot(xs[1].data_ptr(), odd.data_ptr(), H, plan.dest.data_ptr(), T * k, k, H, w.data_ptr(), 0) == -1
+    _lib.assert_healthy()
+
+
 def test_grouped_gemm_clears_the_rows_outside_its_segments():
     from hetu_galvatron_b200 import ops
 
