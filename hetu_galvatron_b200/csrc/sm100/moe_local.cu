@@ -200,7 +200,7 @@ inline int row_grid(int rows) { return rows < 148 * 16 ? rows : 148 * 16; }
 extern "C" {
 
 // `counts`: scratch of ceil(n / 1024) (at least 1) * E ints.  `bound` rows must hold every routing of n pairs:
-// n + E * (align - 1), rounded down to a multiple of align, is enough.
+// n + min(n, E) * (align - 1), rounded down to a multiple of align, is enough.
 int hg_moe_plan(const void* idx, int n, int E, int align, int bound, void* counts, void* row_start, void* dest, void* src,
                 void* stream) {
   if (n < 0 || E < 1 || E > kMaxExperts || align < 1 || bound < 0) return -1;

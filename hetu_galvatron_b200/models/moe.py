@@ -439,10 +439,16 @@ def local_dispatch_usable(x: torch.Tensor, probs: torch.Tensor, idx: torch.Tenso
             and idx.device == probs.device == x.device)
 
 
+def local_rows(n: int, E: int) -> int:
+    """Rows of the least buffer of aligned segments that holds every routing of ``n`` pairs to ``E`` experts (one segment at
+    least): at most ``min(n, E)`` experts get pairs, and each of them pads its segment by up to ``SEG_ALIGN - 1`` rows."""
+    return max((n + min(n, E) * (SEG_ALIGN - 1)) // SEG_ALIGN * SEG_ALIGN, SEG_ALIGN)
+
+
 class _LocalPlan:
     """Placement of every (token, slot) pair in this GPU's expert buffer (built on the device, nothing is read back):
     ``row_start [E + 1]`` aligned segment starts, ``dest [T * k]`` row of each pair (-1: dropped), ``src [rows]`` pair of
-    each row (-1: padding).  ``rows`` is the least static size that holds any routing."""
+    each row (-1: padding)."""
 
     def __init__(self, idx: torch.Tensor, E: int):
         from ..ops import _lib
@@ -450,7 +456,7 @@ class _LocalPlan:
         self.T, self.k = idx.shape
         n = idx.numel()
         flat = idx.reshape(-1).to(torch.int64).contiguous()   # reshaping a column of a wider matrix gives a strided view
-        self.rows = max((n + E * (SEG_ALIGN - 1)) // SEG_ALIGN * SEG_ALIGN, SEG_ALIGN)
+        self.rows = local_rows(n, E)
         i32 = dict(dtype=torch.int32, device=idx.device)
         counts = torch.empty((max(1, (n + 1023) // 1024), E), **i32)
         self.row_start = torch.empty(E + 1, **i32)

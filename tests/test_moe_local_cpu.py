@@ -3,7 +3,7 @@ import pytest
 import torch
 from torch._subclasses.fake_tensor import FakeTensorMode
 
-from hetu_galvatron_b200.models.moe import GalvatronMoEMLP, _rows16, local_dispatch_usable
+from hetu_galvatron_b200.models.moe import SEG_ALIGN, GalvatronMoEMLP, _rows16, local_dispatch_usable, local_rows
 from hetu_galvatron_b200.models.spec import LayerCtx, ModelSpec
 
 
@@ -39,3 +39,17 @@ def test_rows_start_on_16_byte_boundaries(offset, copied):
     for t in (flat[offset:offset + 64].view(4, 16), flat[offset:offset + 64].view(2, 32)[:, :16]):
         r = _rows16(t)
         assert r.data_ptr() % 16 == 0 and torch.equal(r, t) and (r.data_ptr() != t.data_ptr()) is copied
+
+
+@pytest.mark.parametrize("n", [0, 1, 2, 8, 127, 128, 129, 130, 256, 385, 1000])
+@pytest.mark.parametrize("E", [1, 2, 3, 8, 160, 256])
+def test_buffer_rows_are_what_the_worst_routing_fills(n, E):
+    def rows(counts):
+        return sum(-(-c // SEG_ALIGN) for c in counts) * SEG_ALIGN
+
+    m = min(n, E)                                # one pair for every expert, the rest for one of them
+    assert local_rows(n, E) == max(rows([1] * (m - 1) + [n - m + 1]) if n else 0, SEG_ALIGN)
+    g = torch.Generator().manual_seed(n + E)
+    for skew in (0.0, 0.5, 2.0):
+        e = torch.multinomial(torch.rand(E, generator=g) ** (1 + skew), max(n, 1), True, generator=g)[:n]
+        assert rows(e.bincount(minlength=E).tolist()) <= local_rows(n, E)
