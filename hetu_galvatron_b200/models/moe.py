@@ -604,7 +604,9 @@ class GalvatronMoEMLP(nn.Module):
                 w = torch.where(idx >= 0, probs, torch.zeros_like(probs)).to(torch.float32)
                 # the routing weights are applied inside the pull kernel: no [T, k, H] intermediate
                 return fa.moe_combine_weighted(out_buf, w, plan)
-        if ep == 1 and local_dispatch_usable(x2d, probs, idx, E, k):
+        # pairs that other ranks serve are dropped here: the static bound of the kernels' buffer would hold those of all
+        # ranks, where the general path counts this rank's own
+        if ep == 1 and not local_only and local_dispatch_usable(x2d, probs, idx, E, k):
             plan = _LocalPlan(idx, E)
             buf = _LocalDispatch.apply(x2d, plan)
             out_buf = self.experts(buf, plan.row_start)

@@ -1,5 +1,7 @@
 """Single-GPU expert dispatch (csrc/sm100/moe_local.cu): the placement against a list-based restatement, and the row
 passes against index operations in 64 bits."""
+from types import SimpleNamespace
+
 import pytest
 import torch
 
@@ -103,6 +105,35 @@ def test_rows_between_16_byte_boundaries():
     assert lib.hg_moe_scatter(odd.data_ptr(), H, plan.src.data_ptr(), 0, plan.rows, k, H, xs[1].data_ptr(), 0) == -1
     assert lib.hg_moe_gather(odd.data_ptr(), plan.dest.data_ptr(), 0, T, k, H, xs[1].data_ptr(), 0) == -1
     assert lib.hg_moe_dot(xs[1].data_ptr(), odd.data_ptr(), H, plan.dest.data_ptr(), T * k, k, H, w.data_ptr(), 0) == -1
+    _lib.assert_healthy()
+
+
+def test_allgather_dispatcher_buffers_only_the_local_pairs():
+    """One of four ranks' view of the gathered pairs: the expert buffer follows what is routed to its two experts."""
+    from hetu_galvatron_b200.models.moe import GalvatronMoEMLP
+    from hetu_galvatron_b200.models.spec import LayerCtx, ModelSpec
+
+    T, k, E, H = 1024, 2, 8, 128
+    spec = ModelSpec(family="llama", hidden=H, layers=1, heads=1, kv_heads=1, head_dim=128, ffn=128, vocab=512,
+                     padded_vocab=512, seq_len=0, experts=E, moe_ffn=128, topk=k, dispatcher="allgather")
+    m = GalvatronMoEMLP(spec, LayerCtx(ep=SimpleNamespace(size=4, rank=1)), DEV, "mlp")
+    m.reset_parameters()
+    g = torch.Generator().manual_seed(5)
+    idx = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(T)])
+    local = torch.where((idx >= 2) & (idx < 4), idx - 2, -1)
+    x, p = torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV), torch.rand(T, k, generator=g).to(DEV)
+    rows = []
+    hook = m.experts.register_forward_pre_hook(lambda _, a: rows.append(a[0].shape[0]))
+    with torch.no_grad():
+        out = m._routed(x, p, local.to(DEV), local_only=True)
+    hook.remove()
+    assert rows == [placement(local, 2)[0][-1]]
+    w1, w2 = (q.double() for q in (m.experts.linear_fc1.weight, m.experts.linear_fc2.weight))
+    ref = torch.zeros(T, H, dtype=torch.float64, device=DEV)
+    for e in range(2):
+        a, b = (x.double() @ w1[e].t()).chunk(2, -1)
+        ref += (torch.nn.functional.silu(a) * b) @ w2[e].t() * (p * (local.to(DEV) == e)).sum(1, keepdim=True)
+    assert ((out.double() - ref).norm() / ref.norm()).item() < 1e-2      # four roundings to bf16
     _lib.assert_healthy()
 
 
