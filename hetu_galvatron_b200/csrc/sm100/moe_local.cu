@@ -2,7 +2,7 @@
 //
 //   plan      idx [n = T * k] (expert of every (token, slot) pair, negative = dropped)  ->
 //             row_start [E + 1]  aligned segment starts of the experts,
-//             dest [n]           row of the pair in the expert buffer (-1: dropped),
+//             dest [n]           row of the pair in the expert buffer (-1: dropped, -2: no such expert),
 //             src [bound]        pair that fills a row of the buffer (-1: padding)
 //   dispatch  buf[r] = x[src[r] / k] or 0                 backward: dx[t] = sum_j dbuf[dest[t, j]]
 //   combine   out[t] = sum_j w[t, j] * y[dest[t, j]]      backward: dy[r] = w[src[r]] * dout[src[r] / k] or 0,
@@ -20,6 +20,7 @@ namespace {
 
 constexpr int kPlanThreads = 1024;   // pairs per CTA of the plan kernels
 constexpr int kMaxExperts = 256;
+constexpr int kNoSuchExpert = -2;    // a number from E on is a mistake of the caller: its token's result is NaN
 
 __device__ __forceinline__ void unpack8(const uint4& u, float* f) {
   const hg_lp2_t* p = reinterpret_cast<const hg_lp2_t*>(&u);
@@ -55,7 +56,7 @@ moe_count_kernel(const int64_t* __restrict__ idx, int n, int E, int* __restrict_
 // ranks its pairs: inside a warp by matching experts, between the warps of the chunk by a prefix over their counts.
 __global__ void __launch_bounds__(kPlanThreads)
 moe_place_kernel(const int64_t* __restrict__ idx, int n, int E, int align, const int* __restrict__ counts, int bound,
-                 int* __restrict__ row_start, int* __restrict__ dest, int* __restrict__ src) {
+                 int* __restrict__ row_start, int* __restrict__ dest, int* __restrict__ src, int* status) {
   constexpr int kWarps = kPlanThreads / 32;
   __shared__ int padded[kMaxExperts];            // then: first row of this chunk's pairs of an expert
   __shared__ int warp_cnt[kWarps][kMaxExperts];  // then: rank of a warp's first pair of an expert
@@ -99,7 +100,8 @@ moe_place_kernel(const int64_t* __restrict__ idx, int n, int E, int align, const
   }
   __syncthreads();
   if (p < n) {
-    int row = -1;
+    int row = idx[p] >= E ? kNoSuchExpert : -1;
+    if (row == kNoSuchExpert) hg::set_status(status, hg::kBadArgument);
     if (e >= 0) {
       row = padded[e] + warp_cnt[warp][e] + rank;
       if (row < bound) src[row] = p;             // always, for the bound that the host computes
@@ -136,7 +138,7 @@ moe_scatter_kernel(const hg_lp_t* __restrict__ x, int64_t x_pitch, const int* __
   }
 }
 
-// out[t] = sum_j w[t, j] * y[dest[t, j]] (w null: 1), pairs with dest < 0 skipped
+// out[t] = sum_j w[t, j] * y[dest[t, j]] (w null: 1), dropped pairs skipped, NaN where an expert does not exist
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(const hg_lp_t* __restrict__ y, const int* __restrict__ dest, const float* __restrict__ w, int T, int k,
                   int vec, hg_lp_t* __restrict__ out) {
@@ -146,7 +148,12 @@ moe_gather_kernel(const hg_lp_t* __restrict__ y, const int* __restrict__ dest, c
 #pragma unroll 2
       for (int j = 0; j < k; ++j) {
         const int r = dest[t * k + j];
-        if (r < 0) continue;
+        if (r < 0) {
+          if (r == kNoSuchExpert)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = NAN;
+          continue;
+        }
         const float s = w ? w[t * k + j] : 1.f;
         float f[8];
         unpack8(reinterpret_cast<const uint4*>(y + int64_t(r) * vec * 8)[c], f);
@@ -208,7 +215,7 @@ int hg_moe_plan(const void* idx, int n, int E, int align, int bound, void* count
   cudaStream_t st = (cudaStream_t)stream;
   moe_count_kernel<<<chunks, kPlanThreads, 0, st>>>((const int64_t*)idx, n, E, (int*)counts, (int*)src, bound);
   moe_place_kernel<<<chunks, kPlanThreads, 0, st>>>((const int64_t*)idx, n, E, align, (const int*)counts, bound,
-                                                    (int*)row_start, (int*)dest, (int*)src);
+                                                    (int*)row_start, (int*)dest, (int*)src, hg_host::status_ptr());
   return int(cudaGetLastError());
 }
 

@@ -447,8 +447,8 @@ def local_rows(n: int, E: int) -> int:
 
 class _LocalPlan:
     """Placement of every (token, slot) pair in this GPU's expert buffer (built on the device, nothing is read back):
-    ``row_start [E + 1]`` aligned segment starts, ``dest [T * k]`` row of each pair (-1: dropped), ``src [rows]`` pair of
-    each row (-1: padding)."""
+    ``row_start [E + 1]`` aligned segment starts, ``dest [T * k]`` row of each pair (-1: dropped, -2: an expert that does not
+    exist, which also sets the status word), ``src [rows]`` pair of each row (-1: padding)."""
 
     def __init__(self, idx: torch.Tensor, E: int):
         from ..ops import _lib

@@ -137,6 +137,19 @@ def test_allgather_dispatcher_buffers_only_the_local_pairs():
     _lib.assert_healthy()
 
 
+def test_experts_that_do_not_exist_are_not_passed_over():
+    T, k, E, H = 300, 2, 4, 64
+    idx = torch.randint(0, E, (T, k), generator=torch.Generator().manual_seed(9))
+    idx[7, 1], idx[250, 0], idx[3, 0] = E, 1 << 40, -1
+    plan = _LocalPlan(idx.to(DEV), E)
+    assert _lib.read_status(clear=True) == 6                            # bad argument
+    out = _LocalCombine.apply(torch.ones(plan.rows, H, device=DEV, dtype=torch.bfloat16), torch.ones(T, k, device=DEV), plan)
+    bad = torch.zeros(T, dtype=torch.bool, device=DEV)
+    bad[[7, 250]] = True
+    assert out[bad].isnan().all() and out[~bad].isfinite().all()
+    _lib.assert_healthy()
+
+
 def test_grouped_gemm_clears_the_rows_outside_its_segments():
     from hetu_galvatron_b200 import ops
 
