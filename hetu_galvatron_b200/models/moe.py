@@ -496,6 +496,11 @@ def _moe_gather(y, plan, w=None):
     return out
 
 
+def _rows_of(t: torch.Tensor, at: torch.Tensor) -> torch.Tensor:
+    """``t[at]`` in fp32 with zero rows where ``at`` is negative, in differentiable operations."""
+    return torch.where(at[:, None] >= 0, t.index_select(0, at.clamp(min=0)).float(), 0.0)
+
+
 class _LocalDispatch(torch.autograd.Function):
     """Tokens -> aligned, zero-padded expert segments; the gradient of a token is the sum over its copies."""
 
@@ -506,6 +511,9 @@ class _LocalDispatch(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g):
+        if torch.is_grad_enabled() and g.requires_grad:      # a graph of the gradient is wanted
+            plan = ctx.plan
+            return _rows_of(g, plan.dest).view(plan.T, plan.k, -1).sum(1).to(g.dtype), None
         return _moe_gather(_rows16(g.contiguous()), ctx.plan), None
 
 
@@ -525,6 +533,11 @@ class _LocalCombine(torch.autograd.Function):
 
         y, w = ctx.saved_tensors
         plan = ctx.plan
+        if torch.is_grad_enabled() and (y.requires_grad or w.requires_grad or g.requires_grad):   # as above
+            tok = torch.where(plan.src >= 0, plan.src // plan.k, plan.src)
+            dy = (_rows_of(g, tok) * _rows_of(w.reshape(-1, 1), plan.src)).to(y.dtype)
+            dw = (_rows_of(y, plan.dest) * g.float().repeat_interleave(plan.k, 0)).sum(-1).view_as(w)
+            return dy, dw, None
         g = _rows16(g)
         dy = _moe_scatter(g, plan, w) if ctx.needs_input_grad[0] else None
         dw = None

@@ -137,6 +137,39 @@ def test_allgather_dispatcher_buffers_only_the_local_pairs():
     _lib.assert_healthy()
 
 
+@pytest.mark.parametrize("wrt", ["gradient", "weights", "rows"])
+def test_gradients_of_the_gradients(wrt):
+    """Second derivatives of dispatch and combine, against the same sums in 64 bits (the rows themselves are 16-bit)."""
+    T, k, E, H = 40, 2, 4, 32
+    g = torch.Generator().manual_seed(11)
+    idx = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(T)])
+    idx[5, 1] = -1
+    plan = _LocalPlan(idx.to(DEV), E)
+    d, live = plan.dest.long().view(T, k).clamp(min=0), (plan.dest >= 0).view(T, k, 1)
+    y, x, dout, dbuf = (torch.randn(n, H, generator=g).to(torch.bfloat16).to(DEV) for n in (plan.rows, T, T, plan.rows))
+    w, vw, vx = torch.rand(T, k, generator=g).to(DEV), torch.randn(T, k, generator=g).to(DEV), torch.randn(T, H, generator=g).to(DEV)
+    vy = torch.randn(plan.rows, H, generator=g).to(DEV)
+
+    def combined(y, w, dout):                      # out and a functional of its gradients
+        out = _LocalCombine.apply(y, w, plan) if y.dtype == torch.bfloat16 else ((y[d] * live) * w[..., None]).sum(1)
+        gy, gw = torch.autograd.grad(out, (y, w), dout, create_graph=True)
+        return (gy * vy.to(gy.dtype)).sum() + (gw * vw.to(gw.dtype)).sum()
+
+    got, want = ([t.to(dt).requires_grad_() for t, dt in ((y, a), (w, b), (dout, a))]
+                 for a, b in ((torch.bfloat16, torch.float32), (torch.float64, torch.float64)))
+    at = {"rows": 0, "weights": 1, "gradient": 2}[wrt]
+    res, ref = (torch.autograd.grad(combined(*t), t[at])[0] for t in (got, want))
+    assert ((res.double() - ref).norm() / ref.norm()).item() < 2e-2            # vy and gy are rounded to 16 bits
+    if wrt == "gradient":
+        xs, gs = x.clone().requires_grad_(), dbuf.clone().requires_grad_()
+        (gx,) = torch.autograd.grad(_LocalDispatch.apply(xs, plan), xs, gs, create_graph=True)
+        (res,) = torch.autograd.grad((gx.float() * vx).sum(), gs)
+        ref = torch.zeros(plan.rows, H, device=DEV)
+        ref[d[live[..., 0]]] = vx[:, None].expand(T, k, H)[live[..., 0]]
+        assert ((res.float() - ref).norm() / ref.norm()).item() < 1e-2
+    _lib.assert_healthy()
+
+
 def test_experts_that_do_not_exist_are_not_passed_over():
     T, k, E, H = 300, 2, 4, 64
     idx = torch.randint(0, E, (T, k), generator=torch.Generator().manual_seed(9))
