@@ -175,6 +175,8 @@ class _Linear(torch.autograd.Function):
 def column_sums(x: torch.Tensor) -> torch.Tensor:
     """``x.float().sum(0)`` of a matrix, rounded back to its dtype: the gradient of a bias."""
     rows, cols = x.shape
+    if torch.is_grad_enabled() and x.requires_grad:      # a graph of the gradient is wanted
+        return x.float().sum(0).to(x.dtype)
     if x.is_cuda and x.dtype == _lib.lp_dtype():
         x = _rowmajor(x)
     if rows == 0 or cols == 0 or not x.is_cuda or x.dtype != _lib.lp_dtype() or x.stride(0) % 8 or x.data_ptr() % 16:

@@ -73,3 +73,14 @@ def test_column_sums(rows, cols):
     wide = torch.randn(rows, cols + 8, device=DEV).to(torch.bfloat16)
     assert torch.allclose(column_sums(wide[:, :cols]).double(), wide[:, :cols].double().sum(0), rtol=2.0 ** -8,
                           atol=1e-6 * rows)
+
+
+def test_bias_gradient_has_a_gradient():
+    """create_graph: the bias gradient is linear in the incoming gradient."""
+    x, w = (torch.randn(n, 64, device=DEV).to(torch.bfloat16) for n in (24, 40))
+    b = torch.zeros(40, device=DEV, dtype=torch.bfloat16).requires_grad_()
+    dy = torch.randn(24, 40, device=DEV).to(torch.bfloat16).requires_grad_()
+    v = torch.randn(40, device=DEV).to(torch.bfloat16)
+    (gb,) = torch.autograd.grad(ops.linear(x, w, b), b, dy, create_graph=True)
+    assert torch.equal(torch.autograd.grad((gb * v).sum(), dy)[0], v.expand(24, 40))
+    _lib.assert_healthy()
