@@ -141,6 +141,40 @@ def _forward_launch(q, k, v, o, lse, S, Skv, B, nh, ng, hd, causal, q_pos0, k_po
     _lib.count_launch()
 
 
+def _nested(dims, width: int) -> bool:
+    """Whether rows of ``width`` packed elements under outer dimensions of ``(stride, size)`` are all apart: each stride
+    spans everything inside it."""
+    reach = width
+    for stride, n in sorted(d for d in dims if d[1] > 1):
+        if stride < reach:
+            return False
+        reach += stride * (n - 1)
+    return True
+
+
+def _disjoint(a: torch.Tensor, b: torch.Tensor, width: int) -> bool:
+    """Whether two caches ``[seq, batch, heads, hd]`` of ``width`` packed elements per token share no memory: separate ranges,
+    or equal strides and an offset that keeps every token apart from the other cache's (two halves of one buffer)."""
+    lo, hi = (a, b) if a.data_ptr() <= b.data_ptr() else (b, a)
+    apart = (hi.data_ptr() - lo.data_ptr()) // lo.element_size()
+    if lo.stride(0) * (lo.shape[0] - 1) + lo.stride(1) * (lo.shape[1] - 1) + width <= apart:
+        return True
+    dims = [i for i in (0, 1) if max(lo.shape[i], hi.shape[i]) > 1]
+    if any(lo.stride(i) != hi.stride(i) for i in dims):
+        return False
+    if not _nested([(lo.stride(i), max(lo.shape[i], hi.shape[i])) for i in dims], width):
+        return False
+    dims.sort(key=lo.stride, reverse=True)
+
+    def meet(off, at):                # whether tokens of the two can lie closer than a token's width
+        if at == len(dims):
+            return abs(off) < width
+        st, d = lo.stride(dims[at]), -off // lo.stride(dims[at])       # steps that bring them nearest from either side
+        return any(1 - lo.shape[dims[at]] <= n < hi.shape[dims[at]] and meet(off + n * st, at + 1) for n in (d, d + 1))
+
+    return not meet(apart, 0)
+
+
 def caches_usable(like: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, past: int, S: int, b0: int, B: int, ng: int,
                   hd: int) -> bool:
     """Whether the kernels can write ``S`` tokens of ``B`` sequences behind ``past`` cached ones to these caches
@@ -150,7 +184,9 @@ def caches_usable(like: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, past: 
             and not (kc.requires_grad or vc.requires_grad)
             and all(c.dim() == 4 and c.shape[0] >= past + S and c.shape[1] >= b0 + B and c.shape[2:] == (ng, hd)
                     and c.stride(3) == 1 and c.stride(2) == hd and min(c.stride(0), c.stride(1)) >= ng * hd
-                    and c.stride(0) % 8 == c.stride(1) % 8 == 0 and c.data_ptr() % 16 == 0 for c in (kc, vc)))
+                    and c.stride(0) % 8 == c.stride(1) % 8 == 0 and c.data_ptr() % 16 == 0
+                    and _nested(((c.stride(0), c.shape[0]), (c.stride(1), c.shape[1])), ng * hd) for c in (kc, vc))
+            and _disjoint(kc, vc, ng * hd))
 
 
 def cached_attention_usable(qkv, kc, vc, past: int, S: int, b0: int, B: int, ng: int, hd: int) -> bool:
