@@ -556,6 +556,7 @@ class GalvatronDecoderLayer(nn.Module):
         ws = torch.empty(max(d.ws_bytes, 1), dtype=torch.uint8, device=x.device)
         d.ws = ws.data_ptr()
         _lib.check(lib.hg_decoder_step(ctypes.byref(d), _lib.stream()), "hg_decoder_step")
+        ops.attention.caches_written(kc, vc)
         _lib.count_launch(11)
         return out
 

@@ -179,14 +179,21 @@ def caches_usable(like: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, past: 
                   hd: int) -> bool:
     """Whether the kernels can write ``S`` tokens of ``B`` sequences behind ``past`` cached ones to these caches
     ``[max_seq, max_batch, ng, hd]`` and read them: ``like``'s dtype and device, room for the tokens, contiguous heads,
-    whole 16-byte groups, elements that do not share memory, and no gradient recorded through them."""
-    return (past >= 0 and b0 >= 0 and kc.dtype == vc.dtype == like.dtype and kc.device == vc.device == like.device
+    whole 16-byte groups, elements that do not share memory, no gradient recorded through them, and an in-place write that
+    autograd would allow (:func:`caches_written` tells it of the kernels')."""
+    return ((torch.is_inference_mode_enabled() or not (kc.is_inference() or vc.is_inference())) and past >= 0 and b0 >= 0 and kc.dtype == vc.dtype == like.dtype and kc.device == vc.device == like.device
             and not (kc.requires_grad or vc.requires_grad)
             and all(c.dim() == 4 and c.shape[0] >= past + S and c.shape[1] >= b0 + B and c.shape[2:] == (ng, hd)
                     and c.stride(3) == 1 and c.stride(2) == hd and min(c.stride(0), c.stride(1)) >= ng * hd
                     and c.stride(0) % 8 == c.stride(1) % 8 == 0 and c.data_ptr() % 16 == 0
                     and _nested(((c.stride(0), c.shape[0]), (c.stride(1), c.shape[1])), ng * hd) for c in (kc, vc))
             and _disjoint(kc, vc, ng * hd))
+
+
+def caches_written(kc: torch.Tensor, vc: torch.Tensor):
+    """Tell autograd that the kernels have written to the caches, as an in-place operation would: a graph that has saved
+    them must not go backward over other values."""
+    torch.autograd.graph.increment_version((kc, vc))
 
 
 def cached_attention_usable(qkv, kc, vc, past: int, S: int, b0: int, B: int, ng: int, hd: int) -> bool:
@@ -211,6 +218,7 @@ def cached_attention(qkv: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, past
                             kc.stride(0), kc.stride(1), vc.stride(0), vc.stride(1), _lib.stream())
     _lib.check(rc, "hg_rope_append")
     _lib.count_launch()
+    caches_written(kc, vc)
     out = torch.empty((S, B, nh * hd), dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
     k, v = kc[:, b0:], vc[:, b0:]

@@ -58,3 +58,32 @@ def test_native_step_is_left_to_inference_without_gradient():
     with torch.no_grad():
         assert not m._takes_native_step(x) and m._takes_native_step(x[:64].contiguous())
     assert not m._takes_native_step(x[:1])
+
+
+@pytest.mark.parametrize("S", [1, 80])                # one native call; module by module
+def test_autograd_knows_of_the_writes_to_the_caches(S):
+    m = layer("RMSNorm", "swiglu", "rope", False, 4, 4, 64)
+    x = torch.randn(S, 1, 256, device=DEV).to(torch.bfloat16)
+    ic = StaticInferenceContext(1, 2 * S)
+    m.attn.attention.inference_context = ic
+    with torch.no_grad():
+        m(x)
+        kc, vc = ic.key_value_memory_dict[0]
+        before = kc._version, vc._version
+        m(x)
+        assert kc._version > before[0] and vc._version > before[1]
+        # a graph over the cached keys notices that they have changed
+        w = torch.ones(64, device=DEV, dtype=torch.bfloat16).requires_grad_()
+        with torch.enable_grad():
+            loss = (kc[:1] * w).sum()
+        m(x)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        loss.backward()
+    with torch.inference_mode():                      # caches of inference mode are not written outside of it
+        ic.key_value_memory_dict.clear()
+        m(x)
+        m(x)
+    with torch.no_grad(), pytest.raises(RuntimeError, match="[Ii]nference"):
+        m(x)
+    m.attn.attention.inference_context = None
+    _lib.assert_healthy()
