@@ -506,8 +506,10 @@ class GalvatronDecoderLayer(nn.Module):
 
     def _takes_native_step(self, x) -> bool:
         """A cached forward of few tokens whose kernels one native call can launch (csrc/sm100/decoder_step.cu): no
-        gradient, no parallelism inside the layer, nothing hooked into it, 16-bit contiguous tensors on one GPU."""
+        gradient in either mode, no parallelism inside the layer, nothing hooked into it, 16-bit contiguous tensors on
+        one GPU."""
         import torch.nn.modules.module as tm
+        from torch.autograd import forward_ad
 
         from ..ops import _lib
         from ..ops.gemm import NATIVE_STEP_ROWS, _PAIR_MODE
@@ -516,8 +518,9 @@ class GalvatronDecoderLayer(nn.Module):
         s = att.spec
         F1 = mlp.Fl * (2 if s.gated else 1)
         mods = (self, self.attn, self.attn.input_layernorm, att, self.ffn, self.ffn.post_attention_layernorm, mlp)
-        return (x.is_cuda and not torch.is_grad_enabled() and x.dtype == _lib.lp_dtype() and x.is_contiguous()
-                and _PAIR_MODE != "1" and x.dim() == 3 and x.shape[2] == s.hidden
+        return (x.is_cuda and not torch.is_grad_enabled() and forward_ad._current_level < 0
+                and x.dtype == _lib.lp_dtype() and x.is_contiguous() and _PAIR_MODE != "1"
+                and x.dim() == 3 and x.shape[2] == s.hidden
                 and att.linear_qkv.weight.shape == ((att.nh + 2 * att.ng) * att.hd, s.hidden)
                 and att.linear_proj.weight.shape == (s.hidden, att.nh * att.hd)
                 and mlp.linear_fc1.weight.shape == (F1, s.hidden) and mlp.linear_fc2.weight.shape == (s.hidden, mlp.Fl)

@@ -87,3 +87,18 @@ def test_autograd_knows_of_the_writes_to_the_caches(S):
         m(x)
     m.attn.attention.inference_context = None
     _lib.assert_healthy()
+
+
+def test_native_step_drops_no_tangent():
+    """Forward-mode differentiation is refused by the modules' functions, not answered without the tangent."""
+    from torch.autograd import forward_ad
+
+    m = layer("RMSNorm", "swiglu", "rope", False, 4, 4, 64)
+    x = torch.randn(1, 1, 256, device=DEV).to(torch.bfloat16)
+    m.attn.attention.inference_context = StaticInferenceContext(1, 8)
+    with torch.no_grad(), forward_ad.dual_level():
+        with pytest.raises(NotImplementedError):
+            m(forward_ad.make_dual(x, torch.ones_like(x)))
+        m(x)
+    m.attn.attention.inference_context = None
+    _lib.assert_healthy()
