@@ -500,24 +500,29 @@ class GalvatronDecoderLayer(nn.Module):
         self.ffn.reset_parameters(seed, full_init)
 
     def forward(self, x):
-        if self.attn.attention.inference_context is not None and self._takes_native_step(x):
+        att = getattr(self.attn, "attention", None)
+        if getattr(att, "inference_context", None) is not None and self._takes_native_step(x):
             return self._native_step(x)
         return self.ffn(self.attn(x), x)
 
     def _takes_native_step(self, x) -> bool:
         """A cached forward of few tokens whose kernels one native call can launch (csrc/sm100/decoder_step.cu): no
-        gradient in either mode, no parallelism inside the layer, nothing hooked into it, 16-bit contiguous tensors on
-        one GPU."""
+        gradient in either mode, no parallelism inside the layer, its own modules with nothing hooked into them, 16-bit
+        contiguous tensors on one GPU."""
         import torch.nn.modules.module as tm
         from torch.autograd import forward_ad
 
         from ..ops import _lib
         from ..ops.gemm import NATIVE_STEP_ROWS, _PAIR_MODE
 
+        if type(self.attn) is not GalvatronAttention or type(self.ffn) is not GalvatronMLP:
+            return False
         att, mlp, c = self.attn.attention, self.ffn.mlp, self.ctx
+        mods = (self.attn, self.attn.input_layernorm, att, self.ffn, self.ffn.post_attention_layernorm, mlp)
+        if [type(m) for m in mods[1:]] != [Norm, SelfAttention, GalvatronMLP, Norm, MLP]:
+            return False
         s = att.spec
         F1 = mlp.Fl * (2 if s.gated else 1)
-        mods = (self, self.attn, self.attn.input_layernorm, att, self.ffn, self.ffn.post_attention_layernorm, mlp)
         return (x.is_cuda and not torch.is_grad_enabled() and forward_ad._current_level < 0
                 and x.dtype == _lib.lp_dtype() and x.is_contiguous() and _PAIR_MODE != "1"
                 and x.dim() == 3 and x.shape[2] == s.hidden
@@ -530,7 +535,7 @@ class GalvatronDecoderLayer(nn.Module):
                 and not (s.hidden_dropout > 0.0 and self.training)
                 and all(p.dtype == x.dtype and p.device == x.device and p.is_contiguous() and p.data_ptr() % 16 == 0
                         for p in self.parameters())
-                and not any(m._forward_hooks or m._forward_pre_hooks for m in mods[1:])
+                and not any(m._forward_hooks or m._forward_pre_hooks or "forward" in vars(m) for m in mods)
                 and not (tm._global_forward_hooks or tm._global_forward_pre_hooks))
 
     def _native_step(self, x):

@@ -102,3 +102,39 @@ def test_native_step_drops_no_tangent():
         m(x)
     m.attn.attention.inference_context = None
     _lib.assert_healthy()
+
+
+def test_native_step_is_left_to_the_layers_own_modules():
+    from hetu_galvatron_b200.models.modules import MLP, GalvatronMLP
+
+    x = torch.randn(1, 1, 256, device=DEV).to(torch.bfloat16)
+
+    class Twice(MLP):
+        def forward(self, x):
+            return 2 * super().forward(x)
+
+    class Other(GalvatronMLP):
+        def forward(self, attn_out, residual):
+            return attn_out
+
+    def patched(m):
+        plain = m.attn.input_layernorm.forward
+        m.attn.input_layernorm.forward = lambda x, residual=None: plain(2 * x, residual)
+
+    for change in (lambda m: setattr(m.ffn.mlp, "__class__", Twice), lambda m: setattr(m.ffn, "__class__", Other), patched):
+        m = layer("RMSNorm", "swiglu", "rope", False, 4, 4, 64)
+        m.attn.attention.inference_context = StaticInferenceContext(1, 8)
+        with torch.no_grad():
+            assert m._takes_native_step(x)
+            change(m)
+            assert not m._takes_native_step(x)
+            want = m.ffn(m.attn(x), x)
+            assert torch.equal(m(x), want)
+
+
+def test_attention_of_another_kind():
+    m = layer("RMSNorm", "swiglu", "rope", False, 4, 4, 64)
+    m.attn = torch.nn.Identity()
+    x = torch.randn(1, 1, 256, device=DEV).to(torch.bfloat16)
+    with torch.no_grad():
+        assert torch.equal(m(x), m.ffn(x, x))
