@@ -505,6 +505,13 @@ class GalvatronDecoderLayer(nn.Module):
             return self._native_step(x)
         return self.ffn(self.attn(x), x)
 
+    def _step_weights(self):
+        """Weights and biases in the order of ``HgDecoderStep``.  A caller keeps the list until its kernels are launched: a
+        parametrized weight is a new tensor each time it is asked for."""
+        a, m = self.attn, self.ffn
+        return [t for h in (a.input_layernorm, a.attention.linear_qkv, a.attention.linear_proj, m.post_attention_layernorm,
+                            m.mlp.linear_fc1, m.mlp.linear_fc2) for t in (h.weight, h.bias)]
+
     def _takes_native_step(self, x) -> bool:
         """A cached forward of few tokens whose kernels one native call can launch (csrc/sm100/decoder_step.cu): no
         gradient in either mode, no parallelism inside the layer, its own modules with nothing hooked into them, 16-bit
@@ -523,18 +530,19 @@ class GalvatronDecoderLayer(nn.Module):
             return False
         s = att.spec
         F1 = mlp.Fl * (2 if s.gated else 1)
+        weights = self._step_weights()
         return (x.is_cuda and not torch.is_grad_enabled() and forward_ad._current_level < 0
                 and x.dtype == _lib.lp_dtype() and x.is_contiguous() and _PAIR_MODE != "1"
                 and x.dim() == 3 and x.shape[2] == s.hidden
-                and att.linear_qkv.weight.shape == ((att.nh + 2 * att.ng) * att.hd, s.hidden)
-                and att.linear_proj.weight.shape == (s.hidden, att.nh * att.hd)
-                and mlp.linear_fc1.weight.shape == (F1, s.hidden) and mlp.linear_fc2.weight.shape == (s.hidden, mlp.Fl)
+                and [tuple(w.shape) for w in weights[::2]] == [
+                    (s.hidden,), ((att.nh + 2 * att.ng) * att.hd, s.hidden), (s.hidden, att.nh * att.hd),
+                    (s.hidden,), (F1, s.hidden), (s.hidden, mlp.Fl)]
                 and x.data_ptr() % 16 == 0 and 0 < x.shape[0] * x.shape[1] <= NATIVE_STEP_ROWS
                 and c.tp_size == c.sp_size == c.cp_size == 1
                 and att.q_layernorm is None and att.hd in (64, 128) and att.hd * att.nh % 8 == 0
                 and not (s.hidden_dropout > 0.0 and self.training)
                 and all(p.dtype == x.dtype and p.device == x.device and p.is_contiguous() and p.data_ptr() % 16 == 0
-                        for p in self.parameters())
+                        for p in weights if p is not None)
                 and not any(m._forward_hooks or m._forward_pre_hooks or "forward" in vars(m) for m in mods)
                 and not (tm._global_forward_hooks or tm._global_forward_pre_hooks))
 
@@ -551,13 +559,11 @@ class GalvatronDecoderLayer(nn.Module):
         if not ops.attention.caches_usable(x, kc, vc, past, S, b0, B, att.ng, att.hd):
             return self.ffn(self.attn(x), x)
         n1, n2 = self.attn.input_layernorm, self.ffn.post_attention_layernorm
-        out = torch.empty_like(x)
+        out, weights = torch.empty_like(x), self._step_weights()
         d = _lib.DecoderStep(
             S, B, H, att.nh, att.ng, att.hd, mlp.Fl, past, int(n1.rms), _KIND[s.activation],
             2 * cos.shape[1] if cos is not None else 0, int(s.rope_interleaved), n1.eps, 1.0 / math.sqrt(att.hd),
-            *[_lib.ptr(t) for t in (n1.weight, n1.bias, att.linear_qkv.weight, att.linear_qkv.bias, att.linear_proj.weight,
-                                    att.linear_proj.bias, n2.weight, n2.bias, mlp.linear_fc1.weight, mlp.linear_fc1.bias,
-                                    mlp.linear_fc2.weight, mlp.linear_fc2.bias, cos, sin, kc[:, b0:], vc[:, b0:])],
+            *[_lib.ptr(t) for t in (*weights, cos, sin, kc[:, b0:], vc[:, b0:])],
             kc.stride(0), kc.stride(1), vc.stride(0), vc.stride(1), x.data_ptr(), out.data_ptr())
         lib = _lib.load()
         d.ws_bytes = lib.hg_decoder_step_scratch(ctypes.byref(d))

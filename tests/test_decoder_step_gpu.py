@@ -138,3 +138,24 @@ def test_attention_of_another_kind():
     x = torch.randn(1, 1, 256, device=DEV).to(torch.bfloat16)
     with torch.no_grad():
         assert torch.equal(m(x), m.ffn(x, x))
+
+
+def test_native_step_with_a_weight_that_is_computed():
+    """A parametrized weight is a new tensor at every access: it has to live until the kernels that read it are launched."""
+    from torch.nn.utils import parametrize
+
+    class Scaled(torch.nn.Module):
+        def forward(self, w):
+            return w * 2
+
+    m, x = layer("RMSNorm", "swiglu", "rope", False, 4, 4, 64), torch.randn(1, 1, 256, device=DEV).to(torch.bfloat16)
+    got = []
+    for native in (True, False):
+        m.attn.attention.inference_context = StaticInferenceContext(1, 8)
+        if native:
+            parametrize.register_parametrization(m.attn.attention.linear_proj, "weight", Scaled())
+        with torch.no_grad():
+            assert m._takes_native_step(x)
+            got.append(m(x) if native else m.ffn(m.attn(x), x))
+    assert torch.equal(*got)
+    _lib.assert_healthy()
