@@ -47,6 +47,7 @@ struct HgDecoderStep {
   void* out;
   void* ws;
   long long ws_bytes;
+  int launches;                            // set by hg_decoder_step: kernels that it has launched
 };
 
 }  // extern "C"
@@ -110,7 +111,7 @@ long long hg_decoder_step_scratch(const HgDecoderStep* d) {
   return carve(*d, dummy).bytes;
 }
 
-int hg_decoder_step(const HgDecoderStep* dp, void* stream) {
+int hg_decoder_step(HgDecoderStep* dp, void* stream) {
   const HgDecoderStep& d = *dp;
   if (!valid(d)) return -1;
   const Buffers b = carve(d, static_cast<char*>(d.ws));
@@ -138,6 +139,7 @@ int hg_decoder_step(const HgDecoderStep* dp, void* stream) {
   if ((rc = hg_gemm_skinny_bf16(b.norm, d.w_fc1, b.fc1, d.b_fc1, T, F1, d.H, d.H, d.H, F1, 0, 0, 0, stream))) return rc;
   if ((rc = hg_glu_fwd(b.fc1, b.act, T, d.F, d.act, stream))) return rc;
   if ((rc = hg_gemm_skinny_bf16(b.act, d.w_fc2, b.mlp, d.b_fc2, T, d.H, d.F, d.F, d.F, d.H, 0, 0, 0, stream))) return rc;
+  dp->launches = b.part_floats > 0 ? 11 : 10;   // two for attention whose keys are spread over several ranges, else one
   return hg_add_bf16(b.h, b.mlp, d.out, (long long)T * d.H, stream);
 }
 

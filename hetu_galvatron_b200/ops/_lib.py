@@ -68,7 +68,7 @@ class DecoderStep(ctypes.Structure):
                 [(n, c_void_p) for n in ("w_norm1", "b_norm1", "w_qkv", "b_qkv", "w_proj", "b_proj", "w_norm2", "b_norm2",
                                          "w_fc1", "b_fc1", "w_fc2", "b_fc2", "cos_t", "sin_t", "k_cache", "v_cache")] +
                 [(n, c_ll) for n in ("k_ss", "k_sb", "v_ss", "v_sb")] +
-                [("x", c_void_p), ("out", c_void_p), ("ws", c_void_p), ("ws_bytes", c_ll)])
+                [("x", c_void_p), ("out", c_void_p), ("ws", c_void_p), ("ws_bytes", c_ll), ("launches", c_int)])
 
 
 _SIGNATURES = {

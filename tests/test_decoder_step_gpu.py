@@ -159,3 +159,18 @@ def test_native_step_with_a_weight_that_is_computed():
             got.append(m(x) if native else m.ffn(m.attn(x), x))
     assert torch.equal(*got)
     _lib.assert_healthy()
+
+
+# one key range, the tile kernel, several ranges and their merge
+@pytest.mark.parametrize("B,past,launches", [(4, 3, 10), (1, 500, 10), (1, 1600, 11), (64, 100, 11), (64, 3, 10)])
+def test_launches_of_the_native_step(B, past, launches):
+    m, x = layer("RMSNorm", "swiglu", "rope", False, 8, 8, 64), torch.randn(1, B, 512, device=DEV).to(torch.bfloat16)
+    for native in (True, False):
+        ic = StaticInferenceContext(B, past + 1)
+        ic.sequence_len_offset = past
+        m.attn.attention.inference_context = ic
+        with torch.no_grad():
+            before = _lib.launches()
+            m(x) if native else m.ffn(m.attn(x), x)
+            assert _lib.launches() - before == launches
+    _lib.assert_healthy()
