@@ -52,7 +52,9 @@ def _use_skinny(M: int, N: int, K: int, a_mn: bool, out_mode: int, max_ctas: int
     K = 2048 23.6 against 21.9, 3072 24.8 against 28.5; 16384 columns x 4096 41.5 against 39.5)."""
     if a_mn or out_mode not in (OUT_BF16, OUT_F32) or pair is not None or max_ctas != 0 or _PAIR_MODE == "1":
         return False
-    return M <= NATIVE_STEP_ROWS or (M <= 128 and N <= 8192 and K >= (1536 if N <= 4096 else 3072))
+    if M <= NATIVE_STEP_ROWS:
+        return N <= 65535 * 128                          # its grid has one y index per 128 columns
+    return M <= 128 and N <= 8192 and K >= (1536 if N <= 4096 else 3072)
 
 
 def _use_pair(M: int, N: int, pair) -> bool:

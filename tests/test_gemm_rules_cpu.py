@@ -1,0 +1,19 @@
+"""Which kernel a product goes to, on both sides of each line of the rules."""
+import pytest
+
+from hetu_galvatron_b200.ops.gemm import OUT_BF16, _use_grouped_pair, _use_skinny
+
+
+# the last two: as many columns as the few-row kernel's grid has tiles for, and one more
+@pytest.mark.parametrize("M,N,K,few_rows", [(64, 512, 512, True), (65, 512, 512, False), (128, 4096, 1535, False),
+                                            (128, 4096, 1536, True), (128, 8192, 3064, False), (128, 8192, 3072, True),
+                                            (128, 8200, 4096, False), (129, 512, 4096, False), (1, 65535 * 128, 64, True),
+                                            (1, 65535 * 128 + 1, 64, False)])
+def test_rule_of_the_few_row_kernel(M, N, K, few_rows):
+    assert _use_skinny(M, N, K, False, OUT_BF16, 0, None) is few_rows
+
+
+@pytest.mark.parametrize("rows,N,K,G,pair", [(4096, 4096, 2560, 8, True), (4095, 4096, 2560, 8, False), (4096, 4096, 2552, 8, False),
+                                             (4096, 255, 4096, 8, False), (512, 256, 4096, 1, True)])
+def test_rule_of_the_grouped_pair_kernel(rows, N, K, G, pair):
+    assert _use_grouped_pair(rows, N, K, G) is pair

@@ -50,15 +50,6 @@ def test_skinny_gemm_around_its_split_lengths(M, N, K):
     _lib.assert_healthy()
 
 
-@pytest.mark.parametrize("M,N,K,few_rows", [(64, 512, 512, True), (65, 512, 512, False), (128, 4096, 1535, False),
-                                            (128, 4096, 1536, True), (128, 8192, 3064, False), (128, 8192, 3072, True),
-                                            (128, 8200, 4096, False), (129, 512, 4096, False)])
-def test_rule_of_the_few_row_kernel(M, N, K, few_rows):
-    from hetu_galvatron_b200.ops.gemm import OUT_BF16, _use_skinny
-
-    assert _use_skinny(M, N, K, False, OUT_BF16, 0, None) is few_rows
-
-
 def test_skinny_gemm_writes_only_its_rows_of_a_wider_output():
     M, N, K = 5, 200, 512
     x = torch.randn(M, K, device=DEV).to(torch.bfloat16)

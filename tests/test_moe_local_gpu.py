@@ -226,11 +226,3 @@ def test_grouped_gemm_of_ragged_segments(monkeypatch, seg, N, K, b_mn, pair):
     out[first:starts[-1]] = 3.0
     assert (whole == 3.0).all()
     _lib.assert_healthy()
-
-
-@pytest.mark.parametrize("rows,N,K,G,pair", [(4096, 4096, 2560, 8, True), (4095, 4096, 2560, 8, False), (4096, 4096, 2552, 8, False),
-                                             (4096, 255, 4096, 8, False), (512, 256, 4096, 1, True)])
-def test_rule_of_the_grouped_pair_kernel(rows, N, K, G, pair):
-    from hetu_galvatron_b200.ops.gemm import _use_grouped_pair
-
-    assert _use_grouped_pair(rows, N, K, G) is pair
