@@ -12,7 +12,7 @@
 // galvatron/core/runtime/transformer/attention_impl.py:55-111,587-616,696-727.
 #include <type_traits>
 
-#include "attn_tensor.h"
+#include "entry_points.h"
 #include "sm100_common.cuh"
 
 namespace hg {

@@ -8,29 +8,10 @@
 // that: a decode step of four 4096-wide layers, 4 sequences at 1000 cached positions, 1965 us launched one by one, 583
 // us from here with the attention kernels of flash_decode.cu (embedding, head and sampling included).  Host code
 // only.
-#include "attn_tensor.h"
+#include "entry_points.h"
 #include "sm100_common.cuh"
 
 extern "C" {
-
-int hg_norm_fwd(const void* x, const void* residual, const void* w, const void* b, void* y, void* h_out, void* rstd,
-                void* mean, int rows, int H, float eps, int rms, void* stream);
-int hg_gemm_skinny_bf16(const void* x, const void* W, void* C, const void* bias, int M, int N, int K, int ldx, int ldw,
-                        int ldc, int w_mn, int out_mode, int splits, void* stream);
-int hg_rope_append(void* qkv, int tokens, int batch, int ng, int qpg, int hd, int pos_offset, const void* cos_t,
-                   const void* sin_t, int rot_dim, int interleaved, void* kc, void* vc, long long k_ss, long long k_sb,
-                   long long v_ss, long long v_sb, void* stream);
-long long hg_flash_decode_scratch(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, int Sq, int Skv, int B,
-                                  int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0);
-int hg_flash_decode_pays(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0);
-int hg_flash_decode(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o, void* lse,
-                    void* ws, int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0,
-                    float scale, void* stream);
-int hg_flash_fwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o, void* lse,
-                 int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0, float scale,
-                 void* stream);
-int hg_glu_fwd(const void* y, void* out, long long rows, int F, int kind, void* stream);
-int hg_add_bf16(const void* a, const void* b, void* out, long long n, void* stream);
 
 // Mirrored by ``DecoderStep`` in ops/_lib.py.  x and out are [S * B, H] contiguous (S tokens of B sequences, S * B <= 128);
 // the caches point at the first of the B sequences, position 0, and `past` positions of them are filled.

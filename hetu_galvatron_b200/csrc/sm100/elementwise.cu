@@ -3,6 +3,7 @@
 // Oracles: galvatron/core/runtime/transformer/rope_utils.py:86-120 (rotate-half form),
 // galvatron/core/runtime/transformer/fused_kernels.py:19-48,142-168 (activations),
 // galvatron/core/runtime/tensor_parallel/layers.py:120-147 (masked vocab-parallel lookup).
+#include "entry_points.h"
 #include "sm100_common.cuh"
 
 namespace {

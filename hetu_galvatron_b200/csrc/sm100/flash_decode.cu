@@ -10,7 +10,7 @@
 //
 // Rows: r = s * qpg + j is query token s of query head g * qpg + j.  A lane holds eight channels, so HD / 8 lanes share a
 // key and a warp reads 32 / (HD / 8) keys per 16-byte access.
-#include "attn_tensor.h"
+#include "entry_points.h"
 #include "sm100_common.cuh"
 
 namespace {

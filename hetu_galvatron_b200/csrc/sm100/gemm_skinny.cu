@@ -17,6 +17,7 @@
 // = output column, so a warp stores 32 consecutive elements of a token's row).
 #include <mutex>
 
+#include "entry_points.h"
 #include "gemm_core.cuh"
 
 namespace hg {

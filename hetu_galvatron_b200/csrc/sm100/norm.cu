@@ -3,6 +3,7 @@
 // between the statistics pass and the normalisation pass.
 // Replaces the flash-attn RMSNorm / DropoutAddLayerNorm extension calls of
 // galvatron/core/runtime/transformer/norm.py:6-29.
+#include "entry_points.h"
 #include "sm100_common.cuh"
 
 namespace {
