@@ -82,8 +82,9 @@ def _counts(tensors):
 
 def sumsq_list(terms, out: torch.Tensor, accumulate: bool = True):
     """``out[0] (+)= sum(scale * sum(x^2))`` over ``terms`` of ``(x, scale)`` with a fixed reduction order: two launches
-    for up to ``hg_list_capacity()`` fp32 CUDA buffers."""
-    if not terms or not out.is_cuda or any(x.dtype != torch.float32 or not x.is_contiguous() for x, _ in terms):
+    for up to ``hg_list_capacity()`` fp32 buffers on ``out``'s GPU."""
+    if not terms or not out.is_cuda or any(x.device != out.device or x.dtype != torch.float32 or not x.is_contiguous()
+                                           for x, _ in terms):
         if not accumulate:
             out.zero_()
         for x, scale in terms:

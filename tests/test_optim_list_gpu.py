@@ -44,3 +44,12 @@ def test_list_step_equals_single_steps(sizes):
     ops.sumsq_list([(shifted, 1.0)], out, accumulate=False)
     assert abs(out.item() - shifted.double().pow(2).sum().item()) < 1e-2
     _lib.assert_healthy()
+
+
+def test_squared_norm_over_buffers_of_both_memories():
+    """A term in host memory is summed there, as by the one-buffer function."""
+    out = torch.full((1,), 5.0, device=DEV)
+    a, b = torch.randn(1000), torch.randn(777)
+    ops.sumsq_list([(a.to(DEV), 1.0), (b, 0.5)], out, accumulate=False)
+    assert abs(out.item() / (a.double().square().sum() + 0.5 * b.double().square().sum()).item() - 1) < 1e-5
+    _lib.assert_healthy()
