@@ -500,53 +500,55 @@ class GalvatronDecoderLayer(nn.Module):
         self.ffn.reset_parameters(seed, full_init)
 
     def forward(self, x):
-        att = getattr(self.attn, "attention", None)
-        if getattr(att, "inference_context", None) is not None and self._takes_native_step(x):
-            return self._native_step(x)
+        if getattr(getattr(self.attn, "attention", None), "inference_context", None) is not None:
+            weights = self._native_weights(x)
+            if weights is not None:
+                return self._native_step(x, weights)
         return self.ffn(self.attn(x), x)
 
-    def _step_weights(self):
-        """Weights and biases in the order of ``HgDecoderStep``.  A caller keeps the list until its kernels are launched: a
-        parametrized weight is a new tensor each time it is asked for."""
-        a, m = self.attn, self.ffn
-        return [t for h in (a.input_layernorm, a.attention.linear_qkv, a.attention.linear_proj, m.post_attention_layernorm,
-                            m.mlp.linear_fc1, m.mlp.linear_fc2) for t in (h.weight, h.bias)]
-
     def _takes_native_step(self, x) -> bool:
-        """A cached forward of few tokens whose kernels one native call can launch (csrc/sm100/decoder_step.cu): no
-        gradient in either mode, no parallelism inside the layer, its own modules with nothing hooked into them, 16-bit
-        contiguous tensors on one GPU."""
+        return self._native_weights(x) is not None
+
+    def _native_weights(self, x):
+        """The weights and biases of a cached forward of few tokens whose kernels one native call can launch
+        (csrc/sm100/decoder_step.cu), in the order of ``HgDecoderStep``, or None where it does not: no gradient in either mode,
+        no parallelism inside the layer, its own modules with nothing hooked into them, 16-bit contiguous tensors on one GPU.
+        The caller keeps the list until its kernels are launched: a parametrized weight is a new tensor at every access."""
         import torch.nn.modules.module as tm
         from torch.autograd import forward_ad
 
         from ..ops import _lib
         from ..ops.gemm import NATIVE_STEP_ROWS, _PAIR_MODE
 
-        if type(self.attn) is not GalvatronAttention or type(self.ffn) is not GalvatronMLP:
-            return False
-        att, mlp, c = self.attn.attention, self.ffn.mlp, self.ctx
-        mods = (self.attn, self.attn.input_layernorm, att, self.ffn, self.ffn.post_attention_layernorm, mlp)
-        if [type(m) for m in mods[1:]] != [Norm, SelfAttention, GalvatronMLP, Norm, MLP]:
-            return False
+        attn, ffn, c = self.attn, self.ffn, self.ctx
+        if type(attn) is not GalvatronAttention or type(ffn) is not GalvatronMLP:
+            return None
+        n1, att, n2, mlp = attn.input_layernorm, attn.attention, ffn.post_attention_layernorm, ffn.mlp
+        if [type(m) for m in (n1, att, n2, mlp)] != [Norm, SelfAttention, Norm, MLP]:
+            return None
         s = att.spec
-        F1 = mlp.Fl * (2 if s.gated else 1)
-        weights = self._step_weights()
-        return (x.is_cuda and not torch.is_grad_enabled() and forward_ad._current_level < 0
+        if not (x.is_cuda and not torch.is_grad_enabled() and forward_ad._current_level < 0
                 and x.dtype == _lib.lp_dtype() and x.is_contiguous() and _PAIR_MODE != "1"
                 and x.dim() == 3 and x.shape[2] == s.hidden
-                and [tuple(w.shape) for w in weights[::2]] == [
-                    (s.hidden,), ((att.nh + 2 * att.ng) * att.hd, s.hidden), (s.hidden, att.nh * att.hd),
-                    (s.hidden,), (F1, s.hidden), (s.hidden, mlp.Fl)]
                 and x.data_ptr() % 16 == 0 and 0 < x.shape[0] * x.shape[1] <= NATIVE_STEP_ROWS
                 and c.tp_size == c.sp_size == c.cp_size == 1
                 and att.q_layernorm is None and att.hd in (64, 128) and att.hd * att.nh % 8 == 0
                 and not (s.hidden_dropout > 0.0 and self.training)
+                and not any(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__
+                            for m in (attn, n1, att, ffn, n2, mlp))
+                and not (tm._global_forward_hooks or tm._global_forward_pre_hooks)):
+            return None
+        weights = [t for h in (n1, att.linear_qkv, att.linear_proj, n2, mlp.linear_fc1, mlp.linear_fc2)
+                   for t in (h.weight, h.bias)]
+        shapes = ((s.hidden,), ((att.nh + 2 * att.ng) * att.hd, s.hidden), (s.hidden, att.nh * att.hd), (s.hidden,),
+                  (mlp.Fl * (2 if s.gated else 1), s.hidden), (s.hidden, mlp.Fl))
+        if not (all(w.shape == shape for w, shape in zip(weights[::2], shapes))
                 and all(p.dtype == x.dtype and p.device == x.device and p.is_contiguous() and p.data_ptr() % 16 == 0
-                        for p in weights if p is not None)
-                and not any(m._forward_hooks or m._forward_pre_hooks or "forward" in vars(m) for m in mods)
-                and not (tm._global_forward_hooks or tm._global_forward_pre_hooks))
+                        for p in weights if p is not None)):
+            return None
+        return weights
 
-    def _native_step(self, x):
+    def _native_step(self, x, weights):
         import ctypes
 
         from ..ops import _lib
@@ -559,7 +561,7 @@ class GalvatronDecoderLayer(nn.Module):
         if not ops.attention.caches_usable(x, kc, vc, past, S, b0, B, att.ng, att.hd):
             return self.ffn(self.attn(x), x)
         n1, n2 = self.attn.input_layernorm, self.ffn.post_attention_layernorm
-        out, weights = torch.empty_like(x), self._step_weights()
+        out = torch.empty_like(x)
         d = _lib.DecoderStep(
             S, B, H, att.nh, att.ng, att.hd, mlp.Fl, past, int(n1.rms), _KIND[s.activation],
             2 * cos.shape[1] if cos is not None else 0, int(s.rope_interleaved), n1.eps, 1.0 / math.sqrt(att.hd),
