@@ -31,3 +31,25 @@ def test_every_store_of_the_pair_kernel(M, N, K, mode, shift):
     if packed is not None:
         assert ((packed.double() - ref).norm() / ref.norm()).item() < (1e-5 if dt == torch.float32 else 2.0 ** -8)
     _lib.assert_healthy()
+
+
+# C as a window that a tensor map covers (its pitch, width and first column whole 16-byte groups): columns that end in a
+# box of 64, in a tile and on its edge, rows that end in a block of 32 and on its edge, more tiles than pairs
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (300, 328, 72), (257, 1000, 136), (321, 8, 64), (2600, 2568, 64)])
+@pytest.mark.parametrize("left,right", [(0, 8), (8, 8), (8, 64)])
+@pytest.mark.parametrize("a_mn", [False, True])
+def test_tma_stores_stay_inside_their_window(M, N, K, left, right, a_mn):
+    if a_mn and M % 8:
+        pytest.skip("rows of an M-major operand are whole 16-byte groups")
+    g = torch.Generator(device=DEV).manual_seed(M + N + left)
+    a, b = (torch.randn(n, K, device=DEV, generator=g).to(torch.bfloat16) for n in (M, N))
+    bias = torch.randn(N, device=DEV, generator=g).to(torch.bfloat16)
+    whole = torch.full((M + 34, left + N + right), 2.0, device=DEV, dtype=torch.bfloat16)
+    out = whole[1:M + 1, left:left + N]
+    assert out.stride(0) % 8 == 0 and N % 8 == 0 and out.data_ptr() % 16 == 0     # what the tensor map asks for
+    ops.gemm(a.t().contiguous() if a_mn else a, b, out=out, a_mn=a_mn, bias=bias, pair=True)
+    ref = a.double() @ b.double().t() + bias.double()
+    assert torch.allclose(out.double(), ref, rtol=2.0 ** -8, atol=1e-4 * K ** 0.5)  # one rounding; fp32 sums of K products
+    out.fill_(2.0)
+    assert (whole == 2.0).all()
+    _lib.assert_healthy()

@@ -218,11 +218,17 @@ def test_grouped_gemm_of_ragged_segments(monkeypatch, seg, N, K, b_mn, pair):
     b = torch.randn(len(seg), *((K, N) if b_mn else (N, K)), device=DEV, generator=g).to(torch.bfloat16)
     whole = torch.full((rows + 2, N), 3.0, device=DEV, dtype=torch.bfloat16)
     out = whole[1:rows + 1]
-    ops.grouped_gemm(a, b, torch.tensor(starts, device=DEV, dtype=torch.int32), b_mn=b_mn, out=out)
+    row_start = torch.tensor(starts, device=DEV, dtype=torch.int32)
+    ops.grouped_gemm(a, b, row_start, b_mn=b_mn, out=out)
     for i, n in enumerate(seg):
         ref = a[starts[i]:starts[i + 1]].double() @ (b[i].double() if b_mn else b[i].double().t())
         got = out[starts[i]:starts[i + 1]].double()
         assert torch.allclose(got, ref, rtol=2.0 ** -8, atol=1e-4 * K ** 0.5)   # one rounding; fp32 sums of K products
+    junk = torch.full((rows, N), float("nan"), device=DEV, dtype=torch.bfloat16)
+    del junk                                                    # the allocator hands these bytes out again
+    fresh = ops.grouped_gemm(a, b, row_start, b_mn=b_mn)
+    assert torch.equal(fresh[first:starts[-1]], out[first:starts[-1]])
+    assert (fresh[:first] == 0).all() and (fresh[starts[-1]:] == 0).all()
     out[first:starts[-1]] = 3.0
     assert (whole == 3.0).all()
     _lib.assert_healthy()
