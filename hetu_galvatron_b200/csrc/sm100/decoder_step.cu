@@ -3,11 +3,12 @@
 //   n = norm(x);  qkv = n Wqkv^T;  rotate, append to the cache, attend;  a = ctx Wproj^T
 //   h = x + a;  out = h + act(norm(h) W1^T) W2^T
 //
-// The kernels are the ones the layer's modules launch one by one.  A decode step of a 7B-sized layer keeps the GPU busy
-// for about 100 us; eleven launches through the tensor library and the autograd wrappers took the host several times
-// that: a decode step of four 4096-wide layers, 4 sequences at 1000 cached positions, 1965 us launched one by one, 583
-// us from here with the attention kernels of flash_decode.cu (embedding, head and sampling included).  Host code
-// only.
+// The kernels are the ones the layer's modules launch one by one: ten, or eleven where the keys of cached attention are
+// spread over several ranges (flash_decode.cu).  A decode step of a 7B-sized layer keeps the GPU busy for about 110 us;
+// launched through the tensor library and the autograd wrappers it takes the host several times that.  Four 4096-wide
+// layers, 4 sequences at 1000 cached positions, embedding and head included: 1400 us a step when each is waited for, 770 us
+// from here; one after another 590 us, of which 517 us are kernels (attention on the tile kernel, products on
+// gemm_skinny.cu).  Host code only.
 #include "entry_points.h"
 #include "sm100_common.cuh"
 
