@@ -518,6 +518,10 @@ class ShardedUnit:
                 terms.append((g[a - lo:b - lo], inv / rep * (1.0 / self.tp_n - 1.0)))
         return terms
 
+    def has_own_grad_sumsq(self) -> bool:
+        """Whether :meth:`grad_sumsq` has been replaced, so that :meth:`norm_terms` need not be what it adds."""
+        return type(self).grad_sumsq is not ShardedUnit.grad_sumsq or "grad_sumsq" in vars(self)
+
     def grad_sumsq(self, out: torch.Tensor):
         """Add this rank's share of the squared gradient norm (:meth:`norm_terms`) to ``out[0]``."""
         for x, scale in self.norm_terms():
@@ -526,8 +530,10 @@ class ShardedUnit:
     # ---- optimizer --------------------------------------------------------------------------------------
     def takes_list_step(self) -> bool:
         """Whether this unit's update is AdamW on its own buffers and nothing else (no parameter exchange, fp32 gradient
-        and 16-bit parameters on a GPU), so that it can share a launch with other units."""
-        return (bool(self.params) and not self.fused and self.dp_type == "ddp" and self.device.type == "cuda"
+        and 16-bit parameters on a GPU), so that it can share a launch with other units; not where :meth:`optimizer_step` has
+        been replaced."""
+        return (type(self).optimizer_step is ShardedUnit.optimizer_step and "optimizer_step" not in vars(self)
+                and bool(self.params) and not self.fused and self.dp_type == "ddp" and self.device.type == "cuda"
                 and self.dtype in (torch.bfloat16, torch.float16) and self.grad_shard.dtype == torch.float32
                 and all(t.data_ptr() % 16 == 0 for t in (self.master, self.grad_shard, self.exp_avg, self.exp_avg_sq,
                                                          self.shard_lp)))

@@ -68,7 +68,10 @@ class ShardedAdamW:
             REDUCE.join(self.units[0].device)
 
     def compute_grad_norm(self):
-        ops.sumsq_list([t for u in self.units for t in u.norm_terms()], self._sumsq, accumulate=False)
+        own = [u for u in self.units if u.has_own_grad_sumsq()]
+        ops.sumsq_list([t for u in self.units if u not in own for t in u.norm_terms()], self._sumsq, accumulate=False)
+        for u in own:
+            u.grad_sumsq(self._sumsq)
         if dist.is_initialized() and dist.get_world_size() > 1:
             dist.all_reduce(self._sumsq)
         ops.clip_coefficient(self._sumsq, self.clip_grad, self._coef, self._norm)

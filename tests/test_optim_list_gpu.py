@@ -53,3 +53,43 @@ def test_squared_norm_over_buffers_of_both_memories():
     ops.sumsq_list([(a.to(DEV), 1.0), (b, 0.5)], out, accumulate=False)
     assert abs(out.item() / (a.double().square().sum() + 0.5 * b.double().square().sum()).item() - 1) < 1e-5
     _lib.assert_healthy()
+
+
+class _TwiceTheNorm:
+    """Replaced methods of a unit: a norm that counts twice, a step that only counts its calls."""
+
+    steps = 0
+
+    def grad_sumsq(self, out):
+        for x, scale in self.norm_terms():
+            ops.sumsq(x, out, accumulate=True, scale=2.0 * scale)
+
+    def optimizer_step(self, *args, **kwargs):
+        self.steps += 1
+
+
+@pytest.mark.parametrize("device", ["cpu", DEV])
+@pytest.mark.parametrize("by", ["class", "instance"])
+def test_replaced_methods_of_a_unit_are_called(device, by):
+    from hetu_galvatron_b200.parallel.zero import ShardedUnit
+    from hetu_galvatron_b200.runtime.optimizer import ShardedAdamW
+
+    units = []
+    for own in (False, True):
+        lin = torch.nn.Linear(64, 32, bias=False, device=device, dtype=torch.bfloat16)
+        cls = type("Own", (_TwiceTheNorm, ShardedUnit), {}) if own and by == "class" else ShardedUnit
+        u = cls(lin, "unit", None, 1)
+        if own and by == "instance":
+            u.steps = 0
+            u.grad_sumsq = _TwiceTheNorm.grad_sumsq.__get__(u)
+            u.optimizer_step = _TwiceTheNorm.optimizer_step.__get__(u)
+        u.reload_master()
+        u.main_grad.fill_(0.5)
+        for p in u.params:
+            p.mg_fresh = False
+        units.append(u)
+    before = [u.master.clone() for u in units]
+    opt = ShardedAdamW(units, lr=1e-2, clip_grad=1.0)
+    opt.step()
+    assert abs(opt._norm.item() - (64 * 32 * 0.25 * 3) ** 0.5) < 1e-3
+    assert not torch.equal(units[0].master, before[0]) and torch.equal(units[1].master, before[1]) and units[1].steps == 1
