@@ -600,8 +600,6 @@ class GalvatronMoEMLP(nn.Module):
         k, E, ep, E_loc = s.topk, s.experts, c.ep_size, self.experts.E_loc
         if local_only:
             E, ep = E_loc, 1
-        if probs.numel() < idx.numel():
-            raise IndexError("%d routing weights for %d (token, expert) pairs" % (probs.numel(), idx.numel()))
         # "flex" is the reference's fused dispatcher (DeepEP, moe/token_dispatcher.py:743-1037); here it selects the
         # peer-memory pull kernels, which the fused-communication switch also turns on for "alltoall"
         if ep > 1 and (getattr(c, "fused_comm", False) or s.dispatcher == "flex"):
@@ -617,6 +615,8 @@ class GalvatronMoEMLP(nn.Module):
                 w = torch.where(idx >= 0, probs, torch.zeros_like(probs)).to(torch.float32)
                 # the routing weights are applied inside the pull kernel: no [T, k, H] intermediate
                 return fa.moe_combine_weighted(out_buf, w, plan)
+        if probs.numel() < idx.numel():
+            raise IndexError("%d routing weights for %d (token, expert) pairs" % (probs.numel(), idx.numel()))
         # pairs that other ranks serve are dropped here: the static bound of the kernels' buffer would hold those of all
         # ranks, where the general path counts this rank's own
         if ep == 1 and not local_only and local_dispatch_usable(x2d, probs, idx, E, k):
