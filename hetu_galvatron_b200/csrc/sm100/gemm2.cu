@@ -189,6 +189,10 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
       }
       return true;
     });
+    for (int i = 0; ok && i < STAGES2; ++i) {       // as in producer2
+      ok = mbar_wait_warp(&s.empty[stage], phase ^ 1, p.status, kTimeoutSmemEmpty, s.abort);
+      if (++stage == STAGES2) { stage = 0; phase ^= 1; }
+    }
     if (!ok) {
       *s.abort = 1;
       const uint64_t t0 = globaltimer_ns();
@@ -395,12 +399,13 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   return int(e);
 }
 
-// The tensor map of C for the plain 16-bit store (p.c_tma says whether it is used; `any` fills the kernel's parameter else).
+// The tensor map of C for the plain stores (p.c_tma says whether it is used; `any` fills the kernel's parameter else).
 static int store_map(CUtensorMap* tc, const CUtensorMap& any, Params& p, uint64_t rows) {
   p.c_tma = 0;
   *tc = any;
-  if (p.out_mode != kOutBf16) return 0;
-  const int rc = hg_host::make_tmap_2d_store(tc, p.C, rows, uint64_t(p.N), uint64_t(p.ldc));
+  if (p.out_mode != kOutBf16 && p.out_mode != kOutF32) return 0;
+  const int rc = p.out_mode == kOutF32 ? hg_host::make_tmap_2d_store_f32(tc, p.C, rows, uint64_t(p.N), uint64_t(p.ldc))
+                                       : hg_host::make_tmap_2d_store(tc, p.C, rows, uint64_t(p.N), uint64_t(p.ldc));
   if (rc == 0) p.c_tma = 1;
   else *tc = any;
   return rc < 0 ? rc : 0;

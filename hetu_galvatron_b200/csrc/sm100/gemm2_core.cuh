@@ -204,6 +204,11 @@ __device__ __forceinline__ void producer2(const CUtensorMap* tmA, const CUtensor
       if (++stage == STAGES2) { stage = 0; phase ^= 1; }
     }
   }
+  // The leader's commits arrive on this CTA's barriers: leave only when the last of them has.
+  for (int i = 0; ok && i < STAGES2; ++i) {
+    ok = mbar_wait_warp(&s.empty[stage], phase ^ 1, p.status, kTimeoutSmemEmpty, s.abort);
+    if (++stage == STAGES2) { stage = 0; phase ^= 1; }
+  }
   if (!ok) {
     *s.abort = 1;
     if (rank == 0) {
@@ -267,14 +272,14 @@ __device__ __forceinline__ void mma2(const Params& p, const Smem2& s, uint32_t t
 // Plain 16-bit stores: 32 rows x 128 bytes are written to the warp's stage in the layout of the 128-byte
 // swizzle, eight conflict-free 16-byte stores per thread, and leave as one TMA store that clips at the matrix' edges;
 // two blocks alternate, so that one is filled while the other is read.
-// Anything else (fp32 results, accumulating modes, an unaligned C, the ragged end of an expert's rows, a tile shared along
-// K): a 32 x 32 fp32 block at a time through 36-word rows (conflict-free 16-byte accesses both ways), eight lanes on 32
-// consecutive columns of a row, four elements each, all loads of a block before its first store.  (fp32 results by TMA
-// store were slower: expert weight gradients 4.14 against 3.13 ms.)
+// fp32 results and accumulating modes: a 32 x 32 fp32 block at a time through 36-word rows (conflict-free 16-byte
+// accesses both ways), eight lanes on 32 consecutive columns of a row, four elements each, all loads of a block before its
+// first store.  (fp32 results by TMA store were slower: expert weight gradients 4.14 against 3.13 ms.)
 //
-// Before, every mode took the second path row by row through generic pointers, where the compiler has to order each
-// shared-memory read behind the previous row's global store: 9.9 us for the 16-bit and 8.7 us for the fp32 store of a
-// 256 x 256 tile, hidden only under more than thirty k-blocks.
+// What an epilogue costs is instructions, not bytes, and every decision that can be taken once per tile is taken there:
+// whether there is a bias, the output mode, whole or clipped blocks.  Decided per element they were 64 branches around
+// loads that never ran, 2700 cycles of a 64-column block (by clock64()), 5.6 us of every tile: 256 x 256 x 64 12.9 us,
+// 8192 x 8192 x 512 111 us.
 __device__ __forceinline__ void sts128(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
@@ -310,26 +315,64 @@ __device__ __forceinline__ void tma_store_rows(const CUtensorMap* tm, StoreStage
   st.next ^= 1;
 }
 
-// A 32 x 64 block from registers (thread = row) through the tensor map.
-__device__ __forceinline__ void store_block64_tma(const Params& p, const CUtensorMap* tm, StoreStage& st, int y0, int col0,
-                                                  const uint32_t (&r0)[32], const uint32_t (&r1)[32]) {
-  auto add_bias = [&](const uint32_t (&r)[32], int c, uint32_t (&v)[32]) {
+// The bias of N consecutive columns from col0 on, added to a thread's row.  Every lane reads the same 16 bytes.
+template <int N>
+__device__ __forceinline__ void add_bias_row(const Params& p, int col0, uint32_t* r) {
+  const hg_lp_t* src = p.bias + col0;
+  if (col0 + N <= p.N && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) {
-      const float b = p.bias != nullptr && c + i < p.N ? hg_lp2f(p.bias[c + i]) : 0.f;
-      v[i] = p.bias != nullptr ? __float_as_uint(__uint_as_float(r[i]) + b) : r[i];
+    for (int q = 0; q < N / 8; ++q) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(src) + q);
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 b = hg_unpack2(w[j]);
+        r[q * 8 + 2 * j] = __float_as_uint(__uint_as_float(r[q * 8 + 2 * j]) + b.x);
+        r[q * 8 + 2 * j + 1] = __float_as_uint(__uint_as_float(r[q * 8 + 2 * j + 1]) + b.y);
+      }
     }
-  };
-  uint32_t v0[32], v1[32];
-  add_bias(r0, col0, v0);
-  add_bias(r1, col0 + 32, v1);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (col0 + i < p.N) r[i] = __float_as_uint(__uint_as_float(r[i]) + hg_lp2f(src[i]));
+  }
+}
+
+// A 32 x 64 block from registers (thread = row) through the tensor map.
+template <bool BIAS>
+__device__ __forceinline__ void store_block64_tma(const Params& p, const CUtensorMap* tm, StoreStage& st, int y0, int col0,
+                                                  uint32_t (&r0)[32], uint32_t (&r1)[32]) {
+  if (BIAS) {
+    add_bias_row<32>(p, col0, r0);
+    add_bias_row<32>(p, col0 + 32, r1);
+  }
   uint32_t w[32];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    w[i] = pack_bf16(__uint_as_float(v0[2 * i]), __uint_as_float(v0[2 * i + 1]));
-    w[16 + i] = pack_bf16(__uint_as_float(v1[2 * i]), __uint_as_float(v1[2 * i + 1]));
+    w[i] = pack_bf16(__uint_as_float(r0[2 * i]), __uint_as_float(r0[2 * i + 1]));
+    w[16 + i] = pack_bf16(__uint_as_float(r1[2 * i]), __uint_as_float(r1[2 * i + 1]));
   }
   tma_store_rows(tm, st, w, col0, y0);
+}
+
+// Columns n0.. of the tile as TMA stores of 128-byte rows: 64 columns of 16 bits, or 32 of fp32.
+template <bool BIAS, bool F32>
+__device__ __forceinline__ void store_tile_tma(const Params& p, const CUtensorMap* tmC, StoreStage& st, uint32_t src, int row0,
+                                               int y0, int n0) {
+#pragma unroll 1
+  for (int c = 0; c < BN && n0 + c < p.N; c += F32 ? 32 : 64) {
+    uint32_t r0[32], r1[32];
+    tmem_ld32(src + c, r0);
+    if (!F32) tmem_ld32(src + c + 32, r1);
+    tmem_ld_wait();
+    if (!HG_BOUNDS_OK(row0 >= 0 && row0 < p.M, p.status)) continue;
+    if constexpr (F32) {
+      if (BIAS) add_bias_row<32>(p, n0 + c, r0);
+      tma_store_rows(tmC, st, r0, n0 + c, y0);
+    } else {
+      store_block64_tma<BIAS>(p, tmC, st, y0, n0 + c, r0, r1);
+    }
+  }
 }
 
 // Row by row: lane l works on columns 4 (l % 8) .. + 3 of rows l / 8, l / 8 + 4, ... of a 32 x 32 block.
@@ -439,20 +482,91 @@ __device__ __forceinline__ void store_block_rows(const Params& p, uint32_t stg, 
   }
 }
 
+// One whole 32 x 32 block from registers (thread = row): no edge in it, four elements per access.
+template <int MODE>
+__device__ __forceinline__ void store_block_whole(const Params& p, uint32_t stg, int row0, int col0, const uint32_t (&src)[32],
+                                                  const float4 (&old)[8]) {
+  const int lane = int(lane_id());
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    sts128(stg + lane * 144 + j * 16, src[4 * j], src[4 * j + 1], src[4 * j + 2], src[4 * j + 3]);
+  __syncwarp();
+  const int q = (lane & 7) * 4;
+  float4 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = lds128(stg + (i * 4 + (lane >> 3)) * 144 + q * 4);
+  __syncwarp();
+  if (!HG_BOUNDS_OK(row0 >= 0 && row0 + 32 <= p.M && col0 >= 0 && col0 + 32 <= p.N, p.status)) return;
+  float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (p.bias != nullptr)
+    b = make_float4(hg_lp2f(p.bias[col0 + q]), hg_lp2f(p.bias[col0 + q + 1]), hg_lp2f(p.bias[col0 + q + 2]),
+                    hg_lp2f(p.bias[col0 + q + 3]));
+  const size_t at = size_t(row0 + (lane >> 3)) * p.ldc + col0 + q, step = size_t(4) * p.ldc;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float4 o = make_float4(v[i].x + b.x, v[i].y + b.y, v[i].z + b.z, v[i].w + b.w);
+    if (MODE == kOutF32Acc || MODE == kOutBf16Acc) {
+      o.x += old[i].x; o.y += old[i].y; o.z += old[i].z; o.w += old[i].w;
+    }
+    if (MODE == kOutBf16 || MODE == kOutBf16Acc)
+      *reinterpret_cast<uint2*>(reinterpret_cast<hg_lp_t*>(p.C) + at + i * step) = make_uint2(pack_bf16(o.x, o.y), pack_bf16(o.z, o.w));
+    else
+      *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.C) + at + i * step) = o;
+  }
+}
+
+template <int MODE>
+__device__ __forceinline__ void load_old_whole(const Params& p, int row0, int col0, float4 (&old)[8]) {
+  if (MODE != kOutF32Acc && MODE != kOutBf16Acc) return;
+  const int lane = int(lane_id());
+  const size_t at = size_t(row0 + (lane >> 3)) * p.ldc + col0 + (lane & 7) * 4, step = size_t(4) * p.ldc;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (MODE == kOutF32Acc) {
+      old[i] = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.C) + at + i * step);
+    } else {
+      const uint2 u = *reinterpret_cast<const uint2*>(reinterpret_cast<const hg_lp_t*>(p.C) + at + i * step);
+      const float2 lo = hg_unpack2(u.x), hi = hg_unpack2(u.y);
+      old[i] = make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+  }
+}
+
+// The whole blocks of a tile part; returns the first column that is left.  With an accumulating mode the next block's old
+// values are in flight while this one is turned.
+template <int MODE>
+__device__ __forceinline__ int store_tile_whole(const Params& p, uint32_t stg, uint32_t src, int row0, int n0) {
+  const int cols = min(BN, (p.N - n0) & ~31);
+  float4 old[8];
+  if (cols > 0) load_old_whole<MODE>(p, row0, n0, old);
+#pragma unroll 1
+  for (int c = 0; c < cols; c += 32) {
+    uint32_t r0[32];
+    tmem_ld32(src + c, r0);
+    tmem_ld_wait();
+    float4 next[8];
+    if (c + 32 < cols) load_old_whole<MODE>(p, row0, n0 + c + 32, next);
+    store_block_whole<MODE>(p, stg, row0, n0 + c, r0, old);
+    if (MODE == kOutF32Acc || MODE == kOutBf16Acc) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) old[i] = next[i];
+    }
+  }
+  return max(cols, 0);
+}
+
 // The 32 x 256 part of a tile that this warp's lanes hold in tensor memory at `src`: rows row0.. of C (p.M: the first row
 // that is not this tile's), rows y0.. of the tensor map.
 __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorMap* tmC, StoreStage& st, uint32_t src, int row0,
                                                 int y0, int n0, bool whole_rows, const float* part = nullptr,
                                                 int nparts = 0) {
   if (p.c_tma && whole_rows && part == nullptr) {
-#pragma unroll 1
-    for (int c = 0; c < BN && n0 + c < p.N; c += 64) {
-      uint32_t r0[32], r1[32];
-      tmem_ld32(src + c, r0);
-      tmem_ld32(src + c + 32, r1);
-      tmem_ld_wait();
-      if (!HG_BOUNDS_OK(row0 >= 0 && row0 < p.M, p.status)) continue;
-      store_block64_tma(p, tmC, st, y0, n0 + c, r0, r1);
+    if (p.out_mode == kOutF32) {
+      if (p.bias != nullptr) store_tile_tma<true, true>(p, tmC, st, src, row0, y0, n0);
+      else store_tile_tma<false, true>(p, tmC, st, src, row0, y0, n0);
+    } else {
+      if (p.bias != nullptr) store_tile_tma<true, false>(p, tmC, st, src, row0, y0, n0);
+      else store_tile_tma<false, false>(p, tmC, st, src, row0, y0, n0);
     }
     return;
   }
@@ -460,8 +574,17 @@ __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorM
     if (lane_id() == 0) tma_store_wait_read<0>();
     __syncwarp();
   }
+  int c0 = 0;
+  if (part == nullptr && row0 + 32 <= p.M && four_aligned(p)) {
+    switch (p.out_mode) {
+      case kOutF32: c0 = store_tile_whole<kOutF32>(p, st.base, src, row0, n0); break;
+      case kOutF32Acc: c0 = store_tile_whole<kOutF32Acc>(p, st.base, src, row0, n0); break;
+      case kOutBf16Acc: c0 = store_tile_whole<kOutBf16Acc>(p, st.base, src, row0, n0); break;
+      default: c0 = store_tile_whole<kOutBf16>(p, st.base, src, row0, n0); break;
+    }
+  }
 #pragma unroll 1
-  for (int c = 0; c < BN && n0 + c < p.N; c += 32) {
+  for (int c = c0; c < BN && n0 + c < p.N; c += 32) {
     float4 old[8];
     load_old(p, row0, n0 + c, old);
     uint32_t r0[32];

@@ -139,6 +139,27 @@ int make_tmap_2d_store(CUtensorMap* out, const void* base, uint64_t rows, uint64
   return make_tmap_2d_bf16(out, base, rows, cols, ld, 32, 64);
 }
 
+int make_tmap_2d_store_f32(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld) {
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld & 3) || (cols & 3)) return 1;
+  const uint64_t key[8] = {5, uint64_t(reinterpret_cast<uintptr_t>(base)), rows, cols, ld, 0, 0, 0};
+  if (const CUtensorMap* hit = tmap_cache_find(key)) {
+    *out = *hit;
+    return 0;
+  }
+  EncodeTiledFn enc = get_encode_fn();
+  if (enc == nullptr) return -2;
+  cuuint64_t dims[2] = {cols, rows};
+  cuuint64_t strides[1] = {ld * 4};
+  cuuint32_t box[2] = {32, 32};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return -(1000 + int(r));
+  tmap_cache_store(key, *out);
+  return 0;
+}
+
 int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1,
                       uint64_t stride2, uint32_t box0, uint32_t box1, uint32_t box2) {
   EncodeTiledFn enc = get_encode_fn();

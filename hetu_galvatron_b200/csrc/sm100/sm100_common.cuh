@@ -380,6 +380,8 @@ int make_tmap_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_
 // 16-bit output matrix [rows, cols] for stores of 32-row, 128-byte-wide boxes (128B swizzle).  Returns 1
 // when base, pitch or width is not a multiple of 16 bytes (the caller stores without a tensor map), 0 on success.
 int make_tmap_2d_store(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld);
+// The same for an fp32 output matrix.
+int make_tmap_2d_store_f32(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld);
 // rank-3 bf16 tensor [d2, d1, d0] (d0 innermost) with strides in elements.
 int make_tmap_3d_bf16(CUtensorMap* out, const void* base, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1,
                       uint64_t stride2, uint32_t box0, uint32_t box1, uint32_t box2);

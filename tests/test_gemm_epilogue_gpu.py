@@ -53,3 +53,25 @@ def test_tma_stores_stay_inside_their_window(M, N, K, left, right, a_mn):
     out.fill_(2.0)
     assert (whole == 2.0).all()
     _lib.assert_healthy()
+
+
+# fp32 results and accumulating modes in a window of whole 16-byte groups: one box of 32 columns and less, columns that end
+# inside a box and on a tile's edge, whole and clipped blocks of 32 rows, a bias whose last columns are not 16 bytes wide
+@pytest.mark.parametrize("M,N,K", [(256, 256, 64), (300, 36, 72), (257, 1000, 136), (352, 260, 64), (2600, 2568, 64)])
+@pytest.mark.parametrize("mode", [OUT_F32, OUT_F32_ACC, OUT_BF16_ACC])
+@pytest.mark.parametrize("biased", [False, True])
+def test_wide_stores_stay_inside_their_window(M, N, K, mode, biased):
+    g = torch.Generator(device=DEV).manual_seed(M + N + mode)
+    a, b = (torch.randn(n, K, device=DEV, generator=g).to(torch.bfloat16) for n in (M, N))
+    bias = torch.randn(N, device=DEV, generator=g).to(torch.bfloat16) if biased else None
+    dt = torch.bfloat16 if mode == OUT_BF16_ACC else torch.float32
+    whole = torch.full((M + 34, 4 + N + 8), 2.0, device=DEV, dtype=dt)
+    out = whole[1:M + 1, 4:4 + N]
+    assert out.stride(0) % 4 == 0 and N % 4 == 0 and out.data_ptr() % 8 == 0
+    ops.gemm(a, b, out=out, out_mode=mode, bias=bias, pair=True)
+    ref = a.double() @ b.double().t() + (bias.double() if biased else 0.0) + (0.0 if mode == OUT_F32 else 2.0)
+    # fp32 sums of K products of unit normals; one rounding to 16 bits where C is 16 bits wide
+    assert torch.allclose(out.double(), ref, rtol=2.0 ** -8 if dt == torch.bfloat16 else 1e-6, atol=1e-5 * K ** 0.5)
+    out.fill_(2.0)
+    assert (whole == 2.0).all()
+    _lib.assert_healthy()
