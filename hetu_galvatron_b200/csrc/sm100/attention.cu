@@ -819,7 +819,23 @@ struct BwdParams {
   hg_lp_t* dK; int64_t dk_ss, dk_sb; SlotMap dkmap;
   hg_lp_t* dV; int64_t dv_ss, dv_sb; SlotMap dvmap;
   int* status;
+  // dK/dV of a key block shared by several CTAs (see dkv_chunk_steps): at most `chunk` query steps each (0: off), their
+  // fp32 parts in `part`, [CTA][dV, dK][128][HD]
+  int chunk;
+  float* part;
 };
+
+// 128-query steps of key block kb, all query heads of its kv head together
+__host__ __device__ __forceinline__ int dkv_block_steps(const BwdParams& p, int kb) {
+  int first = p.causal ? p.k_pos0 + kb * 128 - p.q_pos0 : 0;       // first query row that can see this key block
+  if (first < 0) first = 0;
+  const int n = (p.Sq + 127) / 128 - first / 128;
+  return n > 0 ? n * p.qpg : 0;
+}
+// CTAs that share key block kb, `steps` being its query steps
+__host__ __device__ __forceinline__ int dkv_block_ctas(const BwdParams& p, int steps) {
+  return p.chunk > 0 && steps > p.chunk ? (steps + p.chunk - 1) / p.chunk : 1;
+}
 
 // =================================================================================================
 // Backward, part 1: one CTA per (key block of 128, kv head, batch); loops over the query heads of the
@@ -1192,7 +1208,8 @@ struct Dkv128Smem {
 // NWG softmax warpgroups (2 or 4): thread == key row, warpgroup g owns query columns [g * 128 / NWG, (g + 1) * 128 / NWG)
 // of every step.  Four warpgroups put four warps on every scheduler, which is what keeps the exp2 unit and the FMA
 // pipe busy through the latencies of the loads from tensor memory and of the dependent exp2 / convert chains.
-template <int HD, int NWG>
+// SHARED: key blocks may be shared between CTAs (p.chunk > 0).
+template <int HD, int NWG, bool SHARED>
 __global__ void __launch_bounds__(64 + 128 * NWG, 1)
 flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
@@ -1233,14 +1250,26 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
-  const int kb = blockIdx.x, g = blockIdx.y, b = blockIdx.z;  // g = kv head
+  const int g = blockIdx.y, b = blockIdx.z;                   // g = kv head
+  int kb = blockIdx.x, mine = 0, sharers = 1;                 // key block, this CTA among those that share it
+  if constexpr (SHARED) {
+    int left = blockIdx.x;
+    for (kb = 0;; ++kb) {
+      sharers = dkv_block_ctas(p, dkv_block_steps(p, kb));
+      if (left < sharers) break;
+      left -= sharers;
+    }
+    mine = left;
+  }
   const int k0 = kb * 128;
   int q_first = 0;                                            // first query row that can see this key block
   if (p.causal) q_first = max(0, p.k_pos0 + k0 - p.q_pos0);
   const int qs0 = q_first / 128;                              // first 128-row query step
   const int n_qs = (p.Sq + 127) / 128;
   const int steps_per_head = max(0, n_qs - qs0);
-  const int n_it = steps_per_head * p.qpg;
+  const int n_steps = steps_per_head * p.qpg;
+  const int it0 = SHARED ? n_steps * mine / sharers : 0;      // this CTA's steps, heads outside, queries inside
+  const int n_it = SHARED ? n_steps * (mine + 1) / sharers - it0 : n_steps;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmDO);
@@ -1269,6 +1298,8 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   const uint32_t tST = tmem, tDPT = tmem + 128, tDV = tmem + 256, tDK = tmem + 384;
 
   const int h0 = g * p.qpg;  // first query head of the group
+  const int h_it0 = h0 + (SHARED && steps_per_head > 0 ? it0 / steps_per_head : 0);   // head and query step of step it0
+  const int qs_it0 = qs0 + (SHARED && steps_per_head > 0 ? it0 % steps_per_head : 0);
   const int kslot = p.kmap.slot(h0, p.qpg), vslot = p.vmap.slot(h0, p.qpg);
 
   if (warp == 0) {
@@ -1283,7 +1314,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       }
       int qs_slot = 0, ds_slot = 0;
       uint32_t qph = 0, dph = 0;
-      int h = h0, qs = qs0;
+      int h = h_it0, qs = qs_it0;
       for (int it = 0; it < n_it; ++it) {
         const int qrow = qs * 128;
         const int qslot = p.qmap.slot(h, p.qpg), doslot = p.domap.slot(h, p.qpg);
@@ -1404,7 +1435,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     bool ok = true;
     // Per-query statistics of a step, fetched one step ahead: thread t < 128 carries -lse * log2 e of query t of the
     // step, thread 128 + t carries D of query t.
-    int ld_h = h0, ld_qs = qs0, ld_it = 0;
+    int ld_h = h_it0, ld_qs = qs_it0, ld_it = 0;
     auto load_stat = [&]() -> float {
       float v = 0.f;
       if (tid < 256 && ld_it < n_it) {
@@ -1427,7 +1458,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       mbar_arrive_warp(&stats_full[0]);
       stat_next = load_stat();
     }
-    int cur_qs = qs0;
+    int cur_qs = qs_it0;
     HG_DKV_TIMERS(tm_wait_a, tm_a, tm_wait_b, tm_b);
     for (int it = 0; it < n_it; ++it) {
       const int sb = it & 1;
@@ -1558,7 +1589,14 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         tmem_ld32(tDV + lane_off + c * 32, r0);
         tmem_ld32(tDK + lane_off + c * 32, r1);
         tmem_ld_wait();
-        if (krow < p.Skv) {
+        if (SHARED && sharers > 1) {                // summed, scaled and rounded by dkv_sum_kernel
+          float* part = p.part + ((size_t(b) * gridDim.y + g) * gridDim.x + blockIdx.x) * (2 * 128 * HD) + row * HD + c * 32;
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            reinterpret_cast<uint4*>(part)[q] = make_uint4(r0[q * 4], r0[q * 4 + 1], r0[q * 4 + 2], r0[q * 4 + 3]);
+            reinterpret_cast<uint4*>(part + 128 * HD)[q] = make_uint4(r1[q * 4], r1[q * 4 + 1], r1[q * 4 + 2], r1[q * 4 + 3]);
+          }
+        } else if (krow < p.Skv) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             uint4 u, w;
@@ -1585,6 +1623,35 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     tc_fence_after();
     tmem_dealloc(tmem, 512);
   }
+}
+
+// dK and dV of the key blocks that several CTAs share: their parts added in CTA order, scaled, rounded once.  A CTA takes
+// 16 rows of a key block, a thread eight columns of one row of dV or dK.
+template <int HD>
+__global__ void __launch_bounds__(4 * HD)
+dkv_sum_kernel(const BwdParams p, int ctas) {
+  const int g = blockIdx.y, b = blockIdx.z, kb = blockIdx.x >> 3;
+  int first = 0;
+  for (int i = 0; i < kb; ++i) first += dkv_block_ctas(p, dkv_block_steps(p, i));
+  const int sharers = dkv_block_ctas(p, dkv_block_steps(p, kb));
+  const int which = threadIdx.x / (2 * HD), t = threadIdx.x % (2 * HD);        // 0: dV, 1: dK
+  const int row = (blockIdx.x & 7) * 16 + t / (HD / 8), c = t % (HD / 8) * 8;
+  const int krow = kb * 128 + row;
+  if (sharers < 2 || krow >= p.Skv) return;
+  const float* part = p.part + ((size_t(b) * gridDim.y + g) * ctas + first) * (2 * 128 * HD) + (which * 128 + row) * HD + c;
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  for (int i = 0; i < sharers; ++i) {
+    const float4 u = __ldcs(reinterpret_cast<const float4*>(part + size_t(i) * (2 * 128 * HD)));
+    const float4 w = __ldcs(reinterpret_cast<const float4*>(part + size_t(i) * (2 * 128 * HD)) + 1);
+    s[0] += u.x; s[1] += u.y; s[2] += u.z; s[3] += u.w;
+    s[4] += w.x; s[5] += w.y; s[6] += w.z; s[7] += w.w;
+  }
+  const float f = which ? p.scale : 1.f;
+  const int h0 = g * p.qpg;
+  hg_lp_t* out = which ? p.dK + int64_t(krow) * p.dk_ss + int64_t(b) * p.dk_sb + int64_t(p.dkmap.slot(h0, p.qpg)) * HD
+                       : p.dV + int64_t(krow) * p.dv_ss + int64_t(b) * p.dv_sb + int64_t(p.dvmap.slot(h0, p.qpg)) * HD;
+  *reinterpret_cast<uint4*>(out + c) = make_uint4(pack_bf16(s[0] * f, s[1] * f), pack_bf16(s[2] * f, s[3] * f),
+                                                  pack_bf16(s[4] * f, s[5] * f), pack_bf16(s[6] * f, s[7] * f));
 }
 
 // =================================================================================================
@@ -1913,6 +1980,9 @@ int g_dkv_variant = 0;
 // tiles per CTA with P in tensor memory wherever a sequence is longer than one tile (1, 2: side-by-side tests and timing).
 int g_fwd_variant = 0;
 
+constexpr int kSmCount = 148;
+constexpr int kDkvMinChunk = 4;   // fewest query steps of a CTA that shares its key block: about what its start and end cost
+
 template <typename K>
 int set_smem(K kernel, int bytes) {
   return int(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
@@ -1945,16 +2015,48 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
   return int(cudaGetLastError());
 }
 
+// CTAs per kv head and sequence of the 128-query dK/dV kernel
+int dkv_ctas(const BwdParams& p, int blocks) {
+  int n = 0;
+  for (int kb = 0; kb < blocks; ++kb) n += dkv_block_ctas(p, dkv_block_steps(p, kb));
+  return n;
+}
+
+// Query steps per CTA when the key blocks are too few for the chip, 0 where each has one CTA.  A grouped layer has a dK/dV
+// CTA per key block and KV head: four kv heads of 1531 tokens are 48 CTAs, and under a causal mask the first of them walks
+// twelve times the steps of the last.  The smallest chunk whose CTAs all run at once is taken: their longest is what counts.
+// It has to end at least six steps (of 2 us) before the longest block alone, which pays for the parts' way through memory and
+// the kernel that adds them.  Whole backward, us, one CTA a block / shared: head dim 128, 28 heads on 4, 1531 tokens 194 / 100,
+// 512 tokens 69 / 40, 256 tokens 44 / 34; 8 heads on 1, 4096 tokens 499 / 153; 4 heads, 2048 tokens 63 / 58; fewer steps saved:
+// 4 heads, 1024 tokens 40 / 41, 16 heads 41 / 45; head dim 64, 28 on 4, 1531 tokens 190 / 82, 32 on 8, 1024 tokens 87 / 55.
+int dkv_chunk_steps(BwdParams p, int Skv, int nkv) {
+  const int blocks = (Skv + 127) / 128, heads = nkv * p.B;
+  if ((long long)blocks * heads > kSmCount) return 0;
+  int longest = 0;
+  for (int kb = 0; kb < blocks; ++kb) longest = dkv_block_steps(p, kb) > longest ? dkv_block_steps(p, kb) : longest;
+  int lo = kDkvMinChunk - 1, hi = longest;            // the CTAs of chunk `hi` run at once, those of `lo` may not
+  while (hi - lo > 1) {
+    p.chunk = (lo + hi) / 2;
+    if (dkv_ctas(p, blocks) * heads <= kSmCount) hi = p.chunk;
+    else lo = p.chunk;
+  }
+  return hi + 6 <= longest ? hi : 0;
+}
+
 template <int HD>
 int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                const BwdParams& p, int Skv, int nkv, bool wide, cudaStream_t st) {
   int rc;
-  const dim3 grid((Skv + 127) / 128, nkv, p.B);
+  dim3 grid((Skv + 127) / 128, nkv, p.B);
   if (wide) {
-    static bool cfg = false;
-    auto k = flash_bwd_dkv128_kernel<HD, kDkvWarpgroups>;
-    if (!cfg) { if ((rc = set_smem(k, Dkv128Smem<HD>::kTotal))) return rc; cfg = true; }
+    const int blocks = int(grid.x);
+    if (p.chunk > 0) grid.x = unsigned(dkv_ctas(p, blocks));
+    static bool cfg[2] = {};
+    const bool shared = p.chunk > 0;
+    auto k = shared ? flash_bwd_dkv128_kernel<HD, kDkvWarpgroups, true> : flash_bwd_dkv128_kernel<HD, kDkvWarpgroups, false>;
+    if (!cfg[shared]) { if ((rc = set_smem(k, Dkv128Smem<HD>::kTotal))) return rc; cfg[shared] = true; }
     k<<<grid, 64 + 128 * kDkvWarpgroups, Dkv128Smem<HD>::kTotal, st>>>(tq, tk, tv, tdo, p);
+    if (p.chunk > 0) dkv_sum_kernel<HD><<<dim3(blocks * 8, nkv, p.B), 4 * HD, 0, st>>>(p, int(grid.x));
   } else {
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(flash_bwd_dkv_kernel<HD>, DkvSmem<HD>::kTotal))) return rc; cfg = true; }
@@ -2013,11 +2115,24 @@ int hg_attn_set_dkv_variant(int v) {
   return old;
 }
 
-// dsum: scratch [B, nheads, Sq] fp32 (filled here with rowsum(dO*O)).
-int hg_flash_bwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o,
-                 const HgAttnTensor* d_o, const void* lse, void* dsum, const HgAttnTensor* dq, const HgAttnTensor* dk,
-                 const HgAttnTensor* dv, int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0,
-                 int k_pos0, float scale, void* stream) {
+// Floats of scratch that hg_flash_bwd_ws asks for: the row sums of dO * O, [B, nheads, Sq], and where key blocks are shared
+// the parts of dK and dV.
+long long hg_flash_bwd_scratch(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
+  if (Sq <= 0 || Skv <= 0 || B <= 0 || nheads <= 0 || nkv <= 0) return 0;
+  BwdParams p{};
+  p.Sq = Sq; p.Skv = Skv; p.B = B; p.qpg = nheads / nkv; p.causal = causal; p.q_pos0 = q_pos0; p.k_pos0 = k_pos0;
+  const long long sums = ((long long)B * nheads * Sq + 3) / 4 * 4;
+  if (g_dkv_variant != 0 || !(p.chunk = dkv_chunk_steps(p, Skv, nkv))) return sums;
+  return sums + (long long)dkv_ctas(p, (Skv + 127) / 128) * nkv * B * 2 * 128 * hd;
+}
+
+// ws: scratch of ws_floats fp32 values, 16-byte aligned, at least [B, nheads, Sq] (filled here with rowsum(dO*O)).  With less
+// than hg_flash_bwd_scratch floats every key block has one CTA.
+int hg_flash_bwd_ws(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o,
+                    const HgAttnTensor* d_o, const void* lse, void* ws, long long ws_floats, const HgAttnTensor* dq,
+                    const HgAttnTensor* dk, const HgAttnTensor* dv, int Sq, int Skv, int B, int nheads, int nkv, int hd,
+                    int causal, int q_pos0, int k_pos0, float scale, void* stream) {
+  void* dsum = ws;
   if (hd != 64 && hd != 128) return -1;
   if (Sq <= 0 || Skv <= 0 || B <= 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
@@ -2042,6 +2157,12 @@ int hg_flash_bwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTenso
   p.dK = (hg_lp_t*)dk->ptr; p.dk_ss = dk->ss; p.dk_sb = dk->sb; p.dkmap = {dk->gs, dk->hs, dk->off};
   p.dV = (hg_lp_t*)dv->ptr; p.dv_ss = dv->ss; p.dv_sb = dv->sb; p.dvmap = {dv->gs, dv->hs, dv->off};
   p.status = hg_host::status_ptr();
+  const long long need = hg_flash_bwd_scratch(Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0);
+  const long long sums = ((long long)B * nheads * Sq + 3) / 4 * 4;
+  if (need > sums && ws_floats >= need && (reinterpret_cast<uintptr_t>(ws) & 15) == 0) {
+    p.chunk = dkv_chunk_steps(p, Skv, nkv);
+    p.part = static_cast<float*>(ws) + sums;
+  }
   {
     CUtensorMap tq, tk, tv, tdo;
     const bool wide = g_dkv_variant == 0;   // 128-query steps, P^T / dS^T in tensor memory
@@ -2059,6 +2180,15 @@ int hg_flash_bwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTenso
   if ((rc = make_map(&tv, v->ptr, hd, v->slots, Skv, B, v->ss, v->sb, 128))) return rc;
   if ((rc = make_map(&tdo, d_o->ptr, hd, d_o->slots, Sq, B, d_o->ss, d_o->sb, 128))) return rc;
   return hd == 128 ? launch_dq<128>(tq, tk, tv, tdo, p, st) : launch_dq<64>(tq, tk, tv, tdo, p, st);
+}
+
+// dsum: scratch [B, nheads, Sq] fp32 (filled here with rowsum(dO*O)); every key block has one CTA.
+int hg_flash_bwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o,
+                 const HgAttnTensor* d_o, const void* lse, void* dsum, const HgAttnTensor* dq, const HgAttnTensor* dk,
+                 const HgAttnTensor* dv, int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0,
+                 int k_pos0, float scale, void* stream) {
+  return hg_flash_bwd_ws(q, k, v, o, d_o, lse, dsum, 0, dq, dk, dv, Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0,
+                         scale, stream);
 }
 
 }  // extern "C"

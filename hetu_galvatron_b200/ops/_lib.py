@@ -132,6 +132,9 @@ _SIGNATURES = {
     "hg_flash_decode": [ctypes.POINTER(AttnTensor)] * 4 + [c_void_p, c_void_p] + [c_int] * 9 + [c_float, c_void_p],
     "hg_flash_bwd": [ctypes.POINTER(AttnTensor)] * 5 + [c_void_p, c_void_p] + [ctypes.POINTER(AttnTensor)] * 3 +
                     [c_int] * 9 + [c_float, c_void_p],
+    "hg_flash_bwd_scratch": [c_int] * 9,
+    "hg_flash_bwd_ws": [ctypes.POINTER(AttnTensor)] * 5 + [c_void_p, c_void_p, c_ll] + [ctypes.POINTER(AttnTensor)] * 3 +
+                       [c_int] * 9 + [c_float, c_void_p],
     "hg_ag_gemm_bf16": [c_void_p] * 7 + [c_int] * 10 + [c_void_p],
     "hg_gemm_rs_bf16": [c_void_p] * 5 + [c_int] * 10 + [c_void_p],
     "hg_ag_gemm2_bf16": [c_void_p] * 7 + [c_int] * 10 + [c_void_p],
@@ -171,7 +174,7 @@ def load():
             continue
         fn.argtypes = argtypes
         fn.restype = c_int
-    for name in ("hg_flash_decode_scratch", "hg_decoder_step_scratch"):
+    for name in ("hg_flash_decode_scratch", "hg_decoder_step_scratch", "hg_flash_bwd_scratch"):
         getattr(lib, name).restype = c_ll
     if hasattr(lib, "hg_status_address"):
         lib.hg_status_address.restype = c_void_p

@@ -50,6 +50,12 @@ def attention_reference(q, k, v, causal=True, scale=None, q_pos0=0, k_pos0=0, dr
     return o.permute(2, 0, 1, 3).to(q.dtype), lse
 
 
+def _backward_scratch(lib, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, device) -> torch.Tensor:
+    """fp32 scratch of the backward kernels: row sums of dO * O and, where key blocks are shared between CTAs, their parts."""
+    n = lib.hg_flash_bwd_scratch(S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0)
+    return torch.empty(n, dtype=torch.float32, device=device)
+
+
 class _FlashPacked(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, S, B, nh, ng, hd, causal, scale):
@@ -82,7 +88,7 @@ class _FlashPacked(torch.autograd.Function):
         slots = nh + 2 * ng
         dout = dout.contiguous()
         dqkv = torch.empty_like(qkv)
-        dsum = torch.empty((B, nh, S), dtype=torch.float32, device=qkv.device)
+        ws = _backward_scratch(lib, S, S, B, nh, ng, hd, causal, 0, 0, qkv.device)
         ss, sb = B * P, P
         q = _desc(qkv, ss, sb, slots, qpg + 2, 1, 0)
         k = _desc(qkv, ss, sb, slots, qpg + 2, 0, qpg)
@@ -92,11 +98,11 @@ class _FlashPacked(torch.autograd.Function):
         dq = _desc(dqkv, ss, sb, slots, qpg + 2, 1, 0)
         dk = _desc(dqkv, ss, sb, slots, qpg + 2, 0, qpg)
         dv = _desc(dqkv, ss, sb, slots, qpg + 2, 0, qpg + 1)
-        rc = lib.hg_flash_bwd(ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(o), ctypes.byref(do),
-                              lse.data_ptr(), dsum.data_ptr(), ctypes.byref(dq), ctypes.byref(dk), ctypes.byref(dv), S,
-                              S, B, nh, ng, hd, int(causal), 0, 0, float(scale), _lib.stream())
+        rc = lib.hg_flash_bwd_ws(ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(o), ctypes.byref(do),
+                                 lse.data_ptr(), ws.data_ptr(), ws.numel(), ctypes.byref(dq), ctypes.byref(dk),
+                                 ctypes.byref(dv), S, S, B, nh, ng, hd, int(causal), 0, 0, float(scale), _lib.stream())
         _lib.check(rc, "hg_flash_bwd")
-        _lib.count_launch(3)
+        _lib.count_launch(4 if ws.numel() > B * nh * S + 3 else 3)
         return dqkv, None, None, None, None, None, None, None
 
 
@@ -261,7 +267,7 @@ def flash_backward(q, k, v, out, dout, lse, causal, scale, q_pos0=0, k_pos0=0):
     Skv, ng = k.shape[0], k.shape[2]
     qpg = nh // ng
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    dsum = torch.empty((B, nh, S), dtype=torch.float32, device=q.device)
+    ws = _backward_scratch(lib, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, q.device)
     qd = _desc(q, q.stride(0), q.stride(1), nh, qpg, 1, 0)
     kd = _desc(k, k.stride(0), k.stride(1), ng, 1, 0, 0)
     vd = _desc(v, v.stride(0), v.stride(1), ng, 1, 0, 0)
@@ -270,11 +276,12 @@ def flash_backward(q, k, v, out, dout, lse, causal, scale, q_pos0=0, k_pos0=0):
     dqd = _desc(dq, dq.stride(0), dq.stride(1), nh, qpg, 1, 0)
     dkd = _desc(dk, dk.stride(0), dk.stride(1), ng, 1, 0, 0)
     dvd = _desc(dv, dv.stride(0), dv.stride(1), ng, 1, 0, 0)
-    rc = lib.hg_flash_bwd(ctypes.byref(qd), ctypes.byref(kd), ctypes.byref(vd), ctypes.byref(od), ctypes.byref(dod),
-                          lse.data_ptr(), dsum.data_ptr(), ctypes.byref(dqd), ctypes.byref(dkd), ctypes.byref(dvd), S,
-                          Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0, float(scale), _lib.stream())
+    rc = lib.hg_flash_bwd_ws(ctypes.byref(qd), ctypes.byref(kd), ctypes.byref(vd), ctypes.byref(od), ctypes.byref(dod),
+                             lse.data_ptr(), ws.data_ptr(), ws.numel(), ctypes.byref(dqd), ctypes.byref(dkd),
+                             ctypes.byref(dvd), S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0, float(scale),
+                             _lib.stream())
     _lib.check(rc, "hg_flash_bwd")
-    _lib.count_launch(3)
+    _lib.count_launch(4 if ws.numel() > B * nh * S + 3 else 3)
     return dq, dk, dv
 
 

@@ -1,0 +1,58 @@
+"""dK and dV of key blocks that several CTAs share, against one CTA per key block and 64-bit arithmetic."""
+import ctypes
+
+import pytest
+import torch
+
+from hetu_galvatron_b200 import ops
+from hetu_galvatron_b200.ops import _lib
+from hetu_galvatron_b200.ops.attention import _desc
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def rel_err(a, b):
+    return ((a.double() - b.double()).norm() / b.double().norm()).item()
+
+
+# grouped heads whose early blocks are shared and late ones are not, no mask, one head of many queries, queries that start
+# behind or before the keys (keys that no query sees among them), a ragged end, the
+# last length that is not shared for one head and the first that is, the last grid of less than a wave and the first of more
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("Sq,Skv,B,nh,ng,causal,q0,k0", [
+    (1531, 1531, 1, 7, 1, True, 0, 0), (640, 640, 1, 6, 2, False, 0, 0), (2049, 2049, 1, 1, 1, True, 0, 0),
+    (1100, 1100, 2, 1, 1, True, 0, 0), (1200, 1200, 2, 1, 1, True, 0, 0),
+    (512, 900, 2, 4, 2, True, 388, 0), (300, 700, 1, 8, 1, True, 0, 100), (4096, 130, 1, 2, 1, True, 0, 64),
+    (257, 129, 37, 2, 2, True, 0, 0), (257, 129, 75, 1, 1, False, 0, 0)])
+def test_shared_key_blocks(hd, Sq, Skv, B, nh, ng, causal, q0, k0):
+    g = torch.Generator(device=DEV).manual_seed(Sq + Skv + hd)
+    q, dout = (torch.randn(Sq, B, nh, hd, device=DEV, generator=g).to(torch.bfloat16) for _ in "qd")
+    k, v = (torch.randn(Skv, B, ng, hd, device=DEV, generator=g).to(torch.bfloat16) for _ in "kv")
+    scale, qpg, lib = hd ** -0.5, nh // ng, _lib.load()
+    out, lse = ops.flash_attention(q, k, v, causal=causal, q_pos0=q0, k_pos0=k0, return_lse=True)
+    dq, dk, dv = ops.flash_backward(q, k, v, out, dout, lse, causal, scale, q0, k0)
+
+    one = [torch.empty_like(t) for t in (q, k, v)]                        # the entry point without scratch for parts
+    heads = lambda t: _desc(t, t.stride(0), t.stride(1), nh, qpg, 1, 0)
+    groups = lambda t: _desc(t, t.stride(0), t.stride(1), ng, 1, 0, 0)
+    args = [heads(q), groups(k), groups(v), heads(out), heads(dout)]
+    outs = [heads(one[0]), groups(one[1]), groups(one[2])]
+    dsum = torch.empty(B, nh, Sq, device=DEV)
+    rc = lib.hg_flash_bwd(*[ctypes.byref(t) for t in args], lse.data_ptr(), dsum.data_ptr(),
+                          *[ctypes.byref(t) for t in outs], Sq, Skv, B, nh, ng, hd, int(causal), q0, k0, scale, _lib.stream())
+    assert rc == 0
+    # the same 16-bit probabilities and dS, summed in fp32 in another order and rounded once
+    assert torch.equal(dq, one[0]) and rel_err(dk, one[1]) < 1e-3 and rel_err(dv, one[2]) < 1e-3
+
+    if B == 1 or Sq * Skv < 1 << 18:
+        qr, kr, vr = (t.double().requires_grad_() for t in (q, k, v))
+        s = torch.einsum("sbhd,tbhd->bhst", qr, kr.repeat_interleave(qpg, 2)) * scale
+        dead = torch.zeros(Sq, Skv, dtype=torch.bool, device=DEV)
+        if causal:
+            dead = (torch.arange(Skv, device=DEV) + k0)[None, :] > (torch.arange(Sq, device=DEV) + q0)[:, None]
+        p = torch.softmax(s.masked_fill(dead, -1e300), -1).masked_fill(dead, 0.0)      # rows that see no key: zeros
+        torch.einsum("bhst,tbhd->sbhd", p, vr.repeat_interleave(qpg, 2)).backward(dout.double())
+        # two 16-bit roundings before a product, one after (see test_attention_hd64_gpu)
+        assert rel_err(dk, kr.grad) < 5e-3 and rel_err(dv, vr.grad) < 5e-3
+    _lib.assert_healthy()
