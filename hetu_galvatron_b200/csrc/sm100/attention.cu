@@ -206,6 +206,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  chain_release();                            // after the allocation: see chain_release
+  chain_wait();
   const uint32_t tS[2] = {tmem, tmem + 128};
   const uint32_t tO = tmem + 256;
 
@@ -509,6 +511,8 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  chain_release();                            // after the allocation: see chain_release
+  chain_wait();
   const uint32_t tS[2] = {tmem, tmem + 128};
   const uint32_t tO[2] = {tmem + 256, tmem + 384};
 
@@ -2005,14 +2009,13 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(flash_fwd2_kernel<HD>, Fwd2Smem<HD>::kTotal))) return rc; cfg = true; }
     const dim3 grid((p.Sq + 255) / 256, p.nheads, p.B);
-    flash_fwd2_kernel<HD><<<grid, kFwd2Threads, Fwd2Smem<HD>::kTotal, st>>>(tq, tk, tv, p);
+    return hg_host::launch(flash_fwd2_kernel<HD>, grid, kFwd2Threads, Fwd2Smem<HD>::kTotal, st, tq, tk, tv, p);
   } else {
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(flash_fwd_kernel<HD>, FwdSmem<HD>::kTotal))) return rc; cfg = true; }
     const dim3 grid((p.Sq + 127) / 128, p.nheads, p.B);
-    flash_fwd_kernel<HD><<<grid, kThreads, FwdSmem<HD>::kTotal, st>>>(tq, tk, tv, p);
+    return hg_host::launch(flash_fwd_kernel<HD>, grid, kThreads, FwdSmem<HD>::kTotal, st, tq, tk, tv, p);
   }
-  return int(cudaGetLastError());
 }
 
 // CTAs per kv head and sequence of the 128-query dK/dV kernel

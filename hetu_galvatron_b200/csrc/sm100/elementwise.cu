@@ -132,6 +132,11 @@ __global__ void rope_append_kernel(hg_lp_t* __restrict__ qkv, int tokens, int ba
                                    int pos_offset, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                    int half, int interleaved, hg_lp_t* __restrict__ kc, hg_lp_t* __restrict__ vc,
                                    int64_t k_ss, int64_t k_sb, int64_t v_ss, int64_t v_sb) {
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  qkv += zero;
+  kc += zero;
+  vc += zero;
   const int vph = hd >> 3, slots = ng * (qpg + 2);
   for (RowColWalk w(slots * vph); w.row < tokens; w.next()) {
     const int t = int(w.row), slot = w.col / vph, c = w.col - slot * vph;
@@ -191,6 +196,8 @@ __device__ __forceinline__ float gelu_tanh_grad(float x) {
 template <int KIND>
 __global__ void glu_fwd_kernel(const hg_lp_t* __restrict__ y, hg_lp_t* __restrict__ out, int64_t rows,
                                int F) {
+  hg::chain_release();
+  y += hg::chain_wait();
   for (RowColWalk w(F >> 3); w.row < rows; w.next()) {
     const int64_t r = w.row;
     const int c = w.col;
@@ -376,6 +383,10 @@ __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ in, hg_lp_t* _
 
 __global__ void add_bf16_kernel(const hg_lp_t* __restrict__ a, const hg_lp_t* __restrict__ b,
                                 hg_lp_t* __restrict__ out, int64_t n) {
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  a += zero;
+  b += zero;
   const int64_t nv = n >> 3;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < nv; i += int64_t(gridDim.x) * blockDim.x) {
     float x[8], y[8];
@@ -474,10 +485,9 @@ int hg_rope_append(void* qkv, int tokens, int batch, int ng, int qpg, int hd, in
   if ((hd & 7) || (half & 7) || batch < 1 || ng < 1 || qpg < 1 || ((k_ss | k_sb | v_ss | v_sb) & 7)) return -1;
   if ((uintptr_t(qkv) | uintptr_t(kc) | uintptr_t(vc)) & 15) return -1;
   const int64_t work = int64_t(tokens) * ng * (qpg + 2) * (hd >> 3);
-  rope_append_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
-      (hg_lp_t*)qkv, tokens, batch, ng, qpg, hd, pos_offset, (const float*)cos_t, (const float*)sin_t, half, interleaved,
-      (hg_lp_t*)kc, (hg_lp_t*)vc, k_ss, k_sb, v_ss, v_sb);
-  return int(cudaGetLastError());
+  return hg_host::launch(rope_append_kernel, grid_for(work, 256), 256, 0, (cudaStream_t)stream, (hg_lp_t*)qkv, tokens, batch,
+                         ng, qpg, hd, pos_offset, (const float*)cos_t, (const float*)sin_t, half, interleaved, (hg_lp_t*)kc,
+                         (hg_lp_t*)vc, k_ss, k_sb, v_ss, v_sb);
 }
 
 int hg_glu_fwd(const void* y, void* out, long long rows, int F, int kind, void* stream) {
@@ -485,10 +495,8 @@ int hg_glu_fwd(const void* y, void* out, long long rows, int F, int kind, void* 
   if (F & 7) return -1;
   const int g = grid_for(rows * (F >> 3), 256);
   cudaStream_t st = (cudaStream_t)stream;
-  if (kind == 0) glu_fwd_kernel<0><<<g, 256, 0, st>>>((const hg_lp_t*)y, (hg_lp_t*)out, rows, F);
-  else if (kind == 1) glu_fwd_kernel<1><<<g, 256, 0, st>>>((const hg_lp_t*)y, (hg_lp_t*)out, rows, F);
-  else glu_fwd_kernel<2><<<g, 256, 0, st>>>((const hg_lp_t*)y, (hg_lp_t*)out, rows, F);
-  return int(cudaGetLastError());
+  auto k = kind == 0 ? glu_fwd_kernel<0> : kind == 1 ? glu_fwd_kernel<1> : glu_fwd_kernel<2>;
+  return hg_host::launch(k, g, 256, 0, st, (const hg_lp_t*)y, (hg_lp_t*)out, rows, F);
 }
 
 int hg_glu_bwd(const void* g_, const void* y, void* dy, long long rows, int F, int kind, void* stream) {
@@ -557,9 +565,8 @@ int hg_cast_f32_bf16(const void* in, void* out, long long n, void* stream) {
 
 int hg_add_bf16(const void* a, const void* b, void* out, long long n, void* stream) {
   if (n <= 0) return 0;
-  add_bf16_kernel<<<grid_for(n >> 3, 256), 256, 0, (cudaStream_t)stream>>>(
-      (const hg_lp_t*)a, (const hg_lp_t*)b, (hg_lp_t*)out, n);
-  return int(cudaGetLastError());
+  return hg_host::launch(add_bf16_kernel, grid_for(n >> 3, 256), 256, 0, (cudaStream_t)stream, (const hg_lp_t*)a,
+                         (const hg_lp_t*)b, (hg_lp_t*)out, n);
 }
 
 // See attn_merge_kernel.  d must be 64 or 128; S * BH rows.

@@ -52,6 +52,8 @@ flash_decode_kernel(const DecodeParams p) {
   __shared__ float sS[R][CH];
   __shared__ float sML[R][2];
   __shared__ float sAcc[4][R][HD];
+  hg::chain_release();
+  hg::chain_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane / LPK, ch = (lane % LPK) * 8;
   const int g = blockIdx.x, b = blockIdx.y, key0 = blockIdx.z * CH, ranges = gridDim.z;
@@ -186,6 +188,8 @@ flash_decode_kernel(const DecodeParams p) {
 template <int HD>
 __global__ void __launch_bounds__(HD)
 flash_decode_merge_kernel(const DecodeParams p, int ranges) {
+  hg::chain_release();
+  hg::chain_wait();
   const int rows = p.Sq * p.qpg;
   const int r = blockIdx.x % rows, g = (blockIdx.x / rows) % p.nkv, b = blockIdx.x / rows / p.nkv, c = threadIdx.x;
   const float* w = p.ws + int64_t(blockIdx.x) * ranges * (HD + 2);
@@ -223,14 +227,12 @@ inline int range_count(int kv_len, int chunk) { return kv_len > chunk ? (kv_len 
 template <int HD, int R>
 int launch(const DecodeParams& p, int chunk, int ranges, cudaStream_t st) {
   const dim3 grid(p.nkv, p.B, ranges);   // neighbours read neighbouring heads of the same cache rows
+  auto k = flash_decode_kernel<HD, R, 64>;
   if constexpr (R > 2) {
-    if (chunk == 128) flash_decode_kernel<HD, R, 128><<<grid, 128, 0, st>>>(p);
-    else flash_decode_kernel<HD, R, 64><<<grid, 128, 0, st>>>(p);
-  } else {
-    flash_decode_kernel<HD, R, 64><<<grid, 128, 0, st>>>(p);
+    if (chunk == 128) k = flash_decode_kernel<HD, R, 128>;
   }
-  if (ranges > 1) flash_decode_merge_kernel<HD><<<p.B * p.nkv * p.Sq * p.qpg, HD, 0, st>>>(p, ranges);
-  return int(cudaGetLastError());
+  if (int rc = hg_host::launch(k, grid, 128, 0, st, p)) return rc;
+  return ranges > 1 ? hg_host::launch(flash_decode_merge_kernel<HD>, p.B * p.nkv * p.Sq * p.qpg, HD, 0, st, p, ranges) : 0;
 }
 
 template <int HD>

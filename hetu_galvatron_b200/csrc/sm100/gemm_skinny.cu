@@ -11,7 +11,9 @@
 // sums meet through distributed shared memory, added in rank order: no workspace, no atomics, the same bits every time.
 // Measured, 4 rows, cold caches: 4096 x 4096 16 us (35 us in 16 tiles of the one-CTA kernel, 5 us for the bytes alone),
 // 4096 x 11008 29 us (78), 22016 x 4096 47 us (53), 152064 x 3584 176 us (208; 164 for the bytes); the seventeen
-// products of a decode step through four 7B-sized layers and the head 386 us instead of 743.
+// products of a decode step through four 7B-sized layers and the head 386 us instead of 743.  In a chain (the native decoder
+// step) a CTA's first stages of W are requested before the kernel in front has ended, up to 190 KB per SM: such a step as a
+// CUDA graph 519 -> 477 us.
 //
 // Roles (192 threads): warp 0 TMA producer, warp 1 TMEM allocator + UMMA issuer, warps 2-5 epilogue (thread = row of W
 // = output column, so a warp stores 32 consecutive elements of a token's row).
@@ -115,23 +117,35 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  chain_release();                            // after the allocation: see chain_release
+  if (warp != 0) chain_wait();
 
   if (warp == 0) {
     uint32_t stage = 0, phase = 0;
     bool ok = true;
     int issued = 0;
     const bool issuer = elect_one() != 0;
+    auto load_w = [&](int st, int kb) {
+      uint8_t* w = sW + st * W_BYTES;
+      mbar_expect_tx(&full[st], C_::kStageBytes);
+      if (W_MN) {
+#pragma unroll
+        for (int j = 0; j < TM / 64; ++j) tma_load_2d(w + j * SLAB_BYTES, &tmW, &full[st], n0 + j * 64, kb * BK);
+      } else {
+        tma_load_2d(w, &tmW, &full[st], kb * BK, n0);
+      }
+    };
+    // In a chain nothing writes weights: the first stages of them are on their way while the kernel before this one, which
+    // makes x, still runs.
+    const int ahead = min(ST, kb1 - kb0);
+    if (issuer)
+      for (int i = 0; i < ahead; ++i) load_w(i, kb0 + i);
+    __syncwarp();
+    chain_wait();
     for (int kb = kb0; kb < kb1; ++kb) {
       if (!mbar_wait_warp(&empty[stage], phase ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
-      uint8_t* w = sW + stage * W_BYTES;
       if (issuer) {
-        mbar_expect_tx(&full[stage], C_::kStageBytes);
-        if (W_MN) {
-#pragma unroll
-          for (int j = 0; j < TM / 64; ++j) tma_load_2d(w + j * SLAB_BYTES, &tmW, &full[stage], n0 + j * 64, kb * BK);
-        } else {
-          tma_load_2d(w, &tmW, &full[stage], kb * BK, n0);
-        }
+        if (issued >= ahead) load_w(stage, kb);
         tma_load_2d(sX + stage * C_::kXBytes, &tmX, &full[stage], kb * BK, 0);
       }
       __syncwarp();
@@ -141,8 +155,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     if (!ok) {
       *abort_flag = 1;
       // our own copies land before this CTA's shared memory is released (bounded)
-      for (int i = 0; i < ST && i < issued; ++i) {
-        const int at = issued - 1 - i;
+      const int flying = max(issued, ahead);
+      for (int i = 0; i < ST && i < flying; ++i) {
+        const int at = flying - 1 - i;
         for (uint32_t spin = 0; spin < (1u << 16); ++spin)
           if (mbar_try_wait(&full[at % ST], uint32_t(at / ST) & 1)) break;
       }
@@ -295,16 +310,18 @@ int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyPara
   }
   if (want_splits > 0) splits = want_splits;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = unsigned(splits);
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.gridDim = dim3(unsigned(splits), unsigned(tiles), 1);
   cfg.blockDim = dim3(192, 1, 1);
   cfg.dynamicSmemBytes = Cfg<NT>::kSmem;
   cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = hg_host::chain_overlaps() ? 2 : 1;
   return int(cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<W_MN, NT>, tw, tx, p));
 }
 

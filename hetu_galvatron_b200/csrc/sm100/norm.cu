@@ -58,6 +58,10 @@ norm_fwd_kernel(const hg_lp_t* __restrict__ x, const hg_lp_t* __restrict__ resid
                 hg_lp_t* __restrict__ y, hg_lp_t* __restrict__ h_out, float* __restrict__ rstd_out,
                 float* __restrict__ mean_out, int rows, int H, float eps) {
   __shared__ float red[kThreads / 32];
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  x += zero;
+  residual += zero;
   const int nvec = H >> 3;
   // The next row's loads are issued before this row's reductions, so that a block always has a row in flight
   // across its __syncthreads (with one row per trip the memory system idles while the block reduces).
@@ -388,11 +392,10 @@ int hg_norm_fwd(const void* x, const void* residual, const void* w, const void* 
   auto B = reinterpret_cast<const hg_lp_t*>(b);
   auto Y = reinterpret_cast<hg_lp_t*>(y);
   auto Ho = reinterpret_cast<hg_lp_t*>(h_out);
-#define HG_FWD(R_, V_) norm_fwd_kernel<R_, V_><<<grid, kThreads, 0, st>>>(X, R, W, B, Y, Ho, (float*)rstd, (float*)mean, rows, H, eps)
+#define HG_FWD(R_, V_) return hg_host::launch(norm_fwd_kernel<R_, V_>, grid, kThreads, 0, st, X, R, W, B, Y, Ho, (float*)rstd, (float*)mean, rows, H, eps)
   if (rms) { if (H <= 4096) HG_FWD(true, 2); else if (H <= 8192) HG_FWD(true, 4); else HG_FWD(true, 8); }
   else     { if (H <= 4096) HG_FWD(false, 2); else if (H <= 8192) HG_FWD(false, 4); else HG_FWD(false, 8); }
 #undef HG_FWD
-  return int(cudaGetLastError());
 }
 
 // `h` is the tensor that was normalised (x + residual).  `partial` is scratch of parts*H floats

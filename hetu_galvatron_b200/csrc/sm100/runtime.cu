@@ -28,6 +28,12 @@ int* status_ptr() {
   return g_status[dev];
 }
 
+// Launches of the open chain on this thread; -1: none is open.
+static thread_local int t_chain = -1;
+Chain::Chain() { t_chain = 0; }
+Chain::~Chain() { t_chain = -1; }
+bool chain_overlaps() { return t_chain >= 0 && t_chain++ > 0; }
+
 // cuTensorMapEncodeTiled is a driver call and needs a current context on the calling thread; threads
 // that have only been handed work by another thread (autograd's backward workers) may not have bound
 // the primary context yet, so bind it once per thread through the runtime.

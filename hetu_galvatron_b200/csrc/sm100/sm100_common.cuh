@@ -343,6 +343,21 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// ---------------------------------------------------------------------------
+// Programmatic dependent launch (hg_host::Chain below).  A kernel that may be launched in a chain calls chain_release() once
+// every resource it has to acquire is its own (tensor memory above all: a CTA of the next kernel that came first would hold
+// what this grid needs and wait for this grid), and chain_wait() in every thread before its first access to memory that an
+// earlier kernel of the chain reads or writes.  Both do nothing in a kernel launched without the attribute.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Returns 0, and has to be added to every `__restrict__` pointer that is read afterwards: such a pointer promises that no one
+// else writes behind it, so that without the dependence the compiler may read it before the wait.
+__device__ __forceinline__ int chain_wait() {
+  int zero;
+  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(zero)::"memory");
+  return zero;
+}
+
 // Byte offset of 16-byte chunk `chunk16` (0..7) of row `row` inside a 128B-swizzled
 // tile whose rows are 128 bytes (tile base 1024-byte aligned).
 __device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t chunk16) {
@@ -360,6 +375,36 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 // Host side: tensor-map encoding through the driver entry point (no -lcuda).
 // ---------------------------------------------------------------------------
 namespace hg_host {
+
+// Kernels that this thread launches while a Chain is open, the first one excepted, may start before the kernel in front of
+// them has ended (see chain_wait).  The first is launched the ordinary way: whatever the stream did before the chain, writing
+// weights included, is over when it starts, so later kernels may read what no kernel of the chain writes (weights) at once.
+class Chain {
+ public:
+  Chain();
+  ~Chain();
+  Chain(const Chain&) = delete;
+  Chain& operator=(const Chain&) = delete;
+};
+// Whether the next launch overlaps the one before it (runtime.cu); counts the launch.
+bool chain_overlaps();
+
+template <typename... P, typename... A>
+inline int launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  if (chain_overlaps()) {
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+  return int(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,

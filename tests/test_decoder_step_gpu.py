@@ -174,3 +174,31 @@ def test_launches_of_the_native_step(B, past, launches):
             m(x) if native else m.ffn(m.attn(x), x)
             assert _lib.launches() - before == launches
     _lib.assert_healthy()
+
+
+def test_weights_written_just_before_a_step_are_the_ones_it_reads():
+    """The step's kernels read weights before the kernel in front of them has ended, but never before the step began."""
+    torch.manual_seed(7)
+    m = layer("RMSNorm", "swiglu", "rope", False, 8, 8, 128)
+    x = torch.randn(1, 4, 1024, device=DEV).to(torch.bfloat16)
+    weights = [p for p in m.parameters() if p.dim() == 2]
+    new = [torch.randn_like(p) * 0.02 for p in weights]
+    got = []
+    for hooked in (False, True):
+        ic = StaticInferenceContext(4, 8)
+        m.attn.attention.inference_context = ic
+        with torch.no_grad():
+            for p in weights:
+                p.zero_()
+            m(x)                                          # fills position 0
+            ic.sequence_len_offset = 1
+            h = m.ffn.mlp.register_forward_hook(lambda *_: None) if hooked else None
+            torch.cuda._sleep(1000000)                    # the writes are still queued when the step is launched
+            for p, w in zip(weights, new):
+                p.copy_(w)
+            got.append(m(x))
+        if h is not None:
+            h.remove()
+        m.attn.attention.inference_context = None
+    assert torch.equal(got[0], got[1])
+    _lib.assert_healthy()
