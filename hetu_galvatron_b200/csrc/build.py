@@ -1,11 +1,11 @@
 """In-tree build of the native code.
 
-Two artefacts are produced under ``hetu_galvatron_b200/_lib``:
+These artefacts are produced under ``hetu_galvatron_b200/_lib``:
 
 * ``libhg_sm100.so``  -- every ``csrc/sm100/*.cu`` kernel, compiled by ``nvcc`` for sm_100a only
   (``-gencode arch=compute_100a,code=sm_100a``) and loaded from Python through ``ctypes``.
-* ``hg_dp_core*.so`` / ``hg_dataset_helpers*.so`` -- the host-side C++ modules (pybind11): the
-  strategy-search dynamic program and the dataset index builders.
+* ``hg_dp_core*.so`` / ``hg_dataset_helpers*.so`` / ``hg_torch_ops*.so`` -- the host-side C++ modules (pybind11): the
+  strategy-search dynamic program, the dataset index builders and the autograd nodes of the layers' operations.
 
 Objects are rebuilt only when a source or header is newer than the object.  ``nvcc`` cross-compiles
 without a GPU, so the build also serves as the "does it compile" check on a CPU-only machine.
@@ -123,7 +123,26 @@ def build_host(verbose: bool = False):
             if verbose:
                 print("[build] g++", src)
         out.append(target)
+    out.append(build_torch_ops(verbose))
     return out
+
+
+def build_torch_ops(verbose: bool = False) -> Path:
+    """``hg_torch_ops``: the autograd nodes of the layers' operations, against this interpreter's torch."""
+    from torch.utils.cpp_extension import include_paths, library_paths
+
+    s = CSRC / "host" / "torch_ops.cpp"
+    target = LIB_DIR / ("hg_torch_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
+    if _newer([s, *(CSRC / "sm100" / h for h in ("attn_tensor.h", "decoder_step.h"))], target):
+        LIB_DIR.mkdir(exist_ok=True)
+        cuda = Path(_nvcc()).resolve().parent.parent / "include"
+        inc = [f for p in (*include_paths(), str(cuda), sysconfig.get_paths()["include"]) for f in ("-I", p)]
+        libs = ["-L" + p for p in library_paths()]
+        _run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=hg_torch_ops", *inc, str(s), "-o",
+              str(target), *libs, "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda"])
+        if verbose:
+            print("[build] g++", s.name)
+    return target
 
 
 def build_all(verbose: bool = False, variants: bool = True):

@@ -10,30 +10,9 @@
 // from here; one after another 590 us, of which 517 us are kernels (attention on the tile kernel, products on
 // gemm_skinny.cu).  The kernels are launched as a chain (sm100_common.cuh): each may start while the one before it ends, and the
 // products read their first weights meanwhile; the same step as a CUDA graph 519 us without and 477 with.  Host code only.
+#include "decoder_step.h"
 #include "entry_points.h"
 #include "sm100_common.cuh"
-
-extern "C" {
-
-// Mirrored by ``DecoderStep`` in ops/_lib.py.  x and out are [S * B, H] contiguous (S tokens of B sequences, S * B <= 128);
-// the caches point at the first of the B sequences, position 0, and `past` positions of them are filled.
-struct HgDecoderStep {
-  int S, B, H, nh, ng, hd, F, past;
-  int rms, act, rot_dim, interleaved;      // act: kind of hg_glu_fwd; rot_dim 0: no rotation
-  float eps, scale;
-  const void *w_norm1, *b_norm1, *w_qkv, *b_qkv, *w_proj, *b_proj;
-  const void *w_norm2, *b_norm2, *w_fc1, *b_fc1, *w_fc2, *b_fc2;
-  const void *cos_t, *sin_t;
-  void *k_cache, *v_cache;
-  long long k_ss, k_sb, v_ss, v_sb;
-  const void* x;
-  void* out;
-  void* ws;
-  long long ws_bytes;
-  int launches;                            // set by hg_decoder_step: kernels that it has launched
-};
-
-}  // extern "C"
 
 namespace {
 

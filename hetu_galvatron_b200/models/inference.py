@@ -53,6 +53,20 @@ def _stage(model):
     return model.model if hasattr(model, "model") and hasattr(model.model, "units") else model
 
 
+def _attentions(root) -> list:
+    """Every attention module below ``root`` once (``root.modules()`` builds a dotted name for each module it passes)."""
+    found, seen, todo = [], set(), [root]
+    while todo:
+        m = todo.pop()
+        if m is None or id(m) in seen:
+            continue
+        seen.add(id(m))
+        if isinstance(m, SelfAttention):
+            found.append(m)
+        todo.extend(m._modules.values())
+    return found
+
+
 @torch.no_grad()
 def forward_step(model, tokens: torch.Tensor, ctx: StaticInferenceContext) -> torch.Tensor:
     """Run ``tokens [B, S_new]`` through the stage with the caches of ``ctx`` and advance it.  Returns the local
@@ -60,7 +74,7 @@ def forward_step(model, tokens: torch.Tensor, ctx: StaticInferenceContext) -> to
     stage = _stage(model)
     if not (stage.has_embedding and stage.has_head):
         raise NotImplementedError("cached generation runs on a single pipeline stage")
-    attns = [m for m in stage.modules() if isinstance(m, SelfAttention)]
+    attns = _attentions(stage)
     for a in attns:
         a.inference_context = ctx
     try:

@@ -481,7 +481,11 @@ class _Add(torch.autograd.Function):
 
 def ops_add(a, b):
     if a.is_cuda and a.dtype in (torch.bfloat16, torch.float16) and a.is_contiguous() and b.is_contiguous() and a.shape == b.shape:
-        return _Add.apply(a, b)
+        from ..ops import _lib
+
+        native = _lib.native()
+        out = native.add(a, b) if native is not None else None
+        return out if out is not None else _Add.apply(a, b)
     return a + b
 
 
@@ -540,6 +544,13 @@ class GalvatronDecoderLayer(nn.Module):
             return None
         weights = [t for h in (n1, att.linear_qkv, att.linear_proj, n2, mlp.linear_fc1, mlp.linear_fc2)
                    for t in (h.weight, h.bias)]
+        native = _lib.native()
+        if native is not None:
+            from ..ops.fused import _KIND
+
+            usable = native.decoder_weights(x, weights, att.nh, att.ng, att.hd, mlp.Fl, _KIND[s.activation])
+            if usable is not None:
+                return weights if usable else None
         shapes = ((s.hidden,), ((att.nh + 2 * att.ng) * att.hd, s.hidden), (s.hidden, att.nh * att.hd), (s.hidden,),
                   (mlp.Fl * (2 if s.gated else 1), s.hidden), (s.hidden, mlp.Fl))
         if not (all(w.shape == shape for w, shape in zip(weights[::2], shapes))
@@ -558,9 +569,15 @@ class GalvatronDecoderLayer(nn.Module):
         s, ic = att.spec, att.inference_context
         S, B, H = x.shape
         kc, vc, past, b0, cos, sin = att.cache_for(ic, x, S, B)
+        n1 = self.attn.input_layernorm
+        native = _lib.native()
+        if native is not None:
+            out = native.decoder_step(x, weights, kc, vc, cos, sin, past, b0, att.nh, att.ng, att.hd, mlp.Fl, n1.rms,
+                                      _KIND[s.activation], s.rope_interleaved, n1.eps)
+            if out is not None:
+                return out
         if not ops.attention.caches_usable(x, kc, vc, past, S, b0, B, att.ng, att.hd):
             return self.ffn(self.attn(x), x)
-        n1, n2 = self.attn.input_layernorm, self.ffn.post_attention_layernorm
         out = torch.empty_like(x)
         d = _lib.DecoderStep(
             S, B, H, att.nh, att.ng, att.hd, mlp.Fl, past, int(n1.rms), _KIND[s.activation],

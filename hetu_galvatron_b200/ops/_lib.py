@@ -180,7 +180,41 @@ def load():
         lib.hg_status_address.restype = c_void_p
         lib.hg_status_address.argtypes = []
     _LIB = lib
+    _bind_native(lib)
     return lib
+
+
+# The autograd nodes of the layers' operations in C++ (csrc/host/torch_ops.cpp), launching the kernels of the loaded library.
+# None until load(), and where the module cannot be had: the Python classes of this package then do the same.
+NATIVE = None
+
+
+def _bind_native(lib):
+    global NATIVE
+    try:
+        from ..csrc import build as _build
+
+        if os.environ.get("HG_AUTOBUILD", "1") == "1" and not list(_LIB_DIR.glob("hg_torch_ops*.so")):
+            _build.build_torch_ops()
+        from .._lib import hg_torch_ops
+    except Exception as e:  # noqa: BLE001  (no compiler, another torch)
+        import warnings
+
+        warnings.warn("hg_torch_ops is not usable (%s): autograd nodes run in Python" % (e,))
+        return
+    names = ("hg_gemm_bf16", "hg_gemm2_bf16", "hg_gemm_skinny_bf16", "hg_colsum_parts", "hg_colsum_bf16", "hg_norm_fwd",
+             "hg_norm_bwd", "hg_glu_fwd", "hg_glu_bwd", "hg_add_bf16", "hg_rope", "hg_flash_fwd", "hg_flash_bwd_scratch",
+             "hg_flash_bwd_ws", "hg_decoder_step", "hg_decoder_step_scratch")
+    mode = {"0": 0, "1": 1}.get(os.environ.get("HG_GEMM_PAIR", "auto"), -1)
+    hg_torch_ops.bind({n: ctypes.cast(getattr(lib, n), c_void_p).value for n in names}, _PRECISION == "fp16", mode, KernelError)
+    NATIVE = hg_torch_ops
+
+
+def native():
+    """The C++ autograd nodes, bound to the loaded library, or None."""
+    if _LIB is None:
+        load()
+    return NATIVE
 
 
 class KernelError(RuntimeError):
@@ -230,9 +264,11 @@ def count_launch(n: int = 1):
 
 
 def launches() -> int:
-    return _launch_count
+    return _launch_count + (NATIVE.launches() if NATIVE is not None else 0)
 
 
 def reset_launches():
     global _launch_count
     _launch_count = 0
+    if NATIVE is not None:
+        NATIVE.reset_launches()

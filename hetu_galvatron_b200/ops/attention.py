@@ -124,6 +124,11 @@ def flash_attention_packed(qkv: torch.Tensor, S: int, B: int, nh: int, ng: int, 
         return o.reshape(S * B, nh * hd)
     if hd not in (64, 128):
         raise ValueError("the sm_100a flash attention kernels support head_dim 64 and 128")
+    native = _lib.native()
+    if native is not None:
+        out = native.flash_packed(qkv, S, B, nh, ng, hd, causal, scale)
+        if out is not None:
+            return out
     return _FlashPacked.apply(qkv.contiguous(), S, B, nh, ng, hd, causal, scale)
 
 

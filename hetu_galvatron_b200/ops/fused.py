@@ -90,6 +90,11 @@ def norm(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor | None = None, eps: f
     if not x.is_cuda:
         h = x if residual is None else x + residual
         return _norm_ref(h, w, b, eps, rms), h
+    native = _lib.native()
+    if native is not None:
+        out = native.norm(x, residual, w, b, eps, rms)
+        if out is not None:
+            return out if residual is not None else (out[0], x)
     x2 = x.reshape(-1, shp[-1]).contiguous()
     r2 = residual.reshape(-1, shp[-1]).contiguous() if residual is not None else None
     if r2 is None:
@@ -207,6 +212,11 @@ def rope_packed(qkv: torch.Tensor, head_slots: torch.Tensor, hd: int, cos: torch
     head_slots = head_slots.to(torch.int32).contiguous()
     if pos is not None:
         pos = pos.to(torch.int32).contiguous()
+    native = _lib.native()
+    if native is not None:
+        out = native.rope_packed(qkv, head_slots, hd, cos, sin, batch, pos, pos_offset, interleaved)
+        if out is not None:
+            return out
     return _RopeInplace.apply(qkv, head_slots, hd, cos, sin, batch, pos, pos_offset, rot_dim, interleaved)
 
 
@@ -287,6 +297,11 @@ def activation(y: torch.Tensor, kind: str = "swiglu") -> torch.Tensor:
     """``swiglu`` / ``geglu``: ``act(y[..., :F]) * y[..., F:]``;  ``gelu``: tanh-approximated GELU."""
     if not y.is_cuda:
         return _act_ref(y, kind)
+    native = _lib.native()
+    if native is not None:
+        out = native.activation(y, _KIND[kind])
+        if out is not None:
+            return out
     shp = y.shape
     out = _Glu.apply(y.reshape(-1, shp[-1]).contiguous(), _KIND[kind])
     return out.view(*shp[:-1], out.shape[-1])

@@ -197,6 +197,11 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None) -
     """``x @ w.T (+ bias)`` over the last dimension; leading dimensions are flattened."""
     if not x.is_cuda:
         return torch.nn.functional.linear(x, w, bias)
+    native = _lib.native()
+    if native is not None:
+        y = native.linear(x, w, bias)
+        if y is not None:
+            return y
     shp = x.shape
     y = _Linear.apply(x.reshape(-1, shp[-1]), w, bias)
     return y if len(shp) == 2 else y.view(*shp[:-1], w.shape[0])

@@ -612,6 +612,18 @@ class _Boundary(torch.autograd.Function):
         return g, None
 
 
+def _boundary(x: torch.Tensor, cb) -> torch.Tensor:
+    """``x`` with ``cb`` called when its gradient passes."""
+    if x.is_cuda:
+        from ..ops import _lib
+
+        native = _lib.native()
+        out = native.boundary(x, cb) if native is not None else None
+        if out is not None:
+            return out
+    return _Boundary.apply(x, cb)
+
+
 class UnitWrapper(nn.Module):
     """Runs a unit's module between the ZeRO hooks (gather before forward / backward, release after,
     gradient reduction after the backward) and optional activation recomputation."""
@@ -666,7 +678,7 @@ class UnitWrapper(nn.Module):
                 if pending[0] <= 0:
                     self._post_backward()
 
-            args = tuple(_Boundary.apply(a, _one_input_done) if torch.is_tensor(a) and a.requires_grad else a
+            args = tuple(_boundary(a, _one_input_done) if torch.is_tensor(a) and a.requires_grad else a
                          for a in args)
         if self.checkpoint and grad_mode:
             out = _torch_checkpoint(self.inner, *args, use_reentrant=False, **kwargs)
@@ -677,9 +689,9 @@ class UnitWrapper(nn.Module):
             e.release()
         if grad_mode:
             if torch.is_tensor(out) and out.requires_grad:
-                out = _Boundary.apply(out, self._pre_backward)
+                out = _boundary(out, self._pre_backward)
             elif isinstance(out, tuple):
-                out = tuple(_Boundary.apply(o, self._pre_backward) if torch.is_tensor(o) and o.requires_grad else o
+                out = tuple(_boundary(o, self._pre_backward) if torch.is_tensor(o) and o.requires_grad else o
                             for o in out)
         return out
 

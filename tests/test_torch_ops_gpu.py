@@ -1,0 +1,150 @@
+"""The C++ autograd nodes against the Python classes that they stand for: the same kernels, hence the same bits."""
+import contextlib
+
+import pytest
+import torch
+
+from hetu_galvatron_b200 import ops
+from hetu_galvatron_b200.models.modules import ops_add
+from hetu_galvatron_b200.ops import _lib
+
+pytestmark = pytest.mark.gpu
+DEV, LP = "cuda", torch.bfloat16
+
+
+@contextlib.contextmanager
+def python_nodes():
+    native, _lib.NATIVE = _lib.native(), None
+    try:
+        yield
+    finally:
+        _lib.NATIVE = native
+
+
+def both(build, inputs, params=()):
+    """Outputs, input gradients and parameter gradients (autograd's and main_grad) of ``build`` on either route."""
+    assert _lib.native() is not None
+    res = []
+    for route in (contextlib.nullcontext, python_nodes):
+        _lib.reset_launches()
+        with route():
+            xs = [t.detach().clone().requires_grad_(t.requires_grad) for t in inputs]
+            ps = []
+            for p in params:
+                q = torch.nn.Parameter(p.detach().clone())
+                if hasattr(p, "fresh"):
+                    q.main_grad, q.mg_fresh = torch.full(p.shape, 2.0, device=DEV), p.fresh
+                ps.append(q)
+            outs = build(*xs, *ps)
+            outs = outs if isinstance(outs, tuple) else (outs,)
+            g = torch.Generator(device=DEV).manual_seed(1)
+            torch.autograd.backward(outs, [torch.randn(o.shape, device=DEV, generator=g).to(o.dtype) for o in outs])
+        res.append(([*outs, *[t.grad for t in xs], *[p.grad for p in ps], *[getattr(p, "main_grad", None) for p in ps]],
+                    [getattr(p, "mg_fresh", None) for p in ps], _lib.launches()))
+    (a, fa, la), (b, fb, lb) = res
+    assert fa == fb and la == lb > 0 and len(a) == len(b)
+    for s, t in zip(a, b):
+        assert (s is None) == (t is None) and (s is None or (s.dtype == t.dtype and torch.equal(s, t)))
+    _lib.assert_healthy()
+
+
+def randn(*shape, grad=True, dtype=LP):
+    return torch.randn(*shape, device=DEV).to(dtype).requires_grad_(grad)
+
+
+def param(*shape, fresh=None):
+    p = torch.nn.Parameter(torch.randn(*shape, device=DEV).to(LP))
+    if fresh is not None:
+        p.fresh = fresh
+    return p
+
+
+# few rows, rows of more than two dimensions and in another order, pair tiles
+@pytest.mark.parametrize("shape,N", [((5, 64), 48), ((3, 7, 72), 104), ((300, 264), 520)])
+@pytest.mark.parametrize("biased", [False, True])
+@pytest.mark.parametrize("fresh", [None, True, False])
+def test_linear(shape, N, biased, fresh):
+    torch.manual_seed(N)
+    ps = [param(N, shape[-1], fresh=fresh)] + ([param(N)] if biased else [])
+    both(lambda x, w, b=None: ops.linear(x, w, b), [randn(*shape)], ps)
+    both(lambda x, w, b=None: ops.linear(x, w, b), [randn(*shape, grad=False)], ps)
+    if len(shape) == 3:
+        both(lambda x, w, b=None: ops.linear(x.transpose(0, 1), w, b), [randn(shape[1], shape[0], shape[2])], ps)
+
+
+@pytest.mark.parametrize("rms", [True, False])
+@pytest.mark.parametrize("residual", [True, False])
+@pytest.mark.parametrize("fresh", [None, True, False])
+def test_norm(rms, residual, fresh):
+    torch.manual_seed(2)
+    ps = [param(136, fresh=fresh)] + ([] if rms else [param(136)])
+
+    def run(x, *rest):
+        r, rest = (rest[0], rest[1:]) if residual else (None, rest)
+        y, h = ops.norm(x, rest[0], rest[1] if not rms else None, 1e-5, rms, residual=r)
+        return (y, h) if residual else y
+
+    both(run, [randn(3, 5, 136) for _ in range(1 + residual)], ps)
+    if residual:
+        both(lambda *a: run(*a)[0], [randn(3, 5, 136) for _ in range(2)], ps)      # the sum itself unused
+        both(lambda *a: run(*a)[1], [randn(3, 5, 136) for _ in range(2)], ps)      # only the sum used
+
+
+@pytest.mark.parametrize("kind,F", [("swiglu", 32), ("geglu", 48), ("gelu", 40)])
+def test_activation_and_add(kind, F):
+    both(lambda y: ops.activation(y, kind), [randn(2, 9, F)])
+    both(lambda y: ops.activation(y.transpose(0, 1), kind), [randn(2, 9, F)])
+    both(ops_add, [randn(4, 9, F), randn(4, 9, F)])
+
+
+@pytest.mark.parametrize("interleaved", [False, True])
+@pytest.mark.parametrize("positions", [False, True])
+@pytest.mark.parametrize("ng", [1, 2])
+def test_rotation_and_attention(interleaved, positions, ng):
+    S, B, nh, hd = 130, 2, 4, 64
+    cos, sin = ops.rope_tables(S + 8, hd, 10000.0, DEV)
+    slots = torch.tensor([g * (nh // ng + 2) + j for g in range(ng) for j in range(nh // ng + 1)], dtype=torch.int32, device=DEV)
+    pos = torch.randint(0, S, (S * B,), device=DEV) if positions else None
+
+    def run(x, w):
+        qkv = ops.rope_packed(ops.linear(x, w), slots, hd, cos, sin, B, pos, 0 if positions else 5, interleaved)
+        return ops.flash_attention_packed(qkv, S, B, nh, ng, hd)
+
+    both(run, [randn(S * B, 64)], [param((nh + 2 * ng) * hd, 64)])
+
+
+def test_saved_tensor_hooks_checkpoints_and_inference():
+    x, w = randn(40, 64), param(64, 64)
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t) or t.clone(), lambda t: t):
+        ops.activation(ops.linear(x, w), "swiglu").sum().backward()
+    assert len(packed) == 3
+    from torch.utils.checkpoint import checkpoint
+
+    got, want = (r(lambda t: ops.activation(ops.linear(t, w), "gelu"), x) for r in
+                 (lambda f, t: checkpoint(f, t, use_reentrant=False), lambda f, t: f(t)))
+    assert all(torch.equal(a, b) for a, b in zip(torch.autograd.grad(got.sum(), (x, w)), torch.autograd.grad(want.sum(), (x, w))))
+    with torch.inference_mode():
+        assert torch.equal(ops.linear(x, w), ops.linear(x, w)) and not ops.linear(x, w).requires_grad
+    y = ops.linear(x, w)
+    y.sum().backward()
+    with pytest.raises(RuntimeError, match="second time"):
+        y.sum().backward()
+    a = ops.linear(x, w)
+    b = ops.activation(a, "gelu")
+    a.detach().add_(1)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        b.sum().backward()
+
+
+def test_errors_are_those_of_the_python_route():
+    with pytest.raises(TypeError):
+        ops.linear(randn(8, 16, dtype=torch.float32), param(8, 16))
+    with pytest.raises(ValueError):
+        ops.linear(randn(8, 16), param(8, 24))
+    with pytest.raises(_lib.KernelError):
+        ops.norm(randn(8, 20), param(20), None, 1e-5, True)
+    w = param(64, 64)
+    w.main_grad = torch.zeros(32, 64, device=DEV)
+    with pytest.raises(ValueError, match="bad output"):
+        ops.linear(randn(300, 64), w).sum().backward()
