@@ -37,7 +37,8 @@ using V = const void*;
 using A = const HgAttnTensor*;
 struct Kernels {
   int (*gemm)(V, V, void*, V, int, int, int, int, int, int, int, int, int, int, void*);
-  int (*gemm2)(V, V, void*, V, int, int, int, int, int, int, int, int, int, int, void*);
+  int (*gemm2)(V, V, void*, V, int, int, int, int, int, int, int, int, int, int, void*, long long, void*);
+  long long (*gemm2_scratch)(int, int, int);
   int (*gemm_skinny)(V, V, void*, V, int, int, int, int, int, int, int, int, int, void*);
   int (*colsum_parts)(int, int);
   int (*colsum)(V, long long, int, int, void*, int, void*, void*);
@@ -119,7 +120,10 @@ void gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& out, const void*
     return count();
   }
   if (how == 1) {
-    const int rc = K.gemm2(a.data_ptr(), b.data_ptr(), out.data_ptr(), bias, m, n, k, lda, ldb, ldc, a_mn, b_mn, mode, 0, st);
+    const long long need = K.gemm2_scratch(m, n, k);        // parts of tiles that several CTA pairs share
+    const Tensor ws = need ? empty({need}, at::kByte, a) : Tensor();
+    const int rc = K.gemm2(a.data_ptr(), b.data_ptr(), out.data_ptr(), bias, m, n, k, lda, ldb, ldc, a_mn, b_mn, mode, 0,
+                           need ? ws.data_ptr() : nullptr, need, st);
     if (rc != -2) {
       check(rc, "hg_gemm2_bf16");
       return count();
@@ -655,7 +659,7 @@ void bind(const py::dict& fn, bool half, int pair_mode, py::object kernel_error)
   auto at = [&](const char* name, auto& slot) {
     slot = reinterpret_cast<std::decay_t<decltype(slot)>>(py::cast<uintptr_t>(fn[name]));
   };
-  at("hg_gemm_bf16", K.gemm); at("hg_gemm2_bf16", K.gemm2); at("hg_gemm_skinny_bf16", K.gemm_skinny);
+  at("hg_gemm_bf16", K.gemm); at("hg_gemm2_bf16", K.gemm2); at("hg_gemm2_scratch", K.gemm2_scratch); at("hg_gemm_skinny_bf16", K.gemm_skinny);
   at("hg_colsum_parts", K.colsum_parts); at("hg_colsum_bf16", K.colsum);
   at("hg_norm_fwd", K.norm_fwd); at("hg_norm_bwd", K.norm_bwd);
   at("hg_glu_fwd", K.glu_fwd); at("hg_glu_bwd", K.glu_bwd); at("hg_add_bf16", K.add); at("hg_rope", K.rope);

@@ -15,8 +15,9 @@
 // Every wait is bounded (2 s); a CTA that gives up raises its abort flag and the status word, its partner runs into
 // its own limit, and both still meet at the final cluster barrier and free their tensor memory.
 // No operand load uses cluster multicast: each CTA loads exactly the bytes it alone needs.
+#include <atomic>
 #include <cstdlib>
-#include <mutex>
+#include <random>
 
 #include "gemm2_core.cuh"
 
@@ -280,50 +281,50 @@ using namespace hg::gemm2;
 
 namespace {
 
-// Scratch of the tail split: partial tiles and arrival counters, one set per (device, stream) for up to four
-// streams per device (a launch on a fifth stream runs without the split).  Allocated on first use, never freed.
-constexpr int kSplitMaxUnits = 128;                 // >= number of CTA pairs
-struct SplitScratch {
-  cudaStream_t stream;
-  float* ws;
-  int* flags;
-};
-SplitScratch g_split[64][4] = {};
-std::mutex g_split_mu;
-
-bool split_scratch(cudaStream_t st, float** ws, int** flags) {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-  std::lock_guard<std::mutex> lk(g_split_mu);
-  for (int i = 0; i < 4; ++i) {
-    SplitScratch& e = g_split[dev][i];
-    if (e.ws != nullptr && e.stream != st) continue;
-    if (e.ws == nullptr) {
-      void* p = nullptr;
-      if (cudaMalloc(&p, size_t(kSplitMaxUnits) * kSplitTileFloats * sizeof(float) + kSplitMaxUnits * sizeof(int)) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-      }
-      e.ws = static_cast<float*>(p);
-      e.flags = reinterpret_cast<int*>(e.ws + size_t(kSplitMaxUnits) * kSplitTileFloats);
-      e.stream = st;
-    }
-    *ws = e.ws;
-    *flags = e.flags;
-    return true;
-  }
-  return false;
+// HG_GEMM_SPLIT_TAIL: 0 never, 1 wherever a slice keeps eight k-blocks, unset: by the rule of split_plan.
+int split_mode() {
+  static const int mode = [] {
+    const char* e = getenv("HG_GEMM_SPLIT_TAIL");
+    return e == nullptr || e[0] == 0 ? -1 : int(e[0] != '0');
+  }();
+  return mode;
 }
 
-// HG_GEMM_SPLIT_TAIL=1 switches the tail split on, 0 off.
-constexpr int kSplitDefault = 0;
-bool split_enabled() {
-  static int on = -1;
-  if (on < 0) {
-    const char* e = getenv("HG_GEMM_SPLIT_TAIL");
-    on = (e == nullptr || e[0] == 0) ? kSplitDefault : (e[0] != '0');
+// What a split costs, in k-blocks (0.3 us each): the parts' way through L2 and the flags, and each part that is added.
+constexpr int kSplitCost = 20, kPartCost = 8;
+
+struct SplitPlan {
+  int s, tail;                       // pairs per tail tile (0: no split), tail tiles
+  long long flag_bytes() const { return ((long long)tail * (s - 1) * 8 * sizeof(unsigned long long) + 255) / 256 * 256; }
+  long long bytes() const { return s < 2 ? 0 : flag_bytes() + (long long)tail * (s - 1) * kSplitTileFloats * sizeof(float); }
+};
+
+// How many pairs share each tile of the last wave, where the tiles leave part of it idle.
+// A tile takes 0.3 us per k-block.  A pair that adds parts reads each of them from L2 for about 2.4 us after its own last
+// product, and the flags and stores in front of that take 6 us, so a split into s slices pays where num_kb * (1 - 1/s) is more
+// than kSplitCost + kPartCost * (s - 1), and slice s pays beside s - 1 where num_kb / (s (s - 1)) is more than kPartCost.
+// One pair a tile against the rule's choice, us, fresh clocks: K = 2048 15.4 (never split; by four 20.9), K = 4096 24.5 by
+// three 21.0, K = 8192 42.3 by four 27.5; 81 tiles, 7 in the last wave, K = 4096 44.9 by three 42.8, K = 8192 83.7 by four
+// 69.7; 98 tiles, 24 in the last wave, K = 18944 211 by three 156; 256 tiles, 34 in the last wave, K = 32000 888 by two 782.
+// An attention block of 1531 x 3584 483 -> 475 us, a GPT2-XL MLP of 2997 rows 520 -> 502.
+SplitPlan split_plan(int tiles, int num_kb, int max_pairs) {
+  SplitPlan p{0, tiles % max_pairs};
+  if (split_mode() == 0 || p.tail == 0) return p;
+  int s = max_pairs / p.tail;
+  if (s > num_kb / 8) s = num_kb / 8;
+  if (split_mode() < 0) {
+    while (s > 1 && kPartCost * s * (s - 1) > num_kb) --s;               // the last part still pays for itself
+    if (s > 1 && num_kb - num_kb / s < kSplitCost + kPartCost * (s - 1)) s = 0;
+  } else if (s > 4) {
+    s = 4;
   }
-  return on != 0;
+  if (s > 1) p.s = s;
+  return p;
+}
+
+unsigned long long split_token() {
+  static std::atomic<unsigned long long> next{((unsigned long long)std::random_device{}() << 32) | 1u};
+  return next.fetch_add(1, std::memory_order_relaxed);
 }
 
 }  // namespace
@@ -371,30 +372,29 @@ static int launch_grouped2(const CUtensorMap& ta, const CUtensorMap& tb, const C
 
 template <bool A_MN, bool B_MN>
 static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p_in, int want_pairs,
-                   cudaStream_t st) {
+                   void* ws, long long ws_bytes, cudaStream_t st) {
   Params p = p_in;
   static int max_pairs = -1;
   auto k = gemm2_bf16_kernel<A_MN, B_MN>;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr;
   if (int rc = pair_config(k, &cfg, &attr, &max_pairs, st)) return rc;
-  const int pairs = want_pairs < max_pairs ? want_pairs : max_pairs;
-  cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
+  int pairs = want_pairs < max_pairs ? want_pairs : max_pairs;
   // Last wave partly filled: let several pairs share each of its tiles (see Params::split_s).
-  p.split_s = 0;
   const int tiles = p.tiles_m * p.tiles_n, num_kb = (p.K + BK - 1) / BK;
-  const int full = tiles / pairs, tail = tiles - full * pairs;
-  if (split_enabled() && p.k_ranges == nullptr && p.ready == nullptr && full >= 1 && tail >= 1 && pairs <= kSplitMaxUnits) {
-    int s = pairs / tail;
-    if (s > 4) s = 4;
-    if (s > num_kb / 8) s = num_kb / 8;
-    if (s >= 2 && split_scratch(st, &p.split_ws, &p.split_flags)) {
-      p.split_s = s;
-      p.split_tail_begin = full * pairs;
-      cudaError_t me = cudaMemsetAsync(p.split_flags, 0, size_t(tail) * s * sizeof(int), st);
-      if (me != cudaSuccess) return int(me);
+  p.split_s = 0;
+  if (ws != nullptr && p.ready == nullptr) {
+    const SplitPlan plan = split_plan(tiles, num_kb, max_pairs);
+    if (plan.s > 1 && ws_bytes >= plan.bytes()) {
+      p.split_s = plan.s;
+      p.split_tail_begin = tiles - plan.tail;
+      p.split_flags = static_cast<unsigned long long*>(ws);
+      p.split_ws = reinterpret_cast<float*>(static_cast<char*>(ws) + plan.flag_bytes());
+      p.split_token = split_token();
+      pairs = p.split_tail_begin > 0 ? max_pairs : plan.tail * plan.s;
     }
   }
+  cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
   cudaError_t e = cudaLaunchKernelEx(&cfg, k, ta, tb, tc, p);
   return int(e);
 }
@@ -415,8 +415,10 @@ extern "C" {
 
 // Same contract as hg_gemm_bf16 (gemm.cu), computed by CTA pairs.  Returns -2 when the device cannot co-schedule a
 // pair of these CTAs (the caller then uses the one-CTA kernel).
+// ws: scratch of ws_bytes bytes, 256-byte aligned (contents do not matter); with less than hg_gemm2_scratch bytes every tile
+// has one pair.
 int hg_gemm2_bf16(const void* A, const void* B, void* C, const void* bias, int M, int N, int K, int lda, int ldb,
-                  int ldc, int a_mn, int b_mn, int out_mode, int max_ctas, void* stream) {
+                  int ldc, int a_mn, int b_mn, int out_mode, int max_ctas, void* ws, long long ws_bytes, void* stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
     return -1;
@@ -443,10 +445,21 @@ int hg_gemm2_bf16(const void* A, const void* B, void* C, const void* bias, int M
   CUtensorMap tc;
   if ((rc = store_map(&tc, ta, p, M))) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (a_mn && b_mn) return launch2<true, true>(ta, tb, tc, p, pairs, st);
-  if (a_mn) return launch2<true, false>(ta, tb, tc, p, pairs, st);
-  if (b_mn) return launch2<false, true>(ta, tb, tc, p, pairs, st);
-  return launch2<false, false>(ta, tb, tc, p, pairs, st);
+  if (max_ctas != 0) ws = nullptr;
+  if (a_mn && b_mn) return launch2<true, true>(ta, tb, tc, p, pairs, ws, ws_bytes, st);
+  if (a_mn) return launch2<true, false>(ta, tb, tc, p, pairs, ws, ws_bytes, st);
+  if (b_mn) return launch2<false, true>(ta, tb, tc, p, pairs, ws, ws_bytes, st);
+  return launch2<false, false>(ta, tb, tc, p, pairs, ws, ws_bytes, st);
+}
+
+// Bytes of scratch that hg_gemm2_bf16 asks for on the current device (0: none).
+long long hg_gemm2_scratch(int M, int N, int K) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  static int max_pairs = -1;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr;
+  if (pair_config(gemm2_bf16_kernel<false, false>, &cfg, &attr, &max_pairs, nullptr)) return 0;
+  return split_plan(((M + CM - 1) / CM) * ((N + BN - 1) / BN), (K + BK - 1) / BK, max_pairs).bytes();
 }
 
 // Same contracts as hg_grouped_gemm_bf16 and hg_grouped_wgrad_bf16 (gemm.cu), computed by CTA pairs; -2 as above.

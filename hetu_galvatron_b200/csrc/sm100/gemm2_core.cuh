@@ -114,6 +114,10 @@ struct Unit {
   int tile, kb0, kb1, slice;
 };
 constexpr int kSplitTileFloats = CM * BN;
+// Word `q` (four columns) of 32-column block `c` of this thread's row in a partial tile: neighbouring lanes, neighbouring words.
+__device__ __forceinline__ int split_word(int warp8, int c, int q) {
+  return (((warp8 * (BN / 32) + c) * 8 + q) * 32 + int(lane_id())) * 4;
+}
 __device__ __forceinline__ int unit_count(const Params& p, int first, int step, int num_tiles) {
   if (p.split_s > 1) return p.split_tail_begin / step + (first < (num_tiles - p.split_tail_begin) * p.split_s ? 1 : 0);
   return first < num_tiles ? (num_tiles - first + step - 1) / step : 0;
@@ -315,6 +319,27 @@ __device__ __forceinline__ void tma_store_rows(const CUtensorMap* tm, StoreStage
   st.next ^= 1;
 }
 
+// The other slices' partial sums of a shared tile, as this warp's threads hold them (n = 0: none).
+struct Parts {
+  const float* base;
+  int n, warp8;
+  __device__ __forceinline__ void add(int c, uint32_t (&r)[32]) const {
+    for (int k = 0; k < n; ++k) {
+      float4 v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        v[q] = __ldcg(reinterpret_cast<const float4*>(base + size_t(k) * kSplitTileFloats + split_word(warp8, c, q)));
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        r[4 * q] = __float_as_uint(__uint_as_float(r[4 * q]) + v[q].x);
+        r[4 * q + 1] = __float_as_uint(__uint_as_float(r[4 * q + 1]) + v[q].y);
+        r[4 * q + 2] = __float_as_uint(__uint_as_float(r[4 * q + 2]) + v[q].z);
+        r[4 * q + 3] = __float_as_uint(__uint_as_float(r[4 * q + 3]) + v[q].w);
+      }
+    }
+  }
+};
+
 // The bias of N consecutive columns from col0 on, added to a thread's row.  Every lane reads the same 16 bytes.
 template <int N>
 __device__ __forceinline__ void add_bias_row(const Params& p, int col0, uint32_t* r) {
@@ -358,7 +383,7 @@ __device__ __forceinline__ void store_block64_tma(const Params& p, const CUtenso
 // Columns n0.. of the tile as TMA stores of 128-byte rows: 64 columns of 16 bits, or 32 of fp32.
 template <bool BIAS, bool F32>
 __device__ __forceinline__ void store_tile_tma(const Params& p, const CUtensorMap* tmC, StoreStage& st, uint32_t src, int row0,
-                                               int y0, int n0) {
+                                               int y0, int n0, const Parts& parts) {
 #pragma unroll 1
   for (int c = 0; c < BN && n0 + c < p.N; c += F32 ? 32 : 64) {
     uint32_t r0[32], r1[32];
@@ -366,6 +391,8 @@ __device__ __forceinline__ void store_tile_tma(const Params& p, const CUtensorMa
     if (!F32) tmem_ld32(src + c + 32, r1);
     tmem_ld_wait();
     if (!HG_BOUNDS_OK(row0 >= 0 && row0 < p.M, p.status)) continue;
+    parts.add(c / 32, r0);
+    if (!F32) parts.add(c / 32 + 1, r1);
     if constexpr (F32) {
       if (BIAS) add_bias_row<32>(p, n0 + c, r0);
       tma_store_rows(tmC, st, r0, n0 + c, y0);
@@ -420,11 +447,9 @@ __device__ __forceinline__ void load_old(const Params& p, int row0, int col0, fl
   }
 }
 
-// One 32 x 32 block from registers (thread = row), any output mode.  `part` (optional): the other slices' partial sums of
-// this block, slice k at part + k * kSplitTileFloats, rows 256 floats apart; they are added in slice order before anything
-// else.
+// One 32 x 32 block from registers (thread = row), any output mode.
 __device__ __forceinline__ void store_block_rows(const Params& p, uint32_t stg, int row0, int col0, const uint32_t (&src)[32],
-                                                 const float4 (&old)[8], const float* part = nullptr, int nparts = 0) {
+                                                 const float4 (&old)[8]) {
   const int lane = int(lane_id());
 #pragma unroll
   for (int j = 0; j < 8; ++j)
@@ -436,15 +461,6 @@ __device__ __forceinline__ void store_block_rows(const Params& p, uint32_t stg, 
   for (int i = 0; i < 8; ++i) v[i] = lds128(stg + (i * 4 + (lane >> 3)) * 144 + q * 4);
   __syncwarp();
   if (!HG_BOUNDS_OK(row0 >= 0 && row0 < p.M && col0 >= 0 && col0 < p.N, p.status)) return;
-  if (part != nullptr) {
-    for (int k = 0; k < nparts; ++k) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 a = __ldcg(reinterpret_cast<const float4*>(part + size_t(k) * kSplitTileFloats + (i * 4 + (lane >> 3)) * BN + q));
-        v[i].x += a.x; v[i].y += a.y; v[i].z += a.z; v[i].w += a.w;
-      }
-    }
-  }
   if (col >= p.N) return;
   float b[4] = {0.f, 0.f, 0.f, 0.f};
   if (p.bias != nullptr) {
@@ -535,7 +551,7 @@ __device__ __forceinline__ void load_old_whole(const Params& p, int row0, int co
 // The whole blocks of a tile part; returns the first column that is left.  With an accumulating mode the next block's old
 // values are in flight while this one is turned.
 template <int MODE>
-__device__ __forceinline__ int store_tile_whole(const Params& p, uint32_t stg, uint32_t src, int row0, int n0) {
+__device__ __forceinline__ int store_tile_whole(const Params& p, uint32_t stg, uint32_t src, int row0, int n0, const Parts& parts) {
   const int cols = min(BN, (p.N - n0) & ~31);
   float4 old[8];
   if (cols > 0) load_old_whole<MODE>(p, row0, n0, old);
@@ -546,6 +562,7 @@ __device__ __forceinline__ int store_tile_whole(const Params& p, uint32_t stg, u
     tmem_ld_wait();
     float4 next[8];
     if (c + 32 < cols) load_old_whole<MODE>(p, row0, n0 + c + 32, next);
+    parts.add(c / 32, r0);
     store_block_whole<MODE>(p, stg, row0, n0 + c, r0, old);
     if (MODE == kOutF32Acc || MODE == kOutBf16Acc) {
 #pragma unroll
@@ -558,15 +575,14 @@ __device__ __forceinline__ int store_tile_whole(const Params& p, uint32_t stg, u
 // The 32 x 256 part of a tile that this warp's lanes hold in tensor memory at `src`: rows row0.. of C (p.M: the first row
 // that is not this tile's), rows y0.. of the tensor map.
 __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorMap* tmC, StoreStage& st, uint32_t src, int row0,
-                                                int y0, int n0, bool whole_rows, const float* part = nullptr,
-                                                int nparts = 0) {
-  if (p.c_tma && whole_rows && part == nullptr) {
+                                                int y0, int n0, bool whole_rows, const Parts& parts = Parts{nullptr, 0, 0}) {
+  if (p.c_tma && whole_rows) {
     if (p.out_mode == kOutF32) {
-      if (p.bias != nullptr) store_tile_tma<true, true>(p, tmC, st, src, row0, y0, n0);
-      else store_tile_tma<false, true>(p, tmC, st, src, row0, y0, n0);
+      if (p.bias != nullptr) store_tile_tma<true, true>(p, tmC, st, src, row0, y0, n0, parts);
+      else store_tile_tma<false, true>(p, tmC, st, src, row0, y0, n0, parts);
     } else {
-      if (p.bias != nullptr) store_tile_tma<true, false>(p, tmC, st, src, row0, y0, n0);
-      else store_tile_tma<false, false>(p, tmC, st, src, row0, y0, n0);
+      if (p.bias != nullptr) store_tile_tma<true, false>(p, tmC, st, src, row0, y0, n0, parts);
+      else store_tile_tma<false, false>(p, tmC, st, src, row0, y0, n0, parts);
     }
     return;
   }
@@ -575,12 +591,12 @@ __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorM
     __syncwarp();
   }
   int c0 = 0;
-  if (part == nullptr && row0 + 32 <= p.M && four_aligned(p)) {
+  if (row0 + 32 <= p.M && four_aligned(p)) {
     switch (p.out_mode) {
-      case kOutF32: c0 = store_tile_whole<kOutF32>(p, st.base, src, row0, n0); break;
-      case kOutF32Acc: c0 = store_tile_whole<kOutF32Acc>(p, st.base, src, row0, n0); break;
-      case kOutBf16Acc: c0 = store_tile_whole<kOutBf16Acc>(p, st.base, src, row0, n0); break;
-      default: c0 = store_tile_whole<kOutBf16>(p, st.base, src, row0, n0); break;
+      case kOutF32: c0 = store_tile_whole<kOutF32>(p, st.base, src, row0, n0, parts); break;
+      case kOutF32Acc: c0 = store_tile_whole<kOutF32Acc>(p, st.base, src, row0, n0, parts); break;
+      case kOutBf16Acc: c0 = store_tile_whole<kOutBf16Acc>(p, st.base, src, row0, n0, parts); break;
+      default: c0 = store_tile_whole<kOutBf16>(p, st.base, src, row0, n0, parts); break;
     }
   }
 #pragma unroll 1
@@ -590,7 +606,8 @@ __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorM
     uint32_t r0[32];
     tmem_ld32(src + c, r0);
     tmem_ld_wait();
-    store_block_rows(p, st.base, row0, n0 + c, r0, old, part ? part + c : nullptr, nparts);
+    parts.add(c / 32, r0);
+    store_block_rows(p, st.base, row0, n0 + c, r0, old);
   }
 }
 
@@ -610,67 +627,64 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
     tile_coords(p, tile, tm, tn);
     const int row0 = tm * CM + int(rank) * BM + wq * 32;   // first of this warp's 32 rows
     const int n0 = tn * BN;
-    // a tail tile shared with other pairs: where this pair's partial goes, or where the others' are
+    // a tail tile shared with other pairs: the last slice writes it, the others leave their parts
     const bool shared_tile = p.split_s > 1 && tile >= p.split_tail_begin;
-    const int tail_idx = tile - p.split_tail_begin;
-    const int in_row = int(rank) * BM + wq * 32;           // this warp's first row inside the 256 x 256 tile
-    float* ws_mine = nullptr;
-    const float* ws_others = nullptr;
-    if (shared_tile) {
-      float* ws_tile = p.split_ws + size_t(tail_idx) * (p.split_s - 1) * kSplitTileFloats;
-      if (w.slice > 0) ws_mine = ws_tile + size_t(w.slice - 1) * kSplitTileFloats;
-      else ws_others = ws_tile;
-    }
+    const int tail_idx = tile - p.split_tail_begin, warp8 = int(rank) * EPI_WARPS + wq;
+    const bool leaves_part = shared_tile && w.slice + 1 < p.split_s;
+    float* ws_tile = shared_tile ? p.split_ws + size_t(tail_idx) * (p.split_s - 1) * kSplitTileFloats : nullptr;
+    unsigned long long* flags = shared_tile ? p.split_flags + size_t(tail_idx) * (p.split_s - 1) * 8 + warp8 : nullptr;
+    const Parts parts{ws_tile, shared_tile && !leaves_part ? p.split_s - 1 : 0, warp8};
     if (!mbar_wait_warp(&s.tmem_full[acc], acc_phase, p.status, kTimeoutTmemFull, s.abort)) {
       *s.abort = 1;
       break;
     }
     tc_fence_after();
-    if (ws_others != nullptr) {
-      // every epilogue warp of the other slices' pairs (8 each) has stored its part: bounded wait, one lane polls
-      int landed = 1;
-      if (lane == 0) {
-        for (int k = 1; landed && k < p.split_s; ++k) {
-          const int* flag = p.split_flags + tail_idx * p.split_s + k;
-          const uint64_t t0 = globaltimer_ns();
-          while (ld_acquire_gpu(flag) < 2 * EPI_WARPS) {
-            if (*s.abort || globaltimer_ns() - t0 > kWaitLimitNs) {
-              set_status(p.status, kTimeoutPeerFlag);
-              landed = 0;
-              break;
+    const uint32_t src = tmem_base + lane_off + acc * BN;
+    if (row0 < p.M) {   // warp-uniform, and the same for the slices of a tile
+      if (leaves_part) {
+        float* dst = ws_tile + size_t(w.slice) * kSplitTileFloats;
+#pragma unroll 1
+        for (int c = 0; c < BN / 32; ++c) {
+          uint32_t r0[32];
+          tmem_ld32(src + c * 32, r0);
+          tmem_ld_wait();
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            __stcg(reinterpret_cast<uint4*>(dst + split_word(warp8, c, q)),
+                   make_uint4(r0[4 * q], r0[4 * q + 1], r0[4 * q + 2], r0[4 * q + 3]));
+        }
+        __threadfence();
+        __syncwarp();
+        if (lane == 0) st_release_gpu(flags + w.slice * 8, p.split_token);
+      } else {
+        // this warp's rows of the other slices' parts: bounded wait, one lane polls.  They are slices of lower-numbered pairs,
+        // which the device starts first.
+        int landed = 1;
+        if (parts.n > 0 && lane == 0) {
+          for (int k = 0; landed && k < parts.n; ++k) {
+            const uint64_t t0 = globaltimer_ns();
+            while (ld_acquire_gpu(flags + k * 8) != p.split_token) {
+              if (*s.abort || globaltimer_ns() - t0 > kWaitLimitNs) {
+                set_status(p.status, kTimeoutPeerFlag);
+                landed = 0;
+                break;
+              }
+              __nanosleep(64);
             }
-            __nanosleep(64);
           }
         }
+        landed = __shfl_sync(0xffffffffu, landed, 0);
+        __syncwarp();                     // what lane 0 has acquired is every lane's
+        if (!landed) {
+          *s.abort = 1;
+          break;
+        }
+        store_tile_part(p, tmC, st, src, row0, row0, n0, true, parts);
+        if (parts.n > 0) {
+          __syncwarp();
+          if (lane < parts.n) flags[lane * 8] = 0;    // the next launch's token is another one; a replayed graph's is not
+        }
       }
-      landed = __shfl_sync(0xffffffffu, landed, 0);
-      if (!landed) {
-        *s.abort = 1;
-        break;
-      }
-    }
-    const uint32_t src = tmem_base + lane_off + acc * BN;
-    if (ws_mine != nullptr) {
-#pragma unroll 1
-      for (int c = 0; c < BN / 32; ++c) {
-        uint32_t r0[32];
-        tmem_ld32(src + c * 32, r0);
-        tmem_ld_wait();
-        // partial tile: row r of this thread's lane = tile row in_row + lane, 32 consecutive floats
-        float* dst = ws_mine + size_t(in_row + lane) * BN + c * 32;
-#pragma unroll
-        for (int i = 0; i < 32; i += 4)
-          __stcg(reinterpret_cast<float4*>(dst + i), make_float4(__uint_as_float(r0[i]), __uint_as_float(r0[i + 1]),
-                                                                 __uint_as_float(r0[i + 2]), __uint_as_float(r0[i + 3])));
-      }
-    } else if (row0 < p.M) {   // warp-uniform
-      store_tile_part(p, tmC, st, src, row0, row0, n0, true, ws_others ? ws_others + size_t(in_row) * BN : nullptr,
-                      p.split_s - 1);
-    }
-    if (ws_mine != nullptr) {
-      __threadfence();
-      __syncwarp();
-      if (lane == 0) atomicAdd(p.split_flags + tail_idx * p.split_s + w.slice, 1);
     }
     tc_fence_before();
     // the accumulator buffer is free again once all 256 epilogue threads of the pair have read it

@@ -66,14 +66,16 @@ struct Params {
   int groups;
   long long c_group_stride;
   // Optional split of the last, partly filled wave (CTA-pair kernel only): tiles from `split_tail_begin` on are each
-  // computed by `split_s` pairs, every pair taking a contiguous share of the k-blocks.  Slices 1.. leave their fp32
-  // partial tile in `split_ws` (256 x 256 floats per (tail tile, slice - 1)) and count their eight epilogue warps into
-  // `split_flags[tail tile * split_s + slice]`; slice 0 waits for them (bounded) and adds the partials in slice order,
-  // so the result does not depend on timing.  split_s < 2: off.
+  // computed by `split_s` pairs, every pair taking a contiguous share of the k-blocks.  All but the last of them leave their
+  // fp32 partial tile in `split_ws` (256 x 256 floats per (tail tile, slice), in the order in which the epilogue's threads hold
+  // it), and each of their eight epilogue warps then writes `split_token` to its word of `split_flags` ([tail tile][slice][8]);
+  // the last slice's warps wait for the words of their own rows (bounded), add the parts in slice order, so that the result
+  // does not depend on timing, and clear the words.  split_s < 2: off.
   int split_s;
   int split_tail_begin;
   float* split_ws;
-  int* split_flags;
+  unsigned long long* split_flags;
+  unsigned long long split_token;    // differs from launch to launch: whatever the words held before is not it
   int c_tma;                  // CTA-pair kernels: full blocks of C leave through the tensor map of C (plain 16-bit store)
 };
 
@@ -125,6 +127,15 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
+}
+
+__device__ __forceinline__ unsigned long long ld_acquire_gpu(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release_gpu(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 struct SmemLayout {

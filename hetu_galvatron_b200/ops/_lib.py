@@ -75,7 +75,8 @@ _SIGNATURES = {
     "hg_decoder_step_scratch": [ctypes.POINTER(DecoderStep)],
     "hg_decoder_step": [ctypes.POINTER(DecoderStep), c_void_p],
     "hg_gemm_bf16": [c_void_p] * 4 + [c_int] * 10 + [c_void_p],
-    "hg_gemm2_bf16": [c_void_p] * 4 + [c_int] * 10 + [c_void_p],
+    "hg_gemm2_bf16": [c_void_p] * 4 + [c_int] * 10 + [c_void_p, c_ll, c_void_p],
+    "hg_gemm2_scratch": [c_int] * 3,
     "hg_gemm_skinny_bf16": [c_void_p] * 4 + [c_int] * 9 + [c_void_p],
     "hg_colsum_parts": [c_int, c_int],
     "hg_colsum_bf16": [c_void_p, c_ll, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p],
@@ -174,7 +175,7 @@ def load():
             continue
         fn.argtypes = argtypes
         fn.restype = c_int
-    for name in ("hg_flash_decode_scratch", "hg_decoder_step_scratch", "hg_flash_bwd_scratch"):
+    for name in ("hg_flash_decode_scratch", "hg_decoder_step_scratch", "hg_flash_bwd_scratch", "hg_gemm2_scratch"):
         getattr(lib, name).restype = c_ll
     if hasattr(lib, "hg_status_address"):
         lib.hg_status_address.restype = c_void_p
@@ -202,7 +203,7 @@ def _bind_native(lib):
 
         warnings.warn("hg_torch_ops is not usable (%s): autograd nodes run in Python" % (e,))
         return
-    names = ("hg_gemm_bf16", "hg_gemm2_bf16", "hg_gemm_skinny_bf16", "hg_colsum_parts", "hg_colsum_bf16", "hg_norm_fwd",
+    names = ("hg_gemm_bf16", "hg_gemm2_bf16", "hg_gemm2_scratch", "hg_gemm_skinny_bf16", "hg_colsum_parts", "hg_colsum_bf16", "hg_norm_fwd",
              "hg_norm_bwd", "hg_glu_fwd", "hg_glu_bwd", "hg_add_bf16", "hg_rope", "hg_flash_fwd", "hg_flash_bwd_scratch",
              "hg_flash_bwd_ws", "hg_decoder_step", "hg_decoder_step_scratch")
     mode = {"0": 0, "1": 1}.get(os.environ.get("HG_GEMM_PAIR", "auto"), -1)

@@ -126,8 +126,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         _lib.count_launch()
         return out
     if _use_pair(M, N, pair):
+        need = lib.hg_gemm2_scratch(M, N, K) if max_ctas == 0 else 0   # parts of tiles that several CTA pairs share
+        ws = torch.empty(need, dtype=torch.uint8, device=a.device) if need else None
         rc = lib.hg_gemm2_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), _lib.ptr(bias), M, N, K, a.stride(0),
-                               b.stride(0), out.stride(0), int(a_mn), int(b_mn), out_mode, max_ctas, _lib.stream())
+                                  b.stride(0), out.stride(0), int(a_mn), int(b_mn), out_mode, max_ctas, _lib.ptr(ws), need,
+                                  _lib.stream())
         if rc == 0:
             _lib.count_launch()
             return out

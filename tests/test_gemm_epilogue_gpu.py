@@ -75,3 +75,45 @@ def test_wide_stores_stay_inside_their_window(M, N, K, mode, biased):
     out.fill_(2.0)
     assert (whole == 2.0).all()
     _lib.assert_healthy()
+
+
+# tiles of the last wave shared along K by the default rule: one tile and no whole wave, a ragged few with every layout's
+# k-blocks uneven over the slices, a last wave behind a whole one; in a window, with a bias, every result type
+@pytest.mark.parametrize("M,N,K", [(256, 256, 4096), (300, 520, 8200), (2304, 2304, 4168)])
+@pytest.mark.parametrize("mode", [OUT_BF16, OUT_F32, OUT_F32_ACC])
+@pytest.mark.parametrize("a_mn,b_mn,biased", [(False, False, True), (False, True, False), (True, True, False)])
+def test_shared_tiles_of_the_last_wave(M, N, K, mode, a_mn, b_mn, biased):
+    assert _lib.load().hg_gemm2_scratch(M, N, K) > 0 and _lib.load().hg_gemm2_scratch(M, N, 512) == 0
+    g = torch.Generator(device=DEV).manual_seed(M + K + mode)
+    pad = lambda r, c: torch.randn(r, (c + 7) // 8 * 8, device=DEV, generator=g).to(torch.bfloat16)[:, :c]
+    a, b = pad(K, M) if a_mn else pad(M, K), pad(K, N) if b_mn else pad(N, K)
+    bias = torch.randn(N, device=DEV, generator=g).to(torch.bfloat16) if biased else None
+    ref = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double() + (bias.double() if biased else 0.0)
+    whole = torch.full((M + 2, N + 8), 2.0, device=DEV, dtype=torch.bfloat16 if mode == OUT_BF16 else torch.float32)
+    out = whole[1:M + 1, 4:4 + N]
+    run = lambda: ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out, out_mode=mode, bias=bias, pair=True)
+    run()
+    first = out.clone()
+    want = ref + (2.0 if mode == OUT_F32_ACC else 0.0)
+    # fp32 sums of K products of unit normals; one rounding to 16 bits where C is 16 bits wide
+    assert torch.allclose(first.double(), want, rtol=2.0 ** -8 if mode == OUT_BF16 else 1e-6, atol=2e-5 * K ** 0.5)
+    graph, other = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    out.fill_(2.0)
+    with torch.cuda.graph(graph):
+        run()
+    for _ in range(3):                                # a replayed launch finds the flags cleared
+        out.fill_(2.0)
+        graph.replay()
+        assert torch.equal(out, first)
+    results = []
+    for s in (torch.cuda.current_stream(), other):    # launches of two streams do not share their parts
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s):
+            for _ in range(4):
+                results.append(ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out_mode=OUT_F32 if mode == OUT_F32_ACC else mode,
+                                        bias=bias, pair=True))
+    torch.cuda.synchronize()
+    assert all(torch.equal(r, results[0]) for r in results)
+    whole[1:M + 1, 4:4 + N] = 2.0
+    assert (whole == 2.0).all()
+    _lib.assert_healthy()
