@@ -1706,9 +1706,9 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   uint64_t* v_empty = bars + 8;    // 1
   uint64_t* s_full = bars + 9;     // 1
   uint64_t* s_empty = bars + 10;   // 1
-  uint64_t* ds_full = bars + 11;   // 1
-  uint64_t* ds_empty = bars + 12;  // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* ds_full = bars + 11;   // 2, by step parity: a warp may store the next step's dS before another has stored this one's
+  uint64_t* ds_empty = bars + 13;  // 2
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
@@ -1730,7 +1730,8 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     mbar_init(v_empty, 1);
     mbar_init(s_full, 1);
     mbar_init(s_empty, kSoftmaxWarps);   // one arrival per softmax warp (mbar_arrive_warp)
-    mbar_init(ds_full, kSoftmaxWarps);
+    mbar_init(&ds_full[0], kSoftmaxWarps);
+    mbar_init(&ds_full[1], kSoftmaxWarps);
     mbar_init(&ds_empty[0], 1);
     mbar_init(&ds_empty[1], 1);
     *abort_flag = 0;
@@ -1817,7 +1818,7 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         HG_DKV_TICK(t0);
         if (it + 1 < n_it) { ok = issue_s(it + 1); if (!ok) break; }
         HG_DKV_TOCK(tm_s, t0);
-        if (!mbar_wait_warp(ds_full, it & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&ds_full[it & 1], (it >> 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
         tc_fence_after();
         HG_DKV_TOCK(tm_wait_ds, t0);
         const uint32_t aK = smem_u32(sK + ks_d * L::kKV);
@@ -1900,7 +1901,7 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive_warp(ds_full);
+      mbar_arrive_warp(&ds_full[it & 1]);
       HG_DKV_TOCK(tm_st, t0);
     }
     HG_DKV_REPORT(24, n_it, tm_wait_s, tm_ld, tm_math, tm_st);
