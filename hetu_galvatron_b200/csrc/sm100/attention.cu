@@ -1224,6 +1224,9 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   // head dim 64: dS^T is formed from fp32 probabilities, as in the 64-query kernel
   constexpr bool kExactP = HD == 64;
   constexpr int CPT = 128 / NWG;               // query columns per thread and step
+  // Works on further blocks of the grid (WorkSlot) where a block is short: 1600 blocks of 8 x 1024 tokens and 25 heads of 64
+  // 156 -> 144 us.  The 2048 blocks of 2 x 4096 tokens and 32 heads of 128 gain less than the running counters cost: 535 -> 542.
+  constexpr bool kTakesMore = HD == 64;
   extern __shared__ uint8_t smem_raw[];
   using L = Dkv128Smem<HD>;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1250,30 +1253,43 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   uint64_t* acc_full = bars + 15;    // the last dK product has completed
   uint64_t* stats_full = bars + 16;  // 2
   uint64_t* x_free = bars + 18;      // every thread has loaded its S^T values: the S^T columns may be overwritten
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+  uint64_t* kv_empty = bars + 19;    // the last products that read K and V have completed
+  uint64_t* acc_empty = bars + 20;   // the epilogue has read dV and dK
+  const WorkSlot work{reinterpret_cast<uint4*>(bars + 24), bars + 21, bars + 22};
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
-  const int g = blockIdx.y, b = blockIdx.z;                   // g = kv head
-  int kb = blockIdx.x, mine = 0, sharers = 1;                 // key block, this CTA among those that share it
-  if constexpr (SHARED) {
-    int left = blockIdx.x;
-    for (kb = 0;; ++kb) {
-      sharers = dkv_block_ctas(p, dkv_block_steps(p, kb));
-      if (left < sharers) break;
-      left -= sharers;
-    }
-    mine = left;
-  }
-  const int k0 = kb * 128;
-  int q_first = 0;                                            // first query row that can see this key block
-  if (p.causal) q_first = max(0, p.k_pos0 + k0 - p.q_pos0);
-  const int qs0 = q_first / 128;                              // first 128-row query step
   const int n_qs = (p.Sq + 127) / 128;
-  const int steps_per_head = max(0, n_qs - qs0);
-  const int n_steps = steps_per_head * p.qpg;
-  const int it0 = SHARED ? n_steps * mine / sharers : 0;      // this CTA's steps, heads outside, queries inside
-  const int n_it = SHARED ? n_steps * (mine + 1) / sharers - it0 : n_steps;
+  // What a block of the grid is: a kv head's key block and some of its query steps, heads outside, queries inside.
+  struct Steps {
+    int g, b, k0, sharers;       // kv head, sequence, first key; blocks of the grid that share this key block
+    int h0, qs0, h, qs, n_it;    // first query head, first 128-row step; head and query step of the first step; steps
+  };
+  auto steps_of = [&](const Block& w) {
+    int kb = w.x, mine = 0, sharers = 1;
+    if constexpr (SHARED) {
+      int left = w.x;
+      for (kb = 0;; ++kb) {
+        sharers = dkv_block_ctas(p, dkv_block_steps(p, kb));
+        if (left < sharers) break;
+        left -= sharers;
+      }
+      mine = left;
+    }
+    Steps t;
+    t.g = w.y; t.b = w.z; t.k0 = kb * 128; t.sharers = sharers;
+    int q_first = 0;                                          // first query row that can see this key block
+    if (p.causal) q_first = max(0, p.k_pos0 + t.k0 - p.q_pos0);
+    t.qs0 = q_first / 128;
+    const int per_head = max(0, n_qs - t.qs0), n_steps = per_head * p.qpg;
+    const int it0 = SHARED ? n_steps * mine / sharers : 0;
+    t.n_it = SHARED ? n_steps * (mine + 1) / sharers - it0 : n_steps;
+    t.h0 = t.g * p.qpg;
+    t.h = t.h0 + (SHARED && per_head > 0 ? it0 / per_head : 0);
+    t.qs = t.qs0 + (SHARED && per_head > 0 ? it0 % per_head : 0);
+    return t;
+  };
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmDO);
@@ -1286,6 +1302,10 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     mbar_init(ds_full, kSoftmaxWarps);
     mbar_init(x_free, kSoftmaxWarps);
     mbar_init(acc_full, 1);
+    mbar_init(kv_empty, 1);
+    mbar_init(acc_empty, kSoftmaxWarps);
+    mbar_init(work.full, 1);
+    mbar_init(work.empty, 2 + kSoftmaxWarps);
     mbar_init(&stats_full[0], kSoftmaxWarps);
     mbar_init(&stats_full[1], kSoftmaxWarps);
     *abort_flag = 0;
@@ -1301,44 +1321,66 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   const uint32_t tmem = *tmem_slot;
   const uint32_t tST = tmem, tDPT = tmem + 128, tDV = tmem + 256, tDK = tmem + 384;
 
-  const int h0 = g * p.qpg;  // first query head of the group
-  const int h_it0 = h0 + (SHARED && steps_per_head > 0 ? it0 / steps_per_head : 0);   // head and query step of step it0
-  const int qs_it0 = qs0 + (SHARED && steps_per_head > 0 ? it0 % steps_per_head : 0);
-  const int kslot = p.kmap.slot(h0, p.qpg), vslot = p.vmap.slot(h0, p.qpg);
+  Block blk{int(blockIdx.x), int(blockIdx.y), int(blockIdx.z)};
 
   if (warp == 0) {
-    if (n_it > 0) {
-      // the whole warp walks the loop, one elected lane issues the copies (see producer_loop in gemm_core.cuh)
-      const bool issuer = elect_one() != 0;
-      if (issuer) mbar_expect_tx(kv_full, 2 * L::kKV);
+    // the whole warp walks the loop, one elected lane issues the copies (see producer_loop in gemm_core.cuh)
+    const bool issuer = elect_one() != 0;
+    int qs_slot = 0, ds_slot = 0, nkv = 0, n = 0;    // ring positions, K / V tiles loaded so far, blocks done
+    uint32_t qph = 0, dph = 0;
+    bool ok = true, asked = false;
+    for (; ok; ++n) {
+      asked = false;
+      auto ask = [&]() {                             // for the next block, once every warp has taken this one
+        if (!kTakesMore || asked || (n > 0 && !mbar_test_warp(work.empty, (n - 1) & 1))) return;
+        if (issuer) work_request(work);
+        __syncwarp();
+        asked = true;
+      };
+      const Steps t = steps_of(blk);
+      const int kslot = p.kmap.slot(t.h0, p.qpg), vslot = p.vmap.slot(t.h0, p.qpg), b = t.b;
+      ask();
+      if (t.n_it > 0) {
+        if (!mbar_wait_warp(kv_empty, (nkv & 1) ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
+        ++nkv;
+        if (issuer) mbar_expect_tx(kv_full, 2 * L::kKV);
 #pragma unroll
-      for (int c = 0; c < HD / 64; ++c) {
-        if (issuer) tma_load_4d(sK + c * 128 * 128, &tmK, kv_full, c * 64, kslot, k0, b);
-        if (issuer) tma_load_4d(sV + c * 128 * 128, &tmV, kv_full, c * 64, vslot, k0, b);
+        for (int c = 0; c < HD / 64; ++c) {
+          if (issuer) tma_load_4d(sK + c * 128 * 128, &tmK, kv_full, c * 64, kslot, t.k0, b);
+          if (issuer) tma_load_4d(sV + c * 128 * 128, &tmV, kv_full, c * 64, vslot, t.k0, b);
+        }
+        int h = t.h, qs = t.qs;
+        for (int it = 0; it < t.n_it; ++it) {
+          const int qrow = qs * 128;
+          const int qslot = p.qmap.slot(h, p.qpg), doslot = p.domap.slot(h, p.qpg);
+          if (!mbar_wait_warp(&q_empty[qs_slot], qph ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
+          if (issuer) mbar_expect_tx(&q_full[qs_slot], L::kQD);
+#pragma unroll
+          for (int c = 0; c < HD / 64; ++c)
+            if (issuer) tma_load_4d(sQ + qs_slot * L::kQD + c * 128 * 128, &tmQ, &q_full[qs_slot], c * 64, qslot, qrow, b);
+          if (!mbar_wait_warp(&do_empty[ds_slot], dph ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
+          if (issuer) mbar_expect_tx(&do_full[ds_slot], L::kQD);
+#pragma unroll
+          for (int c = 0; c < HD / 64; ++c)
+            if (issuer) tma_load_4d(sDO + ds_slot * L::kQD + c * 128 * 128, &tmDO, &do_full[ds_slot], c * 64, doslot, qrow, b);
+          if (++qs_slot == NQ) { qs_slot = 0; qph ^= 1; }
+          if (++ds_slot == ND) { ds_slot = 0; dph ^= 1; }
+          if (++qs == n_qs) { qs = t.qs0; ++h; }
+          ask();
+        }
       }
-      int qs_slot = 0, ds_slot = 0;
-      uint32_t qph = 0, dph = 0;
-      int h = h_it0, qs = qs_it0;
-      for (int it = 0; it < n_it; ++it) {
-        const int qrow = qs * 128;
-        const int qslot = p.qmap.slot(h, p.qpg), doslot = p.domap.slot(h, p.qpg);
-        if (!mbar_wait_warp(&q_empty[qs_slot], qph ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { *abort_flag = 1; break; }
-        if (issuer) mbar_expect_tx(&q_full[qs_slot], L::kQD);
-#pragma unroll
-        for (int c = 0; c < HD / 64; ++c)
-          if (issuer) tma_load_4d(sQ + qs_slot * L::kQD + c * 128 * 128, &tmQ, &q_full[qs_slot], c * 64, qslot, qrow, b);
-        if (!mbar_wait_warp(&do_empty[ds_slot], dph ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { *abort_flag = 1; break; }
-        if (issuer) mbar_expect_tx(&do_full[ds_slot], L::kQD);
-#pragma unroll
-        for (int c = 0; c < HD / 64; ++c)
-          if (issuer) tma_load_4d(sDO + ds_slot * L::kQD + c * 128 * 128, &tmDO, &do_full[ds_slot], c * 64, doslot, qrow, b);
-        if (++qs_slot == NQ) { qs_slot = 0; qph ^= 1; }
-        if (++ds_slot == ND) { ds_slot = 0; dph ^= 1; }
-        if (++qs == n_qs) { qs = qs0; ++h; }
+      if (!ok || !kTakesMore) break;
+      if (!asked) {
+        if (!mbar_wait_warp(work.empty, (n - 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+        ask();
       }
+      if (!work_take(work, n, blk, p.status, abort_flag)) break;
+    }
+    if (!ok) {
+      *abort_flag = 1;
+      if (asked) work_drain(work, n);
     }
   } else if (warp == 1) {
-    if (n_it > 0) {
       // the whole warp walks the loop, one elected lane issues (see mma_loop in gemm_core.cuh)
       const bool issuer = elect_one() != 0;
       constexpr uint32_t idesc_st = make_idesc_lp(128, 128, false, false);
@@ -1378,12 +1420,20 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         if (++d_p == ND) { d_p = 0; dph_p ^= 1; }
         return true;
       };
-      bool ok = mbar_wait_warp(kv_full, 0, p.status, kTimeoutSmemFull, abort_flag);
+      bool ok = true;
+      int nkv = 0;                        // blocks with steps so far
+      uint32_t ph = 1;                    // of a step's barriers
+      for (int n = 0; ok; ++n) {
+      const int n_it = steps_of(blk).n_it;
+      if (n_it > 0) {
+      ok = mbar_wait_warp(kv_full, nkv & 1, p.status, kTimeoutSmemFull, abort_flag);
       if (ok) ok = issue_st();
       if (ok) ok = issue_dpt();
+      if (ok && n_it == 1 && issuer) umma_commit(kv_empty);
+      __syncwarp();
       HG_DKV_TIMERS(tm_wait_x, tm_wait_p, tm_wait_ds, tm_issue);
       for (int it = 0; ok && it < n_it; ++it) {
-        const uint32_t ph = it & 1;
+        ph ^= 1;
         HG_DKV_TICK(t0);
         // ---- S^T(it+1), as soon as the S^T(it) values are in the threads' registers
         if (!mbar_wait_warp(x_free, ph, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
@@ -1391,7 +1441,8 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         HG_DKV_TOCK(tm_wait_x, t0);
         if (it + 1 < n_it) { ok = issue_st(); if (!ok) break; }
         HG_DKV_TOCK(tm_issue, t0);
-        // ---- dV(it)
+        // ---- dV(it); dV and dK still hold the last block's sums until its epilogue has read them
+        if (it == 0 && !mbar_wait_warp(acc_empty, (nkv & 1) ^ 1, p.status, kTimeoutTmemEmpty, abort_flag)) { ok = false; break; }
         if (!mbar_wait_warp(p_full, ph, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
         tc_fence_after();
         HG_DKV_TOCK(tm_wait_p, t0);
@@ -1418,14 +1469,22 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         }
         __syncwarp();
         if (++q_k == NQ) q_k = 0;
-        if (it + 1 < n_it) { ok = issue_dpt(); if (!ok) break; }
+        if (it + 1 < n_it) {
+          ok = issue_dpt();
+          if (!ok) break;
+          if (it + 2 == n_it && issuer) umma_commit(kv_empty);     // the last of the block's products that read K and V
+          __syncwarp();
+        }
         HG_DKV_TOCK(tm_issue, t0);
       }
       HG_DKV_REPORT(8, n_it, tm_wait_x, tm_wait_p, tm_wait_ds, tm_issue);
       if (ok && issuer) umma_commit(acc_full);
       __syncwarp();
+      ++nkv;
+      }
+      if (!kTakesMore || (ok && !work_take(work, n, blk, p.status, abort_flag))) break;
+      }
       if (!ok) *abort_flag = 1;
-    }
   } else {
     const int wq = warp & 3;
     const int half = (warp - 2) >> 2;     // warpgroup: which CPT of the step's 128 query columns these threads own
@@ -1434,12 +1493,17 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     const int tid = threadIdx.x - 64;     // 0..128*NWG-1 among the softmax threads; the first 256 carry the statistics
     const uint32_t lane_off = uint32_t(wq * 32) << 16;
     const float sl2 = p.scale * kLog2e;
+    bool ok = true;
+    int nkv = 0;                          // blocks with steps so far
+    uint32_t done = 0;                    // steps so far
+    for (int n = 0; ok; ++n) {
+    const Steps t = steps_of(blk);
+    const int k0 = t.k0, b = t.b, g = t.g, n_it = t.n_it, h0 = t.h0, qs0 = t.qs0, sharers = t.sharers;
     const int k_pos = p.k_pos0 + k0 + row;
     const bool k_valid = (k0 + row) < p.Skv;
-    bool ok = true;
     // Per-query statistics of a step, fetched one step ahead: thread t < 128 carries -lse * log2 e of query t of the
     // step, thread 128 + t carries D of query t.
-    int ld_h = h_it0, ld_qs = qs_it0, ld_it = 0;
+    int ld_h = t.h, ld_qs = t.qs, ld_it = 0;
     auto load_stat = [&]() -> float {
       float v = 0.f;
       if (tid < 256 && ld_it < n_it) {
@@ -1458,15 +1522,14 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     const float stat_scale = (tid < 128) ? -kLog2e : 1.f;
     float stat_next = load_stat();
     if (n_it > 0) {
-      if (tid < 256) sStats[tid] = stat_next * stat_scale;
-      mbar_arrive_warp(&stats_full[0]);
+      if (tid < 256) sStats[(done & 1) * 256 + tid] = stat_next * stat_scale;
+      mbar_arrive_warp(&stats_full[done & 1]);
       stat_next = load_stat();
     }
-    int cur_qs = qs_it0;
+    int cur_qs = t.qs;
     HG_DKV_TIMERS(tm_wait_a, tm_a, tm_wait_b, tm_b);
-    for (int it = 0; it < n_it; ++it) {
-      const int sb = it & 1;
-      const uint32_t ph = it & 1;
+    for (int it = 0; it < n_it; ++it, ++done) {
+      const uint32_t sb = done & 1, ph = done & 1;
       HG_DKV_TICK(t0);
       const int qrow = cur_qs * 128;
       if (++cur_qs == n_qs) cur_qs = qs0;
@@ -1474,7 +1537,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       uint32_t pp[CPT / 2];               // this thread's probabilities, packed, kept for the second phase
       float pf[kExactP ? CPT : 1];        // and in fp32, where dS^T is formed from those
       // ---------------- S^T -> probabilities (kept in registers; the S^T columns are released at once)
-      if (!mbar_wait_warp(&stats_full[sb], (it >> 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&stats_full[sb], (done >> 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
       if (!mbar_wait_warp(st_full, ph, p.status, kTimeoutTmemFull, abort_flag)) { ok = false; break; }
       tc_fence_after();
       HG_DKV_TOCK(tm_wait_a, t0);
@@ -1585,7 +1648,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           reinterpret_cast<uint4*>(dv)[i] = make_uint4(0, 0, 0, 0);
         }
       }
-    } else if (ok && !*abort_flag && mbar_wait_warp(acc_full, 0, p.status, kTimeoutOther, abort_flag)) {
+    } else if (ok && !*abort_flag && mbar_wait_warp(acc_full, nkv & 1, p.status, kTimeoutOther, abort_flag)) {
       tc_fence_after();
 #pragma unroll
       for (int c = half; c < HD / 32; c += NWG) {   // the warpgroups take alternate 32-column chunks
@@ -1594,7 +1657,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         tmem_ld32(tDK + lane_off + c * 32, r1);
         tmem_ld_wait();
         if (SHARED && sharers > 1) {                // summed, scaled and rounded by dkv_sum_kernel
-          float* part = p.part + ((size_t(b) * gridDim.y + g) * gridDim.x + blockIdx.x) * (2 * 128 * HD) + row * HD + c * 32;
+          float* part = p.part + ((size_t(b) * gridDim.y + g) * gridDim.x + blk.x) * (2 * 128 * HD) + row * HD + c * 32;
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             reinterpret_cast<uint4*>(part)[q] = make_uint4(r0[q * 4], r0[q * 4 + 1], r0[q * 4 + 2], r0[q * 4 + 3]);
@@ -1617,9 +1680,15 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           }
         }
       }
+      tc_fence_before();
+      mbar_arrive_warp(acc_empty);
+      ++nkv;
     } else {
-      *abort_flag = 1;
+      ok = false;
     }
+    if (!kTakesMore || (ok && !work_take(work, n, blk, p.status, abort_flag))) break;
+    }
+    if (!ok) *abort_flag = 1;
   }
   tc_fence_before();
   __syncthreads();
@@ -1687,6 +1756,8 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1)
 flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                        const BwdParams p) {
+  // As in the dK/dV kernel: 8 x 1024 tokens, 25 heads of 64 106 -> 91 us; 2 x 4096, 32 heads of 128 399 -> 403.
+  constexpr bool kTakesMore = HD == 64;
   extern __shared__ uint8_t smem_raw[];
   using L = Dq128Smem<HD>;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1706,18 +1777,21 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   uint64_t* v_empty = bars + 8;    // 1
   uint64_t* s_full = bars + 9;     // 1
   uint64_t* s_empty = bars + 10;   // 1
-  uint64_t* ds_full = bars + 11;   // 2, by step parity: a warp may store the next step's dS before another has stored this one's
-  uint64_t* ds_empty = bars + 13;  // 2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  uint64_t* ds_full = bars + 22;   // 2, by step parity: a warp may store the next step's dS before another has stored this one's
+  uint64_t* ds_empty = bars + 12;  // 2
+  uint64_t* qdo_empty = bars + 14; // 1: the last products that read Q and dO have completed
+  uint64_t* acc_empty = bars + 15; // 1: the epilogue has read dQ
+  const WorkSlot work{reinterpret_cast<uint4*>(bars + 18), bars + 16, bars + 17};
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 20);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5;
-  const int qb = gridDim.x - 1 - blockIdx.x;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int q0 = qb * 128;
-  int kv_len = p.Skv;
-  if (p.causal) kv_len = min(p.Skv, p.q_pos0 + q0 + 127 - p.k_pos0 + 1);
-  const int n_it = kv_len > 0 ? (kv_len + 127) / 128 : 0;
+  auto query_row = [&](const Block& w) { return (int(gridDim.x) - 1 - w.x) * 128; };
+  auto steps_of = [&](const Block& w) {
+    int kv_len = p.Skv;
+    if (p.causal) kv_len = min(p.Skv, p.q_pos0 + query_row(w) + 127 - p.k_pos0 + 1);
+    return kv_len > 0 ? (kv_len + 127) / 128 : 0;
+  };
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmDO);
@@ -1734,6 +1808,10 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     mbar_init(&ds_full[1], kSoftmaxWarps);
     mbar_init(&ds_empty[0], 1);
     mbar_init(&ds_empty[1], 1);
+    mbar_init(qdo_empty, 1);
+    mbar_init(acc_empty, kSoftmaxWarps);
+    mbar_init(work.full, 1);
+    mbar_init(work.empty, 2 + kSoftmaxWarps);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -1748,49 +1826,77 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const uint32_t tS = tmem, tDP = tmem + 128, tDQ = tmem + 256;
   const uint32_t tDS[2] = {tmem + 384, tmem + 448};   // packed dS, step parity
 
-  const int qslot = p.qmap.slot(h, p.qpg), kslot = p.kmap.slot(h, p.qpg), vslot = p.vmap.slot(h, p.qpg),
-            doslot = p.domap.slot(h, p.qpg);
+  Block blk{int(blockIdx.x), int(blockIdx.y), int(blockIdx.z)};
 
   if (warp == 0) {
-    if (n_it > 0) {
-      // the whole warp walks the loop, one elected lane issues the copies (see producer_loop in gemm_core.cuh)
-      const bool issuer = elect_one() != 0;
-      if (issuer) mbar_expect_tx(qdo_full, 2 * L::kQ);
+    // the whole warp walks the loop, one elected lane issues the copies (see producer_loop in gemm_core.cuh)
+    const bool issuer = elect_one() != 0;
+    int ks = 0, nq = 0, n = 0;                       // K ring position, Q tiles loaded so far, blocks done
+    uint32_t kph = 0, vph = 0;
+    bool ok = true, asked = false;
+    for (; ok; ++n) {
+      asked = false;
+      auto ask = [&]() {                             // for the next block, once every warp has taken this one
+        if (!kTakesMore || asked || (n > 0 && !mbar_test_warp(work.empty, (n - 1) & 1))) return;
+        if (issuer) work_request(work);
+        __syncwarp();
+        asked = true;
+      };
+      const int q0 = query_row(blk), h = blk.y, b = blk.z, n_it = steps_of(blk);
+      const int qslot = p.qmap.slot(h, p.qpg), kslot = p.kmap.slot(h, p.qpg), vslot = p.vmap.slot(h, p.qpg),
+                doslot = p.domap.slot(h, p.qpg);
+      ask();
+      if (n_it > 0) {
+        if (!mbar_wait_warp(qdo_empty, (nq & 1) ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
+        ++nq;
+        if (issuer) mbar_expect_tx(qdo_full, 2 * L::kQ);
 #pragma unroll
-      for (int c = 0; c < HD / 64; ++c) {
-        if (issuer) tma_load_4d(sQ + c * 128 * 128, &tmQ, qdo_full, c * 64, qslot, q0, b);
-        if (issuer) tma_load_4d(sDO + c * 128 * 128, &tmDO, qdo_full, c * 64, doslot, q0, b);
+        for (int c = 0; c < HD / 64; ++c) {
+          if (issuer) tma_load_4d(sQ + c * 128 * 128, &tmQ, qdo_full, c * 64, qslot, q0, b);
+          if (issuer) tma_load_4d(sDO + c * 128 * 128, &tmDO, qdo_full, c * 64, doslot, q0, b);
+        }
+        for (int it = 0; it < n_it; ++it) {
+          if (!mbar_wait_warp(&k_empty[ks], kph ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
+          if (issuer) mbar_expect_tx(&k_full[ks], L::kKV);
+#pragma unroll
+          for (int c = 0; c < HD / 64; ++c)
+            if (issuer) tma_load_4d(sK + ks * L::kKV + c * 128 * 128, &tmK, &k_full[ks], c * 64, kslot, it * 128, b);
+          if (!mbar_wait_warp(v_empty, vph ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
+          if (issuer) mbar_expect_tx(v_full, L::kKV);
+#pragma unroll
+          for (int c = 0; c < HD / 64; ++c)
+            if (issuer) tma_load_4d(sV + c * 128 * 128, &tmV, v_full, c * 64, vslot, it * 128, b);
+          if (++ks == NK) { ks = 0; kph ^= 1; }
+          vph ^= 1;
+          ask();
+        }
       }
-      int ks = 0;
-      uint32_t kph = 0;
-      for (int it = 0; it < n_it; ++it) {
-        if (!mbar_wait_warp(&k_empty[ks], kph ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { *abort_flag = 1; break; }
-        if (issuer) mbar_expect_tx(&k_full[ks], L::kKV);
-#pragma unroll
-        for (int c = 0; c < HD / 64; ++c)
-          if (issuer) tma_load_4d(sK + ks * L::kKV + c * 128 * 128, &tmK, &k_full[ks], c * 64, kslot, it * 128, b);
-        if (!mbar_wait_warp(v_empty, (it & 1) ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { *abort_flag = 1; break; }
-        if (issuer) mbar_expect_tx(v_full, L::kKV);
-#pragma unroll
-        for (int c = 0; c < HD / 64; ++c)
-          if (issuer) tma_load_4d(sV + c * 128 * 128, &tmV, v_full, c * 64, vslot, it * 128, b);
-        if (++ks == NK) { ks = 0; kph ^= 1; }
+      if (!ok || !kTakesMore) break;
+      if (!asked) {
+        if (!mbar_wait_warp(work.empty, (n - 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+        ask();
       }
+      if (!work_take(work, n, blk, p.status, abort_flag)) break;
+    }
+    if (!ok) {
+      *abort_flag = 1;
+      if (asked) work_drain(work, n);
     }
   } else if (warp == 1) {
-    if (n_it > 0) {
       // the whole warp walks the loop, one elected lane issues (see mma_loop in gemm_core.cuh)
       const bool issuer = elect_one() != 0;
       constexpr uint32_t idesc_s = make_idesc_lp(128, 128, false, false);
       constexpr uint32_t idesc_dq = make_idesc_lp(128, HD, false, true);
       const uint32_t aQ = smem_u32(sQ), aDO = smem_u32(sDO);
-      bool ok = mbar_wait_warp(qdo_full, 0, p.status, kTimeoutSmemFull, abort_flag);
+      bool ok = true;
+      uint32_t step_s = 0, step_d = 0;   // S / dP and dQ products issued so far
+      int nq = 0;                        // blocks with steps so far
       int ks_s = 0, ks_d = 0;          // K slot of the next S issue and of the next dQ issue
       uint32_t kph_s = 0;
       const uint32_t aV = smem_u32(sV);
-      auto issue_s = [&](int it) -> bool {
+      auto issue_s = [&](bool last) -> bool {
         if (!mbar_wait_warp(&k_full[ks_s], kph_s, p.status, kTimeoutSmemFull, abort_flag)) return false;
-        if (!mbar_wait_warp(s_empty, (it & 1) ^ 1, p.status, kTimeoutTmemEmpty, abort_flag)) return false;
+        if (!mbar_wait_warp(s_empty, (step_s & 1) ^ 1, p.status, kTimeoutTmemEmpty, abort_flag)) return false;
         tc_fence_after();
         const uint32_t aK = smem_u32(sK + ks_s * L::kKV);
         if (issuer) {
@@ -1799,7 +1905,7 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             umma_f16_ss(tS, kmajor_desc(aQ, 128, kk), kmajor_desc(aK, 128, kk), idesc_s, kk != 0);
         }
         __syncwarp();
-        if (!mbar_wait_warp(v_full, it & 1, p.status, kTimeoutSmemFull, abort_flag)) return false;
+        if (!mbar_wait_warp(v_full, step_s & 1, p.status, kTimeoutSmemFull, abort_flag)) return false;
         tc_fence_after();
         if (issuer) {
 #pragma unroll
@@ -1807,35 +1913,47 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             umma_f16_ss(tDP, kmajor_desc(aDO, 128, kk), kmajor_desc(aV, 128, kk), idesc_s, kk != 0);
           umma_commit(v_empty);
           umma_commit(s_full);
+          if (last) umma_commit(qdo_empty);
         }
         __syncwarp();
+        ++step_s;
         if (++ks_s == NK) { ks_s = 0; kph_s ^= 1; }
         return true;
       };
-      if (ok) ok = issue_s(0);
+      for (int n = 0; ok; ++n) {
+      const int n_it = steps_of(blk);
+      if (n_it > 0) {
+      ok = mbar_wait_warp(qdo_full, nq & 1, p.status, kTimeoutSmemFull, abort_flag);
+      if (ok) ok = issue_s(n_it == 1);
       HG_DKV_TIMERS(tm_s, tm_wait_ds, tm_dq, tm_unused);
       for (int it = 0; ok && it < n_it; ++it) {
         HG_DKV_TICK(t0);
-        if (it + 1 < n_it) { ok = issue_s(it + 1); if (!ok) break; }
+        if (it + 1 < n_it) { ok = issue_s(it + 2 == n_it); if (!ok) break; }
         HG_DKV_TOCK(tm_s, t0);
-        if (!mbar_wait_warp(&ds_full[it & 1], (it >> 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+        // dQ still holds the last block's sums until its epilogue has read them
+        if (it == 0 && !mbar_wait_warp(acc_empty, (nq & 1) ^ 1, p.status, kTimeoutTmemEmpty, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&ds_full[step_d & 1], (step_d >> 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
         tc_fence_after();
         HG_DKV_TOCK(tm_wait_ds, t0);
         const uint32_t aK = smem_u32(sK + ks_d * L::kKV);
         if (issuer) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk)   // k-step kk = keys 16kk..16kk+15 = 8 packed columns
-            umma_f16_ts(tDQ, tDS[it & 1] + kk * 8, mnmajor_desc(aK, 128, kk), idesc_dq, (it | kk) != 0);
+            umma_f16_ts(tDQ, tDS[step_d & 1] + kk * 8, mnmajor_desc(aK, 128, kk), idesc_dq, (it | kk) != 0);
           umma_commit(&k_empty[ks_d]);
-          umma_commit(&ds_empty[it & 1]);
+          umma_commit(&ds_empty[step_d & 1]);
         }
         __syncwarp();
+        ++step_d;
         if (++ks_d == NK) ks_d = 0;
         HG_DKV_TOCK(tm_dq, t0);
       }
       HG_DKV_REPORT(32, n_it, tm_s, tm_wait_ds, tm_dq, tm_unused);
+      ++nq;
+      }
+      if (!kTakesMore || (ok && !work_take(work, n, blk, p.status, abort_flag))) break;
+      }
       if (!ok) *abort_flag = 1;
-    }
   } else {
     const int wq = warp & 3;
     const int half = (warp - 2) >> 2;     // warpgroup: which CPT of the step's 128 key columns these threads own
@@ -1843,6 +1961,10 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const int row = wq * 32 + lane_id();
     const uint32_t lane_off = uint32_t(wq * 32) << 16;
     const float sl2 = p.scale * kLog2e;
+    bool ok = true;
+    uint32_t done = 0;                    // steps so far
+    for (int n = 0; ok; ++n) {
+    const int q0 = query_row(blk), h = blk.y, b = blk.z, n_it = steps_of(blk);
     const int srow = q0 + row;
     const int q_pos = p.q_pos0 + srow;
     float lse2 = INFINITY, dsum = 0.f;
@@ -1852,11 +1974,10 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       dsum = p.D[idx];
     }
     const float nlse2 = -lse2;
-    bool ok = true;
     HG_DKV_TIMERS(tm_wait_s, tm_ld, tm_math, tm_st);
-    for (int it = 0; it < n_it; ++it) {
+    for (int it = 0; it < n_it; ++it, ++done) {
       HG_DKV_TICK(t0);
-      if (!mbar_wait_warp(s_full, it & 1, p.status, kTimeoutTmemFull, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(s_full, done & 1, p.status, kTimeoutTmemFull, abort_flag)) { ok = false; break; }
       tc_fence_after();
       HG_DKV_TOCK(tm_wait_s, t0);
       float ds[CPT];
@@ -1888,20 +2009,20 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
       }
       HG_DKV_TOCK(tm_math, t0);
-      if (it >= 2) {   // this dS buffer was last read by the dQ product of step it-2
-        if (!mbar_wait_warp(&ds_empty[it & 1], ((it >> 1) & 1) ^ 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+      if (done >= 2) {   // this dS buffer was last read by the dQ product of step it-2
+        if (!mbar_wait_warp(&ds_empty[done & 1], ((done >> 1) & 1) ^ 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
         tc_fence_after();
       }
       {
         uint32_t w[CPT / 2];
 #pragma unroll
         for (int i = 0; i < CPT / 2; ++i) w[i] = pack_bf16(ds[2 * i], ds[2 * i + 1]);
-        if constexpr (CPT == 64) tmem_st32(tDS[it & 1] + lane_off + half * (CPT / 2), w);
-        else tmem_st16(tDS[it & 1] + lane_off + half * (CPT / 2), w);
+        if constexpr (CPT == 64) tmem_st32(tDS[done & 1] + lane_off + half * (CPT / 2), w);
+        else tmem_st16(tDS[done & 1] + lane_off + half * (CPT / 2), w);
       }
       tmem_st_wait();
       tc_fence_before();
-      mbar_arrive_warp(&ds_full[it & 1]);
+      mbar_arrive_warp(&ds_full[done & 1]);
       HG_DKV_TOCK(tm_st, t0);
     }
     HG_DKV_REPORT(24, n_it, tm_wait_s, tm_ld, tm_math, tm_st);
@@ -1913,7 +2034,7 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         for (int i = half; i < HD / 8; i += NWG) reinterpret_cast<uint4*>(dq)[i] = make_uint4(0, 0, 0, 0);
       }
     } else if (ok && !*abort_flag &&
-               mbar_wait_warp(&ds_empty[(n_it - 1) & 1], ((n_it - 1) >> 1) & 1, p.status, kTimeoutOther, abort_flag)) {
+               mbar_wait_warp(&ds_empty[(done - 1) & 1], ((done - 1) >> 1) & 1, p.status, kTimeoutOther, abort_flag)) {
       tc_fence_after();
 #pragma unroll
       for (int c = half; c < HD / 32; c += NWG) {
@@ -1932,9 +2053,14 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           }
         }
       }
+      tc_fence_before();
+      mbar_arrive_warp(acc_empty);
     } else {
-      *abort_flag = 1;
+      ok = false;
     }
+    if (!kTakesMore || (ok && !work_take(work, n, blk, p.status, abort_flag))) break;
+    }
+    if (!ok) *abort_flag = 1;
   }
   tc_fence_before();
   __syncthreads();

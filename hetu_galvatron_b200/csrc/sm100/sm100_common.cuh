@@ -155,6 +155,21 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   return false;
 }
 
+// Whether the phase is over, without waiting; the same answer for the whole warp.
+__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.b32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return __all_sync(0xffffffffu, ok != 0);
+}
+
 // Warp-collective bounded wait: every lane waits, the verdict is made uniform so that the warp never
 // diverges around the .sync.aligned tcgen05 instructions that follow.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, int code,
@@ -342,6 +357,58 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------
+// Persistent CTAs over an ordinary grid: a running CTA asks the launcher for the block that would start next (cluster launch
+// control), which then never starts, and works on it itself.  Blocks keep their order and go to whoever is free, as without
+// it, but a CTA's set-up is paid once and the loads of its next block overlap the end of this one.  One warp requests
+// (work_request), every role's warps take the answer (work_take): `full` counts 1, `empty` the warps that take.
+// ---------------------------------------------------------------------------
+struct WorkSlot {
+  uint4* answer;                  // 16-byte aligned shared memory
+  uint64_t *full, *empty;
+};
+struct Block {
+  int x, y, z;
+};
+// One thread.  Answer k (k = 0, 1, ...) completes phase k of `full`; the next may be asked for once phase k of `empty` is over.
+__device__ __forceinline__ void work_request(const WorkSlot& s) {
+  mbar_expect_tx(s.full, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(s.answer)),
+               "r"(smem_u32(s.full))
+               : "memory");
+}
+// Whole warp: waits for answer k; false when no block is left (or the wait gave up).
+__device__ __forceinline__ bool work_take(const WorkSlot& s, int k, Block& b, int* status, volatile int* abort) {
+  if (!mbar_wait_warp(s.full, k & 1, status, kTimeoutOther, abort)) return false;
+  uint32_t x, y, z, got;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      ".reg .b128 a;\n"
+      "ld.shared.b128 a, [%4];\n"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n"
+      "selp.u32 %3, 1, 0, p;\n"
+      "mov.u32 %0, 0;\n"
+      "mov.u32 %1, 0;\n"
+      "mov.u32 %2, 0;\n"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%0, %1, %2, _}, a;\n"
+      "}\n"
+      : "=&r"(x), "=&r"(y), "=&r"(z), "=&r"(got)
+      : "r"(smem_u32(s.answer))
+      : "memory");
+  fence_proxy_async_smem();       // the answer is read before the next one overwrites it
+  mbar_arrive_warp(s.empty);
+  b = Block{int(x), int(y), int(z)};
+  return got != 0;
+}
+
+// For a warp that gives up with answer k under way: lets it land (bounded) before shared memory is released.
+__device__ __forceinline__ void work_drain(const WorkSlot& s, int k) {
+  for (uint32_t spin = 0; spin < (1u << 16); ++spin)
+    if (mbar_try_wait(s.full, k & 1)) break;
+}
 
 // ---------------------------------------------------------------------------
 // Programmatic dependent launch (hg_host::Chain below).  A kernel that may be launched in a chain calls chain_release() once
