@@ -4,7 +4,9 @@
 // They do what the Python classes of ops/gemm.py, ops/fused.py, ops/attention.py, models/modules.py and parallel/zero.py do,
 // with the same kernels, saved tensors, gradients and errors.  What they save is the host: a short kernel takes the GPU a few
 // microseconds, and a Python autograd function took the host 30 us for a forward and a backward that do nothing and 75 us
-// for those of a linear layer, so that a two-layer step of hidden 512 (84 launches) took 2.45 ms of which the GPU worked 0.6.
+// for those of a linear layer, so that a two-layer step of hidden 512 (84 launches) took 2.5 ms of which the GPU worked 0.6;
+// from here 1.75 ms, an attention block of 1531 x 3584 483 us instead of 598, and a decode step of four 4096-wide layers 516
+// instead of 587, both now bound by the device.
 //
 // Every function here returns None when a call is not one of the plain ones (see `plain`), and the caller then takes the
 // Python class, which raises what there is to raise.  The kernels' addresses come from the library that ops/_lib.py has
