@@ -2215,6 +2215,8 @@ int hg_flash_fwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTenso
                  float scale, void* stream) {
   if (hd != 64 && hd != 128) return -1;
   if (Sq <= 0 || Skv <= 0 || B <= 0) return 0;
+  if (g_fwd_variant == 0 && hg_flash_stream_takes(q, k, v, Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0))
+    return hg_flash_stream(q, k, v, o, lse, Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0, scale, 0, stream);
   CUtensorMap tq, tk, tv;
   int rc;
   if ((rc = make_map(&tq, q->ptr, hd, q->slots, Sq, B, q->ss, q->sb, 128))) return rc;

@@ -7,9 +7,10 @@
 // spread over several ranges (flash_decode.cu).  A decode step of a 7B-sized layer keeps the GPU busy for about 110 us;
 // launched through the tensor library and the autograd wrappers it takes the host several times that.  Four 4096-wide
 // layers, 4 sequences at 1000 cached positions, embedding and head included: 1400 us a step when each is waited for, 770 us
-// from here; one after another 590 us, of which 517 us are kernels (attention on the tile kernel, products on
-// gemm_skinny.cu).  The kernels are launched as a chain (sm100_common.cuh): each may start while the one before it ends, and the
-// products read their first weights meanwhile; the same step as a CUDA graph 519 us without and 477 with.  Host code only.
+// from here; one after another 590 us, of which 517 us were kernels.  They are launched as a chain (sm100_common.cuh): each
+// may start while the one before it ends, and the products read their first weights meanwhile; the same step as a CUDA graph
+// 519 us without and 477 with, 466 with the keys streamed (flash_decode.cu) and their first copies made before the wait, 498
+// one after another.  Host code only.
 #include "decoder_step.h"
 #include "entry_points.h"
 #include "sm100_common.cuh"
@@ -94,6 +95,8 @@ int hg_decoder_step(HgDecoderStep* dp, void* stream) {
                      v{d.v_cache, d.v_ss, d.v_sb, d.ng, 1, 0, 0}, o{b.ctx, (long long)d.B * C, C, d.nh, qpg, 1, 0};
   if (b.part_floats >= 0)
     rc = hg_flash_decode(&q, &k, &v, &o, b.lse, b.part, d.S, d.past + d.S, d.B, d.nh, d.ng, d.hd, 1, d.past, 0, d.scale, stream);
+  else if (hg_flash_stream_takes(&q, &k, &v, d.S, d.past + d.S, d.B, d.nh, d.ng, d.hd, 1, d.past, 0))
+    rc = hg_flash_stream(&q, &k, &v, &o, b.lse, d.S, d.past + d.S, d.B, d.nh, d.ng, d.hd, 1, d.past, 0, d.scale, d.past, stream);
   else
     rc = hg_flash_fwd(&q, &k, &v, &o, b.lse, d.S, d.past + d.S, d.B, d.nh, d.ng, d.hd, 1, d.past, 0, d.scale, stream);
   if (rc) return rc;

@@ -210,6 +210,222 @@ flash_decode_merge_kernel(const DecodeParams p, int ranges) {
   if (c == 0) p.LSE[(size_t(b) * p.nheads + h) * p.Sq + s] = l > 0.f ? (m + log2f(l)) * kLn2 : -INFINITY;
 }
 
+// ---------------------------------------------------------------------------------------------
+// One query per head and kv head: a CTA streams the keys of a head, or a run of them, and nothing of it is kept but the running
+// maximum, sum and context; the CTAs of a cluster share a head's keys and merge through distributed shared memory, so that
+// there is one launch and no scratch.
+//
+// What bounds it is reading K and V.  A thread copies (cp.async) the 16 bytes of either that it reads itself, kDepth steps
+// ahead, into slots of its own: no barrier inside the loop, 64 KB in flight per CTA, three CTAs per SM.  HD / 8 lanes share a
+// key; eight warps take 2048 / HD keys a step.  Scores of kBatch steps are formed before one rescale, since the chain of
+// shuffles and exponentials of a single key is longer than its bytes take.  In a chain the keys below `settled` are older than
+// the chain: the first copies of those are made before the wait.
+// ---------------------------------------------------------------------------------------------
+constexpr int kDepth = 8, kBatch = 4, kStreamThreads = 256, kMaxCluster = 8;
+
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool on) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(hg::smem_u32(dst)), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_rank(const float* mine, int rank) {
+  uint32_t a;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(hg::smem_u32(mine)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+// What a partial result with maximum m counts beside one with maximum top >= m.
+__device__ __forceinline__ float weight_of(float m, float top) { return ex2(m - (top == -INFINITY ? 0.f : top)); }
+
+template <int HD>
+struct StreamSmem {
+  static constexpr int kRow = HD + 2;                                 // context, maximum, sum
+  static constexpr int kRing = kDepth * 2 * kStreamThreads * 16;      // later the warps' results
+  static constexpr int kTotal = kRing + kRow * 4;
+  static_assert(8 * kRow * 4 <= kRing, "the warps' results reuse the ring");
+};
+
+template <int HD>
+__global__ void __launch_bounds__(kStreamThreads, 3)
+flash_stream_kernel(const DecodeParams p, int settled) {
+  using L = StreamSmem<HD>;
+  constexpr int LPK = HD / 8, KPW = 32 / LPK, KPS = 8 * KPW;
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint4* ring = reinterpret_cast<uint4*>(smem);                       // [kDepth][K, V][thread]
+  float* sums = reinterpret_cast<float*>(smem);                       // [warp][kRow]
+  float* part = reinterpret_cast<float*>(smem + L::kRing);            // [kRow]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int sub = lane / LPK, ch = (lane % LPK) * 8;
+  const int rank = blockIdx.x, splits = gridDim.x, g = blockIdx.y, b = blockIdx.z;
+  const int steps = (p.kv_len + KPS - 1) / KPS;
+  const int first = int((long long)steps * rank / splits), n = int((long long)steps * (rank + 1) / splits) - first;
+  const hg_lp_t* kb = p.K + int64_t(b) * p.k_sb + int64_t(g * p.k_gs + p.k_off) * HD + ch;
+  const hg_lp_t* vb = p.V + int64_t(b) * p.v_sb + int64_t(g * p.v_gs + p.v_off) * HD + ch;
+  hg::chain_release();
+  auto copy = [&](int it) {                                           // step `it` of this CTA, or an empty group
+    if (it < n) {
+      const int key = (first + it) * KPS + warp * KPW + sub;
+      const bool on = key < p.kv_len;                                 // otherwise zeros
+      const int64_t at = on ? key : 0;
+      uint4* slot = ring + (it % kDepth) * 2 * kStreamThreads + tid;
+      copy16(slot, kb + at * p.k_ss, on);
+      copy16(slot + kStreamThreads, vb + at * p.v_ss, on);
+    }
+    copies_commit();
+  };
+  int ahead = 0;
+  for (; ahead < kDepth && (first + ahead + 1) * KPS <= settled; ++ahead) copy(ahead);
+  hg::chain_wait();
+  for (; ahead < kDepth; ++ahead) copy(ahead);
+
+  float q[8], acc[8], m = -INFINITY, l = 0.f;
+  const float sl2 = p.scale * kLog2e;
+  unpack8(*reinterpret_cast<const uint4*>(p.Q + int64_t(b) * p.q_sb + int64_t(g * p.q_gs + p.q_off) * HD + ch), q);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+  for (int it = 0; it < n; it += kBatch) {
+    copies_wait<kDepth - kBatch>();
+    float s[kBatch];
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      const int key = (first + it + j) * KPS + warp * KPW + sub;
+      float f[8], d = 0.f;
+      unpack8(ring[((it + j) % kDepth) * 2 * kStreamThreads + tid], f);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) d = fmaf(q[i], f[i], d);
+#pragma unroll
+      for (int o = LPK / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+      s[j] = it + j < n && key < p.kv_len ? d * sl2 : -INFINITY;
+    }
+    float top = m;
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) top = fmaxf(top, s[j]);
+    const float f = weight_of(m, top);
+    m = top;
+    l *= f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] *= f;
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) {
+      if (it + j >= n) break;                                         // slots that were never filled
+      const float e = weight_of(s[j], top);
+      l += e;
+      float v[8];
+      unpack8(ring[(((it + j) % kDepth) * 2 + 1) * kStreamThreads + tid], v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] = fmaf(e, v[i], acc[i]);
+    }
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j) copy(it + j + kDepth);
+  }
+  // the key streams of a warp, then the warps, then the cluster, always in the same order
+#pragma unroll
+  for (int o = LPK; o < 32; o <<= 1) {
+    const float top = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o)), f = weight_of(m, top);
+    m = top;
+    l *= f;
+    l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      acc[i] *= f;
+      acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+    }
+  }
+  copies_wait<0>();
+  __syncthreads();                                                    // the ring is read out
+  if (sub == 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sums[warp * L::kRow + ch + i] = acc[i];
+  }
+  if (lane == 0) {
+    sums[warp * L::kRow + HD] = m;
+    sums[warp * L::kRow + HD + 1] = l;
+  }
+  __syncthreads();
+  if (tid < HD) {
+    float top = -INFINITY, v = 0.f, sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) top = fmaxf(top, sums[k * L::kRow + HD]);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float f = weight_of(sums[k * L::kRow + HD], top);
+      v = fmaf(f, sums[k * L::kRow + tid], v);
+      sum = fmaf(f, sums[k * L::kRow + HD + 1], sum);
+    }
+    part[tid] = v;
+    if (tid == 0) {
+      part[HD] = top;
+      part[HD + 1] = sum;
+    }
+  }
+  if (splits > 1) cluster_barrier();
+  else __syncthreads();
+  if (rank == 0 && tid < HD) {
+    float top = part[HD], v = part[tid], sum = part[HD + 1];
+    if (splits > 1) {
+      float ms[kMaxCluster], vs[kMaxCluster], ls[kMaxCluster];
+#pragma unroll
+      for (int k = 0; k < kMaxCluster; ++k)
+        if (k < splits) {
+          ms[k] = ld_rank(part + HD, k);
+          vs[k] = ld_rank(part + tid, k);
+          ls[k] = ld_rank(part + HD + 1, k);
+          top = fmaxf(top, ms[k]);
+        }
+      v = sum = 0.f;
+#pragma unroll
+      for (int k = 0; k < kMaxCluster; ++k)
+        if (k < splits) {
+          const float f = weight_of(ms[k], top);
+          v = fmaf(f, vs[k], v);
+          sum = fmaf(f, ls[k], sum);
+        }
+    }
+    p.O[int64_t(b) * p.o_sb + int64_t(g) * HD + tid] = hg_f2lp(sum == 0.f ? 0.f : v / sum);
+    if (tid == 0) p.LSE[size_t(b) * p.nheads + g] = sum > 0.f ? (top + log2f(sum)) * kLn2 : -INFINITY;
+  }
+  if (splits > 1) cluster_barrier();                                  // nobody leaves while its part may be read
+}
+
+// CTAs that share a head's keys, a power of two.  Two CTAs an SM stream at the memory's rate, so a wave is split until it has
+// those, eight steps each at least; heads of more than a wave of three CTAs an SM only where the keys are many enough that a
+// nearly empty last wave costs more than the merge.  Us cold, one, two, four, eight CTAs a head, head dim 128: 32 heads x 4000
+// keys 49, 33, 25, 23; 64 x 4000 53, 41, 35, 41; 128 x 4000 64, 59, 68, 66; 256 x 4000 102, 107, 107, 109; 512 x 300 29, 33,
+// 39, 57; 512 x 1000 72, 66, 68, 82; 512 x 4000 203, 178, 174, 186.
+int stream_splits(long long heads, int steps) {
+  int s = 1;
+  while (s < kMaxCluster && heads * s * 2 <= 296 && steps >= s * 16) s *= 2;
+  if (heads > 444) s = steps >= 192 ? 4 : steps >= 48 ? 2 : 1;
+  return s;
+}
+
+template <int HD>
+int launch_stream(const DecodeParams& p, int settled, cudaStream_t st) {
+  auto k = flash_stream_kernel<HD>;
+  constexpr int kps = 2048 / HD;
+  const int splits = stream_splits((long long)p.nkv * p.B, (p.kv_len + kps - 1) / kps);
+  if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, StreamSmem<HD>::kTotal)) return int(e);
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(splits);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(unsigned(splits), unsigned(p.nkv), unsigned(p.B));
+  cfg.blockDim = dim3(kStreamThreads, 1, 1);
+  cfg.dynamicSmemBytes = StreamSmem<HD>::kTotal;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = hg_host::chain_overlaps() ? 2 : 1;
+  return int(cudaLaunchKernelEx(&cfg, k, p, settled));
+}
+
 inline int keys_seen(int Sq, int Skv, int causal, int q_pos0, int k_pos0) {
   long long n = Skv;
   if (causal) {
@@ -286,21 +502,54 @@ int hg_flash_decode_pays(int Sq, int Skv, int B, int nheads, int nkv, int hd, in
   return keys >= (hd == 128 && rows > 2 ? 2000 : 1536);
 }
 
+static DecodeParams decode_params(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o,
+                                  void* lse, int Sq, int Skv, int B, int nheads, int nkv, int causal, int q_pos0, int k_pos0,
+                                  float scale) {
+  DecodeParams p{};
+  p.Q = (const hg_lp_t*)q->ptr; p.K = (const hg_lp_t*)k->ptr; p.V = (const hg_lp_t*)v->ptr; p.O = (hg_lp_t*)o->ptr;
+  p.q_ss = q->ss; p.q_sb = q->sb; p.k_ss = k->ss; p.k_sb = k->sb; p.v_ss = v->ss; p.v_sb = v->sb; p.o_ss = o->ss; p.o_sb = o->sb;
+  p.q_gs = q->gs; p.q_hs = q->hs; p.q_off = q->off;
+  p.k_gs = k->gs; p.k_off = k->off; p.v_gs = v->gs; p.v_off = v->off;
+  p.LSE = (float*)lse;
+  p.Sq = Sq; p.B = B; p.nheads = nheads; p.nkv = nkv; p.qpg = nheads / nkv; p.causal = causal;
+  p.q_pos0 = q_pos0; p.k_pos0 = k_pos0; p.scale = scale;
+  p.kv_len = keys_seen(Sq, Skv, causal, q_pos0, k_pos0);
+  return p;
+}
+
+// Whether hg_flash_fwd gives the call to hg_flash_stream: one query, a kv head of its own for every head, and not what the
+// spread keys are taken for.  It wins there but for 129 to 148 heads of many keys, two CTAs a head on two to an SM (144 heads x
+// 4000 keys 68 / 68, 16000 197 / 205).  Us cold, tile kernel / here, head dim 128: 32 heads x 100 keys 12 / 8,
+// 300 14 / 12, 1000 21 / 14; 64 x 1000 23 / 16; 128 x 100 12 / 10, 1000 25 / 23, 4000 61 / 59, 16000 186 / 174; 256 x 300 27 / 16,
+// 1000 45 / 35, 4000 115 / 100; head dim 64: 32 x 1000 21 / 12, 128 x 300 14 / 11, 1000 23 / 16.  Probabilities stay in fp32:
+// 0.0017 of the result's norm off 64 bits (the rounding of the result), 0.0023 on the tile kernel.
+int hg_flash_stream_takes(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, int Sq, int Skv, int B,
+                          int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
+  if ((hd != 64 && hd != 128) || Sq != 1 || Skv < 1 || B < 1 || nheads < 1 || nheads != nkv || nkv > 65535 || B > 65535) return 0;
+  for (const HgAttnTensor* t : {q, k, v})
+    if ((uintptr_t(t->ptr) & 15) || (t->ss & 7) || (t->sb & 7)) return 0;
+  const long long heads = (long long)B * nheads;
+  if (heads > 128 && heads <= 148 && keys_seen(Sq, Skv, causal, q_pos0, k_pos0) >= 4000) return 0;
+  return !hg_flash_decode_pays(Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0);
+}
+
+// Same contract as hg_flash_fwd for those calls.  settled: keys that no kernel of an open chain writes.
+int hg_flash_stream(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o, void* lse,
+                    int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0, float scale,
+                    int settled, void* stream) {
+  const DecodeParams p = decode_params(q, k, v, o, lse, Sq, Skv, B, nheads, nkv, causal, q_pos0, k_pos0, scale);
+  cudaStream_t st = (cudaStream_t)stream;
+  return hd == 128 ? launch_stream<128>(p, settled, st) : launch_stream<64>(p, settled, st);
+}
+
 // Same contract as hg_flash_fwd for the calls that hg_flash_decode_scratch accepts; `ws` is its scratch.
 int hg_flash_decode(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o, void* lse,
                     void* ws, int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0,
                     float scale, void* stream) {
   const long long need = hg_flash_decode_scratch(q, k, v, Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0);
   if (need < 0 || (need > 0 && ws == nullptr)) return -1;
-  DecodeParams p{};
-  p.Q = (const hg_lp_t*)q->ptr; p.K = (const hg_lp_t*)k->ptr; p.V = (const hg_lp_t*)v->ptr; p.O = (hg_lp_t*)o->ptr;
-  p.q_ss = q->ss; p.q_sb = q->sb; p.k_ss = k->ss; p.k_sb = k->sb; p.v_ss = v->ss; p.v_sb = v->sb; p.o_ss = o->ss; p.o_sb = o->sb;
-  p.q_gs = q->gs; p.q_hs = q->hs; p.q_off = q->off;
-  p.k_gs = k->gs; p.k_off = k->off; p.v_gs = v->gs; p.v_off = v->off;
-  p.LSE = (float*)lse; p.ws = (float*)ws;
-  p.Sq = Sq; p.B = B; p.nheads = nheads; p.nkv = nkv; p.qpg = nheads / nkv; p.causal = causal;
-  p.q_pos0 = q_pos0; p.k_pos0 = k_pos0; p.scale = scale;
-  p.kv_len = keys_seen(Sq, Skv, causal, q_pos0, k_pos0);
+  DecodeParams p = decode_params(q, k, v, o, lse, Sq, Skv, B, nheads, nkv, causal, q_pos0, k_pos0, scale);
+  p.ws = (float*)ws;
   const int chunk = keys_per_cta(Sq * p.qpg, p.kv_len, nkv, B), ranges = range_count(p.kv_len, chunk);
   cudaStream_t st = (cudaStream_t)stream;
   return hd == 128 ? launch_rows<128>(p, chunk, ranges, st) : launch_rows<64>(p, chunk, ranges, st);
