@@ -64,6 +64,13 @@ struct RowColWalk {
 __global__ void rope_kernel(hg_lp_t* __restrict__ buf, const int* __restrict__ slot, int slot_width, int nheads,
                             int row_pitch, int tokens, int batch, const int* __restrict__ pos, int pos_offset,
                             const float* __restrict__ cos_t, const float* __restrict__ sin_t, int half, float sign) {
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  buf += zero;
+  slot += zero;
+  cos_t += zero;
+  sin_t += zero;
+  if (pos != nullptr) pos += zero;
   const int vec_per_head = half >> 3;  // uint4 chunks in one half
   const int per_token = nheads * vec_per_head;
   for (RowColWalk w(per_token); w.row < tokens; w.next()) {
@@ -100,6 +107,13 @@ __global__ void rope_interleaved_kernel(hg_lp_t* __restrict__ buf, const int* __
                                         int row_pitch, int tokens, int batch, const int* __restrict__ pos,
                                         int pos_offset, const float* __restrict__ cos_t,
                                         const float* __restrict__ sin_t, int half, float sign) {
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  buf += zero;
+  slot += zero;
+  cos_t += zero;
+  sin_t += zero;
+  if (pos != nullptr) pos += zero;
   const int vec_per_head = half >> 2;  // uint4 chunks over the 2*half rotated channels
   const int per_token = nheads * vec_per_head;
   for (RowColWalk w(per_token); w.row < tokens; w.next()) {
@@ -217,6 +231,10 @@ __global__ void glu_fwd_kernel(const hg_lp_t* __restrict__ y, hg_lp_t* __restric
 template <int KIND>
 __global__ void glu_bwd_kernel(const hg_lp_t* __restrict__ g, const hg_lp_t* __restrict__ y,
                                hg_lp_t* __restrict__ dy, int64_t rows, int F) {
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  g += zero;
+  y += zero;
   for (RowColWalk w(F >> 3); w.row < rows; w.next()) {
     const int64_t r = w.row;
     const int c = w.col;
@@ -331,6 +349,9 @@ __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids, const hg_l
 __global__ void __launch_bounds__(256)
 colsum_kernel(const hg_lp_t* __restrict__ x, int64_t pitch, int rows, int cols, float* __restrict__ partial,
               hg_lp_t* __restrict__ out) {
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  x += zero;
   __shared__ float red[8][256];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int c0 = blockIdx.x * 256 + lane * 8;
@@ -377,6 +398,9 @@ colsum_kernel(const hg_lp_t* __restrict__ x, int64_t pitch, int rows, int cols, 
 }
 
 __global__ void colsum_final_kernel(const float* __restrict__ partial, int parts, int cols, hg_lp_t* __restrict__ out) {
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  partial += zero;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= cols) return;
   float t = 0.f;
@@ -473,7 +497,7 @@ int launch_gelu(const void* y, const void* g, void* out, int64_t n, cudaStream_t
   const bool four = n >= 148 * 8 * 1024;
   const int64_t per = four ? 1024 : 256, grid = (n + per - 1) / per;
   if (grid > 0x7fffffff) return -1;
-  return hg_host::launch(four ? gelu_kernel<BWD, 4> : gelu_kernel<BWD, 1>, int(grid), 256, 0, st, (const hg_lp_t*)y,
+  return hg_host::launch_over(four ? gelu_kernel<BWD, 4> : gelu_kernel<BWD, 1>, int(grid), 256, 0, st, (const hg_lp_t*)y,
                          (const hg_lp_t*)g, (hg_lp_t*)out, n);
 }
 
@@ -490,16 +514,14 @@ int hg_rope(void* buf, const void* slots, int slot_width, int nheads, int row_pi
   const float sign = (flags & 1) ? -1.f : 1.f;
   if (flags & 2) {
     const int64_t work = int64_t(tokens) * nheads * (half >> 2);
-    rope_interleaved_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
-        (hg_lp_t*)buf, (const int*)slots, slot_width, nheads, row_pitch, tokens, batch, (const int*)pos, pos_offset,
-        (const float*)cos_t, (const float*)sin_t, half, sign);
-  } else {
-    const int64_t work = int64_t(tokens) * nheads * (half >> 3);
-    rope_kernel<<<grid_for(work, 256), 256, 0, (cudaStream_t)stream>>>(
-        (hg_lp_t*)buf, (const int*)slots, slot_width, nheads, row_pitch, tokens, batch, (const int*)pos, pos_offset,
-        (const float*)cos_t, (const float*)sin_t, half, sign);
+    return hg_host::launch_over(rope_interleaved_kernel, grid_for(work, 256), 256, 0, (cudaStream_t)stream, (hg_lp_t*)buf,
+                           (const int*)slots, slot_width, nheads, row_pitch, tokens, batch, (const int*)pos, pos_offset,
+                           (const float*)cos_t, (const float*)sin_t, half, sign);
   }
-  return int(cudaGetLastError());
+  const int64_t work = int64_t(tokens) * nheads * (half >> 3);
+  return hg_host::launch_over(rope_kernel, grid_for(work, 256), 256, 0, (cudaStream_t)stream, (hg_lp_t*)buf, (const int*)slots,
+                         slot_width, nheads, row_pitch, tokens, batch, (const int*)pos, pos_offset, (const float*)cos_t,
+                         (const float*)sin_t, half, sign);
 }
 
 // See rope_append_kernel.  rot_dim = 0: no rotation (cos_t / sin_t unused).  Strides in elements, multiples of 8; all
@@ -512,7 +534,7 @@ int hg_rope_append(void* qkv, int tokens, int batch, int ng, int qpg, int hd, in
   if ((hd & 7) || (half & 7) || batch < 1 || ng < 1 || qpg < 1 || ((k_ss | k_sb | v_ss | v_sb) & 7)) return -1;
   if ((uintptr_t(qkv) | uintptr_t(kc) | uintptr_t(vc)) & 15) return -1;
   const int64_t work = int64_t(tokens) * ng * (qpg + 2) * (hd >> 3);
-  return hg_host::launch(rope_append_kernel, grid_for(work, 256), 256, 0, (cudaStream_t)stream, (hg_lp_t*)qkv, tokens, batch,
+  return hg_host::launch_over(rope_append_kernel, grid_for(work, 256), 256, 0, (cudaStream_t)stream, (hg_lp_t*)qkv, tokens, batch,
                          ng, qpg, hd, pos_offset, (const float*)cos_t, (const float*)sin_t, half, interleaved, (hg_lp_t*)kc,
                          (hg_lp_t*)vc, k_ss, k_sb, v_ss, v_sb);
 }
@@ -523,7 +545,7 @@ int hg_glu_fwd(const void* y, void* out, long long rows, int F, int kind, void* 
   const int g = grid_for(rows * (F >> 3), 256);
   cudaStream_t st = (cudaStream_t)stream;
   if (kind == 2) return launch_gelu<false>(y, nullptr, out, rows * (F >> 3), st);
-  return hg_host::launch(kind == 0 ? glu_fwd_kernel<0> : glu_fwd_kernel<1>, g, 256, 0, st, (const hg_lp_t*)y, (hg_lp_t*)out, rows, F);
+  return hg_host::launch_over(kind == 0 ? glu_fwd_kernel<0> : glu_fwd_kernel<1>, g, 256, 0, st, (const hg_lp_t*)y, (hg_lp_t*)out, rows, F);
 }
 
 int hg_glu_bwd(const void* g_, const void* y, void* dy, long long rows, int F, int kind, void* stream) {
@@ -533,9 +555,8 @@ int hg_glu_bwd(const void* g_, const void* y, void* dy, long long rows, int F, i
   cudaStream_t st = (cudaStream_t)stream;
   auto G = (const hg_lp_t*)g_;
   if (kind == 2) return launch_gelu<true>(y, g_, dy, rows * (F >> 3), st);
-  if (kind == 0) glu_bwd_kernel<0><<<g, 256, 0, st>>>(G, (const hg_lp_t*)y, (hg_lp_t*)dy, rows, F);
-  else glu_bwd_kernel<1><<<g, 256, 0, st>>>(G, (const hg_lp_t*)y, (hg_lp_t*)dy, rows, F);
-  return int(cudaGetLastError());
+  return hg_host::launch_over(kind == 0 ? glu_bwd_kernel<0> : glu_bwd_kernel<1>, g, 256, 0, st, G, (const hg_lp_t*)y, (hg_lp_t*)dy, rows,
+                         F);
 }
 
 int hg_embedding_fwd(const void* ids, const void* W, const void* pos_emb, void* out, int tokens, int H, int v0, int v1,
@@ -576,11 +597,11 @@ int hg_colsum_bf16(const void* x, long long pitch, int rows, int cols, void* par
   if (cols <= 0) return 0;
   if ((pitch & 7) || (uintptr_t(x) & 15) || parts < 1 || parts > 65535) return -1;
   cudaStream_t st = (cudaStream_t)stream;
-  colsum_kernel<<<dim3((cols + 255) / 256, parts), 256, 0, st>>>((const hg_lp_t*)x, pitch, rows, cols, (float*)partial,
-                                                                 (hg_lp_t*)out);
-  if (parts > 1)
-    colsum_final_kernel<<<(cols + 127) / 128, 128, 0, st>>>((const float*)partial, parts, cols, (hg_lp_t*)out);
-  return int(cudaGetLastError());
+  int rc = hg_host::launch_over(colsum_kernel, dim3((cols + 255) / 256, parts), 256, 0, st, (const hg_lp_t*)x, int64_t(pitch), rows, cols,
+                           (float*)partial, (hg_lp_t*)out);
+  if (rc == 0 && parts > 1)
+    rc = hg_host::launch_over(colsum_final_kernel, (cols + 127) / 128, 128, 0, st, (const float*)partial, parts, cols, (hg_lp_t*)out);
+  return rc;
 }
 
 int hg_cast_f32_bf16(const void* in, void* out, long long n, void* stream) {
@@ -592,7 +613,7 @@ int hg_cast_f32_bf16(const void* in, void* out, long long n, void* stream) {
 
 int hg_add_bf16(const void* a, const void* b, void* out, long long n, void* stream) {
   if (n <= 0) return 0;
-  return hg_host::launch(add_bf16_kernel, grid_for(n >> 3, 256), 256, 0, (cudaStream_t)stream, (const hg_lp_t*)a,
+  return hg_host::launch_over(add_bf16_kernel, grid_for(n >> 3, 256), 256, 0, (cudaStream_t)stream, (const hg_lp_t*)a,
                          (const hg_lp_t*)b, (hg_lp_t*)out, n);
 }
 

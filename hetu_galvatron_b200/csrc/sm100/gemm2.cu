@@ -75,6 +75,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
   const uint32_t tmem_base = pair_setup(s, &tmA, &tmB, warp);
+  chain_release();                            // after the allocation: see chain_release
+  chain_wait();
 
   if (warp == 0) {
     producer2<A_MN, B_MN>(&tmA, &tmB, p, s, rank, pair, pairs, num_tiles);
@@ -157,6 +159,8 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   const uint32_t rank = cluster_ctarank();
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const uint32_t tmem_base = pair_setup(s, &tmA, &tmB, warp);
+  chain_release();                            // after the allocation: see chain_release
+  chain_wait();
 
   if (warp == 0) {
     uint32_t stage = 0, phase = 0;
@@ -331,7 +335,7 @@ unsigned long long split_token() {
 
 // Launch attributes of a kernel of CTA pairs, and how many pairs of it the device holds at once (-2: none).
 template <typename K>
-static int pair_config(K kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int* max_pairs, cudaStream_t st) {
+static int pair_config(K kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int* max_pairs, bool overlaps, cudaStream_t st) {
   attr->id = cudaLaunchAttributeClusterDimension;
   attr->val.clusterDim.x = 2;
   attr->val.clusterDim.y = 1;
@@ -339,6 +343,8 @@ static int pair_config(K kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* a
   cfg->blockDim = dim3(192, 1, 1);
   cfg->dynamicSmemBytes = SMEM2_BYTES;
   cfg->stream = st;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg->attrs = attr;
   cfg->numAttrs = 1;
   if (*max_pairs < 0) {
@@ -354,6 +360,7 @@ static int pair_config(K kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* a
     if (n <= 0) return -2;
     *max_pairs = n;
   }
+  if (overlaps) cfg->numAttrs = 2;
   return 0;
 }
 
@@ -363,8 +370,8 @@ static int launch_grouped2(const CUtensorMap& ta, const CUtensorMap& tb, const C
   static int max_pairs = -1;
   auto k = grouped_gemm2_kernel<A_MN, B_MN, Tiles>;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr;
-  if (int rc = pair_config(k, &cfg, &attr, &max_pairs, st)) return rc;
+  cudaLaunchAttribute attr[2];
+  if (int rc = pair_config(k, &cfg, attr, &max_pairs, hg_host::launch_overlaps(), st)) return rc;
   const int pairs = want_pairs < max_pairs ? want_pairs : max_pairs;
   cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
   return int(cudaLaunchKernelEx(&cfg, k, ta, tb, tc, p, tiles));
@@ -377,8 +384,8 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   static int max_pairs = -1;
   auto k = gemm2_bf16_kernel<A_MN, B_MN>;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr;
-  if (int rc = pair_config(k, &cfg, &attr, &max_pairs, st)) return rc;
+  cudaLaunchAttribute attr[2];
+  if (int rc = pair_config(k, &cfg, attr, &max_pairs, hg_host::launch_overlaps(), st)) return rc;
   int pairs = want_pairs < max_pairs ? want_pairs : max_pairs;
   // Last wave partly filled: let several pairs share each of its tiles (see Params::split_s).
   const int tiles = p.tiles_m * p.tiles_n, num_kb = (p.K + BK - 1) / BK;
@@ -457,8 +464,8 @@ long long hg_gemm2_scratch(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   static int max_pairs = -1;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr;
-  if (pair_config(gemm2_bf16_kernel<false, false>, &cfg, &attr, &max_pairs, nullptr)) return 0;
+  cudaLaunchAttribute attr[2];
+  if (pair_config(gemm2_bf16_kernel<false, false>, &cfg, attr, &max_pairs, false, nullptr)) return 0;
   return split_plan(((M + CM - 1) / CM) * ((N + BN - 1) / BN), (K + BK - 1) / BK, max_pairs).bytes();
 }
 

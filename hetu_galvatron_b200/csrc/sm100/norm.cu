@@ -195,6 +195,14 @@ norm_bwd_kernel(const hg_lp_t* __restrict__ dy, const hg_lp_t* __restrict__ h,
                 hg_lp_t* __restrict__ dx, float* __restrict__ dw_partial, float* __restrict__ db_partial,
                 int rows, int H) {
   constexpr int G = kBwdThreads / TPR;
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  dy += zero;
+  h += zero;
+  w += zero;
+  rstd_in += zero;
+  mean_in += zero;
+  dres += dres ? zero : 0;
   __shared__ float2 red[2][kBwdThreads / 32];
   extern __shared__ __align__(16) float comb[];                      // G > 1: [G - 1][H] accumulators of the other groups
   const int group = threadIdx.x / TPR, t = threadIdx.x - group * TPR;
@@ -328,6 +336,10 @@ norm_bwd_kernel(const hg_lp_t* __restrict__ dy, const hg_lp_t* __restrict__ h,
 // parts; one thread per column with all parts in one chain left most of the chip idle for the whole sum.
 __global__ void __launch_bounds__(512)
 reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, int parts, int H, int accumulate) {
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  partial += zero;
+  out += zero;
   __shared__ float red[16][32];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -355,13 +367,13 @@ int launch_norm_bwd(const void* dy, const void* h, const void* w, const void* rs
   const int grid = want < parts ? want : parts;
   const size_t smem = size_t(G - 1) * H * sizeof(float);
   static_assert(size_t(G - 1) * TPR * VPT * 8 * sizeof(float) <= 48 * 1024, "fits without an opt-in");
-  norm_bwd_kernel<RMS, TPR, VPT><<<grid, kBwdThreads, smem, st>>>(
-      (const hg_lp_t*)dy, (const hg_lp_t*)h, (const hg_lp_t*)w, (const float*)rstd, (const float*)mean,
-      (const hg_lp_t*)dres, (hg_lp_t*)dx, P, RMS ? nullptr : PB, rows, H);
+  int rc = hg_host::launch_over(norm_bwd_kernel<RMS, TPR, VPT>, grid, kBwdThreads, smem, st, (const hg_lp_t*)dy, (const hg_lp_t*)h,
+                           (const hg_lp_t*)w, (const float*)rstd, (const float*)mean, (const hg_lp_t*)dres, (hg_lp_t*)dx, P,
+                           RMS ? nullptr : PB, rows, H);
   const int cols = (H + 31) / 32;
-  reduce_partials_kernel<<<cols, 512, 0, st>>>(P, (float*)dw, grid, H, accumulate);
-  if (!RMS && db) reduce_partials_kernel<<<cols, 512, 0, st>>>(PB, (float*)db, grid, H, accumulate);
-  return int(cudaGetLastError());
+  if (rc == 0) rc = hg_host::launch_over(reduce_partials_kernel, cols, 512, 0, st, P, (float*)dw, grid, H, accumulate);
+  if (rc == 0 && !RMS && db) rc = hg_host::launch_over(reduce_partials_kernel, cols, 512, 0, st, PB, (float*)db, grid, H, accumulate);
+  return rc;
 }
 
 template <bool RMS, typename... A>
@@ -392,7 +404,7 @@ int hg_norm_fwd(const void* x, const void* residual, const void* w, const void* 
   auto B = reinterpret_cast<const hg_lp_t*>(b);
   auto Y = reinterpret_cast<hg_lp_t*>(y);
   auto Ho = reinterpret_cast<hg_lp_t*>(h_out);
-#define HG_FWD(R_, V_) return hg_host::launch(norm_fwd_kernel<R_, V_>, grid, kThreads, 0, st, X, R, W, B, Y, Ho, (float*)rstd, (float*)mean, rows, H, eps)
+#define HG_FWD(R_, V_) return hg_host::launch_over(norm_fwd_kernel<R_, V_>, grid, kThreads, 0, st, X, R, W, B, Y, Ho, (float*)rstd, (float*)mean, rows, H, eps)
   if (rms) { if (H <= 4096) HG_FWD(true, 2); else if (H <= 8192) HG_FWD(true, 4); else HG_FWD(true, 8); }
   else     { if (H <= 4096) HG_FWD(false, 2); else if (H <= 8192) HG_FWD(false, 4); else HG_FWD(false, 8); }
 #undef HG_FWD

@@ -33,6 +33,7 @@ static thread_local int t_chain = -1;
 Chain::Chain() { t_chain = 0; }
 Chain::~Chain() { t_chain = -1; }
 bool chain_overlaps() { return t_chain >= 0 && t_chain++ > 0; }
+bool launch_overlaps() { return t_chain < 0 || t_chain++ > 0; }
 
 // cuTensorMapEncodeTiled is a driver call and needs a current context on the calling thread; threads
 // that have only been handed work by another thread (autograd's backward workers) may not have bound

@@ -24,6 +24,10 @@ __global__ void __launch_bounds__(kThreads)
 xent_stats_kernel(const hg_lp_t* __restrict__ logits, int64_t pitch, const int64_t* __restrict__ targets,
                   int v0, int V, float* __restrict__ out_max, float* __restrict__ out_sum,
                   float* __restrict__ out_pred, float* __restrict__ out_loss, int rows) {
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  logits += zero;
+  targets += zero;
   __shared__ float sm[kThreads / 32], ss[kThreads / 32];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const hg_lp_t* x = logits + size_t(row) * pitch;
@@ -78,6 +82,13 @@ __global__ void __launch_bounds__(kThreads)
 xent_bwd_kernel(hg_lp_t* __restrict__ logits, int64_t pitch, const int64_t* __restrict__ targets, int v0, int V,
                 const float* __restrict__ gmax, const float* __restrict__ gsum, const float* __restrict__ g,
                 int rows) {
+  hg::chain_release();
+  const int zero = hg::chain_wait();
+  logits += zero;
+  targets += zero;
+  gmax += zero;
+  gsum += zero;
+  g += zero;
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     hg_lp_t* x = logits + size_t(row) * pitch;
     const float m = gmax[row], inv = 1.f / gsum[row], gr = g[row];
@@ -117,10 +128,8 @@ int hg_xent_stats(const void* logits, long long pitch, const void* targets, int 
   if (rows <= 0) return 0;
   if (pitch & 7) return -1;
   const int grid = rows < 148 * 8 ? rows : 148 * 8;
-  xent_stats_kernel<<<grid, kThreads, 0, (cudaStream_t)stream>>>((const hg_lp_t*)logits, pitch,
-                                                                 (const int64_t*)targets, v0, V, (float*)out_max,
-                                                                 (float*)out_sum, (float*)out_pred, (float*)out_loss, rows);
-  return int(cudaGetLastError());
+  return hg_host::launch_over(xent_stats_kernel, grid, kThreads, 0, (cudaStream_t)stream, (const hg_lp_t*)logits, int64_t(pitch),
+                         (const int64_t*)targets, v0, V, (float*)out_max, (float*)out_sum, (float*)out_pred, (float*)out_loss, rows);
 }
 
 int hg_xent_bwd(void* logits, long long pitch, const void* targets, int v0, int V, const void* gmax, const void* gsum,
@@ -128,10 +137,8 @@ int hg_xent_bwd(void* logits, long long pitch, const void* targets, int v0, int 
   if (rows <= 0) return 0;
   if (pitch & 7) return -1;
   const int grid = rows < 148 * 8 ? rows : 148 * 8;
-  xent_bwd_kernel<<<grid, kThreads, 0, (cudaStream_t)stream>>>((hg_lp_t*)logits, pitch, (const int64_t*)targets,
-                                                               v0, V, (const float*)gmax, (const float*)gsum,
-                                                               (const float*)g, rows);
-  return int(cudaGetLastError());
+  return hg_host::launch_over(xent_bwd_kernel, grid, kThreads, 0, (cudaStream_t)stream, (hg_lp_t*)logits, int64_t(pitch),
+                         (const int64_t*)targets, v0, V, (const float*)gmax, (const float*)gsum, (const float*)g, rows);
 }
 
 }  // extern "C"

@@ -1,0 +1,46 @@
+"""Kernels that may start before the one in front of them has ended: the same bits as with a wait after every operation."""
+import pytest
+import torch
+
+from hetu_galvatron_b200 import ops
+from hetu_galvatron_b200.ops import _lib
+
+pytestmark = pytest.mark.gpu
+DEV, LP = "cuda", torch.bfloat16
+
+
+@pytest.mark.parametrize("rows,H,F", [(300, 256, 512), (2049, 1600, 6400)])
+@pytest.mark.parametrize("rms", [True, False])
+def test_operations_back_to_back(rows, H, F, rms):
+    torch.manual_seed(rows)
+    x, new = (torch.randn(rows, H, device=DEV).to(LP) for _ in range(2))
+    ps = [torch.nn.Parameter(torch.randn(*s, device=DEV).to(LP) * 0.1) for s in ((H,), (H,), (F, H), (F,), (H, F), (H,))]
+
+    def step(wait):
+        pause = torch.cuda.synchronize if wait else (lambda: None)
+        for p in ps:
+            p.main_grad, p.mg_fresh, p.grad = torch.full(p.shape, 2.0, device=DEV), False, None
+        a = torch.zeros_like(x)
+        torch.cuda.synchronize()
+        if not wait:
+            torch.cuda._sleep(2000000)                # everything is queued before the first kernel runs
+        a.copy_(new)                                  # written by the kernel in front
+        a.requires_grad_()
+        y, _ = ops.norm(a, ps[0], None if rms else ps[1], 1e-5, rms)
+        pause()
+        h = ops.linear(y, ps[2], ps[3])
+        pause()
+        h = ops.activation(h, "gelu")
+        pause()
+        out = ops.linear(h, ps[4], ps[5])
+        pause()
+        loss = ops.cross_entropy(out, torch.arange(rows, device=DEV) % H)
+        loss.sum().backward()
+        pause()
+        return [out.detach().clone(), a.grad, *[p.main_grad for p in ps], *[p.grad for p in ps if p.grad is not None]]
+
+    want = step(True)
+    for _ in range(3):
+        for s, t in zip(step(False), want, strict=True):
+            assert torch.equal(s, t)
+    _lib.assert_healthy()
