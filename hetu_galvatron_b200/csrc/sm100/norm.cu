@@ -62,6 +62,8 @@ norm_fwd_kernel(const hg_lp_t* __restrict__ x, const hg_lp_t* __restrict__ resid
   const int zero = hg::chain_wait();
   x += zero;
   residual += zero;
+  w += zero;
+  b += zero;
   const int nvec = H >> 3;
   // The next row's loads are issued before this row's reductions, so that a block always has a row in flight
   // across its __syncthreads (with one row per trip the memory system idles while the block reduces).

@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from hetu_galvatron_b200 import ops
+from hetu_galvatron_b200.models.modules import ops_add
 from hetu_galvatron_b200.ops import _lib
 
 pytestmark = pytest.mark.gpu
@@ -43,4 +44,23 @@ def test_operations_back_to_back(rows, H, F, rms):
     for _ in range(3):
         for s, t in zip(step(False), want, strict=True):
             assert torch.equal(s, t)
+    _lib.assert_healthy()
+
+
+# the norm's weight and bias are the results of a kernel that lets the next one start before it has written anything
+@pytest.mark.parametrize("rows,H", [(1, 4096), (300, 256), (2049, 1600), (148, 16384)])
+@pytest.mark.parametrize("rms", [True, False])
+def test_norm_weights_written_by_the_kernel_in_front(rows, H, rms):
+    torch.manual_seed(rows)
+    x, (w1, w2) = torch.randn(rows, H, device=DEV).to(LP), torch.randn(2, H, device=DEV).to(LP)
+    w = ops_add(w1, w2)
+    want, _ = ops.norm(x, w, None if rms else w, 1e-5, rms)
+    for _ in range(5):
+        del w
+        torch.zeros(H, device=DEV, dtype=LP)                               # the memory that the next result takes
+        torch.cuda.synchronize()
+        torch.cuda._sleep(500000)                                          # everything is queued before the first kernel runs
+        w = ops_add(w1, w2)
+        y, _ = ops.norm(x, w, None if rms else w, 1e-5, rms)
+        assert torch.equal(y, want)
     _lib.assert_healthy()
