@@ -149,6 +149,8 @@ __global__ void rope_append_kernel(hg_lp_t* __restrict__ qkv, int tokens, int ba
   hg::chain_release();
   const int zero = hg::chain_wait();
   qkv += zero;
+  cos_t += zero;
+  sin_t += zero;
   kc += zero;
   vc += zero;
   const int vph = hd >> 3, slots = ng * (qpg + 2);

@@ -64,3 +64,35 @@ def test_norm_weights_written_by_the_kernel_in_front(rows, H, rms):
         y, _ = ops.norm(x, w, None if rms else w, 1e-5, rms)
         assert torch.equal(y, want)
     _lib.assert_healthy()
+
+
+# the tables are copied right in front of the kernels that rotate by them: inside the packed projection, and into a cache
+@pytest.mark.parametrize("interleaved", [False, True])
+def test_rotation_tables_written_in_front(interleaved):
+    S, B, nh, ng, hd = 40, 2, 8, 2, 128
+    torch.manual_seed(1)
+    qkv = torch.randn(S * B, (nh + 2 * ng) * hd, device=DEV).to(LP)
+    new = torch.randn(2, S, hd // 2, device=DEV)
+    slots = torch.arange(ng * (nh // ng + 2), device=DEV, dtype=torch.int32)
+
+    def run(wait):
+        tables, caches = torch.zeros_like(new), torch.zeros(2, S, B, ng, hd, device=DEV, dtype=LP)
+        mine, other = qkv.clone(), qkv.clone()
+        torch.cuda.synchronize()
+        if not wait:
+            torch.cuda._sleep(500000)
+        tables.copy_(new)
+        if wait:
+            torch.cuda.synchronize()
+        out = ops.attention.cached_attention(mine, *caches, 0, 0, S, B, nh, ng, hd, *tables, interleaved)
+        if not wait:
+            torch.cuda._sleep(500000)
+        tables.copy_(-new)
+        if wait:
+            torch.cuda.synchronize()
+        ops.rope_packed(other, slots, hd, *tables, B, interleaved=interleaved)
+        return out, caches, other
+
+    for s, t in zip(run(False), run(True), strict=True):
+        assert torch.equal(s, t)
+    _lib.assert_healthy()
