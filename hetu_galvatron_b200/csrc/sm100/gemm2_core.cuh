@@ -347,7 +347,7 @@ __device__ __forceinline__ void add_bias_row(const Params& p, int col0, uint32_t
   if (col0 + N <= p.N && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
 #pragma unroll
     for (int q = 0; q < N / 8; ++q) {
-      const uint4 u = __ldg(reinterpret_cast<const uint4*>(src) + q);
+      const uint4 u = reinterpret_cast<const uint4*>(src)[q];
       const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
       for (int j = 0; j < 4; ++j) {

@@ -30,3 +30,11 @@ def test_restrict_inputs_are_tied_to_the_wait(name):
         assert inputs, kernel
         loose = [p for p in inputs if not re.search(r"\b%s \+= [^;]*(zero|chain_wait\(\))" % p, body)]
         assert not loose, (kernel, loose)
+
+
+# A load through the read-only path makes the same promise at the load itself.
+@pytest.mark.parametrize("path", sorted([*SM100.glob("*.cu"), *SM100.glob("*.cuh")]), ids=lambda p: p.name)
+def test_no_read_only_loads_behind_a_wait(path):
+    text = re.sub(r"//.*", "", path.read_text())
+    if path.suffix == ".cuh" or "chain_wait()" in text:
+        assert not re.findall(r"__ldg\b|ld\.global\S*\.nc\b", text)
