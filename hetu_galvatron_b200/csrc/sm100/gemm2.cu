@@ -294,23 +294,23 @@ int split_mode() {
   return mode;
 }
 
-// What a split costs, in k-blocks (0.3 us each): the parts' way through L2 and the flags, and each part that is added.
-constexpr int kSplitCost = 20, kPartCost = 8;
+// What a split costs, in k-blocks (0.3 us each): the parts' way to L2 and the arrivals, and each part that is added.
+constexpr int kSplitCost = 24, kPartCost = 8;
 
 struct SplitPlan {
   int s, tail;                       // pairs per tail tile (0: no split), tail tiles
-  long long flag_bytes() const { return ((long long)tail * (s - 1) * 8 * sizeof(unsigned long long) + 255) / 256 * 256; }
-  long long bytes() const { return s < 2 ? 0 : flag_bytes() + (long long)tail * (s - 1) * kSplitTileFloats * sizeof(float); }
+  long long word_bytes() const { return ((long long)tail * 8 * sizeof(unsigned long long) + 255) / 256 * 256; }
+  long long bytes() const { return s < 2 ? 0 : word_bytes() + (long long)tail * s * kSplitTileFloats * sizeof(float); }
 };
 
 // How many pairs share each tile of the last wave, where the tiles leave part of it idle.
-// A tile takes 0.3 us per k-block.  A pair that adds parts reads each of them from L2 for about 2.4 us after its own last
-// product, and the flags and stores in front of that take 6 us, so a split into s slices pays where num_kb * (1 - 1/s) is more
-// than kSplitCost + kPartCost * (s - 1), and slice s pays beside s - 1 where num_kb / (s (s - 1)) is more than kPartCost.
-// One pair a tile against the rule's choice, us, fresh clocks: K = 2048 15.4 (never split; by four 20.9), K = 4096 24.5 by
-// three 21.0, K = 8192 42.3 by four 27.5; 81 tiles, 7 in the last wave, K = 4096 44.9 by three 42.8, K = 8192 83.7 by four
-// 69.7; 98 tiles, 24 in the last wave, K = 18944 211 by three 156; 256 tiles, 34 in the last wave, K = 32000 888 by two 782.
-// An attention block of 1531 x 3584 483 -> 475 us, a GPT2-XL MLP of 2997 rows 520 -> 502.
+// A tile takes 0.3 us per k-block.  The pair that adds the parts reads each of the others' from L2 for about 2.4 us after its own
+// last product; storing its own part and arriving take 7 us before that.  A split into s slices therefore pays where
+// num_kb * (1 - 1/s) is more than kSplitCost + kPartCost * (s - 1), and slice s pays beside s - 1 where num_kb / (s (s - 1)) is
+// more than kPartCost.  One pair a tile against the rule's choice, us a launch in a graph: one tile, K = 2048 14.3 (not split),
+// K = 4096 23.4 by three 22.5, K = 8192 41.2 by four 27.9; 81 tiles, 7 in the last wave, K = 4096 45.7 by three 44.7, K = 8192
+// 85.2 by four 73.9; 84 tiles, 10 in the last wave, K = 3584 41.0 (not split; by three 42.4), K = 6400 68.0 by four 61.7; 98
+// tiles, 24 in the last wave, K = 18944 194 by three 160; 256 tiles, 34 in the last wave, K = 32000 739 by two 703.
 SplitPlan split_plan(int tiles, int num_kb, int max_pairs) {
   SplitPlan p{0, tiles % max_pairs};
   if (split_mode() == 0 || p.tail == 0) return p;
@@ -322,13 +322,15 @@ SplitPlan split_plan(int tiles, int num_kb, int max_pairs) {
   } else if (s > 4) {
     s = 4;
   }
+  if (s > int(kSplitCountMask)) s = int(kSplitCountMask);
   if (s > 1) p.s = s;
   return p;
 }
 
 unsigned long long split_token() {
-  static std::atomic<unsigned long long> next{((unsigned long long)std::random_device{}() << 32) | 1u};
-  return next.fetch_add(1, std::memory_order_relaxed);
+  constexpr unsigned long long kStep = kSplitCountMask + 1;
+  static std::atomic<unsigned long long> next{((unsigned long long)std::random_device{}() << 32) | kStep};
+  return next.fetch_add(kStep, std::memory_order_relaxed);
 }
 
 }  // namespace
@@ -395,8 +397,8 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
     if (plan.s > 1 && ws_bytes >= plan.bytes()) {
       p.split_s = plan.s;
       p.split_tail_begin = tiles - plan.tail;
-      p.split_flags = static_cast<unsigned long long*>(ws);
-      p.split_ws = reinterpret_cast<float*>(static_cast<char*>(ws) + plan.flag_bytes());
+      p.split_words = static_cast<unsigned long long*>(ws);
+      p.split_ws = reinterpret_cast<float*>(static_cast<char*>(ws) + plan.word_bytes());
       p.split_token = split_token();
       pairs = p.split_tail_begin > 0 ? max_pairs : plan.tail * plan.s;
     }

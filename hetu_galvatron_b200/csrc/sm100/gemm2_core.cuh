@@ -114,6 +114,7 @@ struct Unit {
   int tile, kb0, kb1, slice;
 };
 constexpr int kSplitTileFloats = CM * BN;
+constexpr unsigned long long kSplitCountMask = 255;      // low bits of a word: slices that have arrived; a token has none of them
 // Word `q` (four columns) of 32-column block `c` of this thread's row in a partial tile: neighbouring lanes, neighbouring words.
 __device__ __forceinline__ int split_word(int warp8, int c, int q) {
   return (((warp8 * (BN / 32) + c) * 8 + q) * 32 + int(lane_id())) * 4;
@@ -319,26 +320,76 @@ __device__ __forceinline__ void tma_store_rows(const CUtensorMap* tm, StoreStage
   st.next ^= 1;
 }
 
-// The other slices' partial sums of a shared tile, as this warp's threads hold them (n = 0: none).
+// The slices of a shared tile, as this warp's threads hold its rows (n = 0: a tile of one pair): `mine` is in registers, the
+// others lie in memory.  Added in one order, the last slice first, whoever adds them.
 struct Parts {
   const float* base;
-  int n, warp8;
+  int n, mine, warp8;
   __device__ __forceinline__ void add(int c, uint32_t (&r)[32]) const {
-    for (int k = 0; k < n; ++k) {
-      float4 v[8];
+    if (n == 0) return;
+    auto part = [&](int k, int q) {
+      return __ldcg(reinterpret_cast<const float4*>(base + size_t(k) * kSplitTileFloats + split_word(warp8, c, q)));
+    };
+    if (mine == n - 1) {
+      for (int k = 0; k + 1 < n; ++k) {
+        float4 v[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
-        v[q] = __ldcg(reinterpret_cast<const float4*>(base + size_t(k) * kSplitTileFloats + split_word(warp8, c, q)));
+        for (int q = 0; q < 8; ++q) v[q] = part(k, q);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) plus(r, q, v[q]);
+      }
+    } else {
+      uint32_t own[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) own[i] = r[i];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        r[4 * q] = __float_as_uint(__uint_as_float(r[4 * q]) + v[q].x);
-        r[4 * q + 1] = __float_as_uint(__uint_as_float(r[4 * q + 1]) + v[q].y);
-        r[4 * q + 2] = __float_as_uint(__uint_as_float(r[4 * q + 2]) + v[q].z);
-        r[4 * q + 3] = __float_as_uint(__uint_as_float(r[4 * q + 3]) + v[q].w);
+        const float4 v = part(n - 1, q);
+        r[4 * q] = __float_as_uint(v.x);
+        r[4 * q + 1] = __float_as_uint(v.y);
+        r[4 * q + 2] = __float_as_uint(v.z);
+        r[4 * q + 3] = __float_as_uint(v.w);
+      }
+      for (int k = 0; k + 1 < n; ++k) {
+        if (k == mine) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(own[i]));
+        } else {
+          float4 v[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) v[q] = part(k, q);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) plus(r, q, v[q]);
+        }
       }
     }
   }
+
+ private:
+  static __device__ __forceinline__ void plus(uint32_t (&r)[32], int q, const float4& v) {
+    r[4 * q] = __float_as_uint(__uint_as_float(r[4 * q]) + v.x);
+    r[4 * q + 1] = __float_as_uint(__uint_as_float(r[4 * q + 1]) + v.y);
+    r[4 * q + 2] = __float_as_uint(__uint_as_float(r[4 * q + 2]) + v.z);
+    r[4 * q + 3] = __float_as_uint(__uint_as_float(r[4 * q + 3]) + v.w);
+  }
 };
+
+// One lane, once a warp's part is stored and fenced: whether it is the last of the tile's slices to arrive at `word`.  Whatever the
+// word held before this launch is not its token; the last to arrive clears it, since a replayed graph's token is the same.
+__device__ __forceinline__ bool split_arrive(unsigned long long* word, unsigned long long token, int slices) {
+  unsigned long long seen = *reinterpret_cast<volatile unsigned long long*>(word);
+  for (int i = 0; i < slices; ++i) {                   // a slice arrives once, so that no more than slices - 1 tries can fail
+    const unsigned long long next = (seen & ~kSplitCountMask) == token ? seen + 1 : token + 1;
+    const unsigned long long was = atomicCAS(word, seen, next);
+    if (was == seen) {
+      if (int(next & kSplitCountMask) != slices) return false;
+      *word = 0;
+      return true;
+    }
+    seen = was;
+  }
+  return false;
+}
 
 // The bias of N consecutive columns from col0 on, added to a thread's row.  Every lane reads the same 16 bytes.
 template <int N>
@@ -575,7 +626,7 @@ __device__ __forceinline__ int store_tile_whole(const Params& p, uint32_t stg, u
 // The 32 x 256 part of a tile that this warp's lanes hold in tensor memory at `src`: rows row0.. of C (p.M: the first row
 // that is not this tile's), rows y0.. of the tensor map.
 __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorMap* tmC, StoreStage& st, uint32_t src, int row0,
-                                                int y0, int n0, bool whole_rows, const Parts& parts = Parts{nullptr, 0, 0}) {
+                                                int y0, int n0, bool whole_rows, const Parts& parts = Parts{nullptr, 0, 0, 0}) {
   if (p.c_tma && whole_rows) {
     if (p.out_mode == kOutF32) {
       if (p.bias != nullptr) store_tile_tma<true, true>(p, tmC, st, src, row0, y0, n0, parts);
@@ -627,13 +678,11 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
     tile_coords(p, tile, tm, tn);
     const int row0 = tm * CM + int(rank) * BM + wq * 32;   // first of this warp's 32 rows
     const int n0 = tn * BN;
-    // a tail tile shared with other pairs: the last slice writes it, the others leave their parts
+    // a tail tile shared with other pairs: whichever of them is done last adds the parts and writes it
     const bool shared_tile = p.split_s > 1 && tile >= p.split_tail_begin;
     const int tail_idx = tile - p.split_tail_begin, warp8 = int(rank) * EPI_WARPS + wq;
-    const bool leaves_part = shared_tile && w.slice + 1 < p.split_s;
-    float* ws_tile = shared_tile ? p.split_ws + size_t(tail_idx) * (p.split_s - 1) * kSplitTileFloats : nullptr;
-    unsigned long long* flags = shared_tile ? p.split_flags + size_t(tail_idx) * (p.split_s - 1) * 8 + warp8 : nullptr;
-    const Parts parts{ws_tile, shared_tile && !leaves_part ? p.split_s - 1 : 0, warp8};
+    float* ws_tile = shared_tile ? p.split_ws + size_t(tail_idx) * p.split_s * kSplitTileFloats : nullptr;
+    const Parts parts{ws_tile, shared_tile ? p.split_s : 0, w.slice, warp8};
     if (!mbar_wait_warp(&s.tmem_full[acc], acc_phase, p.status, kTimeoutTmemFull, s.abort)) {
       *s.abort = 1;
       break;
@@ -641,7 +690,9 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
     tc_fence_after();
     const uint32_t src = tmem_base + lane_off + acc * BN;
     if (row0 < p.M) {   // warp-uniform, and the same for the slices of a tile
-      if (leaves_part) {
+      bool writes = true;
+      if (shared_tile) {
+        // Nobody waits for another pair, whatever the order in which the device runs them.
         float* dst = ws_tile + size_t(w.slice) * kSplitTileFloats;
 #pragma unroll 1
         for (int c = 0; c < BN / 32; ++c) {
@@ -655,36 +706,12 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
         }
         __threadfence();
         __syncwarp();
-        if (lane == 0) st_release_gpu(flags + w.slice * 8, p.split_token);
-      } else {
-        // this warp's rows of the other slices' parts: bounded wait, one lane polls.  They are slices of lower-numbered pairs,
-        // which the device starts first.
-        int landed = 1;
-        if (parts.n > 0 && lane == 0) {
-          for (int k = 0; landed && k < parts.n; ++k) {
-            const uint64_t t0 = globaltimer_ns();
-            while (ld_acquire_gpu(flags + k * 8) != p.split_token) {
-              if (*s.abort || globaltimer_ns() - t0 > kWaitLimitNs) {
-                set_status(p.status, kTimeoutPeerFlag);
-                landed = 0;
-                break;
-              }
-              __nanosleep(64);
-            }
-          }
-        }
-        landed = __shfl_sync(0xffffffffu, landed, 0);
-        __syncwarp();                     // what lane 0 has acquired is every lane's
-        if (!landed) {
-          *s.abort = 1;
-          break;
-        }
-        store_tile_part(p, tmC, st, src, row0, row0, n0, true, parts);
-        if (parts.n > 0) {
-          __syncwarp();
-          if (lane < parts.n) flags[lane * 8] = 0;    // the next launch's token is another one; a replayed graph's is not
-        }
+        int last = 0;
+        if (lane == 0) last = split_arrive(p.split_words + size_t(tail_idx) * 8 + warp8, p.split_token, p.split_s);
+        writes = __shfl_sync(0xffffffffu, last, 0) != 0;
+        __threadfence();                  // the other slices' parts are read after their arrivals
       }
+      if (writes) store_tile_part(p, tmC, st, src, row0, row0, n0, true, parts);
     }
     tc_fence_before();
     // the accumulator buffer is free again once all 256 epilogue threads of the pair have read it

@@ -66,15 +66,15 @@ struct Params {
   int groups;
   long long c_group_stride;
   // Optional split of the last, partly filled wave (CTA-pair kernel only): tiles from `split_tail_begin` on are each
-  // computed by `split_s` pairs, every pair taking a contiguous share of the k-blocks.  All but the last of them leave their
-  // fp32 partial tile in `split_ws` (256 x 256 floats per (tail tile, slice), in the order in which the epilogue's threads hold
-  // it), and each of their eight epilogue warps then writes `split_token` to its word of `split_flags` ([tail tile][slice][8]);
-  // the last slice's warps wait for the words of their own rows (bounded), add the parts in slice order, so that the result
-  // does not depend on timing, and clear the words.  split_s < 2: off.
+  // computed by `split_s` pairs, every pair taking a contiguous share of the k-blocks.  Each leaves its fp32 partial tile in
+  // `split_ws` (256 x 256 floats per (tail tile, slice), in the order in which the epilogue's threads hold it), and each of its
+  // eight epilogue warps then counts itself in at its word of `split_words` ([tail tile][8]).  The last warp to arrive at a
+  // word adds the parts of those rows in slice order, so that the result does not depend on timing, and writes them.
+  // split_s < 2: off.
   int split_s;
   int split_tail_begin;
   float* split_ws;
-  unsigned long long* split_flags;
+  unsigned long long* split_words;
   unsigned long long split_token;    // differs from launch to launch: whatever the words held before is not it
   int c_tma;                  // CTA-pair kernels: full blocks of C leave through the tensor map of C (plain 16-bit store)
 };
@@ -127,15 +127,6 @@ __device__ __forceinline__ int ld_acquire_gpu(const int* p) {
   int v;
   asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
-}
-
-__device__ __forceinline__ unsigned long long ld_acquire_gpu(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ __forceinline__ void st_release_gpu(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
 struct SmemLayout {

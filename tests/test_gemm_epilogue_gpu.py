@@ -119,3 +119,24 @@ def test_shared_tiles_of_the_last_wave(M, N, K, mode, a_mn, b_mn, biased):
     whole[1:M + 1, 4:4 + N] = 2.0
     assert (whole == 2.0).all()
     _lib.assert_healthy()
+
+
+# many slices a tile, every one of which may be the last: C is added to once, whoever does it, and the same bits each time
+@pytest.mark.parametrize("M,N,K", [(256, 256, 66000), (300, 300, 20000)])
+def test_shared_tiles_of_many_slices(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(K)
+    a, b = (torch.randn(n, K, device=DEV, generator=g).to(torch.bfloat16) for n in (M, N))
+    once = torch.zeros(M, N, device=DEV)
+    ops.gemm(a, b, out=once, out_mode=OUT_F32_ACC, pair=True)
+    ref = a.double() @ b.double().t()
+    assert torch.allclose(once.double(), ref, rtol=1e-6, atol=K / 16 * 2.0 ** -23 * 6 * K ** 0.5)   # as above
+    outs, streams = [torch.zeros(M, N, device=DEV) for _ in range(6)], [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+    for i, o in enumerate(outs):
+        with torch.cuda.stream(streams[i % 3]):
+            for _ in range(4):
+                o.zero_()
+                ops.gemm(a, b, out=o, out_mode=OUT_F32_ACC, pair=True)
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, once) for o in outs)
+    _lib.assert_healthy()

@@ -1,6 +1,9 @@
 """Which kernel a product goes to, on both sides of each line of the rules."""
+import re
+
 import pytest
 
+from hetu_galvatron_b200.csrc import build
 from hetu_galvatron_b200.ops.gemm import OUT_BF16, _use_grouped_pair, _use_skinny
 
 
@@ -17,3 +20,13 @@ def test_rule_of_the_few_row_kernel(M, N, K, few_rows):
                                              (4096, 255, 4096, 8, False), (512, 256, 4096, 1, True)])
 def test_rule_of_the_grouped_pair_kernel(rows, N, K, G, pair):
     assert _use_grouped_pair(rows, N, K, G) is pair
+
+
+def test_shared_tiles_wait_for_no_other_pair():
+    """Nothing says in which order the device starts the pairs that share a tile: no warp of one may wait for another."""
+    text = (build.CSRC / "sm100" / "gemm2_core.cuh").read_text()
+    body = text.split("void epilogue2(", 1)[1]
+    for name in ("split_arrive", "add"):
+        body += text.split(" %s(" % name, 1)[1].split("\n}\n", 1)[0]
+    body = re.sub(r"//.*", "", body)
+    assert "split_token" in body and not re.findall(r"\bwhile\b|ld_acquire|__nanosleep", body)
