@@ -423,7 +423,7 @@ int launch_stream(const DecodeParams& p, int settled, cudaStream_t st) {
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = hg_host::chain_overlaps() ? 2 : 1;
-  return int(cudaLaunchKernelEx(&cfg, k, p, settled));
+  return hg_host::launched(cudaLaunchKernelEx(&cfg, k, p, settled));
 }
 
 inline int keys_seen(int Sq, int Skv, int causal, int q_pos0, int k_pos0) {

@@ -376,7 +376,7 @@ static int launch_grouped2(const CUtensorMap& ta, const CUtensorMap& tb, const C
   if (int rc = pair_config(k, &cfg, attr, &max_pairs, hg_host::launch_overlaps(), st)) return rc;
   const int pairs = want_pairs < max_pairs ? want_pairs : max_pairs;
   cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
-  return int(cudaLaunchKernelEx(&cfg, k, ta, tb, tc, p, tiles));
+  return hg_host::launched(cudaLaunchKernelEx(&cfg, k, ta, tb, tc, p, tiles));
 }
 
 template <bool A_MN, bool B_MN>
@@ -404,8 +404,7 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
     }
   }
   cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, k, ta, tb, tc, p);
-  return int(e);
+  return hg_host::launched(cudaLaunchKernelEx(&cfg, k, ta, tb, tc, p));
 }
 
 // The tensor map of C for the plain stores (p.c_tma says whether it is used; `any` fills the kernel's parameter else).

@@ -322,7 +322,7 @@ int launch_skinny(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyPara
   cfg.stream = st;
   cfg.attrs = attr;
   cfg.numAttrs = hg_host::chain_overlaps() ? 2 : 1;
-  return int(cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<W_MN, NT>, tw, tx, p));
+  return hg_host::launched(cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<W_MN, NT>, tw, tx, p));
 }
 
 template <bool W_MN>

@@ -461,6 +461,13 @@ bool chain_overlaps();
 // with 32 heads of 128, 1443 us without and 1466 with.
 bool launch_overlaps();
 
+// What a launch returned.  An error is the caller's to report: the runtime must not keep it for whoever asks next
+// (cudaGetLastError after another kernel's launch, here or in the tensor library).
+inline int launched(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return int(e);
+}
+
 template <typename... P, typename... A>
 inline int launch_kernel(bool overlaps, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg = {};
@@ -475,7 +482,7 @@ inline int launch_kernel(bool overlaps, void (*kernel)(P...), dim3 grid, dim3 bl
     cfg.attrs = attr;
     cfg.numAttrs = 1;
   }
-  return int(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+  return launched(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
 }
 template <typename K, typename... A>
 inline int launch(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {

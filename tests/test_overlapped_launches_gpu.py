@@ -96,3 +96,16 @@ def test_rotation_tables_written_in_front(interleaved):
     for s, t in zip(run(False), run(True), strict=True):
         assert torch.equal(s, t)
     _lib.assert_healthy()
+
+
+def test_a_refused_launch_leaves_no_error_behind():
+    """More sequences than a grid has layers: the host refuses the launch, and the next call knows nothing of it."""
+    q = torch.zeros(2, 65536, 1, 64, device=DEV, dtype=LP)
+    x, y = torch.ones(64, device=DEV), torch.empty(64, device=DEV, dtype=LP)
+    with pytest.raises(_lib.KernelError):
+        ops.flash_attention(q, q, q, causal=False)
+    assert _lib.load().hg_cast_f32_bf16(x.data_ptr(), y.data_ptr(), 64, _lib.stream()) == 0
+    with pytest.raises(_lib.KernelError):
+        ops.flash_attention(q, q, q, causal=False)
+    assert torch.equal(x + 1, torch.full_like(x, 2.0)) and torch.equal(y.float(), x)
+    _lib.assert_healthy()
