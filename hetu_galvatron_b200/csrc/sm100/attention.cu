@@ -1224,9 +1224,11 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   // head dim 64: dS^T is formed from fp32 probabilities, as in the 64-query kernel
   constexpr bool kExactP = HD == 64;
   constexpr int CPT = 128 / NWG;               // query columns per thread and step
-  // Works on further blocks of the grid (WorkSlot) where a block is short: 1600 blocks of 8 x 1024 tokens and 25 heads of 64
-  // 156 -> 144 us.  The 2048 blocks of 2 x 4096 tokens and 32 heads of 128 gain less than the running counters cost: 535 -> 542.
-  constexpr bool kTakesMore = HD == 64;
+  // A CTA works on further blocks of the grid (WorkSlot).  Whole backward, us, one block a CTA / so, causal: head dim 64, 16 x 256
+  // tokens and 25 heads 94 / 78, 8 x 1024 283 / 250, 4 x 2048 418 / 383, 1 x 8192 1205 / 1151, 12 heads 4096 210 / 203, 8192 634 /
+  // 608, 32 heads on 8 4 x 2048 525 / 491; head dim 128, 32 heads 16 x 256 168 / 138, 8 x 1024 433 / 389, 4 x 2048 610 / 574,
+  // 2 x 4096 967 / 949, 1 x 8192 1689 / 1688, 28 on 4 8 x 1024 360 / 341.  A grid of one wave pays: 12 heads of 64, 300 tokens
+  // 23.1 / 23.5.
   extern __shared__ uint8_t smem_raw[];
   using L = Dkv128Smem<HD>;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1331,15 +1333,8 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     bool ok = true, asked = false;
     for (; ok; ++n) {
       asked = false;
-      auto ask = [&]() {                             // for the next block, once every warp has taken this one
-        if (!kTakesMore || asked || (n > 0 && !mbar_test_warp(work.empty, (n - 1) & 1))) return;
-        if (issuer) work_request(work);
-        __syncwarp();
-        asked = true;
-      };
       const Steps t = steps_of(blk);
       const int kslot = p.kmap.slot(t.h0, p.qpg), vslot = p.vmap.slot(t.h0, p.qpg), b = t.b;
-      ask();
       if (t.n_it > 0) {
         if (!mbar_wait_warp(kv_empty, (nkv & 1) ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
         ++nkv;
@@ -1366,14 +1361,15 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           if (++qs_slot == NQ) { qs_slot = 0; qph ^= 1; }
           if (++ds_slot == ND) { ds_slot = 0; dph ^= 1; }
           if (++qs == n_qs) { qs = t.qs0; ++h; }
-          ask();
         }
       }
-      if (!ok || !kTakesMore) break;
-      if (!asked) {
-        if (!mbar_wait_warp(work.empty, (n - 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
-        ask();
-      }
+      if (!ok) break;
+      // The next block is asked for once this one's loads are all on their way.  Asked for earlier it waits for a CTA that is busy
+      // while others run dry (12 heads of 64, 4096 tokens: 203 -> 233 us).  The answer slot is free once every warp has this block.
+      if (n > 0 && !mbar_wait_warp(work.empty, (n - 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+      if (issuer) work_request(work);
+      __syncwarp();
+      asked = true;
       if (!work_take(work, n, blk, p.status, abort_flag)) break;
     }
     if (!ok) {
@@ -1482,7 +1478,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       __syncwarp();
       ++nkv;
       }
-      if (!kTakesMore || (ok && !work_take(work, n, blk, p.status, abort_flag))) break;
+      if (ok && !work_take(work, n, blk, p.status, abort_flag)) break;
       }
       if (!ok) *abort_flag = 1;
   } else {
@@ -1686,7 +1682,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     } else {
       ok = false;
     }
-    if (!kTakesMore || (ok && !work_take(work, n, blk, p.status, abort_flag))) break;
+    if (ok && !work_take(work, n, blk, p.status, abort_flag)) break;
     }
     if (!ok) *abort_flag = 1;
   }
@@ -1756,8 +1752,6 @@ __global__ void __launch_bounds__(64 + 128 * NWG, 1)
 flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                        const BwdParams p) {
-  // As in the dK/dV kernel: 8 x 1024 tokens, 25 heads of 64 106 -> 91 us; 2 x 4096, 32 heads of 128 399 -> 403.
-  constexpr bool kTakesMore = HD == 64;
   extern __shared__ uint8_t smem_raw[];
   using L = Dq128Smem<HD>;
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -1836,16 +1830,9 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     bool ok = true, asked = false;
     for (; ok; ++n) {
       asked = false;
-      auto ask = [&]() {                             // for the next block, once every warp has taken this one
-        if (!kTakesMore || asked || (n > 0 && !mbar_test_warp(work.empty, (n - 1) & 1))) return;
-        if (issuer) work_request(work);
-        __syncwarp();
-        asked = true;
-      };
       const int q0 = query_row(blk), h = blk.y, b = blk.z, n_it = steps_of(blk);
       const int qslot = p.qmap.slot(h, p.qpg), kslot = p.kmap.slot(h, p.qpg), vslot = p.vmap.slot(h, p.qpg),
                 doslot = p.domap.slot(h, p.qpg);
-      ask();
       if (n_it > 0) {
         if (!mbar_wait_warp(qdo_empty, (nq & 1) ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
         ++nq;
@@ -1868,14 +1855,15 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
             if (issuer) tma_load_4d(sV + c * 128 * 128, &tmV, v_full, c * 64, vslot, it * 128, b);
           if (++ks == NK) { ks = 0; kph ^= 1; }
           vph ^= 1;
-          ask();
         }
       }
-      if (!ok || !kTakesMore) break;
-      if (!asked) {
-        if (!mbar_wait_warp(work.empty, (n - 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
-        ask();
-      }
+      if (!ok) break;
+      // The next block is asked for once this one's loads are all on their way.  Asked for earlier it waits for a CTA that is busy
+      // while others run dry (12 heads of 64, 4096 tokens: 203 -> 233 us).  The answer slot is free once every warp has this block.
+      if (n > 0 && !mbar_wait_warp(work.empty, (n - 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+      if (issuer) work_request(work);
+      __syncwarp();
+      asked = true;
       if (!work_take(work, n, blk, p.status, abort_flag)) break;
     }
     if (!ok) {
@@ -1951,7 +1939,7 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       HG_DKV_REPORT(32, n_it, tm_s, tm_wait_ds, tm_dq, tm_unused);
       ++nq;
       }
-      if (!kTakesMore || (ok && !work_take(work, n, blk, p.status, abort_flag))) break;
+      if (ok && !work_take(work, n, blk, p.status, abort_flag)) break;
       }
       if (!ok) *abort_flag = 1;
   } else {
@@ -2058,7 +2046,7 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     } else {
       ok = false;
     }
-    if (!kTakesMore || (ok && !work_take(work, n, blk, p.status, abort_flag))) break;
+    if (ok && !work_take(work, n, blk, p.status, abort_flag)) break;
     }
     if (!ok) *abort_flag = 1;
   }

@@ -155,21 +155,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
   return false;
 }
 
-// Whether the phase is over, without waiting; the same answer for the whole warp.
-__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.b32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return __all_sync(0xffffffffu, ok != 0);
-}
-
 // Warp-collective bounded wait: every lane waits, the verdict is made uniform so that the warp never
 // diverges around the .sync.aligned tcgen05 instructions that follow.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* status, int code,
