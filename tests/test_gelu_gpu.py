@@ -46,3 +46,16 @@ def test_every_argument():
     got = ops.activation(special.view(1, 8), "gelu")[0].tolist()
     assert got[0] == float("inf") and got[1] != got[1] and got[2] == 0.0 and got[3] == 0.0
     _lib.assert_healthy()
+
+
+@pytest.mark.parametrize("kind", ["gelu", "geglu"])
+def test_gradient_of_the_largest_arguments(kind):
+    """The gradient is that of a step, 0 below and 1 above, up to where 0.107 x * x overflows."""
+    y = torch.arange(-32768, 32768, device=DEV, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    y = y[(y.double().abs() >= 1e18) & (y.double().abs() <= (3.4e38 / 0.10704) ** 0.5)]
+    y = y[: y.numel() // 8 * 8].view(-1, 8)
+    x = (torch.cat([y, torch.ones_like(y)], 1) if kind == "geglu" else y.clone()).requires_grad_()
+    out = ops.activation(x, kind)
+    out.backward(torch.ones_like(out))
+    assert torch.equal(x.grad[:, :8], (y > 0).to(y.dtype)) and torch.equal(out, torch.where(y > 0, y, torch.zeros_like(y)))
+    _lib.assert_healthy()
