@@ -107,6 +107,7 @@ def _build_cuda_variant(obj_dir: Path, lib_name: str, extra_flags, verbose: bool
 
 
 def build_host(verbose: bool = False):
+    """The modules that need neither CUDA nor torch: the search's dynamic program and the dataset index builders."""
     import pybind11
 
     LIB_DIR.mkdir(exist_ok=True)
@@ -123,7 +124,6 @@ def build_host(verbose: bool = False):
             if verbose:
                 print("[build] g++", src)
         out.append(target)
-    out.append(build_torch_ops(verbose))
     return out
 
 
@@ -146,7 +146,7 @@ def build_torch_ops(verbose: bool = False) -> Path:
 
 
 def build_all(verbose: bool = False, variants: bool = True):
-    host = build_host(verbose)
+    host = [*build_host(verbose), build_torch_ops(verbose)]
     cuda = build_cuda(verbose)
     out = [cuda, *host]
     if variants:
