@@ -12,6 +12,8 @@ without a GPU, so the build also serves as the "does it compile" check on a CPU-
 """
 from __future__ import annotations
 
+import contextlib
+import fcntl
 import os
 import shutil
 import subprocess
@@ -57,6 +59,27 @@ def _run(cmd, log: Path | None = None):
     return proc
 
 
+def _produce(cmd, target: Path, log: Path | None = None):
+    """Run a compiler whose output is ``target``.  The file appears whole or not at all: other processes may be loading it."""
+    part = target.with_name(".%s.%d" % (target.name, os.getpid()))
+    try:
+        _run([*cmd, "-o", str(part)], log)
+        os.replace(part, target)
+    finally:
+        part.unlink(missing_ok=True)
+
+
+@contextlib.contextmanager
+def _one_builder():
+    """The ranks of a job that start without the native code build it once: the first one does, the others wait and find it.
+    A tree that cannot be written to has no lock, and nothing is built there."""
+    with contextlib.ExitStack() as stack:
+        with contextlib.suppress(OSError):
+            OBJ_DIR.mkdir(exist_ok=True)
+            fcntl.flock(stack.enter_context(open(OBJ_DIR / ".lock", "w")), fcntl.LOCK_EX)
+        yield
+
+
 def build_cuda(verbose: bool = False, jobs: int | None = None, debug: bool = False, half: bool = False) -> Path:
     """The kernel library, or one of its variants built from the same sources:
 
@@ -66,18 +89,18 @@ def build_cuda(verbose: bool = False, jobs: int | None = None, debug: bool = Fal
       see ``hg_lp_t`` in sm100_common.cuh), loaded for ``mixed_precision: fp16`` models."""
     if debug and half:
         raise ValueError("one variant at a time")
-    if debug:
-        return _build_cuda_variant(OBJ_DIR / "debug", "libhg_sm100_debug.so", ["-DHG_DEBUG_BOUNDS=1"], verbose, jobs)
-    if half:
-        return _build_cuda_variant(OBJ_DIR / "fp16", "libhg_sm100_fp16.so", ["-DHG_HALF=1"], verbose, jobs)
-    return _build_cuda_variant(OBJ_DIR, "libhg_sm100.so", [], verbose, jobs)
+    with _one_builder():
+        if debug:
+            return _build_cuda_variant(OBJ_DIR / "debug", "libhg_sm100_debug.so", ["-DHG_DEBUG_BOUNDS=1"], verbose, jobs)
+        if half:
+            return _build_cuda_variant(OBJ_DIR / "fp16", "libhg_sm100_fp16.so", ["-DHG_HALF=1"], verbose, jobs)
+        return _build_cuda_variant(OBJ_DIR, "libhg_sm100.so", [], verbose, jobs)
 
 
 def _build_cuda_variant(obj_dir: Path, lib_name: str, extra_flags, verbose: bool, jobs) -> Path:
     src_dir = CSRC / "sm100"
     sources = sorted(src_dir.glob("*.cu"))
     headers = sorted(src_dir.glob("*.cuh")) + sorted(src_dir.glob("*.h"))
-    OBJ_DIR.mkdir(exist_ok=True)
     obj_dir.mkdir(exist_ok=True)
     LIB_DIR.mkdir(exist_ok=True)
     nvcc = _nvcc()
@@ -91,8 +114,7 @@ def _build_cuda_variant(obj_dir: Path, lib_name: str, extra_flags, verbose: bool
 
     def compile_one(pair):
         s, o = pair
-        _run([nvcc, *NVCC_FLAGS, *extra_flags, "-I", str(src_dir), "-c", str(s), "-o", str(o)],
-             log=obj_dir / (s.stem + ".log"))
+        _produce([nvcc, *NVCC_FLAGS, *extra_flags, "-I", str(src_dir), "-c", str(s)], o, log=obj_dir / (s.stem + ".log"))
         if verbose:
             print("[build] nvcc", s.name)
 
@@ -100,7 +122,7 @@ def _build_cuda_variant(obj_dir: Path, lib_name: str, extra_flags, verbose: bool
         list(ex.map(compile_one, todo))
     lib = LIB_DIR / lib_name
     if todo or _newer(objs, lib):
-        _run([nvcc, "-shared", "-o", str(lib), *map(str, objs), "-lcudart"])
+        _produce([nvcc, "-shared", *map(str, objs), "-lcudart"], lib)
         if verbose:
             print("[build] link", lib.name)
     return lib
@@ -114,16 +136,17 @@ def build_host(verbose: bool = False):
     ext = sysconfig.get_config_var("EXT_SUFFIX")
     inc = ["-I", pybind11.get_include(), "-I", sysconfig.get_paths()["include"]]
     out = []
-    for name, src in (("hg_dp_core", "dp_core.cpp"), ("hg_dataset_helpers", "dataset_helpers.cpp")):
-        s = CSRC / "host" / src
-        if not s.exists():
-            continue
-        target = LIB_DIR / (name + ext)
-        if _newer([s], target):
-            _run(["g++", "-O3", "-std=c++17", "-shared", "-fPIC", "-pthread", *inc, str(s), "-o", str(target)])
-            if verbose:
-                print("[build] g++", src)
-        out.append(target)
+    with _one_builder():
+        for name, src in (("hg_dp_core", "dp_core.cpp"), ("hg_dataset_helpers", "dataset_helpers.cpp")):
+            s = CSRC / "host" / src
+            if not s.exists():
+                continue
+            target = LIB_DIR / (name + ext)
+            if _newer([s], target):
+                _produce(["g++", "-O3", "-std=c++17", "-shared", "-fPIC", "-pthread", *inc, str(s)], target)
+                if verbose:
+                    print("[build] g++", src)
+            out.append(target)
     return out
 
 
@@ -133,15 +156,16 @@ def build_torch_ops(verbose: bool = False) -> Path:
 
     s = CSRC / "host" / "torch_ops.cpp"
     target = LIB_DIR / ("hg_torch_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
-    if _newer([s, *(CSRC / "sm100" / h for h in ("attn_tensor.h", "decoder_step.h"))], target):
-        LIB_DIR.mkdir(exist_ok=True)
-        cuda = Path(_nvcc()).resolve().parent.parent / "include"
-        inc = [f for p in (*include_paths(), str(cuda), sysconfig.get_paths()["include"]) for f in ("-I", p)]
-        libs = ["-L" + p for p in library_paths()]
-        _run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=hg_torch_ops", *inc, str(s), "-o",
-              str(target), *libs, "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda"])
-        if verbose:
-            print("[build] g++", s.name)
+    with _one_builder():
+        if _newer([s, *(CSRC / "sm100" / h for h in ("attn_tensor.h", "decoder_step.h"))], target):
+            LIB_DIR.mkdir(exist_ok=True)
+            cuda = Path(_nvcc()).resolve().parent.parent / "include"
+            inc = [f for p in (*include_paths(), str(cuda), sysconfig.get_paths()["include"]) for f in ("-I", p)]
+            libs = ["-L" + p for p in library_paths()]
+            _produce(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=hg_torch_ops", *inc, str(s), *libs,
+                      "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda"], target)
+            if verbose:
+                print("[build] g++", s.name)
     return target
 
 
