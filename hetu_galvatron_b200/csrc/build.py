@@ -15,6 +15,7 @@ from __future__ import annotations
 import contextlib
 import fcntl
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -150,20 +151,42 @@ def build_host(verbose: bool = False):
     return out
 
 
+def _torch_ops() -> Path:
+    return LIB_DIR / ("hg_torch_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def _torch_ops_mark(interface: int) -> str:
+    import torch
+
+    return "torch %s, interface %d" % (torch.__version__, interface)
+
+
+def torch_ops_current(interface: int, unmarked: bool = False) -> bool:
+    """Whether the module that is there was built against this interpreter's torch and for this version of the kernel library's
+    entry points (``native_interface.h``); ``unmarked``: the answer for one that nothing is known about."""
+    mark = _torch_ops().with_suffix(".stamp")
+    if not _torch_ops().exists():
+        return False
+    return mark.read_text() == _torch_ops_mark(interface) if mark.exists() else unmarked
+
+
 def build_torch_ops(verbose: bool = False) -> Path:
     """``hg_torch_ops``: the autograd nodes of the layers' operations, against this interpreter's torch."""
     from torch.utils.cpp_extension import include_paths, library_paths
 
     s = CSRC / "host" / "torch_ops.cpp"
-    target = LIB_DIR / ("hg_torch_ops" + sysconfig.get_config_var("EXT_SUFFIX"))
+    headers = [CSRC / "sm100" / h for h in ("attn_tensor.h", "decoder_step.h", "native_interface.h")]
+    interface = int(re.search(r"kHgNativeInterface = (\d+)", headers[-1].read_text()).group(1))
+    target = _torch_ops()
     with _one_builder():
-        if _newer([s, *(CSRC / "sm100" / h for h in ("attn_tensor.h", "decoder_step.h"))], target):
+        if _newer([s, *headers], target) or not torch_ops_current(interface):
             LIB_DIR.mkdir(exist_ok=True)
             cuda = Path(_nvcc()).resolve().parent.parent / "include"
             inc = [f for p in (*include_paths(), str(cuda), sysconfig.get_paths()["include"]) for f in ("-I", p)]
             libs = ["-L" + p for p in library_paths()]
             _produce(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-DTORCH_EXTENSION_NAME=hg_torch_ops", *inc, str(s), *libs,
                       "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda"], target)
+            target.with_suffix(".stamp").write_text(_torch_ops_mark(interface))
             if verbose:
                 print("[build] g++", s.name)
     return target

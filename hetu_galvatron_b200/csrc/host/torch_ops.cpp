@@ -25,6 +25,7 @@
 
 #include "../sm100/attn_tensor.h"
 #include "../sm100/decoder_step.h"
+#include "../sm100/native_interface.h"
 
 namespace {
 
@@ -687,6 +688,7 @@ PyMethodDef kMethods[] = {HG_METHOD("linear", py_linear),
 }  // namespace
 
 PYBIND11_MODULE(hg_torch_ops, m) {
+  m.attr("interface") = kHgNativeInterface;
   m.def("bind", &bind);
   m.def("launches", [] { return g_launches.load(); });
   m.def("reset_launches", [] { g_launches = 0; });

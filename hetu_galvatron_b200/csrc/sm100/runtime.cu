@@ -4,6 +4,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "native_interface.h"
 #include "sm100_common.cuh"
 
 namespace hg_host {
@@ -199,5 +200,6 @@ int hg_read_status(int clear) {
 void* hg_status_address() { return hg_host::status_ptr(); }
 
 int hg_library_version() { return 100; }
+int hg_native_interface() { return kHgNativeInterface; }
 
 }  // extern "C"

@@ -144,6 +144,7 @@ _SIGNATURES = {
     "hg_read_status": [c_int],
     "hg_gemm_gated_selftest": [c_void_p],
     "hg_library_version": [],
+    "hg_native_interface": [],
 }
 
 
@@ -195,10 +196,16 @@ def _bind_native(lib):
     try:
         from ..csrc import build as _build
 
-        if os.environ.get("HG_AUTOBUILD", "1") == "1" and not list(_LIB_DIR.glob("hg_torch_ops*.so")):
+        interface, autobuild = lib.hg_native_interface(), os.environ.get("HG_AUTOBUILD", "1") == "1"
+        if not _build.torch_ops_current(interface, unmarked=not autobuild):
+            if not autobuild:
+                raise RuntimeError("built for another torch or kernel library")
             _build.build_torch_ops()
         from .._lib import hg_torch_ops
-    except Exception as e:  # noqa: BLE001  (no compiler, another torch)
+
+        if getattr(hg_torch_ops, "interface", None) != interface:
+            raise RuntimeError("its calls are not those of the kernel library")
+    except Exception as e:  # noqa: BLE001  (no compiler, another torch, another version of the library)
         import warnings
 
         warnings.warn("hg_torch_ops is not usable (%s): autograd nodes run in Python" % (e,))

@@ -1,9 +1,12 @@
 """The in-tree build (csrc/build.py): what it needs, and what other processes see of it while it runs."""
+import re
 import threading
 import time
+import zlib
 from pathlib import Path
 
 import pytest
+import torch
 
 from hetu_galvatron_b200.csrc import build
 
@@ -60,3 +63,41 @@ def test_a_built_tree_that_cannot_be_written_to(tree, monkeypatch):
     build.build_host()
     monkeypatch.setattr(build, "OBJ_DIR", tree[0] / "nowhere" / "build")
     assert len(build.build_host()) == 2 and len(tree[1]) == 2
+
+
+def test_autograd_nodes_of_another_build_are_built_again(tree, monkeypatch):
+    torch_ops = build.build_torch_ops()
+    version = int(re.search(r"kHgNativeInterface = (\d+)", (build.CSRC / "sm100" / "native_interface.h").read_text()).group(1))
+    assert build.torch_ops_current(version) and not build.torch_ops_current(version + 1)
+    build.build_torch_ops()
+    assert len(tree[1]) == 1
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + "x")                 # another torch
+    assert not build.torch_ops_current(version)
+    build.build_torch_ops()
+    assert len(tree[1]) == 2 and build.torch_ops_current(version)
+    torch_ops.rename(torch_ops.with_name("hg_torch_ops.cpython-00-elsewhere.so"))      # another interpreter
+    assert not build.torch_ops_current(version, unmarked=True)
+
+
+# Raise kHgNativeInterface with any change that turns up here, and note the new sum beside it.
+INTERFACES = {1: 633082835}
+
+
+def test_entry_points_that_the_nodes_call_by_address():
+    """Their argument lists are those of the library, and a change of them is a new version of the interface."""
+    def kinds(params):
+        return "".join("p" if "*" in p or re.match(r"\s*[VA]\b", p) else {"int": "i", "long long": "l", "float": "f"}[
+            re.match(r"\s*(int|long long|float)\b", p).group(1)] for p in params.split(","))
+
+    nodes = (build.CSRC / "host" / "torch_ops.cpp").read_text()
+    kernels = "".join(p.read_text() for p in sorted((build.CSRC / "sm100").glob("*.cu")))
+    slots = dict(re.findall(r"\(\*(\w+)\)\(([^)]*)\);", nodes.split("struct Kernels {")[1].split("};")[0]))
+    called = []
+    for name, slot in re.findall(r'at\("(hg_\w+)", K\.(\w+)\)', nodes):
+        params = re.search(r"\b%s\(([^)]*)\)\s*\{" % name, kernels).group(1)
+        assert kinds(params) == kinds(slots[slot]), name
+        called.append(name + ":" + kinds(params))
+    assert len(called) == len(slots)
+    structs = [re.sub(r"//.*|\s+", " ", (build.CSRC / "sm100" / h).read_text()) for h in ("attn_tensor.h", "decoder_step.h")]
+    version = int(re.search(r"kHgNativeInterface = (\d+)", (build.CSRC / "sm100" / "native_interface.h").read_text()).group(1))
+    assert INTERFACES[version] == zlib.crc32(" ".join(sorted(called) + structs).encode())
