@@ -202,3 +202,35 @@ def test_weights_written_just_before_a_step_are_the_ones_it_reads():
         m.attn.attention.inference_context = None
     assert torch.equal(got[0], got[1])
     _lib.assert_healthy()
+
+
+def test_norm_weights_and_biases_written_just_before_a_step():
+    """As above for every vector of a layer, the first norm's weight and bias last, against the modules after a wait."""
+    torch.manual_seed(8)
+    m = layer("LayerNorm", "gelu", "none", True, 8, 8, 128)
+    x = torch.randn(1, 4, 1024, device=DEV).to(torch.bfloat16)
+    n1 = m.attn.input_layernorm
+    vectors = sorted((p for p in m.parameters() if p.dim() == 1), key=lambda p: p is n1.weight or p is n1.bias)
+    assert len(vectors) == 8 and vectors[-1] is n1.bias
+    new = [torch.randn_like(p) for p in vectors]
+    got = []
+    for hooked in (False, True):
+        ic = StaticInferenceContext(4, 8)
+        m.attn.attention.inference_context = ic
+        with torch.no_grad():
+            for p in vectors:
+                p.zero_()
+            m(x)                                          # fills position 0
+            ic.sequence_len_offset = 1
+            h = m.ffn.mlp.register_forward_hook(lambda *_: None) if hooked else None
+            torch.cuda._sleep(1000000)
+            for p, v in zip(vectors, new):
+                p.copy_(v)
+            if hooked:
+                torch.cuda.synchronize()
+            got.append(m(x))
+        if h is not None:
+            h.remove()
+        m.attn.attention.inference_context = None
+    assert torch.equal(got[0], got[1]) and got[0].abs().sum() > 0
+    _lib.assert_healthy()

@@ -109,3 +109,24 @@ def test_a_refused_launch_leaves_no_error_behind():
         ops.flash_attention(q, q, q, causal=False)
     assert torch.equal(x + 1, torch.full_like(x, 2.0)) and torch.equal(y.float(), x)
     _lib.assert_healthy()
+
+
+# a product's weight, and then its bias, are the results of such a kernel: the CTA-pair and the few-row kernel
+@pytest.mark.parametrize("rows,K,N", [(300, 512, 1000), (2049, 1600, 6400), (4, 4096, 4096)])
+def test_weights_and_biases_written_by_the_kernel_in_front(rows, K, N):
+    torch.manual_seed(rows)
+    x, (w1, w2), (b1, b2) = (torch.randn(*s, device=DEV).to(LP) for s in ((rows, K), (2, N, K), (2, N)))
+    w, b = ops_add(w1, w2), ops_add(b1, b2)
+    want = ops.linear(x, w, b)
+    for first in ("weight", "bias"):
+        for _ in range(3):
+            del w, b
+            torch.zeros(N, K, device=DEV, dtype=LP), torch.zeros(N, device=DEV, dtype=LP)      # the memory of the next results
+            torch.cuda.synchronize()
+            torch.cuda._sleep(500000)
+            if first == "weight":
+                w, b = ops_add(w1, w2), ops_add(b1, b2)
+            else:
+                b, w = ops_add(b1, b2), ops_add(w1, w2)
+            assert torch.equal(ops.linear(x, w, b), want)
+    _lib.assert_healthy()
