@@ -274,12 +274,12 @@ __device__ __forceinline__ void mma2(const Params& p, const Smem2& s, uint32_t t
 // Epilogue.  tcgen05.ld hands every thread one accumulator ROW (32 consecutive columns), but a row per thread is the
 // wrong shape for global memory, so each warp turns its blocks through shared memory.
 //
-// Plain 16-bit stores: 32 rows x 128 bytes are written to the warp's stage in the layout of the 128-byte
+// Plain 16-bit and fp32 stores: 32 rows x 128 bytes are written to the warp's stage in the layout of the 128-byte
 // swizzle, eight conflict-free 16-byte stores per thread, and leave as one TMA store that clips at the matrix' edges;
 // two blocks alternate, so that one is filled while the other is read.
-// fp32 results and accumulating modes: a 32 x 32 fp32 block at a time through 36-word rows (conflict-free 16-byte
-// accesses both ways), eight lanes on 32 consecutive columns of a row, four elements each, all loads of a block before its
-// first store.  (fp32 results by TMA store were slower: expert weight gradients 4.14 against 3.13 ms.)
+// Accumulating modes, a C that no tensor map covers and the ragged end of an expert's rows: a 32 x 32 fp32 block at a time
+// through 36-word rows (conflict-free 16-byte accesses both ways), eight lanes on 32 consecutive columns of a row, four
+// elements each, all loads of a block before its first store.
 //
 // What an epilogue costs is instructions, not bytes, and every decision that can be taken once per tile is taken there:
 // whether there is a bias, the output mode, whole or clipped blocks.  Decided per element they were 64 branches around

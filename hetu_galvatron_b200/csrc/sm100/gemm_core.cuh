@@ -76,7 +76,7 @@ struct Params {
   float* split_ws;
   unsigned long long* split_words;
   unsigned long long split_token;    // differs from launch to launch: whatever the words held before is not it
-  int c_tma;                  // CTA-pair kernels: full blocks of C leave through the tensor map of C (plain 16-bit store)
+  int c_tma;                  // CTA-pair kernels: full blocks of C leave through the tensor map of C (plain 16-bit and fp32 stores)
 };
 
 struct TileInfo {

@@ -403,7 +403,8 @@ __device__ __forceinline__ void work_drain(const WorkSlot& s, int k) {
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Returns 0, and has to be added to every `__restrict__` pointer that is read afterwards: such a pointer promises that no one
-// else writes behind it, so that without the dependence the compiler may read it before the wait.
+// else writes behind it, so that without the dependence the compiler may read it before the wait.  A load through the read-only
+// path (__ldg) makes the same promise for itself and has no place behind a wait.
 __device__ __forceinline__ int chain_wait() {
   int zero;
   asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(zero)::"memory");
