@@ -16,8 +16,8 @@
 // its own limit, and both still meet at the final cluster barrier and free their tensor memory.
 // No operand load uses cluster multicast: each CTA loads exactly the bytes it alone needs.
 #include <atomic>
+#include <chrono>
 #include <cstdlib>
-#include <random>
 
 #include "gemm2_core.cuh"
 
@@ -327,9 +327,11 @@ SplitPlan split_plan(int tiles, int num_kb, int max_pairs) {
   return p;
 }
 
+// Starts at the clock: no launch of this process has the token of another, and nothing here can throw at a C entry.
 unsigned long long split_token() {
   constexpr unsigned long long kStep = kSplitCountMask + 1;
-  static std::atomic<unsigned long long> next{((unsigned long long)std::random_device{}() << 32) | kStep};
+  static std::atomic<unsigned long long> next{
+      (unsigned long long)std::chrono::system_clock::now().time_since_epoch().count() * kStep + kStep};
   return next.fetch_add(kStep, std::memory_order_relaxed);
 }
 

@@ -30,3 +30,9 @@ def test_shared_tiles_wait_for_no_other_pair():
         body += text.split(" %s(" % name, 1)[1].split("\n}\n", 1)[0]
     body = re.sub(r"//.*", "", body)
     assert "split_token" in body and not re.findall(r"\bwhile\b|ld_acquire|__nanosleep", body)
+
+
+def test_nothing_throws_at_the_entry_points():
+    """They are called from C: std::random_device raises where the system has no source of entropy."""
+    for path in (build.CSRC / "sm100").glob("*.cu*"):
+        assert not re.search(r"random_device|\bthrow\b|\.at\(", re.sub(r"//.*", "", path.read_text())), path.name
