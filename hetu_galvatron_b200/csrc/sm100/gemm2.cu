@@ -18,6 +18,7 @@
 #include <atomic>
 #include <chrono>
 #include <cstdlib>
+#include <utility>
 
 #include "gemm2_core.cuh"
 
@@ -285,7 +286,7 @@ using namespace hg::gemm2;
 
 namespace {
 
-// HG_GEMM_SPLIT_TAIL: 0 never, 1 wherever a slice keeps eight k-blocks, unset: by the rule of split_plan.
+// HG_GEMM_SPLIT_TAIL: 0 never, 1 wherever a slice keeps eight k-blocks, unset: by the cost of the plan.
 int split_mode() {
   static const int mode = [] {
     const char* e = getenv("HG_GEMM_SPLIT_TAIL");
@@ -294,37 +295,93 @@ int split_mode() {
   return mode;
 }
 
-// What a split costs, in k-blocks (0.3 us each): the parts' way to L2 and the arrivals, and each part that is added.
-constexpr int kSplitCost = 24, kPartCost = 8;
-
-struct SplitPlan {
-  int s, tail;                       // pairs per tail tile (0: no split), tail tiles
+// How a product is cut: columns of a tile, whether A and B change places (the tile's 256 rows are then columns of C and its `bn`
+// columns rows of C), and how many pairs share each tile of the last wave (s < 2: none do), `tail` of them.
+struct TilePlan {
+  int bn, turned, s, tail;
   long long word_bytes() const { return ((long long)tail * 8 * sizeof(unsigned long long) + 255) / 256 * 256; }
-  long long bytes() const { return s < 2 ? 0 : word_bytes() + (long long)tail * s * kSplitTileFloats * sizeof(float); }
+  long long bytes() const { return s < 2 ? 0 : word_bytes() + (long long)tail * s * (CM * bn) * sizeof(float); }
 };
 
-// How many pairs share each tile of the last wave, where the tiles leave part of it idle.
-// A tile takes 0.3 us per k-block.  The pair that adds the parts reads each of the others' from L2 for about 2.4 us after its own
-// last product; storing its own part and arriving take 7 us before that.  A split into s slices therefore pays where
-// num_kb * (1 - 1/s) is more than kSplitCost + kPartCost * (s - 1), and slice s pays beside s - 1 where num_kb / (s (s - 1)) is
-// more than kPartCost.  One pair a tile against the rule's choice, us a launch in a graph: one tile, K = 2048 14.3 (not split),
-// K = 4096 23.4 by three 22.5, K = 8192 41.2 by four 27.9; 81 tiles, 7 in the last wave, K = 4096 45.7 by three 44.7, K = 8192
-// 85.2 by four 73.9; 84 tiles, 10 in the last wave, K = 3584 41.0 (not split; by three 42.4), K = 6400 68.0 by four 61.7; 98
-// tiles, 24 in the last wave, K = 18944 194 by three 160; 256 tiles, 34 in the last wave, K = 32000 739 by two 703.
-SplitPlan split_plan(int tiles, int num_kb, int max_pairs) {
-  SplitPlan p{0, tiles % max_pairs};
-  if (split_mode() == 0 || p.tail == 0) return p;
-  int s = max_pairs / p.tail;
-  if (s > num_kb / 8) s = num_kb / 8;
-  if (split_mode() < 0) {
-    while (s > 1 && kPartCost * s * (s - 1) > num_kb) --s;               // the last part still pays for itself
-    if (s > 1 && num_kb - num_kb / s < kSplitCost + kPartCost * (s - 1)) s = 0;
-  } else if (s > 4) {
-    s = 4;
+// Costs in cycles of 1.6 GHz, fitted to 50 products of the three layouts, 128 to 152064 rows and columns, K = 63 to 152064.
+// A k-block moves 16 KB of A and 64 bn bytes of B into each SM, which takes 64 bytes a cycle from L2, and 2 bn cycles on the
+// tensor core: 256 + bn cycles, in which narrower tiles leave the tensor core idle.
+constexpr int kBlockCost = 256;
+// With every SM at work for long it is the power limit that bounds, and with it the products themselves: 2 bn cycles of a
+// k-block at five sixths of the clock, the part of the last wave that idles not counted (1554 x 37888, K = 3584: 1036 tiles of
+// 256 columns 310 us, as many of 224 278, 1332 of 192 295).  An idle last wave still costs a little there: 4096 x 4096, K = 32000,
+// 256 tiles 760 us, the last 34 shared by two 703.
+// A tile's way out of tensor memory: it counts once per launch, and in every wave where it is longer than the products.  One
+// tile of K = 512, bn = 64 to 256, us: 16 bits 6.0 to 8.1, fp32 7.7 to 11.2, turned 6.5 to 11.5; K = 300, fp32, 11008 x 4096 (all
+// stores): bn = 256 50, bn = 128 62, so that a tile has a part that is not its columns'.
+constexpr int kStore = 2400, kStore16 = 10, kStore32 = 21, kStoreTurned = 34, kTurned = 1000;
+// A shared tile, per column: the parts' way to L2 and the arrivals, and each part that is added (200 x 3584, K = 18944: 256
+// columns by five 52 us, 192 by three 44, not shared 89).
+constexpr int kSplitCost = 48, kPartCost = 20;
+// A plan other than whole tiles of 256 columns has to promise a gain of one part in this many.
+constexpr int kWorth = 64;
+
+long long plan_cost(long long tiles, int num_kb, int pairs, int bn, int store, int s) {
+  const long long main = num_kb * (kBlockCost + bn), epi = kStore + bn * store, wave = main > epi ? main : epi;
+  const long long waves = tiles / pairs, tail = tiles % pairs;
+  const long long power = tiles * num_kb * bn * 12 / (5 * pairs) + epi;
+  long long cost = waves * wave + main + epi;
+  if (tail == 0) cost = (waves - 1) * wave + main + epi;
+  else if (s > 1) cost = waves * wave + (num_kb + s - 1) / s * (kBlockCost + bn) + bn * (kSplitCost + kPartCost * (s - 1)) + epi;
+  return cost > power ? cost : (3 * power + cost) / 4;
+}
+int split_most(int tail, int num_kb, int pairs) {
+  const int s = tail == 0 ? 0 : pairs / tail < num_kb / 8 ? pairs / tail : num_kb / 8;
+  return s > int(kSplitCountMask) ? int(kSplitCountMask) : s;
+}
+
+// The cheapest cut of C[M, N] for `max_pairs` pairs.  What there is to gain: rows of tiles that hang over the edge of C (tokens
+// are ragged, the columns of a weight hardly ever are: turned, the tokens are cut into equal tiles of as few columns as they
+// need), a last wave with few tiles in it, and pairs without a tile.
+TilePlan cheapest_plan(int M, int N, int K, bool wide, bool may_turn, int max_pairs) {
+  const int num_kb = (K + BK - 1) / BK;
+  TilePlan best{BN, 0, 0, 0};
+  long long best_cost = 0;
+  for (int turned = 0; turned <= (may_turn ? 1 : 0); ++turned) {
+    const int rows = turned ? N : M, cols = turned ? M : N;
+    const int step = turned || wide ? 32 : 64;           // 16-bit blocks leave 64 columns at a time
+    for (int bn = BN; bn >= 64; bn -= step) {
+      const long long tiles = (long long)((rows + CM - 1) / CM) * ((cols + bn - 1) / bn);
+      const int tail = int(tiles % max_pairs);
+      const int store = turned ? kStoreTurned : wide ? kStore32 : kStore16;
+      int most = split_mode() == 0 ? 0 : split_most(tail, num_kb, max_pairs), least = 0;
+      if (split_mode() > 0 && most > 1) least = most = most > 4 ? 4 : most;
+      long long before = 0;
+      for (int s = least; s == 0 || s <= most; s += s == 0 ? 2 : 1) {
+        const long long cost = plan_cost(tiles, num_kb, max_pairs, bn, store, s) + (turned ? kTurned : 0);
+        if (s > 2 && cost > before && split_mode() < 0) break;      // more slices only cost more from here on
+        before = cost;
+        const bool first = best_cost == 0, whole = bn == BN && !turned;
+        if (first || (whole ? cost < best_cost : cost * kWorth < best_cost * (kWorth - 1))) {
+          best = TilePlan{bn, turned, s, tail};
+          best_cost = cost;
+        }
+      }
+    }
   }
-  if (s > int(kSplitCountMask)) s = int(kSplitCountMask);
-  if (s > 1) p.s = s;
-  return p;
+  return best;
+}
+
+// The same; a thread's last few are kept, because the layers of a model ask for the same ones again and a search takes a
+// microsecond or two.
+TilePlan tile_plan(int M, int N, int K, int out_mode, bool may_turn, int max_pairs) {
+  struct Kept {
+    int m, n, k, kind, pairs;
+    TilePlan plan;
+  };
+  constexpr unsigned kSlots = 64;
+  static thread_local Kept kept[kSlots] = {};
+  const bool wide = out_mode == kOutF32 || out_mode == kOutF32Acc;
+  const int kind = wide ? 2 : may_turn ? 1 : 0;
+  Kept& e = kept[(unsigned(M) * 31u + unsigned(N) * 17u + unsigned(K) / 8u * 7u + unsigned(kind)) % kSlots];
+  if (e.m != M || e.n != N || e.k != K || e.kind != kind || e.pairs != max_pairs)
+    e = Kept{M, N, K, kind, max_pairs, cheapest_plan(M, N, K, wide, !wide && may_turn, max_pairs)};
+  return e.plan;
 }
 
 // Starts at the clock: no launch of this process has the token of another, and nothing here can throw at a C entry.
@@ -382,31 +439,36 @@ static int launch_grouped2(const CUtensorMap& ta, const CUtensorMap& tb, const C
 }
 
 template <bool A_MN, bool B_MN>
-static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p_in, int want_pairs,
-                   void* ws, long long ws_bytes, cudaStream_t st) {
+static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p_in, const TilePlan& plan,
+                   int max_pairs, int want_pairs, void* ws, long long ws_bytes, cudaStream_t st) {
   Params p = p_in;
-  static int max_pairs = -1;
+  static int co_resident = -1;
   auto k = gemm2_bf16_kernel<A_MN, B_MN>;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  if (int rc = pair_config(k, &cfg, attr, &max_pairs, hg_host::launch_overlaps(), st)) return rc;
-  int pairs = want_pairs < max_pairs ? want_pairs : max_pairs;
-  // Last wave partly filled: let several pairs share each of its tiles (see Params::split_s).
-  const int tiles = p.tiles_m * p.tiles_n, num_kb = (p.K + BK - 1) / BK;
+  if (int rc = pair_config(k, &cfg, attr, &co_resident, hg_host::launch_overlaps(), st)) return rc;
+  int pairs = want_pairs < co_resident ? want_pairs : co_resident;
   p.split_s = 0;
-  if (ws != nullptr && p.ready == nullptr) {
-    const SplitPlan plan = split_plan(tiles, num_kb, max_pairs);
-    if (plan.s > 1 && ws_bytes >= plan.bytes()) {
-      p.split_s = plan.s;
-      p.split_tail_begin = tiles - plan.tail;
-      p.split_words = static_cast<unsigned long long*>(ws);
-      p.split_ws = reinterpret_cast<float*>(static_cast<char*>(ws) + plan.word_bytes());
-      p.split_token = split_token();
-      pairs = p.split_tail_begin > 0 ? max_pairs : plan.tail * plan.s;
-    }
+  if (ws != nullptr && plan.s > 1 && ws_bytes >= plan.bytes()) {     // see Params::split_s
+    p.split_s = plan.s;
+    p.split_tail_begin = p.tiles_m * p.tiles_n - plan.tail;
+    p.split_words = static_cast<unsigned long long*>(ws);
+    p.split_ws = reinterpret_cast<float*>(static_cast<char*>(ws) + plan.word_bytes());
+    p.split_token = split_token();
+    pairs = p.split_tail_begin > 0 ? max_pairs : plan.tail * plan.s;   // the plan's pairs, co-resident or not: none waits for another
   }
   cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
   return hg_host::launched(cudaLaunchKernelEx(&cfg, k, ta, tb, tc, p));
+}
+
+// Pairs of the plain kernels that the device holds at once (the four layouts take the same shared memory and threads).
+static int plain_pairs(int* pairs) {
+  static int max_pairs = -1;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  const int rc = max_pairs > 0 ? 0 : pair_config(gemm2_bf16_kernel<false, false>, &cfg, attr, &max_pairs, false, nullptr);
+  *pairs = max_pairs;
+  return rc;
 }
 
 // The tensor map of C for the plain stores (p.c_tma says whether it is used; `any` fills the kernel's parameter else).
@@ -421,6 +483,12 @@ static int store_map(CUtensorMap* tc, const CUtensorMap& any, Params& p, uint64_
   return rc < 0 ? rc : 0;
 }
 
+// Whether C can be stored from turned tiles: 16-bit results, two of a row at a time.  (Turned fp32 tiles were up to half slower:
+// 32000 x 5120, K = 670 219 -> 350 us.)
+static bool turns(const void* C, int N, int ldc, int out_mode) {
+  return out_mode == kOutBf16 && N % 2 == 0 && ldc % 2 == 0 && (reinterpret_cast<uintptr_t>(C) & 3) == 0;
+}
+
 extern "C" {
 
 // Same contract as hg_gemm_bf16 (gemm.cu), computed by CTA pairs.  Returns -2 when the device cannot co-schedule a
@@ -432,44 +500,57 @@ int hg_gemm2_bf16(const void* A, const void* B, void* C, const void* bias, int M
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if ((lda & 7) || (ldb & 7) || (reinterpret_cast<uintptr_t>(A) & 15) || (reinterpret_cast<uintptr_t>(B) & 15))
     return -1;
+  int max_pairs, rc = plain_pairs(&max_pairs);
+  if (rc) return rc;
+  TilePlan plan{BN, 0, 0, 0};
+  if (max_ctas == 0) plan = tile_plan(M, N, K, out_mode, turns(C, N, ldc, out_mode), max_pairs);
+  if (plan.turned) {
+    std::swap(A, B);
+    std::swap(M, N);
+    std::swap(lda, ldb);
+    std::swap(a_mn, b_mn);
+  }
   CUtensorMap ta, tb;
-  int rc;
   if (a_mn) rc = hg_host::make_tmap_2d_bf16(&ta, A, K, M, lda, 64, 64);
   else      rc = hg_host::make_tmap_2d_bf16(&ta, A, M, K, lda, BM, 64);
   if (rc) return rc;
   if (b_mn) rc = hg_host::make_tmap_2d_bf16(&tb, B, K, N, ldb, 64, 64);
-  else      rc = hg_host::make_tmap_2d_bf16(&tb, B, N, K, ldb, HALF_N, 64);
+  else      rc = hg_host::make_tmap_2d_bf16(&tb, B, N, K, ldb, plan.bn / 2, 64);
   if (rc) return rc;
   Params p{};
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.C = C;
   p.bias = reinterpret_cast<const hg_lp_t*>(bias);
   p.out_mode = out_mode;
+  p.bn = plan.bn;
+  p.turned = plan.turned;
   p.tiles_m = (M + CM - 1) / CM;
-  p.tiles_n = (N + BN - 1) / BN;
+  p.tiles_n = (N + plan.bn - 1) / plan.bn;
   p.group_m = 4;
   p.status = hg_host::status_ptr();
   p.ready = nullptr; p.rows_per_flag = 1; p.ready_target = 0; p.m_tile_shift = 0;
   p.k_ranges = nullptr; p.groups = 1; p.c_group_stride = 0;
   int pairs = p.tiles_m * p.tiles_n;
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
-  CUtensorMap tc;
-  if ((rc = store_map(&tc, ta, p, M))) return rc;
+  CUtensorMap tc = ta;
+  if (!plan.turned && (rc = store_map(&tc, ta, p, M))) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (max_ctas != 0) ws = nullptr;
-  if (a_mn && b_mn) return launch2<true, true>(ta, tb, tc, p, pairs, ws, ws_bytes, st);
-  if (a_mn) return launch2<true, false>(ta, tb, tc, p, pairs, ws, ws_bytes, st);
-  if (b_mn) return launch2<false, true>(ta, tb, tc, p, pairs, ws, ws_bytes, st);
-  return launch2<false, false>(ta, tb, tc, p, pairs, ws, ws_bytes, st);
+  if (a_mn && b_mn) return launch2<true, true>(ta, tb, tc, p, plan, max_pairs, pairs, ws, ws_bytes, st);
+  if (a_mn) return launch2<true, false>(ta, tb, tc, p, plan, max_pairs, pairs, ws, ws_bytes, st);
+  if (b_mn) return launch2<false, true>(ta, tb, tc, p, plan, max_pairs, pairs, ws, ws_bytes, st);
+  return launch2<false, false>(ta, tb, tc, p, plan, max_pairs, pairs, ws, ws_bytes, st);
 }
 
-// Bytes of scratch that hg_gemm2_bf16 asks for on the current device (0: none).
+// Bytes of scratch that hg_gemm2_bf16 may ask for on the current device, whatever the type of the result (0: none).
 long long hg_gemm2_scratch(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  static int max_pairs = -1;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[2];
-  if (pair_config(gemm2_bf16_kernel<false, false>, &cfg, attr, &max_pairs, false, nullptr)) return 0;
-  return split_plan(((M + CM - 1) / CM) * ((N + BN - 1) / BN), (K + BK - 1) / BK, max_pairs).bytes();
+  int max_pairs;
+  if (plain_pairs(&max_pairs)) return 0;
+  long long most = 0;
+  for (int kind = 0; kind < 3; ++kind) {
+    const long long need = tile_plan(M, N, K, kind == 2 ? kOutF32 : kOutBf16, kind == 1, max_pairs).bytes();
+    if (need > most) most = need;
+  }
+  return most;
 }
 
 // Same contracts as hg_grouped_gemm_bf16 and hg_grouped_wgrad_bf16 (gemm.cu), computed by CTA pairs; -2 as above.
@@ -484,7 +565,7 @@ int hg_grouped_gemm2_bf16(const void* A, const void* B, void* C, const void* row
   else      rc = hg_host::make_tmap_2d_bf16(&tb, B, uint64_t(G) * N, K, ldb, HALF_N, 64);
   if (rc) return rc;
   Params p{};
-  p.M = max_rows; p.N = N; p.K = K; p.ldc = ldc; p.C = C; p.out_mode = out_mode; p.status = hg_host::status_ptr();
+  p.M = max_rows; p.N = N; p.K = K; p.ldc = ldc; p.C = C; p.out_mode = out_mode; p.bn = BN; p.status = hg_host::status_ptr();
   RowSegments t{reinterpret_cast<const int*>(row_start), G, (N + BN - 1) / BN, (K + BK - 1) / BK, b_mn ? K : N, max_rows,
                 p.status};
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
@@ -504,7 +585,7 @@ int hg_grouped_wgrad2_bf16(const void* dy, const void* x, void* out, const void*
   rc = hg_host::make_tmap_2d_bf16(&tb, x, rows, K, ldx, 64, 64);
   if (rc) return rc;
   Params p{};
-  p.M = N; p.N = K; p.K = rows; p.ldc = K; p.C = out; p.out_mode = out_mode; p.status = hg_host::status_ptr();
+  p.M = N; p.N = K; p.K = rows; p.ldc = K; p.C = out; p.out_mode = out_mode; p.bn = BN; p.status = hg_host::status_ptr();
   ContractionRanges t{reinterpret_cast<const int*>(row_start), G, (N + CM - 1) / CM, (K + BN - 1) / BN, N, (long long)N * K};
   int pairs = t.tiles_m * t.tiles_n * G;
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;

@@ -113,11 +113,10 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
 struct Unit {
   int tile, kb0, kb1, slice;
 };
-constexpr int kSplitTileFloats = CM * BN;
 constexpr unsigned long long kSplitCountMask = 255;      // low bits of a word: slices that have arrived; a token has none of them
 // Word `q` (four columns) of 32-column block `c` of this thread's row in a partial tile: neighbouring lanes, neighbouring words.
-__device__ __forceinline__ int split_word(int warp8, int c, int q) {
-  return (((warp8 * (BN / 32) + c) * 8 + q) * 32 + int(lane_id())) * 4;
+__device__ __forceinline__ int split_word(int bn, int warp8, int c, int q) {
+  return (((warp8 * (bn / 32) + c) * 8 + q) * 32 + int(lane_id())) * 4;
 }
 __device__ __forceinline__ int unit_count(const Params& p, int first, int step, int num_tiles) {
   if (p.split_s > 1) return p.split_tail_begin / step + (first < (num_tiles - p.split_tail_begin) * p.split_s ? 1 : 0);
@@ -149,6 +148,8 @@ __device__ __forceinline__ void producer2(const CUtensorMap* tmA, const CUtensor
 #pragma unroll
   for (int i = 0; i < STAGES2; ++i) { issued[i] = false; issued_parity[i] = 0; }
   const int num_kb = (p.K + BK - 1) / BK;
+  const int half = p.bn / 2;              // of B's rows (columns) of a tile, each CTA stages one half; whole slabs where N-major
+  const uint32_t stage_bytes = 2 * (A2_BYTES + (B_MN ? (half + 63) / 64 * SLAB_BYTES : half * BK * 2));
   bool ok = true;
   const bool issuer = elect_one() != 0;   // the warp walks the loop together; only this lane issues the copies
   const int n_units = unit_count(p, first, step, num_tiles);
@@ -157,7 +158,7 @@ __device__ __forceinline__ void producer2(const CUtensorMap* tmA, const CUtensor
     int tm, tn;
     tile_coords(p, w.tile, tm, tn);
     const int m0 = tm * CM + int(rank) * BM;
-    const int n0 = tn * BN + int(rank) * HALF_N;
+    const int n0 = tn * p.bn + int(rank) * half;
     if (p.ready != nullptr) {
       // readiness gate on this CTA's 128 A rows (all-gather fused variant): one lane polls, bounded, and the verdict
       // is made warp-uniform; the rows were written with ordinary stores, TMA reads through the async proxy
@@ -189,7 +190,7 @@ __device__ __forceinline__ void producer2(const CUtensorMap* tmA, const CUtensor
       uint8_t* sb = s.b + stage * B2_BYTES;
       const int k0 = kb * BK;
       if (issuer) {
-        if (rank == 0) mbar_expect_tx(&s.full[stage], 2 * (A2_BYTES + B2_BYTES));
+        if (rank == 0) mbar_expect_tx(&s.full[stage], stage_bytes);
         if (A_MN) {
 #pragma unroll
           for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * SLAB_BYTES, tmA, bar, m0 + j * 64, k0);
@@ -198,7 +199,8 @@ __device__ __forceinline__ void producer2(const CUtensorMap* tmA, const CUtensor
         }
         if (B_MN) {
 #pragma unroll
-          for (int j = 0; j < HALF_N / 64; ++j) tma_load_2d_pair(sb + j * SLAB_BYTES, tmB, bar, n0 + j * 64, k0);
+          for (int j = 0; j < HALF_N / 64; ++j)
+            if (j * 64 < half) tma_load_2d_pair(sb + j * SLAB_BYTES, tmB, bar, n0 + j * 64, k0);
         } else {
           tma_load_2d_pair(sb, tmB, bar, k0, n0);
         }
@@ -233,7 +235,7 @@ __device__ __forceinline__ void producer2(const CUtensorMap* tmA, const CUtensor
 template <bool A_MN, bool B_MN>
 __device__ __forceinline__ void mma2(const Params& p, const Smem2& s, uint32_t tmem_base, int first, int step,
                                      int num_tiles) {
-  constexpr uint32_t idesc = make_idesc_lp(CM, BN, A_MN, B_MN);
+  const uint32_t idesc = make_idesc_lp(CM, p.bn, A_MN, B_MN);
   constexpr uint32_t a_lbo = A_MN ? SLAB_BYTES : 16, a_sbo = 1024, a_kadv = A_MN ? 2048 : 32;
   constexpr uint32_t b_lbo = B_MN ? SLAB_BYTES : 16, b_sbo = 1024, b_kadv = B_MN ? 2048 : 32;
   const int num_kb = (p.K + BK - 1) / BK;
@@ -324,11 +326,11 @@ __device__ __forceinline__ void tma_store_rows(const CUtensorMap* tm, StoreStage
 // others lie in memory.  Added in one order, the last slice first, whoever adds them.
 struct Parts {
   const float* base;
-  int n, mine, warp8;
+  int n, mine, warp8, bn;
   __device__ __forceinline__ void add(int c, uint32_t (&r)[32]) const {
     if (n == 0) return;
     auto part = [&](int k, int q) {
-      return __ldcg(reinterpret_cast<const float4*>(base + size_t(k) * kSplitTileFloats + split_word(warp8, c, q)));
+      return __ldcg(reinterpret_cast<const float4*>(base + size_t(k) * (CM * bn) + split_word(bn, warp8, c, q)));
     };
     if (mine == n - 1) {
       for (int k = 0; k + 1 < n; ++k) {
@@ -436,7 +438,7 @@ template <bool BIAS, bool F32>
 __device__ __forceinline__ void store_tile_tma(const Params& p, const CUtensorMap* tmC, StoreStage& st, uint32_t src, int row0,
                                                int y0, int n0, const Parts& parts) {
 #pragma unroll 1
-  for (int c = 0; c < BN && n0 + c < p.N; c += F32 ? 32 : 64) {
+  for (int c = 0; c < p.bn && n0 + c < p.N; c += F32 ? 32 : 64) {
     uint32_t r0[32], r1[32];
     tmem_ld32(src + c, r0);
     if (!F32) tmem_ld32(src + c + 32, r1);
@@ -603,7 +605,7 @@ __device__ __forceinline__ void load_old_whole(const Params& p, int row0, int co
 // values are in flight while this one is turned.
 template <int MODE>
 __device__ __forceinline__ int store_tile_whole(const Params& p, uint32_t stg, uint32_t src, int row0, int n0, const Parts& parts) {
-  const int cols = min(BN, (p.N - n0) & ~31);
+  const int cols = min(p.bn, (p.N - n0) & ~31);
   float4 old[8];
   if (cols > 0) load_old_whole<MODE>(p, row0, n0, old);
 #pragma unroll 1
@@ -626,7 +628,7 @@ __device__ __forceinline__ int store_tile_whole(const Params& p, uint32_t stg, u
 // The 32 x 256 part of a tile that this warp's lanes hold in tensor memory at `src`: rows row0.. of C (p.M: the first row
 // that is not this tile's), rows y0.. of the tensor map.
 __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorMap* tmC, StoreStage& st, uint32_t src, int row0,
-                                                int y0, int n0, bool whole_rows, const Parts& parts = Parts{nullptr, 0, 0, 0}) {
+                                                int y0, int n0, bool whole_rows, const Parts& parts = Parts{nullptr, 0, 0, 0, 0}) {
   if (p.c_tma && whole_rows) {
     if (p.out_mode == kOutF32) {
       if (p.bias != nullptr) store_tile_tma<true, true>(p, tmC, st, src, row0, y0, n0, parts);
@@ -651,7 +653,7 @@ __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorM
     }
   }
 #pragma unroll 1
-  for (int c = c0; c < BN && n0 + c < p.N; c += 32) {
+  for (int c = c0; c < p.bn && n0 + c < p.N; c += 32) {
     float4 old[8];
     load_old(p, row0, n0 + c, old);
     uint32_t r0[32];
@@ -659,6 +661,50 @@ __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorM
     tmem_ld_wait();
     parts.add(c / 32, r0);
     store_block_rows(p, st.base, row0, n0 + c, r0, old);
+  }
+}
+
+// A turned tile part: a lane holds one column of C, C[n0 + c, row0 + lane] for its columns c, so that a warp's store of one c is
+// 32 consecutive elements and needs no shared memory.  16 bits: neighbouring lanes trade a value, and each stores two columns
+// of one row, 16 lanes a row and 64 bytes each.
+template <int MODE>
+__device__ __forceinline__ void store_tile_turned(const Params& p, uint32_t src, int row0, int n0, const Parts& parts) {
+  const int lane = int(lane_id()), col = row0 + lane;
+  const bool mine = col < p.M;
+  const float b = p.bias != nullptr && mine ? hg_lp2f(p.bias[col]) : 0.f;
+#pragma unroll 1
+  for (int c = 0; c < p.bn && n0 + c < p.N; c += 32) {
+    uint32_t r[32];
+    tmem_ld32(src + c, r);
+    tmem_ld_wait();
+    if (!HG_BOUNDS_OK(row0 >= 0 && row0 < p.M && n0 >= 0, p.status)) continue;
+    parts.add(c / 32, r);
+    const int rows = p.N - (n0 + c);
+    if constexpr (MODE == kOutBf16) {
+      const int odd = lane & 1;
+      hg_lp_t* at = reinterpret_cast<hg_lp_t*>(p.C) + size_t(n0 + c + odd) * p.ldc + (col - odd);
+#pragma unroll
+      for (int i = 0; i < 32; i += 2, at += size_t(2) * p.ldc) {
+        const float x = __uint_as_float(r[i]) + b, y = __uint_as_float(r[i + 1]) + b;
+        const float z = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
+        if (mine && i + odd < rows) *reinterpret_cast<uint32_t*>(at) = odd ? pack_bf16(z, y) : pack_bf16(x, z);
+      }
+    } else {
+      float* at = reinterpret_cast<float*>(p.C) + size_t(n0 + c) * p.ldc + col;
+      float old[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) old[i] = MODE == kOutF32Acc && mine && i < rows ? at[size_t(i) * p.ldc] : 0.f;
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (mine && i < rows) at[size_t(i) * p.ldc] = MODE == kOutF32Acc ? __uint_as_float(r[i]) + b + old[i] : __uint_as_float(r[i]) + b;
+    }
+  }
+}
+__device__ __forceinline__ void store_tile_turned(const Params& p, uint32_t src, int row0, int n0, const Parts& parts) {
+  switch (p.out_mode) {
+    case kOutF32: store_tile_turned<kOutF32>(p, src, row0, n0, parts); break;
+    case kOutF32Acc: store_tile_turned<kOutF32Acc>(p, src, row0, n0, parts); break;
+    default: store_tile_turned<kOutBf16>(p, src, row0, n0, parts); break;
   }
 }
 
@@ -677,12 +723,12 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
     int tm, tn;
     tile_coords(p, tile, tm, tn);
     const int row0 = tm * CM + int(rank) * BM + wq * 32;   // first of this warp's 32 rows
-    const int n0 = tn * BN;
+    const int n0 = tn * p.bn;
     // a tail tile shared with other pairs: whichever of them is done last adds the parts and writes it
     const bool shared_tile = p.split_s > 1 && tile >= p.split_tail_begin;
     const int tail_idx = tile - p.split_tail_begin, warp8 = int(rank) * EPI_WARPS + wq;
-    float* ws_tile = shared_tile ? p.split_ws + size_t(tail_idx) * p.split_s * kSplitTileFloats : nullptr;
-    const Parts parts{ws_tile, shared_tile ? p.split_s : 0, w.slice, warp8};
+    float* ws_tile = shared_tile ? p.split_ws + size_t(tail_idx) * p.split_s * (CM * p.bn) : nullptr;
+    const Parts parts{ws_tile, shared_tile ? p.split_s : 0, w.slice, warp8, p.bn};
     if (!mbar_wait_warp(&s.tmem_full[acc], acc_phase, p.status, kTimeoutTmemFull, s.abort)) {
       *s.abort = 1;
       break;
@@ -693,15 +739,15 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
       bool writes = true;
       if (shared_tile) {
         // Nobody waits for another pair, whatever the order in which the device runs them.
-        float* dst = ws_tile + size_t(w.slice) * kSplitTileFloats;
+        float* dst = ws_tile + size_t(w.slice) * (CM * p.bn);
 #pragma unroll 1
-        for (int c = 0; c < BN / 32; ++c) {
+        for (int c = 0; c < p.bn / 32; ++c) {
           uint32_t r0[32];
           tmem_ld32(src + c * 32, r0);
           tmem_ld_wait();
 #pragma unroll
           for (int q = 0; q < 8; ++q)
-            __stcg(reinterpret_cast<uint4*>(dst + split_word(warp8, c, q)),
+            __stcg(reinterpret_cast<uint4*>(dst + split_word(p.bn, warp8, c, q)),
                    make_uint4(r0[4 * q], r0[4 * q + 1], r0[4 * q + 2], r0[4 * q + 3]));
         }
         __threadfence();
@@ -711,7 +757,8 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
         writes = __shfl_sync(0xffffffffu, last, 0) != 0;
         __threadfence();                  // the other slices' parts are read after their arrivals
       }
-      if (writes) store_tile_part(p, tmC, st, src, row0, row0, n0, true, parts);
+      if (writes && p.turned) store_tile_turned(p, src, row0, n0, parts);
+      else if (writes) store_tile_part(p, tmC, st, src, row0, row0, n0, true, parts);
     }
     tc_fence_before();
     // the accumulator buffer is free again once all 256 epilogue threads of the pair have read it

@@ -67,7 +67,7 @@ struct Params {
   long long c_group_stride;
   // Optional split of the last, partly filled wave (CTA-pair kernel only): tiles from `split_tail_begin` on are each
   // computed by `split_s` pairs, every pair taking a contiguous share of the k-blocks.  Each leaves its fp32 partial tile in
-  // `split_ws` (256 x 256 floats per (tail tile, slice), in the order in which the epilogue's threads hold it), and each of its
+  // `split_ws` (256 x bn floats per (tail tile, slice), in the order in which the epilogue's threads hold it), and each of its
   // eight epilogue warps then counts itself in at its word of `split_words` ([tail tile][8]).  The last warp to arrive at a
   // word adds the parts of those rows in slice order, so that the result does not depend on timing, and writes them.
   // split_s < 2: off.
@@ -77,6 +77,8 @@ struct Params {
   unsigned long long* split_words;
   unsigned long long split_token;    // differs from launch to launch: whatever the words held before is not it
   int c_tma;                  // CTA-pair kernels: full blocks of C leave through the tensor map of C (plain 16-bit and fp32 stores)
+  int bn;                     // CTA-pair kernels: columns of a tile, a multiple of 32 up to BN (of 64 where c_tma stores 16 bits)
+  int turned;                 // CTA-pair kernel: A and B have changed places, so that row m and column n of the product are C[n, m]
 };
 
 struct TileInfo {

@@ -140,3 +140,27 @@ def test_shared_tiles_of_many_slices(M, N, K):
     torch.cuda.synchronize()
     assert all(torch.equal(o, once) for o in outs)
     _lib.assert_healthy()
+
+
+# products that the plan cuts into tiles of other widths: whole columns of 64 to 224, turned ones whose rows end inside a tile, a
+# block and a pair of columns, alone and shared, and results that turned tiles cannot store (an odd pitch, an odd base)
+@pytest.mark.parametrize("M,N,K", [(1024, 512, 512), (1531, 4608, 712), (333, 3072, 768), (128, 1600, 6400), (258, 1602, 6400),
+                                   (580, 16642, 512), (1554, 9474, 1024), (200, 3584, 8192), (312, 1600, 1600), (1600, 1600, 2997)])
+@pytest.mark.parametrize("a_mn,b_mn,biased", [(False, False, True), (False, True, False), (True, True, False)])
+@pytest.mark.parametrize("mode,left", [(OUT_BF16, 0), (OUT_BF16, 2), (OUT_BF16, 1), (OUT_F32, 0), (OUT_F32_ACC, 4)])
+def test_tiles_of_every_width(M, N, K, a_mn, b_mn, biased, mode, left):
+    g = torch.Generator(device=DEV).manual_seed(M + K + mode)
+    pad = lambda r, c: torch.randn(r, (c + 7) // 8 * 8, device=DEV, generator=g).to(torch.bfloat16)[:, :c]
+    a, b = pad(K, M) if a_mn else pad(M, K), pad(K, N) if b_mn else pad(N, K)
+    bias = torch.randn(N, device=DEV, generator=g).to(torch.bfloat16) if biased else None
+    ref = (a.t() if a_mn else a).double() @ (b if b_mn else b.t()).double() + (bias.double() if biased else 0.0)
+    whole = torch.full((M + 2, N + 8), 2.0, device=DEV, dtype=torch.bfloat16 if mode == OUT_BF16 else torch.float32)
+    out = whole[1:M + 1, left:left + N]
+    ops.gemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out, out_mode=mode, bias=bias, pair=True)
+    # K / 16 additions in the tensor core, each off by at most a unit 2^-23 of a running sum of K products of unit normals, six
+    # standard deviations sqrt(K) at most; one rounding to 16 bits where C is 16 bits wide
+    assert torch.allclose(out.double(), ref + (2.0 if mode == OUT_F32_ACC else 0.0), rtol=2.0 ** -8 if mode == OUT_BF16 else 1e-6,
+                          atol=K / 16 * 2.0 ** -23 * 6 * K ** 0.5)
+    out.fill_(2.0)
+    assert (whole == 2.0).all()                                                 # nothing outside the window
+    _lib.assert_healthy()
