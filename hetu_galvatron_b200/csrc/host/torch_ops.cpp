@@ -53,7 +53,8 @@ struct Kernels {
   int (*rope)(void*, V, int, int, int, int, int, V, int, V, V, int, int, void*);
   int (*flash_fwd)(A, A, A, A, void*, int, int, int, int, int, int, int, int, int, float, void*);
   long long (*flash_bwd_scratch)(int, int, int, int, int, int, int, int, int);
-  int (*flash_bwd)(A, A, A, A, A, V, void*, long long, A, A, A, int, int, int, int, int, int, int, int, int, float, void*);
+  long long (*flash_bwd_scratch_of)(int, int, int, int, int, int, int, int, int, int);
+  int (*flash_bwd)(A, A, A, A, A, V, void*, long long, A, A, A, int, int, int, int, int, int, int, int, int, float, int*, void*);
   long long (*decoder_step_scratch)(const HgDecoderStep*);
   int (*decoder_step)(HgDecoderStep*, void*);
 };
@@ -360,12 +361,18 @@ struct FlashPacked : public Function<FlashPacked> {
     const Packed l = layout(ctx);
     const Tensor dout = grads[0].contiguous();
     Tensor dqkv = at::empty_like(qkv);
-    const Tensor ws = empty({K.flash_bwd_scratch(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0)}, at::kFloat, qkv);
+    Tensor ws;
+    try {
+      ws = empty({K.flash_bwd_scratch(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0)}, at::kFloat, qkv);
+    } catch (const c10::OutOfMemoryError&) {           // no room for dS: the kernels do without
+      ws = empty({K.flash_bwd_scratch_of(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0, 0)}, at::kFloat, qkv);
+    }
+    int kernels = 0;
     const HgAttnTensor q = l.q(qkv.data_ptr()), k = l.k(qkv.data_ptr()), v = l.v(qkv.data_ptr()), o = l.o(out.data_ptr()),
                        d = l.o(dout.data_ptr()), dq = l.q(dqkv.data_ptr()), dk = l.k(dqkv.data_ptr()), dv = l.v(dqkv.data_ptr());
     check(K.flash_bwd(&q, &k, &v, &o, &d, lse.data_ptr(), ws.data_ptr(), ws.numel(), &dq, &dk, &dv, l.S, l.S, l.B, l.nh, l.ng,
-                      l.hd, l.causal, 0, 0, l.scale, stream()), "hg_flash_bwd");
-    count(ws.numel() > (long long)l.B * l.nh * l.S + 3 ? 4 : 3);
+                      l.hd, l.causal, 0, 0, l.scale, &kernels, stream()), "hg_flash_bwd");
+    count(kernels);
     return {dqkv, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
 };
@@ -666,7 +673,7 @@ void bind(const py::dict& fn, bool half, int pair_mode, py::object kernel_error)
   at("hg_colsum_parts", K.colsum_parts); at("hg_colsum_bf16", K.colsum);
   at("hg_norm_fwd", K.norm_fwd); at("hg_norm_bwd", K.norm_bwd);
   at("hg_glu_fwd", K.glu_fwd); at("hg_glu_bwd", K.glu_bwd); at("hg_add_bf16", K.add); at("hg_rope", K.rope);
-  at("hg_flash_fwd", K.flash_fwd); at("hg_flash_bwd_scratch", K.flash_bwd_scratch); at("hg_flash_bwd_ws", K.flash_bwd);
+  at("hg_flash_fwd", K.flash_fwd); at("hg_flash_bwd_scratch", K.flash_bwd_scratch); at("hg_flash_bwd_scratch_of", K.flash_bwd_scratch_of); at("hg_flash_bwd_ws", K.flash_bwd);
   at("hg_decoder_step_scratch", K.decoder_step_scratch); at("hg_decoder_step", K.decoder_step);
   g_lp = half ? at::kHalf : at::kBFloat16;
   g_pair_mode = pair_mode;

@@ -53,11 +53,8 @@ __device__ __forceinline__ float ex2_poly(float x) {
   r = __int_as_float(__float_as_int(r) + (__float_as_int(t) << 23));
   return x < -126.f ? 0.f : r;
 }
-// Softmax warpgroups of the 128-query dK/dV kernel (2 or 4).
-#ifndef HG_DKV_WARPGROUPS
-#define HG_DKV_WARPGROUPS 4
-#endif
-constexpr int kDkvWarpgroups = HG_DKV_WARPGROUPS;
+// Softmax warpgroups of the 128-query dK/dV kernel.
+constexpr int kDkvWarpgroups = 4;
 // Softmax warpgroups of the 128-key dQ kernel (2 or 4).
 #ifndef HG_DQ_WARPGROUPS
 #define HG_DQ_WARPGROUPS 4
@@ -67,10 +64,6 @@ constexpr int kDqWarpgroups = HG_DQ_WARPGROUPS;
 // (its two softmax warpgroups run at the same time and share that unit).
 #ifndef HG_FWD_POLY_OF_4
 #define HG_FWD_POLY_OF_4 0
-#endif
-// How many of every four probabilities of the 128-query dK/dV kernel take ex2_poly instead of the special-function unit.
-#ifndef HG_DKV_POLY_OF_4
-#define HG_DKV_POLY_OF_4 0
 #endif
 
 // Per-role cycle counts of CTA (0, 0, 0), for builds with -DHG_ATTN_TIMING: where a step's time goes (waiting for the
@@ -827,13 +820,35 @@ struct BwdParams {
   // fp32 parts in `part`, [CTA][dV, dK][128][HD]
   int chunk;
   float* part;
+  // dS as the dK/dV kernel leaves it for the dQ product (null: it does not): 128 x 128 tiles of the pairs of a key block and a query
+  // block that see each other, in the order of ds_tiles_before.  A tile is what the tensor core reads as an M-major operand without
+  // swizzle, [2 x 64 keys][16 x 8 queries][64 keys][8 queries]: a warp's store of eight queries of 32 keys is 512 bytes in a row
+  // (as rows of 128 queries, 32 pieces of 32 bytes, these stores doubled the kernel's time), and half a tile one copy.  A launch covers nh_c heads from h0_c on (and their kv heads from
+  // g0_c on) of the sequences from b0_c on: grids count from there.
+  hg_lp_t* dS;
+  int b0_c, g0_c, h0_c, nh_c;
 };
+
+// Tiles of dS of key blocks 0 .. kb - 1 of one head.  Key block j is seen by the query blocks from max(0, j + d) on, d being
+// the distance of the first key behind the first query in blocks, rounded down.
+__host__ __device__ __forceinline__ long long ds_tiles_before(const BwdParams& p, int kb) {
+  const long long n_qs = (p.Sq + 127) / 128;
+  if (!p.causal) return kb * n_qs;
+  const int behind = p.k_pos0 - p.q_pos0, d = behind >= 0 ? behind / 128 : -((127 - behind) / 128);
+  const long long a = kb < -d ? kb : d < 0 ? -d : 0;                   // blocks that every query block sees
+  const long long e = kb < n_qs - d ? kb : n_qs - d;                   // blocks from e on are seen by none
+  const long long n = e > a ? e - a : 0;
+  return a * n_qs + n * n_qs - n * (a + e - 1) / 2 - n * d;
+}
+// First query block that sees key block kb.
+__host__ __device__ __forceinline__ int ds_first_query_block(const BwdParams& p, int kb) {
+  const int first = p.causal ? p.k_pos0 + kb * 128 - p.q_pos0 : 0;
+  return first > 0 ? first / 128 : 0;
+}
 
 // 128-query steps of key block kb, all query heads of its kv head together
 __host__ __device__ __forceinline__ int dkv_block_steps(const BwdParams& p, int kb) {
-  int first = p.causal ? p.k_pos0 + kb * 128 - p.q_pos0 : 0;       // first query row that can see this key block
-  if (first < 0) first = 0;
-  const int n = (p.Sq + 127) / 128 - first / 128;
+  const int n = (p.Sq + 127) / 128 - ds_first_query_block(p, kb);
   return n > 0 ? n * p.qpg : 0;
 }
 // CTAs that share key block kb, `steps` being its query steps
@@ -1194,7 +1209,44 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // The tensor core executes MMAs in issue order, which makes the reuse safe: dP^T(i+1) is issued after dV(i) and
 // dK(i), the readers of P^T(i) and dS^T(i).  Per step the MMA warp issues S^T(i+1) when the S^T(i) columns are
 // free, dV(i) when P^T(i) is stored, dK(i) and dP^T(i+1) when dS^T(i) is stored.
+//
+// Two warps fetch the statistics of the queries a step ahead.  In the softmax threads that cost registers: taken out, with the
+// probabilities kept in fp32, head dim 64, 8 x 1024 tokens and 25 heads 141 -> 106 us.  Where p.dS is set the threads also store
+// dS for the dQ product, half of it between the two halves of their arithmetic (all at the end: 629 against 603 us at 2 x 4096,
+// 32 heads of 128; none: 518).
 // =================================================================================================
+
+constexpr int kDkvAuxRegs = 64, kDkvSoftmaxRegs = 104;
+static_assert(128 * kDkvAuxRegs + 512 * kDkvSoftmaxRegs <= 640 * 96, "setmaxnreg deals out what the block was launched with");
+__device__ __forceinline__ float4 lds_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+
+// Two fp32 operations per instruction, each rounded as alone.  A pair of neighbouring registers is one operand.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\n"
+      "fma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmul.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
 
 template <int HD>
 struct Dkv128Smem {
@@ -1202,7 +1254,7 @@ struct Dkv128Smem {
   static constexpr int kQD = 128 * HD * 2;       // one Q or dO tile
   static constexpr int kQStages = 3;
   static constexpr int kDOStages = 2;
-  static constexpr int kStats = 2 * 2 * 128 * 4;  // -lse*log2e and D of a step, double buffered
+  static constexpr int kStats = 2 * 2 * 128 * 4;  // -lse*log2e and -D of a step, double buffered
   static constexpr int kBars = 256;
   static constexpr int kUsed = 2 * kKV + (kQStages + kDOStages) * kQD + kStats + kBars;
   // head dim 128: everything a CTA can have; the 1024-byte alignment of the tiles comes out of the rest
@@ -1214,15 +1266,13 @@ struct Dkv128Smem {
 // pipe busy through the latencies of the loads from tensor memory and of the dependent exp2 / convert chains.
 // SHARED: key blocks may be shared between CTAs (p.chunk > 0).
 template <int HD, int NWG, bool SHARED>
-__global__ void __launch_bounds__(64 + 128 * NWG, 1)
+__global__ void __launch_bounds__(128 + 128 * NWG, 1)
 flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
                         const BwdParams p) {
   static_assert(HD == 64 || HD == 128, "tensor memory holds S^T, dP^T and two accumulators of up to 128 columns");
-  static_assert(NWG == 2 || NWG == 4, "two or four softmax warpgroups");
+  static_assert(NWG == 4, "a thread's 32 columns: two halves of 16");
   constexpr int kSoftmaxWarps = 4 * NWG;
-  // head dim 64: dS^T is formed from fp32 probabilities, as in the 64-query kernel
-  constexpr bool kExactP = HD == 64;
   constexpr int CPT = 128 / NWG;               // query columns per thread and step
   // A CTA works on further blocks of the grid (WorkSlot).  Whole backward, us, one block a CTA / so, causal: head dim 64, 16 x 256
   // tokens and 25 heads 94 / 78, 8 x 1024 283 / 250, 4 x 2048 418 / 383, 1 x 8192 1205 / 1151, 12 heads 4096 210 / 203, 8192 634 /
@@ -1241,7 +1291,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   constexpr int NQ = L::kQStages, ND = L::kDOStages;
   uint8_t* sQ = sV + L::kKV;                 // NQ tiles
   uint8_t* sDO = sQ + NQ * L::kQD;           // ND tiles
-  float* sStats = reinterpret_cast<float*>(sDO + ND * L::kQD);   // [2][256]: 128 x -lse2, 128 x D
+  float* sStats = reinterpret_cast<float*>(sDO + ND * L::kQD);   // [2][256]: 128 x -lse2, 128 x -D
   uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sStats) + L::kStats);
   uint64_t* kv_full = bars;          // 1
   uint64_t* q_full = bars + 1;       // 3
@@ -1257,6 +1307,8 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   uint64_t* x_free = bars + 18;      // every thread has loaded its S^T values: the S^T columns may be overwritten
   uint64_t* kv_empty = bars + 19;    // the last products that read K and V have completed
   uint64_t* acc_empty = bars + 20;   // the epilogue has read dV and dK
+  uint64_t* stats_empty = bars + 27; // 2
+  int* sStep = reinterpret_cast<int*>(bars + 29);   // [2][2], beside a step's statistics: its first query row, its tile of dS
   const WorkSlot work{reinterpret_cast<uint4*>(bars + 24), bars + 21, bars + 22};
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -1280,7 +1332,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       mine = left;
     }
     Steps t;
-    t.g = w.y; t.b = w.z; t.k0 = kb * 128; t.sharers = sharers;
+    t.g = w.y + p.g0_c; t.b = w.z + p.b0_c; t.k0 = kb * 128; t.sharers = sharers;
     int q_first = 0;                                          // first query row that can see this key block
     if (p.causal) q_first = max(0, p.k_pos0 + t.k0 - p.q_pos0);
     t.qs0 = q_first / 128;
@@ -1307,9 +1359,8 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     mbar_init(kv_empty, 1);
     mbar_init(acc_empty, kSoftmaxWarps);
     mbar_init(work.full, 1);
-    mbar_init(work.empty, 2 + kSoftmaxWarps);
-    mbar_init(&stats_full[0], kSoftmaxWarps);
-    mbar_init(&stats_full[1], kSoftmaxWarps);
+    mbar_init(work.empty, 4 + kSoftmaxWarps);
+    for (int i = 0; i < 2; ++i) { mbar_init(&stats_full[i], 2); mbar_init(&stats_empty[i], kSoftmaxWarps); }
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -1324,6 +1375,9 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   const uint32_t tST = tmem, tDPT = tmem + 128, tDV = tmem + 256, tDK = tmem + 384;
 
   Block blk{int(blockIdx.x), int(blockIdx.y), int(blockIdx.z)};
+  // 640 threads start with 96 registers each.  A spilled one costs a trip to L2: head dim 128 leaves no L1 beside its shared memory
+  // (spills of the step loop doubled the kernel's time).
+  if (warp < 4) regs_dec<kDkvAuxRegs>();
 
   if (warp == 0) {
     // the whole warp walks the loop, one elected lane issues the copies (see producer_loop in gemm_core.cuh)
@@ -1481,97 +1535,107 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       if (ok && !work_take(work, n, blk, p.status, abort_flag)) break;
       }
       if (!ok) *abort_flag = 1;
+  } else if (warp < 4) {
+    // Per-query statistics of the steps, fetched one ahead: a thread carries -lse * log2 e and -D of two queries of a step.
+    const int q2 = threadIdx.x - 64;
+    bool ok = true;
+    uint32_t done = 0;                    // steps so far
+    for (int n = 0; ok; ++n) {
+      const Steps t = steps_of(blk);
+      int h = t.h, qs = t.qs, ld_h = t.h, ld_qs = t.qs;
+      const int per_head = n_qs - t.qs0;
+      int64_t tile = 0;
+      if (p.dS != nullptr && t.n_it > 0)
+        tile = (int64_t(t.b - p.b0_c) * p.nh_c + h - p.h0_c) * ds_tiles_before(p, (p.Skv + 127) / 128) +
+               ds_tiles_before(p, t.k0 / 128) + (qs - t.qs0);
+      float lse[2], d[2];
+      auto fetch = [&]() {
+        const size_t at = (size_t(t.b) * p.nheads + ld_h) * p.Sq;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int q = ld_qs * 128 + q2 + i * 64;
+          lse[i] = q < p.Sq ? p.LSE[at + q] : INFINITY;      // rows past the end: 2^-inf = 0
+          d[i] = q < p.Sq ? p.D[at + q] : 0.f;
+        }
+        if (++ld_qs == n_qs) { ld_qs = t.qs0; ++ld_h; }
+      };
+      if (t.n_it > 0) fetch();
+      for (int it = 0; it < t.n_it; ++it, ++done) {
+        const uint32_t sb = done & 1;
+        if (!mbar_wait_warp(&stats_empty[sb], ((done >> 1) & 1) ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
+        float* st = sStats + sb * 256;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          st[q2 + i * 64] = -lse[i] * kLog2e;
+          st[128 + q2 + i * 64] = -d[i];
+        }
+        if (q2 == 0) {
+          sStep[sb * 2] = qs * 128;
+          sStep[sb * 2 + 1] = int(tile);
+        }
+        mbar_arrive_warp(&stats_full[sb]);
+        ++tile;
+        if (++qs == n_qs) {
+          qs = t.qs0;
+          if (p.dS != nullptr) tile += ds_tiles_before(p, (p.Skv + 127) / 128) - per_head;   // the next head's
+        }
+        if (it + 1 < t.n_it) fetch();
+      }
+      if (ok && !work_take(work, n, blk, p.status, abort_flag)) break;
+    }
+    if (!ok) *abort_flag = 1;
   } else {
+    regs_inc<kDkvSoftmaxRegs>();
     const int wq = warp & 3;
-    const int half = (warp - 2) >> 2;     // warpgroup: which CPT of the step's 128 query columns these threads own
+    const int half = (warp - 4) >> 2;     // warpgroup: which CPT of the step's 128 query columns these threads own
     const int c0 = half * CPT;
     const int row = wq * 32 + lane_id();  // key row inside the block
-    const int tid = threadIdx.x - 64;     // 0..128*NWG-1 among the softmax threads; the first 256 carry the statistics
     const uint32_t lane_off = uint32_t(wq * 32) << 16;
     const float sl2 = p.scale * kLog2e;
     bool ok = true;
     int nkv = 0;                          // blocks with steps so far
     uint32_t done = 0;                    // steps so far
     for (int n = 0; ok; ++n) {
-    const Steps t = steps_of(blk);
-    const int k0 = t.k0, b = t.b, g = t.g, n_it = t.n_it, h0 = t.h0, qs0 = t.qs0, sharers = t.sharers;
-    const int k_pos = p.k_pos0 + k0 + row;
-    const bool k_valid = (k0 + row) < p.Skv;
-    // Per-query statistics of a step, fetched one step ahead: thread t < 128 carries -lse * log2 e of query t of the
-    // step, thread 128 + t carries D of query t.
-    int ld_h = t.h, ld_qs = t.qs, ld_it = 0;
-    auto load_stat = [&]() -> float {
-      float v = 0.f;
-      if (tid < 256 && ld_it < n_it) {
-        const int q = ld_qs * 128 + (tid & 127);
-        if (q >= p.Sq) {
-          v = (tid < 128) ? INFINITY : 0.f;    // rows past the end: -inf after scaling, 2^-inf = 0
-        } else {
-          const float* src = (tid < 128) ? p.LSE : p.D;
-          v = src[(size_t(b) * p.nheads + ld_h) * p.Sq + q];
-        }
-      }
-      ++ld_it;
-      if (++ld_qs == n_qs) { ld_qs = qs0; ++ld_h; }
-      return v;
-    };
-    const float stat_scale = (tid < 128) ? -kLog2e : 1.f;
-    float stat_next = load_stat();
-    if (n_it > 0) {
-      if (tid < 256) sStats[(done & 1) * 256 + tid] = stat_next * stat_scale;
-      mbar_arrive_warp(&stats_full[done & 1]);
-      stat_next = load_stat();
+    int steps = steps_of(blk).n_it, k_row;
+    {
+      const Steps t = steps_of(blk);
+      k_row = t.k0 + row;
     }
-    int cur_qs = t.qs;
     HG_DKV_TIMERS(tm_wait_a, tm_a, tm_wait_b, tm_b);
-    for (int it = 0; it < n_it; ++it, ++done) {
+    for (int it = 0; it < steps; ++it, ++done) {
       const uint32_t sb = done & 1, ph = done & 1;
       HG_DKV_TICK(t0);
-      const int qrow = cur_qs * 128;
-      if (++cur_qs == n_qs) cur_qs = qs0;
-      const float* st = sStats + sb * 256;
-      uint32_t pp[CPT / 2];               // this thread's probabilities, packed, kept for the second phase
-      float pf[kExactP ? CPT : 1];        // and in fp32, where dS^T is formed from those
+      const uint32_t st = smem_u32(sStats) + sb * 1024 + c0 * 4;
+      float pf[CPT];                      // this thread's probabilities, kept for the second phase
       // ---------------- S^T -> probabilities (kept in registers; the S^T columns are released at once)
       if (!mbar_wait_warp(&stats_full[sb], (done >> 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
       if (!mbar_wait_warp(st_full, ph, p.status, kTimeoutTmemFull, abort_flag)) { ok = false; break; }
       tc_fence_after();
       HG_DKV_TOCK(tm_wait_a, t0);
       {
-        // only steps that touch the diagonal, or a key block with rows past the end, need the mask
-        const bool need_mask = !k_valid || (p.causal && (p.q_pos0 + qrow < p.k_pos0 + k0 + 127));
-        uint32_t rr[CPT / 32][32];
-#pragma unroll
-        for (int hh = 0; hh < CPT / 32; ++hh) tmem_ld32(tST + lane_off + c0 + hh * 32, rr[hh]);
+        uint32_t r[CPT];
+        tmem_ld32(tST + lane_off + c0, r);
         tmem_ld_wait();
         tc_fence_before();
         mbar_arrive_warp(x_free);
+        // Only steps that touch the diagonal, or a key block with rows past the end, need the mask: columns before `seen` are 0.
         // The masked and the plain form are two straight-line bodies: a branch inside the element loop would cut it
         // into sixteen basic blocks, and the compiler schedules (overlaps the loads, FMAs and exp2 of different
         // elements) only inside one.
+        const int behind = p.k_pos0 + k_row - p.q_pos0 - sStep[sb * 2];       // of this row's key and the step's first query
+        const int seen = k_row >= p.Skv ? CPT : p.causal ? behind - c0 : 0;
+        const bool need_mask = (k_row - row + 128 > p.Skv) || (p.causal && behind - row + 127 > 0);
         auto probabilities = [&](auto masked) {
 #pragma unroll
-          for (int hh = 0; hh < CPT / 32; ++hh) {
-            const uint32_t(&r)[32] = rr[hh];
-            const float4* nl4 = reinterpret_cast<const float4*>(st + c0 + hh * 32);
-            const int q_base = p.q_pos0 + qrow + c0 + hh * 32;
+          for (int i = 0; i < CPT; i += 4) {
+            const float4 nl = lds_f4(st + i * 4);
 #pragma unroll
-            for (int i = 0; i < 32; i += 4) {
-              const float4 nl = nl4[i >> 2];
-              const float nlv[4] = {nl.x, nl.y, nl.z, nl.w};
-              float e[4];
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const float x = fmaf(__uint_as_float(r[i + u]), sl2, nlv[u]);
-                e[u] = (u < HG_DKV_POLY_OF_4) ? ex2_poly(x) : ex2(x);
-                if (decltype(masked)::value && (!k_valid || (p.causal && k_pos > q_base + i + u))) e[u] = 0.f;
-              }
-              if constexpr (kExactP) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) pf[hh * 32 + i + u] = e[u];
-              }
-              pp[hh * 16 + (i >> 1)] = pack_bf16(e[0], e[1]);
-              pp[hh * 16 + (i >> 1) + 1] = pack_bf16(e[2], e[3]);
+            for (int u = 0; u < 4; u += 2) {
+              const float2 x = fma2(make_float2(__uint_as_float(r[i + u]), __uint_as_float(r[i + u + 1])), make_float2(sl2, sl2),
+                                    u == 0 ? make_float2(nl.x, nl.y) : make_float2(nl.z, nl.w));
+              const float e0 = ex2(x.x), e1 = ex2(x.y);
+              pf[i + u] = decltype(masked)::value && i + u < seen ? 0.f : e0;
+              pf[i + u + 1] = decltype(masked)::value && i + u + 1 < seen ? 0.f : e1;
             }
           }
         };
@@ -1583,53 +1647,63 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
       if (!mbar_wait_warp(dpt_full, ph, p.status, kTimeoutTmemFull, abort_flag)) { ok = false; break; }
       tc_fence_after();
       HG_DKV_TOCK(tm_wait_b, t0);
+      static_assert(CPT == 32, "P^T takes the columns of the first half of dP^T, dS^T those of the second");
+      uint32_t dsp[CPT / 2];
       {
-        uint32_t dsp[CPT / 2];
-        uint32_t rr[CPT / 32][32];
+        const uint32_t dpt = tDPT + lane_off + c0;
+        uint32_t ra[16], rb[16];
+        auto half_ds = [&](const uint32_t(&r)[16], int at) {
 #pragma unroll
-        for (int hh = 0; hh < CPT / 32; ++hh) tmem_ld32(tDPT + lane_off + c0 + hh * 32, rr[hh]);
+          for (int i = 0; i < 16; i += 4) {
+            const float4 nd = lds_f4(st + 512 + (at + i) * 4);
+#pragma unroll
+            for (int u = 0; u < 4; u += 2) {
+              const float2 d = mul2(make_float2(pf[at + i + u], pf[at + i + u + 1]),
+                                    add2(make_float2(__uint_as_float(r[i + u]), __uint_as_float(r[i + u + 1])),
+                                         u == 0 ? make_float2(nd.x, nd.y) : make_float2(nd.z, nd.w)));
+              dsp[(at + i + u) >> 1] = pack_bf16(d.x, d.y);
+            }
+          }
+        };
+        tmem_ld16(dpt, ra);
         tmem_ld_wait();
-        if constexpr (CPT == 64) tmem_st32(tDPT + lane_off + c0, pp);
-        else tmem_st16(tDPT + lane_off + c0, pp);
+        {
+          uint32_t pp[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) pp[i] = pack_bf16(pf[2 * i], pf[2 * i + 1]);
+          tmem_st16(dpt, pp);
+        }
+        tmem_ld16(dpt + 16, rb);
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive_warp(p_full);
+        half_ds(ra, 0);
+        if (p.dS != nullptr) {
+          hg_lp_t* out = p.dS + int64_t(sStep[sb * 2 + 1]) * (128 * 128) + ((row >> 6) * (64 * 128) + c0 * 64 + (row & 63) * 8);
 #pragma unroll
-        for (int hh = 0; hh < CPT / 32; ++hh) {
-          const uint32_t(&r)[32] = rr[hh];
-          const float4* dd4 = reinterpret_cast<const float4*>(st + 128 + c0 + hh * 32);
-#pragma unroll
-          for (int i = 0; i < 32; i += 4) {
-            const float4 dd = dd4[i >> 2];
-            float2 p01, p23;
-            if constexpr (kExactP) {
-              p01 = make_float2(pf[hh * 32 + i], pf[hh * 32 + i + 1]);
-              p23 = make_float2(pf[hh * 32 + i + 2], pf[hh * 32 + i + 3]);
-            } else {
-              p01 = hg_unpack2(pp[hh * 16 + (i >> 1)]);
-              p23 = hg_unpack2(pp[hh * 16 + (i >> 1) + 1]);
-            }
-            dsp[hh * 16 + (i >> 1)] = pack_bf16(p01.x * (__uint_as_float(r[i]) - dd.x),
-                                                 p01.y * (__uint_as_float(r[i + 1]) - dd.y));
-            dsp[hh * 16 + (i >> 1) + 1] = pack_bf16(p23.x * (__uint_as_float(r[i + 2]) - dd.z),
-                                                     p23.y * (__uint_as_float(r[i + 3]) - dd.w));
-          }
+          for (int i = 0; i < 2; ++i)
+            *reinterpret_cast<uint4*>(out + i * 512) = make_uint4(dsp[4 * i], dsp[4 * i + 1], dsp[4 * i + 2], dsp[4 * i + 3]);
         }
-        if constexpr (CPT == 64) tmem_st32(tDPT + lane_off + c0 + CPT / 2, dsp);
-        else tmem_st16(tDPT + lane_off + c0 + CPT / 2, dsp);
-      }
-      // the next step's statistics go to the other buffer: its last readers were the second phases of step it-1,
-      // and every thread finished that before it arrived on this step's statistics barrier
-      if (it + 1 < n_it) {
-        if (tid < 256) sStats[(sb ^ 1) * 256 + tid] = stat_next * stat_scale;
-        mbar_arrive_warp(&stats_full[sb ^ 1]);
-        stat_next = load_stat();
+        tmem_ld_wait();
+        half_ds(rb, 16);
+        tmem_st16(dpt + 16, dsp);
+        if (p.dS != nullptr) {
+          hg_lp_t* out = p.dS + int64_t(sStep[sb * 2 + 1]) * (128 * 128) + ((row >> 6) * (64 * 128) + c0 * 64 + (row & 63) * 8);
+#pragma unroll
+          for (int i = 2; i < 4; ++i)
+            *reinterpret_cast<uint4*>(out + i * 512) = make_uint4(dsp[4 * i], dsp[4 * i + 1], dsp[4 * i + 2], dsp[4 * i + 3]);
+        }
       }
       tmem_st_wait();
       tc_fence_before();
       mbar_arrive_warp(ds_full);
+      mbar_arrive_warp(&stats_empty[sb]);
       HG_DKV_TOCK(tm_b, t0);
     }
+    // the epilogue's numbers are worked out again instead of being kept through the steps, where registers are short
+    asm volatile("" : "+r"(blk.x), "+r"(blk.y), "+r"(blk.z));
+    const Steps t = steps_of(blk);
+    const int k0 = t.k0, b = t.b, g = t.g, n_it = t.n_it, h0 = t.h0, sharers = t.sharers;
     HG_DKV_REPORT(0, n_it, tm_wait_a, tm_a, tm_wait_b, tm_b);
     // ---- epilogue ----
     const int krow = k0 + row;
@@ -2058,6 +2132,236 @@ flash_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   }
 }
 
+// =================================================================================================
+// Backward, part 2 where the dK/dV kernel has left dS in memory: dQ = dS K, a product with nothing to recompute.  Against S, dP
+// and the exponentials a second time (flash_bwd_dq128_kernel: 24 MMAs and 16384 exponentials per 128 x 128 pair) it takes 8 MMAs
+// and reads 32 KB of dS, which bounds it: HBM, and 64 bytes a cycle into an SM, for which a CTA takes 256 queries whose two tiles
+// share the keys (48 KB a pair).  us, causal, dK/dV kernel + dQ kernel, without dS in memory / with: head dim 128, 2 x 4096 and 32
+// heads 518 + 381 / 603 + 203 (the power limit holds the clock at 1.7 GHz, and the stores cost power), 1531 and 28 heads on 4
+// 49 + 42 / 57 + 20; head dim 64, 8 x 1024 and 25 heads 106 + 89 / 113 + 51.  dS is read at 5.4 TB/s at the first of these.
+// A unit of work is 256 queries of a head, a block of the grid, longest first; CTAs take further ones (WorkSlot; dealt out in turn,
+// a CTA had up to 1.3 times the mean), and the four stages of 64 keys run on across them.  Two accumulators of two tiles fill tensor memory (head dim 128), so that a unit's results leave under the next one's
+// products.  Roles: warp 0 TMA, warp 1 MMA, warps 2-5 epilogue.
+// =================================================================================================
+// 128 queries x 16 keys of a half tile of dS (see BwdParams::dS) at `saddr`: 8 x 8 blocks of 128 bytes, 128 bytes apart along the
+// keys and 1024 along the queries, no swizzle.
+__device__ __forceinline__ uint64_t plain_mn_desc(uint32_t saddr) {
+  return (uint64_t(1) << 46) | uint64_t((saddr & 0x3FFFF) >> 4) | (uint64_t(128 >> 4) << 16) | (uint64_t(1024 >> 4) << 32);
+}
+// `bytes` in a row into shared memory; both addresses and the size are multiples of 16.
+__device__ __forceinline__ void bulk_load(void* smem_dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               :
+               : "r"(smem_u32(smem_dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+template <int HD>
+struct DqDsSmem {
+  static constexpr int kTile = 128 * 64 * 2;       // dS^T of 64 keys x 128 queries
+  static constexpr int kK = 64 * HD * 2;
+  static constexpr int kStages = 4;
+  static constexpr int kStage = 2 * kTile + kK;
+  static constexpr int kTotal = kStages * kStage + 1024 + 256;
+};
+
+template <int HD>
+__global__ void __launch_bounds__(192, 1)
+flash_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmK, const BwdParams p, int heads) {
+  extern __shared__ uint8_t smem_raw[];
+  using L = DqDsSmem<HD>;
+  constexpr int NS = L::kStages;
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + NS * L::kStage);
+  uint64_t* full = bars;                 // 4
+  uint64_t* empty = bars + 4;            // 4
+  uint64_t* acc_full = bars + 8;         // 2
+  uint64_t* acc_empty = bars + 10;       // 2
+  const WorkSlot work{reinterpret_cast<uint4*>(bars + 14), bars + 12, bars + 13};
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5;
+  const int n_qs = (p.Sq + 127) / 128, n_kb = (p.Skv + 127) / 128, n_pairs = (n_qs + 1) / 2;
+  const int64_t head_tiles = ds_tiles_before(p, n_kb);
+
+  struct Unit {
+    int qb, h, b, kbs[2];        // first query block, head, sequence; key blocks that each of the two query blocks sees
+    int64_t head;                // among the heads of this launch
+  };
+  auto key_blocks = [&](int qb) {
+    if (qb >= n_qs) return 0;
+    if (!p.causal) return n_kb;
+    const int keys = p.q_pos0 + qb * 128 + 128 - p.k_pos0;       // before the first that no row of the block sees
+    return keys <= 0 ? 0 : min(n_kb, (keys + 127) / 128);
+  };
+  auto unit_at = [&](int u) {
+    Unit w;
+    // some heads at a time, the last ones, whose dS may still be in L2, first
+    const int some = (2 * 148 + n_pairs - 1) / n_pairs, first = u / (some * n_pairs) * some, n = min(some, heads - first);
+    const int r = u - first * n_pairs, pair = n_pairs - 1 - r / n, hb = heads - 1 - first - r % n;
+    w.qb = 2 * pair;
+    w.head = hb;
+    w.b = p.b0_c + hb / p.nh_c;
+    w.h = p.h0_c + hb % p.nh_c;
+    w.kbs[0] = key_blocks(w.qb);
+    w.kbs[1] = key_blocks(w.qb + 1);
+    return w;
+  };
+  // Key blocks of a unit in the order of both roles: the second query block sees at least those of the first, where it exists.
+  auto most = [](const Unit& w) { return max(w.kbs[0], w.kbs[1]); };
+
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tmK);
+    for (int i = 0; i < NS; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+    mbar_init(work.full, 1);
+    mbar_init(work.empty, 6);
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 4 * HD);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  Block blk{int(blockIdx.x), 0, 0};
+
+  if (warp == 0) {
+    const bool issuer = elect_one() != 0;
+    uint32_t stage = 0, phase = 0;
+    bool ok = true, asked = false;
+    int n_done = 0;
+    for (; ok; ++n_done) {
+      asked = false;
+      const Unit w = unit_at(blk.x);
+      const int kslot = p.kmap.slot(w.h, p.qpg), n = most(w);
+      for (int kb = 0; ok && kb < n; ++kb) {
+        // a first query block that does not see this key block has no tile: this is then the one before the second's
+        const hg_lp_t* src = p.dS + (w.head * head_tiles + ds_tiles_before(p, kb) + w.qb - ds_first_query_block(p, kb)) * (128 * 128);
+        for (int half = 0; half < 2; ++half) {
+          if (!mbar_wait_warp(&empty[stage], phase ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
+          uint8_t* s = base + stage * L::kStage;
+          if (issuer) {
+            mbar_expect_tx(&full[stage], (int(kb < w.kbs[0]) + int(kb < w.kbs[1])) * L::kTile + L::kK);
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+              if (kb < w.kbs[j]) bulk_load(s + j * L::kTile, src + (2 * j + half) * (64 * 128), L::kTile, &full[stage]);
+#pragma unroll
+            for (int c = 0; c < HD / 64; ++c)
+              tma_load_4d(s + 2 * L::kTile + c * 64 * 128, &tmK, &full[stage], c * 64, kslot, kb * 128 + half * 64, w.b);
+          }
+          __syncwarp();
+          if (++stage == NS) { stage = 0; phase ^= 1; }
+        }
+      }
+      if (!ok) break;
+      if (n_done > 0 && !mbar_wait_warp(work.empty, (n_done - 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
+      if (issuer) work_request(work);
+      __syncwarp();
+      asked = true;
+      if (!work_take(work, n_done, blk, p.status, abort_flag)) break;
+    }
+    for (int i = 0; ok && i < NS; ++i) {          // leave when the last commits have arrived
+      ok = mbar_wait_warp(&empty[stage], phase ^ 1, p.status, kTimeoutSmemEmpty, abort_flag);
+      if (++stage == NS) { stage = 0; phase ^= 1; }
+    }
+    if (!ok) {
+      *abort_flag = 1;
+      if (asked) work_drain(work, n_done);
+      const uint64_t t0 = globaltimer_ns();
+      while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);  // 2 ms for copies in flight: far longer than a tile load
+    }
+  } else if (warp == 1) {
+    const bool issuer = elect_one() != 0;
+    constexpr uint32_t idesc = make_idesc_lp(128, HD, true, true);
+    uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
+    bool ok = true;
+    for (int n_done = 0; ok; ++n_done) {
+      const Unit w = unit_at(blk.x);
+      const int n = most(w);
+      if (n > 0) {
+      if (!mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1, p.status, kTimeoutTmemEmpty, abort_flag)) { ok = false; break; }
+      tc_fence_after();
+      for (int hs = 0; hs < 2 * n; ++hs) {
+        if (!mbar_wait_warp(&full[stage], phase, p.status, kTimeoutSmemFull, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t s = smem_u32(base + stage * L::kStage), k = s + 2 * L::kTile;
+        if (issuer) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            if (hs < 2 * w.kbs[j]) {
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk)
+                umma_f16_ss(tmem + (acc * 2 + j) * HD, plain_mn_desc(s + j * L::kTile + kk * 256),
+                            make_smem_desc(k + kk * 2048, 64 * 128, 1024), idesc, (hs | kk) != 0);
+            }
+          umma_commit(&empty[stage]);
+        }
+        __syncwarp();
+        if (++stage == NS) { stage = 0; phase ^= 1; }
+      }
+      if (!ok) break;
+      if (issuer) umma_commit(&acc_full[acc]);
+      __syncwarp();
+      if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      }
+      if (!work_take(work, n_done, blk, p.status, abort_flag)) break;
+    }
+    if (!ok) *abort_flag = 1;
+  } else {
+    const int wq = warp & 3, row = wq * 32 + lane_id();
+    const uint32_t lane_off = uint32_t(wq * 32) << 16;
+    uint32_t acc = 0, acc_phase = 0;
+    for (int n_done = 0;; ++n_done) {
+      const Unit w = unit_at(blk.x);
+      const bool any = most(w) > 0;
+      if (any && !mbar_wait_warp(&acc_full[acc], acc_phase, p.status, kTimeoutTmemFull, abort_flag)) { *abort_flag = 1; break; }
+      tc_fence_after();
+#pragma unroll 1
+      for (int j = 0; j < 2; ++j) {
+        const int q = (w.qb + j) * 128 + row;
+        hg_lp_t* dq = p.dQ + int64_t(q) * p.dq_ss + int64_t(w.b) * p.dq_sb + int64_t(p.dqmap.slot(w.h, p.qpg)) * HD;
+#pragma unroll 1
+        for (int c = 0; c < HD / 32; ++c) {
+          uint32_t r[32];
+          tmem_ld32(tmem + lane_off + (acc * 2 + j) * HD + c * 32, r);
+          tmem_ld_wait();
+          if (q < p.Sq) {
+            const float scale = p.scale;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint4 v = make_uint4(0, 0, 0, 0);                      // queries that see no key
+              if (w.kbs[j] > 0) {
+                v.x = pack_bf16(__uint_as_float(r[i * 8 + 0]) * scale, __uint_as_float(r[i * 8 + 1]) * scale);
+                v.y = pack_bf16(__uint_as_float(r[i * 8 + 2]) * scale, __uint_as_float(r[i * 8 + 3]) * scale);
+                v.z = pack_bf16(__uint_as_float(r[i * 8 + 4]) * scale, __uint_as_float(r[i * 8 + 5]) * scale);
+                v.w = pack_bf16(__uint_as_float(r[i * 8 + 6]) * scale, __uint_as_float(r[i * 8 + 7]) * scale);
+              }
+              reinterpret_cast<uint4*>(dq + c * 32)[i] = v;
+            }
+          }
+          __syncwarp();
+        }
+      }
+      if (any) {
+        tc_fence_before();
+        mbar_arrive_warp(&acc_empty[acc]);
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+      }
+      if (!work_take(work, n_done, blk, p.status, abort_flag)) break;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 4 * HD);
+  }
+}
+
 }  // namespace attn
 }  // namespace hg
 
@@ -2163,9 +2467,9 @@ int dkv_chunk_steps(BwdParams p, int Skv, int nkv) {
 
 template <int HD>
 int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-               const BwdParams& p, int Skv, int nkv, bool wide, cudaStream_t st) {
+               const BwdParams& p, int Skv, int nkv, int nb, bool wide, cudaStream_t st) {
   int rc;
-  dim3 grid((Skv + 127) / 128, nkv, p.B);
+  dim3 grid((Skv + 127) / 128, nkv, nb);
   if (wide) {
     const int blocks = int(grid.x);
     if (p.chunk > 0) grid.x = unsigned(dkv_ctas(p, blocks));
@@ -2173,8 +2477,8 @@ int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     const bool shared = p.chunk > 0;
     auto k = shared ? flash_bwd_dkv128_kernel<HD, kDkvWarpgroups, true> : flash_bwd_dkv128_kernel<HD, kDkvWarpgroups, false>;
     if (!cfg[shared]) { if ((rc = set_smem(k, Dkv128Smem<HD>::kTotal))) return rc; cfg[shared] = true; }
-    k<<<grid, 64 + 128 * kDkvWarpgroups, Dkv128Smem<HD>::kTotal, st>>>(tq, tk, tv, tdo, p);
-    if (p.chunk > 0) dkv_sum_kernel<HD><<<dim3(blocks * 8, nkv, p.B), 4 * HD, 0, st>>>(p, int(grid.x));
+    k<<<grid, 128 + 128 * kDkvWarpgroups, Dkv128Smem<HD>::kTotal, st>>>(tq, tk, tv, tdo, p);
+    if (p.chunk > 0) dkv_sum_kernel<HD><<<dim3(blocks * 8, nkv, nb), 4 * HD, 0, st>>>(p, int(grid.x));
   } else {
     static bool cfg = false;
     if (!cfg) { if ((rc = set_smem(flash_bwd_dkv_kernel<HD>, DkvSmem<HD>::kTotal))) return rc; cfg = true; }
@@ -2192,6 +2496,55 @@ int launch_dq(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& t
   if (!cfg) { if ((rc = set_smem(k, Dq128Smem<HD>::kTotal))) return rc; cfg = true; }
   k<<<dim3((p.Sq + 127) / 128, p.nheads, p.B), 64 + 128 * kDqWarpgroups, Dq128Smem<HD>::kTotal, st>>>(tq, tk, tv, tdo, p);
   return int(cudaGetLastError());
+}
+
+template <int HD>
+int launch_dq_ds(const CUtensorMap& tk, const BwdParams& p, int nb, cudaStream_t st) {
+  int rc;
+  static bool cfg = false;
+  auto k = flash_bwd_dq_ds_kernel<HD>;
+  if (!cfg) { if ((rc = set_smem(k, DqDsSmem<HD>::kTotal))) return rc; cfg = true; }
+  const int heads = p.nh_c * nb, units = ((p.Sq + 255) / 256) * heads;
+  k<<<units, 192, DqDsSmem<HD>::kTotal, st>>>(tk, p, heads);
+  return int(cudaGetLastError());
+}
+
+// How the heads of a backward are cut where dS^T goes through memory: launches of `nb` sequences and `ng` kv heads each, whose
+// tiles fit kDsMost.  ng = 0: not even one kv head's do, and the dQ kernel recomputes S and dP.
+constexpr long long kDsTile = 128 * 128 * 2, kDsMost = 3ll << 29;
+struct DsCut {
+  int nb, ng;
+  long long bytes;
+};
+DsCut ds_cut(const BwdParams& p, int Skv, int nkv) {
+  const long long group = ds_tiles_before(p, (Skv + 127) / 128) * p.qpg * kDsTile;
+  if (g_dkv_variant != 0 || group > kDsMost) return {0, 0, 0};
+  if (group == 0) return {p.B, nkv, 0};
+  const long long groups = kDsMost / group;
+  DsCut c;
+  c.ng = groups < nkv ? int(groups) : nkv;
+  c.nb = groups < nkv ? 1 : groups / nkv < p.B ? int(groups / nkv) : p.B;
+  if (p.chunk > 0 && (c.ng < nkv || c.nb < p.B)) return {0, 0, 0};     // shared key blocks are few: they are launched at once
+  const int times = (nkv + c.ng - 1) / c.ng;
+  c.ng = (nkv + times - 1) / times;                                     // launches of about the same size
+  c.bytes = group * c.ng * c.nb;
+  return c;
+}
+// The scratch of a backward, in floats: row sums of dO * O, parts of dK and dV, tiles of dS^T.
+struct BwdScratch {
+  long long sums, parts, ds;
+  int chunk;
+  DsCut cut;
+};
+BwdScratch bwd_scratch(BwdParams p, int Skv, int nkv, int hd) {
+  BwdScratch w{};
+  w.sums = ((long long)p.B * p.nheads * p.Sq + 63) / 64 * 64;
+  if (g_dkv_variant != 0) return w;
+  w.chunk = p.chunk = dkv_chunk_steps(p, Skv, nkv);
+  if (w.chunk) w.parts = (long long)dkv_ctas(p, (Skv + 127) / 128) * nkv * p.B * 2 * 128 * hd;
+  w.cut = ds_cut(p, Skv, nkv);
+  w.ds = w.cut.bytes / 4;
+  return w;
 }
 
 }  // namespace
@@ -2235,28 +2588,32 @@ int hg_attn_set_dkv_variant(int v) {
   return old;
 }
 
-// Floats of scratch that hg_flash_bwd_ws asks for: the row sums of dO * O, [B, nheads, Sq], and where key blocks are shared
-// the parts of dK and dV.
-long long hg_flash_bwd_scratch(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
+// Floats of scratch that hg_flash_bwd_ws asks for: the row sums of dO * O, [B, nheads, Sq], where key blocks are shared the parts
+// of dK and dV, and, if `tiles`, dS^T of up to kDsMost bytes.
+long long hg_flash_bwd_scratch_of(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0, int tiles) {
   if (Sq <= 0 || Skv <= 0 || B <= 0 || nheads <= 0 || nkv <= 0) return 0;
   BwdParams p{};
-  p.Sq = Sq; p.Skv = Skv; p.B = B; p.qpg = nheads / nkv; p.causal = causal; p.q_pos0 = q_pos0; p.k_pos0 = k_pos0;
-  const long long sums = ((long long)B * nheads * Sq + 3) / 4 * 4;
-  if (g_dkv_variant != 0 || !(p.chunk = dkv_chunk_steps(p, Skv, nkv))) return sums;
-  return sums + (long long)dkv_ctas(p, (Skv + 127) / 128) * nkv * B * 2 * 128 * hd;
+  p.Sq = Sq; p.Skv = Skv; p.B = B; p.nheads = nheads; p.qpg = nheads / nkv; p.causal = causal; p.q_pos0 = q_pos0; p.k_pos0 = k_pos0;
+  const BwdScratch w = bwd_scratch(p, Skv, nkv, hd);
+  return w.sums + w.parts + (tiles ? w.ds : 0);
+}
+long long hg_flash_bwd_scratch(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
+  return hg_flash_bwd_scratch_of(Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0, 1);
 }
 
 // ws: scratch of ws_floats fp32 values, 16-byte aligned, at least [B, nheads, Sq] (filled here with rowsum(dO*O)).  With less
-// than hg_flash_bwd_scratch floats every key block has one CTA.
+// than hg_flash_bwd_scratch floats S and dP are computed again for dQ, and with less than hg_flash_bwd_scratch_of(.., 0) every
+// key block has one CTA.  launched (may be null): the kernels that were launched.
 int hg_flash_bwd_ws(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o,
                     const HgAttnTensor* d_o, const void* lse, void* ws, long long ws_floats, const HgAttnTensor* dq,
                     const HgAttnTensor* dk, const HgAttnTensor* dv, int Sq, int Skv, int B, int nheads, int nkv, int hd,
-                    int causal, int q_pos0, int k_pos0, float scale, void* stream) {
+                    int causal, int q_pos0, int k_pos0, float scale, int* launched, void* stream) {
   void* dsum = ws;
+  if (launched != nullptr) *launched = 0;
   if (hd != 64 && hd != 128) return -1;
   if (Sq <= 0 || Skv <= 0 || B <= 0) return 0;
   cudaStream_t st = (cudaStream_t)stream;
-  int rc;
+  int rc, kernels = 1;
   {
     const bool vec = (((uintptr_t(o->ptr) | uintptr_t(d_o->ptr)) & 15) | ((o->ss | o->sb | d_o->ss | d_o->sb) & 7)) == 0;
     const int64_t rows = int64_t(Sq) * B * nheads;
@@ -2277,29 +2634,42 @@ int hg_flash_bwd_ws(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTe
   p.dK = (hg_lp_t*)dk->ptr; p.dk_ss = dk->ss; p.dk_sb = dk->sb; p.dkmap = {dk->gs, dk->hs, dk->off};
   p.dV = (hg_lp_t*)dv->ptr; p.dv_ss = dv->ss; p.dv_sb = dv->sb; p.dvmap = {dv->gs, dv->hs, dv->off};
   p.status = hg_host::status_ptr();
-  const long long need = hg_flash_bwd_scratch(Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0);
-  const long long sums = ((long long)B * nheads * Sq + 3) / 4 * 4;
-  if (need > sums && ws_floats >= need && (reinterpret_cast<uintptr_t>(ws) & 15) == 0) {
-    p.chunk = dkv_chunk_steps(p, Skv, nkv);
-    p.part = static_cast<float*>(ws) + sums;
+  const BwdScratch w = bwd_scratch(p, Skv, nkv, hd);
+  const bool aligned = (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
+  if (w.parts > 0 && aligned && ws_floats >= w.sums + w.parts) {
+    p.chunk = w.chunk;
+    p.part = static_cast<float*>(ws) + w.sums;
   }
-  {
-    CUtensorMap tq, tk, tv, tdo;
-    const bool wide = g_dkv_variant == 0;   // 128-query steps, P^T / dS^T in tensor memory
-    const int q_rows = wide ? 128 : 64;
-    if ((rc = make_map(&tq, q->ptr, hd, q->slots, Sq, B, q->ss, q->sb, q_rows))) return rc;
-    if ((rc = make_map(&tk, k->ptr, hd, k->slots, Skv, B, k->ss, k->sb, 128))) return rc;
-    if ((rc = make_map(&tv, v->ptr, hd, v->slots, Skv, B, v->ss, v->sb, 128))) return rc;
-    if ((rc = make_map(&tdo, d_o->ptr, hd, d_o->slots, Sq, B, d_o->ss, d_o->sb, q_rows))) return rc;
-    if ((rc = hd == 128 ? launch_dkv<128>(tq, tk, tv, tdo, p, Skv, nkv, wide, st)
-                        : launch_dkv<64>(tq, tk, tv, tdo, p, Skv, nkv, wide, st))) return rc;
-  }
-  CUtensorMap tq, tk, tv, tdo;
-  if ((rc = make_map(&tq, q->ptr, hd, q->slots, Sq, B, q->ss, q->sb, 128))) return rc;
+  const bool tiles = w.ds > 0 && aligned && ws_floats >= w.sums + w.parts + w.ds;
+  if (tiles) p.dS = reinterpret_cast<hg_lp_t*>(static_cast<float*>(ws) + w.sums + w.parts);
+  const DsCut cut = tiles ? w.cut : DsCut{B, nkv, 0};
+  CUtensorMap tq, tk, tv, tdo, tk64;
+  const bool wide = g_dkv_variant == 0;   // 128-query steps, P^T / dS^T in tensor memory
+  const int q_rows = wide ? 128 : 64;
+  if ((rc = make_map(&tq, q->ptr, hd, q->slots, Sq, B, q->ss, q->sb, q_rows))) return rc;
   if ((rc = make_map(&tk, k->ptr, hd, k->slots, Skv, B, k->ss, k->sb, 128))) return rc;
   if ((rc = make_map(&tv, v->ptr, hd, v->slots, Skv, B, v->ss, v->sb, 128))) return rc;
-  if ((rc = make_map(&tdo, d_o->ptr, hd, d_o->slots, Sq, B, d_o->ss, d_o->sb, 128))) return rc;
-  return hd == 128 ? launch_dq<128>(tq, tk, tv, tdo, p, st) : launch_dq<64>(tq, tk, tv, tdo, p, st);
+  if ((rc = make_map(&tdo, d_o->ptr, hd, d_o->slots, Sq, B, d_o->ss, d_o->sb, q_rows))) return rc;
+  if (tiles && (rc = make_map(&tk64, k->ptr, hd, k->slots, Skv, B, k->ss, k->sb, 64))) return rc;
+  for (int b0 = 0; b0 < B; b0 += cut.nb)
+    for (int g0 = 0; g0 < nkv; g0 += cut.ng) {
+      const int nb = B - b0 < cut.nb ? B - b0 : cut.nb, ng = nkv - g0 < cut.ng ? nkv - g0 : cut.ng;
+      p.b0_c = b0; p.g0_c = g0; p.h0_c = g0 * p.qpg; p.nh_c = ng * p.qpg;
+      if ((rc = hd == 128 ? launch_dkv<128>(tq, tk, tv, tdo, p, Skv, ng, nb, wide, st)
+                          : launch_dkv<64>(tq, tk, tv, tdo, p, Skv, ng, nb, wide, st))) return rc;
+      kernels += p.chunk > 0 ? 2 : 1;
+      if (!tiles) continue;
+      if ((rc = hd == 128 ? launch_dq_ds<128>(tk64, p, nb, st) : launch_dq_ds<64>(tk64, p, nb, st))) return rc;
+      ++kernels;
+    }
+  if (!tiles) {
+    if ((rc = make_map(&tq, q->ptr, hd, q->slots, Sq, B, q->ss, q->sb, 128))) return rc;
+    if ((rc = make_map(&tdo, d_o->ptr, hd, d_o->slots, Sq, B, d_o->ss, d_o->sb, 128))) return rc;
+    if ((rc = hd == 128 ? launch_dq<128>(tq, tk, tv, tdo, p, st) : launch_dq<64>(tq, tk, tv, tdo, p, st))) return rc;
+    ++kernels;
+  }
+  if (launched != nullptr) *launched = kernels;
+  return 0;
 }
 
 // dsum: scratch [B, nheads, Sq] fp32 (filled here with rowsum(dO*O)); every key block has one CTA.
@@ -2308,7 +2678,7 @@ int hg_flash_bwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTenso
                  const HgAttnTensor* dv, int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0,
                  int k_pos0, float scale, void* stream) {
   return hg_flash_bwd_ws(q, k, v, o, d_o, lse, dsum, 0, dq, dk, dv, Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0,
-                         scale, stream);
+                         scale, nullptr, stream);
 }
 
 }  // extern "C"

@@ -51,9 +51,13 @@ def attention_reference(q, k, v, causal=True, scale=None, q_pos0=0, k_pos0=0, dr
 
 
 def _backward_scratch(lib, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, device) -> torch.Tensor:
-    """fp32 scratch of the backward kernels: row sums of dO * O and, where key blocks are shared between CTAs, their parts."""
-    n = lib.hg_flash_bwd_scratch(S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0)
-    return torch.empty(n, dtype=torch.float32, device=device)
+    """fp32 scratch of the backward kernels: row sums of dO * O, where key blocks are shared between CTAs their parts, and dS,
+    without which, should there be no room for it, dQ takes longer."""
+    args = (S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0)
+    try:
+        return torch.empty(lib.hg_flash_bwd_scratch(*args), dtype=torch.float32, device=device)
+    except torch.cuda.OutOfMemoryError:
+        return torch.empty(lib.hg_flash_bwd_scratch_of(*args, 0), dtype=torch.float32, device=device)
 
 
 class _FlashPacked(torch.autograd.Function):
@@ -98,11 +102,13 @@ class _FlashPacked(torch.autograd.Function):
         dq = _desc(dqkv, ss, sb, slots, qpg + 2, 1, 0)
         dk = _desc(dqkv, ss, sb, slots, qpg + 2, 0, qpg)
         dv = _desc(dqkv, ss, sb, slots, qpg + 2, 0, qpg + 1)
+        kernels = ctypes.c_int()
         rc = lib.hg_flash_bwd_ws(ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(o), ctypes.byref(do),
                                  lse.data_ptr(), ws.data_ptr(), ws.numel(), ctypes.byref(dq), ctypes.byref(dk),
-                                 ctypes.byref(dv), S, S, B, nh, ng, hd, int(causal), 0, 0, float(scale), _lib.stream())
+                                 ctypes.byref(dv), S, S, B, nh, ng, hd, int(causal), 0, 0, float(scale),
+                                 ctypes.byref(kernels), _lib.stream())
         _lib.check(rc, "hg_flash_bwd")
-        _lib.count_launch(4 if ws.numel() > B * nh * S + 3 else 3)
+        _lib.count_launch(kernels.value)
         return dqkv, None, None, None, None, None, None, None
 
 
@@ -281,12 +287,13 @@ def flash_backward(q, k, v, out, dout, lse, causal, scale, q_pos0=0, k_pos0=0):
     dqd = _desc(dq, dq.stride(0), dq.stride(1), nh, qpg, 1, 0)
     dkd = _desc(dk, dk.stride(0), dk.stride(1), ng, 1, 0, 0)
     dvd = _desc(dv, dv.stride(0), dv.stride(1), ng, 1, 0, 0)
+    kernels = ctypes.c_int()
     rc = lib.hg_flash_bwd_ws(ctypes.byref(qd), ctypes.byref(kd), ctypes.byref(vd), ctypes.byref(od), ctypes.byref(dod),
                              lse.data_ptr(), ws.data_ptr(), ws.numel(), ctypes.byref(dqd), ctypes.byref(dkd),
                              ctypes.byref(dvd), S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0, float(scale),
-                             _lib.stream())
+                             ctypes.byref(kernels), _lib.stream())
     _lib.check(rc, "hg_flash_bwd")
-    _lib.count_launch(4 if ws.numel() > B * nh * S + 3 else 3)
+    _lib.count_launch(kernels.value)
     return dq, dk, dv
 
 

@@ -56,3 +56,32 @@ def test_shared_key_blocks(hd, Sq, Skv, B, nh, ng, causal, q0, k0):
         # two 16-bit roundings before a product, one after (see test_attention_hd64_gpu)
         assert rel_err(dk, kr.grad) < 5e-3 and rel_err(dv, vr.grad) < 5e-3
     _lib.assert_healthy()
+
+
+# dS in memory: launches over some of the heads, or of the sequences, where all tiles are too many (1.5 GiB), a last one smaller than
+# the others; one query block, one row more than two, an odd number of them; rows and keys that end inside a block
+@pytest.mark.parametrize("Sq,Skv,B,nh,ng,hd,causal,q0,k0", [
+    (8192, 8192, 1, 32, 32, 64, True, 0, 0), (4096, 4096, 3, 16, 8, 64, False, 0, 0), (8192, 8192, 2, 25, 25, 128, True, 0, 0),
+    (1, 1, 1, 1, 1, 128, True, 0, 0), (128, 65, 2, 3, 1, 64, True, 0, 0), (257, 257, 1, 2, 2, 128, True, 0, 0),
+    (640, 200, 2, 4, 2, 128, False, 0, 0), (385, 1000, 1, 4, 4, 64, True, 615, 0), (300, 300, 1, 2, 1, 128, True, 0, 900)])
+def test_dq_from_stored_ds(Sq, Skv, B, nh, ng, hd, causal, q0, k0):
+    lib = _lib.load()
+    sizes = (Sq, Skv, B, nh, ng, hd, int(causal), q0, k0)
+    assert lib.hg_flash_bwd_scratch(*sizes) > lib.hg_flash_bwd_scratch_of(*sizes, 0) or k0 > q0 + Sq    # pairs to store
+    assert 4 * (lib.hg_flash_bwd_scratch(*sizes) - lib.hg_flash_bwd_scratch_of(*sizes, 0)) <= 3 << 29
+    g = torch.Generator(device=DEV).manual_seed(Sq + Skv + hd)
+    q, dout = (torch.randn(Sq, B, nh, hd, device=DEV, generator=g).to(torch.bfloat16) for _ in "qd")
+    k, v = (torch.randn(Skv, B, ng, hd, device=DEV, generator=g).to(torch.bfloat16) for _ in "kv")
+    out, lse = ops.flash_attention(q, k, v, causal=causal, q_pos0=q0, k_pos0=k0, return_lse=True)
+    grads = ops.flash_backward(q, k, v, out, dout, lse, causal, hd ** -0.5, q0, k0)
+    one = [torch.empty_like(t) for t in (q, k, v)]                       # without scratch S and dP are computed again for dQ
+    kv = lambda t: _desc(t, t.stride(0), t.stride(1), ng, 1, 0, 0)
+    heads = lambda t: _desc(t, t.stride(0), t.stride(1), nh, nh // ng, 1, 0)
+    args, outs = [heads(q), kv(k), kv(v), heads(out), heads(dout)], [heads(one[0]), kv(one[1]), kv(one[2])]
+    dsum = torch.empty(B, nh, Sq, device=DEV)
+    assert lib.hg_flash_bwd(*[ctypes.byref(t) for t in args], lse.data_ptr(), dsum.data_ptr(), *[ctypes.byref(t) for t in outs],
+                            Sq, Skv, B, nh, ng, hd, int(causal), q0, k0, hd ** -0.5, _lib.stream()) == 0
+    # the same 16-bit dS, multiplied and added by the tensor core in the same order
+    assert torch.equal(grads[0], one[0])
+    assert all((a.double() - b.double()).norm() <= 1e-3 * b.double().norm() for a, b in zip(grads[1:], one[1:]))
+    _lib.assert_healthy()
