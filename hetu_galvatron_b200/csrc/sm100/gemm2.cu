@@ -5,13 +5,13 @@
 // from both, so a 128 x 256 slice of the output costs 32 KB of operand traffic per k-block per SM instead of 48 KB,
 // and six stages fit where four did.
 //
-// Roles per CTA (192 threads): warp 0 TMA producer (the warp walks the loop, one elected lane issues), warp 1 TMEM allocator (+ UMMA issuer in the leader
-// CTA only: the warp walks the loop, one elected lane issues), warps 2-5 epilogue.  Barriers (same shared-memory offsets in both CTAs):
+// Roles per CTA (192 or 320 threads): warp 0 TMA producer (the warp walks the loop, one elected lane issues), warp 1 TMEM allocator (+ UMMA issuer in the leader
+// CTA only: the warp walks the loop, one elected lane issues), warps 2-5 or 2-9 epilogue.  Barriers (same shared-memory offsets in both CTAs):
 //   full[s]        leader only; the leader's producer arrives with the byte count of BOTH CTAs' loads, every load
 //                  (from either CTA) completes its bytes on the leader's barrier
 //   empty[s]       both CTAs; signalled by tcgen05.commit with a cluster mask covering the pair
 //   tmem_full[a]   both CTAs; same mechanism, once per tile
-//   tmem_empty[a]  leader only; all 256 epilogue threads of the pair arrive (the peer's through its cluster address)
+//   tmem_empty[a]  leader only; all epilogue threads of the pair arrive (the peer's through its cluster address)
 // Every wait is bounded (2 s); a CTA that gives up raises its abort flag and the status word, its partner runs into
 // its own limit, and both still meet at the final cluster barrier and free their tensor memory.
 // No operand load uses cluster multicast: each CTA loads exactly the bytes it alone needs.
@@ -24,6 +24,8 @@
 
 namespace hg {
 namespace gemm2 {
+
+constexpr int kThreads2 = 64 + 32 * EPI2_WARPS;      // at most; see threads_for
 
 // Barriers, tensor memory and the first meeting of the pair; returns the tensor-memory base address.
 __device__ __forceinline__ uint32_t pair_setup(const Smem2& s, const CUtensorMap* tmA, const CUtensorMap* tmB, int warp) {
@@ -38,7 +40,7 @@ __device__ __forceinline__ uint32_t pair_setup(const Smem2& s, const CUtensorMap
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       mbar_init(&s.tmem_full[i], 1);
-      mbar_init(&s.tmem_empty[i], 2 * EPI_WARPS * 32);
+      mbar_init(&s.tmem_empty[i], 2 * (blockDim.x - 64));
     }
     *s.abort = 0;
     mbar_fence_init();
@@ -65,7 +67,7 @@ __device__ __forceinline__ void pair_teardown(uint32_t tmem_base, int warp) {
 }
 
 template <bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(kThreads2, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmC, const Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -84,7 +86,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   } else if (warp == 1) {
     if (rank == 0) mma2<A_MN, B_MN>(p, s, tmem_base, pair, pairs, num_tiles);
   } else {
-    epilogue2(p, &tmC, s, tmem_base, rank, pair, pairs, num_tiles);
+    epilogue2(p, &tmC, s, tmem_base, rank, int(blockDim.x - 64) / (32 * EPI_WARPS), pair, pairs, num_tiles);
   }
 
   pair_teardown(tmem_base, warp);
@@ -151,7 +153,7 @@ struct ContractionRanges {
 };
 
 template <bool A_MN, bool B_MN, typename Tiles>
-__global__ void __launch_bounds__(192, 1)
+__global__ void __launch_bounds__(kThreads2, 1)
 grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const __grid_constant__ CUtensorMap tmC, const Params p, const Tiles tiles) {
   extern __shared__ uint8_t smem_raw[];
@@ -242,7 +244,9 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
   } else {
     const int wq = warp & 3, lane = int(lane_id());
     const uint32_t lane_off = uint32_t(wq * 32) << 16;
-    StoreStage st{smem_u32(s.epi_stage + wq * EPI_STAGE_FLOATS), 0};
+    const int e = warp - 2;
+    const Share share{e / EPI_WARPS, int(blockDim.x - 64) / (32 * EPI_WARPS)};
+    const uint32_t stg = smem_u32(s.epi_stage + e * EPI_STAGE_FLOATS);
     uint32_t acc = 0, acc_phase = 0;
     tiles.walk(pair, pairs, [&](const GroupedTile& w) {
       const int row0 = w.m + int(rank) * BM + wq * 32;
@@ -256,17 +260,17 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
           __syncwarp();
         }
         const uint32_t zero[32] = {};
-        for (int c = 0; c < BN && row0 < w.m_end && w.n + c < p.N; c += 32) {
+        for (int c = share.h * 32; c < BN && row0 < w.m_end && w.n + c < p.N; c += share.H * 32) {
           float4 old[8];
           load_old(q, row0, w.n + c, old);
-          store_block_rows(q, st.base, row0, w.n + c, zero, old);
+          store_block_rows(q, stg, row0, w.n + c, zero, old);
         }
         return true;
       }
       if (!mbar_wait_warp(&s.tmem_full[acc], acc_phase, p.status, kTimeoutTmemFull, s.abort)) { *s.abort = 1; return false; }
       tc_fence_after();
       if (row0 < w.m_end)   // warp-uniform; a block that reaches into the next group's rows is stored row by row
-        store_tile_part(q, &tmC, st, tmem_base + lane_off + acc * BN, row0, w.c_row + row0, w.n, row0 + 32 <= w.m_end);
+        store_tile_part(q, &tmC, stg, share, tmem_base + lane_off + acc * BN, row0, w.c_row + row0, w.n, row0 + 32 <= w.m_end);
       tc_fence_before();
       if (rank == 0) mbar_arrive(&s.tmem_empty[acc]);
       else mbar_arrive_cluster(map_to_cta(smem_u32(&s.tmem_empty[acc]), 0));
@@ -299,7 +303,7 @@ int split_mode() {
 // columns rows of C), and how many pairs share each tile of the last wave (s < 2: none do), `tail` of them.
 struct TilePlan {
   int bn, turned, s, tail;
-  long long word_bytes() const { return ((long long)tail * 8 * sizeof(unsigned long long) + 255) / 256 * 256; }
+  long long word_bytes() const { return ((long long)tail * kSplitWords * sizeof(unsigned long long) + 255) / 256 * 256; }
   long long bytes() const { return s < 2 ? 0 : word_bytes() + (long long)tail * s * (CM * bn) * sizeof(float); }
 };
 
@@ -312,9 +316,10 @@ constexpr int kBlockCost = 256;
 // 256 columns 310 us, as many of 224 278, 1332 of 192 295).  An idle last wave still costs a little there: 4096 x 4096, K = 32000,
 // 256 tiles 760 us, the last 34 shared by two 703.
 // A tile's way out of tensor memory: it counts once per launch, and in every wave where it is longer than the products.  One
-// tile of K = 512, bn = 64 to 256, us: 16 bits 6.0 to 8.1, fp32 7.7 to 11.2, turned 6.5 to 11.5; K = 300, fp32, 11008 x 4096 (all
-// stores): bn = 256 50, bn = 128 62, so that a tile has a part that is not its columns'.
-constexpr int kStore = 2400, kStore16 = 10, kStore32 = 21, kStoreTurned = 34, kTurned = 1000;
+// tile of K = 512, bn = 64 to 256, us: 16 bits 6.0 to 8.1, fp32 7.7 to 11.2, turned 6.5 to 11.5.  A part is not the columns' (fp32,
+// 11008 x 4096, K = 300, all stores, with one epilogue warp per 32 rows: bn = 256 50 us, bn = 128 62; 37888 x 3584, K = 63, 28 waves:
+// 126 us and 103 with two, 5900 cycles a wave).
+constexpr int kStore = 1400, kStore16 = 10, kStore32 = 21, kStoreTurned = 34, kTurned = 1000;
 // A shared tile, per column: the parts' way to L2 and the arrivals, and each part that is added (200 x 3584, K = 18944: 256
 // columns by five 52 us, 192 by three 44, not shared 89).
 constexpr int kSplitCost = 48, kPartCost = 20;
@@ -394,14 +399,23 @@ unsigned long long split_token() {
 
 }  // namespace
 
+// Threads of a CTA: with two epilogue warps per 32 rows where a tile's way out counts beside its products, which take `main`
+// cycles (see plan_cost), with one elsewhere: on large products, which the power limit bounds, the four more warps cost
+// 1 to 3 % (sustained, us, one and two: 4096 x 32000, K = 4096 827 -> 850 us; 22016 x 4096, K = 8192, added to C 1217 -> 1258; 28672 x 4096, fp32, K = 1024 236 ->
+// 238, K = 512 164 -> 157; added to C, K = 2048 460 -> 453).
+static int threads_for(int out_mode, long long main) {
+  const bool adds = out_mode == kOutF32Acc || out_mode == kOutBf16Acc;
+  return main < (adds ? 20000 : 8000) ? kThreads2 : 64 + 32 * EPI_WARPS;
+}
+
 // Launch attributes of a kernel of CTA pairs, and how many pairs of it the device holds at once (-2: none).
 template <typename K>
-static int pair_config(K kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int* max_pairs, bool overlaps, cudaStream_t st) {
+static int pair_config(K kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int* max_pairs, bool overlaps, cudaStream_t st, int threads = kThreads2) {
   attr->id = cudaLaunchAttributeClusterDimension;
   attr->val.clusterDim.x = 2;
   attr->val.clusterDim.y = 1;
   attr->val.clusterDim.z = 1;
-  cfg->blockDim = dim3(192, 1, 1);
+  cfg->blockDim = dim3(kThreads2, 1, 1);
   cfg->dynamicSmemBytes = SMEM2_BYTES;
   cfg->stream = st;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -422,17 +436,18 @@ static int pair_config(K kernel, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* a
     *max_pairs = n;
   }
   if (overlaps) cfg->numAttrs = 2;
+  cfg->blockDim = dim3(unsigned(threads), 1, 1);
   return 0;
 }
 
 template <bool A_MN, bool B_MN, typename Tiles>
 static int launch_grouped2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const Params& p,
-                           const Tiles& tiles, int want_pairs, cudaStream_t st) {
+                           const Tiles& tiles, int want_pairs, int threads, cudaStream_t st) {
   static int max_pairs = -1;
   auto k = grouped_gemm2_kernel<A_MN, B_MN, Tiles>;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  if (int rc = pair_config(k, &cfg, attr, &max_pairs, hg_host::launch_overlaps(), st)) return rc;
+  if (int rc = pair_config(k, &cfg, attr, &max_pairs, hg_host::launch_overlaps(), st, threads)) return rc;
   const int pairs = want_pairs < max_pairs ? want_pairs : max_pairs;
   cfg.gridDim = dim3(unsigned(2 * pairs), 1, 1);
   return hg_host::launched(cudaLaunchKernelEx(&cfg, k, ta, tb, tc, p, tiles));
@@ -446,7 +461,8 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   auto k = gemm2_bf16_kernel<A_MN, B_MN>;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  if (int rc = pair_config(k, &cfg, attr, &co_resident, hg_host::launch_overlaps(), st)) return rc;
+  const int threads = threads_for(p.out_mode, (long long)((p.K + BK - 1) / BK) * (kBlockCost + p.bn));
+  if (int rc = pair_config(k, &cfg, attr, &co_resident, hg_host::launch_overlaps(), st, threads)) return rc;
   int pairs = want_pairs < co_resident ? want_pairs : co_resident;
   p.split_s = 0;
   if (ws != nullptr && plan.s > 1 && ws_bytes >= plan.bytes()) {     // see Params::split_s
@@ -571,8 +587,9 @@ int hg_grouped_gemm2_bf16(const void* A, const void* B, void* C, const void* row
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   CUtensorMap tc;
   if ((rc = store_map(&tc, ta, p, max_rows))) return rc;
-  return b_mn ? launch_grouped2<false, true>(ta, tb, tc, p, t, 1 << 20, st)
-              : launch_grouped2<false, false>(ta, tb, tc, p, t, 1 << 20, st);
+  const int threads = threads_for(out_mode, (long long)t.num_kb * (kBlockCost + BN));
+  return b_mn ? launch_grouped2<false, true>(ta, tb, tc, p, t, 1 << 20, threads, st)
+              : launch_grouped2<false, false>(ta, tb, tc, p, t, 1 << 20, threads, st);
 }
 
 int hg_grouped_wgrad2_bf16(const void* dy, const void* x, void* out, const void* row_start, int G, int rows, int N,
@@ -591,7 +608,8 @@ int hg_grouped_wgrad2_bf16(const void* dy, const void* x, void* out, const void*
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
   CUtensorMap tc;
   if ((rc = store_map(&tc, ta, p, uint64_t(G) * N))) return rc;
-  return launch_grouped2<true, true>(ta, tb, tc, p, t, pairs, reinterpret_cast<cudaStream_t>(stream));
+  const int threads = threads_for(out_mode, ((long long)rows / G + BK - 1) / BK * (kBlockCost + BN));    // a group's, on average
+  return launch_grouped2<true, true>(ta, tb, tc, p, t, pairs, threads, reinterpret_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

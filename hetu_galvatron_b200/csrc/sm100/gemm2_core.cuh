@@ -14,9 +14,15 @@ constexpr int HALF_N = BN / 2;                // B rows staged by one CTA
 constexpr int STAGES2 = 6;
 constexpr int A2_BYTES = BM * BK * 2;         // 16 KB
 constexpr int B2_BYTES = HALF_N * BK * 2;     // 16 KB
-// Per epilogue warp: two 32-row x 128-byte blocks on their way to C, or one 32 x 32 fp32 block in rows of 36 words.
-constexpr int EPI_STAGE_FLOATS = 2 * 32 * 32;   // >= 32 rows of 36 words
-constexpr int SMEM2_BYTES = STAGES2 * (A2_BYTES + B2_BYTES) + EPI_WARPS * EPI_STAGE_FLOATS * 4 + 1024 + 256;
+// The plain and grouped kernels have one or two epilogue warps per 32 rows; two take turns at the blocks of columns.  A block's
+// way out is a chain (tensor memory, registers, shared memory, fence, copy) of about 1000 cycles of which a warp keeps little in
+// flight.  us, one / two: fp32 results 37888 x 3584, K = 63 126 / 103 (5.3 TB/s written), 22016 x 4096, K = 128 88 / 73, added to
+// what is there, K = 1024 240 / 197; 16 bits 8192 x 22016, K = 512 169 / 158.  Two stages per warp instead of one are worth
+// 0 to 10 % where stores bound, and cost 1 to 1.5 % on large products.
+constexpr int EPI2_WARPS = 2 * EPI_WARPS;
+// Per epilogue warp: a block of 32 rows x 128 bytes on its way to C, as TMA's 128-byte swizzle has it.
+constexpr int EPI_STAGE_FLOATS = 32 * 32;
+constexpr int SMEM2_BYTES = STAGES2 * (A2_BYTES + B2_BYTES) + EPI2_WARPS * EPI_STAGE_FLOATS * 4 + 1024 + 256;
 static_assert(SMEM2_BYTES <= 232448, "one CTA per SM");
 constexpr uint16_t kPairMask = 0x3;
 
@@ -38,7 +44,7 @@ __device__ __forceinline__ Smem2 carve2(uint8_t* raw) {
   s.a = base;
   s.b = base + STAGES2 * A2_BYTES;
   s.epi_stage = reinterpret_cast<float*>(base + STAGES2 * (A2_BYTES + B2_BYTES));   // 1024-byte aligned
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s.epi_stage + EPI_WARPS * EPI_STAGE_FLOATS);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s.epi_stage + EPI2_WARPS * EPI_STAGE_FLOATS);
   s.full = bars;
   s.empty = bars + STAGES2;
   s.tmem_full = bars + 2 * STAGES2;
@@ -113,6 +119,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
 struct Unit {
   int tile, kb0, kb1, slice;
 };
+constexpr int kSplitWords = 2 * EPI2_WARPS;              // of a tile: one per epilogue warp of the pair
 constexpr unsigned long long kSplitCountMask = 255;      // low bits of a word: slices that have arrived; a token has none of them
 // Word `q` (four columns) of 32-column block `c` of this thread's row in a partial tile: neighbouring lanes, neighbouring words.
 __device__ __forceinline__ int split_word(int bn, int warp8, int c, int q) {
@@ -277,10 +284,9 @@ __device__ __forceinline__ void mma2(const Params& p, const Smem2& s, uint32_t t
 // wrong shape for global memory, so each warp turns its blocks through shared memory.
 //
 // Plain 16-bit and fp32 stores: 32 rows x 128 bytes are written to the warp's stage in the layout of the 128-byte
-// swizzle, eight conflict-free 16-byte stores per thread, and leave as one TMA store that clips at the matrix' edges;
-// two blocks alternate, so that one is filled while the other is read.
+// swizzle, eight conflict-free 16-byte stores per thread, and leave as one TMA store that clips at the matrix' edges.
 // Accumulating modes, a C that no tensor map covers and the ragged end of an expert's rows: a 32 x 32 fp32 block at a time
-// through 36-word rows (conflict-free 16-byte accesses both ways), eight lanes on 32 consecutive columns of a row, four
+// through the same stage (conflict-free 16-byte accesses both ways), eight lanes on 32 consecutive columns of a row, four
 // elements each, all loads of a block before its first store.
 //
 // What an epilogue costs is instructions, not bytes, and every decision that can be taken once per tile is taken there:
@@ -296,16 +302,16 @@ __device__ __forceinline__ float4 lds128(uint32_t addr) {
   return v;
 }
 
-// This warp's two store blocks; `next` alternates.  Bulk groups belong to a thread: lane 0 issues and waits.
-struct StoreStage {
-  uint32_t base;
-  int next;
+// w: the 128 bytes of this thread's row, to columns col0.. of rows y0 .. y0 + 31 of the map.
+// H warps share 32 rows: the one with number h takes the blocks h, h + H, ...
+struct Share {
+  int h, H;
 };
 
-// w: the 128 bytes of this thread's row, to columns col0.. of rows y0 .. y0 + 31 of the map.
-__device__ __forceinline__ void tma_store_rows(const CUtensorMap* tm, StoreStage& st, const uint32_t (&w)[32], int col0, int y0) {
-  const uint32_t lane = lane_id(), buf = st.base + st.next * 4096;
-  if (lane == 0) tma_store_wait_read<1>();          // the store before the last one has left this block
+// Bulk groups belong to a thread: lane 0 issues and waits.
+__device__ __forceinline__ void tma_store_rows(const CUtensorMap* tm, uint32_t buf, const uint32_t (&w)[32], int col0, int y0) {
+  const uint32_t lane = lane_id();
+  if (lane == 0) tma_store_wait_read<0>();          // the last store has left the stage
   __syncwarp();
 #pragma unroll
   for (int j = 0; j < 8; ++j)
@@ -319,60 +325,41 @@ __device__ __forceinline__ void tma_store_rows(const CUtensorMap* tm, StoreStage
                  : "memory");
     tma_store_commit();
   }
-  st.next ^= 1;
 }
 
-// The slices of a shared tile, as this warp's threads hold its rows (n = 0: a tile of one pair): `mine` is in registers, the
-// others lie in memory.  Added in one order, the last slice first, whoever adds them.
+// The slices of a shared tile (n = 0: a tile of one pair), all of them in memory by the time that they are added: the last slice
+// first, then the others in order, whoever adds them.
 struct Parts {
   const float* base;
-  int n, mine, warp8, bn;
+  int n, warp8, bn;
   __device__ __forceinline__ void add(int c, uint32_t (&r)[32]) const {
     if (n == 0) return;
-    auto part = [&](int k, int q) {
-      return __ldcg(reinterpret_cast<const float4*>(base + size_t(k) * (CM * bn) + split_word(bn, warp8, c, q)));
-    };
-    if (mine == n - 1) {
-      for (int k = 0; k + 1 < n; ++k) {
-        float4 v[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = part(k, q);
+    for (int q = 0; q < 8; ++q) {
+      const float4 v = part(n - 1, c, q);
+      r[4 * q] = __float_as_uint(v.x);
+      r[4 * q + 1] = __float_as_uint(v.y);
+      r[4 * q + 2] = __float_as_uint(v.z);
+      r[4 * q + 3] = __float_as_uint(v.w);
+    }
+#pragma unroll 1
+    for (int k = 0; k + 1 < n; ++k) {
+      float4 v[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) plus(r, q, v[q]);
-      }
-    } else {
-      uint32_t own[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) own[i] = r[i];
+      for (int q = 0; q < 8; ++q) v[q] = part(k, c, q);
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const float4 v = part(n - 1, q);
-        r[4 * q] = __float_as_uint(v.x);
-        r[4 * q + 1] = __float_as_uint(v.y);
-        r[4 * q + 2] = __float_as_uint(v.z);
-        r[4 * q + 3] = __float_as_uint(v.w);
-      }
-      for (int k = 0; k + 1 < n; ++k) {
-        if (k == mine) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(own[i]));
-        } else {
-          float4 v[8];
-#pragma unroll
-          for (int q = 0; q < 8; ++q) v[q] = part(k, q);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) plus(r, q, v[q]);
-        }
+        r[4 * q] = __float_as_uint(__uint_as_float(r[4 * q]) + v[q].x);
+        r[4 * q + 1] = __float_as_uint(__uint_as_float(r[4 * q + 1]) + v[q].y);
+        r[4 * q + 2] = __float_as_uint(__uint_as_float(r[4 * q + 2]) + v[q].z);
+        r[4 * q + 3] = __float_as_uint(__uint_as_float(r[4 * q + 3]) + v[q].w);
       }
     }
   }
 
  private:
-  static __device__ __forceinline__ void plus(uint32_t (&r)[32], int q, const float4& v) {
-    r[4 * q] = __float_as_uint(__uint_as_float(r[4 * q]) + v.x);
-    r[4 * q + 1] = __float_as_uint(__uint_as_float(r[4 * q + 1]) + v.y);
-    r[4 * q + 2] = __float_as_uint(__uint_as_float(r[4 * q + 2]) + v.z);
-    r[4 * q + 3] = __float_as_uint(__uint_as_float(r[4 * q + 3]) + v.w);
+  __device__ __forceinline__ float4 part(int k, int c, int q) const {
+    return __ldcg(reinterpret_cast<const float4*>(base + size_t(k) * (CM * bn) + split_word(bn, warp8, c, q)));
   }
 };
 
@@ -418,7 +405,7 @@ __device__ __forceinline__ void add_bias_row(const Params& p, int col0, uint32_t
 
 // A 32 x 64 block from registers (thread = row) through the tensor map.
 template <bool BIAS>
-__device__ __forceinline__ void store_block64_tma(const Params& p, const CUtensorMap* tm, StoreStage& st, int y0, int col0,
+__device__ __forceinline__ void store_block64_tma(const Params& p, const CUtensorMap* tm, uint32_t stg, int y0, int col0,
                                                   uint32_t (&r0)[32], uint32_t (&r1)[32]) {
   if (BIAS) {
     add_bias_row<32>(p, col0, r0);
@@ -430,15 +417,16 @@ __device__ __forceinline__ void store_block64_tma(const Params& p, const CUtenso
     w[i] = pack_bf16(__uint_as_float(r0[2 * i]), __uint_as_float(r0[2 * i + 1]));
     w[16 + i] = pack_bf16(__uint_as_float(r1[2 * i]), __uint_as_float(r1[2 * i + 1]));
   }
-  tma_store_rows(tm, st, w, col0, y0);
+  tma_store_rows(tm, stg, w, col0, y0);
 }
 
 // Columns n0.. of the tile as TMA stores of 128-byte rows: 64 columns of 16 bits, or 32 of fp32.
 template <bool BIAS, bool F32>
-__device__ __forceinline__ void store_tile_tma(const Params& p, const CUtensorMap* tmC, StoreStage& st, uint32_t src, int row0,
+__device__ __forceinline__ void store_tile_tma(const Params& p, const CUtensorMap* tmC, uint32_t stg, Share w, uint32_t src, int row0,
                                                int y0, int n0, const Parts& parts) {
+  constexpr int kBlock = F32 ? 32 : 64;
 #pragma unroll 1
-  for (int c = 0; c < p.bn && n0 + c < p.N; c += F32 ? 32 : 64) {
+  for (int c = w.h * kBlock; c < p.bn && n0 + c < p.N; c += w.H * kBlock) {
     uint32_t r0[32], r1[32];
     tmem_ld32(src + c, r0);
     if (!F32) tmem_ld32(src + c + 32, r1);
@@ -448,9 +436,9 @@ __device__ __forceinline__ void store_tile_tma(const Params& p, const CUtensorMa
     if (!F32) parts.add(c / 32 + 1, r1);
     if constexpr (F32) {
       if (BIAS) add_bias_row<32>(p, n0 + c, r0);
-      tma_store_rows(tmC, st, r0, n0 + c, y0);
+      tma_store_rows(tmC, stg, r0, n0 + c, y0);
     } else {
-      store_block64_tma<BIAS>(p, tmC, st, y0, n0 + c, r0, r1);
+      store_block64_tma<BIAS>(p, tmC, stg, y0, n0 + c, r0, r1);
     }
   }
 }
@@ -506,12 +494,12 @@ __device__ __forceinline__ void store_block_rows(const Params& p, uint32_t stg, 
   const int lane = int(lane_id());
 #pragma unroll
   for (int j = 0; j < 8; ++j)
-    sts128(stg + lane * 144 + j * 16, src[4 * j], src[4 * j + 1], src[4 * j + 2], src[4 * j + 3]);
+    sts128(stg + sw128_offset(lane, j), src[4 * j], src[4 * j + 1], src[4 * j + 2], src[4 * j + 3]);
   __syncwarp();
   const int q = (lane & 7) * 4, col = col0 + q;
   float4 v[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = lds128(stg + (i * 4 + (lane >> 3)) * 144 + q * 4);
+  for (int i = 0; i < 8; ++i) v[i] = lds128(stg + sw128_offset(i * 4 + (lane >> 3), lane & 7));
   __syncwarp();
   if (!HG_BOUNDS_OK(row0 >= 0 && row0 < p.M && col0 >= 0 && col0 < p.N, p.status)) return;
   if (col >= p.N) return;
@@ -558,12 +546,12 @@ __device__ __forceinline__ void store_block_whole(const Params& p, uint32_t stg,
   const int lane = int(lane_id());
 #pragma unroll
   for (int j = 0; j < 8; ++j)
-    sts128(stg + lane * 144 + j * 16, src[4 * j], src[4 * j + 1], src[4 * j + 2], src[4 * j + 3]);
+    sts128(stg + sw128_offset(lane, j), src[4 * j], src[4 * j + 1], src[4 * j + 2], src[4 * j + 3]);
   __syncwarp();
   const int q = (lane & 7) * 4;
   float4 v[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = lds128(stg + (i * 4 + (lane >> 3)) * 144 + q * 4);
+  for (int i = 0; i < 8; ++i) v[i] = lds128(stg + sw128_offset(i * 4 + (lane >> 3), lane & 7));
   __syncwarp();
   if (!HG_BOUNDS_OK(row0 >= 0 && row0 + 32 <= p.M && col0 >= 0 && col0 + 32 <= p.N, p.status)) return;
   float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -601,66 +589,59 @@ __device__ __forceinline__ void load_old_whole(const Params& p, int row0, int co
   }
 }
 
-// The whole blocks of a tile part; returns the first column that is left.  With an accumulating mode the next block's old
-// values are in flight while this one is turned.
+// This warp's whole blocks of a tile part.
 template <int MODE>
-__device__ __forceinline__ int store_tile_whole(const Params& p, uint32_t stg, uint32_t src, int row0, int n0, const Parts& parts) {
+__device__ __forceinline__ void store_tile_whole(const Params& p, uint32_t stg, Share w, uint32_t src, int row0, int n0, const Parts& parts) {
   const int cols = min(p.bn, (p.N - n0) & ~31);
-  float4 old[8];
-  if (cols > 0) load_old_whole<MODE>(p, row0, n0, old);
 #pragma unroll 1
-  for (int c = 0; c < cols; c += 32) {
+  for (int c = w.h * 32; c < cols; c += w.H * 32) {
+    float4 old[8];
+    load_old_whole<MODE>(p, row0, n0 + c, old);
     uint32_t r0[32];
     tmem_ld32(src + c, r0);
     tmem_ld_wait();
-    float4 next[8];
-    if (c + 32 < cols) load_old_whole<MODE>(p, row0, n0 + c + 32, next);
     parts.add(c / 32, r0);
     store_block_whole<MODE>(p, stg, row0, n0 + c, r0, old);
-    if (MODE == kOutF32Acc || MODE == kOutBf16Acc) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) old[i] = next[i];
-    }
   }
-  return max(cols, 0);
 }
 
-// The 32 x 256 part of a tile that this warp's lanes hold in tensor memory at `src`: rows row0.. of C (p.M: the first row
+// This warp's blocks of the 32 x bn part of a tile that tensor memory holds at `src`: rows row0.. of C (p.M: the first row
 // that is not this tile's), rows y0.. of the tensor map.
-__device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorMap* tmC, StoreStage& st, uint32_t src, int row0,
-                                                int y0, int n0, bool whole_rows, const Parts& parts = Parts{nullptr, 0, 0, 0, 0}) {
+__device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorMap* tmC, uint32_t stg, Share w, uint32_t src, int row0,
+                                                int y0, int n0, bool whole_rows, const Parts& parts = Parts{nullptr, 0, 0, 0}) {
   if (p.c_tma && whole_rows) {
     if (p.out_mode == kOutF32) {
-      if (p.bias != nullptr) store_tile_tma<true, true>(p, tmC, st, src, row0, y0, n0, parts);
-      else store_tile_tma<false, true>(p, tmC, st, src, row0, y0, n0, parts);
+      if (p.bias != nullptr) store_tile_tma<true, true>(p, tmC, stg, w, src, row0, y0, n0, parts);
+      else store_tile_tma<false, true>(p, tmC, stg, w, src, row0, y0, n0, parts);
     } else {
-      if (p.bias != nullptr) store_tile_tma<true, false>(p, tmC, st, src, row0, y0, n0, parts);
-      else store_tile_tma<false, false>(p, tmC, st, src, row0, y0, n0, parts);
+      if (p.bias != nullptr) store_tile_tma<true, false>(p, tmC, stg, w, src, row0, y0, n0, parts);
+      else store_tile_tma<false, false>(p, tmC, stg, w, src, row0, y0, n0, parts);
     }
     return;
   }
-  if (p.c_tma) {                                    // the stage is about to be written past the stores that read it
+  if (p.c_tma) {                                    // the stage is about to be written past the store that reads it
     if (lane_id() == 0) tma_store_wait_read<0>();
     __syncwarp();
   }
   int c0 = 0;
   if (row0 + 32 <= p.M && four_aligned(p)) {
     switch (p.out_mode) {
-      case kOutF32: c0 = store_tile_whole<kOutF32>(p, st.base, src, row0, n0, parts); break;
-      case kOutF32Acc: c0 = store_tile_whole<kOutF32Acc>(p, st.base, src, row0, n0, parts); break;
-      case kOutBf16Acc: c0 = store_tile_whole<kOutBf16Acc>(p, st.base, src, row0, n0, parts); break;
-      default: c0 = store_tile_whole<kOutBf16>(p, st.base, src, row0, n0, parts); break;
+      case kOutF32: store_tile_whole<kOutF32>(p, stg, w, src, row0, n0, parts); break;
+      case kOutF32Acc: store_tile_whole<kOutF32Acc>(p, stg, w, src, row0, n0, parts); break;
+      case kOutBf16Acc: store_tile_whole<kOutBf16Acc>(p, stg, w, src, row0, n0, parts); break;
+      default: store_tile_whole<kOutBf16>(p, stg, w, src, row0, n0, parts); break;
     }
+    c0 = max(min(p.bn, (p.N - n0) & ~31), 0);       // the columns that are left: one block that the edge of C cuts
   }
 #pragma unroll 1
-  for (int c = c0; c < p.bn && n0 + c < p.N; c += 32) {
+  for (int c = c0 + (w.H - 1 - (c0 / 32 + w.H - 1 - w.h) % w.H) * 32; c < p.bn && n0 + c < p.N; c += w.H * 32) {
     float4 old[8];
     load_old(p, row0, n0 + c, old);
     uint32_t r0[32];
     tmem_ld32(src + c, r0);
     tmem_ld_wait();
     parts.add(c / 32, r0);
-    store_block_rows(p, st.base, row0, n0 + c, r0, old);
+    store_block_rows(p, stg, row0, n0 + c, r0, old);
   }
 }
 
@@ -668,12 +649,12 @@ __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorM
 // 32 consecutive elements and needs no shared memory.  16 bits: neighbouring lanes trade a value, and each stores two columns
 // of one row, 16 lanes a row and 64 bytes each.
 template <int MODE>
-__device__ __forceinline__ void store_tile_turned(const Params& p, uint32_t src, int row0, int n0, const Parts& parts) {
+__device__ __forceinline__ void store_tile_turned(const Params& p, Share w, uint32_t src, int row0, int n0, const Parts& parts) {
   const int lane = int(lane_id()), col = row0 + lane;
   const bool mine = col < p.M;
   const float b = p.bias != nullptr && mine ? hg_lp2f(p.bias[col]) : 0.f;
 #pragma unroll 1
-  for (int c = 0; c < p.bn && n0 + c < p.N; c += 32) {
+  for (int c = w.h * 32; c < p.bn && n0 + c < p.N; c += w.H * 32) {
     uint32_t r[32];
     tmem_ld32(src + c, r);
     tmem_ld_wait();
@@ -700,20 +681,23 @@ __device__ __forceinline__ void store_tile_turned(const Params& p, uint32_t src,
     }
   }
 }
-__device__ __forceinline__ void store_tile_turned(const Params& p, uint32_t src, int row0, int n0, const Parts& parts) {
+__device__ __forceinline__ void store_tile_turned(const Params& p, Share w, uint32_t src, int row0, int n0, const Parts& parts) {
   switch (p.out_mode) {
-    case kOutF32: store_tile_turned<kOutF32>(p, src, row0, n0, parts); break;
-    case kOutF32Acc: store_tile_turned<kOutF32Acc>(p, src, row0, n0, parts); break;
-    default: store_tile_turned<kOutBf16>(p, src, row0, n0, parts); break;
+    case kOutF32: store_tile_turned<kOutF32>(p, w, src, row0, n0, parts); break;
+    case kOutF32Acc: store_tile_turned<kOutF32Acc>(p, w, src, row0, n0, parts); break;
+    default: store_tile_turned<kOutBf16>(p, w, src, row0, n0, parts); break;
   }
 }
 
+// H: epilogue warps per 32 rows, warps 2 .. 1 + 4 H of the block.
 __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tmC, const Smem2& s, uint32_t tmem_base,
-                                          uint32_t rank, int first, int step, int num_tiles) {
+                                          uint32_t rank, int H, int first, int step, int num_tiles) {
   const int wq = (threadIdx.x >> 5) & 3;
   const int lane = int(lane_id());
   const uint32_t lane_off = uint32_t(wq * 32) << 16;
-  StoreStage st{smem_u32(s.epi_stage + wq * EPI_STAGE_FLOATS), 0};
+  const int e = (threadIdx.x >> 5) - 2;
+  const Share share{e / EPI_WARPS, H};
+  const uint32_t stg = smem_u32(s.epi_stage + e * EPI_STAGE_FLOATS);
   uint32_t acc = 0, acc_phase = 0;
   const int num_kb = (p.K + BK - 1) / BK;
   const int n_units = unit_count(p, first, step, num_tiles);
@@ -728,7 +712,7 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
     const bool shared_tile = p.split_s > 1 && tile >= p.split_tail_begin;
     const int tail_idx = tile - p.split_tail_begin, warp8 = int(rank) * EPI_WARPS + wq;
     float* ws_tile = shared_tile ? p.split_ws + size_t(tail_idx) * p.split_s * (CM * p.bn) : nullptr;
-    const Parts parts{ws_tile, shared_tile ? p.split_s : 0, w.slice, warp8, p.bn};
+    const Parts parts{ws_tile, shared_tile ? p.split_s : 0, warp8, p.bn};
     if (!mbar_wait_warp(&s.tmem_full[acc], acc_phase, p.status, kTimeoutTmemFull, s.abort)) {
       *s.abort = 1;
       break;
@@ -741,7 +725,7 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
         // Nobody waits for another pair, whatever the order in which the device runs them.
         float* dst = ws_tile + size_t(w.slice) * (CM * p.bn);
 #pragma unroll 1
-        for (int c = 0; c < p.bn / 32; ++c) {
+        for (int c = share.h; c < p.bn / 32; c += H) {
           uint32_t r0[32];
           tmem_ld32(src + c * 32, r0);
           tmem_ld_wait();
@@ -753,15 +737,15 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
         __threadfence();
         __syncwarp();
         int last = 0;
-        if (lane == 0) last = split_arrive(p.split_words + size_t(tail_idx) * 8 + warp8, p.split_token, p.split_s);
+        if (lane == 0) last = split_arrive(p.split_words + size_t(tail_idx) * kSplitWords + share.h * 8 + warp8, p.split_token, p.split_s);
         writes = __shfl_sync(0xffffffffu, last, 0) != 0;
         __threadfence();                  // the other slices' parts are read after their arrivals
       }
-      if (writes && p.turned) store_tile_turned(p, src, row0, n0, parts);
-      else if (writes) store_tile_part(p, tmC, st, src, row0, row0, n0, true, parts);
+      if (writes && p.turned) store_tile_turned(p, share, src, row0, n0, parts);
+      else if (writes) store_tile_part(p, tmC, stg, share, src, row0, row0, n0, true, parts);
     }
     tc_fence_before();
-    // the accumulator buffer is free again once all 256 epilogue threads of the pair have read it
+    // the accumulator buffer is free again once all epilogue threads of the pair have read it
     if (rank == 0) mbar_arrive(&s.tmem_empty[acc]);
     else mbar_arrive_cluster(map_to_cta(smem_u32(&s.tmem_empty[acc]), 0));
     if (++acc == 2) { acc = 0; acc_phase ^= 1; }

@@ -68,8 +68,8 @@ struct Params {
   // Optional split of the last, partly filled wave (CTA-pair kernel only): tiles from `split_tail_begin` on are each
   // computed by `split_s` pairs, every pair taking a contiguous share of the k-blocks.  Each leaves its fp32 partial tile in
   // `split_ws` (256 x bn floats per (tail tile, slice), in the order in which the epilogue's threads hold it), and each of its
-  // eight epilogue warps then counts itself in at its word of `split_words` ([tail tile][8]).  The last warp to arrive at a
-  // word adds the parts of those rows in slice order, so that the result does not depend on timing, and writes them.
+  // epilogue warps then counts itself in at its word of `split_words` ([tail tile][kSplitWords]).  The last warp to arrive at a
+  // word adds the parts of those blocks in slice order, so that the result does not depend on timing, and writes them.
   // split_s < 2: off.
   int split_s;
   int split_tail_begin;
