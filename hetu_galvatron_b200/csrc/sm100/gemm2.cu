@@ -101,6 +101,7 @@ struct GroupedTile {
   int num_kb;
   int c_row;              // row of the tensor map of C at which this group's rows start
   long long c_off;        // elements of C before this group
+  int bn;                 // columns of the tile
 };
 
 // C[r0:r1] = A[r0:r1] op(B_g) for the row segments [r0, r1) = row_start[g..g+1].  Inside a segment up to eight row tiles
@@ -112,6 +113,7 @@ struct RowSegments {
   int G, tiles_n, num_kb, b_group_rows, max_rows;
   int* status;
   static constexpr int kGroupM = 8;
+  static constexpr bool kTurned = false;
   template <typename F>
   __device__ __forceinline__ void walk(int pair, int pairs, F&& fn) const {
     int counter = 0;
@@ -123,7 +125,34 @@ struct RowSegments {
       for (int t = (pair - counter % pairs + pairs) % pairs; t < cnt; t += pairs) {
         const int first = t / (kGroupM * tiles_n) * kGroupM, gsize = min(kGroupM, tm_cnt - first);
         const int r = t - first * tiles_n;
-        GroupedTile w{r0 + (first + r % gsize) * CM, r1, r / gsize * BN, 0, g * b_group_rows, num_kb, 0, 0};
+        GroupedTile w{r0 + (first + r % gsize) * CM, r1, r / gsize * BN, 0, g * b_group_rows, num_kb, 0, 0, BN};
+        if (!fn(w)) return;
+      }
+      counter += cnt;
+    }
+  }
+};
+
+// The same products with A and B in each other's place: a tile is 256 columns of C (rows of the weight) by up to 256 rows of a
+// segment, which is cut into as few equal tiles as it takes, of a multiple of 64 rows each.  Tiles of 256 rows of C by 256
+// columns were one in eight padding at segments of about 1024 ragged rows.  The tiles of one piece of the weight are neighbours: it
+// is read from HBM once.
+struct TurnedSegments {
+  const int* row_start;
+  int G, tiles_m, num_kb, w_group_rows, max_rows;
+  int* status;
+  static constexpr bool kTurned = true;
+  template <typename F>
+  __device__ __forceinline__ void walk(int pair, int pairs, F&& fn) const {
+    int counter = 0;
+    for (int g = 0; g < G; ++g) {
+      const int r0 = row_start[g], r1 = row_start[g + 1], rows = r1 - r0;
+      if (!HG_BOUNDS_OK(r0 >= 0 && r1 >= r0 && r1 <= max_rows, status)) return;
+      if (rows <= 0) continue;
+      const int pieces = (rows + BN - 1) / BN, bn = ((rows + pieces - 1) / pieces + 63) / 64 * 64;
+      const int tn = (rows + bn - 1) / bn, cnt = tn * tiles_m;
+      for (int t = (pair - counter % pairs + pairs) % pairs; t < cnt; t += pairs) {
+        GroupedTile w{t / tn * CM, r1, r0 + t % tn * bn, 0, g * w_group_rows, num_kb, 0, 0, bn};
         if (!fn(w)) return;
       }
       counter += cnt;
@@ -137,6 +166,7 @@ struct ContractionRanges {
   int G, tiles_m, tiles_n, M;
   long long c_group_stride;
   static constexpr int kGroupM = 4;
+  static constexpr bool kTurned = false;
   template <typename F>
   __device__ __forceinline__ void walk(int pair, int pairs, F&& fn) const {
     const int per = tiles_m * tiles_n;
@@ -146,7 +176,7 @@ struct ContractionRanges {
       const int r = u - first * tiles_n;
       const int k0 = k_start[g];
       GroupedTile w{(first + r % gsize) * CM, M, r / gsize * BN, k0, k0, (k_start[g + 1] - k0 + BK - 1) / BK,
-                    g * M, g * c_group_stride};
+                    g * M, g * c_group_stride, BN};
       if (!fn(w)) return;
     }
   }
@@ -170,7 +200,7 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     bool ok = true;
     const bool issuer = elect_one() != 0;
     tiles.walk(pair, pairs, [&](const GroupedTile& w) {
-      const int m = w.m + int(rank) * BM, n = w.n + int(rank) * HALF_N;
+      const int half = w.bn / 2, m = w.m + int(rank) * BM, n = w.n + int(rank) * half;
       for (int kb = 0; kb < w.num_kb; ++kb) {
         if (!mbar_wait_warp(&s.empty[stage], phase ^ 1, p.status, kTimeoutSmemEmpty, s.abort)) { ok = false; return false; }
         const uint32_t bar = map_to_cta(smem_u32(&s.full[stage]), 0);
@@ -178,16 +208,21 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         uint8_t* sb = s.b + stage * B2_BYTES;
         const int k0 = kb * BK;
         if (issuer) {
-          if (rank == 0) mbar_expect_tx(&s.full[stage], 2 * (A2_BYTES + B2_BYTES));
+          if (rank == 0) mbar_expect_tx(&s.full[stage], 2 * (A2_BYTES + half * BK * 2));
+          const int a_off = Tiles::kTurned ? w.b_off : w.a_k;      // the weight is the stacked operand
           if (A_MN) {
 #pragma unroll
-            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * SLAB_BYTES, &tmA, bar, m + j * 64, w.a_k + k0);
+            for (int j = 0; j < BM / 64; ++j) tma_load_2d_pair(sa + j * SLAB_BYTES, &tmA, bar, m + j * 64, a_off + k0);
           } else {
-            tma_load_2d_pair(sa, &tmA, bar, k0, m);
+            tma_load_2d_pair(sa, &tmA, bar, k0, Tiles::kTurned ? a_off + m : m);
           }
           if (B_MN) {
 #pragma unroll
             for (int j = 0; j < HALF_N / 64; ++j) tma_load_2d_pair(sb + j * SLAB_BYTES, &tmB, bar, n + j * 64, w.b_off + k0);
+          } else if (Tiles::kTurned) {
+#pragma unroll
+            for (int j = 0; j < HALF_N / 32; ++j)
+              if (j * 32 < half) tma_load_2d_pair(sb + j * (32 * BK * 2), &tmB, bar, k0, n + j * 32);
           } else {
             tma_load_2d_pair(sb, &tmB, bar, k0, w.b_off + n);
           }
@@ -208,7 +243,6 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     }
   } else if (warp == 1) {
     if (rank == 0) {
-      constexpr uint32_t idesc = make_idesc_lp(CM, BN, A_MN, B_MN);
       constexpr uint32_t a_lbo = A_MN ? SLAB_BYTES : 16, a_kadv = A_MN ? 2048 : 32;
       constexpr uint32_t b_lbo = B_MN ? SLAB_BYTES : 16, b_kadv = B_MN ? 2048 : 32;
       uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
@@ -218,7 +252,7 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         if (w.num_kb <= 0) return true;   // nothing to contract: the epilogue writes the result
         if (!mbar_wait_warp(&s.tmem_empty[acc], acc_phase ^ 1, p.status, kTimeoutTmemEmpty, s.abort)) { ok = false; return false; }
         tc_fence_after();
-        const uint32_t d = tmem_base + acc * BN;
+        const uint32_t d = tmem_base + acc * BN, idesc = make_idesc_lp(CM, w.bn, A_MN, B_MN);
         for (int kb = 0; kb < w.num_kb; ++kb) {
           if (!mbar_wait_warp(&s.full[stage], phase, p.status, kTimeoutSmemFull, s.abort)) { ok = false; return false; }
           tc_fence_after();
@@ -251,6 +285,18 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
     tiles.walk(pair, pairs, [&](const GroupedTile& w) {
       const int row0 = w.m + int(rank) * BM + wq * 32;
       Params q = p;
+      if (Tiles::kTurned) {
+        q.bn = w.bn;
+        q.N = w.m_end;
+        if (!mbar_wait_warp(&s.tmem_full[acc], acc_phase, p.status, kTimeoutTmemFull, s.abort)) { *s.abort = 1; return false; }
+        tc_fence_after();
+        if (row0 < q.M) store_tile_turned<kOutBf16>(q, share, tmem_base + lane_off + acc * BN, row0, w.n, Parts{nullptr, 0, 0, 0});
+        tc_fence_before();
+        if (rank == 0) mbar_arrive(&s.tmem_empty[acc]);
+        else mbar_arrive_cluster(map_to_cta(smem_u32(&s.tmem_empty[acc]), 0));
+        if (++acc == 2) { acc = 0; acc_phase ^= 1; }
+        return true;
+      }
       q.M = w.m_end;
       q.C = p.out_mode == kOutF32 || p.out_mode == kOutF32Acc ? static_cast<void*>(reinterpret_cast<float*>(p.C) + w.c_off)
                                                               : static_cast<void*>(reinterpret_cast<hg_lp_t*>(p.C) + w.c_off);
@@ -574,20 +620,30 @@ int hg_grouped_gemm2_bf16(const void* A, const void* B, void* C, const void* row
                           int K, int lda, int ldb, int ldc, int b_mn, int out_mode, void* stream) {
   if (G <= 0 || max_rows <= 0) return 0;
   if ((lda & 7) || (ldb & 7)) return -1;
-  CUtensorMap ta, tb;
-  int rc = hg_host::make_tmap_2d_bf16(&ta, A, max_rows, K, lda, BM, 64);
-  if (rc) return rc;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  CUtensorMap ta, tb, tc;
+  int rc;
+  Params p{};
+  p.K = K; p.ldc = ldc; p.C = C; p.out_mode = out_mode; p.bn = BN; p.status = hg_host::status_ptr();
+  const int* starts = reinterpret_cast<const int*>(row_start);
+  const int num_kb = (K + BK - 1) / BK, threads = threads_for(out_mode, (long long)num_kb * (kBlockCost + BN));
+  if (turns(C, N, ldc, out_mode)) {
+    p.M = N; p.N = max_rows;
+    if (b_mn) rc = hg_host::make_tmap_2d_bf16(&ta, B, uint64_t(G) * K, N, ldb, 64, 64);
+    else      rc = hg_host::make_tmap_2d_bf16(&ta, B, uint64_t(G) * N, K, ldb, BM, 64);
+    if (!rc) rc = hg_host::make_tmap_2d_bf16(&tb, A, max_rows, K, lda, 32, 64);
+    if (rc) return rc;
+    const TurnedSegments t{starts, G, (N + CM - 1) / CM, num_kb, b_mn ? K : N, max_rows, p.status};
+    return b_mn ? launch_grouped2<true, false>(ta, tb, ta, p, t, 1 << 20, threads, st)
+                : launch_grouped2<false, false>(ta, tb, ta, p, t, 1 << 20, threads, st);
+  }
+  if ((rc = hg_host::make_tmap_2d_bf16(&ta, A, max_rows, K, lda, BM, 64))) return rc;
   if (b_mn) rc = hg_host::make_tmap_2d_bf16(&tb, B, uint64_t(G) * K, N, ldb, 64, 64);
   else      rc = hg_host::make_tmap_2d_bf16(&tb, B, uint64_t(G) * N, K, ldb, HALF_N, 64);
   if (rc) return rc;
-  Params p{};
-  p.M = max_rows; p.N = N; p.K = K; p.ldc = ldc; p.C = C; p.out_mode = out_mode; p.bn = BN; p.status = hg_host::status_ptr();
-  RowSegments t{reinterpret_cast<const int*>(row_start), G, (N + BN - 1) / BN, (K + BK - 1) / BK, b_mn ? K : N, max_rows,
-                p.status};
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  CUtensorMap tc;
+  p.M = max_rows; p.N = N;
+  RowSegments t{starts, G, (N + BN - 1) / BN, num_kb, b_mn ? K : N, max_rows, p.status};
   if ((rc = store_map(&tc, ta, p, max_rows))) return rc;
-  const int threads = threads_for(out_mode, (long long)t.num_kb * (kBlockCost + BN));
   return b_mn ? launch_grouped2<false, true>(ta, tb, tc, p, t, 1 << 20, threads, st)
               : launch_grouped2<false, false>(ta, tb, tc, p, t, 1 << 20, threads, st);
 }

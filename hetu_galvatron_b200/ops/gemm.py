@@ -66,13 +66,22 @@ def _use_pair(M: int, N: int, pair) -> bool:
 
 
 def _use_grouped_pair(rows: int, N: int, K: int, G: int) -> bool:
-    """Whether grouped products take the CTA-pair tile.  Its 256 rows are mostly padding for groups of one 128-row segment,
-    and the store of a 256 x 256 tile is hidden only under a long contraction, so it pays for groups of about 512 rows
+    """Whether grouped products that cannot be turned (below) take the CTA-pair tile.  Its 256 rows are mostly padding for groups of
+    one 128-row segment, and the store of a 256 x 256 tile is hidden only under a long contraction, so it pays for groups of about 512 rows
     and K from 2560 on.  Ragged groups, us, pair against one CTA: 8 x (128 rows, 28672 columns, K = 4096) 347 / 312, 512 rows
     822 / 796, 1024 rows 1351 / 1554; 64 x (512, 2048, 1408) 220 / 177, 1024 rows 384 / 312; 64 x (1024, 2816, 2048) 615 / 605;
     8 x (512, 4096, 2560) 87 / 89, 32 x (512, 4096, 3072) 323 / 333, 1024 rows 577 / 613.  (Weight gradients contract
     over the rows and gain at every size: 64 x (128, 2816, 2048) 1206 / 1634.)"""
     return _use_pair(rows, N, None) and (_PAIR_MODE == "1" or (rows >= 512 * G and K >= 2560))
+
+
+def _use_grouped_turned(out: torch.Tensor, N: int, K: int) -> bool:
+    """Whether grouped products take the CTA-pair kernel with tiles that are cut along a group's rows (a multiple of 64 of them;
+    ``TurnedSegments`` in csrc/sm100/gemm2.cu), which it does wherever it is called and the results can be stored that way.  Ragged
+    groups, us, one CTA / turned pair: 8 x (1024 rows, 28672 columns, K = 4096) 1667 / 1589, 512 rows 974 / 920, 128 rows 430 / 374,
+    64 rows 350 / 340, 32 rows 344 / 325; 8 x (128, 4096, 14336) 235 / 189, 64 rows 170 / 172; 64 x (128, 2816, 2048) 185 / 176; 64 x
+    (512, 2048, 1408) 230 / 221; 8 x (300, 4096, 1024) 31.1 / 30.8."""
+    return (_use_pair(256, N, None) and K >= 1280 and N % 2 == 0 and out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0)
 
 
 def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False, out: torch.Tensor | None = None,
@@ -239,7 +248,8 @@ def grouped_gemm(a: torch.Tensor, b: torch.Tensor, row_start: torch.Tensor, *, b
     lib = _lib.load()
     args = (a.data_ptr(), b2.data_ptr(), out.data_ptr(), row_start.data_ptr(), G, a.shape[0], N, K, a.stride(0),
             b2.stride(0), out.stride(0), int(b_mn), OUT_BF16, _lib.stream())
-    rc = lib.hg_grouped_gemm2_bf16(*args) if _use_grouped_pair(a.shape[0], N, K, G) else -2
+    pair = _use_grouped_turned(out, N, K) or _use_grouped_pair(a.shape[0], N, K, G)
+    rc = lib.hg_grouped_gemm2_bf16(*args) if pair else -2
     if rc == -2:
         rc = lib.hg_grouped_gemm_bf16(*args)
     _lib.check(rc, "hg_grouped_gemm_bf16")

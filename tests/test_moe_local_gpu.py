@@ -232,3 +232,26 @@ def test_grouped_gemm_of_ragged_segments(monkeypatch, seg, N, K, b_mn, pair):
     out[first:starts[-1]] = 3.0
     assert (whole == 3.0).all()
     _lib.assert_healthy()
+
+
+# tiles along a group's rows: one of 64 rows and one row more, five tiles of unequal need, segments that start anywhere, columns that
+# end inside a tile, a block and (odd: not turned) a pair, K that ends inside a block, by the rule and not by force
+@pytest.mark.parametrize("seg", [[64, 65, 1, 0, 1100], [256, 257, 511]])
+@pytest.mark.parametrize("N,K,b_mn", [(768, 1344, False), (1032, 1344, True), (330, 1288, False), (261, 1280, False)])
+def test_grouped_gemm_along_the_rows(seg, N, K, b_mn):
+    from hetu_galvatron_b200 import ops
+
+    g = torch.Generator(device=DEV).manual_seed(N + K + len(seg))
+    first, rows = 3, 3 + sum(seg) + 9
+    starts = [first + sum(seg[:i]) for i in range(len(seg) + 1)]
+    a = torch.randn(rows, K, device=DEV, generator=g).to(torch.bfloat16)
+    b = torch.randn(len(seg), *((K, N) if b_mn else (N, K)), device=DEV, generator=g).to(torch.bfloat16)
+    whole = torch.full((rows, N + 3 + N % 2), 3.0, device=DEV, dtype=torch.bfloat16)
+    out = whole[:, 2:N + 2]
+    ops.grouped_gemm(a, b, torch.tensor(starts, device=DEV, dtype=torch.int32), b_mn=b_mn, out=out)
+    for i in range(len(seg)):
+        ref = a[starts[i]:starts[i + 1]].double() @ (b[i].double() if b_mn else b[i].double().t())
+        assert torch.allclose(out[starts[i]:starts[i + 1]].double(), ref, rtol=2.0 ** -8, atol=1e-4 * K ** 0.5)
+    out[first:starts[-1]] = 3.0
+    assert (whole == 3.0).all()
+    _lib.assert_healthy()
