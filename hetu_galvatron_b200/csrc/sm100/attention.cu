@@ -37,22 +37,39 @@ __device__ __forceinline__ float ex2(float x) {
   return y;
 }
 
-// 2^x on the FMA pipe, for x <= 0 (probabilities): x is split by the add-a-large-constant rounding trick into an
-// integer n (left in the low mantissa bits of t) and f in [-0.5, 0.5]; 2^f is a degree-3 near-minimax polynomial
-// (maximum relative error 7.5e-5, a fiftieth of the bf16 rounding the result gets next) and n goes straight into
-// the exponent field.  Nine FMA / integer instructions against one on the special-function unit, which delivers
-// far fewer results per clock: giving a share of the elements to this path takes the exp2 unit off the critical path.
-// Inputs below -126 (masked entries, -inf) give exactly 0, as the flushing hardware instruction does.
-__device__ __forceinline__ float ex2_poly(float x) {
-  const float xc = fmaxf(x, -126.f);
-  const float t = xc + 12582912.f;         // 1.5 * 2^23
-  const float f = xc - (t - 12582912.f);
-  float r = fmaf(f, 0.05517165f, 0.24261113f);
-  r = fmaf(r, f, 0.69326097f);
-  r = fmaf(r, f, 0.99992806f);
-  r = __int_as_float(__float_as_int(r) + (__float_as_int(t) << 23));
-  return x < -126.f ? 0.f : r;
+// Two fp32 operations per instruction, each rounded as alone.  A pair of neighbouring registers is one operand.  The softmax of the
+// forward is bound by the instructions of its threads beside the exponentials: 2 x 4096 tokens and 32 heads of 128 317 us without,
+// 301 with these and max3; 8 x 1024 and 25 heads of 64 100, 97; 1531 and 28 heads on 4 46.9, 44.9.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\n"
+      "fma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmul.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+
+// The larger of three: one instruction.
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 // Softmax warpgroups of the 128-query dK/dV kernel.
 constexpr int kDkvWarpgroups = 4;
 // Softmax warpgroups of the 128-key dQ kernel (2 or 4).
@@ -60,12 +77,6 @@ constexpr int kDkvWarpgroups = 4;
 #define HG_DQ_WARPGROUPS 4
 #endif
 constexpr int kDqWarpgroups = HG_DQ_WARPGROUPS;
-// How many of every four exponentials of the two-tile forward kernel take ex2_poly instead of the special-function unit
-// (its two softmax warpgroups run at the same time and share that unit).
-#ifndef HG_FWD_POLY_OF_4
-#define HG_FWD_POLY_OF_4 0
-#endif
-
 // Per-role cycle counts of CTA (0, 0, 0), for builds with -DHG_ATTN_TIMING: where a step's time goes (waiting for the
 // other role, or working).  Lane 0 of the first softmax warp writes words 16..20 of the device status buffer
 // (steps, wait for S^T, probabilities, wait for dP^T, dS^T and stores), lane 0 of the MMA warp words 24..28 (steps, wait
@@ -306,13 +317,15 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           if (dead) s[i] = -INFINITY;
         }
       }
-      float mx4[4] = {s[0], s[1], s[2], s[3]};   // four chains: a single one is 127 dependent instructions long
+      float mx4[4] = {s[0], s[1], s[2], s[3]};   // four chains: a single one is 63 dependent instructions long
 #pragma unroll
-      for (int i = 4; i < 128; i += 4) {
-        mx4[0] = fmaxf(mx4[0], s[i]); mx4[1] = fmaxf(mx4[1], s[i + 1]);
-        mx4[2] = fmaxf(mx4[2], s[i + 2]); mx4[3] = fmaxf(mx4[3], s[i + 3]);
+      for (int i = 4; i < 124; i += 8) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mx4[u] = max3(mx4[u], s[i + u], s[i + 4 + u]);
       }
-      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(mx4[u], s[124 + u]);
+      float mx = max3(mx4[0], mx4[1], fmaxf(mx4[2], mx4[3]));
       mx *= sl2;
       // lazy rescale: keep the running reference max unless the new max exceeds it by more than 2^8
       float alpha = 1.f;
@@ -323,16 +336,15 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         rescale = (j > 0);
       }
       const float nmref = (m_used == -INFINITY) ? 0.f : -m_used;
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+      float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
-      for (int i = 0; i < 128; i += 4) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          s[i + u] = ex2(fmaf(s[i + u], sl2, nmref));
-          sum4[u] += s[i + u];
-        }
+      for (int i = 0; i < 128; i += 2) {
+        const float2 x = fma2(make_float2(s[i], s[i + 1]), make_float2(sl2, sl2), make_float2(nmref, nmref));
+        s[i] = ex2(x.x);
+        s[i + 1] = ex2(x.y);
+        sum2[(i >> 1) & 1] = add2(sum2[(i >> 1) & 1], make_float2(s[i], s[i + 1]));
       }
-      l = l * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
+      l = l * alpha + ((sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y));
       if (j > 0) {
         if (!mbar_wait_warp(o_done, (j - 1) & 1, p.status, kTimeoutOther, abort_flag)) { ok = false; break; }
         tc_fence_after();
@@ -642,13 +654,15 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
           if (dead) s[i] = -INFINITY;
         }
       }
-      float mx4[4] = {s[0], s[1], s[2], s[3]};   // four chains: a single one is 127 dependent instructions long
+      float mx4[4] = {s[0], s[1], s[2], s[3]};   // four chains: a single one is 63 dependent instructions long
 #pragma unroll
-      for (int i = 4; i < 128; i += 4) {
-        mx4[0] = fmaxf(mx4[0], s[i]); mx4[1] = fmaxf(mx4[1], s[i + 1]);
-        mx4[2] = fmaxf(mx4[2], s[i + 2]); mx4[3] = fmaxf(mx4[3], s[i + 3]);
+      for (int i = 4; i < 124; i += 8) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mx4[u] = max3(mx4[u], s[i + u], s[i + 4 + u]);
       }
-      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) mx4[u] = fmaxf(mx4[u], s[124 + u]);
+      float mx = max3(mx4[0], mx4[1], fmaxf(mx4[2], mx4[3]));
       mx *= sl2;
       // lazy rescale: keep the running reference max unless the new max exceeds it by more than 2^8
       float alpha = 1.f;
@@ -673,21 +687,16 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
       }
       // P, packed, over the first 64 of this row's S columns, in two halves: the PV product of keys 0..63 runs while
       // the exponentials of keys 64..127 are taken
-      float sum4[4] = {0.f, 0.f, 0.f, 0.f};
+      float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
         uint32_t pk[32];
 #pragma unroll
-        for (int i = 0; i < 64; i += 4) {
-          float e[4];
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float x = fmaf(s[hh * 64 + i + u], sl2, nmref);
-            e[u] = (u < HG_FWD_POLY_OF_4) ? ex2_poly(x) : ex2(x);
-            sum4[u] += e[u];
-          }
-          pk[i >> 1] = pack_bf16(e[0], e[1]);
-          pk[(i >> 1) + 1] = pack_bf16(e[2], e[3]);
+        for (int i = 0; i < 64; i += 2) {
+          const float2 x = fma2(make_float2(s[hh * 64 + i], s[hh * 64 + i + 1]), make_float2(sl2, sl2), make_float2(nmref, nmref));
+          const float2 e = make_float2(ex2(x.x), ex2(x.y));
+          sum2[(i >> 1) & 1] = add2(sum2[(i >> 1) & 1], e);
+          pk[i >> 1] = pack_bf16(e.x, e.y);
         }
         tmem_st32(tS[t] + lane_off + hh * 32, pk);
         tmem_st_wait();
@@ -695,7 +704,7 @@ flash_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant
         mbar_arrive_warp(&p_full[2 * t + hh]);
         if (hh == 0) { HG_DKV_TOCK(tm_math, t0); }
       }
-      l = l * alpha + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
+      l = l * alpha + ((sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y));
       HG_DKV_TOCK(tm_st, t0);
     }
     if (t == 0) { HG_DKV_REPORT(0, my_kv, tm_wait_s, tm_ld, tm_math, tm_st); }
@@ -1222,30 +1231,6 @@ __device__ __forceinline__ float4 lds_f4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
   return v;
-}
-
-// Two fp32 operations per instruction, each rounded as alone.  A pair of neighbouring registers is one operand.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{\n.reg .b64 a, b, c, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmov.b64 c, {%6, %7};\n"
-      "fma.rn.f32x2 d, a, b, c;\nmov.b64 {%0, %1}, d;\n}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nadd.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n.reg .b64 a, b, d;\nmov.b64 a, {%2, %3};\nmov.b64 b, {%4, %5};\nmul.rn.f32x2 d, a, b;\nmov.b64 {%0, %1}, d;\n}"
-      : "=f"(d.x), "=f"(d.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
 }
 
 template <int HD>
