@@ -44,7 +44,7 @@ struct Kernels {
   long long (*gemm2_scratch)(int, int, int);
   int (*gemm_skinny)(V, V, void*, V, int, int, int, int, int, int, int, int, int, void*);
   int (*colsum_parts)(int, int);
-  int (*colsum)(V, long long, int, int, void*, int, void*, void*);
+  int (*colsum)(V, long long, int, int, void*, int, void*, void*, int, void*);
   int (*norm_fwd)(V, V, V, V, void*, void*, void*, void*, int, int, float, int, void*);
   int (*norm_bwd)(V, V, V, V, V, V, void*, void*, void*, void*, int, int, int, int, int, void*);
   int (*glu_fwd)(V, void*, long long, int, int, void*);
@@ -137,17 +137,23 @@ void gemm(const Tensor& a_in, const Tensor& b_in, const Tensor& out, const void*
   check(K.gemm(a.data_ptr(), b.data_ptr(), out.data_ptr(), bias, m, n, k, lda, ldb, ldc, a_mn, b_mn, mode, 0, st), "hg_gemm_bf16");
   count();
 }
-Tensor column_sums(const Tensor& x_in) {
+// The sums of the columns of x, in its type; or, where `into` is defined, written or added to that fp32 vector.
+Tensor column_sums(const Tensor& x_in, const Tensor& into = Tensor(), bool accumulate = false) {
   const int64_t rows = x_in.size(0), cols = x_in.size(1);
   const bool graph = at::GradMode::is_enabled() && x_in.requires_grad();     // a graph of the gradient is wanted
   const Tensor x = graph || x_in.scalar_type() != g_lp ? x_in : rowmajor(x_in);
-  if (graph || rows == 0 || cols == 0 || x.scalar_type() != g_lp || x.stride(0) % 8 || !aligned(x))
-    return x.to(at::kFloat).sum(0).to(x.scalar_type());
-  Tensor out = empty({cols}, g_lp, x);
+  if (graph || rows == 0 || cols == 0 || x.scalar_type() != g_lp || x.stride(0) % 8 || !aligned(x)) {
+    const Tensor sums = x.to(at::kFloat).sum(0);
+    if (!into.defined()) return sums.to(x.scalar_type());
+    at::NoGradGuard no_grad;
+    return accumulate ? into.add_(sums) : into.copy_(sums);
+  }
+  Tensor out = into.defined() ? into : empty({cols}, g_lp, x);
   const int parts = K.colsum_parts(int(rows), int(cols));
   const Tensor partial = parts > 1 ? empty({parts, cols}, at::kFloat, x) : Tensor();
   check(K.colsum(x.data_ptr(), x.stride(0), int(rows), int(cols), parts > 1 ? partial.data_ptr() : nullptr, parts,
-                 out.data_ptr(), stream()), "hg_colsum_bf16");
+                 into.defined() ? nullptr : out.data_ptr(), into.defined() ? out.data_ptr() : nullptr, accumulate, stream()),
+        "hg_colsum");
   count(parts > 1 ? 2 : 1);
   return out;
 }
@@ -157,6 +163,7 @@ Tensor column_sums(const Tensor& x_in) {
 struct MainGrad {
   Tensor buf;
   bool fresh = false;
+  MainGrad() = default;
   explicit MainGrad(const Tensor& p) {
     pybind11::gil_scoped_acquire gil;
     py::object o = py::reinterpret_steal<py::object>(THPVariable_Wrap(p));
@@ -173,9 +180,19 @@ struct MainGrad {
   }
 };
 
+// The gradient buffer of a bias or norm bias, if this node may write it itself: a vector of `n` fp32 values, and nobody on the way
+// to the parameter who wants to see the gradient (hooks of the tensor or behind its accumulation).
+bool takes_vector(const MainGrad& mg, const Tensor& p, int64_t n) {
+  if (!mg.buf.defined() || mg.buf.scalar_type() != at::kFloat || !mg.buf.is_cuda() || mg.buf.numel() != n || !mg.buf.is_contiguous())
+    return false;
+  if (!p.is_leaf() || !torch::autograd::impl::hooks(p).empty() || torch::autograd::impl::post_acc_grad_hooks(p) != nullptr) return false;
+  const auto node = torch::autograd::impl::try_get_grad_accumulator(p);
+  return node == nullptr || (node->pre_hooks().empty() && node->post_hooks().empty() && node->tensor_pre_hooks().empty());
+}
+
 struct Linear : public Function<Linear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& bias) {
-    ctx->save_for_backward({x, w});
+    ctx->save_for_backward(bias ? variable_list{x, w, *bias} : variable_list{x, w});
     ctx->saved_data["bias"] = bias.has_value();
     Tensor y = empty({x.size(0), w.size(0)}, g_lp, x);
     gemm(x, w, y, bias ? bias->data_ptr() : nullptr, false, false, kOutLp);
@@ -203,7 +220,15 @@ struct Linear : public Function<Linear> {
         gemm(dy, x, dw, nullptr, true, true, kOutLp);
       }
     }
-    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) db = column_sums(dy);
+    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) {
+      const MainGrad mg(saved[2]);
+      if (takes_vector(mg, saved[2], dy.size(1))) {
+        column_sums(dy, mg.buf, !mg.fresh);
+        MainGrad::written(saved[2]);
+      } else {
+        db = column_sums(dy);
+      }
+    }
     return {dx, dw, db};
   }
 };
@@ -221,7 +246,7 @@ struct Norm : public Function<Norm> {
                      y.data_ptr(), residual ? h.data_ptr() : nullptr, rstd.data_ptr(), rms ? nullptr : mean.data_ptr(),
                      int(rows), int(H), float(eps), rms, stream()), "hg_norm_fwd");
     count();
-    ctx->save_for_backward({h, w, rstd, rms ? rstd : mean});
+    ctx->save_for_backward(b ? variable_list{h, w, rstd, rms ? rstd : mean, *b} : variable_list{h, w, rstd, rms ? rstd : mean});
     ctx->saved_data["rms"] = rms;
     ctx->saved_data["residual"] = residual.has_value();
     ctx->saved_data["bias"] = b.has_value();
@@ -242,17 +267,21 @@ struct Norm : public Function<Norm> {
     if (mg.buf.defined() && (mg.buf.scalar_type() != at::kFloat || !mg.buf.is_cuda() || mg.buf.numel() != H || !mg.buf.is_contiguous()))
       raise(PyExc_ValueError, "bad output tensor");
     const Tensor dw = mg.buf.defined() ? mg.buf : empty({H}, at::kFloat, h);
-    // zero-filled: the kernel's accumulate switch is shared with dw (which may add into main_grad)
-    const Tensor db = bias ? at::zeros({H}, h.options().dtype(at::kFloat)) : Tensor();
+    // The kernel's accumulate switch is shared with dw (which may add into main_grad): db goes the same way, or into zeros.
+    const bool adds = mg.buf.defined() && !mg.fresh;
+    const MainGrad mg_b = bias ? MainGrad(saved[4]) : MainGrad();
+    const bool b_direct = bias && ctx->needs_input_grad(residual ? 3 : 2) && takes_vector(mg_b, saved[4], H) && !mg_b.fresh == adds;
+    const Tensor db = b_direct ? mg_b.buf : bias ? at::zeros({H}, h.options().dtype(at::kFloat)) : Tensor();
     check(K.norm_bwd(dy.data_ptr(), h.data_ptr(), w.data_ptr(), rstd.data_ptr(), rms ? nullptr : mean.data_ptr(),
                      dres.defined() ? dres.data_ptr() : nullptr, dx.data_ptr(), dw.data_ptr(), bias ? db.data_ptr() : nullptr,
-                     partial.data_ptr(), kNormParts, int(rows), int(H), rms, mg.buf.defined() && !mg.fresh, stream()),
+                     partial.data_ptr(), kNormParts, int(rows), int(H), rms, adds, stream()),
           "hg_norm_bwd");
-    count(rms ? 2 : 3);
+    count(2);
     if (mg.buf.defined()) MainGrad::written(w);
+    if (b_direct) MainGrad::written(saved[4]);
     // dx is the gradient of both x and the residual input (they are summed in the forward)
     return {dx, residual ? dx : Tensor(), mg.buf.defined() ? Tensor() : dw.to(w.scalar_type()),
-            bias ? db.to(w.scalar_type()) : Tensor(), Tensor(), Tensor()};
+            bias && !b_direct ? db.to(w.scalar_type()) : Tensor(), Tensor(), Tensor()};
   }
 };
 
@@ -670,7 +699,7 @@ void bind(const py::dict& fn, bool half, int pair_mode, py::object kernel_error)
     slot = reinterpret_cast<std::decay_t<decltype(slot)>>(py::cast<uintptr_t>(fn[name]));
   };
   at("hg_gemm_bf16", K.gemm); at("hg_gemm2_bf16", K.gemm2); at("hg_gemm2_scratch", K.gemm2_scratch); at("hg_gemm_skinny_bf16", K.gemm_skinny);
-  at("hg_colsum_parts", K.colsum_parts); at("hg_colsum_bf16", K.colsum);
+  at("hg_colsum_parts", K.colsum_parts); at("hg_colsum", K.colsum);
   at("hg_norm_fwd", K.norm_fwd); at("hg_norm_bwd", K.norm_bwd);
   at("hg_glu_fwd", K.glu_fwd); at("hg_glu_bwd", K.glu_bwd); at("hg_add_bf16", K.add); at("hg_rope", K.rope);
   at("hg_flash_fwd", K.flash_fwd); at("hg_flash_bwd_scratch", K.flash_bwd_scratch); at("hg_flash_bwd_scratch_of", K.flash_bwd_scratch_of); at("hg_flash_bwd_ws", K.flash_bwd);

@@ -337,11 +337,18 @@ norm_bwd_kernel(const hg_lp_t* __restrict__ dy, const hg_lp_t* __restrict__ h,
 // out[c] (+)= sum_p partial[p, c], parts taken in a fixed order.  A CTA owns 32 columns and its 16 warps share the
 // parts; one thread per column with all parts in one chain left most of the chip idle for the whole sum.
 __global__ void __launch_bounds__(512)
-reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, int parts, int H, int accumulate) {
+reduce_partials_kernel(const float* __restrict__ partial, float* __restrict__ out, const float* __restrict__ partial_b,
+                       float* __restrict__ out_b, int parts, int H, int accumulate) {
   hg::chain_release();
   const int zero = hg::chain_wait();
   partial += zero;
   out += zero;
+  partial_b += zero;
+  out_b += zero;
+  if (blockIdx.y == 1) {                     // a LayerNorm's bias, in the same launch
+    partial = partial_b;
+    out = out_b;
+  }
   __shared__ float red[16][32];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + lane;
@@ -373,8 +380,9 @@ int launch_norm_bwd(const void* dy, const void* h, const void* w, const void* rs
                            (const hg_lp_t*)w, (const float*)rstd, (const float*)mean, (const hg_lp_t*)dres, (hg_lp_t*)dx, P,
                            RMS ? nullptr : PB, rows, H);
   const int cols = (H + 31) / 32;
-  if (rc == 0) rc = hg_host::launch_over(reduce_partials_kernel, cols, 512, 0, st, P, (float*)dw, grid, H, accumulate);
-  if (rc == 0 && !RMS && db) rc = hg_host::launch_over(reduce_partials_kernel, cols, 512, 0, st, PB, (float*)db, grid, H, accumulate);
+  if (rc == 0)
+    rc = hg_host::launch_over(reduce_partials_kernel, dim3(cols, !RMS && db ? 2 : 1), 512, 0, st, P, (float*)dw, PB, (float*)db, grid, H,
+                              accumulate);
   return rc;
 }
 

@@ -80,6 +80,7 @@ _SIGNATURES = {
     "hg_gemm_skinny_bf16": [c_void_p] * 4 + [c_int] * 9 + [c_void_p],
     "hg_colsum_parts": [c_int, c_int],
     "hg_colsum_bf16": [c_void_p, c_ll, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p],
+    "hg_colsum": [c_void_p, c_ll, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p],
     "hg_moe_plan": [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
     "hg_moe_scatter": [c_void_p, c_ll, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
     "hg_moe_gather": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p],
@@ -211,7 +212,7 @@ def _bind_native(lib):
 
         warnings.warn("hg_torch_ops is not usable (%s): autograd nodes run in Python" % (e,))
         return
-    names = ("hg_gemm_bf16", "hg_gemm2_bf16", "hg_gemm2_scratch", "hg_gemm_skinny_bf16", "hg_colsum_parts", "hg_colsum_bf16", "hg_norm_fwd",
+    names = ("hg_gemm_bf16", "hg_gemm2_bf16", "hg_gemm2_scratch", "hg_gemm_skinny_bf16", "hg_colsum_parts", "hg_colsum", "hg_norm_fwd",
              "hg_norm_bwd", "hg_glu_fwd", "hg_glu_bwd", "hg_add_bf16", "hg_rope", "hg_flash_fwd", "hg_flash_bwd_scratch",
              "hg_flash_bwd_scratch_of", "hg_flash_bwd_ws", "hg_decoder_step", "hg_decoder_step_scratch")
     mode = {"0": 0, "1": 1}.get(os.environ.get("HG_GEMM_PAIR", "auto"), -1)

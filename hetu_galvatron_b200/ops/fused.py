@@ -72,7 +72,7 @@ class _Norm(torch.autograd.Function):
         if mgw is not None:
             w.mg_fresh = False
         _lib.check(rc, "hg_norm_bwd")
-        _lib.count_launch(2 if ctx.rms else 3)
+        _lib.count_launch(2)
         gw = None if mgw is not None else dw.to(w.dtype)
         gb = db.to(w.dtype) if db is not None else None
         # dx carries the gradient of both x and the residual input (they are summed in the forward)
@@ -84,8 +84,8 @@ def norm(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor | None = None, eps: f
     """Returns ``(normalised, h)`` with ``h = x + residual`` (``h is x`` without a residual).
 
     Fusing the residual add means the block computes ``h = x + attn_out`` and ``norm(h)`` in one pass
-    over memory.  Note for LayerNorm with bias: the bias gradient is returned through the normal
-    autograd path (fp32 -> parameter dtype)."""
+    over memory.  The bias gradient goes to ``b.main_grad`` where one is bound and nothing hooks
+    the parameter's gradient (C++ nodes), else through the normal autograd path (fp32 -> parameter dtype)."""
     shp = x.shape
     if not x.is_cuda:
         h = x if residual is None else x + residual

@@ -148,3 +148,33 @@ def test_errors_are_those_of_the_python_route():
     w.main_grad = torch.zeros(32, 64, device=DEV)
     with pytest.raises(ValueError, match="bad output"):
         ops.linear(randn(300, 64), w).sum().backward()
+
+
+# the gradients of a bias and a norm's bias written, or added, straight to their buffers; with a hook on the parameter they take the
+# way through autograd that shows them to it
+@pytest.mark.parametrize("rows", [1, 40, 999])
+@pytest.mark.parametrize("fresh", [True, False])
+@pytest.mark.parametrize("hooked", [False, True])
+def test_bias_gradients_go_to_their_buffers(rows, fresh, hooked):
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g).to(torch.bfloat16)
+    w, b, nw, nb = [torch.nn.Parameter(t) for t in (rand(520, 264), rand(520), rand(264), rand(264))]
+    seen = []
+    for p in (w, b, nw, nb):
+        p.main_grad, p.mg_fresh = torch.full(p.shape, 2.0, device="cuda"), fresh
+        if hooked and p.dim() == 1 and p is not nw:
+            p.register_hook(lambda t: seen.append(t.shape))
+    x, dy = rand(rows, 264).requires_grad_(), rand(rows, 520)
+    n = ops.norm(x, nw, nb, 1e-5, rms=False)[0]
+    ops.linear(n, w, b).backward(dy)
+    ref = dy.double().sum(0)
+    dn = (dy.double() @ w.detach().double()).sum(0)
+    for p, want in ((b, ref), (nb, dn)):
+        if hooked:
+            assert p.mg_fresh is fresh and (p.main_grad == 2.0).all() and len(seen) == 2
+        else:
+            assert p.grad is None and not p.mg_fresh
+            got = p.main_grad.double() - (0.0 if fresh else 2.0)
+            # fp32 sums of 16-bit rows; dy of the norm was rounded to 16 bits once: rows of about 23 (520 products of unit normals)
+            atol = 1e-5 * rows ** 0.5 * 10 if p is b else 2.0 ** -9 * 23 * 6 * rows ** 0.5
+            assert torch.allclose(got, want, rtol=1e-5, atol=atol)
