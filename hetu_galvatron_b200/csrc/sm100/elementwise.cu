@@ -342,6 +342,87 @@ __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids, const hg_l
   }
 }
 
+// The same gradient with the tokens of a row of dW brought together, for up to kSortTokens tokens: what bounds the scatter above is
+// its reductions in L2, and in text more than half of them meet a row that another token of the batch has as well.  One block sorts
+// (row, token) in shared memory, 7 us per 1024 tokens in 91 passes of a bitonic network, while the others clear dW.  A block of the second kernel then adds the tokens of kRunTokens
+// neighbouring keys in registers and leaves one row of sums per run, as plain stores where the run is all of its row's tokens.  8192 tokens x 4096 of 32000 rows, frequencies as in text, us: cleared 72 and scattered 59, 110 so; 8192 x 3584 of 152064 347, 322.
+constexpr int kSortTokens = 16384, kSortIndexBits = 14, kRunTokens = 8, kClearVecs = 8192;
+constexpr unsigned kNoRow = 0xffffffffu;
+static_assert(1 << kSortIndexBits == kSortTokens, "an index of a key");
+
+__global__ void __launch_bounds__(1024)
+embedding_sort_kernel(const int64_t* __restrict__ ids, unsigned* __restrict__ keys, int tokens, int v0, int v1, float4* __restrict__ dW,
+                      int64_t n4) {
+  extern __shared__ unsigned k[];
+  if (blockIdx.x > 0) {
+    const int64_t at = int64_t(blockIdx.x - 1) * kClearVecs + threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < kClearVecs; i += 1024)
+      if (at + i < n4) dW[at + i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    return;
+  }
+  int n = 1;
+  while (n < tokens) n <<= 1;
+  for (int i = threadIdx.x; i < n; i += 1024) {
+    const int64_t id = i < tokens ? ids[i] : -1;
+    k[i] = id >= v0 && id < v1 && i < tokens ? unsigned(id - v0) << kSortIndexBits | unsigned(i) : kNoRow;
+  }
+  for (int width = 2; width <= n; width <<= 1)
+    for (int d = width >> 1; d > 0; d >>= 1) {
+      __syncthreads();
+      for (int p = threadIdx.x; p < n >> 1; p += 1024) {
+        const int lo = 2 * (p & ~(d - 1)) + (p & (d - 1)), hi = lo + d;
+        const unsigned a = k[lo], b = k[hi];
+        if ((a > b) == ((lo & width) == 0)) {
+          k[lo] = b;
+          k[hi] = a;
+        }
+      }
+    }
+  __syncthreads();
+  for (int i = threadIdx.x; i < tokens; i += 1024) keys[i] = k[i];
+}
+
+__global__ void __launch_bounds__(256)
+embedding_run_kernel(const unsigned* __restrict__ keys, const hg_lp_t* __restrict__ dout, float* __restrict__ dW, int tokens, int H) {
+  const int c = blockIdx.y * 256 + threadIdx.x, first = blockIdx.x * kRunTokens;
+  if (c >= H >> 3) return;
+  unsigned key[kRunTokens + 2];                     // with a neighbour on either side
+#pragma unroll
+  for (int i = 0; i < kRunTokens + 2; ++i) {
+    const int at = first + i - 1;
+    key[i] = at >= 0 && at < tokens ? keys[at] : kNoRow;
+  }
+  uint4 v[kRunTokens];
+#pragma unroll
+  for (int i = 0; i < kRunTokens; ++i)
+    if (key[i + 1] != kNoRow) v[i] = reinterpret_cast<const uint4*>(dout + size_t(key[i + 1] & (kSortTokens - 1)) * H)[c];
+  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  bool whole = true;                                // the run starts in this block
+#pragma unroll
+  for (int i = 1; i <= kRunTokens; ++i) {
+    if (key[i] == kNoRow) break;                    // sorted behind all others
+    const unsigned row = key[i] >> kSortIndexBits;
+    if (i == 1) whole = key[0] == kNoRow || key[0] >> kSortIndexBits != row;
+    float g[8];
+    unpack8(v[i - 1], g);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] += g[j];
+    const bool goes_on = key[i + 1] != kNoRow && key[i + 1] >> kSortIndexBits == row;
+    if (goes_on && i < kRunTokens) continue;
+    float* dst = dW + size_t(row) * H + c * 8;
+    if (whole && !goes_on) {
+      reinterpret_cast<float4*>(dst)[0] = make_float4(s[0], s[1], s[2], s[3]);
+      reinterpret_cast<float4*>(dst)[1] = make_float4(s[4], s[5], s[6], s[7]);
+    } else {
+      add8<true>(dst, s);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] = 0.f;
+    whole = true;
+  }
+}
+
 // ---------------------------------------------------------------------------------------------
 // Column sums of a 16-bit matrix (bias gradients): out[c] = sum_r x[r, c] in fp32, rounded once, or written or added to fp32.
 // A CTA takes 256 columns (32 lanes of eight) and one of `parts` row ranges, its eight warps share the rows.
@@ -602,6 +683,29 @@ int hg_embedding_bwd(const void* ids, const void* dout, void* dW, void* dpos, in
   else
     embedding_bwd_kernel<false><<<g, 256, 0, (cudaStream_t)stream>>>(
         (const int64_t*)ids, (const hg_lp_t*)dout, (float*)dW, (float*)dpos, tokens, H, v0, v1, batch, pos_offset);
+  return int(cudaGetLastError());
+}
+
+// Whether hg_embedding_bwd_runs takes a batch: where the sort is over before the table is cleared (7 us per 1024 tokens against
+// 7.3 TB/s); into a table that holds something, where the sort has nothing to hide behind, 8192 tokens take 85 us and 54 scattered.
+int hg_embedding_bwd_runs_takes(const void* dW, int tokens, int H, int rows) {
+  return tokens >= 256 && tokens <= kSortTokens && H > 0 && H % 8 == 0 && rows > 0 && rows <= (int)(kNoRow >> kSortIndexBits) &&
+         (uintptr_t(dW) & 15) == 0 && (long long)rows * H >= 12288ll * tokens;
+}
+// dW [rows, H] = the sums of the gradients of the tokens of rows v0 .. v0 + rows - 1.  keys: scratch of `tokens` words.
+int hg_embedding_bwd_runs(const void* ids, const void* dout, void* dW, void* keys, int tokens, int H, int v0, int rows, void* stream) {
+  if (!hg_embedding_bwd_runs_takes(dW, tokens, H, rows)) return -1;
+  cudaStream_t st = (cudaStream_t)stream;
+  int n = 1;
+  while (n < tokens) n <<= 1;
+  static const cudaError_t rc0 =
+      cudaFuncSetAttribute(embedding_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSortTokens * int(sizeof(unsigned)));
+  if (rc0 != cudaSuccess) return int(rc0);
+  const int64_t n4 = int64_t(rows) * H / 4;
+  embedding_sort_kernel<<<unsigned(1 + (n4 + kClearVecs - 1) / kClearVecs), 1024, n * sizeof(unsigned), st>>>(
+      (const int64_t*)ids, (unsigned*)keys, tokens, v0, v0 + rows, (float4*)dW, n4);
+  embedding_run_kernel<<<dim3((tokens + kRunTokens - 1) / kRunTokens, (H / 8 + 255) / 256), 256, 0, st>>>(
+      (const unsigned*)keys, (const hg_lp_t*)dout, (float*)dW, tokens, H);
   return int(cudaGetLastError());
 }
 

@@ -114,6 +114,8 @@ _SIGNATURES = {
     "hg_glu_fwd": [c_void_p, c_void_p, c_ll, c_int, c_int, c_void_p],
     "hg_glu_bwd": [c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int, c_void_p],
     "hg_embedding_fwd": [c_void_p] * 4 + [c_int] * 6 + [c_void_p],
+    "hg_embedding_bwd_runs_takes": [c_void_p, c_int, c_int, c_int],
+    "hg_embedding_bwd_runs": [c_void_p] * 4 + [c_int] * 4 + [c_void_p],
     "hg_embedding_bwd": [c_void_p] * 4 + [c_int] * 6 + [c_void_p],
     "hg_cast_f32_bf16": [c_void_p, c_void_p, c_ll, c_void_p],
     "hg_add_bf16": [c_void_p, c_void_p, c_void_p, c_ll, c_void_p],

@@ -332,10 +332,19 @@ class _Embedding(torch.autograd.Function):
         lib = _lib.load()
         g = g.contiguous()
         mg = getattr(W, "main_grad", None)
-        if mg is not None and getattr(W, "mg_fresh", False):
-            mg.zero_()
+        clear = mg is None or getattr(W, "mg_fresh", False)          # nothing in the buffer yet
+        dW = mg if mg is not None else torch.empty(W.shape, dtype=torch.float32, device=W.device)
+        tokens, H = ids.numel(), W.shape[1]
+        runs = clear and bool(lib.hg_embedding_bwd_runs_takes(dW.data_ptr(), tokens, H, W.shape[0]))
+        if clear and not runs:
+            dW.zero_()
+        if mg is not None:
             W.mg_fresh = False
-        dW = mg if mg is not None else torch.zeros(W.shape, dtype=torch.float32, device=W.device)
+        if runs:
+            keys = torch.empty(tokens, dtype=torch.int32, device=W.device)
+            _lib.check(lib.hg_embedding_bwd_runs(ids.data_ptr(), g.data_ptr(), dW.data_ptr(), keys.data_ptr(), tokens, H, v0,
+                                                 W.shape[0], _lib.stream()), "hg_embedding_bwd_runs")
+            _lib.count_launch(2)
         dpos = None
         if pos_emb is not None:
             mgp = getattr(pos_emb, "main_grad", None)
@@ -343,10 +352,11 @@ class _Embedding(torch.autograd.Function):
                 mgp.zero_()
                 pos_emb.mg_fresh = False
             dpos = mgp if mgp is not None else torch.zeros(pos_emb.shape, dtype=torch.float32, device=W.device)
-        _lib.check(lib.hg_embedding_bwd(ids.data_ptr(), g.data_ptr(), dW.data_ptr(), _lib.ptr(dpos), ids.numel(),
-                                        W.shape[1], v0, v0 + W.shape[0], batch, pos_offset, _lib.stream()),
-                   "hg_embedding_bwd")
-        _lib.count_launch()
+        if not runs or dpos is not None:
+            v1 = v0 if runs else v0 + W.shape[0]                     # no rows of W: the positions alone
+            _lib.check(lib.hg_embedding_bwd(ids.data_ptr(), g.data_ptr(), dW.data_ptr(), _lib.ptr(dpos), tokens, H, v0, v1, batch,
+                                            pos_offset, _lib.stream()), "hg_embedding_bwd")
+            _lib.count_launch()
         gW = None if mg is not None else dW.to(W.dtype)
         gP = None
         if pos_emb is not None and getattr(pos_emb, "main_grad", None) is None:

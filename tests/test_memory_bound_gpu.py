@@ -84,3 +84,34 @@ def test_bias_gradient_has_a_gradient():
     (gb,) = torch.autograd.grad(ops.linear(x, w, b), b, dy, create_graph=True)
     assert torch.equal(torch.autograd.grad((gb * v).sum(), dy)[0], v.expand(24, 40))
     _lib.assert_healthy()
+
+
+# the fewest tokens that are sorted and one less, counts around a power of two and a block of eight, the most and one more, tables on
+# both sides of the rule; tokens of other shards, a buffer that holds something
+@pytest.mark.parametrize("tokens,rows,H", [(255, 12288, 264), (256, 12288, 264), (1025, 6145, 2056), (1024, 3071, 4096),
+                                           (1024, 3072, 4096), (16384, 98304, 2056), (16385, 98304, 2056)])
+@pytest.mark.parametrize("fresh", [True, False])
+@pytest.mark.parametrize("positions", [False, True])
+def test_embedding_gradient(tokens, rows, H, fresh, positions):
+    from hetu_galvatron_b200 import ops
+    from hetu_galvatron_b200.ops import _lib
+
+    g = torch.Generator(device="cuda").manual_seed(tokens + H)
+    v0 = 7
+    u = torch.rand(tokens, device="cuda", generator=g, dtype=torch.float64)
+    ids = (torch.exp(u * float(torch.tensor(rows + 2.0).log())).long() - 1).clamp_(0, rows + 1) + v0 - 1   # some before, some behind
+    W = torch.nn.Parameter(torch.zeros(rows, H, device="cuda", dtype=torch.bfloat16))
+    W.main_grad, W.mg_fresh = torch.full((rows, H), float("nan") if fresh else 2.0, device="cuda"), fresh
+    pos = torch.nn.Parameter(torch.zeros(tokens // 2 + 1, H, device="cuda", dtype=torch.bfloat16)) if positions else None
+    dout = torch.randn(tokens, H, device="cuda", generator=g).to(torch.bfloat16)
+    ops.embedding(ids, W, v0, pos, 2).backward(dout)
+    want = torch.full((rows + 2, H), 0.0 if fresh else 2.0, device="cuda", dtype=torch.float64)
+    want.index_add_(0, ids - v0 + 1, dout.double())
+    most = int(torch.bincount(ids - v0 + 1).max())
+    # fp32 sums of at most `most` unit normals and what was there, each addition off by half a unit in the last place
+    assert torch.allclose(W.main_grad.double(), want[1:-1], rtol=0, atol=most * 2.0 ** -24 * (2 + 6 * most ** 0.5))
+    assert not W.mg_fresh
+    if positions:
+        ref = torch.zeros(pos.shape, device="cuda", dtype=torch.float64).index_add_(0, torch.arange(tokens, device="cuda") // 2, dout.double())
+        assert torch.allclose(pos.grad.double(), ref, rtol=2.0 ** -8, atol=1e-6)
+    _lib.assert_healthy()
