@@ -774,19 +774,22 @@ __global__ void __launch_bounds__(256)
 attn_bwd_dot_kernel(const hg_lp_t* __restrict__ O, const hg_lp_t* __restrict__ dO, int64_t ss, int64_t sb, int64_t dss,
                     int64_t dsb, int S, int B, int nheads, float* __restrict__ D) {
   constexpr int LPR = HD / 8, U = 4;              // lanes per row, rows in flight per thread
-  const int64_t total = int64_t(S) * B * nheads;
+  // 2^31 rows of 64 channels would be 275 GB: rows are counted in 32 bits, since a 64-bit division per row is most of the kernel's
+  // instructions, which bound it (us with / without: 2 x 4096 tokens and 32 heads of 128 34 / 29, 8 x 1024 and 25 of 64 16.5 / 14.3)
+  const unsigned total = unsigned(S) * unsigned(B) * unsigned(nheads);
   const int sub = threadIdx.x % LPR;
-  const int64_t stride = int64_t(gridDim.x) * (256 / LPR);
-  for (int64_t r0 = int64_t(blockIdx.x) * (256 / LPR) + threadIdx.x / LPR; r0 - threadIdx.x / LPR < total; r0 += U * stride) {
+  const unsigned stride = gridDim.x * (256 / LPR);
+  for (unsigned r0 = blockIdx.x * (256 / LPR) + threadIdx.x / LPR; r0 - threadIdx.x / LPR < total; r0 += U * stride) {
     uint4 a[U], c[U];
     float* dst[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      const int64_t row = r0 + u * stride;
+      const unsigned row = r0 + u * stride;
       dst[u] = nullptr;
       a[u] = c[u] = make_uint4(0, 0, 0, 0);
       if (row < total) {
-        const int tok = int(row / nheads), h = int(row - int64_t(tok) * nheads), s = tok / B, b = tok - s * B;
+        const unsigned tok = row / unsigned(nheads);
+        const int h = int(row - tok * unsigned(nheads)), s = int(tok / unsigned(B)), b = int(tok) - s * B;
         a[u] = dot_load8<VEC>(O + s * ss + b * sb + h * HD + sub * 8);
         c[u] = dot_load8<VEC>(dO + s * dss + b * dsb + h * HD + sub * 8);
         dst[u] = D + (size_t(b) * nheads + h) * S + s;
