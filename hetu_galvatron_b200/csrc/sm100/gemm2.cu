@@ -602,6 +602,16 @@ int hg_gemm2_bf16(const void* A, const void* B, void* C, const void* bias, int M
   return launch2<false, false>(ta, tb, tc, p, plan, max_pairs, pairs, ws, ws_bytes, st);
 }
 
+// How hg_gemm2_bf16 cuts a product for `pairs` pairs: columns of a tile, whether A and B change places (`may_turn`: if C allows it),
+// pairs per tile of the last wave (below 2: one), its tiles, epilogue warps per 32 rows.  Needs no device.
+int hg_gemm2_plan(int M, int N, int K, int out_mode, int may_turn, int pairs, int* plan) {
+  const TilePlan t = tile_plan(M, N, K, out_mode, may_turn && out_mode == kOutBf16, pairs);
+  const int threads = threads_for(out_mode, (long long)((K + BK - 1) / BK) * (kBlockCost + t.bn));
+  const int of_plan[5] = {t.bn, t.turned, t.s, t.tail, (threads - 64) / (32 * EPI_WARPS)};
+  for (int i = 0; i < 5; ++i) plan[i] = of_plan[i];
+  return 0;
+}
+
 // Bytes of scratch that hg_gemm2_bf16 may ask for on the current device, whatever the type of the result (0: none).
 long long hg_gemm2_scratch(int M, int N, int K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;

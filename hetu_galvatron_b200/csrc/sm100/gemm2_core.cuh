@@ -302,12 +302,15 @@ __device__ __forceinline__ float4 lds128(uint32_t addr) {
   return v;
 }
 
-// w: the 128 bytes of this thread's row, to columns col0.. of rows y0 .. y0 + 31 of the map.
 // H warps share 32 rows: the one with number h takes the blocks h, h + H, ...
 struct Share {
   int h, H;
 };
+// Columns of a block: 128 bytes of a row where C leaves by TMA, else 32.  The parts of a shared tile are stored in the same
+// blocks, because a warp that adds them has counted the arrivals of the warps of its own number alone.
+__host__ __device__ constexpr int block_columns(bool tma, int out_mode) { return tma && out_mode == kOutBf16 ? 64 : 32; }
 
+// w: the 128 bytes of this thread's row, to columns col0.. of rows y0 .. y0 + 31 of the map.
 // Bulk groups belong to a thread: lane 0 issues and waits.
 __device__ __forceinline__ void tma_store_rows(const CUtensorMap* tm, uint32_t buf, const uint32_t (&w)[32], int col0, int y0) {
   const uint32_t lane = lane_id();
@@ -424,7 +427,7 @@ __device__ __forceinline__ void store_block64_tma(const Params& p, const CUtenso
 template <bool BIAS, bool F32>
 __device__ __forceinline__ void store_tile_tma(const Params& p, const CUtensorMap* tmC, uint32_t stg, Share w, uint32_t src, int row0,
                                                int y0, int n0, const Parts& parts) {
-  constexpr int kBlock = F32 ? 32 : 64;
+  constexpr int kBlock = block_columns(true, F32 ? kOutF32 : kOutBf16);
 #pragma unroll 1
   for (int c = w.h * kBlock; c < p.bn && n0 + c < p.N; c += w.H * kBlock) {
     uint32_t r0[32], r1[32];
@@ -724,16 +727,19 @@ __device__ __forceinline__ void epilogue2(const Params& p, const CUtensorMap* tm
       if (shared_tile) {
         // Nobody waits for another pair, whatever the order in which the device runs them.
         float* dst = ws_tile + size_t(w.slice) * (CM * p.bn);
+        const int cols = block_columns(p.c_tma != 0, p.out_mode);          // bn is a multiple of it
 #pragma unroll 1
-        for (int c = share.h; c < p.bn / 32; c += H) {
-          uint32_t r0[32];
-          tmem_ld32(src + c * 32, r0);
-          tmem_ld_wait();
+        for (int c0 = share.h * cols; c0 < p.bn; c0 += H * cols)
+#pragma unroll 1
+          for (int c = c0; c < c0 + cols; c += 32) {
+            uint32_t r0[32];
+            tmem_ld32(src + c, r0);
+            tmem_ld_wait();
 #pragma unroll
-          for (int q = 0; q < 8; ++q)
-            __stcg(reinterpret_cast<uint4*>(dst + split_word(p.bn, warp8, c, q)),
-                   make_uint4(r0[4 * q], r0[4 * q + 1], r0[4 * q + 2], r0[4 * q + 3]));
-        }
+            for (int q = 0; q < 8; ++q)
+              __stcg(reinterpret_cast<uint4*>(dst + split_word(p.bn, warp8, c / 32, q)),
+                     make_uint4(r0[4 * q], r0[4 * q + 1], r0[4 * q + 2], r0[4 * q + 3]));
+          }
         __threadfence();
         __syncwarp();
         int last = 0;

@@ -1,4 +1,8 @@
 """Stores of the CTA-pair GEMM: blocks that leave by TMA and blocks that are stored row by row, in every output mode."""
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -164,3 +168,29 @@ def test_tiles_of_every_width(M, N, K, a_mn, b_mn, biased, mode, left):
     out.fill_(2.0)
     assert (whole == 2.0).all()                                                 # nothing outside the window
     _lib.assert_healthy()
+
+
+# 16-bit results of shared tiles with two epilogue warps per 32 rows, which only HG_GEMM_SPLIT_TAIL=1 leads to: the blocks in which a
+# warp leaves its parts are those in which it adds them
+@pytest.mark.parametrize("M,N,K", [(256, 256, 1024), (343, 448, 1064), (600, 328, 1088), (512, 512, 1536)])
+def test_shared_16_bit_tiles_with_two_warps(M, N, K):
+    code = """
+import ctypes, torch
+from hetu_galvatron_b200 import ops
+from hetu_galvatron_b200.ops import _lib
+M, N, K = %r
+plan = (ctypes.c_int * 5)()
+_lib.load().hg_gemm2_plan(M, N, K, 0, 1, 74, plan)
+assert plan[0] == 64 and not plan[1] and plan[2] > 1 and plan[4] == 2, list(plan)
+g = torch.Generator(device="cuda").manual_seed(K)
+a, b = (torch.randn(n, K, device="cuda", generator=g).to(torch.bfloat16) for n in (M, N))
+ref = a.double() @ b.double().t()
+outs = [ops.gemm(a, b, pair=True) for _ in range(200)]
+assert torch.allclose(outs[0].double(), ref, rtol=2.0 ** -8, atol=K / 16 * 2.0 ** -23 * 6 * K ** 0.5)     # as above
+assert all(torch.equal(o, outs[0]) for o in outs)
+_lib.assert_healthy()
+""" % ((M, N, K),)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, HG_GEMM_SPLIT_TAIL="1"), capture_output=True, text=True,
+                         timeout=300, cwd=root)
+    assert run.returncode == 0, run.stderr[-2000:]

@@ -32,6 +32,16 @@ def test_shared_tiles_wait_for_no_other_pair():
     assert "split_token" in body and not re.findall(r"\bwhile\b|ld_acquire|__nanosleep", body)
 
 
+def test_parts_of_shared_tiles_are_dealt_in_the_blocks_of_the_stores():
+    """A warp that adds parts has counted the arrivals of the warps of its own number alone: both deals have one block size."""
+    text = re.sub(r"//.*", "", (build.CSRC / "sm100" / "gemm2_core.cuh").read_text())
+    store = text.split("void store_tile_tma(", 1)[1].split("\n}\n", 1)[0]
+    parts = text.split("void epilogue2(", 1)[1].split("split_arrive(", 1)[0]
+    assert "kBlock = block_columns(true," in store and "cols = block_columns(p.c_tma != 0, p.out_mode)" in parts
+    assert "c = w.h * kBlock;" in store and "c += w.H * kBlock" in store
+    assert "c0 = share.h * cols;" in parts and "c0 += H * cols" in parts
+
+
 def test_nothing_throws_at_the_entry_points():
     """They are called from C: std::random_device raises where the system has no source of entropy."""
     for path in (build.CSRC / "sm100").glob("*.cu*"):
