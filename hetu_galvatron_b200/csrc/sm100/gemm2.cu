@@ -135,12 +135,15 @@ struct RowSegments {
 
 // The same products with A and B in each other's place: a tile is 256 columns of C (rows of the weight) by up to 256 rows of a
 // segment, which is cut into as few equal tiles as it takes, of a multiple of 64 rows each.  Tiles of 256 rows of C by 256
-// columns were one in eight padding at segments of about 1024 ragged rows.  The tiles of one piece of the weight are neighbours: it
-// is read from HBM once.
+// columns were one in eight padding at segments of about 1024 ragged rows.  Up to kGroupN tiles along the rows are walked
+// together, piece of the weight by piece, so that both operands are reused out of L2: with all of a segment's tiles together, more
+// rows than L2 holds came from HBM again for every few pieces (sustained, us, all / 8 / 4 together: 16384 rows, 28672 columns, K = 4096
+// 3520 / 2855 / 2918; 8192 rows, 4096 columns, K = 14336 786 / 734 / 729; 8 x (4096, 28672, 4096) 5853 / 5979 / 6123).
 struct TurnedSegments {
   const int* row_start;
   int G, tiles_m, num_kb, w_group_rows, max_rows;
   int* status;
+  static constexpr int kGroupN = 8;
   static constexpr bool kTurned = true;
   template <typename F>
   __device__ __forceinline__ void walk(int pair, int pairs, F&& fn) const {
@@ -152,7 +155,9 @@ struct TurnedSegments {
       const int pieces = (rows + BN - 1) / BN, bn = ((rows + pieces - 1) / pieces + 63) / 64 * 64;
       const int tn = (rows + bn - 1) / bn, cnt = tn * tiles_m;
       for (int t = (pair - counter % pairs + pairs) % pairs; t < cnt; t += pairs) {
-        GroupedTile w{t / tn * CM, r1, r0 + t % tn * bn, 0, g * w_group_rows, num_kb, 0, 0, bn};
+        const int first = t / (kGroupN * tiles_m) * kGroupN, gsize = min(kGroupN, tn - first);
+        const int r = t - first * tiles_m;
+        GroupedTile w{r / gsize * CM, r1, r0 + (first + r % gsize) * bn, 0, g * w_group_rows, num_kb, 0, 0, bn};
         if (!fn(w)) return;
       }
       counter += cnt;

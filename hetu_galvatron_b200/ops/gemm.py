@@ -80,7 +80,8 @@ def _use_grouped_turned(out: torch.Tensor, N: int, K: int) -> bool:
     ``TurnedSegments`` in csrc/sm100/gemm2.cu), which it does wherever it is called and the results can be stored that way.  Ragged
     groups, us, one CTA / turned pair: 8 x (1024 rows, 28672 columns, K = 4096) 1667 / 1589, 512 rows 974 / 920, 128 rows 430 / 374,
     64 rows 350 / 340, 32 rows 344 / 325; 8 x (128, 4096, 14336) 235 / 189, 64 rows 170 / 172; 64 x (128, 2816, 2048) 185 / 176; 64 x
-    (512, 2048, 1408) 230 / 221; 8 x (300, 4096, 1024) 31.1 / 30.8."""
+    (512, 2048, 1408) 230 / 221; 8 x (300, 4096, 1024) 31.1 / 30.8; 16384 rows of one group, 28672 columns, K = 4096 3927 / 2855, as the
+    pair kernel without turning."""
     return (_use_pair(256, N, None) and K >= 1280 and N % 2 == 0 and out.stride(0) % 2 == 0 and out.data_ptr() % 4 == 0)
 
 

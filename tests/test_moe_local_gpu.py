@@ -255,3 +255,22 @@ def test_grouped_gemm_along_the_rows(seg, N, K, b_mn):
     out[first:starts[-1]] = 3.0
     assert (whole == 3.0).all()
     _lib.assert_healthy()
+
+
+# more tiles along a group's rows than are walked together: one more, two groups of them and a last one of three; columns that end
+# inside a tile, so that tiles whose order was wrong would be missing or done twice
+@pytest.mark.parametrize("seg", [[2049, 70], [64, 4864, 0, 300]])
+@pytest.mark.parametrize("N,K,b_mn", [(520, 1280, False), (768, 1344, True)])
+def test_grouped_gemm_of_many_tiles_along_the_rows(seg, N, K, b_mn):
+    from hetu_galvatron_b200 import ops
+
+    g = torch.Generator(device=DEV).manual_seed(N + sum(seg))
+    starts = [sum(seg[:i]) for i in range(len(seg) + 1)]
+    a = torch.randn(starts[-1], K, device=DEV, generator=g).to(torch.bfloat16)
+    b = torch.randn(len(seg), *((K, N) if b_mn else (N, K)), device=DEV, generator=g).to(torch.bfloat16)
+    out = torch.full((starts[-1], N), float("nan"), device=DEV, dtype=torch.bfloat16)
+    ops.grouped_gemm(a, b, torch.tensor(starts, device=DEV, dtype=torch.int32), b_mn=b_mn, out=out)
+    for i in range(len(seg)):
+        ref = a[starts[i]:starts[i + 1]].double() @ (b[i].double() if b_mn else b[i].double().t())
+        assert torch.allclose(out[starts[i]:starts[i + 1]].double(), ref, rtol=2.0 ** -8, atol=1e-4 * K ** 0.5)   # as above
+    _lib.assert_healthy()
