@@ -52,7 +52,7 @@ struct Kernels {
   int (*add)(V, V, void*, long long, void*);
   int (*rope)(void*, V, int, int, int, int, int, V, int, V, V, int, int, void*);
   int (*flash_fwd)(A, A, A, A, void*, int, int, int, int, int, int, int, int, int, float, void*);
-  long long (*flash_bwd_scratch)(int, int, int, int, int, int, int, int, int);
+  int (*flash_bwd_tiles_pay)(int, int, int, int, int, int, int, int, int);
   long long (*flash_bwd_scratch_of)(int, int, int, int, int, int, int, int, int, int);
   int (*flash_bwd)(A, A, A, A, A, V, void*, long long, A, A, A, int, int, int, int, int, int, int, int, int, float, int*, void*);
   long long (*decoder_step_scratch)(const HgDecoderStep*);
@@ -390,12 +390,17 @@ struct FlashPacked : public Function<FlashPacked> {
     const Packed l = layout(ctx);
     const Tensor dout = grads[0].contiguous();
     Tensor dqkv = at::empty_like(qkv);
+    auto scratch = [&](int tiles) {
+      return empty({K.flash_bwd_scratch_of(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0, tiles)}, at::kFloat, qkv);
+    };
     Tensor ws;
-    try {
-      ws = empty({K.flash_bwd_scratch(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0)}, at::kFloat, qkv);
-    } catch (const c10::OutOfMemoryError&) {           // no room for dS: the kernels do without
-      ws = empty({K.flash_bwd_scratch_of(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0, 0)}, at::kFloat, qkv);
+    if (K.flash_bwd_tiles_pay(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0)) {
+      try {
+        ws = scratch(1);
+      } catch (const c10::OutOfMemoryError&) {         // no room for dS: the kernels do without
+      }
     }
+    if (!ws.defined()) ws = scratch(0);
     int kernels = 0;
     const HgAttnTensor q = l.q(qkv.data_ptr()), k = l.k(qkv.data_ptr()), v = l.v(qkv.data_ptr()), o = l.o(out.data_ptr()),
                        d = l.o(dout.data_ptr()), dq = l.q(dqkv.data_ptr()), dk = l.k(dqkv.data_ptr()), dv = l.v(dqkv.data_ptr());
@@ -702,7 +707,7 @@ void bind(const py::dict& fn, bool half, int pair_mode, py::object kernel_error)
   at("hg_colsum_parts", K.colsum_parts); at("hg_colsum", K.colsum);
   at("hg_norm_fwd", K.norm_fwd); at("hg_norm_bwd", K.norm_bwd);
   at("hg_glu_fwd", K.glu_fwd); at("hg_glu_bwd", K.glu_bwd); at("hg_add_bf16", K.add); at("hg_rope", K.rope);
-  at("hg_flash_fwd", K.flash_fwd); at("hg_flash_bwd_scratch", K.flash_bwd_scratch); at("hg_flash_bwd_scratch_of", K.flash_bwd_scratch_of); at("hg_flash_bwd_ws", K.flash_bwd);
+  at("hg_flash_fwd", K.flash_fwd); at("hg_flash_bwd_tiles_pay", K.flash_bwd_tiles_pay); at("hg_flash_bwd_scratch_of", K.flash_bwd_scratch_of); at("hg_flash_bwd_ws", K.flash_bwd);
   at("hg_decoder_step_scratch", K.decoder_step_scratch); at("hg_decoder_step", K.decoder_step);
   g_lp = half ? at::kHalf : at::kBFloat16;
   g_pair_mode = pair_mode;

@@ -2513,10 +2513,24 @@ DsCut ds_cut(const BwdParams& p, int Skv, int nkv) {
   c.ng = groups < nkv ? int(groups) : nkv;
   c.nb = groups < nkv ? 1 : groups / nkv < p.B ? int(groups / nkv) : p.B;
   if (p.chunk > 0 && (c.ng < nkv || c.nb < p.B)) return {0, 0, 0};     // shared key blocks are few: they are launched at once
-  const int times = (nkv + c.ng - 1) / c.ng;
-  c.ng = (nkv + times - 1) / times;                                     // launches of about the same size
+  auto even = [](int n, int most) {                                     // launches of about the same size
+    const int times = (n + most - 1) / most;
+    return (n + times - 1) / times;
+  };
+  c.ng = even(nkv, c.ng);
+  c.nb = even(p.B, c.nb);
   c.bytes = group * c.ng * c.nb;
   return c;
+}
+// Whether storing dS pays.  In one launch it does.  Several end one by one, with fewer and fewer CTAs at work, which costs more than
+// dS saves unless the smallest has five key blocks per SM, and with head dim 64 whatever it has.  Whole backward, us, dS stored / S and
+// dP again: head dim 128, 8192 tokens, 32 heads (launches of 1024 key blocks) 1814 / 1935, 40 heads (1280) 2210 / 2378, 2 x 8192, 32 heads
+// (1024) 3590 / 3730; 16384, 32 heads (640) 7060 / 7000; 8192, 32 heads on 8 (256) 1980 / 1955, 28 on 4 (128) 2165 / 1815; 16384, 32 on 8
+// (128) 9705 / 7000; head dim 64, 2 x 8192, 25 heads (768) 2116 / 1942, 16384 4010 / 3731.
+bool ds_pays(const DsCut& c, const BwdParams& p, int Skv, int nkv, int hd) {
+  if (c.bytes == 0 || (c.ng == nkv && c.nb == p.B)) return c.bytes > 0;
+  const int last = c.ng < nkv ? (nkv - 1) % c.ng + 1 : ((p.B - 1) % c.nb + 1) * nkv;
+  return hd == 128 && (long long)((Skv + 127) / 128) * last >= 5 * kSmCount;
 }
 // The scratch of a backward, in floats: row sums of dO * O, parts of dK and dV, tiles of dS^T.
 struct BwdScratch {
@@ -2576,17 +2590,27 @@ int hg_attn_set_dkv_variant(int v) {
   return old;
 }
 
-// Floats of scratch that hg_flash_bwd_ws asks for: the row sums of dO * O, [B, nheads, Sq], where key blocks are shared the parts
+static BwdParams bwd_sizes(int Sq, int Skv, int B, int nheads, int nkv, int causal, int q_pos0, int k_pos0) {
+  BwdParams p{};
+  p.Sq = Sq; p.Skv = Skv; p.B = B; p.nheads = nheads; p.qpg = nheads / nkv; p.causal = causal; p.q_pos0 = q_pos0; p.k_pos0 = k_pos0;
+  return p;
+}
+
+// Floats of scratch that hg_flash_bwd_ws can use: the row sums of dO * O, [B, nheads, Sq], where key blocks are shared the parts
 // of dK and dV, and, if `tiles`, dS^T of up to kDsMost bytes.
 long long hg_flash_bwd_scratch_of(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0, int tiles) {
   if (Sq <= 0 || Skv <= 0 || B <= 0 || nheads <= 0 || nkv <= 0) return 0;
-  BwdParams p{};
-  p.Sq = Sq; p.Skv = Skv; p.B = B; p.nheads = nheads; p.qpg = nheads / nkv; p.causal = causal; p.q_pos0 = q_pos0; p.k_pos0 = k_pos0;
-  const BwdScratch w = bwd_scratch(p, Skv, nkv, hd);
+  const BwdScratch w = bwd_scratch(bwd_sizes(Sq, Skv, B, nheads, nkv, causal, q_pos0, k_pos0), Skv, nkv, hd);
   return w.sums + w.parts + (tiles ? w.ds : 0);
 }
 long long hg_flash_bwd_scratch(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
   return hg_flash_bwd_scratch_of(Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0, 1);
+}
+// Whether it is worth giving hg_flash_bwd_ws the scratch for dS.
+int hg_flash_bwd_tiles_pay(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
+  if (Sq <= 0 || Skv <= 0 || B <= 0 || nheads <= 0 || nkv <= 0) return 0;
+  const BwdParams p = bwd_sizes(Sq, Skv, B, nheads, nkv, causal, q_pos0, k_pos0);
+  return ds_pays(bwd_scratch(p, Skv, nkv, hd).cut, p, Skv, nkv, hd);
 }
 
 // ws: scratch of ws_floats fp32 values, 16-byte aligned, at least [B, nheads, Sq] (filled here with rowsum(dO*O)).  With less

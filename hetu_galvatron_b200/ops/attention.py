@@ -51,13 +51,15 @@ def attention_reference(q, k, v, causal=True, scale=None, q_pos0=0, k_pos0=0, dr
 
 
 def _backward_scratch(lib, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, device) -> torch.Tensor:
-    """fp32 scratch of the backward kernels: row sums of dO * O, where key blocks are shared between CTAs their parts, and dS,
-    without which, should there be no room for it, dQ takes longer."""
+    """fp32 scratch of the backward kernels: row sums of dO * O, where key blocks are shared between CTAs their parts, and, where
+    storing it pays, dS, without which, should there be no room for it, dQ takes longer."""
     args = (S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0)
-    try:
-        return torch.empty(lib.hg_flash_bwd_scratch(*args), dtype=torch.float32, device=device)
-    except torch.cuda.OutOfMemoryError:
-        return torch.empty(lib.hg_flash_bwd_scratch_of(*args, 0), dtype=torch.float32, device=device)
+    if lib.hg_flash_bwd_tiles_pay(*args):
+        try:
+            return torch.empty(lib.hg_flash_bwd_scratch(*args), dtype=torch.float32, device=device)
+        except torch.cuda.OutOfMemoryError:
+            pass
+    return torch.empty(lib.hg_flash_bwd_scratch_of(*args, 0), dtype=torch.float32, device=device)
 
 
 class _FlashPacked(torch.autograd.Function):

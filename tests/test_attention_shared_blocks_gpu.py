@@ -85,3 +85,31 @@ def test_dq_from_stored_ds(Sq, Skv, B, nh, ng, hd, causal, q0, k0):
     assert torch.equal(grads[0], one[0])
     assert all((a.double() - b.double()).norm() <= 1e-3 * b.double().norm() for a, b in zip(grads[1:], one[1:]))
     _lib.assert_healthy()
+
+
+# scratch for everything, one float less, for shared key blocks alone, one float less, for the row sums alone; launches over some of the
+# heads and of the sequences, which the callers of this package do not ask for; key blocks that are shared
+@pytest.mark.parametrize("Sq,Skv,B,nh,ng,hd,causal", [(8192, 8192, 1, 32, 32, 64, True), (4096, 4096, 3, 16, 8, 64, False),
+                                                      (1531, 1531, 1, 7, 1, 128, True), (640, 640, 1, 6, 2, 64, False)])
+def test_backward_with_any_scratch(Sq, Skv, B, nh, ng, hd, causal):
+    lib, sizes = _lib.load(), (Sq, Skv, B, nh, ng, hd, int(causal), 0, 0)
+    g = torch.Generator(device=DEV).manual_seed(Sq + hd)
+    q, dout = (torch.randn(Sq, B, nh, hd, device=DEV, generator=g).to(torch.bfloat16) for _ in "qd")
+    k, v = (torch.randn(Skv, B, ng, hd, device=DEV, generator=g).to(torch.bfloat16) for _ in "kv")
+    out, lse = ops.flash_attention(q, k, v, causal=causal, return_lse=True)
+    most, parts, sums = lib.hg_flash_bwd_scratch(*sizes), lib.hg_flash_bwd_scratch_of(*sizes, 0), B * nh * Sq
+    results = []
+    for floats in (most, most - 1, parts, max(parts - 1, sums), sums):
+        got, ws = [torch.full_like(t, float("nan")) for t in (q, k, v)], torch.full((floats,), float("nan"), device=DEV)
+        heads = lambda t: ctypes.byref(_desc(t, t.stride(0), t.stride(1), nh, nh // ng, 1, 0))
+        kv = lambda t: ctypes.byref(_desc(t, t.stride(0), t.stride(1), ng, 1, 0, 0))
+        assert lib.hg_flash_bwd_ws(heads(q), kv(k), kv(v), heads(out), heads(dout), lse.data_ptr(), ws.data_ptr(), floats, heads(got[0]),
+                                   kv(got[1]), kv(got[2]), *sizes[:6], int(causal), 0, 0, hd ** -0.5, None, _lib.stream()) == 0
+        results.append(got)
+    for got in results:
+        assert torch.equal(got[0], results[0][0])                         # dQ: the same bits, stored dS or not
+        assert rel_err(got[1], results[0][1]) < 1e-3 and rel_err(got[2], results[0][2]) < 1e-3
+    for i in (1, 2):                                                      # dK and dV: as long as the same CTAs share
+        assert torch.equal(results[0][i], results[1][i]) and torch.equal(results[0][i], results[2][i])
+        assert torch.equal(results[3][i], results[4][i])
+    _lib.assert_healthy()
