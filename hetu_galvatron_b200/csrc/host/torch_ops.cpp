@@ -53,6 +53,8 @@ struct Kernels {
   int (*rope)(void*, V, int, int, int, int, int, V, int, V, V, int, int, void*);
   int (*flash_fwd)(A, A, A, A, void*, int, int, int, int, int, int, int, int, int, float, void*);
   int (*flash_bwd_tiles_pay)(int, int, int, int, int, int, int, int, int);
+  int (*flash_bwd_has_room)(int);
+  int (*flash_bwd_no_room)(int);
   long long (*flash_bwd_scratch_of)(int, int, int, int, int, int, int, int, int, int);
   int (*flash_bwd)(A, A, A, A, A, V, void*, long long, A, A, A, int, int, int, int, int, int, int, int, int, float, int*, void*);
   long long (*decoder_step_scratch)(const HgDecoderStep*);
@@ -394,10 +396,11 @@ struct FlashPacked : public Function<FlashPacked> {
       return empty({K.flash_bwd_scratch_of(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0, tiles)}, at::kFloat, qkv);
     };
     Tensor ws;
-    if (K.flash_bwd_tiles_pay(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0)) {
+    if (K.flash_bwd_tiles_pay(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0) && K.flash_bwd_has_room(qkv.get_device())) {
       try {
         ws = scratch(1);
       } catch (const c10::OutOfMemoryError&) {         // no room for dS: the kernels do without
+        K.flash_bwd_no_room(qkv.get_device());
       }
     }
     if (!ws.defined()) ws = scratch(0);
@@ -707,7 +710,7 @@ void bind(const py::dict& fn, bool half, int pair_mode, py::object kernel_error)
   at("hg_colsum_parts", K.colsum_parts); at("hg_colsum", K.colsum);
   at("hg_norm_fwd", K.norm_fwd); at("hg_norm_bwd", K.norm_bwd);
   at("hg_glu_fwd", K.glu_fwd); at("hg_glu_bwd", K.glu_bwd); at("hg_add_bf16", K.add); at("hg_rope", K.rope);
-  at("hg_flash_fwd", K.flash_fwd); at("hg_flash_bwd_tiles_pay", K.flash_bwd_tiles_pay); at("hg_flash_bwd_scratch_of", K.flash_bwd_scratch_of); at("hg_flash_bwd_ws", K.flash_bwd);
+  at("hg_flash_fwd", K.flash_fwd); at("hg_flash_bwd_tiles_pay", K.flash_bwd_tiles_pay); at("hg_flash_bwd_has_room", K.flash_bwd_has_room); at("hg_flash_bwd_no_room", K.flash_bwd_no_room); at("hg_flash_bwd_scratch_of", K.flash_bwd_scratch_of); at("hg_flash_bwd_ws", K.flash_bwd);
   at("hg_decoder_step_scratch", K.decoder_step_scratch); at("hg_decoder_step", K.decoder_step);
   g_lp = half ? at::kHalf : at::kBFloat16;
   g_pair_mode = pair_mode;

@@ -10,6 +10,7 @@
 //
 // Replaces flash_attn_varlen_func / _flash_attn_forward / _flash_attn_backward as called from
 // galvatron/core/runtime/transformer/attention_impl.py:55-111,587-616,696-727.
+#include <atomic>
 #include <type_traits>
 
 #include "entry_points.h"
@@ -2611,6 +2612,20 @@ int hg_flash_bwd_tiles_pay(int Sq, int Skv, int B, int nheads, int nkv, int hd, 
   if (Sq <= 0 || Skv <= 0 || B <= 0 || nheads <= 0 || nkv <= 0) return 0;
   const BwdParams p = bwd_sizes(Sq, Skv, B, nheads, nkv, causal, q_pos0, k_pos0);
   return ds_pays(bwd_scratch(p, Skv, nkv, hd).cut, p, Skv, nkv, hd);
+}
+
+// Where the caller's allocator had no room for dS, the next kNoRoomCalls backwards of that device do not ask it again: a caching
+// allocator gives all that it holds back to the device before it says so, and every buffer then has to be had anew.
+static std::atomic<int> g_no_room[64];
+constexpr int kNoRoomCalls = 256;
+int hg_flash_bwd_no_room(int device) {
+  g_no_room[unsigned(device) % 64].store(kNoRoomCalls, std::memory_order_relaxed);
+  return 0;
+}
+// Whether the allocator is to be asked; counts a call that is not.
+int hg_flash_bwd_has_room(int device) {
+  std::atomic<int>& left = g_no_room[unsigned(device) % 64];
+  return left.load(std::memory_order_relaxed) <= 0 || left.fetch_sub(1, std::memory_order_relaxed) <= 0;
 }
 
 // ws: scratch of ws_floats fp32 values, 16-byte aligned, at least [B, nheads, Sq] (filled here with rowsum(dO*O)).  With less

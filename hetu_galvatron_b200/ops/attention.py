@@ -54,11 +54,11 @@ def _backward_scratch(lib, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, device
     """fp32 scratch of the backward kernels: row sums of dO * O, where key blocks are shared between CTAs their parts, and, where
     storing it pays, dS, without which, should there be no room for it, dQ takes longer."""
     args = (S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0)
-    if lib.hg_flash_bwd_tiles_pay(*args):
+    if lib.hg_flash_bwd_tiles_pay(*args) and lib.hg_flash_bwd_has_room(device.index):
         try:
             return torch.empty(lib.hg_flash_bwd_scratch(*args), dtype=torch.float32, device=device)
         except torch.cuda.OutOfMemoryError:
-            pass
+            lib.hg_flash_bwd_no_room(device.index)
     return torch.empty(lib.hg_flash_bwd_scratch_of(*args, 0), dtype=torch.float32, device=device)
 
 

@@ -1,5 +1,8 @@
 """dK and dV of key blocks that several CTAs share, against one CTA per key block and 64-bit arithmetic."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -113,3 +116,39 @@ def test_backward_with_any_scratch(Sq, Skv, B, nh, ng, hd, causal):
         assert torch.equal(results[0][i], results[1][i]) and torch.equal(results[0][i], results[2][i])
         assert torch.equal(results[3][i], results[4][i])
     _lib.assert_healthy()
+
+
+# a process that may have less memory than dS takes: one failed allocation, not one a layer, and the same gradients; by the C++ nodes and
+# by the function of the parallel paths
+@pytest.mark.parametrize("route", ["node", "function"])
+def test_backward_without_room_for_ds(route):
+    code = """
+import torch
+from hetu_galvatron_b200 import ops
+from hetu_galvatron_b200.ops import _lib
+S, nh, hd, route = 2048, 32, 128, %r
+g = torch.Generator(device="cuda").manual_seed(1)
+qkv = torch.randn(S, 3 * nh * hd, device="cuda", generator=g).to(torch.bfloat16).requires_grad_()
+d = torch.randn(S, nh * hd, device="cuda", generator=g).to(torch.bfloat16)
+if route == "node":
+    assert _lib.load() and _lib.NATIVE is not None
+    out = ops.flash_attention_packed(qkv, S, 1, nh, nh, hd, causal=True)
+    run = lambda: torch.autograd.grad(out, qkv, d, retain_graph=True)
+else:
+    q, k, v = (t.contiguous() for t in qkv.detach().view(S, 1, nh, 3, hd).unbind(3))
+    out, lse = ops.flash_attention(q, k, v, causal=True, return_lse=True)
+    run = lambda: ops.flash_backward(q, k, v, out, d.view(S, 1, nh, hd), lse, True, hd ** -0.5)
+want = [t.cpu() for t in run()]
+ooms = lambda: torch.cuda.memory_stats()["num_ooms"]
+assert ooms() == 0
+torch.cuda.empty_cache()
+total = torch.cuda.get_device_properties(0).total_memory
+torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 120e6) / total)      # dS: 142 MB
+for _ in range(3):
+    assert all(torch.equal(a.cpu(), b) for a, b in zip(run(), want))
+assert ooms() == 1, ooms()
+_lib.assert_healthy()
+""" % (route,)
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300, cwd=root)
+    assert run.returncode == 0, run.stderr[-2000:]
