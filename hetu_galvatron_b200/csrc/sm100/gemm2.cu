@@ -374,8 +374,10 @@ constexpr int kStore = 1400, kStore16 = 10, kStore32 = 21, kStoreTurned = 34, kT
 // A shared tile, per column: the parts' way to L2 and the arrivals, and each part that is added (200 x 3584, K = 18944: 256
 // columns by five 52 us, 192 by three 44, not shared 89).
 constexpr int kSplitCost = 48, kPartCost = 20;
-// A plan other than whole tiles of 256 columns has to promise a gain of one part in this many.
-constexpr int kWorth = 64;
+// A plan other than whole tiles of 256 columns has to promise a gain of one part in this many: turned tiles, which never lost, and
+// narrower ones that are not turned, whose small promises do not hold over several waves (of 2 to 6 % in the cost, us, whole / narrower:
+// 12288 x 1600, K = 808 30.8 / 34.0, fp32 K = 1168 49.5 / 56.0, fp32 15360 x 3584, K = 72 46.8 / 48.9).
+constexpr int kWorth = 64, kWorthNarrow = 20;
 
 long long plan_cost(long long tiles, int num_kb, int pairs, int bn, int store, int s) {
   const long long main = num_kb * (kBlockCost + bn), epi = kStore + bn * store, wave = main > epi ? main : epi;
@@ -397,7 +399,7 @@ int split_most(int tail, int num_kb, int pairs) {
 TilePlan cheapest_plan(int M, int N, int K, bool wide, bool may_turn, int max_pairs) {
   const int num_kb = (K + BK - 1) / BK;
   TilePlan best{BN, 0, 0, 0};
-  long long best_cost = 0;
+  long long best_cost = 0, whole_cost = 0;              // whole: tiles of 256 columns, not turned, which come first
   for (int turned = 0; turned <= (may_turn ? 1 : 0); ++turned) {
     const int rows = turned ? N : M, cols = turned ? M : N;
     const int step = turned || wide ? 32 : 64;           // 16-bit blocks leave 64 columns at a time
@@ -413,7 +415,9 @@ TilePlan cheapest_plan(int M, int N, int K, bool wide, bool may_turn, int max_pa
         if (s > 2 && cost > before && split_mode() < 0) break;      // more slices only cost more from here on
         before = cost;
         const bool first = best_cost == 0, whole = bn == BN && !turned;
+        if (!turned && !whole && cost * kWorthNarrow >= whole_cost * (kWorthNarrow - 1)) continue;
         if (first || (whole ? cost < best_cost : cost * kWorth < best_cost * (kWorth - 1))) {
+          if (whole) whole_cost = cost;
           best = TilePlan{bn, turned, s, tail};
           best_cost = cost;
         }

@@ -1,10 +1,12 @@
 """Which kernel a product goes to, on both sides of each line of the rules."""
+import ctypes
 import re
 
 import pytest
 
 from hetu_galvatron_b200.csrc import build
-from hetu_galvatron_b200.ops.gemm import OUT_BF16, _use_grouped_pair, _use_skinny
+from hetu_galvatron_b200.ops import _lib
+from hetu_galvatron_b200.ops.gemm import OUT_BF16, OUT_F32, _use_grouped_pair, _use_skinny
 
 
 # the last two: as many columns as the few-row kernel's grid has tiles for, and one more
@@ -46,3 +48,14 @@ def test_nothing_throws_at_the_entry_points():
     """They are called from C: std::random_device raises where the system has no source of entropy."""
     for path in (build.CSRC / "sm100").glob("*.cu*"):
         assert not re.search(r"random_device|\bthrow\b|\.at\(", re.sub(r"//.*", "", path.read_text())), path.name
+
+
+# 74 pairs.  Narrower tiles that promise more than a twentieth, less, and turned ones that promise less; a last wave that is shared
+@pytest.mark.parametrize("M,N,K,mode,bn,turned,shared", [
+    (1531, 3584, 3584, OUT_BF16, 192, 0, False), (4608, 2304, 1248, OUT_BF16, 192, 0, False), (12288, 1600, 808, OUT_BF16, 256, 0, False),
+    (12288, 1600, 1168, OUT_F32, 256, 0, False), (11008, 2304, 784, OUT_F32, 256, 0, False), (6400, 1600, 4160, OUT_F32, 224, 0, False),
+    (345, 32000, 1600, OUT_BF16, 192, 1, False), (320, 4096, 22016, OUT_BF16, 160, 1, True), (200, 3584, 8192, OUT_F32, 160, 0, True)])
+def test_plans_of_products(M, N, K, mode, bn, turned, shared):
+    plan = (ctypes.c_int * 5)()
+    _lib.load().hg_gemm2_plan(M, N, K, mode, 1, 74, plan)
+    assert plan[:2] == [bn, turned] and (plan[2] > 1) is shared
