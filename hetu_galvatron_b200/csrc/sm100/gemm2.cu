@@ -457,10 +457,11 @@ unsigned long long split_token() {
 // Threads of a CTA: with two epilogue warps per 32 rows where a tile's way out counts beside its products, which take `main`
 // cycles (see plan_cost), with one elsewhere: on large products, which the power limit bounds, the four more warps cost
 // 1 to 3 % (sustained, us, one and two: 4096 x 32000, K = 4096 827 -> 850 us; 22016 x 4096, K = 8192, added to C 1217 -> 1258; 28672 x 4096, fp32, K = 1024 236 ->
-// 238, K = 512 164 -> 157; added to C, K = 2048 460 -> 453).
-static int threads_for(int out_mode, long long main) {
+// 238, K = 512 164 -> 157; added to C, K = 2048 460 -> 453).  16-bit results of two operands that are M- and N-major pay it sooner
+// (4608 x 37888, K = 760 241 -> 257; 13824 x 27648, K = 800 545 -> 589; K = 520 and 640 still gain 3 to 4 %).
+static int threads_for(int out_mode, long long main, bool mn) {
   const bool adds = out_mode == kOutF32Acc || out_mode == kOutBf16Acc;
-  return main < (adds ? 20000 : 8000) ? kThreads2 : 64 + 32 * EPI_WARPS;
+  return main < (adds ? 20000 : mn && out_mode == kOutBf16 ? 5300 : 8000) ? kThreads2 : 64 + 32 * EPI_WARPS;
 }
 
 // Launch attributes of a kernel of CTA pairs, and how many pairs of it the device holds at once (-2: none).
@@ -516,7 +517,7 @@ static int launch2(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorM
   auto k = gemm2_bf16_kernel<A_MN, B_MN>;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  const int threads = threads_for(p.out_mode, (long long)((p.K + BK - 1) / BK) * (kBlockCost + p.bn));
+  const int threads = threads_for(p.out_mode, (long long)((p.K + BK - 1) / BK) * (kBlockCost + p.bn), A_MN && B_MN);
   if (int rc = pair_config(k, &cfg, attr, &co_resident, hg_host::launch_overlaps(), st, threads)) return rc;
   int pairs = want_pairs < co_resident ? want_pairs : co_resident;
   p.split_s = 0;
@@ -612,10 +613,11 @@ int hg_gemm2_bf16(const void* A, const void* B, void* C, const void* bias, int M
 }
 
 // How hg_gemm2_bf16 cuts a product for `pairs` pairs: columns of a tile, whether A and B change places (`may_turn`: if C allows it),
-// pairs per tile of the last wave (below 2: one), its tiles, epilogue warps per 32 rows.  Needs no device.
-int hg_gemm2_plan(int M, int N, int K, int out_mode, int may_turn, int pairs, int* plan) {
+// pairs per tile of the last wave (below 2: one), its tiles, epilogue warps per 32 rows (`mn`: of M- and N-major operands).
+// Needs no device.
+int hg_gemm2_plan(int M, int N, int K, int out_mode, int may_turn, int mn, int pairs, int* plan) {
   const TilePlan t = tile_plan(M, N, K, out_mode, may_turn && out_mode == kOutBf16, pairs);
-  const int threads = threads_for(out_mode, (long long)((K + BK - 1) / BK) * (kBlockCost + t.bn));
+  const int threads = threads_for(out_mode, (long long)((K + BK - 1) / BK) * (kBlockCost + t.bn), mn);
   const int of_plan[5] = {t.bn, t.turned, t.s, t.tail, (threads - 64) / (32 * EPI_WARPS)};
   for (int i = 0; i < 5; ++i) plan[i] = of_plan[i];
   return 0;
@@ -645,7 +647,7 @@ int hg_grouped_gemm2_bf16(const void* A, const void* B, void* C, const void* row
   Params p{};
   p.K = K; p.ldc = ldc; p.C = C; p.out_mode = out_mode; p.bn = BN; p.status = hg_host::status_ptr();
   const int* starts = reinterpret_cast<const int*>(row_start);
-  const int num_kb = (K + BK - 1) / BK, threads = threads_for(out_mode, (long long)num_kb * (kBlockCost + BN));
+  const int num_kb = (K + BK - 1) / BK, threads = threads_for(out_mode, (long long)num_kb * (kBlockCost + BN), false);
   if (turns(C, N, ldc, out_mode)) {
     p.M = N; p.N = max_rows;
     if (b_mn) rc = hg_host::make_tmap_2d_bf16(&ta, B, uint64_t(G) * K, N, ldb, 64, 64);
@@ -683,7 +685,7 @@ int hg_grouped_wgrad2_bf16(const void* dy, const void* x, void* out, const void*
   if (max_ctas > 1 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
   CUtensorMap tc;
   if ((rc = store_map(&tc, ta, p, uint64_t(G) * N))) return rc;
-  const int threads = threads_for(out_mode, ((long long)rows / G + BK - 1) / BK * (kBlockCost + BN));    // a group's, on average
+  const int threads = threads_for(out_mode, ((long long)rows / G + BK - 1) / BK * (kBlockCost + BN), true);    // a group's, on average
   return launch_grouped2<true, true>(ta, tb, tc, p, t, pairs, threads, reinterpret_cast<cudaStream_t>(stream));
 }
 

@@ -77,7 +77,7 @@ _SIGNATURES = {
     "hg_gemm_bf16": [c_void_p] * 4 + [c_int] * 10 + [c_void_p],
     "hg_gemm2_bf16": [c_void_p] * 4 + [c_int] * 10 + [c_void_p, c_ll, c_void_p],
     "hg_gemm2_scratch": [c_int] * 3,
-    "hg_gemm2_plan": [c_int] * 6 + [ctypes.POINTER(c_int)],
+    "hg_gemm2_plan": [c_int] * 7 + [ctypes.POINTER(c_int)],
     "hg_gemm_skinny_bf16": [c_void_p] * 4 + [c_int] * 9 + [c_void_p],
     "hg_colsum_parts": [c_int, c_int],
     "hg_colsum_bf16": [c_void_p, c_ll, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p],

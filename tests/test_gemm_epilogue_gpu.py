@@ -180,7 +180,7 @@ from hetu_galvatron_b200 import ops
 from hetu_galvatron_b200.ops import _lib
 M, N, K = %r
 plan = (ctypes.c_int * 5)()
-_lib.load().hg_gemm2_plan(M, N, K, 0, 1, 74, plan)
+_lib.load().hg_gemm2_plan(M, N, K, 0, 1, 0, 74, plan)
 assert plan[0] == 64 and not plan[1] and plan[2] > 1 and plan[4] == 2, list(plan)
 g = torch.Generator(device="cuda").manual_seed(K)
 a, b = (torch.randn(n, K, device="cuda", generator=g).to(torch.bfloat16) for n in (M, N))

@@ -6,7 +6,7 @@ import pytest
 
 from hetu_galvatron_b200.csrc import build
 from hetu_galvatron_b200.ops import _lib
-from hetu_galvatron_b200.ops.gemm import OUT_BF16, OUT_F32, _use_grouped_pair, _use_skinny
+from hetu_galvatron_b200.ops.gemm import OUT_BF16, OUT_F32, OUT_F32_ACC, _use_grouped_pair, _use_skinny
 
 
 # the last two: as many columns as the few-row kernel's grid has tiles for, and one more
@@ -57,5 +57,14 @@ def test_nothing_throws_at_the_entry_points():
     (345, 32000, 1600, OUT_BF16, 192, 1, False), (320, 4096, 22016, OUT_BF16, 160, 1, True), (200, 3584, 8192, OUT_F32, 160, 0, True)])
 def test_plans_of_products(M, N, K, mode, bn, turned, shared):
     plan = (ctypes.c_int * 5)()
-    _lib.load().hg_gemm2_plan(M, N, K, mode, 1, 74, plan)
+    _lib.load().hg_gemm2_plan(M, N, K, mode, 1, 0, 74, plan)
     assert plan[:2] == [bn, turned] and (plan[2] > 1) is shared
+
+
+# K-blocks of 512 cycles in tiles of 256 columns: the last with two epilogue warps per 32 rows and the first with one
+@pytest.mark.parametrize("mode,mn,blocks", [(OUT_BF16, 0, 15), (OUT_BF16, 1, 10), (OUT_F32, 0, 15), (OUT_F32, 1, 15), (OUT_F32_ACC, 1, 39)])
+def test_rule_of_the_epilogue_warps(mode, mn, blocks):
+    for n, warps in ((blocks, 2), (blocks + 1, 1)):
+        plan = (ctypes.c_int * 5)()
+        _lib.load().hg_gemm2_plan(256 * 74, 256, 64 * n, mode, 0, mn, 74, plan)
+        assert plan[0] == 256 and plan[4] == warps
