@@ -344,8 +344,10 @@ __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids, const hg_l
 
 // The same gradient with the tokens of a row of dW brought together, for up to kSortTokens tokens: what bounds the scatter above is
 // its reductions in L2, and in text more than half of them meet a row that another token of the batch has as well.  One block sorts
-// (row, token) in shared memory, 7 us per 1024 tokens in 91 passes of a bitonic network, while the others clear dW.  A block of the second kernel then adds the tokens of kRunTokens
-// neighbouring keys in registers and leaves one row of sums per run, as plain stores where the run is all of its row's tokens.  8192 tokens x 4096 of 32000 rows, frequencies as in text, us: cleared 72 and scattered 59, 110 so; 8192 x 3584 of 152064 347, 322.
+// (row, token) in shared memory by a bitonic network (8192 keys 68 us in 91 passes) while the others clear dW.  A block of the
+// second kernel then adds the tokens of kRunTokens neighbouring keys in registers and leaves one row of sums per run, as plain stores
+// where the run is all of its row's tokens.  8192 tokens x 4096 of 32000 rows, frequencies as in text, us: cleared 72 and scattered 59,
+// 114 so; 8200 x 3584 of 152064 354, 322.
 constexpr int kSortTokens = 16384, kSortIndexBits = 14, kRunTokens = 8, kClearVecs = 8192;
 constexpr unsigned kNoRow = 0xffffffffu;
 static_assert(1 << kSortIndexBits == kSortTokens, "an index of a key");
@@ -686,15 +688,29 @@ int hg_embedding_bwd(const void* ids, const void* dout, void* dW, void* dpos, in
   return int(cudaGetLastError());
 }
 
-// Whether hg_embedding_bwd_runs takes a batch: where the sort is over before the table is cleared (7 us per 1024 tokens against
-// 7.3 TB/s); into a table that holds something, where the sort has nothing to hide behind, 8192 tokens take 85 us and 54 scattered.
+static bool runs_can(const void* dW, int tokens, int H, int rows) {
+  return tokens > 0 && tokens <= kSortTokens && H > 0 && H % 8 == 0 && rows > 0 && rows <= (int)(kNoRow >> kSortIndexBits) &&
+         (uintptr_t(dW) & 15) == 0;
+}
+// Whether it pays to bring the tokens together, for a table that holds nothing.  Into one that does, where the sort has nothing to
+// hide behind, 8192 tokens take 85 us and 54 scattered.
+// The table is cleared at 7.3 TB/s.  The sort is of the next power of two: log2 n (log2 n + 1) / 2 passes of 0.25 us and 0.06 ns a key
+// (8192 keys 68 us, 16384 131), a little longer beside the clearing.  Sums of runs instead of a scatter save about 1 ps per element
+// of the gradient; clearing in this kernel and the second one cost up to 1 us and a fortieth.  us, cleared and scattered / so: 8192 tokens
+// of 24576 rows x 4096 115 / 106, of 32000 132 / 114; 8193 of 32000 140 / 159 (not taken), of 58479 186 / 182; 4097 of 24327 86 / 91 (not
+// taken), of 39532 118 / 107; 4096 of 152064 x 3584 318 / 309, of 50304 x 1600 60 / 54, of 50304 x 768 34 / 40 (not taken); 1024 of 3072
+// x 4096 20 / 22 (not taken), of 16000 46 / 45, of 128256 288 / 290 (not taken); 256 of 8521 24 / 26 (not taken).
 int hg_embedding_bwd_runs_takes(const void* dW, int tokens, int H, int rows) {
-  return tokens >= 256 && tokens <= kSortTokens && H > 0 && H % 8 == 0 && rows > 0 && rows <= (int)(kNoRow >> kSortIndexBits) &&
-         (uintptr_t(dW) & 15) == 0 && (long long)rows * H >= 12288ll * tokens;
+  if (!runs_can(dW, tokens, H, rows)) return 0;
+  long long n = 1, log2n = 0;
+  while (n < tokens) n <<= 1, ++log2n;
+  const long long clear = (long long)rows * H / 1825, saved = (long long)tokens * H / 1024;        // ns
+  const long long sort = log2n * (log2n + 1) / 2 * (250 + n / 16);
+  return clear * 4 / 5 + saved >= sort * 9 / 10 && clear / 40 + 1000 <= saved;
 }
 // dW [rows, H] = the sums of the gradients of the tokens of rows v0 .. v0 + rows - 1.  keys: scratch of `tokens` words.
 int hg_embedding_bwd_runs(const void* ids, const void* dout, void* dW, void* keys, int tokens, int H, int v0, int rows, void* stream) {
-  if (!hg_embedding_bwd_runs_takes(dW, tokens, H, rows)) return -1;
+  if (!runs_can(dW, tokens, H, rows)) return -1;
   cudaStream_t st = (cudaStream_t)stream;
   int n = 1;
   while (n < tokens) n <<= 1;

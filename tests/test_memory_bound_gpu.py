@@ -115,3 +115,24 @@ def test_embedding_gradient(tokens, rows, H, fresh, positions):
         ref = torch.zeros(pos.shape, device="cuda", dtype=torch.float64).index_add_(0, torch.arange(tokens, device="cuda") // 2, dout.double())
         assert torch.allclose(pos.grad.double(), ref, rtol=2.0 ** -8, atol=1e-6)
     _lib.assert_healthy()
+
+
+# the kernels on their own, whatever the rule says: one token, counts around a block of eight, a power of two and the most there can be;
+# more columns than a block takes; a shard that has none of the tokens
+@pytest.mark.parametrize("tokens", [1, 7, 8, 9, 255, 256, 257, 1025, 16384])
+@pytest.mark.parametrize("rows,H", [(3, 8), (300, 2056)])
+@pytest.mark.parametrize("v0", [0, 7, 10 ** 6])
+def test_sums_of_sorted_tokens(tokens, rows, H, v0):
+    from hetu_galvatron_b200.ops import _lib
+
+    lib, g = _lib.load(), torch.Generator(device="cuda").manual_seed(tokens + H)
+    ids = torch.randint(0, rows + 12, (tokens,), device="cuda", generator=g)
+    dout = torch.randn(tokens, H, device="cuda", generator=g).to(torch.bfloat16)
+    dW, keys = torch.full((rows + 1, H), float("nan"), device="cuda"), torch.empty(tokens, dtype=torch.int32, device="cuda")
+    assert lib.hg_embedding_bwd_runs(ids.data_ptr(), dout.data_ptr(), dW.data_ptr(), keys.data_ptr(), tokens, H, v0, rows, _lib.stream()) == 0
+    want, mine = torch.zeros(rows, H, device="cuda", dtype=torch.float64), (ids >= v0) & (ids < v0 + rows)
+    want.index_add_(0, ids[mine] - v0, dout[mine].double())
+    most = int(torch.bincount(ids).max())
+    assert torch.allclose(dW[:rows].double(), want, rtol=0, atol=most * 2.0 ** -24 * (2 + 6 * most ** 0.5))      # as above
+    assert dW[rows].isnan().all()
+    _lib.assert_healthy()
