@@ -16,6 +16,7 @@
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
@@ -182,9 +183,12 @@ struct MainGrad {
   }
 };
 
-// The gradient buffer of a bias or norm bias, if this node may write it itself: a vector of `n` fp32 values, and nobody on the way
-// to the parameter who wants to see the gradient (hooks of the tensor or behind its accumulation).
+// Whether this node may write the gradient of a bias or norm bias to its buffer itself: a vector of `n` fp32 values, in a plain
+// backward() into the leaves (autograd.grad, backward(inputs=...) and a graph of the gradient get it through autograd), and nobody on
+// the way to the parameter who wants to see it (hooks of the tensor or behind its accumulation).
 bool takes_vector(const MainGrad& mg, const Tensor& p, int64_t n) {
+  const auto* asked = torch::autograd::get_current_graph_task_exec_info();
+  if (at::GradMode::is_enabled() || asked == nullptr || !asked->empty()) return false;
   if (!mg.buf.defined() || mg.buf.scalar_type() != at::kFloat || !mg.buf.is_cuda() || mg.buf.numel() != n || !mg.buf.is_contiguous())
     return false;
   if (!p.is_leaf() || !torch::autograd::impl::hooks(p).empty() || torch::autograd::impl::post_acc_grad_hooks(p) != nullptr) return false;
@@ -194,8 +198,8 @@ bool takes_vector(const MainGrad& mg, const Tensor& p, int64_t n) {
 
 struct Linear : public Function<Linear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& bias) {
-    ctx->save_for_backward(bias ? variable_list{x, w, *bias} : variable_list{x, w});
-    ctx->saved_data["bias"] = bias.has_value();
+    ctx->save_for_backward({x, w});
+    if (bias) ctx->saved_data["bias"] = *bias;      // to find its buffer; its values are not needed and may change
     Tensor y = empty({x.size(0), w.size(0)}, g_lp, x);
     gemm(x, w, y, bias ? bias->data_ptr() : nullptr, false, false, kOutLp);
     return y;
@@ -222,11 +226,12 @@ struct Linear : public Function<Linear> {
         gemm(dy, x, dw, nullptr, true, true, kOutLp);
       }
     }
-    if (ctx->saved_data["bias"].toBool() && ctx->needs_input_grad(2)) {
-      const MainGrad mg(saved[2]);
-      if (takes_vector(mg, saved[2], dy.size(1))) {
+    if (ctx->saved_data.count("bias") && ctx->needs_input_grad(2)) {
+      const Tensor b = ctx->saved_data["bias"].toTensor();
+      const MainGrad mg(b);
+      if (takes_vector(mg, b, dy.size(1))) {
         column_sums(dy, mg.buf, !mg.fresh);
-        MainGrad::written(saved[2]);
+        MainGrad::written(b);
       } else {
         db = column_sums(dy);
       }
@@ -248,10 +253,10 @@ struct Norm : public Function<Norm> {
                      y.data_ptr(), residual ? h.data_ptr() : nullptr, rstd.data_ptr(), rms ? nullptr : mean.data_ptr(),
                      int(rows), int(H), float(eps), rms, stream()), "hg_norm_fwd");
     count();
-    ctx->save_for_backward(b ? variable_list{h, w, rstd, rms ? rstd : mean, *b} : variable_list{h, w, rstd, rms ? rstd : mean});
+    ctx->save_for_backward({h, w, rstd, rms ? rstd : mean});
+    if (b) ctx->saved_data["bias"] = *b;            // as in Linear
     ctx->saved_data["rms"] = rms;
     ctx->saved_data["residual"] = residual.has_value();
-    ctx->saved_data["bias"] = b.has_value();
     ctx->set_materialize_grads(false);
     return residual ? variable_list{y, h} : variable_list{y};
   }
@@ -259,7 +264,7 @@ struct Norm : public Function<Norm> {
     const variable_list saved = ctx->get_saved_variables();
     const Tensor &h = saved[0], &w = saved[1], &rstd = saved[2], &mean = saved[3];
     const bool rms = ctx->saved_data["rms"].toBool(), residual = ctx->saved_data["residual"].toBool(),
-               bias = ctx->saved_data["bias"].toBool();
+               bias = ctx->saved_data.count("bias") != 0;
     const int64_t rows = h.size(0), H = h.size(1);
     const Tensor dy = grads[0].defined() ? grads[0].contiguous() : at::zeros_like(h);
     const Tensor dres = grads.size() > 1 && grads[1].defined() ? grads[1].contiguous() : Tensor();
@@ -271,8 +276,9 @@ struct Norm : public Function<Norm> {
     const Tensor dw = mg.buf.defined() ? mg.buf : empty({H}, at::kFloat, h);
     // The kernel's accumulate switch is shared with dw (which may add into main_grad): db goes the same way, or into zeros.
     const bool adds = mg.buf.defined() && !mg.fresh;
-    const MainGrad mg_b = bias ? MainGrad(saved[4]) : MainGrad();
-    const bool b_direct = bias && ctx->needs_input_grad(residual ? 3 : 2) && takes_vector(mg_b, saved[4], H) && !mg_b.fresh == adds;
+    const Tensor b = bias ? ctx->saved_data["bias"].toTensor() : Tensor();
+    const MainGrad mg_b = bias ? MainGrad(b) : MainGrad();
+    const bool b_direct = bias && ctx->needs_input_grad(residual ? 3 : 2) && takes_vector(mg_b, b, H) && !mg_b.fresh == adds;
     const Tensor db = b_direct ? mg_b.buf : bias ? at::zeros({H}, h.options().dtype(at::kFloat)) : Tensor();
     check(K.norm_bwd(dy.data_ptr(), h.data_ptr(), w.data_ptr(), rstd.data_ptr(), rms ? nullptr : mean.data_ptr(),
                      dres.defined() ? dres.data_ptr() : nullptr, dx.data_ptr(), dw.data_ptr(), bias ? db.data_ptr() : nullptr,
@@ -280,7 +286,7 @@ struct Norm : public Function<Norm> {
           "hg_norm_bwd");
     count(2);
     if (mg.buf.defined()) MainGrad::written(w);
-    if (b_direct) MainGrad::written(saved[4]);
+    if (b_direct) MainGrad::written(b);
     // dx is the gradient of both x and the residual input (they are summed in the forward)
     return {dx, residual ? dx : Tensor(), mg.buf.defined() ? Tensor() : dw.to(w.scalar_type()),
             bias && !b_direct ? db.to(w.scalar_type()) : Tensor(), Tensor(), Tensor()};

@@ -84,7 +84,7 @@ def norm(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor | None = None, eps: f
     """Returns ``(normalised, h)`` with ``h = x + residual`` (``h is x`` without a residual).
 
     Fusing the residual add means the block computes ``h = x + attn_out`` and ``norm(h)`` in one pass
-    over memory.  The bias gradient goes to ``b.main_grad`` where one is bound and nothing hooks
+    over memory.  In a plain ``backward()`` the bias gradient goes to ``b.main_grad`` where one is bound and nothing hooks
     the parameter's gradient (C++ nodes), else through the normal autograd path (fp32 -> parameter dtype)."""
     shp = x.shape
     if not x.is_cuda:

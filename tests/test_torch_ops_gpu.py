@@ -178,3 +178,38 @@ def test_bias_gradients_go_to_their_buffers(rows, fresh, hooked):
             # fp32 sums of 16-bit rows; dy of the norm was rounded to 16 bits once: rows of about 23 (520 products of unit normals)
             atol = 1e-5 * rows ** 0.5 * 10 if p is b else 2.0 ** -9 * 23 * 6 * rows ** 0.5
             assert torch.allclose(got, want, rtol=1e-5, atol=atol)
+
+
+# with a buffer bound: autograd.grad and backward(inputs=...) give the gradient of a bias and leave its buffer alone, a graph of the
+# gradient is one, and a bias may change between forward and backward; afterwards a plain backward writes the buffers
+def test_bias_gradients_that_are_asked_for():
+    rand = lambda *shape: torch.randn(*shape, device=DEV).to(LP)
+    w, b, nw, nb = [torch.nn.Parameter(t) for t in (rand(520, 264), rand(520), rand(264), rand(264))]
+    for p in (w, b, nw, nb):
+        p.main_grad, p.mg_fresh = torch.full(p.shape, 2.0, device=DEV), True
+    x, dy, dn = rand(40, 264), rand(40, 520).requires_grad_(), rand(40, 264)
+    linear, norm = lambda: ops.linear(x, w, b), lambda: ops.norm(x, nw, nb, 1e-5, rms=False)[0]
+    assert _lib.native() is not None
+    untouched = lambda: all(p.mg_fresh and (p.main_grad == 2.0).all() for p in (b, nb))
+    want = dy.detach().double().sum(0), dn.double().sum(0)
+    close = lambda got, ref: torch.allclose(got.double(), ref, rtol=2.0 ** -8, atol=1e-4)      # fp32 sums of 40, one rounding
+    got = torch.autograd.grad(linear(), b, dy.detach())[0], torch.autograd.grad(norm(), nb, dn)[0]
+    assert all(close(g, r) for g, r in zip(got, want)) and untouched()
+    torch.autograd.backward(linear(), dy.detach(), inputs=[b])
+    torch.autograd.backward(norm(), dn, inputs=[nb])
+    assert close(b.grad, want[0]) and close(nb.grad, want[1]) and untouched()
+    b.grad = nb.grad = None
+    (g,) = torch.autograd.grad(linear(), b, dy, create_graph=True)
+    v = torch.randn(520, device=DEV)
+    assert torch.equal(torch.autograd.grad((g * v).sum(), dy)[0], v.to(LP).expand(40, 520)) and untouched()
+    y, n = linear(), norm()
+    with torch.no_grad():
+        b.mul_(2.0)
+        nb.mul_(2.0)
+    nw.mg_fresh = True                       # the norm's kernel has one switch for both sums
+    y.backward(dy.detach())
+    n.backward(dn)
+    assert b.grad is None and nb.grad is None and not b.mg_fresh and not nb.mg_fresh
+    assert torch.allclose(b.main_grad.double(), want[0], rtol=1e-5, atol=1e-4)
+    assert torch.allclose(nb.main_grad.double(), want[1], rtol=1e-5, atol=1e-4)
+    _lib.assert_healthy()
