@@ -295,7 +295,7 @@ grouped_gemm2_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_const
         q.N = w.m_end;
         if (!mbar_wait_warp(&s.tmem_full[acc], acc_phase, p.status, kTimeoutTmemFull, s.abort)) { *s.abort = 1; return false; }
         tc_fence_after();
-        if (row0 < q.M) store_tile_turned<kOutBf16>(q, share, tmem_base + lane_off + acc * BN, row0, w.n, Parts{nullptr, 0, 0, 0});
+        if (row0 < q.M) store_tile_turned(q, share, tmem_base + lane_off + acc * BN, row0, w.n, Parts{nullptr, 0, 0, 0});
         tc_fence_before();
         if (rank == 0) mbar_arrive(&s.tmem_empty[acc]);
         else mbar_arrive_cluster(map_to_cta(smem_u32(&s.tmem_empty[acc]), 0));
@@ -358,7 +358,8 @@ struct TilePlan {
   long long bytes() const { return s < 2 ? 0 : word_bytes() + (long long)tail * s * (CM * bn) * sizeof(float); }
 };
 
-// Costs in cycles of 1.6 GHz, fitted to 50 products of the three layouts, 128 to 152064 rows and columns, K = 63 to 152064.
+// Costs in cycles of 1.6 GHz, fitted to 50 products of the three layouts, 128 to 152064 rows and columns, K = 63 to 152064 (kStore
+// later, by the two given beside it).
 // A k-block moves 16 KB of A and 64 bn bytes of B into each SM, which takes 64 bytes a cycle from L2, and 2 bn cycles on the
 // tensor core: 256 + bn cycles, in which narrower tiles leave the tensor core idle.
 constexpr int kBlockCost = 256;

@@ -648,12 +648,11 @@ __device__ __forceinline__ void store_tile_part(const Params& p, const CUtensorM
   }
 }
 
-// A turned tile part: a lane holds one column of C, C[n0 + c, row0 + lane] for its columns c, so that a warp's store of one c is
-// 32 consecutive elements and needs no shared memory.  16 bits: neighbouring lanes trade a value, and each stores two columns
-// of one row, 16 lanes a row and 64 bytes each.
-template <int MODE>
+// A turned tile part, 16-bit results: a lane holds one column of C, C[n0 + c, row0 + lane] for its columns c, so that a warp's values
+// of one c are 32 consecutive elements and need no shared memory.  Neighbouring lanes trade a value, and each stores two columns of
+// one row, 16 lanes a row and 64 bytes each.
 __device__ __forceinline__ void store_tile_turned(const Params& p, Share w, uint32_t src, int row0, int n0, const Parts& parts) {
-  const int lane = int(lane_id()), col = row0 + lane;
+  const int lane = int(lane_id()), col = row0 + lane, odd = lane & 1;
   const bool mine = col < p.M;
   const float b = p.bias != nullptr && mine ? hg_lp2f(p.bias[col]) : 0.f;
 #pragma unroll 1
@@ -664,31 +663,13 @@ __device__ __forceinline__ void store_tile_turned(const Params& p, Share w, uint
     if (!HG_BOUNDS_OK(row0 >= 0 && row0 < p.M && n0 >= 0, p.status)) continue;
     parts.add(c / 32, r);
     const int rows = p.N - (n0 + c);
-    if constexpr (MODE == kOutBf16) {
-      const int odd = lane & 1;
-      hg_lp_t* at = reinterpret_cast<hg_lp_t*>(p.C) + size_t(n0 + c + odd) * p.ldc + (col - odd);
+    hg_lp_t* at = reinterpret_cast<hg_lp_t*>(p.C) + size_t(n0 + c + odd) * p.ldc + (col - odd);
 #pragma unroll
-      for (int i = 0; i < 32; i += 2, at += size_t(2) * p.ldc) {
-        const float x = __uint_as_float(r[i]) + b, y = __uint_as_float(r[i + 1]) + b;
-        const float z = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
-        if (mine && i + odd < rows) *reinterpret_cast<uint32_t*>(at) = odd ? pack_bf16(z, y) : pack_bf16(x, z);
-      }
-    } else {
-      float* at = reinterpret_cast<float*>(p.C) + size_t(n0 + c) * p.ldc + col;
-      float old[32];
-#pragma unroll
-      for (int i = 0; i < 32; ++i) old[i] = MODE == kOutF32Acc && mine && i < rows ? at[size_t(i) * p.ldc] : 0.f;
-#pragma unroll
-      for (int i = 0; i < 32; ++i)
-        if (mine && i < rows) at[size_t(i) * p.ldc] = MODE == kOutF32Acc ? __uint_as_float(r[i]) + b + old[i] : __uint_as_float(r[i]) + b;
+    for (int i = 0; i < 32; i += 2, at += size_t(2) * p.ldc) {
+      const float x = __uint_as_float(r[i]) + b, y = __uint_as_float(r[i + 1]) + b;
+      const float z = __shfl_xor_sync(0xffffffffu, odd ? x : y, 1);
+      if (mine && i + odd < rows) *reinterpret_cast<uint32_t*>(at) = odd ? pack_bf16(z, y) : pack_bf16(x, z);
     }
-  }
-}
-__device__ __forceinline__ void store_tile_turned(const Params& p, Share w, uint32_t src, int row0, int n0, const Parts& parts) {
-  switch (p.out_mode) {
-    case kOutF32: store_tile_turned<kOutF32>(p, w, src, row0, n0, parts); break;
-    case kOutF32Acc: store_tile_turned<kOutF32Acc>(p, w, src, row0, n0, parts); break;
-    default: store_tile_turned<kOutBf16>(p, w, src, row0, n0, parts); break;
   }
 }
 

@@ -68,3 +68,18 @@ def test_rule_of_the_epilogue_warps(mode, mn, blocks):
         plan = (ctypes.c_int * 5)()
         _lib.load().hg_gemm2_plan(256 * 74, 256, 64 * n, mode, 0, mn, 74, plan)
         assert plan[0] == 256 and plan[4] == warps
+
+
+def test_tiles_of_every_width_are_tested():
+    """What the cases of the GPU test are cut into: narrower and turned tiles, alone and shared."""
+    from tests.test_gemm_epilogue_gpu import test_tiles_of_every_width as tested
+
+    shapes = next(m.args[1] for m in tested.pytestmark if m.name == "parametrize" and m.args[0] == "M,N,K")
+    found = set()
+    for mode, may_turn in ((OUT_BF16, 1), (OUT_BF16, 0), (OUT_F32, 0)):
+        for shape in shapes:
+            plan = (ctypes.c_int * 5)()
+            _lib.load().hg_gemm2_plan(*shape, mode, may_turn, 0, 74, plan)
+            found.add((mode, plan[0] < 256, bool(plan[1]), plan[2] > 1))
+    assert found >= {(OUT_BF16, True, True, True), (OUT_BF16, True, False, False), (OUT_BF16, True, False, True),
+                     (OUT_BF16, False, False, False), (OUT_F32, True, False, False), (OUT_F32, True, False, True)}
