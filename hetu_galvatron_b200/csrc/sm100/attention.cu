@@ -28,6 +28,7 @@ constexpr int kBwdThreads = 320;
 constexpr int kBwdSoftmaxThreads = 256;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
+constexpr int kSmCount = 148;
 
 // 2^x on the special-function unit: one instruction, results below 2^-126 flush to zero, 2^-inf = 0.
 // (exp2f() wraps the same instruction in range handling that costs several more per element, and the score
@@ -1250,7 +1251,7 @@ struct Dkv128Smem {
   static constexpr int kTotal = HD == 128 ? 232448 : kUsed + 1024;
 };
 
-// NWG softmax warpgroups (2 or 4): thread == key row, warpgroup g owns query columns [g * 128 / NWG, (g + 1) * 128 / NWG)
+// NWG = 4 softmax warpgroups: thread == key row, warpgroup g owns query columns [g * 128 / NWG, (g + 1) * 128 / NWG)
 // of every step.  Four warpgroups put four warps on every scheduler, which is what keeps the exp2 unit and the FMA
 // pipe busy through the latencies of the loads from tensor memory and of the dependent exp2 / convert chains.
 // SHARED: key blocks may be shared between CTAs (p.chunk > 0).
@@ -2186,7 +2187,7 @@ flash_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmK, const BwdParams 
   auto unit_at = [&](int u) {
     Unit w;
     // some heads at a time, the last ones, whose dS may still be in L2, first
-    const int some = (2 * 148 + n_pairs - 1) / n_pairs, first = u / (some * n_pairs) * some, n = min(some, heads - first);
+    const int some = (2 * kSmCount + n_pairs - 1) / n_pairs, first = u / (some * n_pairs) * some, n = min(some, heads - first);
     const int r = u - first * n_pairs, pair = n_pairs - 1 - r / n, hb = heads - 1 - first - r % n;
     w.qb = 2 * pair;
     w.head = hb;
@@ -2392,7 +2393,6 @@ int g_dkv_variant = 0;
 // tiles per CTA with P in tensor memory wherever a sequence is longer than one tile (1, 2: side-by-side tests and timing).
 int g_fwd_variant = 0;
 
-constexpr int kSmCount = 148;
 constexpr int kDkvMinChunk = 4;   // fewest query steps of a CTA that shares its key block: about what its start and end cost
 
 template <typename K>
@@ -2407,7 +2407,7 @@ int set_smem(K kernel, int bytes) {
 template <int HD>
 bool two_tile_forward(const FwdParams& p) {
   if (p.Sq <= 128 || g_fwd_variant == 1) return false;
-  return HD == 128 || g_fwd_variant == 2 || (long long)((p.Sq + 127) / 128) * p.nheads * p.B > 148;
+  return HD == 128 || g_fwd_variant == 2 || (long long)((p.Sq + 127) / 128) * p.nheads * p.B > kSmCount;
 }
 
 template <int HD>
@@ -2645,7 +2645,7 @@ int hg_flash_bwd_ws(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTe
     const bool vec = (((uintptr_t(o->ptr) | uintptr_t(d_o->ptr)) & 15) | ((o->ss | o->sb | d_o->ss | d_o->sb) & 7)) == 0;
     const int64_t rows = int64_t(Sq) * B * nheads;
     const int64_t want = (rows * (hd / 8) + 256 * 4 - 1) / (256 * 4);
-    const int blocks = int(want < 148 * 8 ? want : 148 * 8);
+    const int blocks = int(want < kSmCount * 8 ? want : kSmCount * 8);
     auto k = hd == 128 ? (vec ? attn_bwd_dot_kernel<128, true> : attn_bwd_dot_kernel<128, false>)
                        : (vec ? attn_bwd_dot_kernel<64, true> : attn_bwd_dot_kernel<64, false>);
     k<<<blocks, 256, 0, st>>>((const hg_lp_t*)o->ptr, (const hg_lp_t*)d_o->ptr, o->ss, o->sb, d_o->ss, d_o->sb, Sq, B,
