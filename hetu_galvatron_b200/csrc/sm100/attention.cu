@@ -834,12 +834,7 @@ struct BwdParams {
   // fp32 parts in `part`, [CTA][dV, dK][128][HD]
   int chunk;
   float* part;
-  // dS as the dK/dV kernel leaves it for the dQ product (null: it does not): 128 x 128 tiles of the pairs of a key block and a query
-  // block that see each other, in the order of ds_tiles_before.  A tile is what the tensor core reads as an M-major operand without
-  // swizzle, [2 x 64 keys][16 x 8 queries][64 keys][8 queries]: a warp's store of eight queries of 32 keys is 512 bytes in a row
-  // (as rows of 128 queries, 32 pieces of 32 bytes, these stores doubled the kernel's time), and half a tile one copy.  A launch covers nh_c heads from h0_c on (and their kv heads from
-  // g0_c on) of the sequences from b0_c on: grids count from there.
-  hg_lp_t* dS;
+  // A launch covers nh_c heads from h0_c on (and their kv heads from g0_c on) of the sequences from b0_c on: grids count from there.
   int b0_c, g0_c, h0_c, nh_c;
 };
 
@@ -854,6 +849,22 @@ __host__ __device__ __forceinline__ long long ds_tiles_before(const BwdParams& p
   const long long n = e > a ? e - a : 0;
   return a * n_qs + n * n_qs - n * (a + e - 1) / 2 - n * d;
 }
+// dS as the dK/dV kernel leaves it for the dQ product: 128 x 128 tiles of the pairs of a key block and a query block that see each
+// other, in the order of ds_tiles_before, `heads` heads of the launch one after the other in each of up to kDsPieces pieces (0: dS is
+// not stored).  A tile is what the tensor core reads as an M-major operand without swizzle, [2 x 64 keys][16 x 8 queries][64 keys][8
+// queries]: a warp's store of eight queries of 32 keys is 512 bytes in a row (as rows of 128 queries, 32 pieces of 32 bytes, these
+// stores doubled the kernel's time), and half a tile one copy.
+constexpr int kDsPieces = 64;
+struct DsPieces {
+  hg_lp_t* at[kDsPieces];
+  int heads;
+};
+// Tile `tile` of a head, counted from the launch's first; `head_tiles`: of each.
+__device__ __forceinline__ hg_lp_t* ds_tile(const DsPieces& ds, int head, int64_t head_tiles, int64_t tile) {
+  const int piece = head / ds.heads;
+  return ds.at[piece] + ((head - piece * ds.heads) * head_tiles + tile) * (128 * 128);
+}
+
 // First query block that sees key block kb.
 __host__ __device__ __forceinline__ int ds_first_query_block(const BwdParams& p, int kb) {
   const int first = p.causal ? p.k_pos0 + kb * 128 - p.q_pos0 : 0;
@@ -1225,7 +1236,7 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // free, dV(i) when P^T(i) is stored, dK(i) and dP^T(i+1) when dS^T(i) is stored.
 //
 // Two warps fetch the statistics of the queries a step ahead.  In the softmax threads that cost registers: taken out, with the
-// probabilities kept in fp32, head dim 64, 8 x 1024 tokens and 25 heads 141 -> 106 us.  Where p.dS is set the threads also store
+// probabilities kept in fp32, head dim 64, 8 x 1024 tokens and 25 heads 141 -> 106 us.  Where ds has pieces the threads also store
 // dS for the dQ product, half of it between the two halves of their arithmetic (all at the end: 629 against 603 us at 2 x 4096,
 // 32 heads of 128; none: 518).
 // =================================================================================================
@@ -1259,7 +1270,7 @@ template <int HD, int NWG, bool SHARED>
 __global__ void __launch_bounds__(128 + 128 * NWG, 1)
 flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                         const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO,
-                        const BwdParams p) {
+                        const BwdParams p, const __grid_constant__ DsPieces ds) {
   static_assert(HD == 64 || HD == 128, "tensor memory holds S^T, dP^T and two accumulators of up to 128 columns");
   static_assert(NWG == 4, "a thread's 32 columns: two halves of 16");
   constexpr int kSoftmaxWarps = 4 * NWG;
@@ -1298,7 +1309,9 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
   uint64_t* kv_empty = bars + 19;    // the last products that read K and V have completed
   uint64_t* acc_empty = bars + 20;   // the epilogue has read dV and dK
   uint64_t* stats_empty = bars + 27; // 2
-  int* sStep = reinterpret_cast<int*>(bars + 29);   // [2][2], beside a step's statistics: its first query row, its tile of dS
+  // [2], beside a step's statistics: its tile of dS, its first query row
+  hg_lp_t** sTile = reinterpret_cast<hg_lp_t**>(bars + 29);
+  int* sRow = reinterpret_cast<int*>(bars + 31);
   const WorkSlot work{reinterpret_cast<uint4*>(bars + 24), bars + 21, bars + 22};
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -1533,11 +1546,11 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
     for (int n = 0; ok; ++n) {
       const Steps t = steps_of(blk);
       int h = t.h, qs = t.qs, ld_h = t.h, ld_qs = t.qs;
-      const int per_head = n_qs - t.qs0;
-      int64_t tile = 0;
-      if (p.dS != nullptr && t.n_it > 0)
-        tile = (int64_t(t.b - p.b0_c) * p.nh_c + h - p.h0_c) * ds_tiles_before(p, (p.Skv + 127) / 128) +
-               ds_tiles_before(p, t.k0 / 128) + (qs - t.qs0);
+      auto head_tile = [&]() {             // the first of this key block's and head's
+        return ds_tile(ds, (t.b - p.b0_c) * p.nh_c + h - p.h0_c, ds_tiles_before(p, (p.Skv + 127) / 128), ds_tiles_before(p, t.k0 / 128));
+      };
+      hg_lp_t* tile = nullptr;
+      if (ds.heads > 0 && t.n_it > 0) tile = head_tile() + (qs - t.qs0) * (128 * 128);
       float lse[2], d[2];
       auto fetch = [&]() {
         const size_t at = (size_t(t.b) * p.nheads + ld_h) * p.Sq;
@@ -1560,14 +1573,15 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
           st[128 + q2 + i * 64] = -d[i];
         }
         if (q2 == 0) {
-          sStep[sb * 2] = qs * 128;
-          sStep[sb * 2 + 1] = int(tile);
+          sTile[sb] = tile;
+          sRow[sb] = qs * 128;
         }
         mbar_arrive_warp(&stats_full[sb]);
-        ++tile;
+        tile += 128 * 128;
         if (++qs == n_qs) {
           qs = t.qs0;
-          if (p.dS != nullptr) tile += ds_tiles_before(p, (p.Skv + 127) / 128) - per_head;   // the next head's
+          ++h;
+          if (ds.heads > 0 && it + 1 < t.n_it) tile = head_tile();
         }
         if (it + 1 < t.n_it) fetch();
       }
@@ -1612,7 +1626,7 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         // The masked and the plain form are two straight-line bodies: a branch inside the element loop would cut it
         // into sixteen basic blocks, and the compiler schedules (overlaps the loads, FMAs and exp2 of different
         // elements) only inside one.
-        const int behind = p.k_pos0 + k_row - p.q_pos0 - sStep[sb * 2];       // of this row's key and the step's first query
+        const int behind = p.k_pos0 + k_row - p.q_pos0 - sRow[sb];       // of this row's key and the step's first query
         const int seen = k_row >= p.Skv ? CPT : p.causal ? behind - c0 : 0;
         const bool need_mask = (k_row - row + 128 > p.Skv) || (p.causal && behind - row + 127 > 0);
         auto probabilities = [&](auto masked) {
@@ -1668,8 +1682,8 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         tc_fence_before();
         mbar_arrive_warp(p_full);
         half_ds(ra, 0);
-        if (p.dS != nullptr) {
-          hg_lp_t* out = p.dS + int64_t(sStep[sb * 2 + 1]) * (128 * 128) + ((row >> 6) * (64 * 128) + c0 * 64 + (row & 63) * 8);
+        if (ds.heads > 0) {
+          hg_lp_t* out = sTile[sb] + ((row >> 6) * (64 * 128) + c0 * 64 + (row & 63) * 8);
 #pragma unroll
           for (int i = 0; i < 2; ++i)
             *reinterpret_cast<uint4*>(out + i * 512) = make_uint4(dsp[4 * i], dsp[4 * i + 1], dsp[4 * i + 2], dsp[4 * i + 3]);
@@ -1677,8 +1691,8 @@ flash_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_co
         tmem_ld_wait();
         half_ds(rb, 16);
         tmem_st16(dpt + 16, dsp);
-        if (p.dS != nullptr) {
-          hg_lp_t* out = p.dS + int64_t(sStep[sb * 2 + 1]) * (128 * 128) + ((row >> 6) * (64 * 128) + c0 * 64 + (row & 63) * 8);
+        if (ds.heads > 0) {
+          hg_lp_t* out = sTile[sb] + ((row >> 6) * (64 * 128) + c0 * 64 + (row & 63) * 8);
 #pragma unroll
           for (int i = 2; i < 4; ++i)
             *reinterpret_cast<uint4*>(out + i * 512) = make_uint4(dsp[4 * i], dsp[4 * i + 1], dsp[4 * i + 2], dsp[4 * i + 3]);
@@ -2157,7 +2171,7 @@ struct DqDsSmem {
 
 template <int HD>
 __global__ void __launch_bounds__(192, 1)
-flash_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmK, const BwdParams p, int heads) {
+flash_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmK, const BwdParams p, int heads, const __grid_constant__ DsPieces ds) {
   extern __shared__ uint8_t smem_raw[];
   using L = DqDsSmem<HD>;
   constexpr int NS = L::kStages;
@@ -2176,7 +2190,7 @@ flash_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmK, const BwdParams 
 
   struct Unit {
     int qb, h, b, kbs[2];        // first query block, head, sequence; key blocks that each of the two query blocks sees
-    int64_t head;                // among the heads of this launch
+    int head;                    // among the heads of this launch
   };
   auto key_blocks = [&](int qb) {
     if (qb >= n_qs) return 0;
@@ -2228,9 +2242,10 @@ flash_bwd_dq_ds_kernel(const __grid_constant__ CUtensorMap tmK, const BwdParams 
       asked = false;
       const Unit w = unit_at(blk.x);
       const int kslot = p.kmap.slot(w.h, p.qpg), n = most(w);
+      const hg_lp_t* tiles = ds_tile(ds, w.head, head_tiles, 0);
       for (int kb = 0; ok && kb < n; ++kb) {
         // a first query block that does not see this key block has no tile: this is then the one before the second's
-        const hg_lp_t* src = p.dS + (w.head * head_tiles + ds_tiles_before(p, kb) + w.qb - ds_first_query_block(p, kb)) * (128 * 128);
+        const hg_lp_t* src = tiles + (ds_tiles_before(p, kb) + w.qb - ds_first_query_block(p, kb)) * (128 * 128);
         for (int half = 0; half < 2; ++half) {
           if (!mbar_wait_warp(&empty[stage], phase ^ 1, p.status, kTimeoutSmemEmpty, abort_flag)) { ok = false; break; }
           uint8_t* s = base + stage * L::kStage;
@@ -2456,7 +2471,7 @@ int dkv_chunk_steps(BwdParams p, int Skv, int nkv) {
 
 template <int HD>
 int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-               const BwdParams& p, int Skv, int nkv, int nb, bool wide, cudaStream_t st) {
+               const BwdParams& p, const DsPieces& ds, int Skv, int nkv, int nb, bool wide, cudaStream_t st) {
   int rc;
   dim3 grid((Skv + 127) / 128, nkv, nb);
   if (wide) {
@@ -2466,7 +2481,7 @@ int launch_dkv(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
     const bool shared = p.chunk > 0;
     auto k = shared ? flash_bwd_dkv128_kernel<HD, kDkvWarpgroups, true> : flash_bwd_dkv128_kernel<HD, kDkvWarpgroups, false>;
     if (!cfg[shared]) { if ((rc = set_smem(k, Dkv128Smem<HD>::kTotal))) return rc; cfg[shared] = true; }
-    k<<<grid, 128 + 128 * kDkvWarpgroups, Dkv128Smem<HD>::kTotal, st>>>(tq, tk, tv, tdo, p);
+    k<<<grid, 128 + 128 * kDkvWarpgroups, Dkv128Smem<HD>::kTotal, st>>>(tq, tk, tv, tdo, p, ds);
     if (p.chunk > 0) dkv_sum_kernel<HD><<<dim3(blocks * 8, nkv, nb), 4 * HD, 0, st>>>(p, int(grid.x));
   } else {
     static bool cfg = false;
@@ -2488,32 +2503,37 @@ int launch_dq(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& t
 }
 
 template <int HD>
-int launch_dq_ds(const CUtensorMap& tk, const BwdParams& p, int nb, cudaStream_t st) {
+int launch_dq_ds(const CUtensorMap& tk, const BwdParams& p, const DsPieces& ds, int nb, cudaStream_t st) {
   int rc;
   static bool cfg = false;
   auto k = flash_bwd_dq_ds_kernel<HD>;
   if (!cfg) { if ((rc = set_smem(k, DqDsSmem<HD>::kTotal))) return rc; cfg = true; }
   const int heads = p.nh_c * nb, units = ((p.Sq + 255) / 256) * heads;
-  k<<<units, 192, DqDsSmem<HD>::kTotal, st>>>(tk, p, heads);
+  k<<<units, 192, DqDsSmem<HD>::kTotal, st>>>(tk, p, heads, ds);
   return int(cudaGetLastError());
 }
 
 // How the heads of a backward are cut where dS^T goes through memory: launches of `nb` sequences and `ng` kv heads each, whose
 // tiles fit kDsMost.  ng = 0: not even one kv head's do, and the dQ kernel recomputes S and dP.
-constexpr long long kDsTile = 128 * 128 * 2, kDsMost = 3ll << 29;
+// The tiles are kept in pieces of `heads` heads and at most kDsPiece bytes (one head, if that has more): a caching allocator finds them
+// among the blocks that it holds, where one block for all had to be had from the device for every few new layers (1531 tokens, 28
+// heads: the first pass of a layer 0.97 instead of 0.60 ms).  More than half of kDsPiece in each, so that there are kDsPieces at most.
+constexpr long long kDsTile = 128 * 128 * 2, kDsMost = 3ll << 29, kDsPiece = 48ll << 20;
+static_assert(kDsMost / (kDsPiece / 2) <= kDsPieces, "the table of pieces");
 struct DsCut {
   int nb, ng;
   long long bytes;
+  int pieces, heads;
 };
 DsCut ds_cut(const BwdParams& p, int Skv, int nkv) {
   const long long group = ds_tiles_before(p, (Skv + 127) / 128) * p.qpg * kDsTile;
-  if (g_dkv_variant != 0 || group > kDsMost) return {0, 0, 0};
-  if (group == 0) return {p.B, nkv, 0};
+  if (g_dkv_variant != 0 || group > kDsMost) return {};
+  if (group == 0) return {p.B, nkv, 0, 0, 0};
   const long long groups = kDsMost / group;
-  DsCut c;
+  DsCut c{};
   c.ng = groups < nkv ? int(groups) : nkv;
   c.nb = groups < nkv ? 1 : groups / nkv < p.B ? int(groups / nkv) : p.B;
-  if (p.chunk > 0 && (c.ng < nkv || c.nb < p.B)) return {0, 0, 0};     // shared key blocks are few: they are launched at once
+  if (p.chunk > 0 && (c.ng < nkv || c.nb < p.B)) return {};     // shared key blocks are few: they are launched at once
   auto even = [](int n, int most) {                                     // launches of about the same size
     const int times = (n + most - 1) / most;
     return (n + times - 1) / times;
@@ -2521,6 +2541,10 @@ DsCut ds_cut(const BwdParams& p, int Skv, int nkv) {
   c.ng = even(nkv, c.ng);
   c.nb = even(p.B, c.nb);
   c.bytes = group * c.ng * c.nb;
+  const long long head = group / p.qpg;
+  const int all = c.ng * c.nb * p.qpg;
+  c.heads = head < kDsPiece ? even(all, int(kDsPiece / head)) : 1;
+  c.pieces = (all + c.heads - 1) / c.heads;
   return c;
 }
 // Whether storing dS pays.  In one launch it does.  Several end one by one, with fewer and fewer CTAs at work, which costs more than
@@ -2533,9 +2557,9 @@ bool ds_pays(const DsCut& c, const BwdParams& p, int Skv, int nkv, int hd) {
   const int last = c.ng < nkv ? (nkv - 1) % c.ng + 1 : ((p.B - 1) % c.nb + 1) * nkv;
   return hd == 128 && (long long)((Skv + 127) / 128) * last >= 5 * kSmCount;
 }
-// The scratch of a backward, in floats: row sums of dO * O, parts of dK and dV, tiles of dS^T.
+// The scratch of a backward, in floats: row sums of dO * O, parts of dK and dV, and each piece of the tiles of dS^T.
 struct BwdScratch {
-  long long sums, parts, ds;
+  long long sums, parts, piece;
   int chunk;
   DsCut cut;
 };
@@ -2546,7 +2570,7 @@ BwdScratch bwd_scratch(BwdParams p, int Skv, int nkv, int hd) {
   w.chunk = p.chunk = dkv_chunk_steps(p, Skv, nkv);
   if (w.chunk) w.parts = (long long)dkv_ctas(p, (Skv + 127) / 128) * nkv * p.B * 2 * 128 * hd;
   w.cut = ds_cut(p, Skv, nkv);
-  w.ds = w.cut.bytes / 4;
+  if (w.cut.bytes > 0) w.piece = w.cut.bytes / (w.cut.nb * w.cut.ng * p.qpg) * w.cut.heads / 4;
   return w;
 }
 
@@ -2598,16 +2622,24 @@ static BwdParams bwd_sizes(int Sq, int Skv, int B, int nheads, int nkv, int caus
 }
 
 // Floats of scratch that hg_flash_bwd_ws can use: the row sums of dO * O, [B, nheads, Sq], where key blocks are shared the parts
-// of dK and dV, and, if `tiles`, dS^T of up to kDsMost bytes.
+// of dK and dV, and, if `tiles`, all pieces of dS^T, of up to kDsMost bytes (see hg_flash_bwd_pieces).
 long long hg_flash_bwd_scratch_of(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0, int tiles) {
   if (Sq <= 0 || Skv <= 0 || B <= 0 || nheads <= 0 || nkv <= 0) return 0;
   const BwdScratch w = bwd_scratch(bwd_sizes(Sq, Skv, B, nheads, nkv, causal, q_pos0, k_pos0), Skv, nkv, hd);
-  return w.sums + w.parts + (tiles ? w.ds : 0);
+  return w.sums + w.parts + (tiles ? w.piece * w.cut.pieces : 0);
 }
 long long hg_flash_bwd_scratch(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
   return hg_flash_bwd_scratch_of(Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0, 1);
 }
-// Whether it is worth giving hg_flash_bwd_ws the scratch for dS.
+// Pieces of scratch that hg_flash_bwd_ws can use for dS^T, and the floats of each.
+int hg_flash_bwd_pieces(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0, long long* floats) {
+  *floats = 0;
+  if (Sq <= 0 || Skv <= 0 || B <= 0 || nheads <= 0 || nkv <= 0) return 0;
+  const BwdScratch w = bwd_scratch(bwd_sizes(Sq, Skv, B, nheads, nkv, causal, q_pos0, k_pos0), Skv, nkv, hd);
+  *floats = w.piece;
+  return w.cut.pieces;
+}
+// Whether it is worth giving them.
 int hg_flash_bwd_tiles_pay(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
   if (Sq <= 0 || Skv <= 0 || B <= 0 || nheads <= 0 || nkv <= 0) return 0;
   const BwdParams p = bwd_sizes(Sq, Skv, B, nheads, nkv, causal, q_pos0, k_pos0);
@@ -2628,13 +2660,15 @@ int hg_flash_bwd_has_room(int device) {
   return left.load(std::memory_order_relaxed) <= 0 || left.fetch_sub(1, std::memory_order_relaxed) <= 0;
 }
 
-// ws: scratch of ws_floats fp32 values, 16-byte aligned, at least [B, nheads, Sq] (filled here with rowsum(dO*O)).  With less
-// than hg_flash_bwd_scratch floats S and dP are computed again for dQ, and with less than hg_flash_bwd_scratch_of(.., 0) every
-// key block has one CTA.  launched (may be null): the kernels that were launched.
+// ws: scratch of ws_floats fp32 values, 16-byte aligned, at least [B, nheads, Sq] (filled here with rowsum(dO*O)).  With less than
+// hg_flash_bwd_scratch_of(.., 0) floats every key block has one CTA.  tiles: n_tiles pieces of tile_floats fp32 values, 16-byte
+// aligned; with fewer or smaller ones than hg_flash_bwd_pieces says, S and dP are computed again for dQ.
+// launched (may be null): the kernels that were launched.
 int hg_flash_bwd_ws(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTensor* v, const HgAttnTensor* o,
-                    const HgAttnTensor* d_o, const void* lse, void* ws, long long ws_floats, const HgAttnTensor* dq,
-                    const HgAttnTensor* dk, const HgAttnTensor* dv, int Sq, int Skv, int B, int nheads, int nkv, int hd,
-                    int causal, int q_pos0, int k_pos0, float scale, int* launched, void* stream) {
+                    const HgAttnTensor* d_o, const void* lse, void* ws, long long ws_floats, void* const* tiles, int n_tiles,
+                    long long tile_floats, const HgAttnTensor* dq, const HgAttnTensor* dk, const HgAttnTensor* dv, int Sq, int Skv,
+                    int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0, float scale, int* launched,
+                    void* stream) {
   void* dsum = ws;
   if (launched != nullptr) *launched = 0;
   if (hd != 64 && hd != 128) return -1;
@@ -2662,14 +2696,18 @@ int hg_flash_bwd_ws(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTe
   p.dV = (hg_lp_t*)dv->ptr; p.dv_ss = dv->ss; p.dv_sb = dv->sb; p.dvmap = {dv->gs, dv->hs, dv->off};
   p.status = hg_host::status_ptr();
   const BwdScratch w = bwd_scratch(p, Skv, nkv, hd);
-  const bool aligned = (reinterpret_cast<uintptr_t>(ws) & 15) == 0;
-  if (w.parts > 0 && aligned && ws_floats >= w.sums + w.parts) {
+  if (w.parts > 0 && (reinterpret_cast<uintptr_t>(ws) & 15) == 0 && ws_floats >= w.sums + w.parts) {
     p.chunk = w.chunk;
     p.part = static_cast<float*>(ws) + w.sums;
   }
-  const bool tiles = w.ds > 0 && aligned && ws_floats >= w.sums + w.parts + w.ds;
-  if (tiles) p.dS = reinterpret_cast<hg_lp_t*>(static_cast<float*>(ws) + w.sums + w.parts);
-  const DsCut cut = tiles ? w.cut : DsCut{B, nkv, 0};
+  bool stored = w.cut.pieces > 0 && n_tiles >= w.cut.pieces && tile_floats >= w.piece;
+  for (int i = 0; stored && i < w.cut.pieces; ++i) stored = tiles[i] != nullptr && (reinterpret_cast<uintptr_t>(tiles[i]) & 15) == 0;
+  DsPieces ds{};
+  if (stored) {
+    ds.heads = w.cut.heads;
+    for (int i = 0; i < w.cut.pieces; ++i) ds.at[i] = static_cast<hg_lp_t*>(tiles[i]);
+  }
+  const DsCut cut = stored ? w.cut : DsCut{B, nkv, 0, 0, 0};
   CUtensorMap tq, tk, tv, tdo, tk64;
   const bool wide = g_dkv_variant == 0;   // 128-query steps, P^T / dS^T in tensor memory
   const int q_rows = wide ? 128 : 64;
@@ -2677,19 +2715,19 @@ int hg_flash_bwd_ws(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTe
   if ((rc = make_map(&tk, k->ptr, hd, k->slots, Skv, B, k->ss, k->sb, 128))) return rc;
   if ((rc = make_map(&tv, v->ptr, hd, v->slots, Skv, B, v->ss, v->sb, 128))) return rc;
   if ((rc = make_map(&tdo, d_o->ptr, hd, d_o->slots, Sq, B, d_o->ss, d_o->sb, q_rows))) return rc;
-  if (tiles && (rc = make_map(&tk64, k->ptr, hd, k->slots, Skv, B, k->ss, k->sb, 64))) return rc;
+  if (stored && (rc = make_map(&tk64, k->ptr, hd, k->slots, Skv, B, k->ss, k->sb, 64))) return rc;
   for (int b0 = 0; b0 < B; b0 += cut.nb)
     for (int g0 = 0; g0 < nkv; g0 += cut.ng) {
       const int nb = B - b0 < cut.nb ? B - b0 : cut.nb, ng = nkv - g0 < cut.ng ? nkv - g0 : cut.ng;
       p.b0_c = b0; p.g0_c = g0; p.h0_c = g0 * p.qpg; p.nh_c = ng * p.qpg;
-      if ((rc = hd == 128 ? launch_dkv<128>(tq, tk, tv, tdo, p, Skv, ng, nb, wide, st)
-                          : launch_dkv<64>(tq, tk, tv, tdo, p, Skv, ng, nb, wide, st))) return rc;
+      if ((rc = hd == 128 ? launch_dkv<128>(tq, tk, tv, tdo, p, ds, Skv, ng, nb, wide, st)
+                          : launch_dkv<64>(tq, tk, tv, tdo, p, ds, Skv, ng, nb, wide, st))) return rc;
       kernels += p.chunk > 0 ? 2 : 1;
-      if (!tiles) continue;
-      if ((rc = hd == 128 ? launch_dq_ds<128>(tk64, p, nb, st) : launch_dq_ds<64>(tk64, p, nb, st))) return rc;
+      if (!stored) continue;
+      if ((rc = hd == 128 ? launch_dq_ds<128>(tk64, p, ds, nb, st) : launch_dq_ds<64>(tk64, p, ds, nb, st))) return rc;
       ++kernels;
     }
-  if (!tiles) {
+  if (!stored) {
     if ((rc = make_map(&tq, q->ptr, hd, q->slots, Sq, B, q->ss, q->sb, 128))) return rc;
     if ((rc = make_map(&tdo, d_o->ptr, hd, d_o->slots, Sq, B, d_o->ss, d_o->sb, 128))) return rc;
     if ((rc = hd == 128 ? launch_dq<128>(tq, tk, tv, tdo, p, st) : launch_dq<64>(tq, tk, tv, tdo, p, st))) return rc;
@@ -2704,8 +2742,8 @@ int hg_flash_bwd(const HgAttnTensor* q, const HgAttnTensor* k, const HgAttnTenso
                  const HgAttnTensor* d_o, const void* lse, void* dsum, const HgAttnTensor* dq, const HgAttnTensor* dk,
                  const HgAttnTensor* dv, int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0,
                  int k_pos0, float scale, void* stream) {
-  return hg_flash_bwd_ws(q, k, v, o, d_o, lse, dsum, 0, dq, dk, dv, Sq, Skv, B, nheads, nkv, hd, causal, q_pos0, k_pos0,
-                         scale, nullptr, stream);
+  return hg_flash_bwd_ws(q, k, v, o, d_o, lse, dsum, 0, nullptr, 0, 0, dq, dk, dv, Sq, Skv, B, nheads, nkv, hd, causal, q_pos0,
+                         k_pos0, scale, nullptr, stream);
 }
 
 }  // extern "C"

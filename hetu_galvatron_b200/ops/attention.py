@@ -50,16 +50,24 @@ def attention_reference(q, k, v, causal=True, scale=None, q_pos0=0, k_pos0=0, dr
     return o.permute(2, 0, 1, 3).to(q.dtype), lse
 
 
-def _backward_scratch(lib, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, device) -> torch.Tensor:
-    """fp32 scratch of the backward kernels: row sums of dO * O, where key blocks are shared between CTAs their parts, and, where
-    storing it pays, dS, without which, should there be no room for it, dQ takes longer."""
+def _backward_scratch(lib, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, device):
+    """fp32 scratch of the backward kernels: row sums of dO * O and, where key blocks are shared between CTAs, their parts; and the
+    pieces that hold dS where storing it pays, none if there is no room for them: dQ then takes longer."""
     args = (S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0)
+    ws = torch.empty(lib.hg_flash_bwd_scratch_of(*args, 0), dtype=torch.float32, device=device)
     if lib.hg_flash_bwd_tiles_pay(*args) and lib.hg_flash_bwd_has_room(device.index):
+        floats = ctypes.c_longlong()
         try:
-            return torch.empty(lib.hg_flash_bwd_scratch(*args), dtype=torch.float32, device=device)
+            n = lib.hg_flash_bwd_pieces(*args, ctypes.byref(floats))
+            return ws, [torch.empty(floats.value, dtype=torch.float32, device=device) for _ in range(n)]
         except torch.cuda.OutOfMemoryError:
             lib.hg_flash_bwd_no_room(device.index)
-    return torch.empty(lib.hg_flash_bwd_scratch_of(*args, 0), dtype=torch.float32, device=device)
+    return ws, []
+
+
+def _tiles_args(tiles):
+    """The pieces as the kernels' entry point takes them."""
+    return (ctypes.c_void_p * len(tiles))(*[t.data_ptr() for t in tiles]), len(tiles), tiles[0].numel() if tiles else 0
 
 
 class _FlashPacked(torch.autograd.Function):
@@ -94,7 +102,7 @@ class _FlashPacked(torch.autograd.Function):
         slots = nh + 2 * ng
         dout = dout.contiguous()
         dqkv = torch.empty_like(qkv)
-        ws = _backward_scratch(lib, S, S, B, nh, ng, hd, causal, 0, 0, qkv.device)
+        ws, tiles = _backward_scratch(lib, S, S, B, nh, ng, hd, causal, 0, 0, qkv.device)
         ss, sb = B * P, P
         q = _desc(qkv, ss, sb, slots, qpg + 2, 1, 0)
         k = _desc(qkv, ss, sb, slots, qpg + 2, 0, qpg)
@@ -106,7 +114,7 @@ class _FlashPacked(torch.autograd.Function):
         dv = _desc(dqkv, ss, sb, slots, qpg + 2, 0, qpg + 1)
         kernels = ctypes.c_int()
         rc = lib.hg_flash_bwd_ws(ctypes.byref(q), ctypes.byref(k), ctypes.byref(v), ctypes.byref(o), ctypes.byref(do),
-                                 lse.data_ptr(), ws.data_ptr(), ws.numel(), ctypes.byref(dq), ctypes.byref(dk),
+                                 lse.data_ptr(), ws.data_ptr(), ws.numel(), *_tiles_args(tiles), ctypes.byref(dq), ctypes.byref(dk),
                                  ctypes.byref(dv), S, S, B, nh, ng, hd, int(causal), 0, 0, float(scale),
                                  ctypes.byref(kernels), _lib.stream())
         _lib.check(rc, "hg_flash_bwd")
@@ -280,7 +288,7 @@ def flash_backward(q, k, v, out, dout, lse, causal, scale, q_pos0=0, k_pos0=0):
     Skv, ng = k.shape[0], k.shape[2]
     qpg = nh // ng
     dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-    ws = _backward_scratch(lib, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, q.device)
+    ws, tiles = _backward_scratch(lib, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, q.device)
     qd = _desc(q, q.stride(0), q.stride(1), nh, qpg, 1, 0)
     kd = _desc(k, k.stride(0), k.stride(1), ng, 1, 0, 0)
     vd = _desc(v, v.stride(0), v.stride(1), ng, 1, 0, 0)
@@ -291,7 +299,7 @@ def flash_backward(q, k, v, out, dout, lse, causal, scale, q_pos0=0, k_pos0=0):
     dvd = _desc(dv, dv.stride(0), dv.stride(1), ng, 1, 0, 0)
     kernels = ctypes.c_int()
     rc = lib.hg_flash_bwd_ws(ctypes.byref(qd), ctypes.byref(kd), ctypes.byref(vd), ctypes.byref(od), ctypes.byref(dod),
-                             lse.data_ptr(), ws.data_ptr(), ws.numel(), ctypes.byref(dqd), ctypes.byref(dkd),
+                             lse.data_ptr(), ws.data_ptr(), ws.numel(), *_tiles_args(tiles), ctypes.byref(dqd), ctypes.byref(dkd),
                              ctypes.byref(dvd), S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0, float(scale),
                              ctypes.byref(kernels), _lib.stream())
     _lib.check(rc, "hg_flash_bwd")

@@ -1,4 +1,6 @@
 """Which way a backward of attention goes, on both sides of each line of the rule."""
+import ctypes
+
 import pytest
 import torch
 
@@ -19,23 +21,34 @@ def test_rule_of_stored_ds(S, B, nh, ng, hd, causal, k0, stored):
     assert 4 * (lib.hg_flash_bwd_scratch(*sizes) - lib.hg_flash_bwd_scratch_of(*sizes, 0)) <= 3 << 29
 
 
+# heads of 18, 69 and 45 MB, of 2.6 MB in even pieces, one query of one head, the most pieces, none
+@pytest.mark.parametrize("S,B,nh,ng,hd,pieces,heads", [(4096, 2, 32, 32, 128, 32, 2), (8192, 1, 20, 20, 64, 20, 1),
+                                                       (6600, 1, 32, 32, 64, 32, 1), (1531, 1, 28, 4, 128, 2, 14), (1, 1, 1, 1, 64, 1, 1),
+                                                       (4992, 1, 60, 60, 128, 60, 1), (16384, 1, 64, 8, 128, 0, 0)])
+def test_pieces_of_ds(S, B, nh, ng, hd, pieces, heads):
+    lib, sizes, floats = _lib.load(), (S, S, B, nh, ng, hd, 1, 0, 0), ctypes.c_longlong()
+    assert lib.hg_flash_bwd_pieces(*sizes, ctypes.byref(floats)) == pieces <= 64
+    blocks = (S + 127) // 128
+    head = blocks * (blocks + 1) // 2 * 128 * 128 // 2                   # floats of a head's tiles
+    assert floats.value == heads * head and (heads <= 1 or 4 * heads * head <= 48 << 20)
+    assert lib.hg_flash_bwd_scratch(*sizes) - lib.hg_flash_bwd_scratch_of(*sizes, 0) == pieces * floats.value
+
+
 def test_an_allocator_without_room_is_left_alone(monkeypatch):
-    """It is asked for dS once, not at every layer of every backward, and later again; a smaller scratch it has to have."""
+    """It is asked for dS once, not at every layer of every backward, and later again; the other scratch it has to have."""
     lib, sizes, device = _lib.load(), (4096, 4096, 2, 32, 32, 128, True, 0, 0), torch.device("cuda", 7)
-    small, asked = lib.hg_flash_bwd_scratch_of(*sizes, 0), []
+    small, floats, asked = lib.hg_flash_bwd_scratch_of(*sizes, 0), ctypes.c_longlong(), []
+    assert lib.hg_flash_bwd_pieces(*sizes, ctypes.byref(floats)) == 32
 
     def empty(n, dtype, device):
         asked.append(n)
-        if n > small:
+        if len(asked) % 4 == 0 and n == floats.value:                    # the third piece
             raise torch.cuda.OutOfMemoryError("no room")
         return torch.zeros(1)
 
     monkeypatch.setattr(attention.torch, "empty", empty)
-    calls = lambda n: [attention._backward_scratch(lib, *sizes, device) for _ in range(n)]
-    calls(1)
-    assert asked == [lib.hg_flash_bwd_scratch(*sizes), small]
-    calls(256)
-    assert asked[2:] == [small] * 256
+    calls = lambda n: [attention._backward_scratch(lib, *sizes, device)[1] for _ in range(n)]
+    assert calls(1) == [[]] and asked == [small] + [floats.value] * 3
+    assert calls(256) == [[]] * 256 and asked[4:] == [small] * 256
     assert lib.hg_flash_bwd_has_room(6)                                  # another device
-    calls(1)
-    assert asked[258:] == asked[:2]
+    assert calls(1) == [[]] and asked[260:] == asked[:4]

@@ -90,31 +90,43 @@ def test_dq_from_stored_ds(Sq, Skv, B, nh, ng, hd, causal, q0, k0):
     _lib.assert_healthy()
 
 
-# scratch for everything, one float less, for shared key blocks alone, one float less, for the row sums alone; launches over some of the
-# heads and of the sequences, which the callers of this package do not ask for; key blocks that are shared
+# all pieces, one piece less, pieces of one float less, one that starts at an odd place; scratch for shared key blocks, one float less, for
+# the row sums alone; launches over some of the heads and of the sequences, which the callers of this package do not ask for; key blocks
+# that are shared; pieces of several heads and of one
 @pytest.mark.parametrize("Sq,Skv,B,nh,ng,hd,causal", [(8192, 8192, 1, 32, 32, 64, True), (4096, 4096, 3, 16, 8, 64, False),
-                                                      (1531, 1531, 1, 7, 1, 128, True), (640, 640, 1, 6, 2, 64, False)])
+                                                      (1531, 1531, 1, 28, 4, 128, True), (1531, 1531, 1, 7, 1, 128, True),
+                                                      (640, 640, 1, 6, 2, 64, False), (4096, 4096, 1, 10, 5, 128, True)])
 def test_backward_with_any_scratch(Sq, Skv, B, nh, ng, hd, causal):
-    lib, sizes = _lib.load(), (Sq, Skv, B, nh, ng, hd, int(causal), 0, 0)
+    lib, sizes, each = _lib.load(), (Sq, Skv, B, nh, ng, hd, int(causal), 0, 0), ctypes.c_longlong()
     g = torch.Generator(device=DEV).manual_seed(Sq + hd)
     q, dout = (torch.randn(Sq, B, nh, hd, device=DEV, generator=g).to(torch.bfloat16) for _ in "qd")
     k, v = (torch.randn(Skv, B, ng, hd, device=DEV, generator=g).to(torch.bfloat16) for _ in "kv")
     out, lse = ops.flash_attention(q, k, v, causal=causal, return_lse=True)
-    most, parts, sums = lib.hg_flash_bwd_scratch(*sizes), lib.hg_flash_bwd_scratch_of(*sizes, 0), B * nh * Sq
-    results = []
-    for floats in (most, most - 1, parts, max(parts - 1, sums), sums):
+    parts, sums = lib.hg_flash_bwd_scratch_of(*sizes, 0), B * nh * Sq
+    n = lib.hg_flash_bwd_pieces(*sizes, ctypes.byref(each))
+    assert n > 0
+    pieces = [torch.empty(each.value + 64, device=DEV) for _ in range(n)]
+    at = [t.data_ptr() for t in pieces]
+    heads = lambda t: ctypes.byref(_desc(t, t.stride(0), t.stride(1), nh, nh // ng, 1, 0))
+    kv = lambda t: ctypes.byref(_desc(t, t.stride(0), t.stride(1), ng, 1, 0, 0))
+    results, launched = [], ctypes.c_int()
+    for floats, tiles, most in ((parts, at, each.value), (parts, at[1:], each.value), (parts, at, each.value - 1),
+                                (parts, [*at[:-1], at[-1] + 4], each.value), (max(parts - 1, sums), at, each.value), (sums, [], 0)):
         got, ws = [torch.full_like(t, float("nan")) for t in (q, k, v)], torch.full((floats,), float("nan"), device=DEV)
-        heads = lambda t: ctypes.byref(_desc(t, t.stride(0), t.stride(1), nh, nh // ng, 1, 0))
-        kv = lambda t: ctypes.byref(_desc(t, t.stride(0), t.stride(1), ng, 1, 0, 0))
-        assert lib.hg_flash_bwd_ws(heads(q), kv(k), kv(v), heads(out), heads(dout), lse.data_ptr(), ws.data_ptr(), floats, heads(got[0]),
-                                   kv(got[1]), kv(got[2]), *sizes[:6], int(causal), 0, 0, hd ** -0.5, None, _lib.stream()) == 0
+        for t in pieces:
+            t.fill_(float("nan"))
+        assert lib.hg_flash_bwd_ws(heads(q), kv(k), kv(v), heads(out), heads(dout), lse.data_ptr(), ws.data_ptr(), floats,
+                                   (ctypes.c_void_p * len(tiles))(*tiles), len(tiles), most, heads(got[0]), kv(got[1]), kv(got[2]),
+                                   *sizes[:6], int(causal), 0, 0, hd ** -0.5, ctypes.byref(launched), _lib.stream()) == 0
+        stored = not all(t.isnan().all() for t in pieces)
+        assert stored == (tiles is at and most == each.value)
+        assert all(t[each.value:].isnan().all() for t in pieces)         # nothing behind them
         results.append(got)
     for got in results:
-        assert torch.equal(got[0], results[0][0])                         # dQ: the same bits, stored dS or not
+        assert torch.equal(got[0], results[0][0])                        # dQ: the same bits, stored dS or not
         assert rel_err(got[1], results[0][1]) < 1e-3 and rel_err(got[2], results[0][2]) < 1e-3
-    for i in (1, 2):                                                      # dK and dV: as long as the same CTAs share
-        assert torch.equal(results[0][i], results[1][i]) and torch.equal(results[0][i], results[2][i])
-        assert torch.equal(results[3][i], results[4][i])
+    for i in (1, 2):                                                     # dK and dV: as long as the same CTAs share
+        assert all(torch.equal(results[0][i], r[i]) for r in results[1:4]) and torch.equal(results[4][i], results[5][i])
     _lib.assert_healthy()
 
 
