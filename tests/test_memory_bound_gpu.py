@@ -86,10 +86,11 @@ def test_bias_gradient_has_a_gradient():
     _lib.assert_healthy()
 
 
-# the fewest tokens that are sorted and one less, counts around a power of two and a block of eight, the most and one more, tables on
-# both sides of the rule; tokens of other shards, a buffer that holds something
+# few tokens and small tables, which are scattered, the most that are sorted and one more, two more that are sorted (the kernels on their
+# own: below); tokens of other shards, a buffer that holds something
 @pytest.mark.parametrize("tokens,rows,H", [(255, 12288, 264), (256, 12288, 264), (1025, 6145, 2056), (1024, 3071, 4096),
-                                           (1024, 3072, 4096), (16384, 98304, 2056), (16385, 98304, 2056)])
+                                           (1024, 3072, 4096), (16384, 98304, 2056), (16385, 98304, 2056), (1024, 16000, 4096),
+                                           (4097, 39532, 4096)])
 @pytest.mark.parametrize("fresh", [True, False])
 @pytest.mark.parametrize("positions", [False, True])
 def test_embedding_gradient(tokens, rows, H, fresh, positions):
