@@ -53,11 +53,9 @@ struct Kernels {
   int (*add)(V, V, void*, long long, void*);
   int (*rope)(void*, V, int, int, int, int, int, V, int, V, V, int, int, void*);
   int (*flash_fwd)(A, A, A, A, void*, int, int, int, int, int, int, int, int, int, float, void*);
-  int (*flash_bwd_tiles_pay)(int, int, int, int, int, int, int, int, int);
-  int (*flash_bwd_pieces)(int, int, int, int, int, int, int, int, int, long long*);
+  int (*flash_bwd_wants)(int, int, int, int, int, int, int, int, int, long long*);
   int (*flash_bwd_has_room)(int);
   int (*flash_bwd_no_room)(int);
-  long long (*flash_bwd_scratch_of)(int, int, int, int, int, int, int, int, int, int);
   int (*flash_bwd)(A, A, A, A, A, V, void*, long long, void* const*, int, long long, A, A, A, int, int, int, int, int, int, int, int, int, float, int*, void*);
   long long (*decoder_step_scratch)(const HgDecoderStep*);
   int (*decoder_step)(HgDecoderStep*, void*);
@@ -399,26 +397,30 @@ struct FlashPacked : public Function<FlashPacked> {
     const Packed l = layout(ctx);
     const Tensor dout = grads[0].contiguous();
     Tensor dqkv = at::empty_like(qkv);
-    const Tensor ws = empty({K.flash_bwd_scratch_of(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0, 0)}, at::kFloat, qkv);
-    variable_list tiles;                               // dS
-    std::vector<void*> tiles_at;
-    long long piece = 0;
-    if (K.flash_bwd_tiles_pay(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0) && K.flash_bwd_has_room(qkv.get_device())) {
-      const int n = K.flash_bwd_pieces(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0, &piece);
-      try {
-        for (int i = 0; i < n; ++i) tiles.push_back(empty({piece}, at::kFloat, qkv));
-      } catch (const c10::OutOfMemoryError&) {         // no room for dS: the kernels do without
-        K.flash_bwd_no_room(qkv.get_device());
-        tiles.clear();
-      }
-      for (const Tensor& t : tiles) tiles_at.push_back(t.data_ptr());
+    // Row sums and parts, and the pieces of dS; a single piece shares an allocation with the others.
+    long long wants[3];
+    K.flash_bwd_wants(l.S, l.S, l.B, l.nh, l.ng, l.hd, l.causal, 0, 0, wants);
+    int n = wants[1] > 0 && K.flash_bwd_has_room(qkv.get_device()) ? int(wants[1]) : 0;
+    Tensor ws;
+    variable_list tiles;
+    try {
+      ws = empty({wants[0] + (n == 1 ? wants[2] : 0)}, at::kFloat, qkv);
+      for (int i = 0; n > 1 && i < n; ++i) tiles.push_back(empty({wants[2]}, at::kFloat, qkv));
+    } catch (const c10::OutOfMemoryError&) {           // no room for dS: the kernels do without
+      if (n == 0) throw;
+      K.flash_bwd_no_room(qkv.get_device());
+      n = 0;
+      tiles.clear();
+      if (!ws.defined()) ws = empty({wants[0]}, at::kFloat, qkv);
     }
+    void* tiles_at[kHgDsPieces];
+    if (n == 1) tiles_at[0] = ws.data_ptr<float>() + wants[0];
+    for (int i = 0; n > 1 && i < n; ++i) tiles_at[i] = tiles[i].data_ptr();
     int kernels = 0;
     const HgAttnTensor q = l.q(qkv.data_ptr()), k = l.k(qkv.data_ptr()), v = l.v(qkv.data_ptr()), o = l.o(out.data_ptr()),
                        d = l.o(dout.data_ptr()), dq = l.q(dqkv.data_ptr()), dk = l.k(dqkv.data_ptr()), dv = l.v(dqkv.data_ptr());
-    check(K.flash_bwd(&q, &k, &v, &o, &d, lse.data_ptr(), ws.data_ptr(), ws.numel(), tiles_at.data(), int(tiles_at.size()), piece, &dq,
-                      &dk, &dv, l.S, l.S, l.B, l.nh, l.ng,
-                      l.hd, l.causal, 0, 0, l.scale, &kernels, stream()), "hg_flash_bwd");
+    check(K.flash_bwd(&q, &k, &v, &o, &d, lse.data_ptr(), ws.data_ptr(), wants[0], tiles_at, n, wants[2], &dq, &dk, &dv, l.S, l.S,
+                      l.B, l.nh, l.ng, l.hd, l.causal, 0, 0, l.scale, &kernels, stream()), "hg_flash_bwd");
     count(kernels);
     return {dqkv, Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
   }
@@ -720,7 +722,7 @@ void bind(const py::dict& fn, bool half, int pair_mode, py::object kernel_error)
   at("hg_colsum_parts", K.colsum_parts); at("hg_colsum", K.colsum);
   at("hg_norm_fwd", K.norm_fwd); at("hg_norm_bwd", K.norm_bwd);
   at("hg_glu_fwd", K.glu_fwd); at("hg_glu_bwd", K.glu_bwd); at("hg_add_bf16", K.add); at("hg_rope", K.rope);
-  at("hg_flash_fwd", K.flash_fwd); at("hg_flash_bwd_tiles_pay", K.flash_bwd_tiles_pay); at("hg_flash_bwd_pieces", K.flash_bwd_pieces); at("hg_flash_bwd_has_room", K.flash_bwd_has_room); at("hg_flash_bwd_no_room", K.flash_bwd_no_room); at("hg_flash_bwd_scratch_of", K.flash_bwd_scratch_of); at("hg_flash_bwd_ws", K.flash_bwd);
+  at("hg_flash_fwd", K.flash_fwd); at("hg_flash_bwd_wants", K.flash_bwd_wants); at("hg_flash_bwd_has_room", K.flash_bwd_has_room); at("hg_flash_bwd_no_room", K.flash_bwd_no_room); at("hg_flash_bwd_ws", K.flash_bwd);
   at("hg_decoder_step_scratch", K.decoder_step_scratch); at("hg_decoder_step", K.decoder_step);
   g_lp = half ? at::kHalf : at::kBFloat16;
   g_pair_mode = pair_mode;

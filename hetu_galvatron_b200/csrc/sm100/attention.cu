@@ -854,7 +854,7 @@ __host__ __device__ __forceinline__ long long ds_tiles_before(const BwdParams& p
 // not stored).  A tile is what the tensor core reads as an M-major operand without swizzle, [2 x 64 keys][16 x 8 queries][64 keys][8
 // queries]: a warp's store of eight queries of 32 keys is 512 bytes in a row (as rows of 128 queries, 32 pieces of 32 bytes, these
 // stores doubled the kernel's time), and half a tile one copy.
-constexpr int kDsPieces = 64;
+constexpr int kDsPieces = kHgDsPieces;
 struct DsPieces {
   hg_lp_t* at[kDsPieces];
   int heads;
@@ -2639,11 +2639,18 @@ int hg_flash_bwd_pieces(int Sq, int Skv, int B, int nheads, int nkv, int hd, int
   *floats = w.piece;
   return w.cut.pieces;
 }
-// Whether it is worth giving them.
-int hg_flash_bwd_tiles_pay(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0) {
+// What a caller should give hg_flash_bwd_ws: floats of scratch, pieces for dS (0 where storing it does not pay), floats of each.
+int hg_flash_bwd_wants(int Sq, int Skv, int B, int nheads, int nkv, int hd, int causal, int q_pos0, int k_pos0, long long* wants) {
+  wants[0] = wants[1] = wants[2] = 0;
   if (Sq <= 0 || Skv <= 0 || B <= 0 || nheads <= 0 || nkv <= 0) return 0;
   const BwdParams p = bwd_sizes(Sq, Skv, B, nheads, nkv, causal, q_pos0, k_pos0);
-  return ds_pays(bwd_scratch(p, Skv, nkv, hd).cut, p, Skv, nkv, hd);
+  const BwdScratch w = bwd_scratch(p, Skv, nkv, hd);
+  wants[0] = w.sums + w.parts;
+  if (ds_pays(w.cut, p, Skv, nkv, hd)) {
+    wants[1] = w.cut.pieces;
+    wants[2] = w.piece;
+  }
+  return 0;
 }
 
 // Where the caller's allocator had no room for dS, the next kNoRoomCalls backwards of that device do not ask it again: a caching

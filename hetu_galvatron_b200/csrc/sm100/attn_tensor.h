@@ -8,3 +8,6 @@ struct HgAttnTensor {
   int slots;
   int gs, hs, off;
 };
+
+// Most pieces of scratch that the backward keeps dS in.
+constexpr int kHgDsPieces = 64;

@@ -2,4 +2,4 @@
 // address, and the structs that it hands them.  Both sides export it; raise it with any change of those.
 #pragma once
 
-constexpr int kHgNativeInterface = 6;
+constexpr int kHgNativeInterface = 7;

@@ -139,7 +139,7 @@ _SIGNATURES = {
                     [c_int] * 9 + [c_float, c_void_p],
     "hg_flash_bwd_scratch": [c_int] * 9,
     "hg_flash_bwd_scratch_of": [c_int] * 10,
-    "hg_flash_bwd_tiles_pay": [c_int] * 9,
+    "hg_flash_bwd_wants": [c_int] * 9 + [ctypes.POINTER(c_ll)],
     "hg_flash_bwd_pieces": [c_int] * 9 + [ctypes.POINTER(c_ll)],
     "hg_flash_bwd_has_room": [c_int],
     "hg_flash_bwd_no_room": [c_int],
@@ -221,8 +221,8 @@ def _bind_native(lib):
         warnings.warn("hg_torch_ops is not usable (%s): autograd nodes run in Python" % (e,))
         return
     names = ("hg_gemm_bf16", "hg_gemm2_bf16", "hg_gemm2_scratch", "hg_gemm_skinny_bf16", "hg_colsum_parts", "hg_colsum", "hg_norm_fwd",
-             "hg_norm_bwd", "hg_glu_fwd", "hg_glu_bwd", "hg_add_bf16", "hg_rope", "hg_flash_fwd", "hg_flash_bwd_tiles_pay", "hg_flash_bwd_pieces", "hg_flash_bwd_has_room", "hg_flash_bwd_no_room",
-             "hg_flash_bwd_scratch_of", "hg_flash_bwd_ws", "hg_decoder_step", "hg_decoder_step_scratch")
+             "hg_norm_bwd", "hg_glu_fwd", "hg_glu_bwd", "hg_add_bf16", "hg_rope", "hg_flash_fwd", "hg_flash_bwd_wants", "hg_flash_bwd_has_room", "hg_flash_bwd_no_room",
+             "hg_flash_bwd_ws", "hg_decoder_step", "hg_decoder_step_scratch")
     mode = {"0": 0, "1": 1}.get(os.environ.get("HG_GEMM_PAIR", "auto"), -1)
     hg_torch_ops.bind({n: ctypes.cast(getattr(lib, n), c_void_p).value for n in names}, _PRECISION == "fp16", mode, KernelError)
     NATIVE = hg_torch_ops

@@ -53,13 +53,12 @@ def attention_reference(q, k, v, causal=True, scale=None, q_pos0=0, k_pos0=0, dr
 def _backward_scratch(lib, S, Skv, B, nh, ng, hd, causal, q_pos0, k_pos0, device):
     """fp32 scratch of the backward kernels: row sums of dO * O and, where key blocks are shared between CTAs, their parts; and the
     pieces that hold dS where storing it pays, none if there is no room for them: dQ then takes longer."""
-    args = (S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0)
-    ws = torch.empty(lib.hg_flash_bwd_scratch_of(*args, 0), dtype=torch.float32, device=device)
-    if lib.hg_flash_bwd_tiles_pay(*args) and lib.hg_flash_bwd_has_room(device.index):
-        floats = ctypes.c_longlong()
+    wants = (ctypes.c_longlong * 3)()
+    lib.hg_flash_bwd_wants(S, Skv, B, nh, ng, hd, int(causal), q_pos0, k_pos0, wants)
+    ws = torch.empty(wants[0], dtype=torch.float32, device=device)
+    if wants[1] and lib.hg_flash_bwd_has_room(device.index):
         try:
-            n = lib.hg_flash_bwd_pieces(*args, ctypes.byref(floats))
-            return ws, [torch.empty(floats.value, dtype=torch.float32, device=device) for _ in range(n)]
+            return ws, [torch.empty(wants[2], dtype=torch.float32, device=device) for _ in range(wants[1])]
         except torch.cuda.OutOfMemoryError:
             lib.hg_flash_bwd_no_room(device.index)
     return ws, []

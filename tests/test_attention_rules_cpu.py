@@ -17,7 +17,10 @@ from hetu_galvatron_b200.ops import _lib, attention
     (300, 1, 2, 1, 128, 1, 900, False)])
 def test_rule_of_stored_ds(S, B, nh, ng, hd, causal, k0, stored):
     lib, sizes = _lib.load(), (S, S, B, nh, ng, hd, causal, 0, k0)
-    assert bool(lib.hg_flash_bwd_tiles_pay(*sizes)) is stored
+    wants, floats = (ctypes.c_longlong * 3)(), ctypes.c_longlong()
+    lib.hg_flash_bwd_wants(*sizes, wants)
+    n = lib.hg_flash_bwd_pieces(*sizes, ctypes.byref(floats))
+    assert list(wants) == [lib.hg_flash_bwd_scratch_of(*sizes, 0), *((n, floats.value) if stored else (0, 0))]
     assert 4 * (lib.hg_flash_bwd_scratch(*sizes) - lib.hg_flash_bwd_scratch_of(*sizes, 0)) <= 3 << 29
 
 
